@@ -1,5 +1,7 @@
 // extern "C" surface declared in include/nerve_b200.h: exception -> status + thread-local message.
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <exception>
 #include <string>
 
@@ -467,9 +469,65 @@ int32_t nerve_b200_debug_target_logits(nerve_b200_engine *engine, int64_t stream
 
 // ---- operator-level entry points
 
+namespace {
+
+// The INT4 linears of more than eight lanes read their activations in the GEMM's operand form; the callers of the
+// operator-level entry points lend no scratch for it, so it comes stream-ordered from a pool of this library's own per
+// device: safe with any number of streams and threads, a call costs no device allocation once the pool is warm, and
+// what the pool keeps beyond 64 MB goes back to the device at the next synchronisation.
+class PreparedActivations {
+public:
+    PreparedActivations(const void *x, int32_t lanes, int32_t n, int32_t k, cudaStream_t stream) : stream_(stream) {
+        if (!linear_int4_gemm_supported(lanes, n, k)) return;
+        cudaMemPool_t pool = nullptr;
+        status_ = device_pool(&pool);
+        if (status_ == cudaSuccess) status_ = cudaMallocFromPoolAsync(&buffer_, int4_activation_bytes(lanes, k), pool, stream);
+        if (status_ == cudaSuccess) status_ = launch_prepare_activations(static_cast<const uint16_t *>(x), buffer_, lanes, k, stream);
+    }
+    ~PreparedActivations() {
+        if (buffer_ != nullptr) cudaFreeAsync(buffer_, stream_);
+    }
+    PreparedActivations(const PreparedActivations &) = delete;
+    cudaError_t status() const { return status_; }
+    const void *get() const { return buffer_; }
+
+private:
+    static cudaError_t device_pool(cudaMemPool_t *out) {
+        static std::mutex mutex;
+        static std::map<int, cudaMemPool_t> pools;
+        int device = 0;
+        cudaError_t status = cudaGetDevice(&device);
+        if (status != cudaSuccess) return status;
+        std::lock_guard<std::mutex> lock(mutex);
+        auto found = pools.find(device);
+        if (found == pools.end()) {
+            cudaMemPoolProps properties = {};
+            properties.allocType = cudaMemAllocationTypePinned;
+            properties.location.type = cudaMemLocationTypeDevice;
+            properties.location.id = device;
+            cudaMemPool_t pool = nullptr;
+            status = cudaMemPoolCreate(&pool, &properties);
+            if (status != cudaSuccess) return status;
+            uint64_t keep = uint64_t(64) << 20;
+            status = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            if (status != cudaSuccess) return status;
+            found = pools.emplace(device, pool).first;
+        }
+        *out = found->second;
+        return cudaSuccess;
+    }
+    cudaStream_t stream_;
+    void *buffer_ = nullptr;
+    cudaError_t status_ = cudaSuccess;
+};
+
+}  // namespace
+
 int32_t nerve_b200_op_linear_int4(const void *x, const void *qweight, const void *scales, void *y, const void *residual, int32_t lanes,
                                   int32_t n, int32_t k, int32_t group, void *stream) {
-    return cuda_status(launch_linear_int4(static_cast<const uint16_t *>(x), static_cast<const uint32_t *>(qweight),
+    const PreparedActivations prepared(x, group == 128 ? lanes : 0, n, k, static_cast<cudaStream_t>(stream));
+    if (prepared.status() != cudaSuccess) return cuda_status(prepared.status(), "nerve_b200_op_linear_int4 (activations)");
+    return cuda_status(launch_linear_int4(static_cast<const uint16_t *>(x), prepared.get(), static_cast<const uint32_t *>(qweight),
                                           static_cast<const uint16_t *>(scales), static_cast<uint16_t *>(y),
                                           static_cast<const uint16_t *>(residual), lanes, n, k, group,
                                           residual ? EPILOGUE_RESIDUAL_ROUNDED : EPILOGUE_BF16, static_cast<cudaStream_t>(stream)),
@@ -478,7 +536,9 @@ int32_t nerve_b200_op_linear_int4(const void *x, const void *qweight, const void
 
 int32_t nerve_b200_op_linear_int4_silu_pair(const void *x, const void *gate_q, const void *gate_s, const void *up_q, const void *up_s,
                                             void *y, int32_t lanes, int32_t n, int32_t k, void *stream) {
-    return cuda_status(launch_linear_int4_silu_pair(static_cast<const uint16_t *>(x), static_cast<const uint32_t *>(gate_q),
+    const PreparedActivations prepared(x, lanes, n, k, static_cast<cudaStream_t>(stream));
+    if (prepared.status() != cudaSuccess) return cuda_status(prepared.status(), "nerve_b200_op_linear_int4_silu_pair (activations)");
+    return cuda_status(launch_linear_int4_silu_pair(static_cast<const uint16_t *>(x), prepared.get(), static_cast<const uint32_t *>(gate_q),
                                                     static_cast<const uint16_t *>(gate_s), static_cast<const uint32_t *>(up_q),
                                                     static_cast<const uint16_t *>(up_s), static_cast<uint16_t *>(y), lanes, n, k,
                                                     static_cast<cudaStream_t>(stream)),

@@ -518,6 +518,15 @@ Engine::Engine(std::shared_ptr<MountedModel> model) : model_(std::move(model)) {
         for (const ComponentPlan &layer : plan.draft_layers) declare(layer);
     }
     for (auto &entry : signals_) entry.second = device_alloc(entry.second.bytes);
+    int64_t int4_columns = 0;
+    auto widest = [&](const ComponentPlan &component) {
+        for (const OpSpec &op : component.ops)
+            for (const WeightRef &w : op.weights)
+                if (w.storage == TensorStorage::INT4_CT) int4_columns = std::max(int4_columns, w.k);
+    };
+    for (const ComponentPlan &layer : plan.layers) widest(layer);
+    for (const ComponentPlan &layer : plan.draft_layers) widest(layer);
+    if (int4_columns > 0) int4_activations_ = device_alloc(int4_activation_bytes(options.max_lanes, static_cast<int>(int4_columns)));
 
     frame_a_ = device_alloc(lanes * frame);
     frame_b_ = device_alloc(lanes * frame);
@@ -600,7 +609,7 @@ Engine::~Engine() {
     for (auto &entry : signals_) cudaFree(entry.second.ptr);
     for (DeviceBuffer *buffer : {&frame_a_, &frame_b_, &embedding_out_, &normalized_, &draft_normalized_, &draft_hidden_in_, &logits_,
                                  &records_, &argmax_scratch_, &sampler_scratch_, &sampler_table_, &lane_tokens_, &lane_positions_, &lane_slots_, &pending_hidden_, &pending_backup_, &attention_scratch_,
-                                 &cycle_state_, &kernel_error_, &tp_partial_, &tp_exchange_, &tp_description_, &stack_q_, &stack_attention_out_, &stack_activation_, &stack_barrier_, &stack_timing_, &prefix_pending_})
+                                 &cycle_state_, &int4_activations_, &kernel_error_, &tp_partial_, &tp_exchange_, &tp_description_, &stack_q_, &stack_attention_out_, &stack_activation_, &stack_barrier_, &stack_timing_, &prefix_pending_})
         cudaFree(buffer->ptr);
     cudaFreeHost(staging_);
     cudaFreeHost(host_records_);
@@ -1174,6 +1183,17 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
         if (signal == plan.boundary_output) count += 1;
         return count;
     };
+    // The activations of an INT4 linear of more than eight lanes in the GEMM's operand form: prepared once per signal,
+    // whichever linears read it.
+    std::string prepared_signal;
+    auto prepared = [&](const std::string &signal) -> const void * {
+        if (lanes <= 8) return nullptr;
+        if (prepared_signal != signal) {
+            check(launch_prepare_activations(u16(signal), int4_activations_.ptr, lanes, width(signal), st), "int4 activations");
+            prepared_signal = signal;
+        }
+        return int4_activations_.ptr;
+    };
     auto is_int4_single = [&](const OpSpec &op) {
         return op.kind == OpKind::Linear && op.weights.size() == 1 && op.weights[0].storage == TensorStorage::INT4_CT &&
                op.weights[0].group == 128;
@@ -1195,7 +1215,7 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
                 float *partial = static_cast<float *>(tp_partial_.ptr);
                 if (w.storage == TensorStorage::INT4_CT) {
                     profile_begin(static_cast<uint64_t>(w.n) * (w.k / 2 + w.k / 64));
-                    check(launch_linear_int4(u16(op.inputs[0]), static_cast<const uint32_t *>(weight(w.tensor)),
+                    check(launch_linear_int4(u16(op.inputs[0]), prepared(op.inputs[0]), static_cast<const uint32_t *>(weight(w.tensor)),
                                              static_cast<const uint16_t *>(weight(w.scale)), reinterpret_cast<uint16_t *>(partial), nullptr, lanes,
                                              static_cast<int>(w.n), static_cast<int>(w.k), w.group, EPILOGUE_F32_SCALED, st, static_cast<int *>(kernel_error_.ptr)),
                           "linear_int4 (row-parallel)");
@@ -1220,21 +1240,19 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
                 break;
             }
             if (is_int4_single(op)) {
-                // gate/up + SiLU*up in one launch (batches below the GEMM threshold; wide batches run the three operators
-                // as the package lists them, the two projections as tensor-core GEMMs)
-                if (!linear_int4_gemm_supported(lanes, static_cast<int>(op.weights[0].n), static_cast<int>(op.weights[0].k)) &&
-                    index + 2 < plan.ops.size() && is_int4_single(plan.ops[index + 1]) && plan.ops[index + 2].kind == OpKind::SiluMultiply &&
+                // gate/up + SiLU*up in one launch
+                if (index + 2 < plan.ops.size() && is_int4_single(plan.ops[index + 1]) && plan.ops[index + 2].kind == OpKind::SiluMultiply &&
                     plan.ops[index + 1].inputs[0] == op.inputs[0] && plan.ops[index + 2].inputs[0] == op.outputs[0] &&
                     plan.ops[index + 2].inputs[1] == plan.ops[index + 1].outputs[0] && op.weights[0].n == plan.ops[index + 1].weights[0].n &&
                     consumers(op.outputs[0], index + 3) == 0 && consumers(plan.ops[index + 1].outputs[0], index + 3) == 0) {
                     const OpSpec &up = plan.ops[index + 1];
                     profile_begin(2 * static_cast<uint64_t>(op.weights[0].n) * (op.weights[0].k / 2 + op.weights[0].k / 64));
-                    check(launch_linear_int4_silu_pair(u16(op.inputs[0]), static_cast<const uint32_t *>(weight(op.weights[0].tensor)),
+                    check(launch_linear_int4_silu_pair(u16(op.inputs[0]), prepared(op.inputs[0]), static_cast<const uint32_t *>(weight(op.weights[0].tensor)),
                                                        static_cast<const uint16_t *>(weight(op.weights[0].scale)),
                                                        static_cast<const uint32_t *>(weight(up.weights[0].tensor)),
                                                        static_cast<const uint16_t *>(weight(up.weights[0].scale)),
                                                        u16(plan.ops[index + 2].outputs[0]), lanes, static_cast<int>(op.weights[0].n),
-                                                       static_cast<int>(op.weights[0].k), st),
+                                                       static_cast<int>(op.weights[0].k), st, static_cast<int *>(kernel_error_.ptr)),
                           "linear_int4 gate/up");
                     profile_end();
                     index += 2;
@@ -1252,7 +1270,7 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
                     const OpSpec &add = plan.ops[index + 1];
                     const std::string &residual = add.inputs[0] == op.outputs[0] ? add.inputs[1] : add.inputs[0];
                     profile_begin(static_cast<uint64_t>(op.weights[0].n) * (op.weights[0].k / 2 + op.weights[0].k / 64));
-                    check(launch_linear_int4(u16(op.inputs[0]), static_cast<const uint32_t *>(weight(op.weights[0].tensor)),
+                    check(launch_linear_int4(u16(op.inputs[0]), prepared(op.inputs[0]), static_cast<const uint32_t *>(weight(op.weights[0].tensor)),
                                              static_cast<const uint16_t *>(weight(op.weights[0].scale)), u16(add.outputs[0]), u16(residual),
                                              lanes, static_cast<int>(op.weights[0].n), static_cast<int>(op.weights[0].k), 128,
                                              EPILOGUE_RESIDUAL_ROUNDED, st, static_cast<int *>(kernel_error_.ptr)),
@@ -1275,7 +1293,7 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
                     ns[branches] = static_cast<int>(plan.ops[i].weights[0].n);
                 }
                 profile_begin(branch_bytes);
-                check(launch_linear_int4_multi(u16(op.inputs[0]), branches, qweights, scales, outputs, ns, nullptr, lanes,
+                check(launch_linear_int4_multi(u16(op.inputs[0]), prepared(op.inputs[0]), branches, qweights, scales, outputs, ns, nullptr, lanes,
                                                static_cast<int>(op.weights[0].k), EPILOGUE_BF16, st, static_cast<int *>(kernel_error_.ptr)),
                       "linear_int4");
                 profile_end();
@@ -1296,7 +1314,7 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
                               "linear_bf16");
                     }
                 } else if (w.storage == TensorStorage::INT4_CT) {
-                    check(launch_linear_int4(u16(op.inputs[0]), static_cast<const uint32_t *>(weight(w.tensor)),
+                    check(launch_linear_int4(u16(op.inputs[0]), prepared(op.inputs[0]), static_cast<const uint32_t *>(weight(w.tensor)),
                                              static_cast<const uint16_t *>(weight(w.scale)), u16(op.outputs[branch]), nullptr, lanes,
                                              static_cast<int>(w.n), static_cast<int>(w.k), w.group, EPILOGUE_BF16, st, static_cast<int *>(kernel_error_.ptr)),
                           "linear_int4");
@@ -1325,7 +1343,7 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
                                         EPILOGUE_RESIDUAL_F32, st),
                       "linear_residual_fp8");
             } else {
-                check(launch_linear_int4(u16(op.inputs[0]), static_cast<const uint32_t *>(weight(w.tensor)),
+                check(launch_linear_int4(u16(op.inputs[0]), prepared(op.inputs[0]), static_cast<const uint32_t *>(weight(w.tensor)),
                                          static_cast<const uint16_t *>(weight(w.scale)), u16(op.outputs[0]), u16(op.residual_input), lanes,
                                          static_cast<int>(w.n), static_cast<int>(w.k), w.group, EPILOGUE_RESIDUAL_ROUNDED, st, static_cast<int *>(kernel_error_.ptr)),
                       "linear_residual_int4");
@@ -1348,11 +1366,11 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
                                                       static_cast<int>(gate.n), static_cast<int>(gate.k), st),
                       "linear_silu_multiply_fp8");
             } else {
-                check(launch_linear_int4_silu_pair(u16(op.inputs[0]), static_cast<const uint32_t *>(weight(gate.tensor)),
+                check(launch_linear_int4_silu_pair(u16(op.inputs[0]), prepared(op.inputs[0]), static_cast<const uint32_t *>(weight(gate.tensor)),
                                                    static_cast<const uint16_t *>(weight(gate.scale)),
                                                    static_cast<const uint32_t *>(weight(up.tensor)),
                                                    static_cast<const uint16_t *>(weight(up.scale)), u16(op.outputs[0]), lanes,
-                                                   static_cast<int>(gate.n), static_cast<int>(gate.k), st),
+                                                   static_cast<int>(gate.n), static_cast<int>(gate.k), st, static_cast<int *>(kernel_error_.ptr)),
                       "linear_silu_multiply_int4");
             }
             break;

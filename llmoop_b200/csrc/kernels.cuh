@@ -61,8 +61,10 @@ cudaError_t launch_linear_silu_multiply_bf16(const uint16_t *x, const uint16_t *
                                              int lanes, int n, int k, cudaStream_t stream);
 
 // INT4 compressed-tensors weight-only linear: qweight [n][k/8] u32, scales bf16 [n][k/group].
-// error_flag (optional device word): set to 3 by the wide-batch GEMM if one of its bounded waits expires.
-cudaError_t launch_linear_int4(const uint16_t *x, const uint32_t *qweight, const uint16_t *scales, uint16_t *y,
+// Batches of more than 8 lanes run the tensor-core GEMM, which reads the activations from `prepared`
+// (launch_prepare_activations of the same x); smaller ones read x.
+// error_flag (optional device word): set to 3 by the GEMM if one of its bounded waits expires.
+cudaError_t launch_linear_int4(const uint16_t *x, const void *prepared, const uint32_t *qweight, const uint16_t *scales, uint16_t *y,
                                const uint16_t *residual, int lanes, int n, int k, int group, int epilogue,
                                cudaStream_t stream, int *error_flag = nullptr);
 
@@ -100,13 +102,13 @@ cudaError_t launch_attention(const uint16_t *q, uint16_t *out, const KvLayer &kv
                              float *scratch, cudaStream_t stream);
 
 // INT4 multi-branch forms (one launch for q/k/v; gate/up with the SiLU*up epilogue).
-cudaError_t launch_linear_int4_multi(const uint16_t *x, int branches, const uint32_t *const *qweights,
+cudaError_t launch_linear_int4_multi(const uint16_t *x, const void *prepared, int branches, const uint32_t *const *qweights,
                                      const uint16_t *const *scales, uint16_t *const *ys, const int *ns,
                                      const uint16_t *residual, int lanes, int k, int epilogue, cudaStream_t stream,
                                      int *error_flag = nullptr);
-cudaError_t launch_linear_int4_silu_pair(const uint16_t *x, const uint32_t *gate_q, const uint16_t *gate_s,
+cudaError_t launch_linear_int4_silu_pair(const uint16_t *x, const void *prepared, const uint32_t *gate_q, const uint16_t *gate_s,
                                          const uint32_t *up_q, const uint16_t *up_s, uint16_t *y, int lanes, int n,
-                                         int k, cudaStream_t stream);
+                                         int k, cudaStream_t stream, int *error_flag = nullptr);
 
 // ---- streaming output projection for at most 8 lanes (kernels_projection.cu) ----
 // logits[lane][row] = scale * x[lane] . table[first_row + row], f32, rows of a slice that starts at a multiple of 16.
@@ -118,20 +120,21 @@ bool output_projection_supported(int lanes, int k);
 cudaError_t launch_output_projection(const uint16_t *x, const void *streamed_table, int first_row, float *logits, int lanes, int rows, int k, float scale,
                                      int grid, int *error_flag, cudaStream_t stream, uint16_t *rounded = nullptr);
 
-// ---- INT4 g128 GEMM on the tcgen05 tensor cores for 64 lanes and more (kernels_int4_gemm.cu) ----
-// One CTA per 128 rows x 64 lanes; the launchers above use it for such batches.  y and the epilogues as for
-// launch_linear_int4 (EPILOGUE_F32_SCALED writes f32 * scale).  error_flag (optional device word) is set to 3 if a
-// bounded wait for the tensor core expires.
+// ---- INT4 g128 GEMM on the tcgen05 tensor cores for more than 8 lanes (kernels_int4_gemm.cu) ----
+// `prepared` holds the activations in the GEMM's operand form (int4_activation_bytes bytes, 16-byte aligned), written
+// by launch_prepare_activations from bf16 [lanes][k].  y and the epilogues as for launch_linear_int4
+// (EPILOGUE_F32_SCALED writes f32 * scale); with `silu` the two matrices are a gate/up pair and ys[0] takes
+// bf16(silu_bf16(bf16 gate) * bf16 up).  error_flag (optional device word) is set to 3 if a bounded wait expires.
 bool linear_int4_gemm_supported(int lanes, int n, int k);
+size_t int4_activation_bytes(int lanes, int k);
+cudaError_t launch_prepare_activations(const uint16_t *x, void *prepared, int lanes, int k, cudaStream_t stream);
+cudaError_t launch_linear_int4_gemm(const void *prepared, int branches, const uint32_t *const *qweights, const uint16_t *const *scales, void *const *ys,
+                                    const int *ns, const uint16_t *residual, int lanes, int k, int epilogue, float scale, bool silu, int *error_flag,
+                                    cudaStream_t stream);
 // bf16 weights, batches of 16 lanes and more (tcgen05): called by launch_linear_bf16.
 bool linear_bf16_gemm_supported(int lanes, int n, int k);
 cudaError_t launch_linear_bf16_gemm(const uint16_t *x, const uint16_t *w, void *y, const uint16_t *residual, int lanes, int n, int k, int epilogue,
                                     float scale, int *error_flag, cudaStream_t stream);
-cudaError_t launch_linear_int4_gemm_multi(const uint16_t *x, int branches, const uint32_t *const *qweights, const uint16_t *const *scales, void *const *ys,
-                                          const int *ns, const uint16_t *residual, int lanes, int k, int epilogue, float scale, int *error_flag,
-                                          cudaStream_t stream);
-cudaError_t launch_linear_int4_gemm(const uint16_t *x, const uint32_t *qweight, const uint16_t *scales, void *y, const uint16_t *residual, int lanes,
-                                    int n, int k, int epilogue, float scale, int *error_flag, cudaStream_t stream);
 
 // ---- persistent decode stack (kernels_stack.cu) ----
 // One cooperative launch runs a whole stack of dense INT4 g128 Llama-style layers for a batch of at most 8 lanes:

@@ -1,23 +1,31 @@
-// INT4 g128 weight-only linear for batches of 64 lanes and more (prefill chunks, wide verify batches) on the
-// fifth-generation tensor cores: y[m][n] = sum_k x[m][k] * (q[n][k] - 8) * scale[n][k / 128], the arithmetic of
-// linear_int4_ct.comp.template:80-150 with the tile-level structure of the reference's prefill kernel
-// (linear_batch_cooperative_int4.comp.template:78-212).
+// INT4 g128 weight-only linear for batches of more than eight lanes (prefill chunks, many-stream verify and draft
+// batches) on the fifth-generation tensor cores: y[m][n] = sum_k x[m][k] * (q[n][k] - 8) * scale[n][k / 128], the
+// arithmetic of linear_int4_ct.comp.template:80-150 (tile structure of the reference's prefill kernel:
+// linear_batch_cooperative_int4.comp.template:78-212).
 //
-// One CTA computes a 128 (weight rows) x 64 (lanes) tile.  The weight rows are the M side of tcgen05.mma, the lanes
-// its N side; both operands are bf16 in shared memory in the K-major core-matrix layout (8 rows x 16 bytes per core
-// matrix, no swizzle), the f32 accumulator lives in tensor memory.  Per quantisation group of 128 columns:
-//   1. all 256 threads fetch the group's packed nibbles (64 bytes per row) and the lanes' activations, turn the
-//      nibbles into exact bf16 (q - 8) - lop3 into the mantissa of 128.0, subtract 136 - and store both tiles; the
-//      eight values of a 16-byte piece sit in the order (0,4,1,5,2,6,3,7) on both sides, which the contraction
-//      does not see;
-//   2. one thread issues eight tcgen05.mma (K = 16 each) into one of two accumulator buffers, starting it from zero,
-//      and commits them to an mbarrier;
-//   3. while the tensor core works on this group, the threads read the previous group's accumulator back
-//      (tcgen05.ld, one row per thread), multiply it by the row's group scale and add it to f32 registers - the
-//      reference's order: f32 sum inside a group, one multiplication by the scale, f32 sum over the groups.
-// Shared-memory tiles and accumulators are double-buffered, so fetching, the MMAs and the scaling of three
-// consecutive groups overlap.  Waits are bounded; a wait that expires sets the error word, and the CTA still frees
-// its tensor memory before it leaves.
+// Operands.  (q - 8) has at most three significant bits and a bf16 scale eight, so their product fits the eleven of
+// fp16 exactly: the weights enter the tensor core as fp16 (q - 8) * scale * 2^p with p chosen per row so that the
+// row's largest scale lies in [2^11, 2^12) - exact for every scale down to 2^-29 of the largest, and below that the
+// loss is 2^-40 of the row's largest weight.  The activations are bf16 times a power of two chosen per lane so that
+// the lane's largest value lies in [2^14, 2^15), as fp16: exact down to 2^-29 of the largest value.  Both powers of
+// two come off again in the epilogue.  No group scale is left to apply to partial sums, so the f32 accumulator stays
+// in tensor memory over the whole of K (one that is read back, scaled and added up in registers for every group of
+// 128 columns ran at 140-175 TFLOP/s: the tensor pipe was idle 87 % of the time).
+//
+// Roles.  A CTA computes ROW_TILES x 128 weight rows (M side) by up to 256 / ROW_TILES lanes (N side):
+//   8 x ROW_TILES warps bring their rows' packed nibbles into shared memory with cp.async several groups ahead (32 rows x 64
+//              bytes per warp and group, private to the warp), turn them into fp16 and write them into tensor memory
+//              (tcgen05.st): the A operand never touches shared memory, whose bandwidth the B operand needs;
+//   the next warp: one thread issues the MMAs (A from tensor memory, B from shared memory) and commits;
+//   the last warp: one thread copies the activations, which prepare_activations_kernel left in global memory in the
+//              order of the 128-byte-swizzled shared-memory tiles: two bulk copies per group of 128 columns.
+// With ROW_TILES = 2 every activation byte read from L2 feeds two MMAs.  K may be split over a cluster of CTAs whose
+// partial sums meet through distributed shared memory (shapes with too few tiles to fill the chip).
+// Waits are bounded; a wait that expires sets the error word, and the CTA still frees its tensor memory.
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -25,37 +33,17 @@ namespace nerve {
 
 namespace {
 
-constexpr int GEMM_ROWS = 128;     // weight rows per CTA (MMA M)
-constexpr int GEMM_MIN_LANES = 64; // lanes per CTA (MMA N): 64, or 128 for batches of 128 lanes and more - the weights
-                                   // are then dequantised once per 128 lanes
-constexpr int GEMM_THREADS = 256;
-constexpr int GEMM_A_BYTES = GEMM_ROWS * 128 * 2;    // one group of a row block, bf16
-constexpr int GEMM_BLOCK_STRIDE = 16 * 128;          // bytes between 8-row blocks: 16 core matrices of a group's K
-constexpr unsigned int GEMM_SPIN_LIMIT = 1u << 22;
-template <int LANES>
-constexpr size_t gemm_smem() { return 2 * (GEMM_A_BYTES + LANES * 128 * 2) + 64; }
+template <int ROW_TILES>
+constexpr int gemm_threads() { return ROW_TILES * 256 + 64; }
+constexpr unsigned int GEMM_SPIN_LIMIT = 1u << 17;
+constexpr int GEMM_MAX_B_STAGES = 8, GEMM_MAX_A_STAGES = 4;
+constexpr size_t GEMM_SMEM_ONE = 225 * 1024, GEMM_SMEM_TWO = 111 * 1024;  // one or two CTAs per SM
+constexpr size_t GEMM_BARRIER_BYTES = 256, GEMM_TAIL_BYTES = GEMM_BARRIER_BYTES + 256 * sizeof(float);  // barriers, lane factors
 
-// 32-bit instruction descriptor of tcgen05.mma kind::f16: f32 accumulator (bits 4-5 = 1), A and B bf16 (bits 7-9 and
-// 10-12 = 1), both K-major (bits 15, 16 = 0), N / 8 in bits 17-22, M / 16 in bits 24-28.
-template <int LANES>
-constexpr uint32_t gemm_instruction() {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(LANES / 8) << 17) | (static_cast<uint32_t>(GEMM_ROWS / 16) << 24);
-}
-
-// Shared-memory matrix descriptor, K-major without swizzle: start address / 16 in bits 0-13, the byte distance
-// between the two core matrices of a K = 16 step (128) / 16 in bits 16-29, the distance between 8-row blocks / 16 in
-// bits 32-45, descriptor version 1 in bits 46-47.
-__device__ __forceinline__ uint64_t matrix_descriptor(uint32_t shared_address) {
-    return static_cast<uint64_t>((shared_address & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(128 >> 4) << 16) |
-           (static_cast<uint64_t>(GEMM_BLOCK_STRIDE >> 4) << 32) | (1ull << 46);
-}
-
-// Two nibbles (bits s..s+3 and s+16..s+19 of `word`) -> bf16x2 (q - 8, q' - 8), exact.
-__device__ __forceinline__ uint32_t nibble_pair_bf16(uint32_t word, int shift) {
-    uint32_t biased, out;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(biased) : "r"(word >> shift), "n"(0x000F000F), "n"(0x43004300));
-    asm("sub.bf16x2 %0, %1, %2;" : "=r"(out) : "r"(biased), "r"(0x43084308u));
-    return out;
+// Shared-memory matrix descriptor, K-major, 128-byte swizzle: start address / 16 in bits 0-13, 1024 bytes between
+// 8-row atoms / 16 in bits 32-45, descriptor version 1 in bits 46-47, swizzle mode 2 (128 bytes) in bits 61-63.
+__device__ __forceinline__ uint64_t swizzled_descriptor(uint32_t shared_address) {
+    return static_cast<uint64_t>((shared_address & 0x3FFFFu) >> 4) | (1ull << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
 
 __device__ __forceinline__ bool wait_barrier(uint32_t barrier, uint32_t parity, int *error_flag) {
@@ -78,194 +66,595 @@ __device__ __forceinline__ bool wait_barrier(uint32_t barrier, uint32_t parity, 
         }
     }
 }
+__device__ __forceinline__ void commit_to(uint32_t barrier) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(barrier) : "memory");
+}
+__device__ __forceinline__ uint32_t shared_address(const void *pointer) { return static_cast<uint32_t>(__cvta_generic_to_shared(pointer)); }
+
+// Half-precision pair arithmetic on 32-bit words.
+__device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {
+    uint32_t out;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(out) : "r"(a), "r"(b));
+    return out;
+}
+// The nibbles of `word` as fp16 (q - 8) * scale, pairs (0,4) (1,5) (2,6) (3,7): a nibble in the low mantissa bits of
+// 1024 is 1024 + q, one in the next four is 1024 + 16 q; the offset comes off exactly and the product is exact.
+__device__ __forceinline__ void dequantise_word(uint32_t word, uint32_t scale2, uint32_t (&out)[4]) {
+    const uint32_t shifted = word >> 8;
+    uint32_t a, b, c, d;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(a) : "r"(word), "n"(0x000F000F), "n"(0x64006400));
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(b) : "r"(word), "n"(0x00F000F0), "n"(0x64006400));
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(c) : "r"(shifted), "n"(0x000F000F), "n"(0x64006400));
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(shifted), "n"(0x00F000F0), "n"(0x64006400));
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(a) : "r"(a), "r"(0x64086408u));                      // - 1032
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(b) : "r"(b), "r"(0x2C002C00u), "r"(0xD480D480u));  // / 16 - 72
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(c) : "r"(c), "r"(0x64086408u));
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(d), "r"(0x2C002C00u), "r"(0xD480D480u));
+    out[0] = mul2(a, scale2);
+    out[1] = mul2(b, scale2);
+    out[2] = mul2(c, scale2);
+    out[3] = mul2(d, scale2);
+}
+
+// A power of two as f32 from its biased exponent.
+__device__ __forceinline__ float power_of_two(int biased_exponent) { return __uint_as_float(static_cast<uint32_t>(biased_exponent) << 23); }
 
 struct GemmArgs {
-    const uint16_t *x;
-    const uint32_t *qweights[3];  // up to three matrices that share the activations (q, k, v) in one launch:
+    const uint8_t *x;          // prepared activations: [k / 64][lane block of 8] atoms of 1024 bytes
+    const float *x_factor;     // [lanes] power of two that undoes the lane's scaling
+    const uint32_t *qweights[3];  // up to three matrices that share the activations (q, k, v; gate, up) in one launch:
     const uint16_t *scale_rows[3];
     void *ys[3];
     int ns[3];
-    int first_tile[4];            // ... matrix b owns the row tiles first_tile[b] .. first_tile[b + 1] - 1 of the grid
+    int first_tile[4];         // ... matrix b owns the 128-row tiles first_tile[b] .. first_tile[b + 1] - 1
     const uint16_t *residual;
-    int lanes, k, epilogue;
+    int lanes, lane_blocks, tile_lanes, k, epilogue, silu;
     float scale;
     int *error_flag;
-};
-struct GemmMatrix {  // the matrix a CTA works on
-    const uint32_t *qweight;
-    const uint16_t *scales;
-    void *y;
-    int n;
+    int a_stages, b_stages, raw_stages;
+    uint32_t tmem_columns, barrier_offset;
 };
 
-template <int GEMM_LANES>
-__global__ void __launch_bounds__(GEMM_THREADS) linear_int4_gemm_kernel(const GemmArgs a) {
-    constexpr int GEMM_B_BYTES = GEMM_LANES * 128 * 2;
-    extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t *tile_a[2] = {smem, smem + GEMM_A_BYTES + GEMM_B_BYTES};
-    uint8_t *tile_b[2] = {smem + GEMM_A_BYTES, smem + 2 * GEMM_A_BYTES + GEMM_B_BYTES};
-    uint64_t *barriers = reinterpret_cast<uint64_t *>(smem + 2 * (GEMM_A_BYTES + GEMM_B_BYTES));
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(barriers + 2);
-    const uint32_t barrier_address = static_cast<uint32_t>(__cvta_generic_to_shared(barriers));
+// Which 32 rows a quarter of a row tile holds: the matrix and the first row.  A SiLU pair (matrix 0 gate, 1 up, equal
+// shapes) takes the same rows of both: as two row tiles, or as the two halves of one.
+template <int ROW_TILES>
+__device__ __forceinline__ void locate_rows(const GemmArgs &a, int block_tile, int row_tile, int quarter, int &matrix, int &row) {
+    if (a.silu) {
+        if (ROW_TILES == 2) {
+            matrix = row_tile;
+            row = block_tile * 128 + quarter * 32;
+        } else {
+            matrix = quarter >> 1;
+            row = block_tile * 64 + (quarter & 1) * 32;
+        }
+        return;
+    }
+    const int tile = block_tile * ROW_TILES + row_tile;
+    matrix = 0;
+    row = 1 << 30;
+    if (tile >= a.first_tile[3]) return;  // the odd tile out: repeats the last row, nothing of it is stored
+    while (matrix < 2 && tile >= a.first_tile[matrix + 1]) matrix++;
+    row = (tile - a.first_tile[matrix]) * 128 + quarter * 32;
+}
+
+template <int ROW_TILES>
+__global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 : 1) linear_int4_gemm_kernel(const __grid_constant__ GemmArgs a) {
+    constexpr int ROWS = 128 * ROW_TILES, WARPS = 8 * ROW_TILES;  // warps that prepare the A operand: two sets, one for every other group
+    constexpr uint32_t SLOT = WARPS * 2048;                         // one raw stage: 32 rows x 64 bytes of every such warp
+    extern __shared__ __align__(1024) uint8_t smem[];
+    // [B stages][raw nibbles of eight warps][row scales][barriers]; the f32 partial sums take the front in the end
+    const int splits = gridDim.z, split = blockIdx.z;
+    const int groups = a.k >> 7, first_group = groups * split / splits, own_groups = groups * (split + 1) / splits - first_group;
+    const int m0 = blockIdx.x * a.tile_lanes;
+    const int n_lanes = min(a.tile_lanes, a.lane_blocks * 8 - m0);  // multiple of 16
+    const uint32_t b_stage_bytes = static_cast<uint32_t>(a.tile_lanes) * 256;
+    uint8_t *const raw = smem + static_cast<size_t>(a.b_stages) * b_stage_bytes;
+    uint16_t *const scales = reinterpret_cast<uint16_t *>(raw + a.raw_stages * SLOT);
+    const uint32_t a_full = shared_address(smem) + a.barrier_offset, a_empty = a_full + 8 * GEMM_MAX_A_STAGES, b_full = a_empty + 8 * GEMM_MAX_A_STAGES,
+                   b_empty = b_full + 8 * GEMM_MAX_B_STAGES, all_done = b_empty + 8 * GEMM_MAX_B_STAGES, tmem_slot = all_done + 8;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int branch = 0;
-    while (branch < 2 && static_cast<int>(blockIdx.y) >= a.first_tile[branch + 1]) branch++;
-    GemmMatrix matrix;  // the same fields under the names the single-matrix kernel used: a.qweight, a.scales, a.y, a.n
-    matrix.qweight = a.qweights[branch];
-    matrix.scales = a.scale_rows[branch];
-    matrix.y = a.ys[branch];
-    matrix.n = a.ns[branch];
-    const int m0 = blockIdx.x * GEMM_LANES, row0 = (static_cast<int>(blockIdx.y) - a.first_tile[branch]) * GEMM_ROWS;
-    const int groups = a.k >> 7, words_per_row = a.k >> 3;
 
     if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(barrier_address) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(barrier_address + 8) : "memory");
+        for (int s = 0; s < GEMM_MAX_A_STAGES; s++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a_full + s * 8), "r"(4 * ROW_TILES) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(a_empty + s * 8) : "memory");
+        }
+        for (int s = 0; s < GEMM_MAX_B_STAGES; s++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b_full + s * 8) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b_empty + s * 8) : "memory");
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(all_done) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) {  // two accumulators of LANES columns of tensor memory
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(tmem_slot))), "r"(static_cast<uint32_t>(2 * GEMM_LANES))
-                     : "memory");
+    if (warp == WARPS) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(a.tmem_columns) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(tmem_slot);
+    uint32_t tmem;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot) : "memory");
+    const uint32_t d_stride = (static_cast<uint32_t>(a.tile_lanes) + 31u) & ~31u, tmem_a = tmem + ROW_TILES * d_stride;
 
-    // fetch roles: thread t turns the 64 nibbles of half `t & 1` of row `t >> 1` into eight 16-byte pieces, and
-    // moves four 16-byte pieces of the activations
-    const int fetch_row = threadIdx.x >> 1, fetch_half = threadIdx.x & 1;
-    const int weight_row = row0 + fetch_row < matrix.n ? row0 + fetch_row : matrix.n - 1;
-    const uint4 *weight_source = reinterpret_cast<const uint4 *>(matrix.qweight + static_cast<size_t>(weight_row) * words_per_row) + fetch_half * 2;
-    const uint32_t weight_offset = static_cast<uint32_t>((fetch_row >> 3) * GEMM_BLOCK_STRIDE + fetch_half * 8 * 128 + (fetch_row & 7) * 16);
-    // accumulator roles: thread = row 32 * (warp & 3) + lane of the tile, one half of the tile's columns
-    constexpr int COLUMNS = GEMM_LANES / 2;
-    const int out_row = 32 * (warp & 3) + lane, column0 = COLUMNS * (warp >> 2);
-    const uint16_t *scale_row = matrix.scales + static_cast<size_t>(row0 + out_row < matrix.n ? row0 + out_row : matrix.n - 1) * groups;
-    float acc[COLUMNS];
-#pragma unroll
-    for (int i = 0; i < COLUMNS; i++) acc[i] = 0.0f;
     bool alive = true;
+    float row_factor = 1.0f;  // operand warps: the power of two that undoes the row's scaling
+    const int quarter = warp & 3, row_tile = (warp >> 2) % ROW_TILES, set = warp / (4 * ROW_TILES);
+    if (warp < WARPS) {
+        int matrix, row0;
+        locate_rows<ROW_TILES>(a, blockIdx.y, row_tile, quarter, matrix, row0);
+        const int n = a.ns[matrix];
+        const int items = (own_groups - set + 1) / 2;  // groups set, set + 2, ...
+        // cp.async: four neighbouring threads bring the 64 bytes of one row; the chunk's place is swizzled with the row
+        const uint8_t *source[4];
+        uint32_t destination[4];
+        const uint32_t warp_raw = shared_address(raw) + static_cast<uint32_t>(warp) * 2048;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = (lane >> 2) + 8 * i, global_row = min(row0 + r, n - 1);
+            source[i] = reinterpret_cast<const uint8_t *>(a.qweights[matrix]) + static_cast<size_t>(global_row) * (a.k >> 1) +
+                        static_cast<size_t>(first_group) * 64 + (lane & 3) * 16;
+            destination[i] = warp_raw + static_cast<uint32_t>(r * 64 + (((lane & 3) ^ ((r >> 1) & 3)) * 16));
+        }
+        int requested = 0;            // items asked for so far
+        uint32_t request_slot = 0;    // ... and the slot of the next one, in bytes
+        const uint32_t slots_end = static_cast<uint32_t>(a.raw_stages) * SLOT;
+        auto request = [&]() {
+            if (requested < items) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(destination[i] + request_slot), "l"(source[i]) : "memory");
+                    source[i] += 128;
+                }
+                requested++;
+                request_slot = request_slot + SLOT == slots_end ? 0 : request_slot + SLOT;
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+#pragma unroll
+        for (int i = 0; i < 4; i++) source[i] += set * 64;
+        for (int item = 0; item < a.raw_stages - 1; item++) request();
+        // the row's scales into shared memory ([group][row], read by this thread alone) and their largest exponent
+        float factor;
+        {
+            const uint16_t *row_scales = a.scale_rows[matrix] + static_cast<size_t>(min(row0 + lane, n - 1)) * groups + first_group;
+            uint16_t *const own = scales + row_tile * 128 + quarter * 32 + lane;
+            uint32_t largest = 16u << 7;
+            if (groups % 8 == 0 && own_groups % 8 == 0 && (reinterpret_cast<uintptr_t>(row_scales) & 15) == 0) {
+                constexpr int BATCH = 4;  // 16-byte loads in flight
+                for (int g = 0; g < own_groups; g += 8 * BATCH) {
+                    uint4 eight[BATCH];
+#pragma unroll
+                    for (int i = 0; i < BATCH; i++)
+                        if (g + 8 * i < own_groups) eight[i] = __ldg(reinterpret_cast<const uint4 *>(row_scales + g + 8 * i));
+#pragma unroll
+                    for (int i = 0; i < BATCH; i++) {
+                        if (g + 8 * i >= own_groups) break;
+                        const uint32_t words[4] = {eight[i].x, eight[i].y, eight[i].z, eight[i].w};
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            const uint32_t bits = (words[j >> 1] >> (16 * (j & 1))) & 0xFFFFu;
+                            largest = max(largest, bits & 0x7FFFu);
+                            own[(g + 8 * i + j) * ROWS] = static_cast<uint16_t>(bits);
+                        }
+                    }
+                }
+            } else {
+#pragma unroll 8
+                for (int g = 0; g < own_groups; g++) {
+                    const uint16_t bits = __ldg(row_scales + g);
+                    largest = max(largest, static_cast<uint32_t>(bits) & 0x7FFFu);
+                    own[g * ROWS] = bits;
+                }
+            }
+            const int exponent = static_cast<int>(largest >> 7);
+            factor = power_of_two(min(265 - exponent, 254));
+            row_factor = power_of_two(max(exponent - 11, 1));
+        }
+        const uint32_t read_base = warp_raw + static_cast<uint32_t>(lane * 64);
+        const uint32_t read_swizzle = static_cast<uint32_t>((lane >> 1) & 3);
+        const uint32_t tmem_rows = tmem_a + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(row_tile) * 64;
+        const uint16_t *scale = scales + set * ROWS + row_tile * 128 + quarter * 32 + lane;
+        uint32_t read_slot = 0;
+        // ring position of the item's group among the A stages, and the parity of its last release (the first round waits for none)
+        int stage = set;
+        uint32_t parity = 1;
+        for (int item = 0; item < items; item++) {
+            request();
+            switch (a.raw_stages) {  // the item's own copies have landed
+            case 3: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+            case 4: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+            case 5: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+            default: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
+            }
+            __syncwarp();
+            uint32_t scale2 = __half_as_ushort(__float2half_rn(bf16_bits_to_f32(*scale) * factor));
+            scale2 |= scale2 << 16;
+            scale += 2 * ROWS;
+            uint4 words[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const uint32_t address = read_base + read_slot + ((static_cast<uint32_t>(c) ^ read_swizzle) * 16);
+                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(words[c].x), "=r"(words[c].y), "=r"(words[c].z), "=r"(words[c].w) : "r"(address));
+            }
+            read_slot = read_slot + SLOT == slots_end ? 0 : read_slot + SLOT;
+            if (!wait_barrier(a_empty + stage * 8, parity, a.error_flag)) {
+                alive = false;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t target = tmem_rows + static_cast<uint32_t>(stage) * (64 * ROW_TILES);
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                uint32_t v[4][4];
+                dequantise_word(words[c].x, scale2, v[0]);
+                dequantise_word(words[c].y, scale2, v[1]);
+                dequantise_word(words[c].z, scale2, v[2]);
+                dequantise_word(words[c].w, scale2, v[3]);
+                asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(target + c * 16),
+                             "r"(v[0][0]), "r"(v[0][1]), "r"(v[0][2]), "r"(v[0][3]), "r"(v[1][0]), "r"(v[1][1]), "r"(v[1][2]), "r"(v[1][3]), "r"(v[2][0]),
+                             "r"(v[2][1]), "r"(v[2][2]), "r"(v[2][3]), "r"(v[3][0]), "r"(v[3][1]), "r"(v[3][2]), "r"(v[3][3])
+                             : "memory");
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a_full + stage * 8) : "memory");
+            stage += 2;
+            if (stage >= a.a_stages) {
+                stage -= a.a_stages;
+                parity ^= 1;
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if (warp == WARPS) {
+        if (lane == 0) {
+            // instruction descriptor: f32 accumulator, A and B fp16, both K-major, N / 8 in bits 17-22, M / 16 in bits 24-28
+            const uint32_t instruction = (1u << 4) | (static_cast<uint32_t>(n_lanes / 8) << 17) | (8u << 24);
+            int stage_a = 0, stage_b = 0;
+            uint32_t parity_a = 0, parity_b = 0;
+            for (int group = 0; group < own_groups; group++) {
+                if (!wait_barrier(b_full + stage_b * 8, parity_b, a.error_flag) || !wait_barrier(a_full + stage_a * 8, parity_a, a.error_flag)) {
+                    alive = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t b_address = shared_address(smem) + static_cast<uint32_t>(stage_b) * b_stage_bytes;
+#pragma unroll
+                for (int t = 0; t < ROW_TILES; t++) {
+                    const uint32_t d_address = tmem + t * d_stride;
+                    const uint32_t a_address = tmem_a + static_cast<uint32_t>(stage_a * ROW_TILES + t) * 64;
+#pragma unroll
+                    for (int step = 0; step < 8; step++) {  // K = 16 per instruction; four steps to a 128-byte row of the swizzled tile
+                        const uint64_t b_descriptor = swizzled_descriptor(b_address + static_cast<uint32_t>(step >> 2) * static_cast<uint32_t>(n_lanes) * 128 + (step & 3) * 32);
+                        const uint32_t accumulate = (group > 0 || step > 0) ? 1u : 0u;
+                        asm volatile(
+                            "{\n"
+                            ".reg .pred p;\n"
+                            "setp.ne.b32 p, %4, 0;\n"
+                            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+                            "}\n" ::"r"(d_address),
+                            "r"(a_address + step * 8), "l"(b_descriptor), "r"(instruction), "r"(accumulate)
+                            : "memory");
+                    }
+                }
+                commit_to(a_empty + stage_a * 8);
+                commit_to(b_empty + stage_b * 8);
+                if (++stage_a == a.a_stages) {
+                    stage_a = 0;
+                    parity_a ^= 1;
+                }
+                if (++stage_b == a.b_stages) {
+                    stage_b = 0;
+                    parity_b ^= 1;
+                }
+            }
+            commit_to(all_done);
+        }
+    } else if (lane == 0) {
+        grid_dependency_wait();
+        const uint8_t *source = a.x + static_cast<size_t>(m0 >> 3) * 1024;
+        const uint32_t bytes = static_cast<uint32_t>(n_lanes) * 128;
+        int stage = 0;
+        uint32_t parity = 1;  // the first round waits for no release
+        for (int group = 0; group < own_groups; group++) {
+            if (!wait_barrier(b_empty + stage * 8, parity, a.error_flag)) {
+                for (int g = group - a.b_stages; g < group; g++)  // the copies in flight land before the CTA gives its memory up
+                    wait_barrier(b_full + (g % a.b_stages) * 8, static_cast<uint32_t>((g / a.b_stages) & 1), a.error_flag);
+                break;
+            }
+            const uint32_t target = shared_address(smem) + static_cast<uint32_t>(stage) * b_stage_bytes, full = b_full + stage * 8;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"(2 * bytes) : "memory");
+#pragma unroll
+            for (int part = 0; part < 2; part++)
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(target + part * bytes),
+                             "l"(source + static_cast<size_t>(2 * (first_group + group) + part) * a.lane_blocks * 1024), "r"(bytes), "r"(full)
+                             : "memory");
+            if (++stage == a.b_stages) {
+                stage = 0;
+                parity ^= 1;
+            }
+        }
+    }
+    __syncwarp();
+    grid_launch_dependents();
+    grid_dependency_wait();  // outputs may be inputs of the kernel in front
 
-    // The packed nibbles and the activations of a group are requested one group ahead (into registers) and turned
-    // into the shared-memory tiles when their turn comes, so the memory latency of group g + 1 hides behind the
-    // MMAs of group g and the scaling of group g - 1.
-    uint4 raw_weights[2], raw_x[GEMM_LANES * 16 / GEMM_THREADS];
-    auto request = [&](int group) {
-        raw_weights[0] = __ldg(weight_source + group * 4);
-        raw_weights[1] = __ldg(weight_source + group * 4 + 1);
-#pragma unroll
-        for (int i = 0; i < GEMM_LANES * 16 / GEMM_THREADS; i++) {
-            const int piece = threadIdx.x + i * GEMM_THREADS, n = piece >> 4, block = piece & 15;
-            raw_x[i] = make_uint4(0, 0, 0, 0);
-            if (m0 + n < a.lanes) raw_x[i] = __ldg(reinterpret_cast<const uint4 *>(a.x + static_cast<size_t>(m0 + n) * a.k + group * 128) + block);
-        }
-    };
-    auto store_tiles = [&](int buffer) {
-        const uint32_t words[8] = {raw_weights[0].x, raw_weights[0].y, raw_weights[0].z, raw_weights[0].w,
-                                   raw_weights[1].x, raw_weights[1].y, raw_weights[1].z, raw_weights[1].w};
-        uint8_t *destination = tile_a[buffer] + weight_offset;
-#pragma unroll
-        for (int w = 0; w < 8; w++)
-            *reinterpret_cast<uint4 *>(destination + w * 128) = make_uint4(nibble_pair_bf16(words[w], 0), nibble_pair_bf16(words[w], 4),
-                                                                           nibble_pair_bf16(words[w], 8), nibble_pair_bf16(words[w], 12));
-#pragma unroll
-        for (int i = 0; i < GEMM_LANES * 16 / GEMM_THREADS; i++) {
-            const int piece = threadIdx.x + i * GEMM_THREADS, n = piece >> 4, block = piece & 15;
-            const uint4 raw = raw_x[i];
-            // (x0,x1)(x2,x3)(x4,x5)(x6,x7) -> (x0,x4)(x1,x5)(x2,x6)(x3,x7): the order the nibble pairs come out in
-            const uint4 ordered = make_uint4(__byte_perm(raw.x, raw.z, 0x5410), __byte_perm(raw.x, raw.z, 0x7632), __byte_perm(raw.y, raw.w, 0x5410),
-                                             __byte_perm(raw.y, raw.w, 0x7632));
-            *reinterpret_cast<uint4 *>(tile_b[buffer] + (n >> 3) * GEMM_BLOCK_STRIDE + block * 128 + (n & 7) * 16) = ordered;
-        }
-    };
-    // adds scale(group) x the accumulator of `buffer` to the registers
-    auto drain = [&](int group, int buffer) {
-        if (!wait_barrier(barrier_address + buffer * 8, static_cast<uint32_t>((group >> 1) & 1), a.error_flag)) alive = false;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const float scale = bf16_bits_to_f32(scale_row[group]);
-        const uint32_t address = tmem_base + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + static_cast<uint32_t>(buffer * GEMM_LANES + column0);
-#pragma unroll
-        for (int half = 0; half < COLUMNS / 16; half++) {
+    // ---- accumulators -> f32 [lane][row] in shared memory (every copy and MMA that used it is done by then)
+    float *const sums = reinterpret_cast<float *>(smem);
+    float *const factors = reinterpret_cast<float *>(smem + a.barrier_offset + GEMM_BARRIER_BYTES);
+    if (threadIdx.x < n_lanes && m0 + static_cast<int>(threadIdx.x) < a.lanes) factors[threadIdx.x] = a.x_factor[m0 + threadIdx.x];
+    if (warp < WARPS) {
+        if (!wait_barrier(all_done, 0u, a.error_flag)) alive = false;
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp < WARPS && alive) {  // the two sets share the lanes; both know the row's factor
+        const int local_row = row_tile * 128 + quarter * 32 + lane;
+        for (int column = set * 16; column < n_lanes; column += 32) {
             uint32_t d[16];
             asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
                          : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]), "=r"(d[8]), "=r"(d[9]),
                            "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15])
-                         : "r"(address + half * 16)
+                         : "r"(tmem + (static_cast<uint32_t>(quarter * 32) << 16) + row_tile * d_stride + static_cast<uint32_t>(column))
                          : "memory");
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int i = 0; i < 16; i++) acc[half * 16 + i] = fmaf(scale, __uint_as_float(d[i]), acc[half * 16 + i]);
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    };
-
-    if (groups > 0) request(0);
-    for (int group = 0; group < groups && alive; group++) {
-        const int buffer = group & 1;
-        store_tiles(buffer);  // the MMAs that read this buffer two groups ago were waited for in the last drain
-        if (group + 1 < groups) request(group + 1);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tiles were written with ordinary stores; the tensor core reads them
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t a_address = static_cast<uint32_t>(__cvta_generic_to_shared(tile_a[buffer]));
-            const uint32_t b_address = static_cast<uint32_t>(__cvta_generic_to_shared(tile_b[buffer]));
-            const uint32_t d_address = tmem_base + static_cast<uint32_t>(buffer * GEMM_LANES);
-#pragma unroll
-            for (int step = 0; step < 8; step++) {  // K = 16 per instruction: two core matrices = 256 bytes further per step
-                const uint64_t a_descriptor = matrix_descriptor(a_address + step * 256), b_descriptor = matrix_descriptor(b_address + step * 256);
-                const uint32_t accumulate = step > 0 ? 1u : 0u;
-                asm volatile(
-                    "{\n"
-                    ".reg .pred p;\n"
-                    "setp.ne.b32 p, %4, 0;\n"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n"
-                    "}\n" ::"r"(d_address),
-                    "l"(a_descriptor), "l"(b_descriptor), "r"(gemm_instruction<GEMM_LANES>()), "r"(accumulate), "r"(0u)
-                    : "memory");
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(barrier_address + buffer * 8) : "memory");
-        }
-        if (group > 0) drain(group - 1, buffer ^ 1);
-    }
-    if (alive && groups > 0) drain(groups - 1, (groups - 1) & 1);
-
-    // ---- epilogue: this thread's row, 32 lanes
-    if (alive && row0 + out_row < matrix.n) {
-#pragma unroll
-        for (int i = 0; i < COLUMNS; i++) {
-            const int m = m0 + column0 + i;
-            if (m >= a.lanes) break;
-            const size_t index = static_cast<size_t>(m) * matrix.n + row0 + out_row;
-            float sum = acc[i];
-            if (a.epilogue == EPILOGUE_F32_SCALED) {
-                reinterpret_cast<float *>(matrix.y)[index] = sum * a.scale;
-            } else {
-                if (a.epilogue == EPILOGUE_RESIDUAL_ROUNDED) sum = round_bf16(sum) + bf16_bits_to_f32(a.residual[index]);
-                else if (a.epilogue == EPILOGUE_RESIDUAL_F32) sum = sum + bf16_bits_to_f32(a.residual[index]);
-                reinterpret_cast<uint16_t *>(matrix.y)[index] = static_cast<uint16_t>(f32_to_bf16_bits(sum));
-            }
+            for (int i = 0; i < 16; i++) sums[(column + i) * ROWS + local_row] = __uint_as_float(d[i]) * row_factor;
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(static_cast<uint32_t>(2 * GEMM_LANES)) : "memory");
+    if (warp == WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(a.tmem_columns) : "memory");
+    const bool good = __syncthreads_and(alive ? 1 : 0) != 0;
+    if (splits > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+
+    // ---- outputs: this CTA's share of the tile's lanes; a thread keeps two neighbouring rows and walks the lanes
+    const int lane_begin = n_lanes * split / splits, lane_end = min(n_lanes * (split + 1) / splits, a.lanes - m0);
+    const int pairs = a.silu ? ROWS / 4 : ROWS / 2, r = (threadIdx.x & (pairs - 1)) * 2;  // pairs is a power of two
+    int matrix, row;
+    locate_rows<ROW_TILES>(a, blockIdx.y, r >> 7, (r >> 5) & 3, matrix, row);
+    row += r & 31;
+    const int n = a.ns[matrix];
+    if (good && threadIdx.x < WARPS * 32 && row < n) {
+        auto pair_sum = [&](int m, int at) {
+            if (splits == 1) return *reinterpret_cast<const float2 *>(sums + m * ROWS + at);
+            float2 sum = make_float2(0.0f, 0.0f);
+            const uint32_t local = shared_address(sums + m * ROWS + at);
+            for (int s = 0; s < splits; s++) {
+                uint32_t remote;
+                float2 part;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(s));
+                asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(part.x), "=f"(part.y) : "r"(remote));
+                sum.x += part.x;
+                sum.y += part.y;
+            }
+            return sum;
+        };
+        const bool whole = (n & 1) == 0;  // both rows exist and their outputs share an aligned word
+        const bool second_row = row + 1 < n;
+        const int step = WARPS * 32 / pairs;
+        constexpr int BATCH = 8;
+        for (int m = lane_begin + static_cast<int>(threadIdx.x) / pairs; m < lane_end; m += step * BATCH) {
+            float2 sum[BATCH], other[BATCH];  // other: the up rows of a SiLU pair, or the residual
+#pragma unroll
+            for (int i = 0; i < BATCH; i++) {
+                const int mi = m + i * step;
+                if (mi >= lane_end) break;
+                sum[i] = pair_sum(mi, r);
+                other[i] = make_float2(0.0f, 0.0f);
+                if (a.silu) {
+                    other[i] = pair_sum(mi, r + ROWS / 2);
+                } else if (a.residual != nullptr) {
+                    const uint16_t *residual = a.residual + static_cast<size_t>(m0 + mi) * n + row;
+                    if (whole) {
+                        const uint32_t both = *reinterpret_cast<const uint32_t *>(residual);
+                        other[i] = make_float2(bf16_lo(both), bf16_hi(both));
+                    } else {
+                        other[i].x = bf16_bits_to_f32(residual[0]);
+                        if (second_row) other[i].y = bf16_bits_to_f32(residual[1]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < BATCH; i++) {
+                const int mi = m + i * step;
+                if (mi >= lane_end) break;
+                const float factor = factors[mi];
+                const size_t out = static_cast<size_t>(m0 + mi) * n + row;
+                float first = sum[i].x * factor, second = sum[i].y * factor;
+                if (a.epilogue == EPILOGUE_F32_SCALED) {
+                    float *y = static_cast<float *>(a.ys[matrix]) + out;
+                    y[0] = first * a.scale;
+                    if (second_row) y[1] = second * a.scale;
+                    continue;
+                }
+                if (a.silu) {
+                    first = rounded_silu(round_bf16(first)) * round_bf16(other[i].x * factor);
+                    second = rounded_silu(round_bf16(second)) * round_bf16(other[i].y * factor);
+                } else if (a.residual != nullptr) {
+                    first = (a.epilogue == EPILOGUE_RESIDUAL_ROUNDED ? round_bf16(first) : first) + other[i].x;
+                    second = (a.epilogue == EPILOGUE_RESIDUAL_ROUNDED ? round_bf16(second) : second) + other[i].y;
+                }
+                uint16_t *y = static_cast<uint16_t *>(a.ys[matrix]) + out;
+                if (whole) {
+                    *reinterpret_cast<uint32_t *>(y) = pack_bf16(first, second);
+                } else {
+                    y[0] = static_cast<uint16_t>(f32_to_bf16_bits(first));
+                    if (second_row) y[1] = static_cast<uint16_t>(f32_to_bf16_bits(second));
+                }
+            }
+        }
+    }
+    if (splits > 1) {  // nobody leaves while a peer may still read its sums
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+}
+
+// bf16 [lanes][k] -> fp16 x 2^e in the GEMM's tile order, one CTA per lane (lanes beyond the batch are zero): largest
+// magnitude of the row, then the conversion; a 16-byte piece of eight columns holds them in the order (0,4)(1,5)(2,6)
+// (3,7) the nibble pairs come out in, at its swizzled place in the 8-lane x 64-column atom.
+constexpr int PREPARE_THREADS = 256;
+__global__ void __launch_bounds__(PREPARE_THREADS) prepare_activations_kernel(const uint16_t *__restrict__ x, uint8_t *__restrict__ out, float *__restrict__ factors,
+                                                                             int lanes, int lane_blocks, int k) {
+    __shared__ uint32_t warp_largest[PREPARE_THREADS / 32];
+    const int m = blockIdx.x, pieces = k >> 3;
+    grid_dependency_wait();
+    const uint4 *row = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(m) * k);
+    uint32_t largest = 0;
+    if (m < lanes) {
+        for (int p = threadIdx.x; p < pieces; p += PREPARE_THREADS) {
+            const uint4 v = row[p];
+            const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) largest = max(largest, max((words[i] & 0x7FFFu), (words[i] >> 16) & 0x7FFFu));
+        }
+#pragma unroll
+        for (int offset = 16; offset > 0; offset >>= 1) largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, offset));
+        if ((threadIdx.x & 31) == 0) warp_largest[threadIdx.x >> 5] = largest;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < PREPARE_THREADS / 32; w++) largest = max(largest, warp_largest[w]);
+    }
+    const int exponent = max(static_cast<int>(largest >> 7), 16);
+    const float factor = power_of_two(min(268 - exponent, 254));
+    if (m < lanes && threadIdx.x == 0) factors[m] = power_of_two(max(exponent - 14, 1));
+    for (int p = threadIdx.x; p < pieces; p += PREPARE_THREADS) {
+        uint4 packed = make_uint4(0, 0, 0, 0);
+        if (m < lanes) {
+            const uint4 v = row[p];
+            auto both = [&](uint32_t a, uint32_t b) {
+                const __half2 h = __floats2half2_rn(__uint_as_float(a) * factor, __uint_as_float(b) * factor);
+                return *reinterpret_cast<const uint32_t *>(&h);
+            };
+            packed.x = both(v.x << 16, v.z << 16);
+            packed.y = both(v.x & 0xffff0000u, v.z & 0xffff0000u);
+            packed.z = both(v.y << 16, v.w << 16);
+            packed.w = both(v.y & 0xffff0000u, v.w & 0xffff0000u);
+        }
+        *reinterpret_cast<uint4 *>(out + (static_cast<size_t>(p >> 3) * lane_blocks + (m >> 3)) * 1024 + (m & 7) * 128 + (((p & 7) ^ (m & 7)) * 16)) = packed;
+    }
+    grid_launch_dependents();
+}
+
+struct GemmPlan {
+    int row_tiles = 1, lane_tiles = 1, tile_lanes = 16, splits = 1, a_stages = 2, b_stages = 2, raw_stages = 3;
+    uint32_t tmem_columns = 512;
+    size_t smem = 0;
+};
+
+// Tile shape and K split by an estimate of the launch's time in SM cycles.  Per group of 128 columns a CTA needs 4
+// cycles per lane and row tile on the tensor cores and about 280 per row tile to dequantise; a wave that is not full
+// costs as much as a full one, every CTA pays for filling its pipeline and for its epilogue, and two CTAs share an SM
+// where shared and tensor memory allow.
+GemmPlan plan_gemm(int matrix_tiles, int lanes, int groups, bool silu) {
+    const int padded = (lanes + 15) / 16 * 16;
+    GemmPlan best;
+    double best_cycles = 1e30;
+    for (int row_tiles = 1; row_tiles <= 2; row_tiles++) {
+        const int most = 256 / row_tiles;
+        const int fewest_tiles = (padded + most - 1) / most;
+        // (a SiLU pair covers 64 rows of both matrices per row tile)
+        const int blocks = silu ? (row_tiles == 2 ? matrix_tiles / 2 : matrix_tiles) : (matrix_tiles + row_tiles - 1) / row_tiles;
+        for (int lane_tiles = fewest_tiles; lane_tiles <= fewest_tiles + 2; lane_tiles++) {
+            const int tile_lanes = ((padded + lane_tiles - 1) / lane_tiles + 15) / 16 * 16;
+            if (tile_lanes > most || (lane_tiles > 1 && tile_lanes * (lane_tiles - 1) >= padded)) continue;
+            for (int splits = 1; splits <= 8 && (splits == 1 || splits * 2 <= groups); splits *= 2) {
+                const int own = (groups + splits - 1) / splits;
+                GemmPlan plan;
+                plan.row_tiles = row_tiles;
+                plan.lane_tiles = lane_tiles;
+                plan.tile_lanes = tile_lanes;
+                plan.splits = splits;
+                const size_t scales = static_cast<size_t>(own) * 256 * row_tiles, b_stage = static_cast<size_t>(tile_lanes) * 256;
+                const size_t sums = static_cast<size_t>(tile_lanes) * 512 * row_tiles;
+                int per_sm = 0;
+                for (int share = row_tiles == 1 && tile_lanes <= 64 ? 2 : 1; share >= 1 && per_sm == 0; share--) {
+                    const size_t limit = share == 2 ? GEMM_SMEM_TWO : GEMM_SMEM_ONE;
+                    for (int raw = row_tiles == 2 ? 4 : 6; raw >= 3 && per_sm == 0; raw--)
+                        for (int b = std::min(GEMM_MAX_B_STAGES, std::max(2, own)); b >= 2; b--) {
+                            if (raw > (row_tiles == 2 ? 3 : 4) && b < 4 && b < own) break;  // rather fewer raw stages than fewer than four of the activations
+                            const size_t bytes = std::max(static_cast<size_t>(b) * b_stage + static_cast<size_t>(raw) * 16384 * row_tiles + scales, sums);
+                            if (bytes > limit) continue;
+                            plan.b_stages = b;
+                            plan.raw_stages = raw;
+                            plan.smem = bytes;
+                            per_sm = share;
+                            break;
+                        }
+                }
+                if (per_sm == 0) continue;
+                const int d_columns = (tile_lanes + 31) / 32 * 32 * row_tiles;
+                plan.tmem_columns = per_sm == 2 ? 256 : 512;
+                plan.a_stages = std::min(GEMM_MAX_A_STAGES, (static_cast<int>(plan.tmem_columns) - d_columns) / (64 * row_tiles));
+                if (plan.a_stages < 2) continue;
+                const double per_group = std::max(row_tiles * 4.0 * tile_lanes, row_tiles * 280.0);
+                const double ctas = static_cast<double>(blocks) * lane_tiles * splits;
+                const double waves = std::max(1.0, (ctas + 148 * per_sm - 1) / (148 * per_sm));
+                const double whole = static_cast<double>(static_cast<long>(waves));
+                const double shared_sm = ctas > 148 ? per_sm : 1;
+                const double cycles = whole * (own * per_group * shared_sm + 5000.0 + row_tiles * tile_lanes * 12.0) + (splits > 1 ? 1500.0 : 0.0);
+                if (cycles < best_cycles) {
+                    best_cycles = cycles;
+                    best = plan;
+                }
+            }
+        }
+    }
+    return best;
 }
 
 }  // namespace
 
-bool linear_int4_gemm_supported(int lanes, int n, int k) { return lanes >= GEMM_MIN_LANES && k % 128 == 0 && k >= 128 && n >= 1; }
+bool linear_int4_gemm_supported(int lanes, int n, int k) { return lanes > 8 && k % 128 == 0 && k >= 128 && n >= 1; }
 
-cudaError_t launch_linear_int4_gemm_multi(const uint16_t *x, int branches, const uint32_t *const *qweights, const uint16_t *const *scales, void *const *ys,
-                                          const int *ns, const uint16_t *residual, int lanes, int k, int epilogue, float scale, int *error_flag,
-                                          cudaStream_t stream) {
+size_t int4_activation_bytes(int lanes, int k) {
+    const size_t padded = static_cast<size_t>(lanes + 15) / 16 * 16;
+    return padded * k * 2 + padded * sizeof(float);
+}
+
+static float *activation_factors(void *prepared, int lanes, int k) {
+    const size_t padded = static_cast<size_t>(lanes + 15) / 16 * 16;
+    return reinterpret_cast<float *>(static_cast<uint8_t *>(prepared) + padded * k * 2);
+}
+
+// Launch with the programmatic-dependent-launch attribute (and a cluster over the K splits).
+template <typename... Parameters, typename... Arguments>
+static cudaError_t launch_dependent(void (*kernel)(Parameters...), dim3 grid, int threads, size_t smem, int cluster, cudaStream_t stream, Arguments... arguments) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid;
+    config.blockDim = dim3(threads);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[0].val.programmaticStreamSerializationAllowed = 1;
+    attributes[1].id = cudaLaunchAttributeClusterDimension;
+    attributes[1].val.clusterDim.x = 1;
+    attributes[1].val.clusterDim.y = 1;
+    attributes[1].val.clusterDim.z = static_cast<unsigned int>(cluster);
+    config.attrs = attributes;
+    config.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&config, kernel, Parameters(arguments)...);
+}
+
+cudaError_t launch_prepare_activations(const uint16_t *x, void *prepared, int lanes, int k, cudaStream_t stream) {
     if (lanes <= 0) return cudaSuccess;
-    if (branches < 1 || branches > 3 || (residual != nullptr && branches != 1)) return cudaErrorInvalidValue;
+    const int padded = (lanes + 15) / 16 * 16;
+    return launch_dependent(prepare_activations_kernel, dim3(padded), PREPARE_THREADS, 0, 1, stream, x, static_cast<uint8_t *>(prepared),
+                            activation_factors(prepared, lanes, k), lanes, padded / 8, k);
+}
+
+cudaError_t launch_linear_int4_gemm(const void *prepared, int branches, const uint32_t *const *qweights, const uint16_t *const *scales, void *const *ys,
+                                    const int *ns, const uint16_t *residual, int lanes, int k, int epilogue, float scale, bool silu, int *error_flag,
+                                    cudaStream_t stream) {
+    if (lanes <= 0) return cudaSuccess;
+    if (branches < 1 || branches > 3 || (residual != nullptr && branches != 1) || (silu && (branches != 2 || ns[0] != ns[1]))) return cudaErrorInvalidValue;
     GemmArgs args = {};
-    args.x = x;
     int tiles = 0;
     for (int b = 0; b < 3; b++) {
         const int source = b < branches ? b : branches - 1;
@@ -275,31 +664,35 @@ cudaError_t launch_linear_int4_gemm_multi(const uint16_t *x, int branches, const
         args.ys[b] = ys[source];
         args.ns[b] = ns[source];
         args.first_tile[b] = tiles;
-        if (b < branches) tiles += (ns[b] + GEMM_ROWS - 1) / GEMM_ROWS;
+        if (b < branches) tiles += (ns[b] + 127) / 128;
     }
     args.first_tile[3] = tiles;
-    for (int b = branches; b < 3; b++) args.first_tile[b] = tiles;  // no tile belongs to an absent matrix
+    for (int b = branches; b < 3; b++) args.first_tile[b] = tiles;  // no tile belongs to an absent matrix ...
+    const GemmPlan plan = plan_gemm(tiles, lanes, k >> 7, silu);
+    if (plan.smem == 0) return cudaErrorInvalidValue;
+    args.x = static_cast<const uint8_t *>(prepared);
+    args.x_factor = activation_factors(const_cast<void *>(prepared), lanes, k);
     args.residual = residual;
     args.lanes = lanes;
+    args.lane_blocks = (lanes + 15) / 16 * 2;
+    args.tile_lanes = plan.tile_lanes;
     args.k = k;
     args.epilogue = epilogue;
+    args.silu = silu ? 1 : 0;
     args.scale = scale;
     args.error_flag = error_flag;
-    if (lanes >= 128) {
-        cudaError_t status = cudaFuncSetAttribute(linear_int4_gemm_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(gemm_smem<128>()));
-        if (status != cudaSuccess) return status;
-        linear_int4_gemm_kernel<128><<<dim3((lanes + 127) / 128, tiles), GEMM_THREADS, gemm_smem<128>(), stream>>>(args);
-    } else {
-        cudaError_t status = cudaFuncSetAttribute(linear_int4_gemm_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(gemm_smem<64>()));
-        if (status != cudaSuccess) return status;
-        linear_int4_gemm_kernel<64><<<dim3((lanes + 63) / 64, tiles), GEMM_THREADS, gemm_smem<64>(), stream>>>(args);
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_linear_int4_gemm(const uint16_t *x, const uint32_t *qweight, const uint16_t *scales, void *y, const uint16_t *residual, int lanes,
-                                    int n, int k, int epilogue, float scale, int *error_flag, cudaStream_t stream) {
-    return launch_linear_int4_gemm_multi(x, 1, &qweight, &scales, &y, &n, residual, lanes, k, epilogue, scale, error_flag, stream);
+    args.a_stages = plan.a_stages;
+    args.b_stages = plan.b_stages;
+    args.raw_stages = plan.raw_stages;
+    args.tmem_columns = plan.tmem_columns;
+    args.barrier_offset = static_cast<uint32_t>(plan.smem);
+    int blocks = (tiles + plan.row_tiles - 1) / plan.row_tiles;
+    if (silu) blocks = (ns[0] + 64 * plan.row_tiles - 1) / (64 * plan.row_tiles);
+    const dim3 grid(plan.lane_tiles, blocks, plan.splits);
+    auto kernel = plan.row_tiles == 2 ? linear_int4_gemm_kernel<2> : linear_int4_gemm_kernel<1>;
+    cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(GEMM_SMEM_ONE + GEMM_TAIL_BYTES));
+    if (status != cudaSuccess) return status;
+    return launch_dependent(kernel, grid, plan.row_tiles == 2 ? gemm_threads<2>() : gemm_threads<1>(), plan.smem + GEMM_TAIL_BYTES, plan.splits, stream, args);
 }
 
 }  // namespace nerve

@@ -223,7 +223,7 @@ linear_int4_mma_kernel(const Int4Launch p) {
     __shared__ float reduce[INT4_WARPS][RT * 16][8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, j = lane & 3;
-    const int m0 = blockIdx.y * 8;
+    constexpr int m0 = 0;  // at most eight lanes
 
     int b = 0;
     if (!SILU_PAIR) {
@@ -382,19 +382,17 @@ static cudaError_t launch_pdl(Kernel kernel, dim3 grid, dim3 block, cudaStream_t
     return cudaLaunchKernelEx(&config, kernel, params);
 }
 
-cudaError_t launch_linear_int4_multi(const uint16_t *x, int branches, const uint32_t *const *qweights,
+cudaError_t launch_linear_int4_multi(const uint16_t *x, const void *prepared, int branches, const uint32_t *const *qweights,
                                      const uint16_t *const *scales, uint16_t *const *ys, const int *ns,
                                      const uint16_t *residual, int lanes, int k, int epilogue, cudaStream_t stream, int *error_flag) {
     if (lanes <= 0) return cudaSuccess;
     if (k % 128 != 0 || branches < 1 || branches > 3) return cudaErrorInvalidValue;
     if (linear_int4_gemm_supported(lanes, ns[0], k)) {
-        // wide batches (prefill chunks, many-stream verify): one tcgen05 GEMM launch for all the matrices that share
-        // the activations, the weights read once per 64 lanes
-        for (int b = 1; b < branches; b++)
-            if (!linear_int4_gemm_supported(lanes, ns[b], k)) return cudaErrorInvalidValue;
+        // more than eight lanes: one tcgen05 GEMM launch for all the matrices that share the activations
+        if (prepared == nullptr) return cudaErrorInvalidValue;
         void *outputs[3] = {ys[0], branches > 1 ? ys[1] : nullptr, branches > 2 ? ys[2] : nullptr};
-        return launch_linear_int4_gemm_multi(x, branches, qweights, scales, outputs, ns, branches == 1 ? residual : nullptr, lanes, k, epilogue, 1.0f, error_flag,
-                                             stream);
+        return launch_linear_int4_gemm(prepared, branches, qweights, scales, outputs, ns, branches == 1 ? residual : nullptr, lanes, k, epilogue, 1.0f, false,
+                                       error_flag, stream);
     }
     Int4Launch params = {};
     params.branches = branches;
@@ -411,24 +409,32 @@ cudaError_t launch_linear_int4_multi(const uint16_t *x, int branches, const uint
         params.branch[b] = Int4Branch{qweights[b], scales[b], ys[b], ns[b], tiles};
         tiles += (ns[b] + 16 * rt - 1) / (16 * rt);
     }
-    dim3 grid(tiles, (lanes + 7) / 8);
+    dim3 grid(tiles);
     return launch_pdl(linear_int4_mma_kernel<1, false, 4>, grid, dim3(INT4_WARPS * 32), stream, params);
 }
 
-cudaError_t launch_linear_int4(const uint16_t *x, const uint32_t *qweight, const uint16_t *scales, uint16_t *y,
+cudaError_t launch_linear_int4(const uint16_t *x, const void *prepared, const uint32_t *qweight, const uint16_t *scales, uint16_t *y,
                                const uint16_t *residual, int lanes, int n, int k, int group, int epilogue,
                                cudaStream_t stream, int *error_flag) {
     if (group != 128) return cudaErrorInvalidValue;
-    return launch_linear_int4_multi(x, 1, &qweight, &scales, &y, &n, residual, lanes, k, epilogue, stream, error_flag);
+    return launch_linear_int4_multi(x, prepared, 1, &qweight, &scales, &y, &n, residual, lanes, k, epilogue, stream, error_flag);
 }
 
 // gate/up pair with the SiLU*up epilogue (gate -> bf16, SiLU -> bf16, up -> bf16, product -> bf16: the
 // rounding chain of linear + linear + silu_multiply_bf16.comp.template:30-52).
-cudaError_t launch_linear_int4_silu_pair(const uint16_t *x, const uint32_t *gate_q, const uint16_t *gate_s,
+cudaError_t launch_linear_int4_silu_pair(const uint16_t *x, const void *prepared, const uint32_t *gate_q, const uint16_t *gate_s,
                                          const uint32_t *up_q, const uint16_t *up_s, uint16_t *y, int lanes, int n,
-                                         int k, cudaStream_t stream) {
+                                         int k, cudaStream_t stream, int *error_flag) {
     if (lanes <= 0) return cudaSuccess;
     if (k % 128 != 0) return cudaErrorInvalidValue;
+    if (linear_int4_gemm_supported(lanes, n, k)) {
+        if (prepared == nullptr) return cudaErrorInvalidValue;
+        const uint32_t *qweights[2] = {gate_q, up_q};
+        const uint16_t *scales[2] = {gate_s, up_s};
+        void *outputs[2] = {y, y};
+        const int ns[2] = {n, n};
+        return launch_linear_int4_gemm(prepared, 2, qweights, scales, outputs, ns, nullptr, lanes, k, EPILOGUE_BF16, 1.0f, true, error_flag, stream);
+    }
     Int4Launch params = {};
     params.branches = 2;
     params.x = x;
@@ -437,7 +443,7 @@ cudaError_t launch_linear_int4_silu_pair(const uint16_t *x, const uint32_t *gate
     params.branch[0] = Int4Branch{gate_q, gate_s, nullptr, n, 0};
     params.branch[1] = Int4Branch{up_q, up_s, nullptr, n, 0};
     params.branch[2] = Int4Branch{nullptr, nullptr, y, n, 0};
-    dim3 grid((n + 15) / 16, (lanes + 7) / 8);
+    dim3 grid((n + 15) / 16);
     return launch_pdl(linear_int4_mma_kernel<2, true, 2>, grid, dim3(INT4_WARPS * 32), stream, params);
 }
 
