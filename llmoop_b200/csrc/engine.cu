@@ -556,20 +556,27 @@ Engine::Engine(std::shared_ptr<MountedModel> model) : model_(std::move(model)) {
     for (const ComponentPlan &layer : plan.layers) scan(layer);
     for (const ComponentPlan &layer : plan.draft_layers) scan(layer);
     // Scratch of the split attention.  The persistent kernel (at most eight lanes) takes 64-token splits over the
-    // whole ring.  The kernel-per-operator path takes splits of a length fixed per engine - 64 tokens where the
-    // partials of the largest batch over the whole ring fit 1 GB, else the next multiple of 64 that makes them fit
-    // (a prefill chunk of 2048 lanes over a 32K ring: 1152 tokens), walked tile by tile inside the kernel - so the
-    // arithmetic of a lane never depends on which batch it runs in.
+    // whole ring.  On the kernel-per-operator path verify, draft and single-tick batches take splits of a length fixed
+    // per engine - 128 tokens (64 in FP8 packages) where the partials of the largest batch over the whole ring fit 1 GB,
+    // else the next multiple that makes them fit - so that the arithmetic of such a lane does not depend on its batch;
+    // prefill chunks are split only as far as they need to be to fill the chip (plan_splits), except in FP8 packages.
+    auto has_fp8 = [](const ComponentPlan &component) {
+        for (const OpSpec &op : component.ops)
+            for (const WeightRef &w : op.weights)
+                if (w.storage == TensorStorage::FP8_BLOCK) return true;
+        return false;
+    };
+    scalar_attention_ = std::any_of(plan.layers.begin(), plan.layers.end(), has_fp8) || std::any_of(plan.draft_layers.begin(), plan.draft_layers.end(), has_fp8);
     max_q_heads_ = max_q_heads;
     const size_t partial_bytes = static_cast<size_t>(max_head_width + 2) * sizeof(float);
     const size_t budget = (size_t(1) << 30) / partial_bytes;
-    const size_t all = static_cast<size_t>(options.max_lanes) * max_q_heads * max_splits_;
-    const int factor = static_cast<int>(std::max<size_t>(1, (all + budget - 1) / budget));
-    op_split_tokens_ = split_tokens_ * factor;
+    const size_t op_base = scalar_attention_ ? 64 : 128, all = static_cast<size_t>(options.max_lanes) * max_q_heads * ((model_->capacity() + op_base - 1) / op_base);
+    op_split_tokens_ = static_cast<int>(op_base * std::max<size_t>(1, (all + budget - 1) / budget));
     const size_t op_splits = (model_->capacity() + op_split_tokens_ - 1) / op_split_tokens_;
     // (the persistent kernel merges rows of more than 32 splits in two levels: one more partial per 32 splits)
     const size_t small_batches = static_cast<size_t>(std::min(options.max_lanes, 8)) * max_q_heads * (max_splits_ + (max_splits_ + 31) / 32);
-    attention_scratch_ = device_alloc(std::max(small_batches, static_cast<size_t>(options.max_lanes) * max_q_heads * op_splits) * partial_bytes);
+    attention_partials_ = std::max(small_batches, static_cast<size_t>(options.max_lanes) * max_q_heads * op_splits);
+    attention_scratch_ = device_alloc(attention_partials_ * partial_bytes);
 
     // cycle arrays: verify tokens, forced drafts, stop tokens/counts, accept rows, per-step draft tokens, slots
     cycle_state_ = device_alloc(lanes * 64 * sizeof(uint32_t) + static_cast<size_t>(options.max_streams) * (MAX_STOP_TOKENS + 64) * sizeof(uint32_t) * 4);
@@ -1199,10 +1206,59 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
                op.weights[0].group == 128;
     };
 
+    // Whether every reader of `signal` is an INT4 linear of one branch.
+    auto only_int4_reads = [&](const std::string &signal, size_t after) {
+        int readers = 0;
+        for (size_t i = after; i < plan.ops.size(); i++)
+            if (is_int4_single(plan.ops[i]) && plan.ops[i].inputs[0] == signal) readers++;
+        return readers > 0 && readers == consumers(signal, after);
+    };
+    // Whether `attention` reads exactly these rotated q and k, and nothing else reads that k.
+    auto append_takes = [&](const OpSpec &attention, const std::string &q, const std::string &k, size_t after) {
+        return attention.inputs[0] == q && attention.inputs[1] == k && consumers(k, after) == 0;
+    };
+    // KV append and attention; with rotary attributes the rotation of q (q_in -> q) and of k on its way into its slot too.
+    auto rope_append = [&](const OpSpec &attention, const std::string &q_in, const std::string &k, const std::string &q, const RopeAttrs *q_rope,
+                           const RopeAttrs *k_rope, const OpSpec *norms) {
+        if (kv_index < 0) fail("attention op in a component without KV state");
+        const KvLayer kv = model_->kv_layer(kv_index);
+        auto form = [&](const RopeAttrs *rope) {
+            RopeForm out{nullptr, 1, 0, 0};
+            if (rope != nullptr) out = RopeForm{model_->rope_table(rope->theta, rope->rotary_width), model_->rope_positions(), rope->rotary_width, rope->interleaved ? 1 : 0};
+            return out;
+        };
+        RopeAppend append{};
+        append.q = q_rope != nullptr ? u16(q_in) : nullptr;
+        append.k = u16(k);
+        append.v = u16(attention.inputs[2]);
+        append.q_out = u16(q);
+        if (norms != nullptr) {
+            append.q_norm = static_cast<const uint16_t *>(weight(norms->norm_weights[0]));
+            append.k_norm = static_cast<const uint16_t *>(weight(norms->norm_weights[1]));
+            append.eps = norms->eps;
+            append.norm_offset = norms->weight_offset;
+        }
+        append.q_heads = q_rope != nullptr ? attention.q_heads : 0;
+        append.q_form = form(q_rope);
+        append.k_form = form(k_rope);
+        check(launch_rope_append(append, kv, lane_table, lanes, st), "rope and kv append");
+        check(launch_attention(u16(attention.inputs[0]), u16(attention.outputs[0]), kv, lane_table, lanes, current_width_, attention.q_heads,
+                               attention.attention_scale, current_op_split_tokens_, current_op_splits_, static_cast<float *>(attention_scratch_.ptr), scalar_attention_, st),
+              "attention");
+        if (current_op_splits_ > 1 || scalar_attention_) counters_.kernel_launches++;
+    };
+
     for (size_t index = 0; index < plan.ops.size(); index++) {
         const OpSpec &op = plan.ops[index];
         switch (op.kind) {
         case OpKind::RmsNorm:
+            if (lanes > 8 && only_int4_reads(op.outputs[0], index + 1)) {  // straight into the GEMM's operand form
+                check(launch_rms_norm_prepared(u16(op.inputs[0]), static_cast<const uint16_t *>(weight(op.norm_weights[0])), int4_activations_.ptr, lanes,
+                                               width(op.inputs[0]), op.eps, op.weight_offset, st),
+                      "rms_norm");
+                prepared_signal = op.outputs[0];
+                break;
+            }
             check(launch_rms_norm(u16(op.inputs[0]), static_cast<const uint16_t *>(weight(op.norm_weights[0])), u16(op.outputs[0]), lanes,
                                   width(op.inputs[0]), op.eps, op.weight_offset, st),
                   "rms_norm");
@@ -1381,6 +1437,12 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
                   "quantize_fp8");
             break;
         case OpKind::Rope: {
+            if (index + 2 < plan.ops.size() && plan.ops[index + 1].kind == OpKind::Rope && plan.ops[index + 2].kind == OpKind::AppendAttention &&
+                append_takes(plan.ops[index + 2], op.outputs[0], plan.ops[index + 1].outputs[0], index + 3)) {
+                rope_append(plan.ops[index + 2], op.inputs[0], plan.ops[index + 1].inputs[0], op.outputs[0], &op.rope[0], &plan.ops[index + 1].rope[0], nullptr);
+                index += 2;
+                break;
+            }
             const RopeAttrs &rope = op.rope[0];
             check(launch_rope(u16(op.inputs[0]), u16(op.outputs[0]), model_->rope_table(rope.theta, rope.rotary_width), model_->rope_positions(),
                               lane_table.position, lanes, rope.heads, rope.head_width, rope.rotary_width, rope.interleaved, nullptr, 0.0f, 0.0f,
@@ -1389,6 +1451,12 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
             break;
         }
         case OpKind::HeadNormRope:
+            if (op.rope.size() == 2 && index + 1 < plan.ops.size() && plan.ops[index + 1].kind == OpKind::AppendAttention &&
+                append_takes(plan.ops[index + 1], op.outputs[0], op.outputs[1], index + 2)) {
+                rope_append(plan.ops[index + 1], op.inputs[0], op.inputs[1], op.outputs[0], &op.rope[0], &op.rope[1], &op);
+                index += 1;
+                break;
+            }
             for (size_t branch = 0; branch < op.rope.size(); branch++) {
                 const RopeAttrs &rope = op.rope[branch];
                 check(launch_rope(u16(op.inputs[branch]), u16(op.outputs[branch]), model_->rope_table(rope.theta, rope.rotary_width),
@@ -1398,16 +1466,9 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
                       "head_norm_rope");
             }
             break;
-        case OpKind::AppendAttention: {
-            if (kv_index < 0) fail("attention op in a component without KV state");
-            KvLayer kv = model_->kv_layer(kv_index);
-            check(launch_kv_append(u16(op.inputs[1]), u16(op.inputs[2]), kv, lane_table, lanes, st), "kv_append");
-            check(launch_attention(u16(op.inputs[0]), u16(op.outputs[0]), kv, lane_table, lanes, current_width_, op.q_heads, op.attention_scale, op_split_tokens_,
-                                   current_op_splits_, static_cast<float *>(attention_scratch_.ptr), st),
-                  "attention");
-            counters_.kernel_launches++;
+        case OpKind::AppendAttention:
+            rope_append(op, std::string(), op.inputs[1], op.inputs[0], nullptr, nullptr, nullptr);
             break;
-        }
         case OpKind::ResidualAdd:
             check(launch_add(u16(op.inputs[0]), u16(op.inputs[1]), u16(op.outputs[0]), static_cast<size_t>(lanes) * width(op.inputs[0]), st),
                   "residual_add");
@@ -1496,13 +1557,14 @@ void Engine::profile_end() {
     profile_used_ += 2;
 }
 
-void Engine::upload_lanes(const std::vector<uint32_t> &positions, const std::vector<int32_t> &slots) {
+void Engine::upload_lanes(const std::vector<uint32_t> &positions, const std::vector<int32_t> &slots, int lanes_per_stream) {
     upload(lane_positions_.ptr, positions.data(), positions.size() * sizeof(uint32_t), "lane positions upload");
     upload(lane_slots_.ptr, slots.data(), slots.size() * sizeof(int32_t), "lane slots upload");
     current_lanes_ = LaneTable{static_cast<const uint32_t *>(lane_positions_.ptr), static_cast<const int32_t *>(lane_slots_.ptr)};
     uint32_t newest = 0;
     for (uint32_t position : positions) newest = std::max(newest, position);
-    plan_splits(static_cast<int>(positions.size()), newest);
+    current_width_ = lanes_per_stream;
+    plan_splits(static_cast<int>(positions.size()), lanes_per_stream, newest);
 }
 
 void Engine::upload_tokens(const uint32_t *tokens, int count) {
@@ -1510,11 +1572,13 @@ void Engine::upload_tokens(const uint32_t *tokens, int count) {
     current_tokens_ = static_cast<const uint32_t *>(lane_tokens_.ptr);
 }
 
-// Attention launches cover ceil(context / split) splits, rounded up to a power of two so that a handful of graph
-// shapes serves a growing context: splits of 64 tokens in the persistent kernel, of the engine's fixed length on the
-// kernel-per-operator path.  Returns a word for graph keys.
-int Engine::plan_splits(int lanes, uint64_t newest_tick) {
-    (void)lanes;
+// Splits of the attention launches that follow.  Decode forms (verify, draft, single ticks): ceil(context / split) splits,
+// rounded up to a power of two so that a handful of graph shapes serves a growing context - 64 tokens in the persistent
+// kernel, the engine's fixed length on the kernel-per-operator path.  A prefill chunk (never replayed from a graph)
+// takes the number of splits that brings its last wave of CTAs, one per SM, closest to full: a CTA walks a tile of 64
+// tokens in about 1.7 us, needs three tiles' time to start, and more than one split costs the merge's traffic.
+// Returns a word for graph keys.
+int Engine::plan_splits(int lanes, int lanes_per_stream, uint64_t newest_tick) {
     const uint64_t tokens = std::min<uint64_t>(newest_tick + 1, model_->capacity());
     auto bucket = [&](int split_tokens) {
         const int needed = std::max(1, static_cast<int>((tokens + split_tokens - 1) / split_tokens));
@@ -1524,7 +1588,26 @@ int Engine::plan_splits(int lanes, uint64_t newest_tick) {
         return std::min(count, most);
     };
     current_splits_ = bucket(split_tokens_);
+    current_op_split_tokens_ = op_split_tokens_;
     current_op_splits_ = bucket(op_split_tokens_);
+    const ModelPlan &plan = model_->plan();
+    const auto attention = std::find_if(plan.layers.begin(), plan.layers.end(), [](const ComponentPlan &layer) { return layer.has_kv; });
+    if (!scalar_attention_ && attention != plan.layers.end() && attention_is_prefill(lanes_per_stream, attention->q_heads, attention->kv_heads)) {
+        const int rows = lanes_per_stream * (attention->q_heads / attention->kv_heads);
+        const double ctas = static_cast<double>(lanes / lanes_per_stream) * ((rows + 127) / 128) * attention->kv_heads;
+        const double tiles = static_cast<double>((tokens + 63) / 64);
+        double best = 0.0;
+        for (int splits = 1; splits <= 16; splits++) {
+            if (splits > 1 && (tiles < 4.0 * splits || static_cast<size_t>(lanes) * max_q_heads_ * splits > attention_partials_)) break;
+            const double waves = std::ceil(ctas * splits / model_->sm_count());
+            const double microseconds = waves * (std::ceil(tiles / splits) + 3.0) * 1.7 + (splits > 1 ? 4.0 + lanes * attention->q_heads * splits * 2.1e-4 : 0.0);
+            if (splits == 1 || microseconds < best) {
+                best = microseconds;
+                current_op_splits_ = splits;
+                current_op_split_tokens_ = static_cast<int>(std::ceil(tiles / splits)) * 64;
+            }
+        }
+    }
     return current_splits_ | (current_op_splits_ << 16);
 }
 
@@ -1675,9 +1758,8 @@ void Engine::run_prefill_chunk(Stream &s, const uint32_t *tokens, int count, boo
     std::vector<uint32_t> positions(count);
     std::vector<int32_t> slots(count, s.slot);
     for (int i = 0; i < count; i++) positions[i] = static_cast<uint32_t>(s.next_tick + i);
-    upload_lanes(positions, slots);
+    upload_lanes(positions, slots, count);
     upload_tokens(tokens, count);
-    current_width_ = count;
     target_forward(count, false);
     const size_t frame = static_cast<size_t>(plan.hidden) * 2;
     uint8_t *pending = static_cast<uint8_t *>(pending_hidden_.ptr) + s.slot * frame;
@@ -1764,9 +1846,8 @@ void Engine::run_single_ticks(std::vector<Stream *> &batch, const std::function<
         any_emit |= !s.active->feedback_closes && s.active->remaining > 0;
     }
     sync_block_tables();
-    upload_lanes(positions, slots);
+    upload_lanes(positions, slots, 1);
     upload_tokens(tokens.data(), lanes);
-    current_width_ = 1;
     if (plan.has_draft) backup_pending();
     target_forward(lanes, any_emit);
     if (plan.has_draft) {
@@ -1858,7 +1939,7 @@ void Engine::run_speculative_cycles(std::vector<Stream *> &batch, int drafts, co
     }
     sync_block_tables();
     upload(base, staging.data(), upload_words * sizeof(uint32_t), "cycle state upload");
-    const int splits = plan_splits(streams * (drafts + 1), newest_tick);
+    const int splits = plan_splits(streams, 1, newest_tick);
 
     backup_pending();
     cuda_check(cudaEventRecord(event_begin_, cuda_stream_), "event record");
@@ -2190,9 +2271,8 @@ void Engine::debug_target_logits(int64_t id, const std::vector<uint32_t> &tokens
     std::vector<uint32_t> positions(lanes);
     std::vector<int32_t> slots(lanes, s.slot);
     for (int i = 0; i < lanes; i++) positions[i] = static_cast<uint32_t>(s.next_tick + i);
-    upload_lanes(positions, slots);
+    upload_lanes(positions, slots, lanes);
     upload_tokens(tokens.data(), lanes);
-    current_width_ = lanes;
     full_logits_ = true;  // the whole vocabulary on every rank, whatever the sampling path would project
     try {
         target_forward(lanes, true);

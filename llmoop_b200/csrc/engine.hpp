@@ -324,7 +324,7 @@ private:
     };
     void upload(void *device_destination, const void *host_source, size_t bytes, const char *what);
     void synchronize(const char *what);
-    void upload_lanes(const std::vector<uint32_t> &positions, const std::vector<int32_t> &slots);
+    void upload_lanes(const std::vector<uint32_t> &positions, const std::vector<int32_t> &slots, int lanes_per_stream);
     void upload_tokens(const uint32_t *tokens, int count);
     void run_component(const ComponentPlan &plan, int kv_index, int lanes,
                        const std::map<std::string, void *> &bound, void *output);
@@ -413,9 +413,11 @@ private:
     const uint32_t *current_tokens_ = nullptr;
     int current_width_ = 1;                 // lanes per stream of the current batch (stream-major lane order)
     int current_splits_ = 1;                // attention split count (stride of the scratch partials) of this launch
-    int op_split_tokens_ = 64;              // tokens per split on the kernel-per-operator path: fixed per engine, so that a lane's
-                                            // arithmetic does not depend on the batch it runs in
-    int current_op_splits_ = 1;             // split count of this launch on that path
+    int op_split_tokens_ = 128;             // tokens per split of decode batches on the kernel-per-operator path: fixed per engine, so
+                                            // that a lane's arithmetic does not depend on the batch it runs in
+    int current_op_split_tokens_ = 128, current_op_splits_ = 1;  // split length and count of the next launches on that path
+    bool scalar_attention_ = false;         // FP8 packages: the attention form in scalar f32
+    size_t attention_partials_ = 0;         // partials attention_scratch_ holds
     int max_q_heads_ = 1;
     struct GraphEntry {
         cudaGraphExec_t exec = nullptr;
@@ -424,7 +426,7 @@ private:
     };
     std::map<std::vector<int>, GraphEntry> graphs_;
     void run_phase(const std::vector<int> &key, const std::function<void()> &body);
-    int plan_splits(int lanes, uint64_t newest_tick);  // sets the split length and count of the next launches, returns a graph-key word
+    int plan_splits(int lanes, int lanes_per_stream, uint64_t newest_tick);  // sets the split length and count of the next launches, returns a graph-key word
 };
 
 }  // namespace nerve

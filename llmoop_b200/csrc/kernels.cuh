@@ -90,16 +90,30 @@ cudaError_t launch_moe_down_fp8(const uint16_t *intermediates, const uint32_t *r
 cudaError_t launch_moe_reduce(const uint16_t *outputs, uint16_t *y, int lanes, int hidden_size, int top_k,
                               float routed_scale, cudaStream_t stream);
 
-// Append K,V of every lane at its position, then causal GQA attention over the
-// stream's pages: split over the context, partials merged by a second kernel.
-// scratch holds [lanes][q_heads][splits][head_width + 2] f32.
-size_t attention_scratch_bytes(int lanes, int q_heads, int head_width, int max_splits);
-cudaError_t launch_kv_append(const uint16_t *k, const uint16_t *v, const KvLayer &kv, const LaneTable &lanes_meta,
-                             int lanes, cudaStream_t stream);
+// Rotary embedding of q and k (with a per-head RMSNorm in front where norm weights are given) and the append of K and V
+// at every lane's position, in one launch.
+struct RopeForm {
+    const uint32_t *cos_sin;  // [position][rotary / 2] packed (sin << 16 | cos) bf16
+    uint32_t positions;
+    int rotary, interleaved;  // rotary 0: the values as they are
+};
+struct RopeAppend {
+    const uint16_t *q, *k, *v;
+    uint16_t *q_out;
+    const uint16_t *q_norm, *k_norm;  // nullptr = no norm
+    float eps, norm_offset;
+    int q_heads;                      // 0: k and v only
+    RopeForm q_form, k_form;
+};
+cudaError_t launch_rope_append(const RopeAppend &rope, const KvLayer &kv, const LaneTable &lanes_meta, int lanes, cudaStream_t stream);
+// Causal GQA attention over the stream's pages, split over the context: split s covers split_tokens tokens, partials are
+// merged by a second kernel (max_splits 1: none).  scratch holds [lanes][q_heads][max_splits][head_width + 2] f32.
 // Lanes are stream-major: every stream of the batch contributes `lanes_per_stream` consecutive lanes.
+// scalar_f32: the form for layers whose attention output is quantised to FP8.
+bool attention_is_prefill(int lanes_per_stream, int q_heads, int kv_heads);  // the form with 128 query rows per CTA
 cudaError_t launch_attention(const uint16_t *q, uint16_t *out, const KvLayer &kv, const LaneTable &lanes_meta,
                              int lanes, int lanes_per_stream, int q_heads, float scale, int split_tokens, int max_splits,
-                             float *scratch, cudaStream_t stream);
+                             float *scratch, bool scalar_f32, cudaStream_t stream);
 
 // INT4 multi-branch forms (one launch for q/k/v; gate/up with the SiLU*up epilogue).
 cudaError_t launch_linear_int4_multi(const uint16_t *x, const void *prepared, int branches, const uint32_t *const *qweights,
@@ -128,6 +142,9 @@ cudaError_t launch_output_projection(const uint16_t *x, const void *streamed_tab
 bool linear_int4_gemm_supported(int lanes, int n, int k);
 size_t int4_activation_bytes(int lanes, int k);
 cudaError_t launch_prepare_activations(const uint16_t *x, void *prepared, int lanes, int k, cudaStream_t stream);
+// ... of the RMSNorm of x (the values launch_rms_norm writes), without writing them
+cudaError_t launch_rms_norm_prepared(const uint16_t *x, const uint16_t *weight, void *prepared, int lanes, int width, float eps, float weight_offset,
+                                     cudaStream_t stream);
 cudaError_t launch_linear_int4_gemm(const void *prepared, int branches, const uint32_t *const *qweights, const uint16_t *const *scales, void *const *ys,
                                     const int *ns, const uint16_t *residual, int lanes, int k, int epilogue, float scale, bool silu, int *error_flag,
                                     cudaStream_t stream);
@@ -190,7 +207,7 @@ struct StackShape {
 struct StackBuffers {
     uint16_t *hidden;            // [lanes][hidden] residual stream, updated in place
     uint16_t *q;                 // [lanes][q_heads * head_width]
-    float *attention_scratch;    // split partials, attention_scratch_bytes()
+    float *attention_scratch;    // split partials
     uint16_t *attention_out;     // [lanes][q_heads * head_width] fp16 in fragment order (see kernels_stack.cu)
     uint16_t *activation;        // [lanes][ffn] fp16 in fragment order
     unsigned int *barrier;       // STACK_BARRIER_WORDS words, zero before the first launch

@@ -6,76 +6,608 @@
 // of one stream carry increasing ticks, lane i sees exactly the tokens of
 // lanes < i plus the committed context - the same result as the reference's
 // serial per-lane execution, in one launch.
-//
-// Work split: one warp per (lane, kv head, context split) serves all
-// query heads of that kv head (K/V rows are read once for the group); splits of
-// `split_tokens` tokens are merged by a second kernel with a log-sum-exp
-// combine.  HBM traffic per launch = the KV bytes of the attended context
-// (2 * kv_heads * head_width * 2 B per token) per lane; the scratch partials
-// are (head_width + 2) f32 per (lane, q head, split).
 #include <atomic>
 
-#include "attention_body.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
+#include "launch.cuh"
 
 namespace nerve {
 
-__global__ void kv_append_kernel(const uint32_t *__restrict__ k, const uint32_t *__restrict__ v, KvLayer kv,
-                                 LaneTable lanes_meta) {
+namespace {
+
+__device__ __forceinline__ size_t kv_token_offset(const KvLayer &kv, int slot, uint32_t token, int head, bool value) {
+    // token is the ring index (tick % capacity)
+    int logical_page = static_cast<int>(token / kv.page_tokens);
+    int within = static_cast<int>(token % kv.page_tokens);
+    int physical = kv.block_table[static_cast<size_t>(slot) * kv.pages_per_slot + logical_page];
+    size_t half = static_cast<size_t>(kv.kv_heads) * kv.page_tokens * kv.head_width;
+    return static_cast<size_t>(physical) * (2 * half) + (value ? half : 0) +
+           (static_cast<size_t>(head) * kv.page_tokens + within) * kv.head_width;
+}
+
+constexpr float LOWEST = -3.4028234663852886e38f;
+
+// ---- tiled attention -------------------------------------------------------------------------------------------
+// A CTA serves ROW_WARPS x 16 query rows of one (stream, kv head) - row r is query head r % group of the stream's lane
+// r / group, so the query heads that share a kv head share its K/V tiles - over one split of the context.  K and V
+// tiles of 64 tokens go through two shared-memory stages (cp.async one tile ahead, the tokens' page offsets two tiles
+// ahead), Q stays in registers; Q.K^T and P.V run on mma.sync bf16 with f32 sums.  The probabilities enter P.V as a
+// bf16 pair hi + lo, so that they are not rounded to eight bits.
+// TOKEN_WARPS warps share a row tile's context: each takes 64 / TOKEN_WARPS tokens of every tile with a softmax of its
+// own, and they merge at the end.  Prefill chunks (many rows per stream) run 8 x 1 warps; verify and draft batches
+// (few rows, many tokens) 1 or 2 x 4, where four warps per row tile hide the tile's latency.
+// What bounds it: prefill the legacy tensor path (three MMAs per 16 x 8 x 16 of K or V), decode the KV bytes.
+// (One scalar f32 product per thread and token, the form this replaced, took 4.5 ms per 8B layer for 713 lanes at an
+// 8700-token context; this takes 0.5 ms.)
+
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void load_matrices(uint32_t (&r)[4], uint32_t address) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(address));
+}
+__device__ __forceinline__ void load_matrices_transposed(uint32_t (&r)[4], uint32_t address) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(address));
+}
+__device__ __forceinline__ uint32_t pack_bf16_rn(float lo, float hi) {
+    const __nv_bfloat162 pair = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&pair);
+}
+
+constexpr int TILE = 64;
+// 16-byte chunk `c` of a tile row, permuted with the row so that eight rows' equal chunks hit eight bank groups
+template <int HD>
+__device__ __forceinline__ uint32_t tile_chunk(int row, int c) {
+    return static_cast<uint32_t>(row * (HD / 8) + ((c & ~7) | ((c ^ row) & 7))) * 16;
+}
+
+struct AttentionArgs {
+    const uint16_t *q;
+    uint16_t *out;
+    KvLayer kv;
+    LaneTable meta;
+    int lanes, lanes_per_stream, q_heads, group, row_blocks;
+    float scale;
+    int split_tokens, max_splits;
+    float *scratch;
+};
+
+template <int HD, int ROW_WARPS, int TOKEN_WARPS>
+constexpr size_t attention_smem() {
+    constexpr size_t tiles = 2 * 2 * static_cast<size_t>(TILE) * HD * 2;
+    constexpr size_t merge = TOKEN_WARPS > 1 ? static_cast<size_t>(ROW_WARPS) * TOKEN_WARPS * 16 * (HD + 4) * 4 : 0;
+    return tiles > merge ? tiles : merge;
+}
+
+template <int HD, int ROW_WARPS, int TOKEN_WARPS>
+__global__ void __launch_bounds__(ROW_WARPS *TOKEN_WARPS * 32) attention_tile_kernel(const __grid_constant__ AttentionArgs a) {
+    constexpr int THREADS = ROW_WARPS * TOKEN_WARPS * 32, ROWS = ROW_WARPS * 16;
+    constexpr int TOKENS = TILE / TOKEN_WARPS;  // of a tile, per warp
+    constexpr int K_STEPS = HD / 16, N_TILES = TOKENS / 8, D_TILES = HD / 8;
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ size_t token_offset[2][TILE];
+    grid_launch_dependents();
     grid_dependency_wait();
-    int lane = blockIdx.x;
-    int slot = lanes_meta.slot[lane];
-    if (slot < 0 || kv.capacity == 0) return;
-    uint32_t token = lanes_meta.position[lane] % kv.capacity;
-    int words_per_head = kv.head_width / 2;
-    int total = kv.kv_heads * words_per_head;
-    uint32_t *pool = reinterpret_cast<uint32_t *>(kv.pool);
-    for (int index = threadIdx.x; index < total; index += blockDim.x) {
-        int head = index / words_per_head, word = index % words_per_head;
-        size_t k_off = kv_token_offset(kv, slot, token, head, false) / 2 + word;
-        size_t v_off = kv_token_offset(kv, slot, token, head, true) / 2 + word;
-        pool[k_off] = k[static_cast<size_t>(lane) * total + index];
-        pool[v_off] = v[static_cast<size_t>(lane) * total + index];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
+    const int row_warp = warp / TOKEN_WARPS, token_warp = warp % TOKEN_WARPS;
+    // the blocks with the longest contexts (the last rows of a chunk) start first
+    const int block = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x), kv_head = blockIdx.y, split = blockIdx.z;
+    const int stream = block / a.row_blocks, row0 = (block - stream * a.row_blocks) * ROWS;
+    const int rows = a.lanes_per_stream * a.group;
+    const int lane0 = stream * a.lanes_per_stream;
+    const int slot = a.meta.slot[lane0];
+    if (slot < 0) return;
+    const uint32_t capacity = a.kv.capacity;
+    const int last_row = min(row0 + ROWS, rows) - 1;
+    const uint32_t newest = a.meta.position[lane0 + last_row / a.group];
+    const uint32_t tokens = min(newest + 1u, capacity), first_tick = newest + 1u - tokens;  // attended window of the newest lane
+    const uint32_t begin = static_cast<uint32_t>(split) * a.split_tokens;
+    if (begin >= tokens) return;
+    const uint32_t end = min(begin + a.split_tokens, tokens);
+    const int tiles = static_cast<int>((end - begin + TILE - 1) / TILE);
+
+    // this thread's two rows (g and g + 8 of the warp's sixteen) and their Q fragments
+    const int r_lo = row0 + row_warp * 16 + g, r_hi = r_lo + 8;
+    const bool warp_active = row0 + row_warp * 16 < rows;
+    uint32_t tick[2];
+    uint32_t q_frag[K_STEPS][4];
+    {
+        const int rr[2] = {min(r_lo, rows - 1), min(r_hi, rows - 1)};
+        const uint32_t *source[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int l = lane0 + rr[h] / a.group;
+            tick[h] = a.meta.position[l];
+            source[h] = reinterpret_cast<const uint32_t *>(a.q + (static_cast<size_t>(l) * a.q_heads + kv_head * a.group + rr[h] % a.group) * HD) + j;
+        }
+#pragma unroll
+        for (int s = 0; s < K_STEPS; s++) {
+            q_frag[s][0] = source[0][s * 8];
+            q_frag[s][1] = source[1][s * 8];
+            q_frag[s][2] = source[0][s * 8 + 4];
+            q_frag[s][3] = source[1][s * 8 + 4];
+        }
+    }
+    // the oldest of the warp's rows: tiles that end at or before its tick need no causal mask
+    const uint32_t oldest_tick = __reduce_min_sync(0xffffffffu, min(tick[0], tick[1]));
+
+    auto offset_of = [&](int tile, int t) -> size_t {
+        const uint32_t index = min(begin + static_cast<uint32_t>(tile) * TILE + t, end - 1);
+        uint32_t ring = first_tick + index;
+        if (ring >= capacity) ring %= capacity;
+        return kv_token_offset(a.kv, slot, ring, kv_head, false);
+    };
+    const size_t value_half = static_cast<size_t>(a.kv.kv_heads) * a.kv.page_tokens * HD;
+    const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+    constexpr uint32_t TILE_BYTES = TILE * HD * 2;
+    auto request = [&](int tile) {
+        const uint32_t k_tile = base + static_cast<uint32_t>(tile & 1) * 2 * TILE_BYTES, v_tile = k_tile + TILE_BYTES;
+        constexpr int CHUNKS = HD / 8;
+#pragma unroll
+        for (int i = 0; i < TILE * CHUNKS / THREADS; i++) {
+            const int index = threadIdx.x + i * THREADS, t = index / CHUNKS, c = index % CHUNKS;
+            const uint16_t *source = a.kv.pool + token_offset[tile & 1][t] + c * 8;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(k_tile + tile_chunk<HD>(t, c)), "l"(source) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(v_tile + tile_chunk<HD>(t, c)), "l"(source + value_half) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    float acc[D_TILES][4];
+#pragma unroll
+    for (int d = 0; d < D_TILES; d++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) acc[d][i] = 0.0f;
+    float row_max[2] = {-INFINITY, -INFINITY}, row_sum[2] = {0.0f, 0.0f};
+    const float log2_scale = a.scale * 1.4426950408889634f;
+
+    if (threadIdx.x < TILE) {
+        token_offset[0][threadIdx.x] = offset_of(0, threadIdx.x);
+        token_offset[1][threadIdx.x] = offset_of(tiles > 1 ? 1 : 0, threadIdx.x);
+    }
+    __syncthreads();
+    request(0);
+    for (int tile = 0; tile < tiles; tile++) {
+        if (tile + 1 < tiles) request(tile + 1);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        size_t next_offset = 0;
+        if (threadIdx.x < TILE && tile + 2 < tiles) next_offset = offset_of(tile + 2, threadIdx.x);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const uint32_t k_tile = base + static_cast<uint32_t>(tile & 1) * 2 * TILE_BYTES, v_tile = k_tile + TILE_BYTES;
+        const uint32_t tile_begin = begin + static_cast<uint32_t>(tile) * TILE + token_warp * TOKENS;  // this warp's first token
+        if (warp_active && tile_begin < end) {
+            float score[N_TILES][4];
+#pragma unroll
+            for (int n = 0; n < N_TILES; n++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) score[n][i] = 0.0f;
+#pragma unroll
+            for (int s = 0; s < K_STEPS; s++) {
+#pragma unroll
+                for (int pair = 0; pair < N_TILES / 2; pair++) {
+                    const int matrix = lane >> 3, t = token_warp * TOKENS + pair * 16 + (matrix >> 1) * 8 + (lane & 7);
+                    uint32_t b[4];
+                    load_matrices(b, k_tile + tile_chunk<HD>(t, s * 2 + (matrix & 1)));
+                    mma_bf16(score[2 * pair], q_frag[s], b[0], b[1]);
+                    mma_bf16(score[2 * pair + 1], q_frag[s], b[2], b[3]);
+                }
+            }
+            // causal and ring limits: tick - capacity < token's tick <= tick
+            const bool masked = tile_begin + TOKENS > end || first_tick + tile_begin + TOKENS - 1 > oldest_tick || newest >= capacity;
+            if (masked) {
+#pragma unroll
+                for (int n = 0; n < N_TILES; n++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const uint32_t index = tile_begin + n * 8 + 2 * j + (i & 1), token_tick = first_tick + index, own = tick[i >> 1];
+                        if (index >= end || token_tick > own || token_tick + capacity <= own) score[n][i] = -INFINITY;
+                    }
+            }
+            float factor[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                float largest = row_max[h];
+#pragma unroll
+                for (int n = 0; n < N_TILES; n++) largest = fmaxf(largest, fmaxf(score[n][2 * h], score[n][2 * h + 1]));
+                largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, 1));
+                largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, 2));
+                const float reference = largest == -INFINITY ? 0.0f : largest;  // nothing visible yet
+                factor[h] = exp2f((row_max[h] - reference) * log2_scale);
+                row_max[h] = largest;
+                const float shift = reference * log2_scale;
+                float sum = 0.0f;
+#pragma unroll
+                for (int n = 0; n < N_TILES; n++)
+#pragma unroll
+                    for (int i = 0; i < 2; i++) {
+                        const float p = exp2f(fmaf(score[n][2 * h + i], log2_scale, -shift));
+                        score[n][2 * h + i] = p;
+                        sum += p;
+                    }
+                row_sum[h] = row_sum[h] * factor[h] + sum;  // this thread's columns; added up over the four threads in the end
+            }
+#pragma unroll
+            for (int d = 0; d < D_TILES; d++) {
+                acc[d][0] *= factor[0];
+                acc[d][1] *= factor[0];
+                acc[d][2] *= factor[1];
+                acc[d][3] *= factor[1];
+            }
+#pragma unroll
+            for (int kt = 0; kt < TOKENS / 16; kt++) {
+                uint32_t hi[4], lo[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float p0 = score[2 * kt + (i >> 1)][2 * (i & 1)], p1 = score[2 * kt + (i >> 1)][2 * (i & 1) + 1];
+                    hi[i] = pack_bf16_rn(p0, p1);
+                    lo[i] = pack_bf16_rn(p0 - bf16_lo(hi[i]), p1 - bf16_hi(hi[i]));
+                }
+#pragma unroll
+                for (int pair = 0; pair < D_TILES / 2; pair++) {
+                    const int matrix = lane >> 3, t = token_warp * TOKENS + kt * 16 + (matrix & 1) * 8 + (lane & 7);
+                    uint32_t b[4];
+                    load_matrices_transposed(b, v_tile + tile_chunk<HD>(t, pair * 2 + (matrix >> 1)));
+                    mma_bf16(acc[2 * pair], hi, b[0], b[1]);
+                    mma_bf16(acc[2 * pair + 1], hi, b[2], b[3]);
+                    mma_bf16(acc[2 * pair], lo, b[0], b[1]);
+                    mma_bf16(acc[2 * pair + 1], lo, b[2], b[3]);
+                }
+            }
+        }
+        // (this tile's offsets were last read before the barrier above, when it was requested)
+        if (threadIdx.x < TILE && tile + 2 < tiles) token_offset[tile & 1][threadIdx.x] = next_offset;
+        __syncthreads();  // the tile is read; its stage may be overwritten
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        row_sum[h] += __shfl_xor_sync(0xffffffffu, row_sum[h], 1);
+        row_sum[h] += __shfl_xor_sync(0xffffffffu, row_sum[h], 2);
+    }
+
+    // a finished row: the output itself, or the split's partial (unnormalised row, then maximum and sum)
+    auto finish = [&](int r, int d, float x0, float x1, float maximum, float sum) {
+        const size_t pair = static_cast<size_t>(lane0 + r / a.group) * a.q_heads + kv_head * a.group + r % a.group;
+        if (a.max_splits == 1) {
+            const float inverse = sum == 0.0f ? 0.0f : 1.0f / sum;
+            *reinterpret_cast<uint32_t *>(a.out + pair * HD + d) = sum == 0.0f ? 0u : pack_bf16(x0 * inverse, x1 * inverse);
+        } else {
+            float *part = a.scratch + (pair * a.max_splits + split) * (HD + 2);
+            *reinterpret_cast<float2 *>(part + d) = make_float2(x0, x1);
+            if (d == 0) *reinterpret_cast<float2 *>(part + HD) = make_float2(maximum == -INFINITY ? LOWEST : maximum * a.scale, sum);
+        }
+    };
+    if (TOKEN_WARPS == 1) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int r = h == 0 ? r_lo : r_hi;
+            if (r >= rows) continue;
+#pragma unroll
+            for (int d = 0; d < D_TILES; d++) finish(r, d * 8 + 2 * j, acc[d][2 * h], acc[d][2 * h + 1], row_max[h], row_sum[h]);
+        }
+        return;
+    }
+    // merge the token warps of a row tile: [warp][row][HD + maximum, sum]
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    constexpr int STRIDE = HD + 4;
+    float *const parts = reinterpret_cast<float *>(smem);
+    if (warp_active) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            float *row = parts + (warp * 16 + g + 8 * h) * STRIDE;
+#pragma unroll
+            for (int d = 0; d < D_TILES; d++) *reinterpret_cast<float2 *>(row + d * 8 + 2 * j) = make_float2(acc[d][2 * h], acc[d][2 * h + 1]);
+            if (j == 0) *reinterpret_cast<float2 *>(row + HD) = make_float2(row_max[h], row_sum[h]);
+        }
+    }
+    __syncthreads();
+    for (int index = threadIdx.x; index < ROWS * (HD / 2); index += THREADS) {
+        const int local = index / (HD / 2), d = (index % (HD / 2)) * 2, r = row0 + local;
+        if (r >= rows) continue;
+        const float *row = parts + ((local / 16) * TOKEN_WARPS * 16 + local % 16) * STRIDE;
+        float maximum = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < TOKEN_WARPS; w++) maximum = fmaxf(maximum, row[w * 16 * STRIDE + HD]);
+        const float reference = maximum == -INFINITY ? 0.0f : maximum;
+        float x0 = 0.0f, x1 = 0.0f, sum = 0.0f;
+#pragma unroll
+        for (int w = 0; w < TOKEN_WARPS; w++) {
+            const float *part = row + w * 16 * STRIDE;
+            const float weight = exp2f((part[HD] - reference) * log2_scale);
+            sum = fmaf(part[HD + 1], weight, sum);
+            x0 = fmaf(part[d], weight, x0);
+            x1 = fmaf(part[d + 1], weight, x1);
+        }
+        finish(r, d, x0, x1, maximum, sum);
     }
 }
 
-cudaError_t launch_kv_append(const uint16_t *k, const uint16_t *v, const KvLayer &kv, const LaneTable &lanes_meta,
-                             int lanes, cudaStream_t stream) {
-    if (lanes <= 0) return cudaSuccess;
-    kv_append_kernel<<<lanes, 128, 0, stream>>>(reinterpret_cast<const uint32_t *>(k), reinterpret_cast<const uint32_t *>(v),
-                                                kv, lanes_meta);
-    return cudaGetLastError();
+// ---- attention in scalar f32 ---------------------------------------------------------------------------------------
+// The form for layers whose attention output is quantised to FP8: there a last-bit change of a sum turns into a step of
+// one part in sixteen wherever a value sits on a rounding boundary (and, behind it, into another choice of experts), so
+// these layers keep the plain f32 order of additions - one product after the other, no split probabilities.
+__device__ __forceinline__ uint4 load16(const void *address) { return *reinterpret_cast<const uint4 *>(address); }
+
+template <int HD, int GROUP, int QL>
+constexpr size_t attention_f32_smem() {
+    constexpr int Q = QL * GROUP;
+    // K tile (padded rows), V tile, Q tile, probabilities, three per-query rows, the lanes' ticks
+    return static_cast<size_t>(TILE) * (HD + 8) * 2 + static_cast<size_t>(TILE) * HD * 2 + static_cast<size_t>(Q) * HD * 2 + static_cast<size_t>(Q) * TILE * 4 +
+           3 * Q * 4 + ((QL * 4 + 15) / 16) * 16;
 }
 
-size_t attention_scratch_bytes(int lanes, int q_heads, int head_width, int max_splits) {
-    return static_cast<size_t>(lanes) * q_heads * max_splits * (head_width + 2) * sizeof(float);
+// A CTA of 128 threads serves QL consecutive lanes of one stream x the GROUP query heads of one kv head (Q = QL*GROUP query
+// vectors) over one split of the context, tile by tile (TILE tokens):
+//   1. the K and V tiles are staged in shared memory with 16-byte loads issued back to back (one exposed
+//      latency per tile instead of one per token);
+//   2. scores: thread (t = tid % TILE, half = tid / TILE) dots K row t with Q/2 queries (K row stride is padded
+//      to HD+8 elements so the 16-byte shared loads of 8 consecutive rows hit distinct banks);
+//   3. per-query online softmax over the tile (one warp per query slice), probabilities to shared memory;
+//   4. P.V: thread d owns output dims d, d+128, .. for all Q queries, V rows read conflict-free.
+// A batch may mix streams: each stream contributes `lanes_per_stream` consecutive lanes, and a team never spans
+// two streams.  `group_slot` enumerates (stream, lane group) pairs.
+template <int HD, int GROUP, int QL>
+__device__ void attention_f32_body(const uint16_t *__restrict__ q, const KvLayer &kv, const LaneTable &lanes_meta, int lanes,
+                                   int lanes_per_stream, int q_heads, float scale, int split_tokens, int max_splits,
+                                   float *__restrict__ scratch, int kv_head, int split, int group_slot, uint8_t *smem_raw,
+                                   int tid) {
+    constexpr int Q = QL * GROUP;
+    constexpr int KSTRIDE = HD + 8;
+    constexpr int DPT = HD / 128 > 0 ? HD / 128 : 1;  // output dims per thread (HD = 128 -> 1)
+    uint16_t *k_tile = reinterpret_cast<uint16_t *>(smem_raw);                 // [TILE][KSTRIDE]
+    uint16_t *v_tile = k_tile + TILE * KSTRIDE;                                 // [TILE][HD]
+    uint16_t *q_tile = v_tile + TILE * HD;                                      // [Q][HD]
+    float *p_tile = reinterpret_cast<float *>(q_tile + Q * HD);                 // [Q][TILE]
+    float *row_max = p_tile + Q * TILE;                                         // [Q]
+    float *row_sum = row_max + Q;                                               // [Q]
+    float *row_alpha = row_sum + Q;                                             // [Q]
+    uint32_t *lane_tick = reinterpret_cast<uint32_t *>(row_alpha + Q);          // [QL]
+
+    // lanes of one stream are consecutive and every stream of the batch has `lanes_per_stream` of them
+    const int groups_per_stream = (lanes_per_stream + QL - 1) / QL;
+    const int stream_index = group_slot / groups_per_stream, group_index = group_slot % groups_per_stream;
+    const int lane0 = stream_index * lanes_per_stream + group_index * QL;
+    if (lane0 >= lanes) return;
+    const int slot = lanes_meta.slot[lane0];
+    if (slot < 0) return;
+    const uint32_t capacity = kv.capacity;
+    __syncthreads();  // the previous item of this team no longer reads the shared arrays
+    // the newest tick among this team's lanes bounds the context the CTA has to look at
+    uint32_t newest = 0;
+    if (tid < QL) {
+        int lane = lane0 + tid;
+        bool valid = lane < lanes && group_index * QL + tid < lanes_per_stream;
+        lane_tick[tid] = valid ? lanes_meta.position[lane] : 0xffffffffu;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < QL; i++)
+        if (lane_tick[i] != 0xffffffffu && lane_tick[i] > newest) newest = lane_tick[i];
+    const uint32_t tokens = newest + 1u < capacity ? newest + 1u : capacity;  // attended window of the newest lane
+    const uint32_t first_tick = newest + 1u - tokens;
+    const uint32_t begin = static_cast<uint32_t>(split) * split_tokens;
+    if (begin >= tokens) return;
+    const uint32_t end = begin + split_tokens < tokens ? begin + split_tokens : tokens;
+
+    for (int index = tid; index < Q * HD / 8; index += 128) {
+        int query = index / (HD / 8), piece = index % (HD / 8);
+        int lane = lane0 + query / GROUP;
+        uint4 value = make_uint4(0, 0, 0, 0);
+        if (lane_tick[query / GROUP] != 0xffffffffu)
+            value = load16(q + (static_cast<size_t>(lane) * q_heads + kv_head * GROUP + query % GROUP) * HD + piece * 8);
+        *reinterpret_cast<uint4 *>(q_tile + query * HD + piece * 8) = value;
+    }
+    if (tid < Q) {
+        row_max[tid] = -3.4028234663852886e38f;
+        row_sum[tid] = 0.0f;
+    }
+    float acc[Q][DPT];
+#pragma unroll
+    for (int query = 0; query < Q; query++)
+#pragma unroll
+        for (int d = 0; d < DPT; d++) acc[query][d] = 0.0f;
+
+    for (uint32_t tile_begin = begin; tile_begin < end; tile_begin += TILE) {
+        const int count = static_cast<int>(end - tile_begin < TILE ? end - tile_begin : TILE);
+        __syncthreads();  // previous tile fully consumed (and q_tile / row_* initialised)
+        // ---- stage K and V rows: HD/8 16-byte pieces per row
+        for (int index = tid; index < count * (HD / 8); index += 128) {
+            int t = index / (HD / 8), piece = index % (HD / 8);
+            uint32_t ring = (first_tick + tile_begin + t) % capacity;
+            const uint16_t *krow = kv.pool + kv_token_offset(kv, slot, ring, kv_head, false);
+            const uint16_t *vrow = kv.pool + kv_token_offset(kv, slot, ring, kv_head, true);
+            *reinterpret_cast<uint4 *>(k_tile + t * KSTRIDE + piece * 8) = load16(krow + piece * 8);
+            *reinterpret_cast<uint4 *>(v_tile + t * HD + piece * 8) = load16(vrow + piece * 8);
+        }
+        __syncthreads();
+        // ---- scores
+        {
+            const int t = tid % TILE, half = tid / TILE;
+            constexpr int QH = Q / 2 > 0 ? Q / 2 : 1;
+            float score[QH];
+#pragma unroll
+            for (int i = 0; i < QH; i++) score[i] = 0.0f;
+            if (t < count && half * QH < Q) {
+                for (int piece = 0; piece < HD / 8; piece++) {
+                    uint4 kraw = *reinterpret_cast<const uint4 *>(k_tile + t * KSTRIDE + piece * 8);
+                    const uint32_t kw[4] = {kraw.x, kraw.y, kraw.z, kraw.w};
+#pragma unroll
+                    for (int i = 0; i < QH; i++) {
+                        uint4 qraw = *reinterpret_cast<const uint4 *>(q_tile + (half * QH + i) * HD + piece * 8);
+                        const uint32_t qw[4] = {qraw.x, qraw.y, qraw.z, qraw.w};
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            score[i] = fmaf(bf16_lo(qw[j]), bf16_lo(kw[j]), score[i]);
+                            score[i] = fmaf(bf16_hi(qw[j]), bf16_hi(kw[j]), score[i]);
+                        }
+                    }
+                }
+            }
+            const uint32_t token_tick = first_tick + tile_begin + t;
+#pragma unroll
+            for (int i = 0; i < QH; i++) {
+                int query = half * QH + i;
+                if (query >= Q) break;
+                uint32_t tick = lane_tick[query / GROUP];
+                // causal + ring window of this lane: ticks in (tick - capacity, tick]
+                bool visible = t < count && tick != 0xffffffffu && token_tick <= tick && token_tick + capacity > tick;
+                p_tile[query * TILE + t] = visible ? score[i] * scale : -INFINITY;
+            }
+        }
+        __syncthreads();
+        // ---- online softmax: warp w handles queries w, w+4, ...
+        {
+            const int warp = tid >> 5, lane_id = tid & 31;
+            for (int query = warp; query < Q; query += 4) {
+                float s0 = p_tile[query * TILE + lane_id], s1 = p_tile[query * TILE + 32 + lane_id];
+                float tile_max = warp_max(fmaxf(s0, s1));
+                float old_max = row_max[query];
+                float next_max = fmaxf(old_max, tile_max);
+                float p0 = 0.0f, p1 = 0.0f, alpha = 1.0f;
+                if (next_max > -3.0e38f) {
+                    alpha = expf(old_max - next_max);
+                    p0 = s0 == -INFINITY ? 0.0f : expf(s0 - next_max);
+                    p1 = s1 == -INFINITY ? 0.0f : expf(s1 - next_max);
+                }
+                float tile_sum = warp_sum(p0 + p1);
+                p_tile[query * TILE + lane_id] = p0;
+                p_tile[query * TILE + 32 + lane_id] = p1;
+                if (lane_id == 0) {
+                    row_alpha[query] = alpha;
+                    row_sum[query] = row_sum[query] * alpha + tile_sum;
+                    row_max[query] = next_max;
+                }
+            }
+        }
+        __syncthreads();
+        // ---- P.V
+#pragma unroll
+        for (int query = 0; query < Q; query++) {
+            float alpha = row_alpha[query];
+#pragma unroll
+            for (int d = 0; d < DPT; d++) acc[query][d] *= alpha;
+        }
+        if (tid < HD || DPT > 1) {
+            for (int t = 0; t < count; t++) {
+                float vv[DPT];
+#pragma unroll
+                for (int d = 0; d < DPT; d++) vv[d] = (tid + d * 128 < HD) ? bf16_bits_to_f32(v_tile[t * HD + tid + d * 128]) : 0.0f;
+#pragma unroll
+                for (int query = 0; query < Q; query++) {
+                    float p = p_tile[query * TILE + t];
+#pragma unroll
+                    for (int d = 0; d < DPT; d++) acc[query][d] = fmaf(p, vv[d], acc[query][d]);
+                }
+            }
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int query = 0; query < Q; query++) {
+        if (lane_tick[query / GROUP] == 0xffffffffu) continue;
+        int lane = lane0 + query / GROUP;
+        float *out = scratch + ((static_cast<size_t>(lane) * q_heads + kv_head * GROUP + query % GROUP) * max_splits + split) * (HD + 2);
+#pragma unroll
+        for (int d = 0; d < DPT; d++)
+            if (tid + d * 128 < HD) out[tid + d * 128] = acc[query][d];
+        if (tid == 0) {
+            out[HD] = row_max[query];
+            out[HD + 1] = row_sum[query];
+        }
+    }
 }
 
-// One CTA (128 threads) = one team of attention_tile_body (attention_body.cuh): grid (kv head, split, stream x lane group).
 template <int HD, int GROUP, int QL>
 __global__ void __launch_bounds__(128)
-attention_tile_kernel(const uint16_t *__restrict__ q, KvLayer kv, LaneTable lanes_meta, int lanes, int lanes_per_stream,
-                      int q_heads, float scale, int split_tokens, int max_splits, float *__restrict__ scratch) {
+attention_f32_kernel(const uint16_t *__restrict__ q, KvLayer kv, LaneTable lanes_meta, int lanes, int lanes_per_stream,
+                     int q_heads, float scale, int split_tokens, int max_splits, float *__restrict__ scratch) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
+    grid_launch_dependents();
     grid_dependency_wait();
-    attention_tile_body<HD, GROUP, QL, false>(q, kv, lanes_meta, lanes, lanes_per_stream, q_heads, scale, split_tokens, max_splits,
-                                              scratch, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw, threadIdx.x, 0);
+    attention_f32_body<HD, GROUP, QL>(q, kv, lanes_meta, lanes, lanes_per_stream, q_heads, scale, split_tokens, max_splits, scratch, blockIdx.x, blockIdx.y,
+                                      blockIdx.z, smem_raw, threadIdx.x);
+}
+
+// Log-sum-exp merge of the split partials of one (lane, q head) pair by one warp.
+__device__ __forceinline__ void attention_f32_merge_pair(const float *__restrict__ scratch, uint16_t *__restrict__ out, const KvLayer &kv,
+                                                     const LaneTable &lanes_meta, int pair, int lane_id, int q_heads, int head_width,
+                                                     int split_tokens, int max_splits) {
+    int lane = pair / q_heads;
+    int slot = lanes_meta.slot[lane];
+    if (slot < 0) return;
+    uint32_t tick = lanes_meta.position[lane];
+    uint32_t tokens = tick + 1u < kv.capacity ? tick + 1u : kv.capacity;
+    int splits = static_cast<int>((tokens + split_tokens - 1) / split_tokens);
+    if (splits > max_splits) splits = max_splits;
+    const float *base = scratch + static_cast<size_t>(pair) * max_splits * (head_width + 2);
+    auto read = [&](const float *address) { return *address; };
+    float maximum = -3.4028234663852886e38f;
+    for (int s = 0; s < splits; s++) maximum = fmaxf(maximum, read(base + static_cast<size_t>(s) * (head_width + 2) + head_width));
+    float denominator = 0.0f;
+    for (int s = 0; s < splits; s++) {
+        const float *part = base + static_cast<size_t>(s) * (head_width + 2);
+        denominator += read(part + head_width + 1) * expf(read(part + head_width) - maximum);
+    }
+    for (int d = lane_id; d < head_width; d += 32) {
+        float acc = 0.0f;
+        for (int s = 0; s < splits; s++) {
+            const float *part = base + static_cast<size_t>(s) * (head_width + 2);
+            acc += read(part + d) * expf(read(part + head_width) - maximum);
+        }
+        out[static_cast<size_t>(pair) * head_width + d] =
+            static_cast<uint16_t>(f32_to_bf16_bits(denominator == 0.0f ? 0.0f : acc / denominator));
+    }
+}
+
+__global__ void attention_f32_merge_kernel(const float *__restrict__ scratch, uint16_t *__restrict__ out, KvLayer kv,
+                                           LaneTable lanes_meta, int lanes, int q_heads, int head_width, int split_tokens,
+                                           int max_splits) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    int pair = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (pair >= lanes * q_heads) return;
+    attention_f32_merge_pair(scratch, out, kv, lanes_meta, pair, threadIdx.x & 31, q_heads, head_width, split_tokens, max_splits);
 }
 
 template <int HD, int GROUP, int QL>
-static size_t attention_tile_smem() {
-    return attention_team_smem<HD, GROUP, QL>();
+cudaError_t launch_f32(const AttentionArgs &a, cudaStream_t stream) {
+    auto kernel = attention_f32_kernel<HD, GROUP, QL>;
+    constexpr size_t smem = attention_f32_smem<HD, GROUP, QL>();
+    cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (status != cudaSuccess) return status;
+    const dim3 grid(a.kv.kv_heads, a.max_splits, a.lanes / a.lanes_per_stream * ((a.lanes_per_stream + QL - 1) / QL));
+    status = launch_dependent(kernel, grid, dim3(128), smem, 1, stream, a.q, a.kv, a.meta, a.lanes, a.lanes_per_stream, a.q_heads, a.scale, a.split_tokens,
+                              a.max_splits, a.scratch);
+    if (status != cudaSuccess) return status;
+    return launch_dependent(attention_f32_merge_kernel, dim3((a.lanes * a.q_heads + 3) / 4), dim3(128), 0, 1, stream, a.scratch, a.out, a.kv, a.meta, a.lanes,
+                            a.q_heads, a.kv.head_width, a.split_tokens, a.max_splits);
 }
 
-// Small heads (head_width < 32, tiny test models): one thread per (lane, q head), plain loops.
+template <int HD>
+cudaError_t launch_f32_of_width(const AttentionArgs &args, cudaStream_t stream) {
+    switch (args.group) {
+    case 1: return launch_f32<HD, 1, 4>(args, stream);
+    case 2: return launch_f32<HD, 2, 4>(args, stream);
+    case 4: return launch_f32<HD, 4, 4>(args, stream);
+    default: return launch_f32<HD, 8, 2>(args, stream);
+    }
+}
+
+// Heads of at most 32 (tiny models, short contexts: latency, not bandwidth): one warp per (lane, q head), scalar f32; its
+// threads take every 32nd token with a softmax of their own and merge in the end.  (One thread per (lane, q head), the
+// form this replaced, took 32 us for a 30-token context; this takes 8.)
 __global__ void attention_small_kernel(const uint16_t *__restrict__ q, uint16_t *__restrict__ out, KvLayer kv,
                                        LaneTable lanes_meta, int lanes, int q_heads, float scale) {
+    grid_launch_dependents();
     grid_dependency_wait();
-    int index = blockIdx.x * blockDim.x + threadIdx.x;
+    const int index = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), thread = threadIdx.x & 31;
     if (index >= lanes * q_heads) return;
-    int lane = index / q_heads, head = index % q_heads;
-    int slot = lanes_meta.slot[lane];
+    const int lane = index / q_heads, head = index % q_heads;
+    const int slot = lanes_meta.slot[lane];
     if (slot < 0) return;
     const int hd = kv.head_width;
     const int kv_head = head / (q_heads / kv.kv_heads);
@@ -84,91 +616,230 @@ __global__ void attention_small_kernel(const uint16_t *__restrict__ q, uint16_t 
     const uint32_t tokens = tick + 1u < capacity ? tick + 1u : capacity;
     const uint32_t first_tick = tick + 1u - tokens;
     const uint16_t *qv = q + (static_cast<size_t>(lane) * q_heads + head) * hd;
-    float acc[32];
-    for (int d = 0; d < hd; d++) acc[d] = 0.0f;
-    float maximum = -3.4028234663852886e38f, denominator = 0.0f;
-    for (uint32_t i = 0; i < tokens; i++) {
-        uint32_t ring = (first_tick + i) % capacity;
+    float query[32], acc[32];
+#pragma unroll
+    for (int d = 0; d < 32; d++) {
+        query[d] = d < hd ? bf16_bits_to_f32(qv[d]) : 0.0f;
+        acc[d] = 0.0f;
+    }
+    float maximum = LOWEST, denominator = 0.0f;
+    for (uint32_t i = thread; i < tokens; i += 32) {
+        const uint32_t ring = (first_tick + i) % capacity;
         const uint16_t *kr = kv.pool + kv_token_offset(kv, slot, ring, kv_head, false);
         const uint16_t *vr = kv.pool + kv_token_offset(kv, slot, ring, kv_head, true);
         float dot = 0.0f;
-        for (int d = 0; d < hd; d++) dot = fmaf(bf16_bits_to_f32(qv[d]), bf16_bits_to_f32(kr[d]), dot);
-        float score = dot * scale;
-        float next_max = fmaxf(maximum, score);
-        float alpha = expf(maximum - next_max), beta = expf(score - next_max);
+#pragma unroll
+        for (int d = 0; d < 32; d++)
+            if (d < hd) dot = fmaf(query[d], bf16_bits_to_f32(kr[d]), dot);
+        const float score = dot * scale, next_max = fmaxf(maximum, score);
+        const float alpha = expf(maximum - next_max), beta = expf(score - next_max);
         denominator = denominator * alpha + beta;
         maximum = next_max;
-        for (int d = 0; d < hd; d++) acc[d] = acc[d] * alpha + beta * bf16_bits_to_f32(vr[d]);
+#pragma unroll
+        for (int d = 0; d < 32; d++)
+            if (d < hd) acc[d] = acc[d] * alpha + beta * bf16_bits_to_f32(vr[d]);
     }
-    uint16_t *o = out + (static_cast<size_t>(lane) * q_heads + head) * hd;
-    for (int d = 0; d < hd; d++) o[d] = static_cast<uint16_t>(f32_to_bf16_bits(denominator == 0.0f ? 0.0f : acc[d] / denominator));
+    const float whole_max = warp_max(maximum), weight = expf(maximum - whole_max);
+    denominator = warp_sum(denominator * weight);
+    float own = 0.0f;  // thread d keeps dimension d
+#pragma unroll
+    for (int d = 0; d < 32; d++) {
+        if (d >= hd) break;
+        const float sum = warp_sum(acc[d] * weight);
+        if (thread == d) own = sum;
+    }
+    if (thread < hd)
+        out[(static_cast<size_t>(lane) * q_heads + head) * hd + thread] =
+            static_cast<uint16_t>(f32_to_bf16_bits(denominator == 0.0f ? 0.0f : own / denominator));
 }
 
 // Log-sum-exp merge of the split partials; one warp per (lane, q head).
 __global__ void attention_merge_kernel(const float *__restrict__ scratch, uint16_t *__restrict__ out, KvLayer kv,
                                        LaneTable lanes_meta, int lanes, int q_heads, int head_width, int split_tokens,
                                        int max_splits) {
+    grid_launch_dependents();
     grid_dependency_wait();
-    int pair = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int pair = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), thread = threadIdx.x & 31;
     if (pair >= lanes * q_heads) return;
-    attention_merge_pair<false>(scratch, out, kv, lanes_meta, pair, threadIdx.x & 31, q_heads, head_width, split_tokens, max_splits);
+    const int lane = pair / q_heads;
+    if (lanes_meta.slot[lane] < 0) return;
+    const uint32_t tick = lanes_meta.position[lane];
+    const uint32_t tokens = tick + 1u < kv.capacity ? tick + 1u : kv.capacity;
+    const int splits = min(static_cast<int>((tokens + split_tokens - 1) / split_tokens), max_splits), stride = head_width + 2;
+    const float *base = scratch + static_cast<size_t>(pair) * max_splits * stride;
+    float maximum = LOWEST;
+    for (int s = thread; s < splits; s += 32) maximum = fmaxf(maximum, base[static_cast<size_t>(s) * stride + head_width]);
+    maximum = warp_max(maximum);
+    float denominator = 0.0f;
+    float2 acc[2] = {};  // two dimensions per thread and 64 of the head
+    for (int first = 0; first < splits; first += 32) {
+        float weight = 0.0f;
+        if (first + thread < splits) {
+            const float2 state = *reinterpret_cast<const float2 *>(base + static_cast<size_t>(first + thread) * stride + head_width);
+            weight = expf(state.x - maximum);
+            denominator = fmaf(state.y, weight, denominator);
+        }
+        const int count = min(32, splits - first);
+#pragma unroll 4
+        for (int s = 0; s < count; s++) {
+            const float w = __shfl_sync(0xffffffffu, weight, s);
+            const float2 *part = reinterpret_cast<const float2 *>(base + static_cast<size_t>(first + s) * stride);
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+                if (2 * thread + 64 * i < head_width) {
+                    const float2 v = part[thread + 32 * i];
+                    acc[i].x = fmaf(v.x, w, acc[i].x);
+                    acc[i].y = fmaf(v.y, w, acc[i].y);
+                }
+        }
+    }
+    denominator = warp_sum(denominator);
+    const float inverse = denominator == 0.0f ? 0.0f : 1.0f / denominator;
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+        if (2 * thread + 64 * i < head_width)
+            *reinterpret_cast<uint32_t *>(out + static_cast<size_t>(pair) * head_width + 2 * thread + 64 * i) = pack_bf16(acc[i].x * inverse, acc[i].y * inverse);
 }
 
-template <int HD, int GROUP, int QL>
-static cudaError_t launch_tile(const uint16_t *q, const KvLayer &kv, const LaneTable &lanes_meta, int lanes, int lanes_per_stream,
-                               int q_heads, float scale, int split_tokens, int max_splits, float *scratch, cudaStream_t stream) {
-    static bool configured = false;
-    const size_t smem = attention_tile_smem<HD, GROUP, QL>();
-    if (!configured) {
-        cudaError_t status = cudaFuncSetAttribute(attention_tile_kernel<HD, GROUP, QL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  static_cast<int>(smem));
-        if (status != cudaSuccess) return status;
-        configured = true;
-    }
-    const int streams = (lanes + lanes_per_stream - 1) / lanes_per_stream;
-    dim3 grid(kv.kv_heads, max_splits, streams * ((lanes_per_stream + QL - 1) / QL));
-    attention_tile_kernel<HD, GROUP, QL><<<grid, 128, smem, stream>>>(q, kv, lanes_meta, lanes, lanes_per_stream, q_heads, scale, split_tokens,
-                                                                      max_splits, scratch);
-    return cudaGetLastError();
+template <int HD, int ROW_WARPS, int TOKEN_WARPS>
+cudaError_t launch_tiles(const AttentionArgs &args, dim3 grid, cudaStream_t stream) {
+    auto kernel = attention_tile_kernel<HD, ROW_WARPS, TOKEN_WARPS>;
+    constexpr size_t smem = attention_smem<HD, ROW_WARPS, TOKEN_WARPS>();
+    cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (status != cudaSuccess) return status;
+    return launch_dependent(kernel, grid, dim3(ROW_WARPS * TOKEN_WARPS * 32), smem, 1, stream, args);
 }
 
 template <int HD>
-static cudaError_t launch_tile_group(int group, const uint16_t *q, const KvLayer &kv, const LaneTable &lanes_meta, int lanes,
-                                     int lanes_per_stream, int q_heads, float scale, int split_tokens, int max_splits, float *scratch,
-                                     cudaStream_t stream) {
-    switch (group) {
-    case 1: return launch_tile<HD, 1, 4>(q, kv, lanes_meta, lanes, lanes_per_stream, q_heads, scale, split_tokens, max_splits, scratch, stream);
-    case 2: return launch_tile<HD, 2, 4>(q, kv, lanes_meta, lanes, lanes_per_stream, q_heads, scale, split_tokens, max_splits, scratch, stream);
-    case 4: return launch_tile<HD, 4, 4>(q, kv, lanes_meta, lanes, lanes_per_stream, q_heads, scale, split_tokens, max_splits, scratch, stream);
-    case 8: return launch_tile<HD, 8, 2>(q, kv, lanes_meta, lanes, lanes_per_stream, q_heads, scale, split_tokens, max_splits, scratch, stream);
-    default: return cudaErrorInvalidValue;
+cudaError_t launch_tiles_of_width(AttentionArgs args, int streams, cudaStream_t stream) {
+    const int rows = args.lanes_per_stream * args.group;
+    auto grid = [&](int block_rows) {
+        args.row_blocks = (rows + block_rows - 1) / block_rows;
+        return dim3(static_cast<unsigned int>(streams * args.row_blocks), static_cast<unsigned int>(args.kv.kv_heads), static_cast<unsigned int>(args.max_splits));
+    };
+    if (attention_is_prefill(args.lanes_per_stream, args.q_heads, args.kv.kv_heads)) {
+        const dim3 blocks = grid(128);
+        return launch_tiles<HD, 8, 1>(args, blocks, stream);
     }
+    if (rows <= 16) {
+        const dim3 blocks = grid(16);
+        return launch_tiles<HD, 1, 4>(args, blocks, stream);
+    }
+    const dim3 blocks = grid(32);
+    return launch_tiles<HD, 2, 4>(args, blocks, stream);
 }
+
+}  // namespace
+
+// Up to 96 rows (lanes x query heads per kv head) of a stream run the small-batch form: three blocks of 32 rows read the
+// context three times at most, and from there on the 128-row form wastes less than it saves.
+bool attention_is_prefill(int lanes_per_stream, int q_heads, int kv_heads) { return lanes_per_stream * (q_heads / kv_heads) > 96; }
 
 cudaError_t launch_attention(const uint16_t *q, uint16_t *out, const KvLayer &kv, const LaneTable &lanes_meta,
                              int lanes, int lanes_per_stream, int q_heads, float scale, int split_tokens, int max_splits,
-                             float *scratch, cudaStream_t stream) {
+                             float *scratch, bool scalar_f32, cudaStream_t stream) {
     if (lanes <= 0) return cudaSuccess;
     if (lanes_per_stream <= 0 || lanes % lanes_per_stream != 0) return cudaErrorInvalidValue;
     const int group = q_heads / kv.kv_heads;
-    const bool wide = kv.head_width == 32 || kv.head_width == 64 || kv.head_width == 128;
+    const bool wide = kv.head_width == 64 || kv.head_width == 128;
     if (!wide || (group != 1 && group != 2 && group != 4 && group != 8)) {
         if (kv.head_width > 32) return cudaErrorInvalidValue;
-        int total = lanes * q_heads;
-        attention_small_kernel<<<(total + 63) / 64, 64, 0, stream>>>(q, out, kv, lanes_meta, lanes, q_heads, scale);
-        return cudaGetLastError();
+        return launch_dependent(attention_small_kernel, dim3((lanes * q_heads + 3) / 4), dim3(128), 0, 1, stream, q, out, kv, lanes_meta, lanes, q_heads, scale);
     }
-    cudaError_t status;
-    switch (kv.head_width) {
-    case 128: status = launch_tile_group<128>(group, q, kv, lanes_meta, lanes, lanes_per_stream, q_heads, scale, split_tokens, max_splits, scratch, stream); break;
-    case 64: status = launch_tile_group<64>(group, q, kv, lanes_meta, lanes, lanes_per_stream, q_heads, scale, split_tokens, max_splits, scratch, stream); break;
-    default: status = launch_tile_group<32>(group, q, kv, lanes_meta, lanes, lanes_per_stream, q_heads, scale, split_tokens, max_splits, scratch, stream); break;
+    AttentionArgs args = {};
+    args.q = q;
+    args.out = out;
+    args.kv = kv;
+    args.meta = lanes_meta;
+    args.lanes = lanes;
+    args.lanes_per_stream = lanes_per_stream;
+    args.q_heads = q_heads;
+    args.group = group;
+    args.scale = scale;
+    args.split_tokens = split_tokens;
+    args.max_splits = max_splits;
+    args.scratch = scratch;
+    if (scalar_f32) return kv.head_width == 128 ? launch_f32_of_width<128>(args, stream) : launch_f32_of_width<64>(args, stream);
+    const int streams = lanes / lanes_per_stream;
+    cudaError_t status = kv.head_width == 128 ? launch_tiles_of_width<128>(args, streams, stream) : launch_tiles_of_width<64>(args, streams, stream);
+    if (status != cudaSuccess || max_splits == 1) return status;
+    return launch_dependent(attention_merge_kernel, dim3((lanes * q_heads + 3) / 4), dim3(128), 0, 1, stream, scratch, out, kv, lanes_meta, lanes, q_heads,
+                            kv.head_width, split_tokens, max_splits);
+}
+
+// ---- rotary embedding of q and k and the KV append in one launch -------------------------------------------------
+// rotary_bf16.comp.template:99-109 (five bf16 roundings per element; cos/sin from the table the mounter fills with the
+// same f32 pow/cos/sin sequence), parallel_head_norm_rope_2way_bf16.comp.template:166-209 where norm weights are given
+// (per-head RMSNorm rounded to bf16 first), then the append of append_gqa_attention_bf16.comp.template:189-215.  One
+// warp per (lane, head): query heads go to q_out, key heads and values straight into the lane's KV slot.
+namespace {
+
+constexpr int ROPE_WARPS = 8;
+__global__ void __launch_bounds__(ROPE_WARPS * 32) rope_append_kernel(const __grid_constant__ RopeAppend r, const KvLayer kv, const LaneTable meta) {
+    extern __shared__ float rows[];  // [warp][head width]
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int warp = threadIdx.x >> 5, thread = threadIdx.x & 31, lane = blockIdx.x, head = blockIdx.y * ROPE_WARPS + warp;
+    const int width = kv.head_width;
+    if (head >= r.q_heads + 2 * kv.kv_heads) return;
+    const int part = head < r.q_heads ? 0 : (head < r.q_heads + kv.kv_heads ? 1 : 2);  // q, k, v
+    const int own_head = part == 0 ? head : head - r.q_heads - (part == 2 ? kv.kv_heads : 0);
+    const int heads = part == 0 ? r.q_heads : kv.kv_heads;
+    const uint16_t *in = (part == 0 ? r.q : part == 1 ? r.k : r.v) + (static_cast<size_t>(lane) * heads + own_head) * width;
+    uint16_t *out;
+    if (part == 0) {
+        out = r.q_out + (static_cast<size_t>(lane) * heads + own_head) * width;
+    } else {
+        const int slot = meta.slot[lane];
+        if (slot < 0 || kv.capacity == 0) return;
+        out = kv.pool + kv_token_offset(kv, slot, meta.position[lane] % kv.capacity, own_head, part == 2);
     }
-    if (status != cudaSuccess) return status;
-    int pairs = lanes * q_heads;
-    attention_merge_kernel<<<(pairs + 3) / 4, 128, 0, stream>>>(scratch, out, kv, lanes_meta, lanes, q_heads, kv.head_width,
-                                                                split_tokens, max_splits);
-    return cudaGetLastError();
+    if (part == 2) {
+        for (int word = thread; word < width / 2; word += 32) reinterpret_cast<uint32_t *>(out)[word] = reinterpret_cast<const uint32_t *>(in)[word];
+        return;
+    }
+    float *values = rows + warp * width;
+    for (int word = thread; word < width / 2; word += 32) {
+        const uint32_t packed = reinterpret_cast<const uint32_t *>(in)[word];
+        values[2 * word] = bf16_lo(packed);
+        values[2 * word + 1] = bf16_hi(packed);
+    }
+    const uint16_t *norm = part == 0 ? r.q_norm : r.k_norm;
+    if (norm != nullptr) {
+        __syncwarp();
+        // the squares are added as rope_kernel's CTA of `lanes_of` threads adds them: per thread, per warp, over the warps
+        const int lanes_of = min((width / 2 + 31) / 32 * 32, 256);
+        float total = 0.0f;
+        for (int first = 0; first < lanes_of; first += 32) {
+            float sum = 0.0f;
+            for (int d = first + thread; d < width; d += lanes_of) sum = fmaf(values[d], values[d], sum);
+            total += warp_sum(sum);
+        }
+        const float inv_rms = 1.0f / sqrtf(total / static_cast<float>(width) + r.eps);
+        for (int d = thread; d < width; d += 32) values[d] = round_bf16(values[d] * inv_rms * (bf16_bits_to_f32(norm[d]) + r.norm_offset));
+    }
+    __syncwarp();
+    const RopeForm &form = part == 0 ? r.q_form : r.k_form;
+    const int half = form.rotary / 2;
+    const uint32_t *table = form.cos_sin + static_cast<size_t>(meta.position[lane] % form.positions) * half;
+    auto rotated = [&](int d) {
+        if (d >= form.rotary) return values[d];
+        const uint32_t packed = table[form.interleaved ? d / 2 : d % half];
+        float other;
+        if (form.interleaved) other = (d & 1) == 0 ? -values[d + 1] : values[d - 1];
+        else other = d < half ? -values[d + half] : values[d - half];
+        return round_bf16(values[d] * bf16_lo(packed)) + round_bf16(other * bf16_hi(packed));
+    };
+    for (int word = thread; word < width / 2; word += 32) reinterpret_cast<uint32_t *>(out)[word] = pack_bf16(rotated(2 * word), rotated(2 * word + 1));
+}
+
+}  // namespace
+
+cudaError_t launch_rope_append(const RopeAppend &rope, const KvLayer &kv, const LaneTable &lanes_meta, int lanes, cudaStream_t stream) {
+    if (lanes <= 0) return cudaSuccess;
+    const int heads = rope.q_heads + 2 * kv.kv_heads;
+    return launch_dependent(rope_append_kernel, dim3(lanes, (heads + ROPE_WARPS - 1) / ROPE_WARPS), dim3(ROPE_WARPS * 32),
+                            static_cast<size_t>(ROPE_WARPS) * kv.head_width * sizeof(float), 1, stream, rope, kv, lanes_meta);
 }
 
 // greedy_sampler_f32.comp.template:31-34,52-109: arg-max with ties -> lowest id.  Two stages so that a

@@ -28,6 +28,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "launch.cuh"
 
 namespace nerve {
 
@@ -153,6 +154,7 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
     const uint32_t a_full = shared_address(smem) + a.barrier_offset, a_empty = a_full + 8 * GEMM_MAX_A_STAGES, b_full = a_empty + 8 * GEMM_MAX_A_STAGES,
                    b_empty = b_full + 8 * GEMM_MAX_B_STAGES, all_done = b_empty + 8 * GEMM_MAX_B_STAGES, tmem_slot = all_done + 8;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    grid_launch_dependents();
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < GEMM_MAX_A_STAGES; s++) {
@@ -377,7 +379,6 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
         }
     }
     __syncwarp();
-    grid_launch_dependents();
     grid_dependency_wait();  // outputs may be inputs of the kernel in front
 
     // ---- accumulators -> f32 [lane][row] in shared memory (every copy and MMA that used it is done by then)
@@ -497,28 +498,66 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
 
 // bf16 [lanes][k] -> fp16 x 2^e in the GEMM's tile order, one CTA per lane (lanes beyond the batch are zero): largest
 // magnitude of the row, then the conversion; a 16-byte piece of eight columns holds them in the order (0,4)(1,5)(2,6)
-// (3,7) the nibble pairs come out in, at its swizzled place in the 8-lane x 64-column atom.
-constexpr int PREPARE_THREADS = 256;
-__global__ void __launch_bounds__(PREPARE_THREADS) prepare_activations_kernel(const uint16_t *__restrict__ x, uint8_t *__restrict__ out, float *__restrict__ factors,
-                                                                             int lanes, int lane_blocks, int k) {
-    __shared__ uint32_t warp_largest[PREPARE_THREADS / 32];
+// (3,7) the nibble pairs come out in, at its swizzled place in the 8-lane x 64-column atom.  With NORM the row is the
+// RMSNorm of x (rms_norm_bf16.comp.template:49-72), kept in shared memory between its two passes.
+constexpr int PREPARE_THREADS = 512;
+template <bool NORM>
+__global__ void __launch_bounds__(PREPARE_THREADS) prepare_activations_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ weight, float eps,
+                                                                             float weight_offset, uint8_t *__restrict__ out, float *__restrict__ factors, int lanes,
+                                                                             int lane_blocks, int k) {
+    constexpr int WARPS = PREPARE_THREADS / 32;
+    extern __shared__ __align__(16) uint4 normalised[];
+    __shared__ float warp_sums[WARPS];
+    __shared__ uint32_t warp_largest[WARPS];
     const int m = blockIdx.x, pieces = k >> 3;
+    grid_launch_dependents();
     grid_dependency_wait();
     const uint4 *row = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(m) * k);
     uint32_t largest = 0;
     if (m < lanes) {
-        for (int p = threadIdx.x; p < pieces; p += PREPARE_THREADS) {
-            const uint4 v = row[p];
-            const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+        if (NORM) {
+            float sum = 0.0f;
+            for (int p = threadIdx.x; p < pieces; p += PREPARE_THREADS) {
+                const uint4 v = row[p];
+                normalised[p] = v;
+                const uint32_t words[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-            for (int i = 0; i < 4; i++) largest = max(largest, max((words[i] & 0x7FFFu), (words[i] >> 16) & 0x7FFFu));
+                for (int i = 0; i < 4; i++) {
+                    sum = fmaf(bf16_lo(words[i]), bf16_lo(words[i]), sum);
+                    sum = fmaf(bf16_hi(words[i]), bf16_hi(words[i]), sum);
+                }
+            }
+            sum = warp_sum(sum);
+            if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = sum;
+            __syncthreads();
+            float total = 0.0f;
+#pragma unroll
+            for (int w = 0; w < WARPS; w++) total += warp_sums[w];
+            const float inv_rms = 1.0f / sqrtf(total * (1.0f / static_cast<float>(k)) + eps);
+            for (int p = threadIdx.x; p < pieces; p += PREPARE_THREADS) {
+                const uint4 v = normalised[p], w = reinterpret_cast<const uint4 *>(weight)[p];
+                auto norm = [&](uint32_t value, uint32_t factor) {
+                    return pack_bf16(bf16_lo(value) * inv_rms * (bf16_lo(factor) + weight_offset), bf16_hi(value) * inv_rms * (bf16_hi(factor) + weight_offset));
+                };
+                const uint4 y = make_uint4(norm(v.x, w.x), norm(v.y, w.y), norm(v.z, w.z), norm(v.w, w.w));
+                normalised[p] = y;
+                const uint32_t words[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++) largest = max(largest, max((words[i] & 0x7FFFu), (words[i] >> 16) & 0x7FFFu));
+            }
+        } else {
+            for (int p = threadIdx.x; p < pieces; p += PREPARE_THREADS) {
+                const uint4 v = row[p];
+                const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++) largest = max(largest, max((words[i] & 0x7FFFu), (words[i] >> 16) & 0x7FFFu));
+            }
         }
-#pragma unroll
-        for (int offset = 16; offset > 0; offset >>= 1) largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, offset));
+        largest = __reduce_max_sync(0xffffffffu, largest);
         if ((threadIdx.x & 31) == 0) warp_largest[threadIdx.x >> 5] = largest;
         __syncthreads();
 #pragma unroll
-        for (int w = 0; w < PREPARE_THREADS / 32; w++) largest = max(largest, warp_largest[w]);
+        for (int w = 0; w < WARPS; w++) largest = max(largest, warp_largest[w]);
     }
     const int exponent = max(static_cast<int>(largest >> 7), 16);
     const float factor = power_of_two(min(268 - exponent, 254));
@@ -526,7 +565,7 @@ __global__ void __launch_bounds__(PREPARE_THREADS) prepare_activations_kernel(co
     for (int p = threadIdx.x; p < pieces; p += PREPARE_THREADS) {
         uint4 packed = make_uint4(0, 0, 0, 0);
         if (m < lanes) {
-            const uint4 v = row[p];
+            const uint4 v = NORM ? normalised[p] : row[p];
             auto both = [&](uint32_t a, uint32_t b) {
                 const __half2 h = __floats2half2_rn(__uint_as_float(a) * factor, __uint_as_float(b) * factor);
                 return *reinterpret_cast<const uint32_t *>(&h);
@@ -538,7 +577,6 @@ __global__ void __launch_bounds__(PREPARE_THREADS) prepare_activations_kernel(co
         }
         *reinterpret_cast<uint4 *>(out + (static_cast<size_t>(p >> 3) * lane_blocks + (m >> 3)) * 1024 + (m & 7) * 128 + (((p & 7) ^ (m & 7)) * 16)) = packed;
     }
-    grid_launch_dependents();
 }
 
 struct GemmPlan {
@@ -622,31 +660,24 @@ static float *activation_factors(void *prepared, int lanes, int k) {
     return reinterpret_cast<float *>(static_cast<uint8_t *>(prepared) + padded * k * 2);
 }
 
-// Launch with the programmatic-dependent-launch attribute (and a cluster over the K splits).
-template <typename... Parameters, typename... Arguments>
-static cudaError_t launch_dependent(void (*kernel)(Parameters...), dim3 grid, int threads, size_t smem, int cluster, cudaStream_t stream, Arguments... arguments) {
-    cudaLaunchConfig_t config = {};
-    config.gridDim = grid;
-    config.blockDim = dim3(threads);
-    config.dynamicSmemBytes = smem;
-    config.stream = stream;
-    cudaLaunchAttribute attributes[2];
-    attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attributes[0].val.programmaticStreamSerializationAllowed = 1;
-    attributes[1].id = cudaLaunchAttributeClusterDimension;
-    attributes[1].val.clusterDim.x = 1;
-    attributes[1].val.clusterDim.y = 1;
-    attributes[1].val.clusterDim.z = static_cast<unsigned int>(cluster);
-    config.attrs = attributes;
-    config.numAttrs = cluster > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&config, kernel, Parameters(arguments)...);
-}
-
 cudaError_t launch_prepare_activations(const uint16_t *x, void *prepared, int lanes, int k, cudaStream_t stream) {
     if (lanes <= 0) return cudaSuccess;
     const int padded = (lanes + 15) / 16 * 16;
-    return launch_dependent(prepare_activations_kernel, dim3(padded), PREPARE_THREADS, 0, 1, stream, x, static_cast<uint8_t *>(prepared),
-                            activation_factors(prepared, lanes, k), lanes, padded / 8, k);
+    return launch_dependent(prepare_activations_kernel<false>, dim3(padded), dim3(PREPARE_THREADS), 0, 1, stream, x, static_cast<const uint16_t *>(nullptr), 0.0f,
+                            0.0f, static_cast<uint8_t *>(prepared), activation_factors(prepared, lanes, k), lanes, padded / 8, k);
+}
+
+cudaError_t launch_rms_norm_prepared(const uint16_t *x, const uint16_t *weight, void *prepared, int lanes, int width, float eps, float weight_offset,
+                                     cudaStream_t stream) {
+    if (lanes <= 0) return cudaSuccess;
+    const int padded = (lanes + 15) / 16 * 16;
+    const size_t smem = static_cast<size_t>(width) * 2;
+    if (smem > 48 * 1024) {
+        cudaError_t status = cudaFuncSetAttribute(prepare_activations_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (status != cudaSuccess) return status;
+    }
+    return launch_dependent(prepare_activations_kernel<true>, dim3(padded), dim3(PREPARE_THREADS), smem, 1, stream, x, weight, eps, weight_offset,
+                            static_cast<uint8_t *>(prepared), activation_factors(prepared, lanes, width), lanes, padded / 8, width);
 }
 
 cudaError_t launch_linear_int4_gemm(const void *prepared, int branches, const uint32_t *const *qweights, const uint16_t *const *scales, void *const *ys,
@@ -692,7 +723,7 @@ cudaError_t launch_linear_int4_gemm(const void *prepared, int branches, const ui
     auto kernel = plan.row_tiles == 2 ? linear_int4_gemm_kernel<2> : linear_int4_gemm_kernel<1>;
     cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(GEMM_SMEM_ONE + GEMM_TAIL_BYTES));
     if (status != cudaSuccess) return status;
-    return launch_dependent(kernel, grid, plan.row_tiles == 2 ? gemm_threads<2>() : gemm_threads<1>(), plan.smem + GEMM_TAIL_BYTES, plan.splits, stream, args);
+    return launch_dependent(kernel, grid, dim3(plan.row_tiles == 2 ? gemm_threads<2>() : gemm_threads<1>()), plan.smem + GEMM_TAIL_BYTES, plan.splits, stream, args);
 }
 
 }  // namespace nerve
