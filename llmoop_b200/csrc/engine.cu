@@ -526,6 +526,21 @@ Engine::Engine(std::shared_ptr<MountedModel> model) : model_(std::move(model)) {
     };
     for (const ComponentPlan &layer : plan.layers) widest(layer);
     for (const ComponentPlan &layer : plan.draft_layers) widest(layer);
+    size_t moe_values = 0, moe_bytes = 0;
+    auto experts = [&](const ComponentPlan &component) {
+        for (const OpSpec &op : component.ops)
+            if (op.kind == OpKind::MoeGateUp || op.kind == OpKind::MoeDown) {
+                moe_values = std::max(moe_values, lanes * (op.kind == OpKind::MoeGateUp ? op.moe_hidden : op.top_k * op.moe_inter));
+                moe_bytes = std::max(moe_bytes, moe_group_bytes(options.max_lanes, op.top_k, op.experts));
+            }
+    };
+    for (const ComponentPlan &layer : plan.layers) experts(layer);
+    for (const ComponentPlan &layer : plan.draft_layers) experts(layer);
+    if (moe_values > 0) {
+        moe_quantised_ = device_alloc(moe_values);
+        moe_quantised_scales_ = device_alloc((moe_values + 127) / 128 * sizeof(float));
+        moe_groups_ = device_alloc(moe_bytes);
+    }
     if (int4_columns > 0) int4_activations_ = device_alloc(int4_activation_bytes(options.max_lanes, static_cast<int>(int4_columns)));
 
     frame_a_ = device_alloc(lanes * frame);
@@ -616,7 +631,7 @@ Engine::~Engine() {
     for (auto &entry : signals_) cudaFree(entry.second.ptr);
     for (DeviceBuffer *buffer : {&frame_a_, &frame_b_, &embedding_out_, &normalized_, &draft_normalized_, &draft_hidden_in_, &logits_,
                                  &records_, &argmax_scratch_, &sampler_scratch_, &sampler_table_, &lane_tokens_, &lane_positions_, &lane_slots_, &pending_hidden_, &pending_backup_, &attention_scratch_,
-                                 &cycle_state_, &int4_activations_, &kernel_error_, &tp_partial_, &tp_exchange_, &tp_description_, &stack_q_, &stack_attention_out_, &stack_activation_, &stack_barrier_, &stack_timing_, &prefix_pending_})
+                                 &cycle_state_, &int4_activations_, &moe_quantised_, &moe_quantised_scales_, &moe_groups_, &kernel_error_, &tp_partial_, &tp_exchange_, &tp_description_, &stack_q_, &stack_attention_out_, &stack_activation_, &stack_barrier_, &stack_timing_, &prefix_pending_})
         cudaFree(buffer->ptr);
     cudaFreeHost(staging_);
     cudaFreeHost(host_records_);
@@ -1192,7 +1207,7 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
     };
     // The activations of an INT4 linear of more than eight lanes in the GEMM's operand form: prepared once per signal,
     // whichever linears read it.
-    std::string prepared_signal;
+    std::string prepared_signal, grouped_signal;
     auto prepared = [&](const std::string &signal) -> const void * {
         if (lanes <= 8) return nullptr;
         if (prepared_signal != signal) {
@@ -1486,22 +1501,29 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
         case OpKind::MoeTopk:
             check(launch_moe_topk(u16(op.inputs[0]), static_cast<uint32_t *>(ptr(op.outputs[0])), lanes, op.experts, op.top_k, st), "moe_topk");
             break;
-        case OpKind::MoeGateUp: {
-            const WeightRef &w = op.weights[0];
-            if (w.storage != TensorStorage::FP8_BLOCK) fail("only FP8 expert weights are mounted");
-            check(launch_moe_gate_up_fp8(u16(op.inputs[0]), static_cast<const uint32_t *>(ptr(op.inputs[1])),
-                                         static_cast<const uint8_t *>(weight(w.tensor)), static_cast<const uint16_t *>(weight(w.scale)),
-                                         u16(op.outputs[0]), lanes, op.moe_hidden, op.moe_inter, op.experts, op.top_k, 0, op.experts, st),
-                  "sparse_moe_gate_up");
-            break;
-        }
+        case OpKind::MoeGateUp:
         case OpKind::MoeDown: {
             const WeightRef &w = op.weights[0];
             if (w.storage != TensorStorage::FP8_BLOCK) fail("only FP8 expert weights are mounted");
-            check(launch_moe_down_fp8(u16(op.inputs[0]), static_cast<const uint32_t *>(ptr(op.inputs[1])),
-                                      static_cast<const uint8_t *>(weight(w.tensor)), static_cast<const uint16_t *>(weight(w.scale)),
-                                      u16(op.outputs[0]), lanes, op.moe_hidden, op.moe_inter, op.experts, op.top_k, 0, op.experts, st),
-                  "sparse_moe_down");
+            // the experts' tiles (once per routing) and the quantised input: a frame per lane, or one per (lane, route)
+            const MoeGroups groups = moe_groups(moe_groups_.ptr, model_->options().max_lanes, op.top_k, op.experts);
+            if (grouped_signal != op.inputs[1]) {
+                check(launch_moe_group(static_cast<const uint32_t *>(ptr(op.inputs[1])), groups, lanes, op.top_k, op.experts, 0, op.experts, st), "moe_group");
+                grouped_signal = op.inputs[1];
+            }
+            const bool gate_up = op.kind == OpKind::MoeGateUp;
+            uint8_t *xq = static_cast<uint8_t *>(moe_quantised_.ptr);
+            float *xscale = static_cast<float *>(moe_quantised_scales_.ptr);
+            check(launch_quantize_fp8(u16(op.inputs[0]), xq, xscale, gate_up ? lanes : lanes * op.top_k, gate_up ? op.moe_hidden : op.moe_inter, st), "expert input");
+            if (gate_up)
+                check(launch_moe_gate_up_fp8(xq, xscale, groups, static_cast<const uint8_t *>(weight(w.tensor)), static_cast<const uint16_t *>(weight(w.scale)),
+                                             u16(op.outputs[0]), lanes, op.moe_hidden, op.moe_inter, op.experts, op.top_k, 0, st),
+                      "sparse_moe_gate_up");
+            else
+                check(launch_moe_down_fp8(xq, xscale, groups, static_cast<const uint32_t *>(ptr(op.inputs[1])), static_cast<const uint8_t *>(weight(w.tensor)),
+                                          static_cast<const uint16_t *>(weight(w.scale)), u16(op.outputs[0]), lanes, op.moe_hidden, op.moe_inter, op.experts,
+                                          op.top_k, 0, st),
+                      "sparse_moe_down");
             break;
         }
         case OpKind::MoeReduce:

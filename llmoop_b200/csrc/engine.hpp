@@ -368,6 +368,7 @@ private:
     DeviceBuffer attention_scratch_;
     DeviceBuffer kernel_error_;             // device word set by pipelined kernels whose bounded waits expired
     DeviceBuffer int4_activations_;         // the INT4 GEMM's operand form of one signal (more than eight lanes)
+    DeviceBuffer moe_quantised_, moe_quantised_scales_, moe_groups_;  // FP8 input of the expert kernels, the experts' tiles
     DeviceBuffer tp_partial_;               // f32 [max_lanes][hidden] partial sums of row-parallel linears
     void *nccl_library_ = nullptr, *nccl_comm_ = nullptr;
     DeviceBuffer tp_exchange_;              // this rank's exchange buffer + arrival counter + consumed-arrivals word

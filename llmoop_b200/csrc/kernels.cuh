@@ -80,13 +80,23 @@ cudaError_t launch_linear_silu_multiply_fp8(const uint8_t *xq, const float *xsca
 // MoE (softmax over the selected experts, routes sorted by expert id).
 cudaError_t launch_moe_topk(const uint16_t *router_logits, uint32_t *routes, int lanes, int experts, int top_k,
                             cudaStream_t stream);
-cudaError_t launch_moe_gate_up_fp8(const uint16_t *hidden, const uint32_t *routes, const uint8_t *w,
+// The (token, route) pairs of a batch grouped by expert, up to eight of one expert to a tile.
+struct MoeGroups {
+    int4 *tiles;      // {expert, first place in order, count, 0}
+    int *order;       // pair = token * top_k + route
+    int *tile_count;
+};
+size_t moe_group_bytes(int lanes, int top_k, int experts);
+MoeGroups moe_groups(void *scratch, int lanes, int top_k, int experts);  // carves moe_group_bytes bytes
+cudaError_t launch_moe_group(const uint32_t *routes, const MoeGroups &groups, int lanes, int top_k, int experts, int expert_start, int expert_count,
+                             cudaStream_t stream);
+// xq / xscale: the hidden frames [lanes], or the intermediates [lanes * top_k], as launch_quantize_fp8 writes them.
+cudaError_t launch_moe_gate_up_fp8(const uint8_t *xq, const float *xscale, const MoeGroups &groups, const uint8_t *w,
                                    const uint16_t *wscale, uint16_t *intermediates, int lanes, int hidden_size,
-                                   int inter, int experts, int top_k, int expert_start, int expert_count,
-                                   cudaStream_t stream);
-cudaError_t launch_moe_down_fp8(const uint16_t *intermediates, const uint32_t *routes, const uint8_t *w,
+                                   int inter, int experts, int top_k, int expert_start, cudaStream_t stream);
+cudaError_t launch_moe_down_fp8(const uint8_t *xq, const float *xscale, const MoeGroups &groups, const uint32_t *routes, const uint8_t *w,
                                 const uint16_t *wscale, uint16_t *outputs, int lanes, int hidden_size, int inter,
-                                int experts, int top_k, int expert_start, int expert_count, cudaStream_t stream);
+                                int experts, int top_k, int expert_start, cudaStream_t stream);
 cudaError_t launch_moe_reduce(const uint16_t *outputs, uint16_t *y, int lanes, int hidden_size, int top_k,
                               float routed_scale, cudaStream_t stream);
 

@@ -5,6 +5,7 @@
 // verify batch (<= 160 lanes) fills the SMs with one CTA per lane (x head).
 #include "common.cuh"
 #include "kernels.cuh"
+#include "launch.cuh"
 
 namespace nerve {
 
@@ -12,6 +13,7 @@ namespace nerve {
 // token id >= vocab leaves the frame untouched.
 __global__ void embedding_kernel(const uint32_t *__restrict__ table, const uint32_t *__restrict__ tokens,
                                  uint32_t *__restrict__ out, int width_words, int vocab, float scale) {
+    grid_launch_dependents();
     grid_dependency_wait();
     int lane = blockIdx.y;
     uint32_t token = tokens[lane];
@@ -26,14 +28,13 @@ cudaError_t launch_embedding(const uint16_t *table, const uint32_t *tokens, uint
                              int vocab, float scale, cudaStream_t stream) {
     int words = width / 2;
     dim3 grid((words + 255) / 256, lanes);
-    embedding_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<const uint32_t *>(table), tokens,
-                                               reinterpret_cast<uint32_t *>(out), words, vocab, scale);
-    return cudaGetLastError();
+    return launch_dependent(embedding_kernel, grid, dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(table), tokens, reinterpret_cast<uint32_t *>(out), words, vocab, scale);
 }
 
 // rms_norm_bf16.comp.template:49-72: y = bf16(x * rsqrt(mean(x^2) + eps) * (w + offset)), f32 math.
 __global__ void rms_norm_kernel(const uint32_t *__restrict__ x, const uint32_t *__restrict__ weight,
                                 uint32_t *__restrict__ y, int width_words, float inv_width, float eps, float offset) {
+    grid_launch_dependents();
     grid_dependency_wait();
     __shared__ float partial[32];
     const uint32_t *row = x + static_cast<size_t>(blockIdx.x) * width_words;
@@ -63,16 +64,13 @@ cudaError_t launch_rms_norm(const uint16_t *x, const uint16_t *weight, uint16_t 
                             float weight_offset, cudaStream_t stream) {
     int words = width / 2;
     int threads = words >= 1024 ? 512 : (words >= 256 ? 256 : (words >= 64 ? 64 : 32));
-    rms_norm_kernel<<<lanes, threads, 0, stream>>>(reinterpret_cast<const uint32_t *>(x),
-                                                   reinterpret_cast<const uint32_t *>(weight),
-                                                   reinterpret_cast<uint32_t *>(y), words, 1.0f / static_cast<float>(width),
-                                                   eps, weight_offset);
-    return cudaGetLastError();
+    return launch_dependent(rms_norm_kernel, dim3(lanes), dim3(threads), 0, 1, stream, reinterpret_cast<const uint32_t *>(x), reinterpret_cast<const uint32_t *>(weight), reinterpret_cast<uint32_t *>(y), words, 1.0f / static_cast<float>(width), eps, weight_offset);
 }
 
 // add_bf16.comp.template:17-24
 __global__ void add_kernel(const uint32_t *__restrict__ a, const uint32_t *__restrict__ b, uint32_t *__restrict__ y,
                            size_t words) {
+    grid_launch_dependents();
     grid_dependency_wait();
     for (size_t word = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; word < words;
          word += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -86,15 +84,15 @@ cudaError_t launch_add(const uint16_t *a, const uint16_t *b, uint16_t *y, size_t
     int blocks = static_cast<int>((words + 255) / 256);
     if (blocks > 148 * 8) blocks = 148 * 8;
     if (blocks < 1) blocks = 1;
-    add_kernel<<<blocks, 256, 0, stream>>>(reinterpret_cast<const uint32_t *>(a), reinterpret_cast<const uint32_t *>(b),
-                                           reinterpret_cast<uint32_t *>(y), words);
-    return cudaGetLastError();
+    return launch_dependent(add_kernel, dim3(blocks), dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(a), reinterpret_cast<const uint32_t *>(b), reinterpret_cast<uint32_t *>(y), words);
 }
 
 // After the tensor-parallel all-reduce of a row-parallel linear: the reference's linear rounds its f32 sum to bf16
 // and its residual_add rounds again (add_bf16.comp.template:17-24).
 __global__ void round_add_kernel(const float *__restrict__ sums, const uint16_t *__restrict__ residual, uint16_t *__restrict__ out,
                                  size_t count) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     for (size_t index = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; index < count;
          index += static_cast<size_t>(gridDim.x) * blockDim.x) {
         float value = round_bf16(sums[index]);
@@ -107,13 +105,13 @@ cudaError_t launch_round_add(const float *sums, const uint16_t *residual, uint16
     int blocks = static_cast<int>((count + 255) / 256);
     if (blocks > 148 * 8) blocks = 148 * 8;
     if (blocks < 1) blocks = 1;
-    round_add_kernel<<<blocks, 256, 0, stream>>>(sums, residual, out, count);
-    return cudaGetLastError();
+    return launch_dependent(round_add_kernel, dim3(blocks), dim3(256), 0, 1, stream, sums, residual, out, count);
 }
 
 // silu_multiply_bf16.comp.template:30-52: bf16(bf16(silu(gate)) * up)
 __global__ void silu_multiply_kernel(const uint32_t *__restrict__ gate, const uint32_t *__restrict__ up,
                                      uint32_t *__restrict__ y, size_t words) {
+    grid_launch_dependents();
     grid_dependency_wait();
     for (size_t word = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; word < words;
          word += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -128,15 +126,13 @@ cudaError_t launch_silu_multiply(const uint16_t *gate, const uint16_t *up, uint1
     int blocks = static_cast<int>((words + 255) / 256);
     if (blocks > 148 * 8) blocks = 148 * 8;
     if (blocks < 1) blocks = 1;
-    silu_multiply_kernel<<<blocks, 256, 0, stream>>>(reinterpret_cast<const uint32_t *>(gate),
-                                                     reinterpret_cast<const uint32_t *>(up),
-                                                     reinterpret_cast<uint32_t *>(y), words);
-    return cudaGetLastError();
+    return launch_dependent(silu_multiply_kernel, dim3(blocks), dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(gate), reinterpret_cast<const uint32_t *>(up), reinterpret_cast<uint32_t *>(y), words);
 }
 
 // concatenate_bf16.comp.template:20-30 (per lane: [a | b])
 __global__ void concat_kernel(const uint32_t *__restrict__ a, const uint32_t *__restrict__ b, uint32_t *__restrict__ y,
                               int words_a, int words_b) {
+    grid_launch_dependents();
     grid_dependency_wait();
     int lane = blockIdx.x;
     int total = words_a + words_b;
@@ -147,9 +143,7 @@ __global__ void concat_kernel(const uint32_t *__restrict__ a, const uint32_t *__
 
 cudaError_t launch_concat(const uint16_t *a, const uint16_t *b, uint16_t *y, int lanes, int width_a, int width_b,
                           cudaStream_t stream) {
-    concat_kernel<<<lanes, 256, 0, stream>>>(reinterpret_cast<const uint32_t *>(a), reinterpret_cast<const uint32_t *>(b),
-                                             reinterpret_cast<uint32_t *>(y), width_a / 2, width_b / 2);
-    return cudaGetLastError();
+    return launch_dependent(concat_kernel, dim3(lanes), dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(a), reinterpret_cast<const uint32_t *>(b), reinterpret_cast<uint32_t *>(y), width_a / 2, width_b / 2);
 }
 
 // rotary_bf16.comp.template:99-109 (five bf16 roundings per element) with
@@ -160,6 +154,7 @@ cudaError_t launch_concat(const uint16_t *a, const uint16_t *b, uint16_t *y, int
 __global__ void rope_kernel(const uint16_t *__restrict__ x, uint16_t *__restrict__ y, const uint32_t *__restrict__ cos_sin,
                             uint32_t table_positions, const uint32_t *__restrict__ positions, int heads, int head_width,
                             int rotary, int interleaved, const uint16_t *__restrict__ norm_weight, float eps, float offset) {
+    grid_launch_dependents();
     grid_dependency_wait();
     extern __shared__ float values[];  // head_width normalised (or raw) inputs as f32
     __shared__ float partial[32];
@@ -210,16 +205,14 @@ cudaError_t launch_rope(const uint16_t *x, uint16_t *y, const uint32_t *cos_sin,
     int threads = ((head_width / 2 + 31) / 32) * 32;
     if (threads > 256) threads = 256;
     dim3 grid(heads, lanes);
-    rope_kernel<<<grid, threads, head_width * sizeof(float), stream>>>(x, y, cos_sin, table_positions, positions, heads,
-                                                                       head_width, rotary, interleaved, norm_weight, eps,
-                                                                       weight_offset);
-    return cudaGetLastError();
+    return launch_dependent(rope_kernel, grid, dim3(threads), head_width * sizeof(float), 1, stream, x, y, cos_sin, table_positions, positions, heads, head_width, rotary, interleaved, norm_weight, eps, weight_offset);
 }
 
 // quantize_fp8_e4m3.comp.template:41-60: per 128-column block scale = absmax/448
 // (1 when the block is all zero), q = e4m3(x / scale).  One warp per block.
 __global__ void quantize_fp8_kernel(const uint32_t *__restrict__ x, uint32_t *__restrict__ q, float *__restrict__ scales,
                                     int blocks_total) {
+    grid_launch_dependents();
     grid_dependency_wait();
     int block = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (block >= blocks_total) return;
@@ -241,9 +234,7 @@ __global__ void quantize_fp8_kernel(const uint32_t *__restrict__ x, uint32_t *__
 cudaError_t launch_quantize_fp8(const uint16_t *x, uint8_t *q, float *scales, int lanes, int k, cudaStream_t stream) {
     int blocks_total = lanes * (k / 128);
     int warps_per_cta = 8;
-    quantize_fp8_kernel<<<(blocks_total + warps_per_cta - 1) / warps_per_cta, warps_per_cta * 32, 0, stream>>>(
-        reinterpret_cast<const uint32_t *>(x), reinterpret_cast<uint32_t *>(q), scales, blocks_total);
-    return cudaGetLastError();
+    return launch_dependent(quantize_fp8_kernel, dim3((blocks_total + warps_per_cta - 1) / warps_per_cta), dim3(warps_per_cta * 32), 0, 1, stream, reinterpret_cast<const uint32_t *>(x), reinterpret_cast<uint32_t *>(q), scales, blocks_total);
 }
 
 // moe_topk_bf16.comp.template:42-84.  One warp per lane: top_k rounds of
@@ -252,6 +243,7 @@ cudaError_t launch_quantize_fp8(const uint16_t *x, uint8_t *q, float *scales, in
 // word = bf16(weight) << 16 | expert.
 __global__ void moe_topk_kernel(const uint16_t *__restrict__ router_logits, uint32_t *__restrict__ routes, int experts,
                                 int top_k) {
+    grid_launch_dependents();
     grid_dependency_wait();
     int token = blockIdx.x;
     int lane = threadIdx.x;
@@ -309,14 +301,14 @@ __global__ void moe_topk_kernel(const uint16_t *__restrict__ router_logits, uint
 cudaError_t launch_moe_topk(const uint16_t *router_logits, uint32_t *routes, int lanes, int experts, int top_k,
                             cudaStream_t stream) {
     if (top_k > 64) return cudaErrorInvalidValue;
-    moe_topk_kernel<<<lanes, 32, 0, stream>>>(router_logits, routes, experts, top_k);
-    return cudaGetLastError();
+    return launch_dependent(moe_topk_kernel, dim3(lanes), dim3(32), 0, 1, stream, router_logits, routes, experts, top_k);
 }
 
 // moe_reduce_bf16.comp.template:28-45: bf16-rounded running sum over the routes
 // in route (expert-id) order, then * routed scale.
 __global__ void moe_reduce_kernel(const uint32_t *__restrict__ outputs, uint32_t *__restrict__ y, int hidden_words,
                                   int top_k, float routed_scale) {
+    grid_launch_dependents();
     grid_dependency_wait();
     int token = blockIdx.x;
     for (int word = threadIdx.x; word < hidden_words; word += blockDim.x) {
@@ -332,9 +324,7 @@ __global__ void moe_reduce_kernel(const uint32_t *__restrict__ outputs, uint32_t
 
 cudaError_t launch_moe_reduce(const uint16_t *outputs, uint16_t *y, int lanes, int hidden_size, int top_k,
                               float routed_scale, cudaStream_t stream) {
-    moe_reduce_kernel<<<lanes, 256, 0, stream>>>(reinterpret_cast<const uint32_t *>(outputs),
-                                                 reinterpret_cast<uint32_t *>(y), hidden_size / 2, top_k, routed_scale);
-    return cudaGetLastError();
+    return launch_dependent(moe_reduce_kernel, dim3(lanes), dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(outputs), reinterpret_cast<uint32_t *>(y), hidden_size / 2, top_k, routed_scale);
 }
 
 }  // namespace nerve

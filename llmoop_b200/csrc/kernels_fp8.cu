@@ -1,0 +1,482 @@
+// FP8 (e4m3, block-scaled) linears and sparse experts.
+//
+// Arithmetic (linear_prequant_fp8_e4m3.comp.template:69-120, sparse_moe_gate_up_fp8_e4m3.comp.template:94-198,
+// sparse_moe_down_fp8_e4m3.comp.template:90-176): per 4 columns an f32 dot of e4m3 values, fma'd with
+// act_scale * weight_scale.  The order of additions is fixed: column group l (columns 4 l .. 4 l + 3 of every block of
+// 128) is added up over the blocks in order, then the 32 groups in a butterfly (distance 16, 8, 4, 2, 1).  The outputs
+// are requantised to FP8 by the next linear and feed the choice of experts, where a last-bit difference of a sum becomes
+// a step of a sixteenth or another expert, so no form of these kernels departs from that order - which leaves the work
+// to the FP32 pipe (a tensor-core sum would add the groups in another order).
+//
+// A warp computes ROWS x M outputs: thread l owns column group l, keeps ROWS x M partial sums in registers and walks the
+// blocks; weights come straight from global memory (one coalesced 128-byte row piece per warp and block, requested
+// PIPE blocks ahead), the activations as f32 from shared memory, two lanes to a packed f32x2 operand.  Per block and
+// warp: 5 FP32 operations per weight word and lane against 6 conversions per weight word, so from eight lanes on the
+// FP32 pipe is the bound (1024 lanes x 2048 x 4096: 480 us with one row and eight lanes per warp, the form this
+// replaced), below that the weight bytes.
+// Sparse experts are grouped: a small kernel sorts the (token, route) pairs by expert into tiles of up to eight, and an
+// expert's rows are read once per tile instead of once per pair.
+#include <cstdlib>
+
+#include "common.cuh"
+#include "kernels.cuh"
+#include "launch.cuh"
+
+namespace nerve {
+
+namespace {
+
+constexpr int FP8_WARPS = 8, FP8_ROWS = 8, TILE_LANES = 8;
+constexpr int CHUNK = 16;  // blocks of 128 columns whose activations are staged at a time: 64 KB for eight lanes, two CTAs per SM
+
+using pair_t = unsigned long long;  // two f32
+__device__ __forceinline__ pair_t pack(float lo, float hi) {
+    pair_t out;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(out) : "f"(lo), "f"(hi));
+    return out;
+}
+__device__ __forceinline__ float2 unpack(pair_t v) {
+    float2 out;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(out.x), "=f"(out.y) : "l"(v));
+    return out;
+}
+__device__ __forceinline__ pair_t mul(pair_t a, pair_t b) {
+    pair_t out;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(out) : "l"(a), "l"(b));
+    return out;
+}
+__device__ __forceinline__ pair_t fma2(pair_t a, pair_t b, pair_t c) {
+    pair_t out;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(out) : "l"(a), "l"(b), "l"(c));
+    return out;
+}
+// four e4m3 values of a word as f32, exact
+__device__ __forceinline__ void widen(uint32_t word, float (&out)[4]) {
+    uint32_t lo, hi;
+    asm("{\n.reg .b16 a, b;\nmov.b32 {a, b}, %2;\ncvt.rn.f16x2.e4m3x2 %0, a;\ncvt.rn.f16x2.e4m3x2 %1, b;\n}\n" : "=r"(lo), "=r"(hi) : "r"(word));
+    const float2 first = __half22float2(*reinterpret_cast<const __half2 *>(&lo)), second = __half22float2(*reinterpret_cast<const __half2 *>(&hi));
+    out[0] = first.x;
+    out[1] = first.y;
+    out[2] = second.x;
+    out[3] = second.y;
+}
+
+// The activations of up to M lanes (rows of xq / xscale picked by `row_of`) in shared memory:
+// x [block][lane pair][column pair][thread][column of the pair][lane of the pair] f32, scales [block][M].
+template <int M>
+__device__ __forceinline__ size_t x_index(int block, int pair, int half, int thread) {
+    return ((static_cast<size_t>(block) * (M / 2) + pair) * 2 + half) * 128 + thread * 4;
+}
+template <int M, typename RowOf>
+__device__ __forceinline__ void stage_activations(const uint8_t *__restrict__ xq, const float *__restrict__ xscale, int k, int first, int blocks, int count, float *x,
+                                                  RowOf row_of) {
+    const int words = blocks * 32, all_blocks = k >> 7;
+    float *scales = x + static_cast<size_t>(CHUNK) * 128 * M;
+    for (int index = threadIdx.x; index < words * (M / 2); index += FP8_WARPS * 32) {
+        const int pair = index / words, word = index - pair * words, block = word >> 5, thread = word & 31;
+        float lo[4] = {}, hi[4] = {};
+        if (2 * pair < count) widen(reinterpret_cast<const uint32_t *>(xq + static_cast<size_t>(row_of(2 * pair)) * k)[first * 32 + word], lo);
+        if (2 * pair + 1 < count) widen(reinterpret_cast<const uint32_t *>(xq + static_cast<size_t>(row_of(2 * pair + 1)) * k)[first * 32 + word], hi);
+        *reinterpret_cast<float4 *>(x + x_index<M>(block, pair, 0, thread)) = make_float4(lo[0], hi[0], lo[1], hi[1]);
+        *reinterpret_cast<float4 *>(x + x_index<M>(block, pair, 1, thread)) = make_float4(lo[2], hi[2], lo[3], hi[3]);
+    }
+    for (int index = threadIdx.x; index < blocks * M; index += FP8_WARPS * 32) {
+        const int m = index % M, block = index / M;
+        scales[index] = m < count ? xscale[static_cast<size_t>(row_of(m)) * all_blocks + first + block] : 0.0f;
+    }
+}
+
+// Sums of FP8_ROWS rows x M lanes over all of K; rows 0..3 and 4..7 may have scale rows of their own (gate and up).
+// On return thread t holds the outputs sum_index(t, i), i < FP8_ROWS * M / 32 (or the one of its thread pair for M = 2).
+template <int M>
+struct RowSums {
+    static constexpr int VALUES = FP8_ROWS * M, PER_THREAD = VALUES >= 32 ? VALUES / 32 : 1;
+    static constexpr int PIPE = M == 8 ? 1 : 4;  // blocks of weights in flight: eight lanes are bound by arithmetic, not latency
+    float sums[PER_THREAD];
+
+    // output index = row * M + lane
+    __device__ static int index(int thread, int i) {
+        if (VALUES >= 32) return ((thread >> 4) & 1) * (VALUES / 2) + ((thread >> 3) & 1) * (VALUES / 4) + ((thread >> 2) & 1) * (VALUES / 8) +
+                                 ((thread >> 1) & 1) * (VALUES / 16) + (thread & 1) * (VALUES / 32) + i;
+        return thread >> 1;  // sixteen values: the last butterfly step leaves both threads of a pair with the same one
+    }
+
+    // stage(first, n) brings the activations of blocks first .. first + n - 1 into x
+    template <typename RowPointer, typename Stage>
+    __device__ void run(RowPointer row_pointer, const uint16_t *__restrict__ scales_a, const uint16_t *__restrict__ scales_b, int blocks, float *x, Stage stage_blocks) {
+        const float *x_scales = x + static_cast<size_t>(CHUNK) * 128 * M;
+        const int thread = threadIdx.x & 31;
+        const uint32_t *source[FP8_ROWS];
+#pragma unroll
+        for (int r = 0; r < FP8_ROWS; r++) source[r] = reinterpret_cast<const uint32_t *>(row_pointer(r)) + thread;
+        uint32_t words[PIPE][FP8_ROWS];
+#pragma unroll
+        for (int p = 0; p < PIPE; p++)
+#pragma unroll
+            for (int r = 0; r < FP8_ROWS; r++) words[p][r] = p < blocks ? __ldg(source[r] + p * 32) : 0u;
+        pair_t acc[FP8_ROWS][M / 2];
+#pragma unroll
+        for (int r = 0; r < FP8_ROWS; r++)
+#pragma unroll
+            for (int p = 0; p < M / 2; p++) acc[r][p] = 0ull;
+        for (int base = 0; base < blocks; base += PIPE) {
+            if (base % CHUNK == 0) {
+                if (base > 0) __syncthreads();
+                stage_blocks(base, min(CHUNK, blocks - base));
+                __syncthreads();
+            }
+#pragma unroll
+            for (int stage = 0; stage < PIPE; stage++) {
+                const int block = base + stage, staged = block % CHUNK;
+                if (block >= blocks) break;
+                const float wa = bf16_bits_to_f32(__ldg(scales_a + block)), wb = bf16_bits_to_f32(__ldg(scales_b + block));
+                pair_t xv[M / 2][4], sa[M / 2], sb[M / 2];
+#pragma unroll
+                for (int p = 0; p < M / 2; p++) {
+                    const ulonglong2 first = *reinterpret_cast<const ulonglong2 *>(x + x_index<M>(staged, p, 0, thread));
+                    const ulonglong2 second = *reinterpret_cast<const ulonglong2 *>(x + x_index<M>(staged, p, 1, thread));
+                    xv[p][0] = first.x;
+                    xv[p][1] = first.y;
+                    xv[p][2] = second.x;
+                    xv[p][3] = second.y;
+                    const pair_t xs = *reinterpret_cast<const pair_t *>(x_scales + staged * M + 2 * p);
+                    sa[p] = mul(xs, pack(wa, wa));
+                    sb[p] = mul(xs, pack(wb, wb));
+                }
+#pragma unroll
+                for (int r = 0; r < FP8_ROWS; r++) {
+                    float w[4];
+                    widen(words[stage][r], w);
+                    const pair_t w2[4] = {pack(w[0], w[0]), pack(w[1], w[1]), pack(w[2], w[2]), pack(w[3], w[3])};
+#pragma unroll
+                    for (int p = 0; p < M / 2; p++) {
+                        pair_t d = mul(xv[p][0], w2[0]);
+                        d = fma2(xv[p][1], w2[1], d);
+                        d = fma2(xv[p][2], w2[2], d);
+                        d = fma2(xv[p][3], w2[3], d);
+                        acc[r][p] = fma2(d, r < FP8_ROWS / 2 ? sa[p] : sb[p], acc[r][p]);
+                    }
+                    words[stage][r] = block + PIPE < blocks ? __ldg(source[r] + (block + PIPE) * 32) : 0u;
+                }
+            }
+        }
+        // butterfly over the threads: at every step a thread keeps half of its values and passes on the other half
+        float v[VALUES];
+#pragma unroll
+        for (int r = 0; r < FP8_ROWS; r++)
+#pragma unroll
+            for (int p = 0; p < M / 2; p++) {
+                const float2 both = unpack(acc[r][p]);
+                v[r * M + 2 * p] = both.x;
+                v[r * M + 2 * p + 1] = both.y;
+            }
+#pragma unroll
+        for (int step = 0; step < 5; step++) {
+            const int offset = 16 >> step, live = VALUES >> step, half = live / 2;
+            if (live > 1) {
+                const bool upper = (thread & offset) != 0;
+#pragma unroll
+                for (int i = 0; i < half; i++) {
+                    const float keep = upper ? v[half + i] : v[i], send = upper ? v[i] : v[half + i];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, offset);
+                }
+            } else {
+                v[0] = v[0] + __shfl_xor_sync(0xffffffffu, v[0], offset);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < PER_THREAD; i++) sums[i] = v[i];
+    }
+};
+
+// M lanes of a tile: the smallest form that holds them
+template <typename Two, typename Four, typename Eight>
+__device__ __forceinline__ void by_count(int count, Two two, Four four, Eight eight) {
+    if (count <= 2) two();
+    else if (count <= 4) four();
+    else eight();
+}
+
+struct Fp8LinearArgs {
+    const uint8_t *xq;
+    const float *xscale;
+    const uint8_t *w[2];  // a SiLU pair: gate, up
+    const uint16_t *wscale[2];
+    uint16_t *y;
+    const uint16_t *residual;
+    int lanes, n, k, epilogue;
+};
+
+template <int M>
+__device__ __forceinline__ void fp8_linear_tile(const Fp8LinearArgs &a, int m0, int count, float *smem) {
+    const int warp = threadIdx.x >> 5, thread = threadIdx.x & 31, blocks = a.k >> 7;
+    auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, a.k, first, n, count, smem, [&](int m) { return m0 + m; }); };
+    const int row0 = (blockIdx.x * FP8_WARPS + warp) * FP8_ROWS;
+    RowSums<M> sums;
+    const uint16_t *scale_row[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) scale_row[h] = a.wscale[0] + static_cast<size_t>(min(row0 + 4 * h, a.n - 1) >> 7) * blocks;
+    sums.run([&](int r) { return a.w[0] + static_cast<size_t>(min(row0 + r, a.n - 1)) * a.k; }, scale_row[0], scale_row[1], blocks, smem, stage);
+    if (RowSums<M>::VALUES < 32 && (thread & 1) != 0) return;
+#pragma unroll
+    for (int i = 0; i < RowSums<M>::PER_THREAD; i++) {
+        const int output = RowSums<M>::index(thread, i), row = row0 + output / M, m = output % M;
+        if (row >= a.n || m >= count) continue;
+        const size_t out = static_cast<size_t>(m0 + m) * a.n + row;
+        float sum = sums.sums[i];
+        if (a.epilogue == EPILOGUE_RESIDUAL_F32) sum = bf16_bits_to_f32(a.residual[out]) + sum;
+        else if (a.epilogue == EPILOGUE_RESIDUAL_ROUNDED) sum = round_bf16(sum) + bf16_bits_to_f32(a.residual[out]);
+        a.y[out] = static_cast<uint16_t>(f32_to_bf16_bits(sum));
+    }
+}
+
+// grid (row tiles of 64, lane tiles of 8)
+__global__ void __launch_bounds__(FP8_WARPS * 32, 2) linear_fp8_kernel(const __grid_constant__ Fp8LinearArgs a) {
+    extern __shared__ __align__(16) float fp8_smem[];
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int m0 = blockIdx.y * TILE_LANES, count = min(TILE_LANES, a.lanes - m0);
+    by_count(count, [&] { fp8_linear_tile<2>(a, m0, count, fp8_smem); }, [&] { fp8_linear_tile<4>(a, m0, count, fp8_smem); },
+             [&] { fp8_linear_tile<8>(a, m0, count, fp8_smem); });
+}
+
+// rounded_silu(round(gate)) * round(up) from a warp's sums: rows 0..3 gate, rows 4..7 the same rows of up
+template <int M, typename Store>
+__device__ __forceinline__ void silu_outputs(const RowSums<M> &sums, Store store) {
+    const int thread = threadIdx.x & 31;
+    constexpr int PER = RowSums<M>::PER_THREAD;
+    float other[PER];
+    // the up sums of a thread's gate outputs sit in the thread 16 further (the top bit of the output index)
+#pragma unroll
+    for (int i = 0; i < PER; i++) other[i] = __shfl_xor_sync(0xffffffffu, sums.sums[i], 16);
+    if (thread >= 16 || (RowSums<M>::VALUES < 32 && (thread & 1) != 0)) return;
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+        const int output = RowSums<M>::index(thread, i);
+        store(output / M, output % M, round_bf16(sums.sums[i]), round_bf16(other[i]));
+    }
+}
+
+template <int M>
+__device__ __forceinline__ void fp8_silu_tile(const Fp8LinearArgs &a, int m0, int count, float *smem) {
+    const int warp = threadIdx.x >> 5, blocks = a.k >> 7;
+    auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, a.k, first, n, count, smem, [&](int m) { return m0 + m; }); };
+    const int row0 = (blockIdx.x * FP8_WARPS + warp) * (FP8_ROWS / 2), first = min(row0, a.n - 1);
+    RowSums<M> sums;
+    sums.run([&](int r) { return a.w[r / 4] + static_cast<size_t>(min(row0 + (r & 3), a.n - 1)) * a.k; }, a.wscale[0] + static_cast<size_t>(first >> 7) * blocks,
+             a.wscale[1] + static_cast<size_t>(first >> 7) * blocks, blocks, smem, stage);
+    silu_outputs<M>(sums, [&](int r, int m, float gate, float up) {
+        if (row0 + r >= a.n || m >= count) return;
+        a.y[static_cast<size_t>(m0 + m) * a.n + row0 + r] = static_cast<uint16_t>(f32_to_bf16_bits(rounded_silu(gate) * up));
+    });
+}
+
+__global__ void __launch_bounds__(FP8_WARPS * 32, 2) linear_silu_multiply_fp8_kernel(const __grid_constant__ Fp8LinearArgs a) {
+    extern __shared__ __align__(16) float fp8_smem[];
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int m0 = blockIdx.y * TILE_LANES, count = min(TILE_LANES, a.lanes - m0);
+    by_count(count, [&] { fp8_silu_tile<2>(a, m0, count, fp8_smem); }, [&] { fp8_silu_tile<4>(a, m0, count, fp8_smem); },
+             [&] { fp8_silu_tile<8>(a, m0, count, fp8_smem); });
+}
+
+// ---- sparse experts
+
+// Groups the (token, route) pairs by expert: order[] = pair indices expert by expert, tiles[t] = {expert, first place in
+// order, count <= 8}, tile_count.  Experts outside [expert_start, expert_start + expert_count) have no tiles.  One CTA.
+constexpr int GROUP_THREADS = 1024, GROUP_MAX_EXPERTS = 1024;
+__global__ void __launch_bounds__(GROUP_THREADS) moe_group_kernel(const uint32_t *__restrict__ routes, int pairs, int experts, int expert_start, int expert_count,
+                                                                 MoeGroups groups) {
+    __shared__ int counts[GROUP_MAX_EXPERTS], places[GROUP_MAX_EXPERTS], tile_places[GROUP_MAX_EXPERTS];
+    __shared__ int warp_pairs[32], warp_tiles[32];
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int e = threadIdx.x;
+    counts[e] = 0;
+    __syncthreads();
+    auto expert_of = [&](int pair) {
+        const int expert = static_cast<int>(routes[pair] & 0xffffu);
+        return expert < experts && expert >= expert_start && expert < expert_start + expert_count ? expert : -1;
+    };
+    for (int pair = threadIdx.x; pair < pairs; pair += GROUP_THREADS) {
+        const int expert = expert_of(pair);
+        if (expert >= 0) atomicAdd(&counts[expert], 1);
+    }
+    __syncthreads();
+    // exclusive sums of pairs and tiles over the experts
+    const int own = counts[e], own_tiles = (own + TILE_LANES - 1) / TILE_LANES;
+    int before = own, tiles_before = own_tiles;
+    for (int offset = 1; offset < 32; offset <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, before, offset), b = __shfl_up_sync(0xffffffffu, tiles_before, offset);
+        if ((e & 31) >= offset) {
+            before += a;
+            tiles_before += b;
+        }
+    }
+    if ((e & 31) == 31) {
+        warp_pairs[e >> 5] = before;
+        warp_tiles[e >> 5] = tiles_before;
+    }
+    __syncthreads();
+    int base = 0, tile_base = 0;
+    for (int w = 0; w < (e >> 5); w++) {
+        base += warp_pairs[w];
+        tile_base += warp_tiles[w];
+    }
+    places[e] = base + before - own;
+    tile_places[e] = tile_base + tiles_before - own_tiles;
+    for (int t = 0; t < own_tiles; t++) groups.tiles[tile_places[e] + t] = make_int4(e, places[e] + t * TILE_LANES, min(TILE_LANES, own - t * TILE_LANES), 0);
+    if (e == GROUP_MAX_EXPERTS - 1) *groups.tile_count = tile_base + tiles_before;
+    __syncthreads();
+    for (int pair = threadIdx.x; pair < pairs; pair += GROUP_THREADS) {
+        const int expert = expert_of(pair);
+        if (expert >= 0) groups.order[atomicAdd(&places[expert], 1)] = pair;
+    }
+}
+
+struct MoeArgs {
+    const uint8_t *xq;
+    const float *xscale;
+    const uint32_t *routes;
+    const uint8_t *w;
+    const uint16_t *wscale;
+    uint16_t *out;
+    MoeGroups groups;
+    int hidden, inter, top_k, expert_start;
+};
+
+// grid (tiles of 32 intermediate rows, expert tiles); the activations of a pair are its token's row
+template <int M>
+__device__ __forceinline__ void moe_gate_up_tile(const MoeArgs &a, int4 tile, float *smem) {
+    const int warp = threadIdx.x >> 5, k = a.hidden, blocks = k >> 7, count = tile.z;
+    const int *order = a.groups.order + tile.y;
+    auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, k, first, n, count, smem, [&](int m) { return order[m] / a.top_k; }); };
+    const int row0 = (blockIdx.x * FP8_WARPS + warp) * (FP8_ROWS / 2), expert = tile.x - a.expert_start, first = min(row0, a.inter - 1);
+    const uint8_t *w = a.w + static_cast<size_t>(expert) * 2 * a.inter * k;
+    const uint16_t *ws = a.wscale + static_cast<size_t>(expert) * ((2 * a.inter + 127) >> 7) * blocks;
+    RowSums<M> sums;
+    sums.run([&](int r) { return w + static_cast<size_t>((r >= 4 ? a.inter : 0) + min(row0 + (r & 3), a.inter - 1)) * k; },
+             ws + static_cast<size_t>(first >> 7) * blocks, ws + static_cast<size_t>((a.inter + first) >> 7) * blocks, blocks, smem, stage);
+    silu_outputs<M>(sums, [&](int r, int m, float gate, float up) {
+        if (row0 + r >= a.inter || m >= count) return;
+        const float value = round_bf16(round_bf16(gate / (1.0f + expf(-gate))) * up);
+        a.out[static_cast<size_t>(order[m]) * a.inter + row0 + r] = static_cast<uint16_t>(f32_to_bf16_bits(value));
+    });
+}
+
+__global__ void __launch_bounds__(FP8_WARPS * 32, 2) moe_gate_up_fp8_kernel(const __grid_constant__ MoeArgs a) {
+    extern __shared__ __align__(16) float fp8_smem[];
+    grid_launch_dependents();
+    grid_dependency_wait();
+    if (static_cast<int>(blockIdx.y) >= *a.groups.tile_count) return;
+    const int4 tile = a.groups.tiles[blockIdx.y];
+    by_count(tile.z, [&] { moe_gate_up_tile<2>(a, tile, fp8_smem); }, [&] { moe_gate_up_tile<4>(a, tile, fp8_smem); }, [&] { moe_gate_up_tile<8>(a, tile, fp8_smem); });
+}
+
+// grid (tiles of 64 hidden rows, expert tiles); out = bf16(bf16(sum) * route weight) per pair
+template <int M>
+__device__ __forceinline__ void moe_down_tile(const MoeArgs &a, int4 tile, float *smem) {
+    const int warp = threadIdx.x >> 5, thread = threadIdx.x & 31, k = a.inter, blocks = k >> 7, count = tile.z;
+    const int *order = a.groups.order + tile.y;
+    auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, k, first, n, count, smem, [&](int m) { return order[m]; }); };
+    const int row0 = (blockIdx.x * FP8_WARPS + warp) * FP8_ROWS, expert = tile.x - a.expert_start;
+    const uint8_t *w = a.w + static_cast<size_t>(expert) * a.hidden * k;
+    const uint16_t *ws = a.wscale + static_cast<size_t>(expert) * ((a.hidden + 127) >> 7) * blocks;
+    RowSums<M> sums;
+    sums.run([&](int r) { return w + static_cast<size_t>(min(row0 + r, a.hidden - 1)) * k; }, ws + static_cast<size_t>(min(row0, a.hidden - 1) >> 7) * blocks,
+             ws + static_cast<size_t>(min(row0 + 4, a.hidden - 1) >> 7) * blocks, blocks, smem, stage);
+    if (RowSums<M>::VALUES < 32 && (thread & 1) != 0) return;
+#pragma unroll
+    for (int i = 0; i < RowSums<M>::PER_THREAD; i++) {
+        const int output = RowSums<M>::index(thread, i), row = row0 + output / M, m = output % M;
+        if (row >= a.hidden || m >= count) continue;
+        const float weight = bf16_bits_to_f32(a.routes[order[m]] >> 16);
+        a.out[static_cast<size_t>(order[m]) * a.hidden + row] = static_cast<uint16_t>(f32_to_bf16_bits(round_bf16(sums.sums[i]) * weight));
+    }
+}
+
+__global__ void __launch_bounds__(FP8_WARPS * 32, 2) moe_down_fp8_kernel(const __grid_constant__ MoeArgs a) {
+    extern __shared__ __align__(16) float fp8_smem[];
+    grid_launch_dependents();
+    grid_dependency_wait();
+    if (static_cast<int>(blockIdx.y) >= *a.groups.tile_count) return;
+    const int4 tile = a.groups.tiles[blockIdx.y];
+    by_count(tile.z, [&] { moe_down_tile<2>(a, tile, fp8_smem); }, [&] { moe_down_tile<4>(a, tile, fp8_smem); }, [&] { moe_down_tile<8>(a, tile, fp8_smem); });
+}
+
+template <typename Args>
+cudaError_t launch_rows(void (*kernel)(Args), dim3 grid, int tile_lanes, cudaStream_t stream, const Args &args) {
+    auto bytes = [](int m) { return static_cast<size_t>(CHUNK) * 128 * m * sizeof(float) + static_cast<size_t>(CHUNK) * m * sizeof(float); };
+    cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes(8)));
+    if (status != cudaSuccess) return status;
+    return launch_dependent(kernel, grid, dim3(FP8_WARPS * 32), bytes(tile_lanes <= 2 ? 2 : tile_lanes <= 4 ? 4 : 8), 1, stream, args);
+}
+
+}  // namespace
+
+cudaError_t launch_linear_fp8(const uint8_t *xq, const float *xscale, const uint8_t *w, const uint16_t *wscale,
+                              uint16_t *y, const uint16_t *residual, int lanes, int n, int k, int epilogue,
+                              cudaStream_t stream) {
+    if (lanes <= 0) return cudaSuccess;
+    if (k % 128 != 0) return cudaErrorInvalidValue;
+    const Fp8LinearArgs args{xq, xscale, {w, nullptr}, {wscale, nullptr}, y, residual, lanes, n, k, epilogue};
+    const int rows = FP8_WARPS * FP8_ROWS;
+    return launch_rows(linear_fp8_kernel, dim3((n + rows - 1) / rows, (lanes + TILE_LANES - 1) / TILE_LANES), lanes, stream, args);
+}
+
+cudaError_t launch_linear_silu_multiply_fp8(const uint8_t *xq, const float *xscale, const uint8_t *wg,
+                                            const uint16_t *wg_scale, const uint8_t *wu, const uint16_t *wu_scale,
+                                            uint16_t *y, int lanes, int n, int k, cudaStream_t stream) {
+    if (lanes <= 0) return cudaSuccess;
+    if (k % 128 != 0) return cudaErrorInvalidValue;
+    const Fp8LinearArgs args{xq, xscale, {wg, wu}, {wg_scale, wu_scale}, y, nullptr, lanes, n, k, EPILOGUE_BF16};
+    const int rows = FP8_WARPS * FP8_ROWS / 2;
+    return launch_rows(linear_silu_multiply_fp8_kernel, dim3((n + rows - 1) / rows, (lanes + TILE_LANES - 1) / TILE_LANES), lanes, stream, args);
+}
+
+size_t moe_group_bytes(int lanes, int top_k, int experts) {
+    const size_t pairs = static_cast<size_t>(lanes) * top_k;
+    return (pairs / TILE_LANES + experts + 1) * sizeof(int4) + (pairs + 4) * sizeof(int);
+}
+MoeGroups moe_groups(void *scratch, int lanes, int top_k, int experts) {
+    MoeGroups groups;
+    const size_t pairs = static_cast<size_t>(lanes) * top_k;
+    groups.tiles = static_cast<int4 *>(scratch);
+    groups.order = reinterpret_cast<int *>(groups.tiles + pairs / TILE_LANES + experts + 1);
+    groups.tile_count = groups.order + pairs;
+    return groups;
+}
+
+cudaError_t launch_moe_group(const uint32_t *routes, const MoeGroups &groups, int lanes, int top_k, int experts, int expert_start, int expert_count,
+                             cudaStream_t stream) {
+    if (lanes <= 0) return cudaSuccess;
+    if (experts > GROUP_MAX_EXPERTS) return cudaErrorInvalidValue;
+    return launch_dependent(moe_group_kernel, dim3(1), dim3(GROUP_THREADS), 0, 1, stream, routes, lanes * top_k, experts, expert_start, expert_count, groups);
+}
+
+static int most_tiles(int lanes, int top_k, int experts) {
+    const int pairs = lanes * top_k;
+    return pairs < pairs / TILE_LANES + experts ? pairs : pairs / TILE_LANES + experts;
+}
+
+cudaError_t launch_moe_gate_up_fp8(const uint8_t *xq, const float *xscale, const MoeGroups &groups, const uint8_t *w,
+                                   const uint16_t *wscale, uint16_t *intermediates, int lanes, int hidden_size,
+                                   int inter, int experts, int top_k, int expert_start, cudaStream_t stream) {
+    if (lanes <= 0) return cudaSuccess;
+    if (hidden_size % 128 != 0) return cudaErrorInvalidValue;
+    const MoeArgs args{xq, xscale, nullptr, w, wscale, intermediates, groups, hidden_size, inter, top_k, expert_start};
+    const int rows = FP8_WARPS * FP8_ROWS / 2;
+    return launch_rows(moe_gate_up_fp8_kernel, dim3((inter + rows - 1) / rows, most_tiles(lanes, top_k, experts)), TILE_LANES, stream, args);
+}
+
+cudaError_t launch_moe_down_fp8(const uint8_t *xq, const float *xscale, const MoeGroups &groups, const uint32_t *routes, const uint8_t *w,
+                                const uint16_t *wscale, uint16_t *outputs, int lanes, int hidden_size, int inter,
+                                int experts, int top_k, int expert_start, cudaStream_t stream) {
+    if (lanes <= 0) return cudaSuccess;
+    if (inter % 128 != 0) return cudaErrorInvalidValue;
+    const MoeArgs args{xq, xscale, routes, w, wscale, outputs, groups, hidden_size, inter, top_k, expert_start};
+    const int rows = FP8_WARPS * FP8_ROWS;
+    return launch_rows(moe_down_fp8_kernel, dim3((hidden_size + rows - 1) / rows, most_tiles(lanes, top_k, experts)), TILE_LANES, stream, args);
+}
+
+}  // namespace nerve

@@ -447,250 +447,4 @@ cudaError_t launch_linear_int4_silu_pair(const uint16_t *x, const void *prepared
     return launch_pdl(linear_int4_mma_kernel<2, true, 2>, grid, dim3(INT4_WARPS * 32), stream, params);
 }
 
-// ----------------------------------------------------------------------------- FP8 W8A8 (block-scaled)
-
-// linear_prequant_fp8_e4m3.comp.template:69-120: per 4 elements an exact f32
-// dot of e4m3 values, fma'd with act_scale*weight_scale.  Here the 128-column
-// block partial is accumulated first and scaled once (same value up to f32
-// rounding order).  One warp per output row; lane handles 4 columns per step.
-template <int MT>
-__device__ __forceinline__ void fp8_row_dot(const uint8_t *__restrict__ xq, const float *__restrict__ xscale,
-                                            const uint8_t *__restrict__ wrow, const uint16_t *__restrict__ wscale_row,
-                                            int k, int lanes, int m0, int lane, float (&acc)[MT]) {
-    const int blocks = k >> 7;
-    for (int block = 0; block < blocks; block++) {
-        uint32_t wpacked = __ldg(reinterpret_cast<const uint32_t *>(wrow + block * 128) + lane);
-        float wf[4] = {e4m3_to_f32(wpacked & 0xff), e4m3_to_f32((wpacked >> 8) & 0xff), e4m3_to_f32((wpacked >> 16) & 0xff),
-                       e4m3_to_f32(wpacked >> 24)};
-        float ws = bf16_bits_to_f32(wscale_row[block]);
-#pragma unroll
-        for (int m = 0; m < MT; m++) {
-            if (m0 + m >= lanes) break;
-            uint32_t xpacked = __ldg(reinterpret_cast<const uint32_t *>(xq + static_cast<size_t>(m0 + m) * k + block * 128) + lane);
-            float d = e4m3_to_f32(xpacked & 0xff) * wf[0];
-            d += e4m3_to_f32((xpacked >> 8) & 0xff) * wf[1];
-            d += e4m3_to_f32((xpacked >> 16) & 0xff) * wf[2];
-            d += e4m3_to_f32(xpacked >> 24) * wf[3];
-            acc[m] = fmaf(d, xscale[static_cast<size_t>(m0 + m) * blocks + block] * ws, acc[m]);
-        }
-    }
-}
-
-template <int MT>
-__global__ void __launch_bounds__(256)
-linear_fp8_kernel(const uint8_t *__restrict__ xq, const float *__restrict__ xscale, const uint8_t *__restrict__ w,
-                  const uint16_t *__restrict__ wscale, uint16_t *__restrict__ y, const uint16_t *__restrict__ residual,
-                  int lanes, int n, int k, int epilogue) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row = blockIdx.x * 8 + warp;
-    const int m0 = blockIdx.y * MT;
-    if (row >= n) return;
-    float acc[MT];
-#pragma unroll
-    for (int m = 0; m < MT; m++) acc[m] = 0.0f;
-    grid_dependency_wait();
-    fp8_row_dot<MT>(xq, xscale, w + static_cast<size_t>(row) * k, wscale + static_cast<size_t>(row >> 7) * (k >> 7), k, lanes,
-                    m0, lane, acc);
-#pragma unroll
-    for (int m = 0; m < MT; m++) acc[m] = warp_sum(acc[m]);
-    if (lane == 0)
-#pragma unroll
-        for (int m = 0; m < MT; m++) {
-            if (m0 + m >= lanes) break;
-            size_t index = static_cast<size_t>(m0 + m) * n + row;
-            float sum = acc[m];
-            if (epilogue == EPILOGUE_RESIDUAL_F32) sum = bf16_bits_to_f32(residual[index]) + sum;
-            else if (epilogue == EPILOGUE_RESIDUAL_ROUNDED) sum = round_bf16(sum) + bf16_bits_to_f32(residual[index]);
-            y[index] = static_cast<uint16_t>(f32_to_bf16_bits(sum));
-        }
-}
-
-cudaError_t launch_linear_fp8(const uint8_t *xq, const float *xscale, const uint8_t *w, const uint16_t *wscale,
-                              uint16_t *y, const uint16_t *residual, int lanes, int n, int k, int epilogue,
-                              cudaStream_t stream) {
-    if (lanes <= 0) return cudaSuccess;
-    if (k % 128 != 0) return cudaErrorInvalidValue;
-    dim3 grid((n + 7) / 8, (lanes + 7) / 8);
-    linear_fp8_kernel<8><<<grid, 256, 0, stream>>>(xq, xscale, w, wscale, y, residual, lanes, n, k, epilogue);
-    return cudaGetLastError();
-}
-
-template <int MT>
-__global__ void __launch_bounds__(256)
-linear_silu_multiply_fp8_kernel(const uint8_t *__restrict__ xq, const float *__restrict__ xscale,
-                                const uint8_t *__restrict__ wg, const uint16_t *__restrict__ wg_scale,
-                                const uint8_t *__restrict__ wu, const uint16_t *__restrict__ wu_scale,
-                                uint16_t *__restrict__ y, int lanes, int n, int k) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row = blockIdx.x * 8 + warp;
-    const int m0 = blockIdx.y * MT;
-    if (row >= n) return;
-    float gate[MT], up[MT];
-#pragma unroll
-    for (int m = 0; m < MT; m++) gate[m] = up[m] = 0.0f;
-    grid_dependency_wait();
-    fp8_row_dot<MT>(xq, xscale, wg + static_cast<size_t>(row) * k, wg_scale + static_cast<size_t>(row >> 7) * (k >> 7), k,
-                    lanes, m0, lane, gate);
-    fp8_row_dot<MT>(xq, xscale, wu + static_cast<size_t>(row) * k, wu_scale + static_cast<size_t>(row >> 7) * (k >> 7), k,
-                    lanes, m0, lane, up);
-#pragma unroll
-    for (int m = 0; m < MT; m++) {
-        gate[m] = warp_sum(gate[m]);
-        up[m] = warp_sum(up[m]);
-    }
-    if (lane == 0)
-#pragma unroll
-        for (int m = 0; m < MT; m++) {
-            if (m0 + m >= lanes) break;
-            float value = rounded_silu(round_bf16(gate[m])) * round_bf16(up[m]);
-            y[static_cast<size_t>(m0 + m) * n + row] = static_cast<uint16_t>(f32_to_bf16_bits(value));
-        }
-}
-
-cudaError_t launch_linear_silu_multiply_fp8(const uint8_t *xq, const float *xscale, const uint8_t *wg,
-                                            const uint16_t *wg_scale, const uint8_t *wu, const uint16_t *wu_scale,
-                                            uint16_t *y, int lanes, int n, int k, cudaStream_t stream) {
-    if (lanes <= 0) return cudaSuccess;
-    if (k % 128 != 0) return cudaErrorInvalidValue;
-    dim3 grid((n + 7) / 8, (lanes + 7) / 8);
-    linear_silu_multiply_fp8_kernel<8><<<grid, 256, 0, stream>>>(xq, xscale, wg, wg_scale, wu, wu_scale, y, lanes, n, k);
-    return cudaGetLastError();
-}
-
-// ----------------------------------------------------------------------------- MoE experts (FP8)
-
-// sparse_moe_gate_up_fp8_e4m3.comp.template:94-198.  grid = (ceil(inter/8), top_k, lanes); each CTA quantises the
-// lane's hidden frame per 128 columns into shared memory (as the shader does), then one warp per intermediate row
-// computes gate and up of the routed expert.  Experts outside [expert_start, expert_start+expert_count) are skipped
-// (expert-parallel shards); their slot of `intermediates` is left untouched.
-__global__ void __launch_bounds__(256)
-moe_gate_up_fp8_kernel(const uint16_t *__restrict__ hidden, const uint32_t *__restrict__ routes,
-                       const uint8_t *__restrict__ w, const uint16_t *__restrict__ wscale,
-                       uint16_t *__restrict__ intermediates, int hidden_size, int inter, int experts, int top_k,
-                       int expert_start, int expert_count) {
-    extern __shared__ uint8_t shared[];
-    const int token = blockIdx.z, route = blockIdx.y;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int blocks = hidden_size >> 7;
-    uint8_t *hq = shared;
-    float *hs = reinterpret_cast<float *>(shared + hidden_size);
-    grid_dependency_wait();
-    uint32_t packed_route = routes[static_cast<size_t>(token) * top_k + route];
-    int expert = static_cast<int>(packed_route & 0xffffu);
-    if (expert >= experts || expert < expert_start || expert >= expert_start + expert_count) return;
-    expert -= expert_start;
-    for (int block = warp; block < blocks; block += 8) {
-        const uint32_t *src = reinterpret_cast<const uint32_t *>(hidden + static_cast<size_t>(token) * hidden_size + block * 128) + lane * 2;
-        uint32_t w0 = src[0], w1 = src[1];
-        float v0 = bf16_lo(w0), v1 = bf16_hi(w0), v2 = bf16_lo(w1), v3 = bf16_hi(w1);
-        float block_max = warp_max(fmaxf(fmaxf(fabsf(v0), fabsf(v1)), fmaxf(fabsf(v2), fabsf(v3))));
-        float scale = block_max > 0.0f ? block_max / 448.0f : 1.0f;
-        if (lane == 0) hs[block] = scale;
-        uint32_t q = static_cast<uint32_t>(f32_to_e4m3(v0 / scale)) | (static_cast<uint32_t>(f32_to_e4m3(v1 / scale)) << 8) |
-                     (static_cast<uint32_t>(f32_to_e4m3(v2 / scale)) << 16) | (static_cast<uint32_t>(f32_to_e4m3(v3 / scale)) << 24);
-        reinterpret_cast<uint32_t *>(hq + block * 128)[lane] = q;
-    }
-    __syncthreads();
-    const int row = blockIdx.x * 8 + warp;
-    if (row >= inter) return;
-    const int scale_rows = (2 * inter + 127) >> 7;
-    const uint8_t *wbase = w + static_cast<size_t>(expert) * 2 * inter * hidden_size;
-    const uint16_t *sbase = wscale + static_cast<size_t>(expert) * scale_rows * blocks;
-    float gate = 0.0f, up = 0.0f;
-    for (int block = 0; block < blocks; block++) {
-        uint32_t xq = reinterpret_cast<const uint32_t *>(hq + block * 128)[lane];
-        float xf[4] = {e4m3_to_f32(xq & 0xff), e4m3_to_f32((xq >> 8) & 0xff), e4m3_to_f32((xq >> 16) & 0xff), e4m3_to_f32(xq >> 24)};
-        uint32_t gq = __ldg(reinterpret_cast<const uint32_t *>(wbase + static_cast<size_t>(row) * hidden_size + block * 128) + lane);
-        uint32_t uq = __ldg(reinterpret_cast<const uint32_t *>(wbase + static_cast<size_t>(inter + row) * hidden_size + block * 128) + lane);
-        float gd = xf[0] * e4m3_to_f32(gq & 0xff) + xf[1] * e4m3_to_f32((gq >> 8) & 0xff) + xf[2] * e4m3_to_f32((gq >> 16) & 0xff) +
-                   xf[3] * e4m3_to_f32(gq >> 24);
-        float ud = xf[0] * e4m3_to_f32(uq & 0xff) + xf[1] * e4m3_to_f32((uq >> 8) & 0xff) + xf[2] * e4m3_to_f32((uq >> 16) & 0xff) +
-                   xf[3] * e4m3_to_f32(uq >> 24);
-        gate = fmaf(gd, hs[block] * bf16_bits_to_f32(sbase[static_cast<size_t>(row >> 7) * blocks + block]), gate);
-        up = fmaf(ud, hs[block] * bf16_bits_to_f32(sbase[static_cast<size_t>((inter + row) >> 7) * blocks + block]), up);
-    }
-    gate = warp_sum(gate);
-    up = warp_sum(up);
-    if (lane == 0) {
-        gate = round_bf16(gate);
-        up = round_bf16(up);
-        float value = round_bf16(round_bf16(gate / (1.0f + expf(-gate))) * up);
-        intermediates[(static_cast<size_t>(token) * top_k + route) * inter + row] = static_cast<uint16_t>(f32_to_bf16_bits(value));
-    }
-}
-
-cudaError_t launch_moe_gate_up_fp8(const uint16_t *hidden, const uint32_t *routes, const uint8_t *w,
-                                   const uint16_t *wscale, uint16_t *intermediates, int lanes, int hidden_size,
-                                   int inter, int experts, int top_k, int expert_start, int expert_count,
-                                   cudaStream_t stream) {
-    if (lanes <= 0) return cudaSuccess;
-    if (hidden_size % 128 != 0) return cudaErrorInvalidValue;
-    dim3 grid((inter + 7) / 8, top_k, lanes);
-    size_t shared = hidden_size + sizeof(float) * (hidden_size / 128);
-    moe_gate_up_fp8_kernel<<<grid, 256, shared, stream>>>(hidden, routes, w, wscale, intermediates, hidden_size, inter,
-                                                          experts, top_k, expert_start, expert_count);
-    return cudaGetLastError();
-}
-
-// sparse_moe_down_fp8_e4m3.comp.template:90-176: out = bf16(bf16(sum) * route_weight)
-__global__ void __launch_bounds__(256)
-moe_down_fp8_kernel(const uint16_t *__restrict__ intermediates, const uint32_t *__restrict__ routes,
-                    const uint8_t *__restrict__ w, const uint16_t *__restrict__ wscale, uint16_t *__restrict__ outputs,
-                    int hidden_size, int inter, int experts, int top_k, int expert_start, int expert_count) {
-    extern __shared__ uint8_t shared[];
-    const int token = blockIdx.z, route = blockIdx.y;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int blocks = inter >> 7;
-    uint8_t *mq = shared;
-    float *ms = reinterpret_cast<float *>(shared + inter);
-    grid_dependency_wait();
-    uint32_t packed_route = routes[static_cast<size_t>(token) * top_k + route];
-    int expert = static_cast<int>(packed_route & 0xffffu);
-    if (expert >= experts || expert < expert_start || expert >= expert_start + expert_count) return;
-    expert -= expert_start;
-    float route_weight = bf16_bits_to_f32(packed_route >> 16);
-    const uint16_t *mid = intermediates + (static_cast<size_t>(token) * top_k + route) * inter;
-    for (int block = warp; block < blocks; block += 8) {
-        const uint32_t *src = reinterpret_cast<const uint32_t *>(mid + block * 128) + lane * 2;
-        uint32_t w0 = src[0], w1 = src[1];
-        float v0 = bf16_lo(w0), v1 = bf16_hi(w0), v2 = bf16_lo(w1), v3 = bf16_hi(w1);
-        float block_max = warp_max(fmaxf(fmaxf(fabsf(v0), fabsf(v1)), fmaxf(fabsf(v2), fabsf(v3))));
-        float scale = block_max > 0.0f ? block_max / 448.0f : 1.0f;
-        if (lane == 0) ms[block] = scale;
-        uint32_t q = static_cast<uint32_t>(f32_to_e4m3(v0 / scale)) | (static_cast<uint32_t>(f32_to_e4m3(v1 / scale)) << 8) |
-                     (static_cast<uint32_t>(f32_to_e4m3(v2 / scale)) << 16) | (static_cast<uint32_t>(f32_to_e4m3(v3 / scale)) << 24);
-        reinterpret_cast<uint32_t *>(mq + block * 128)[lane] = q;
-    }
-    __syncthreads();
-    const int row = blockIdx.x * 8 + warp;
-    if (row >= hidden_size) return;
-    const int scale_rows = (hidden_size + 127) >> 7;
-    const uint8_t *wbase = w + static_cast<size_t>(expert) * hidden_size * inter;
-    const uint16_t *sbase = wscale + static_cast<size_t>(expert) * scale_rows * blocks;
-    float sum = 0.0f;
-    for (int block = 0; block < blocks; block++) {
-        uint32_t xq = reinterpret_cast<const uint32_t *>(mq + block * 128)[lane];
-        uint32_t wq = __ldg(reinterpret_cast<const uint32_t *>(wbase + static_cast<size_t>(row) * inter + block * 128) + lane);
-        float d = e4m3_to_f32(xq & 0xff) * e4m3_to_f32(wq & 0xff) + e4m3_to_f32((xq >> 8) & 0xff) * e4m3_to_f32((wq >> 8) & 0xff) +
-                  e4m3_to_f32((xq >> 16) & 0xff) * e4m3_to_f32((wq >> 16) & 0xff) + e4m3_to_f32(xq >> 24) * e4m3_to_f32(wq >> 24);
-        sum = fmaf(d, ms[block] * bf16_bits_to_f32(sbase[static_cast<size_t>(row >> 7) * blocks + block]), sum);
-    }
-    sum = warp_sum(sum);
-    if (lane == 0)
-        outputs[(static_cast<size_t>(token) * top_k + route) * hidden_size + row] =
-            static_cast<uint16_t>(f32_to_bf16_bits(round_bf16(sum) * route_weight));
-}
-
-cudaError_t launch_moe_down_fp8(const uint16_t *intermediates, const uint32_t *routes, const uint8_t *w,
-                                const uint16_t *wscale, uint16_t *outputs, int lanes, int hidden_size, int inter,
-                                int experts, int top_k, int expert_start, int expert_count, cudaStream_t stream) {
-    if (lanes <= 0) return cudaSuccess;
-    if (inter % 128 != 0) return cudaErrorInvalidValue;
-    dim3 grid((hidden_size + 7) / 8, top_k, lanes);
-    size_t shared = inter + sizeof(float) * (inter / 128);
-    moe_down_fp8_kernel<<<grid, 256, shared, stream>>>(intermediates, routes, w, wscale, outputs, hidden_size, inter,
-                                                       experts, top_k, expert_start, expert_count);
-    return cudaGetLastError();
-}
-
 }  // namespace nerve
