@@ -581,6 +581,14 @@ Engine::Engine(std::shared_ptr<MountedModel> model) : model_(std::move(model)) {
                 if (w.storage == TensorStorage::FP8_BLOCK) return true;
         return false;
     };
+    const ComponentPlan *attention = nullptr;
+    auto same_heads = [&](const ComponentPlan &component) {
+        if (!component.has_kv) return true;
+        if (attention == nullptr) attention = &component;
+        return component.head_width == attention->head_width && component.q_heads * attention->kv_heads == attention->q_heads * component.kv_heads;
+    };
+    ragged_prefill_ = std::all_of(plan.layers.begin(), plan.layers.end(), same_heads) && std::all_of(plan.draft_layers.begin(), plan.draft_layers.end(), same_heads) &&
+                      attention != nullptr;
     scalar_attention_ = std::any_of(plan.layers.begin(), plan.layers.end(), has_fp8) || std::any_of(plan.draft_layers.begin(), plan.draft_layers.end(), has_fp8);
     max_q_heads_ = max_q_heads;
     const size_t partial_bytes = static_cast<size_t>(max_head_width + 2) * sizeof(float);
@@ -592,6 +600,7 @@ Engine::Engine(std::shared_ptr<MountedModel> model) : model_(std::move(model)) {
     const size_t small_batches = static_cast<size_t>(std::min(options.max_lanes, 8)) * max_q_heads * (max_splits_ + (max_splits_ + 31) / 32);
     attention_partials_ = std::max(small_batches, static_cast<size_t>(options.max_lanes) * max_q_heads * op_splits);
     attention_scratch_ = device_alloc(attention_partials_ * partial_bytes);
+    attention_blocks_ = device_alloc(lanes * sizeof(AttentionBlock));  // (a block covers at least one lane)
 
     // cycle arrays: verify tokens, forced drafts, stop tokens/counts, accept rows, per-step draft tokens, slots
     cycle_state_ = device_alloc(lanes * 64 * sizeof(uint32_t) + static_cast<size_t>(options.max_streams) * (MAX_STOP_TOKENS + 64) * sizeof(uint32_t) * 4);
@@ -630,7 +639,7 @@ Engine::~Engine() {
     for (void *mapping : tp_peer_mappings_) cudaIpcCloseMemHandle(mapping);
     for (auto &entry : signals_) cudaFree(entry.second.ptr);
     for (DeviceBuffer *buffer : {&frame_a_, &frame_b_, &embedding_out_, &normalized_, &draft_normalized_, &draft_hidden_in_, &logits_,
-                                 &records_, &argmax_scratch_, &sampler_scratch_, &sampler_table_, &lane_tokens_, &lane_positions_, &lane_slots_, &pending_hidden_, &pending_backup_, &attention_scratch_,
+                                 &records_, &argmax_scratch_, &sampler_scratch_, &sampler_table_, &lane_tokens_, &lane_positions_, &lane_slots_, &pending_hidden_, &pending_backup_, &attention_scratch_, &attention_blocks_,
                                  &cycle_state_, &int4_activations_, &moe_quantised_, &moe_quantised_scales_, &moe_groups_, &kernel_error_, &tp_partial_, &tp_exchange_, &tp_description_, &stack_q_, &stack_attention_out_, &stack_activation_, &stack_barrier_, &stack_timing_, &prefix_pending_})
         cudaFree(buffer->ptr);
     cudaFreeHost(staging_);
@@ -1258,7 +1267,8 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
         append.k_form = form(k_rope);
         check(launch_rope_append(append, kv, lane_table, lanes, st), "rope and kv append");
         check(launch_attention(u16(attention.inputs[0]), u16(attention.outputs[0]), kv, lane_table, lanes, current_width_, attention.q_heads,
-                               attention.attention_scale, current_op_split_tokens_, current_op_splits_, static_cast<float *>(attention_scratch_.ptr), scalar_attention_, st),
+                               attention.attention_scale, current_op_split_tokens_, current_op_splits_, static_cast<float *>(attention_scratch_.ptr), scalar_attention_, st,
+                               current_blocks_ > 0 ? static_cast<const AttentionBlock *>(attention_blocks_.ptr) : nullptr, current_blocks_),
               "attention");
         if (current_op_splits_ > 1 || scalar_attention_) counters_.kernel_launches++;
     };
@@ -1381,7 +1391,8 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
                               "linear_bf16 (streamed)");
                     } else {
                         check(launch_linear_bf16(u16(op.inputs[0]), static_cast<const uint16_t *>(weight(w.tensor)), ptr(op.outputs[branch]), nullptr,
-                                                 lanes, static_cast<int>(w.n), static_cast<int>(w.k), EPILOGUE_BF16, 1.0f, st, static_cast<int *>(kernel_error_.ptr)),
+                                                 lanes, static_cast<int>(w.n), static_cast<int>(w.k), EPILOGUE_BF16, 1.0f, st, static_cast<int *>(kernel_error_.ptr),
+                                                 current_form_lanes_),
                               "linear_bf16");
                     }
                 } else if (w.storage == TensorStorage::INT4_CT) {
@@ -1773,39 +1784,97 @@ void Engine::draft_forward(int lanes, const uint16_t *hidden_in, bool want_logit
 
 // ---------------------------------------------------------------------------- prefill (temporal_prompt.rs:298-478)
 
-void Engine::run_prefill_chunk(Stream &s, const uint32_t *tokens, int count, bool sample_last, uint32_t *sampled) {
+// One chunk each of one or several streams in one pass over the weights.  Lanes are stream-major; chunks of equal length
+// are a uniform batch, others a ragged one (the attention then takes its row blocks from a table; at most eight lanes run
+// as streams of one lane each).  Batches of FP8 packages hold chunks of one form of the bf16 linears only (see
+// launch_linear_bf16): a router's sums must not depend on the other streams' chunks.
+void Engine::run_prefill_batch(std::vector<PrefillPart> &parts) {
     const ModelPlan &plan = model_->plan();
-    ensure_pages(s, s.next_tick + count - 1);
+    std::vector<uint32_t> positions, tokens;
+    std::vector<int32_t> slots;
+    int widest = 0;
+    bool uniform = true;
+    for (const PrefillPart &part : parts) {
+        Stream &s = *part.stream;
+        ensure_pages(s, s.next_tick + part.count - 1);
+        for (int i = 0; i < part.count; i++) {
+            positions.push_back(static_cast<uint32_t>(s.next_tick + i));
+            slots.push_back(s.slot);
+            tokens.push_back(part.tokens[i]);
+        }
+        widest = std::max(widest, part.count);
+        uniform &= part.count == parts[0].count;
+    }
+    const int lanes = static_cast<int>(positions.size());
+    const bool ragged = !uniform && lanes > 8;
     sync_block_tables();
-    std::vector<uint32_t> positions(count);
-    std::vector<int32_t> slots(count, s.slot);
-    for (int i = 0; i < count; i++) positions[i] = static_cast<uint32_t>(s.next_tick + i);
-    upload_lanes(positions, slots, count);
-    upload_tokens(tokens, count);
-    target_forward(count, false);
-    const size_t frame = static_cast<size_t>(plan.hidden) * 2;
-    uint8_t *pending = static_cast<uint8_t *>(pending_hidden_.ptr) + s.slot * frame;
+    upload_lanes(positions, slots, uniform || ragged ? widest : 1);
+    upload_tokens(tokens.data(), lanes);
+    current_form_lanes_ = scalar_attention_ ? parts[0].count : 0;
+    if (ragged) {
+        const auto attention = std::find_if(plan.layers.begin(), plan.layers.end(), [](const ComponentPlan &layer) { return layer.has_kv; });
+        const int block_lanes = attention_block_lanes(widest, attention->q_heads, attention->kv_heads, attention->head_width, scalar_attention_);
+        std::vector<AttentionBlock> blocks;
+        int first = 0;
+        for (const PrefillPart &part : parts) {
+            for (int index = 0; index * block_lanes < part.count; index++) blocks.push_back(AttentionBlock{first, part.count, index});
+            first += part.count;
+        }
+        upload(attention_blocks_.ptr, blocks.data(), blocks.size() * sizeof(AttentionBlock), "attention blocks upload");
+        current_blocks_ = static_cast<int>(blocks.size());
+    }
+    target_forward(lanes, false);
+    const int32_t *lane_slots = static_cast<const int32_t *>(lane_slots_.ptr);
     if (plan.has_draft) {
         // draft state steps for every prompt token: token i pairs with the target hidden of tick i-1
-        // (verification.rs:10-34): lane 0 takes the pending hidden, lane i the normalised frame i-1.
-        check(launch_shift_hidden(static_cast<const uint16_t *>(pending_hidden_.ptr), static_cast<const int32_t *>(lane_slots_.ptr),
-                                  static_cast<const uint16_t *>(normalized_.ptr), static_cast<uint16_t *>(draft_hidden_in_.ptr), 1, count,
-                                  static_cast<int>(plan.hidden), cuda_stream_),
+        // (verification.rs:10-34): a stream's first lane takes its pending hidden, lane i the normalised frame i-1.
+        check(launch_shift_hidden_lanes(static_cast<const uint16_t *>(pending_hidden_.ptr), lane_slots, static_cast<const uint16_t *>(normalized_.ptr),
+                                        static_cast<uint16_t *>(draft_hidden_in_.ptr), lanes, static_cast<int>(plan.hidden), cuda_stream_),
               "prefill draft hidden");
-        draft_forward(count, static_cast<const uint16_t *>(draft_hidden_in_.ptr), false);
-        cuda_check(cudaMemcpyAsync(pending, static_cast<uint8_t *>(normalized_.ptr) + static_cast<size_t>(count - 1) * frame, frame,
-                                   cudaMemcpyDeviceToDevice, cuda_stream_),
-                   "commit target hidden");
+        draft_forward(lanes, static_cast<const uint16_t *>(draft_hidden_in_.ptr), false);
+        check(launch_commit_hidden(static_cast<const uint16_t *>(normalized_.ptr), lane_slots, static_cast<uint16_t *>(pending_hidden_.ptr), lanes,
+                                   static_cast<int>(plan.hidden), cuda_stream_),
+              "commit target hidden");
     }
-    if (sample_last) {
-        project_and_sample(static_cast<const uint16_t *>(normalized_.ptr) + static_cast<size_t>(count - 1) * plan.hidden, plan.output.projection_tensor,
-                           plan.output.logits_scale, 1, current_lanes_.slot + (count - 1), current_lanes_.position + (count - 1), "prefill sampler");
-        cuda_check(cudaMemcpyAsync(host_records_, records_.ptr, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, cuda_stream_), "record readback");
+    current_blocks_ = 0;
+    current_form_lanes_ = 0;
+    // the first tokens of the events whose prompts end here
+    std::vector<int32_t> last_lanes;
+    int first = 0;
+    for (const PrefillPart &part : parts) {
+        first += part.count;
+        if (part.sample) last_lanes.push_back(first - 1);
+    }
+    if (!last_lanes.empty()) {
+        const int count = static_cast<int>(last_lanes.size());
+        const uint16_t *rows = static_cast<const uint16_t *>(normalized_.ptr) + static_cast<size_t>(last_lanes[0]) * plan.hidden;
+        const int32_t *row_slots = current_lanes_.slot + last_lanes[0];
+        const uint32_t *row_positions = current_lanes_.position + last_lanes[0];
+        if (count > 1) {  // gathered: [lane | slot | position] of every sampled row
+            std::vector<uint32_t> table(3 * static_cast<size_t>(count));
+            for (int i = 0; i < count; i++) {
+                table[i] = static_cast<uint32_t>(last_lanes[i]);
+                table[count + i] = static_cast<uint32_t>(slots[last_lanes[i]]);
+                table[2 * count + i] = positions[last_lanes[i]];
+            }
+            uint32_t *device_table = static_cast<uint32_t *>(cycle_state_.ptr);
+            upload(device_table, table.data(), table.size() * sizeof(uint32_t), "sampled rows upload");
+            check(launch_gather_rows(static_cast<const uint16_t *>(normalized_.ptr), reinterpret_cast<const int32_t *>(device_table),
+                                     static_cast<uint16_t *>(draft_hidden_in_.ptr), count, static_cast<int>(plan.hidden), cuda_stream_),
+                  "gather sampled rows");
+            rows = static_cast<const uint16_t *>(draft_hidden_in_.ptr);
+            row_slots = reinterpret_cast<const int32_t *>(device_table + count);
+            row_positions = device_table + 2 * count;
+        }
+        project_and_sample(rows, plan.output.projection_tensor, plan.output.logits_scale, count, row_slots, row_positions, "prefill sampler");
+        cuda_check(cudaMemcpyAsync(host_records_, records_.ptr, static_cast<size_t>(count) * 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, cuda_stream_), "record readback");
         synchronize("prefill synchronize");
-        counters_.d2h_bytes += 16;
-        *sampled = host_records_[0];
+        counters_.d2h_bytes += static_cast<uint64_t>(count) * 16;
+        int row = 0;
+        for (PrefillPart &part : parts)
+            if (part.sample) part.sampled = host_records_[4 * row++];
     }
-    s.next_tick += count;
+    for (const PrefillPart &part : parts) part.stream->next_tick += part.count;
 }
 
 void Engine::emit(Stream &s, uint32_t token, uint64_t tick, const std::function<void(const OutputEvent &)> &on_output, RunReport &report) {
@@ -1877,11 +1946,9 @@ void Engine::run_single_ticks(std::vector<Stream *> &batch, const std::function<
                                  static_cast<uint16_t *>(draft_hidden_in_.ptr), lanes, static_cast<int>(plan.hidden), cuda_stream_),
               "gather pending hidden");
         draft_forward(lanes, static_cast<const uint16_t *>(draft_hidden_in_.ptr), false);
-        const size_t frame = static_cast<size_t>(plan.hidden) * 2;
-        for (int i = 0; i < lanes; i++)
-            cuda_check(cudaMemcpyAsync(static_cast<uint8_t *>(pending_hidden_.ptr) + batch[i]->slot * frame,
-                                       static_cast<uint8_t *>(normalized_.ptr) + i * frame, frame, cudaMemcpyDeviceToDevice, cuda_stream_),
-                       "commit target hidden");
+        check(launch_commit_hidden(static_cast<const uint16_t *>(normalized_.ptr), static_cast<const int32_t *>(lane_slots_.ptr),
+                                   static_cast<uint16_t *>(pending_hidden_.ptr), lanes, static_cast<int>(plan.hidden), cuda_stream_),
+              "commit target hidden");
     }
     if (any_emit) {
         cuda_check(cudaMemcpyAsync(host_records_, records_.ptr, lanes * 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, cuda_stream_),
@@ -2146,18 +2213,30 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
             works.push_back(Work{std::move(activation), &s, s.next_tick, s.active->generated.size(), {}});
         }
         try {
-        // 2. prefill chunks, one stream at a time
+        // 2. prefill chunks, as many streams' in one pass as the lanes allow
+        struct Pending {
+            Work *work;
+            size_t left;
+        };
+        std::vector<Pending> pending;
         for (Work &work : works) {
             if (work.activation.kind != runtime::ActivationKind::PrefillChunk) continue;
-            Stream &s = *work.stream;
-            ActiveEvent &event = *s.active;
+            const ActiveEvent &event = *work.stream->active;
             if (event.next_external != work.activation.token_offset || event.input.token_ids.size() < work.activation.token_offset + work.activation.token_ids.size())
                 fail("scheduler and engine disagree about the prompt position of stream " + work.activation.stream_id);
-            uint64_t start = now_ns();
-            size_t left = work.activation.token_ids.size();
-            const bool ends_prompt = work.activation.remaining_prompt_token_count == 0;
-            while (left > 0) {
-                int count = static_cast<int>(left);
+            pending.push_back(Pending{&work, work.activation.token_ids.size()});
+            report.activation_count++;
+        }
+        const uint64_t prefill_start = now_ns();
+        const bool any_prefill = !pending.empty();
+        while (!pending.empty()) {
+            std::vector<PrefillPart> parts;
+            std::vector<size_t> members;  // of pending
+            int lanes = 0;
+            for (size_t p = 0; p < pending.size(); p++) {
+                Stream &s = *pending[p].work->stream;
+                ActiveEvent &event = *s.active;
+                int count = static_cast<int>(pending[p].left);
                 // A batch appends the K/V of all its lanes before any lane attends.  Once the KV ring wraps, a later
                 // lane's slot is the one an earlier lane's window still ends in, and the reference runs the lanes one
                 // after the other (append_gqa_attention_bf16.comp.template:189-215 per tick).  So a chunk stops at the
@@ -2167,30 +2246,37 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
                 // with the prefix cache on, a chunk also stops at the prompt's last page boundary: the state there is retained
                 const uint64_t checkpoint_tick = prefix_checkpoint_tick(s);
                 if (checkpoint_tick > s.next_tick && checkpoint_tick < s.next_tick + static_cast<uint64_t>(count)) count = static_cast<int>(checkpoint_tick - s.next_tick);
-                const bool last = ends_prompt && static_cast<size_t>(count) == left;
-                const bool sample = last && event.remaining > 0;
-                uint32_t sampled = 0;
-                const uint64_t tick_of_last = s.next_tick + count - 1;
-                run_prefill_chunk(s, event.input.token_ids.data() + event.next_external, count, sample, &sampled);
-                if (prefix_cache_on() && s.history.size() + static_cast<size_t>(count) == s.next_tick) {
-                    s.history.insert(s.history.end(), event.input.token_ids.begin() + static_cast<std::ptrdiff_t>(event.next_external),
-                                     event.input.token_ids.begin() + static_cast<std::ptrdiff_t>(event.next_external + count));
-                    if (checkpoint_tick != 0 && s.next_tick == checkpoint_tick) capture_prefix_checkpoint(s);
+                if (!parts.empty() && (lanes + count > model_->options().max_lanes || (!ragged_prefill_ && count != parts[0].count) || (scalar_attention_ && (count >= 16) != (parts[0].count >= 16)))) continue;
+                const bool last = pending[p].work->activation.remaining_prompt_token_count == 0 && static_cast<size_t>(count) == pending[p].left;
+                parts.push_back(PrefillPart{&s, event.input.token_ids.data() + event.next_external, count, last && event.remaining > 0, last, 0, checkpoint_tick});
+                members.push_back(p);
+                lanes += count;
+            }
+            run_prefill_batch(parts);
+            for (size_t i = 0; i < parts.size(); i++) {
+                PrefillPart &part = parts[i];
+                Pending &entry = pending[members[i]];
+                Stream &s = *part.stream;
+                ActiveEvent &event = *s.active;
+                if (prefix_cache_on() && s.history.size() + static_cast<size_t>(part.count) == s.next_tick) {
+                    s.history.insert(s.history.end(), part.tokens, part.tokens + part.count);
+                    if (part.checkpoint_tick != 0 && s.next_tick == part.checkpoint_tick) capture_prefix_checkpoint(s);
                 }
-                event.next_external += count;
-                left -= static_cast<size_t>(count);
-                report.prefill_tokens += count;
-                if (sample) emit(s, sampled, tick_of_last, on_output, report);
-                else if (last) {
+                event.next_external += static_cast<size_t>(part.count);
+                entry.left -= static_cast<size_t>(part.count);
+                report.prefill_tokens += static_cast<uint64_t>(part.count);
+                if (part.sample) {
+                    emit(s, part.sampled, s.next_tick - 1, on_output, report);
+                } else if (part.last) {
                     synchronize("prefill synchronize");
-                    note_generated(work);
+                    note_generated(*entry.work);
                     s.active.reset();  // no public outputs requested: the event ends with the prompt
                     s.completed_events++;
                 }
             }
-            report.activation_count++;
-            report.prefill_ns += now_ns() - start;
+            pending.erase(std::remove_if(pending.begin(), pending.end(), [](const Pending &entry) { return entry.left == 0; }), pending.end());
         }
+        if (any_prefill) report.prefill_ns += now_ns() - prefill_start;
         // 3. decode windows: grouped into speculative cycles of equal draft count and single ticks
         std::map<int, std::vector<Stream *>> speculative;
         std::vector<Stream *> single;

@@ -331,7 +331,15 @@ private:
     // embedding -> layers -> final norm (-> logits -> argmax records)
     void target_forward(int lanes, bool want_logits);
     void draft_forward(int lanes, const uint16_t *hidden_in, bool want_logits);
-    void run_prefill_chunk(Stream &s, const uint32_t *tokens, int count, bool sample_last, uint32_t *sampled);
+    struct PrefillPart {  // a stream's chunk in a prefill batch
+        Stream *stream;
+        const uint32_t *tokens;
+        int count;
+        bool sample, last;         // the event's first token is sampled behind it; the event's prompt ends with it
+        uint32_t sampled;          // ... and the token
+        uint64_t checkpoint_tick;  // where the prompt's prefix is retained (0 = nowhere)
+    };
+    void run_prefill_batch(std::vector<PrefillPart> &parts);
     void run_single_ticks(std::vector<Stream *> &batch, const std::function<void(const OutputEvent &)> &on_output,
                           RunReport &report);
     void run_speculative_cycles(std::vector<Stream *> &batch, int draft_count,
@@ -417,6 +425,10 @@ private:
     int op_split_tokens_ = 128;             // tokens per split of decode batches on the kernel-per-operator path: fixed per engine, so
                                             // that a lane's arithmetic does not depend on the batch it runs in
     int current_op_split_tokens_ = 128, current_op_splits_ = 1;  // split length and count of the next launches on that path
+    DeviceBuffer attention_blocks_;         // row blocks of a ragged prefill batch
+    int current_blocks_ = 0;                // ... of the next launches (0: uniform batch)
+    int current_form_lanes_ = 0;            // lanes by which the next launches choose the form of a bf16 linear (0: the batch's)
+    bool ragged_prefill_ = false;           // one table of row blocks serves every layer (equal head shapes)
     bool scalar_attention_ = false;         // FP8 packages: the attention form in scalar f32
     size_t attention_partials_ = 0;         // partials attention_scratch_ holds
     int max_q_heads_ = 1;

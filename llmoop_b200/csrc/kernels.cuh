@@ -53,9 +53,10 @@ enum LinearEpilogue {
     EPILOGUE_F32_SCALED = 3,      // y_f32 = sum * scale                     (logits; tensor-parallel partial sums)
 };
 
-// y[m][n] = sum_k x[m][k] * W[n][k], bf16 weights.
+// y[m][n] = sum_k x[m][k] * W[n][k], bf16 weights.  form_lanes: choose the form (and so the order of additions) of a batch
+// of that many lanes.
 cudaError_t launch_linear_bf16(const uint16_t *x, const uint16_t *w, void *y, const uint16_t *residual, int lanes,
-                               int n, int k, int epilogue, float scale, cudaStream_t stream, int *error_flag = nullptr);
+                               int n, int k, int epilogue, float scale, cudaStream_t stream, int *error_flag = nullptr, int form_lanes = 0);
 // y = bf16( silu_bf16(bf16(x.Wg)) * bf16(x.Wu) )
 cudaError_t launch_linear_silu_multiply_bf16(const uint16_t *x, const uint16_t *wg, const uint16_t *wu, uint16_t *y,
                                              int lanes, int n, int k, cudaStream_t stream);
@@ -118,12 +119,18 @@ struct RopeAppend {
 cudaError_t launch_rope_append(const RopeAppend &rope, const KvLayer &kv, const LaneTable &lanes_meta, int lanes, cudaStream_t stream);
 // Causal GQA attention over the stream's pages, split over the context: split s covers split_tokens tokens, partials are
 // merged by a second kernel (max_splits 1: none).  scratch holds [lanes][q_heads][max_splits][head_width + 2] f32.
-// Lanes are stream-major: every stream of the batch contributes `lanes_per_stream` consecutive lanes.
+// Lanes are stream-major: every stream of the batch contributes `lanes_per_stream` consecutive lanes - or, in a ragged
+// batch, up to as many, described by a device array of blocks of attention_block_lanes lanes of one stream each.
 // scalar_f32: the form for layers whose attention output is quantised to FP8.
+struct AttentionBlock {
+    int first_lane, lanes;  // of the stream
+    int index;              // of the block in the stream
+};
+int attention_block_lanes(int lanes_per_stream, int q_heads, int kv_heads, int head_width, bool scalar_f32);
 bool attention_is_prefill(int lanes_per_stream, int q_heads, int kv_heads);  // the form with 128 query rows per CTA
 cudaError_t launch_attention(const uint16_t *q, uint16_t *out, const KvLayer &kv, const LaneTable &lanes_meta,
                              int lanes, int lanes_per_stream, int q_heads, float scale, int split_tokens, int max_splits,
-                             float *scratch, bool scalar_f32, cudaStream_t stream);
+                             float *scratch, bool scalar_f32, cudaStream_t stream, const AttentionBlock *blocks = nullptr, int block_count = 0);
 
 // INT4 multi-branch forms (one launch for q/k/v; gate/up with the SiLU*up epilogue).
 cudaError_t launch_linear_int4_multi(const uint16_t *x, const void *prepared, int branches, const uint32_t *const *qweights,
@@ -277,6 +284,11 @@ cudaError_t launch_gather_rows(const uint16_t *src, const int32_t *index, uint16
 // Hidden inputs of the draft catch-up: lane (s, 0) takes pending[slot[s]], lane (s, i>0) takes normalized (s, i-1).
 cudaError_t launch_shift_hidden(const uint16_t *pending, const int32_t *slots, const uint16_t *normalized,
                                 uint16_t *dst, int streams, int lanes_per_stream, int hidden, cudaStream_t stream);
+// The same for lanes of any number per stream (neighbouring lanes of one slot are one stream's), and the way back: the
+// normalised frame of every stream's last lane becomes its pending hidden state.
+cudaError_t launch_shift_hidden_lanes(const uint16_t *pending, const int32_t *slots, const uint16_t *normalized, uint16_t *dst, int lanes, int hidden,
+                                      cudaStream_t stream);
+cudaError_t launch_commit_hidden(const uint16_t *normalized, const int32_t *slots, uint16_t *pending, int lanes, int hidden, cudaStream_t stream);
 // After draft step `step`: token = forced[s][step] unless it is 0xffffffff, else the sampled record; written to
 // next_tokens[s] and verify_tokens[s][step + 1].
 cudaError_t launch_draft_select(const uint32_t *records, const uint32_t *forced, int step, int streams, int drafts,

@@ -73,6 +73,7 @@ struct AttentionArgs {
     float scale;
     int split_tokens, max_splits;
     float *scratch;
+    const AttentionBlock *blocks;  // ragged batches: what each block of rows covers; nullptr: lanes_per_stream lanes per stream
 };
 
 template <int HD, int ROW_WARPS, int TOKEN_WARPS>
@@ -95,9 +96,18 @@ __global__ void __launch_bounds__(ROW_WARPS *TOKEN_WARPS * 32) attention_tile_ke
     const int row_warp = warp / TOKEN_WARPS, token_warp = warp % TOKEN_WARPS;
     // the blocks with the longest contexts (the last rows of a chunk) start first
     const int block = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x), kv_head = blockIdx.y, split = blockIdx.z;
-    const int stream = block / a.row_blocks, row0 = (block - stream * a.row_blocks) * ROWS;
-    const int rows = a.lanes_per_stream * a.group;
-    const int lane0 = stream * a.lanes_per_stream;
+    int lane0, rows, row0;
+    if (a.blocks != nullptr) {
+        const AttentionBlock entry = a.blocks[block];
+        lane0 = entry.first_lane;
+        rows = entry.lanes * a.group;
+        row0 = entry.index * ROWS;
+    } else {
+        const int stream = block / a.row_blocks;
+        lane0 = stream * a.lanes_per_stream;
+        rows = a.lanes_per_stream * a.group;
+        row0 = (block - stream * a.row_blocks) * ROWS;
+    }
     const int slot = a.meta.slot[lane0];
     if (slot < 0) return;
     const uint32_t capacity = a.kv.capacity;
@@ -353,8 +363,8 @@ constexpr size_t attention_f32_smem() {
 template <int HD, int GROUP, int QL>
 __device__ void attention_f32_body(const uint16_t *__restrict__ q, const KvLayer &kv, const LaneTable &lanes_meta, int lanes,
                                    int lanes_per_stream, int q_heads, float scale, int split_tokens, int max_splits,
-                                   float *__restrict__ scratch, int kv_head, int split, int group_slot, uint8_t *smem_raw,
-                                   int tid) {
+                                   float *__restrict__ scratch, const AttentionBlock *__restrict__ ragged, int kv_head, int split, int group_slot,
+                                   uint8_t *smem_raw, int tid) {
     constexpr int Q = QL * GROUP;
     constexpr int KSTRIDE = HD + 8;
     constexpr int DPT = HD / 128 > 0 ? HD / 128 : 1;  // output dims per thread (HD = 128 -> 1)
@@ -369,8 +379,14 @@ __device__ void attention_f32_body(const uint16_t *__restrict__ q, const KvLayer
 
     // lanes of one stream are consecutive and every stream of the batch has `lanes_per_stream` of them
     const int groups_per_stream = (lanes_per_stream + QL - 1) / QL;
-    const int stream_index = group_slot / groups_per_stream, group_index = group_slot % groups_per_stream;
-    const int lane0 = stream_index * lanes_per_stream + group_index * QL;
+    const int stream_index = group_slot / groups_per_stream;
+    int group_index = group_slot % groups_per_stream, lane0 = stream_index * lanes_per_stream + group_index * QL;
+    if (ragged != nullptr) {
+        const AttentionBlock entry = ragged[group_slot];
+        group_index = entry.index;
+        lane0 = entry.first_lane + entry.index * QL;
+        lanes_per_stream = entry.lanes;
+    }
     if (lane0 >= lanes) return;
     const int slot = lanes_meta.slot[lane0];
     if (slot < 0) return;
@@ -524,12 +540,12 @@ __device__ void attention_f32_body(const uint16_t *__restrict__ q, const KvLayer
 template <int HD, int GROUP, int QL>
 __global__ void __launch_bounds__(128)
 attention_f32_kernel(const uint16_t *__restrict__ q, KvLayer kv, LaneTable lanes_meta, int lanes, int lanes_per_stream,
-                     int q_heads, float scale, int split_tokens, int max_splits, float *__restrict__ scratch) {
+                     int q_heads, float scale, int split_tokens, int max_splits, float *__restrict__ scratch, const AttentionBlock *__restrict__ ragged) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     grid_launch_dependents();
     grid_dependency_wait();
-    attention_f32_body<HD, GROUP, QL>(q, kv, lanes_meta, lanes, lanes_per_stream, q_heads, scale, split_tokens, max_splits, scratch, blockIdx.x, blockIdx.y,
-                                      blockIdx.z, smem_raw, threadIdx.x);
+    attention_f32_body<HD, GROUP, QL>(q, kv, lanes_meta, lanes, lanes_per_stream, q_heads, scale, split_tokens, max_splits, scratch, ragged, blockIdx.x,
+                                      blockIdx.y, blockIdx.z, smem_raw, threadIdx.x);
 }
 
 // Log-sum-exp merge of the split partials of one (lane, q head) pair by one warp.
@@ -579,9 +595,10 @@ cudaError_t launch_f32(const AttentionArgs &a, cudaStream_t stream) {
     constexpr size_t smem = attention_f32_smem<HD, GROUP, QL>();
     cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (status != cudaSuccess) return status;
-    const dim3 grid(a.kv.kv_heads, a.max_splits, a.lanes / a.lanes_per_stream * ((a.lanes_per_stream + QL - 1) / QL));
+    const int groups = a.blocks != nullptr ? a.row_blocks : a.lanes / a.lanes_per_stream * ((a.lanes_per_stream + QL - 1) / QL);
+    const dim3 grid(a.kv.kv_heads, a.max_splits, groups);
     status = launch_dependent(kernel, grid, dim3(128), smem, 1, stream, a.q, a.kv, a.meta, a.lanes, a.lanes_per_stream, a.q_heads, a.scale, a.split_tokens,
-                              a.max_splits, a.scratch);
+                              a.max_splits, a.scratch, a.blocks);
     if (status != cudaSuccess) return status;
     return launch_dependent(attention_f32_merge_kernel, dim3((a.lanes * a.q_heads + 3) / 4), dim3(128), 0, 1, stream, a.scratch, a.out, a.kv, a.meta, a.lanes,
                             a.q_heads, a.kv.head_width, a.split_tokens, a.max_splits);
@@ -714,8 +731,8 @@ template <int HD>
 cudaError_t launch_tiles_of_width(AttentionArgs args, int streams, cudaStream_t stream) {
     const int rows = args.lanes_per_stream * args.group;
     auto grid = [&](int block_rows) {
-        args.row_blocks = (rows + block_rows - 1) / block_rows;
-        return dim3(static_cast<unsigned int>(streams * args.row_blocks), static_cast<unsigned int>(args.kv.kv_heads), static_cast<unsigned int>(args.max_splits));
+        if (args.blocks == nullptr) args.row_blocks = (rows + block_rows - 1) / block_rows;
+        return dim3(static_cast<unsigned int>(args.blocks != nullptr ? args.row_blocks : streams * args.row_blocks), static_cast<unsigned int>(args.kv.kv_heads), static_cast<unsigned int>(args.max_splits));
     };
     if (attention_is_prefill(args.lanes_per_stream, args.q_heads, args.kv.kv_heads)) {
         const dim3 blocks = grid(128);
@@ -735,11 +752,19 @@ cudaError_t launch_tiles_of_width(AttentionArgs args, int streams, cudaStream_t 
 // context three times at most, and from there on the 128-row form wastes less than it saves.
 bool attention_is_prefill(int lanes_per_stream, int q_heads, int kv_heads) { return lanes_per_stream * (q_heads / kv_heads) > 96; }
 
+int attention_block_lanes(int lanes_per_stream, int q_heads, int kv_heads, int head_width, bool scalar_f32) {
+    const int group = q_heads / kv_heads;
+    if ((head_width != 64 && head_width != 128) || (group != 1 && group != 2 && group != 4 && group != 8)) return 1;
+    if (scalar_f32) return group == 8 ? 2 : 4;
+    const int rows = lanes_per_stream * group;
+    return (attention_is_prefill(lanes_per_stream, q_heads, kv_heads) ? 128 : rows <= 16 ? 16 : 32) / group;
+}
+
 cudaError_t launch_attention(const uint16_t *q, uint16_t *out, const KvLayer &kv, const LaneTable &lanes_meta,
                              int lanes, int lanes_per_stream, int q_heads, float scale, int split_tokens, int max_splits,
-                             float *scratch, bool scalar_f32, cudaStream_t stream) {
+                             float *scratch, bool scalar_f32, cudaStream_t stream, const AttentionBlock *blocks, int block_count) {
     if (lanes <= 0) return cudaSuccess;
-    if (lanes_per_stream <= 0 || lanes % lanes_per_stream != 0) return cudaErrorInvalidValue;
+    if (lanes_per_stream <= 0 || (blocks == nullptr && lanes % lanes_per_stream != 0)) return cudaErrorInvalidValue;
     const int group = q_heads / kv.kv_heads;
     const bool wide = kv.head_width == 64 || kv.head_width == 128;
     if (!wide || (group != 1 && group != 2 && group != 4 && group != 8)) {
@@ -759,6 +784,8 @@ cudaError_t launch_attention(const uint16_t *q, uint16_t *out, const KvLayer &kv
     args.split_tokens = split_tokens;
     args.max_splits = max_splits;
     args.scratch = scratch;
+    args.blocks = blocks;
+    args.row_blocks = block_count;
     if (scalar_f32) return kv.head_width == 128 ? launch_f32_of_width<128>(args, stream) : launch_f32_of_width<64>(args, stream);
     const int streams = lanes / lanes_per_stream;
     cudaError_t status = kv.head_width == 128 ? launch_tiles_of_width<128>(args, streams, stream) : launch_tiles_of_width<64>(args, streams, stream);
@@ -879,6 +906,7 @@ __device__ __forceinline__ void argmax_block_reduce(float &best, uint32_t &token
 
 __global__ void argmax_partial_kernel(const float *__restrict__ logits, float *__restrict__ partial_logit,
                                       uint32_t *__restrict__ partial_token, int vocab) {
+    grid_launch_dependents();
     grid_dependency_wait();
     __shared__ float shared_logit[32];
     __shared__ uint32_t shared_token[32];
@@ -904,6 +932,7 @@ __global__ void argmax_partial_kernel(const float *__restrict__ logits, float *_
 
 __global__ void argmax_final_kernel(const float *__restrict__ partial_logit, const uint32_t *__restrict__ partial_token,
                                     uint32_t *__restrict__ records) {
+    grid_launch_dependents();
     grid_dependency_wait();
     __shared__ float shared_logit[32];
     __shared__ uint32_t shared_token[32];
@@ -927,11 +956,9 @@ cudaError_t launch_argmax(const float *logits, uint32_t *records, int lanes, int
     float *partial_logit = static_cast<float *>(scratch);
     uint32_t *partial_token = reinterpret_cast<uint32_t *>(partial_logit + static_cast<size_t>(lanes) * ARGMAX_CHUNKS);
     dim3 grid(ARGMAX_CHUNKS, lanes);
-    argmax_partial_kernel<<<grid, 256, 0, stream>>>(logits, partial_logit, partial_token, vocab);
-    cudaError_t status = cudaGetLastError();
+    cudaError_t status = launch_dependent(argmax_partial_kernel, grid, dim3(256), 0, 1, stream, logits, partial_logit, partial_token, vocab);
     if (status != cudaSuccess) return status;
-    argmax_final_kernel<<<lanes, ARGMAX_CHUNKS, 0, stream>>>(partial_logit, partial_token, records);
-    return cudaGetLastError();
+    return launch_dependent(argmax_final_kernel, dim3(lanes), dim3(ARGMAX_CHUNKS), 0, 1, stream, partial_logit, partial_token, records);
 }
 
 // ---- greedy arg-max without a caller-provided scratch buffer -------------------------------------------------

@@ -4,11 +4,13 @@
 // so that one cycle is a single stream of launches with one host read-back.
 #include "common.cuh"
 #include "kernels.cuh"
+#include "launch.cuh"
 
 namespace nerve {
 
 __global__ void gather_rows_kernel(const uint32_t *__restrict__ src, const int32_t *__restrict__ index,
                                    uint32_t *__restrict__ dst, int words) {
+    grid_launch_dependents();
     grid_dependency_wait();
     int row = blockIdx.x;
     int source = index[row];
@@ -20,14 +22,13 @@ __global__ void gather_rows_kernel(const uint32_t *__restrict__ src, const int32
 cudaError_t launch_gather_rows(const uint16_t *src, const int32_t *index, uint16_t *dst, int rows, int width,
                                cudaStream_t stream) {
     if (rows <= 0) return cudaSuccess;
-    gather_rows_kernel<<<rows, 256, 0, stream>>>(reinterpret_cast<const uint32_t *>(src), index,
-                                                 reinterpret_cast<uint32_t *>(dst), width / 2);
-    return cudaGetLastError();
+    return launch_dependent(gather_rows_kernel, dim3(rows), dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(src), index, reinterpret_cast<uint32_t *>(dst), width / 2);
 }
 
 __global__ void shift_hidden_kernel(const uint32_t *__restrict__ pending, const int32_t *__restrict__ slots,
                                     const uint32_t *__restrict__ normalized, uint32_t *__restrict__ dst,
                                     int lanes_per_stream, int words) {
+    grid_launch_dependents();
     grid_dependency_wait();
     int lane = blockIdx.x;
     int s = lane / lanes_per_stream, i = lane % lanes_per_stream;
@@ -39,15 +40,44 @@ __global__ void shift_hidden_kernel(const uint32_t *__restrict__ pending, const 
 cudaError_t launch_shift_hidden(const uint16_t *pending, const int32_t *slots, const uint16_t *normalized,
                                 uint16_t *dst, int streams, int lanes_per_stream, int hidden, cudaStream_t stream) {
     if (streams <= 0) return cudaSuccess;
-    shift_hidden_kernel<<<streams * lanes_per_stream, 256, 0, stream>>>(
-        reinterpret_cast<const uint32_t *>(pending), slots, reinterpret_cast<const uint32_t *>(normalized),
-        reinterpret_cast<uint32_t *>(dst), lanes_per_stream, hidden / 2);
-    return cudaGetLastError();
+    return launch_dependent(shift_hidden_kernel, dim3(streams * lanes_per_stream), dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(pending), slots, reinterpret_cast<const uint32_t *>(normalized), reinterpret_cast<uint32_t *>(dst), lanes_per_stream, hidden / 2);
+}
+
+// Prefill batches: the lanes of a stream are neighbours, a lane whose neighbour has another slot is its stream's first or last.
+__global__ void shift_hidden_lanes_kernel(const uint32_t *__restrict__ pending, const int32_t *__restrict__ slots, const uint32_t *__restrict__ normalized,
+                                          uint32_t *__restrict__ dst, int words) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int lane = blockIdx.x;
+    const bool first = lane == 0 || slots[lane - 1] != slots[lane];
+    const uint32_t *source = first ? pending + static_cast<size_t>(slots[lane]) * words : normalized + static_cast<size_t>(lane - 1) * words;
+    for (int word = threadIdx.x; word < words; word += blockDim.x) dst[static_cast<size_t>(lane) * words + word] = source[word];
+}
+cudaError_t launch_shift_hidden_lanes(const uint16_t *pending, const int32_t *slots, const uint16_t *normalized, uint16_t *dst, int lanes, int hidden,
+                                      cudaStream_t stream) {
+    if (lanes <= 0) return cudaSuccess;
+    return launch_dependent(shift_hidden_lanes_kernel, dim3(lanes), dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(pending), slots,
+                            reinterpret_cast<const uint32_t *>(normalized), reinterpret_cast<uint32_t *>(dst), hidden / 2);
+}
+
+__global__ void commit_hidden_kernel(const uint32_t *__restrict__ normalized, const int32_t *__restrict__ slots, uint32_t *__restrict__ pending, int words) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int lane = blockIdx.x;
+    if (lane + 1 < static_cast<int>(gridDim.x) && slots[lane + 1] == slots[lane]) return;
+    for (int word = threadIdx.x; word < words; word += blockDim.x)
+        pending[static_cast<size_t>(slots[lane]) * words + word] = normalized[static_cast<size_t>(lane) * words + word];
+}
+cudaError_t launch_commit_hidden(const uint16_t *normalized, const int32_t *slots, uint16_t *pending, int lanes, int hidden, cudaStream_t stream) {
+    if (lanes <= 0) return cudaSuccess;
+    return launch_dependent(commit_hidden_kernel, dim3(lanes), dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(normalized), slots,
+                            reinterpret_cast<uint32_t *>(pending), hidden / 2);
 }
 
 __global__ void draft_select_kernel(const uint32_t *__restrict__ records, const uint32_t *__restrict__ forced, int step,
                                     int streams, int drafts, uint32_t *__restrict__ next_tokens,
                                     uint32_t *__restrict__ verify_tokens) {
+    grid_launch_dependents();
     grid_dependency_wait();
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= streams) return;
@@ -63,15 +93,14 @@ __global__ void draft_select_kernel(const uint32_t *__restrict__ records, const 
 cudaError_t launch_draft_select(const uint32_t *records, const uint32_t *forced, int step, int streams, int drafts,
                                 uint32_t *next_tokens, uint32_t *verify_tokens, cudaStream_t stream) {
     if (streams <= 0) return cudaSuccess;
-    draft_select_kernel<<<(streams + 63) / 64, 64, 0, stream>>>(records, forced, step, streams, drafts, next_tokens,
-                                                                verify_tokens);
-    return cudaGetLastError();
+    return launch_dependent(draft_select_kernel, dim3((streams + 63) / 64), dim3(64), 0, 1, stream, records, forced, step, streams, drafts, next_tokens, verify_tokens);
 }
 
 __global__ void accept_kernel(const uint32_t *__restrict__ verify_tokens, const uint32_t *__restrict__ target_records,
                               const uint32_t *__restrict__ stop_tokens, const int32_t *__restrict__ stop_counts,
                               int max_stop, int drafts, uint32_t *__restrict__ out, const uint32_t *__restrict__ normalized,
                               uint32_t *__restrict__ pending, const int32_t *__restrict__ slots, int words) {
+    grid_launch_dependents();
     grid_dependency_wait();
     __shared__ int committed_shared;
     const int s = blockIdx.x;
@@ -114,10 +143,7 @@ cudaError_t launch_accept(const uint32_t *verify_tokens, const uint32_t *target_
                           const uint16_t *normalized, uint16_t *pending, const int32_t *slots, int hidden,
                           cudaStream_t stream) {
     if (streams <= 0) return cudaSuccess;
-    accept_kernel<<<streams, 256, 0, stream>>>(verify_tokens, target_records, stop_tokens, stop_counts, max_stop, drafts,
-                                               out, reinterpret_cast<const uint32_t *>(normalized),
-                                               reinterpret_cast<uint32_t *>(pending), slots, hidden / 2);
-    return cudaGetLastError();
+    return launch_dependent(accept_kernel, dim3(streams), dim3(256), 0, 1, stream, verify_tokens, target_records, stop_tokens, stop_counts, max_stop, drafts, out, reinterpret_cast<const uint32_t *>(normalized), reinterpret_cast<uint32_t *>(pending), slots, hidden / 2);
 }
 
 // ---- vocabulary-parallel arg-max ------------------------------------------------------------------------------
@@ -184,8 +210,7 @@ cudaError_t launch_tensor_parallel_argmax(const uint32_t *records_local, uint32_
                                           int *error_flag, cudaStream_t stream) {
     if (lanes <= 0) return cudaSuccess;
     if (lanes > STACK_TP_VOTE_LANES || tp_device == nullptr) return cudaErrorInvalidValue;
-    tensor_parallel_argmax_kernel<<<1, STACK_TP_VOTE_LANES, 0, stream>>>(records_local, first_token, records, lanes, tp_device, error_flag);
-    return cudaGetLastError();
+    return launch_dependent(tensor_parallel_argmax_kernel, dim3(1), dim3(STACK_TP_VOTE_LANES), 0, 1, stream, records_local, first_token, records, lanes, tp_device, error_flag);
 }
 
 }  // namespace nerve

@@ -86,12 +86,14 @@ __device__ __forceinline__ void stage_activations(const uint8_t *__restrict__ xq
     }
 }
 
-// Sums of FP8_ROWS rows x M lanes over all of K; rows 0..3 and 4..7 may have scale rows of their own (gate and up).
-// On return thread t holds the outputs sum_index(t, i), i < FP8_ROWS * M / 32 (or the one of its thread pair for M = 2).
+// Sums of ROWS rows x M lanes over all of K; the two halves of the rows may have scale rows of their own (gate and up).
+// Eight lanes take four rows at a time (the partial sums of more do not fit the registers of two CTAs per SM), fewer
+// lanes eight.  On return thread t holds the outputs index(t, i) (or the one of its thread pair for M = 2).
 template <int M>
 struct RowSums {
-    static constexpr int VALUES = FP8_ROWS * M, PER_THREAD = VALUES >= 32 ? VALUES / 32 : 1;
-    static constexpr int PIPE = M == 8 ? 1 : 4;  // blocks of weights in flight: eight lanes are bound by arithmetic, not latency
+    static constexpr int ROWS = M == 8 ? 4 : 8;
+    static constexpr int VALUES = ROWS * M, PER_THREAD = VALUES >= 32 ? VALUES / 32 : 1;
+    static constexpr int PIPE = M == 2 ? 4 : 2;  // blocks of weights in flight
     float sums[PER_THREAD];
 
     // output index = row * M + lane
@@ -101,27 +103,27 @@ struct RowSums {
         return thread >> 1;  // sixteen values: the last butterfly step leaves both threads of a pair with the same one
     }
 
-    // stage(first, n) brings the activations of blocks first .. first + n - 1 into x
+    // stage(first, n) brings the activations of blocks first .. first + n - 1 into x (which may hold all of them already)
     template <typename RowPointer, typename Stage>
-    __device__ void run(RowPointer row_pointer, const uint16_t *__restrict__ scales_a, const uint16_t *__restrict__ scales_b, int blocks, float *x, Stage stage_blocks) {
+    __device__ void run(RowPointer row_pointer, const uint16_t *__restrict__ scales_a, const uint16_t *__restrict__ scales_b, int blocks, float *x, bool staged_already, Stage stage_blocks) {
         const float *x_scales = x + static_cast<size_t>(CHUNK) * 128 * M;
         const int thread = threadIdx.x & 31;
-        const uint32_t *source[FP8_ROWS];
+        const uint32_t *source[ROWS];
 #pragma unroll
-        for (int r = 0; r < FP8_ROWS; r++) source[r] = reinterpret_cast<const uint32_t *>(row_pointer(r)) + thread;
-        uint32_t words[PIPE][FP8_ROWS];
+        for (int r = 0; r < ROWS; r++) source[r] = reinterpret_cast<const uint32_t *>(row_pointer(r)) + thread;
+        uint32_t words[PIPE][ROWS];
 #pragma unroll
         for (int p = 0; p < PIPE; p++)
 #pragma unroll
-            for (int r = 0; r < FP8_ROWS; r++) words[p][r] = p < blocks ? __ldg(source[r] + p * 32) : 0u;
-        pair_t acc[FP8_ROWS][M / 2];
+            for (int r = 0; r < ROWS; r++) words[p][r] = p < blocks ? __ldg(source[r] + p * 32) : 0u;
+        pair_t acc[ROWS][M / 2];
 #pragma unroll
-        for (int r = 0; r < FP8_ROWS; r++)
+        for (int r = 0; r < ROWS; r++)
 #pragma unroll
             for (int p = 0; p < M / 2; p++) acc[r][p] = 0ull;
         for (int base = 0; base < blocks; base += PIPE) {
-            if (base % CHUNK == 0) {
-                if (base > 0) __syncthreads();
+            if (base % CHUNK == 0 && (!staged_already || blocks > CHUNK)) {
+                __syncthreads();
                 stage_blocks(base, min(CHUNK, blocks - base));
                 __syncthreads();
             }
@@ -144,7 +146,7 @@ struct RowSums {
                     sb[p] = mul(xs, pack(wb, wb));
                 }
 #pragma unroll
-                for (int r = 0; r < FP8_ROWS; r++) {
+                for (int r = 0; r < ROWS; r++) {
                     float w[4];
                     widen(words[stage][r], w);
                     const pair_t w2[4] = {pack(w[0], w[0]), pack(w[1], w[1]), pack(w[2], w[2]), pack(w[3], w[3])};
@@ -154,7 +156,7 @@ struct RowSums {
                         d = fma2(xv[p][1], w2[1], d);
                         d = fma2(xv[p][2], w2[2], d);
                         d = fma2(xv[p][3], w2[3], d);
-                        acc[r][p] = fma2(d, r < FP8_ROWS / 2 ? sa[p] : sb[p], acc[r][p]);
+                        acc[r][p] = fma2(d, r < ROWS / 2 ? sa[p] : sb[p], acc[r][p]);
                     }
                     words[stage][r] = block + PIPE < blocks ? __ldg(source[r] + (block + PIPE) * 32) : 0u;
                 }
@@ -163,7 +165,7 @@ struct RowSums {
         // butterfly over the threads: at every step a thread keeps half of its values and passes on the other half
         float v[VALUES];
 #pragma unroll
-        for (int r = 0; r < FP8_ROWS; r++)
+        for (int r = 0; r < ROWS; r++)
 #pragma unroll
             for (int p = 0; p < M / 2; p++) {
                 const float2 both = unpack(acc[r][p]);
@@ -205,28 +207,30 @@ struct Fp8LinearArgs {
     uint16_t *y;
     const uint16_t *residual;
     int lanes, n, k, epilogue;
+    int passes;  // a CTA covers 32 or 64 rows (1 or 2)
 };
 
 template <int M>
 __device__ __forceinline__ void fp8_linear_tile(const Fp8LinearArgs &a, int m0, int count, float *smem) {
     const int warp = threadIdx.x >> 5, thread = threadIdx.x & 31, blocks = a.k >> 7;
     auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, a.k, first, n, count, smem, [&](int m) { return m0 + m; }); };
-    const int row0 = (blockIdx.x * FP8_WARPS + warp) * FP8_ROWS;
-    RowSums<M> sums;
-    const uint16_t *scale_row[2];
+    const int warps = 32 * a.passes / RowSums<M>::ROWS;  // with rows to do in a pass
+    for (int pass = 0; pass < (warps > FP8_WARPS ? 2 : 1); pass++) {
+        const int row0 = blockIdx.x * 32 * a.passes + (pass * FP8_WARPS + warp) * RowSums<M>::ROWS;
+        RowSums<M> sums;
+        const uint16_t *scale_row = a.wscale[0] + static_cast<size_t>(min(row0, a.n - 1) >> 7) * blocks;  // eight rows lie in one block of 128
+        sums.run([&](int r) { return a.w[0] + static_cast<size_t>(min(row0 + r, a.n - 1)) * a.k; }, scale_row, scale_row, blocks, smem, pass > 0, stage);
+        if (RowSums<M>::VALUES < 32 && (thread & 1) != 0) continue;
 #pragma unroll
-    for (int h = 0; h < 2; h++) scale_row[h] = a.wscale[0] + static_cast<size_t>(min(row0 + 4 * h, a.n - 1) >> 7) * blocks;
-    sums.run([&](int r) { return a.w[0] + static_cast<size_t>(min(row0 + r, a.n - 1)) * a.k; }, scale_row[0], scale_row[1], blocks, smem, stage);
-    if (RowSums<M>::VALUES < 32 && (thread & 1) != 0) return;
-#pragma unroll
-    for (int i = 0; i < RowSums<M>::PER_THREAD; i++) {
-        const int output = RowSums<M>::index(thread, i), row = row0 + output / M, m = output % M;
-        if (row >= a.n || m >= count) continue;
-        const size_t out = static_cast<size_t>(m0 + m) * a.n + row;
-        float sum = sums.sums[i];
-        if (a.epilogue == EPILOGUE_RESIDUAL_F32) sum = bf16_bits_to_f32(a.residual[out]) + sum;
-        else if (a.epilogue == EPILOGUE_RESIDUAL_ROUNDED) sum = round_bf16(sum) + bf16_bits_to_f32(a.residual[out]);
-        a.y[out] = static_cast<uint16_t>(f32_to_bf16_bits(sum));
+        for (int i = 0; i < RowSums<M>::PER_THREAD; i++) {
+            const int output = RowSums<M>::index(thread, i), row = row0 + output / M, m = output % M;
+            if (row >= a.n || m >= count || warp >= warps) continue;
+            const size_t out = static_cast<size_t>(m0 + m) * a.n + row;
+            float sum = sums.sums[i];
+            if (a.epilogue == EPILOGUE_RESIDUAL_F32) sum = bf16_bits_to_f32(a.residual[out]) + sum;
+            else if (a.epilogue == EPILOGUE_RESIDUAL_ROUNDED) sum = round_bf16(sum) + bf16_bits_to_f32(a.residual[out]);
+            a.y[out] = static_cast<uint16_t>(f32_to_bf16_bits(sum));
+        }
     }
 }
 
@@ -240,7 +244,7 @@ __global__ void __launch_bounds__(FP8_WARPS * 32, 2) linear_fp8_kernel(const __g
              [&] { fp8_linear_tile<8>(a, m0, count, fp8_smem); });
 }
 
-// rounded_silu(round(gate)) * round(up) from a warp's sums: rows 0..3 gate, rows 4..7 the same rows of up
+// rounded_silu(round(gate)) * round(up) from a warp's sums: the first half of the rows is gate, the second the same rows of up
 template <int M, typename Store>
 __device__ __forceinline__ void silu_outputs(const RowSums<M> &sums, Store store) {
     const int thread = threadIdx.x & 31;
@@ -261,14 +265,18 @@ template <int M>
 __device__ __forceinline__ void fp8_silu_tile(const Fp8LinearArgs &a, int m0, int count, float *smem) {
     const int warp = threadIdx.x >> 5, blocks = a.k >> 7;
     auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, a.k, first, n, count, smem, [&](int m) { return m0 + m; }); };
-    const int row0 = (blockIdx.x * FP8_WARPS + warp) * (FP8_ROWS / 2), first = min(row0, a.n - 1);
-    RowSums<M> sums;
-    sums.run([&](int r) { return a.w[r / 4] + static_cast<size_t>(min(row0 + (r & 3), a.n - 1)) * a.k; }, a.wscale[0] + static_cast<size_t>(first >> 7) * blocks,
-             a.wscale[1] + static_cast<size_t>(first >> 7) * blocks, blocks, smem, stage);
-    silu_outputs<M>(sums, [&](int r, int m, float gate, float up) {
-        if (row0 + r >= a.n || m >= count) return;
-        a.y[static_cast<size_t>(m0 + m) * a.n + row0 + r] = static_cast<uint16_t>(f32_to_bf16_bits(rounded_silu(gate) * up));
-    });
+    constexpr int HALF = RowSums<M>::ROWS / 2;
+    const int warps = 32 * a.passes / RowSums<M>::ROWS;
+    for (int pass = 0; pass < (warps > FP8_WARPS ? 2 : 1); pass++) {
+        const int row0 = blockIdx.x * 16 * a.passes + (pass * FP8_WARPS + warp) * HALF, first = min(row0, a.n - 1);
+        RowSums<M> sums;
+        sums.run([&](int r) { return a.w[r / HALF] + static_cast<size_t>(min(row0 + r % HALF, a.n - 1)) * a.k; }, a.wscale[0] + static_cast<size_t>(first >> 7) * blocks,
+                 a.wscale[1] + static_cast<size_t>(first >> 7) * blocks, blocks, smem, pass > 0, stage);
+        silu_outputs<M>(sums, [&](int r, int m, float gate, float up) {
+            if (row0 + r >= a.n || m >= count || warp >= warps) return;
+            a.y[static_cast<size_t>(m0 + m) * a.n + row0 + r] = static_cast<uint16_t>(f32_to_bf16_bits(rounded_silu(gate) * up));
+        });
+    }
 }
 
 __global__ void __launch_bounds__(FP8_WARPS * 32, 2) linear_silu_multiply_fp8_kernel(const __grid_constant__ Fp8LinearArgs a) {
@@ -351,17 +359,21 @@ __device__ __forceinline__ void moe_gate_up_tile(const MoeArgs &a, int4 tile, fl
     const int warp = threadIdx.x >> 5, k = a.hidden, blocks = k >> 7, count = tile.z;
     const int *order = a.groups.order + tile.y;
     auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, k, first, n, count, smem, [&](int m) { return order[m] / a.top_k; }); };
-    const int row0 = (blockIdx.x * FP8_WARPS + warp) * (FP8_ROWS / 2), expert = tile.x - a.expert_start, first = min(row0, a.inter - 1);
+    constexpr int HALF = RowSums<M>::ROWS / 2;
+    const int expert = tile.x - a.expert_start;
     const uint8_t *w = a.w + static_cast<size_t>(expert) * 2 * a.inter * k;
     const uint16_t *ws = a.wscale + static_cast<size_t>(expert) * ((2 * a.inter + 127) >> 7) * blocks;
-    RowSums<M> sums;
-    sums.run([&](int r) { return w + static_cast<size_t>((r >= 4 ? a.inter : 0) + min(row0 + (r & 3), a.inter - 1)) * k; },
-             ws + static_cast<size_t>(first >> 7) * blocks, ws + static_cast<size_t>((a.inter + first) >> 7) * blocks, blocks, smem, stage);
-    silu_outputs<M>(sums, [&](int r, int m, float gate, float up) {
-        if (row0 + r >= a.inter || m >= count) return;
-        const float value = round_bf16(round_bf16(gate / (1.0f + expf(-gate))) * up);
-        a.out[static_cast<size_t>(order[m]) * a.inter + row0 + r] = static_cast<uint16_t>(f32_to_bf16_bits(value));
-    });
+    for (int pass = 0; pass < FP8_ROWS / RowSums<M>::ROWS; pass++) {
+        const int row0 = (blockIdx.x * FP8_WARPS + warp) * (FP8_ROWS / 2) + pass * HALF, first = min(row0, a.inter - 1);
+        RowSums<M> sums;
+        sums.run([&](int r) { return w + static_cast<size_t>((r >= HALF ? a.inter : 0) + min(row0 + r % HALF, a.inter - 1)) * k; },
+                 ws + static_cast<size_t>(first >> 7) * blocks, ws + static_cast<size_t>((a.inter + first) >> 7) * blocks, blocks, smem, pass > 0, stage);
+        silu_outputs<M>(sums, [&](int r, int m, float gate, float up) {
+            if (row0 + r >= a.inter || m >= count) return;
+            const float value = round_bf16(round_bf16(gate / (1.0f + expf(-gate))) * up);
+            a.out[static_cast<size_t>(order[m]) * a.inter + row0 + r] = static_cast<uint16_t>(f32_to_bf16_bits(value));
+        });
+    }
 }
 
 __global__ void __launch_bounds__(FP8_WARPS * 32, 2) moe_gate_up_fp8_kernel(const __grid_constant__ MoeArgs a) {
@@ -379,19 +391,22 @@ __device__ __forceinline__ void moe_down_tile(const MoeArgs &a, int4 tile, float
     const int warp = threadIdx.x >> 5, thread = threadIdx.x & 31, k = a.inter, blocks = k >> 7, count = tile.z;
     const int *order = a.groups.order + tile.y;
     auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, k, first, n, count, smem, [&](int m) { return order[m]; }); };
-    const int row0 = (blockIdx.x * FP8_WARPS + warp) * FP8_ROWS, expert = tile.x - a.expert_start;
+    const int expert = tile.x - a.expert_start;
     const uint8_t *w = a.w + static_cast<size_t>(expert) * a.hidden * k;
     const uint16_t *ws = a.wscale + static_cast<size_t>(expert) * ((a.hidden + 127) >> 7) * blocks;
-    RowSums<M> sums;
-    sums.run([&](int r) { return w + static_cast<size_t>(min(row0 + r, a.hidden - 1)) * k; }, ws + static_cast<size_t>(min(row0, a.hidden - 1) >> 7) * blocks,
-             ws + static_cast<size_t>(min(row0 + 4, a.hidden - 1) >> 7) * blocks, blocks, smem, stage);
-    if (RowSums<M>::VALUES < 32 && (thread & 1) != 0) return;
+    for (int pass = 0; pass < FP8_ROWS / RowSums<M>::ROWS; pass++) {
+        const int row0 = (blockIdx.x * FP8_WARPS + warp) * FP8_ROWS + pass * RowSums<M>::ROWS;
+        const uint16_t *scale_row = ws + static_cast<size_t>(min(row0, a.hidden - 1) >> 7) * blocks;
+        RowSums<M> sums;
+        sums.run([&](int r) { return w + static_cast<size_t>(min(row0 + r, a.hidden - 1)) * k; }, scale_row, scale_row, blocks, smem, pass > 0, stage);
+        if (RowSums<M>::VALUES < 32 && (thread & 1) != 0) continue;
 #pragma unroll
-    for (int i = 0; i < RowSums<M>::PER_THREAD; i++) {
-        const int output = RowSums<M>::index(thread, i), row = row0 + output / M, m = output % M;
-        if (row >= a.hidden || m >= count) continue;
-        const float weight = bf16_bits_to_f32(a.routes[order[m]] >> 16);
-        a.out[static_cast<size_t>(order[m]) * a.hidden + row] = static_cast<uint16_t>(f32_to_bf16_bits(round_bf16(sums.sums[i]) * weight));
+        for (int i = 0; i < RowSums<M>::PER_THREAD; i++) {
+            const int output = RowSums<M>::index(thread, i), row = row0 + output / M, m = output % M;
+            if (row >= a.hidden || m >= count) continue;
+            const float weight = bf16_bits_to_f32(a.routes[order[m]] >> 16);
+            a.out[static_cast<size_t>(order[m]) * a.hidden + row] = static_cast<uint16_t>(f32_to_bf16_bits(round_bf16(sums.sums[i]) * weight));
+        }
     }
 }
 
@@ -412,6 +427,9 @@ cudaError_t launch_rows(void (*kernel)(Args), dim3 grid, int tile_lanes, cudaStr
     return launch_dependent(kernel, grid, dim3(FP8_WARPS * 32), bytes(tile_lanes <= 2 ? 2 : tile_lanes <= 4 ? 4 : 8), 1, stream, args);
 }
 
+// Rows of a CTA: 64 save half of the staging, 32 spread a small launch over more SMs.
+int fp8_passes(int row_tiles, int lanes) { return row_tiles * ((lanes + TILE_LANES - 1) / TILE_LANES) < 296 ? 1 : 2; }
+
 }  // namespace
 
 cudaError_t launch_linear_fp8(const uint8_t *xq, const float *xscale, const uint8_t *w, const uint16_t *wscale,
@@ -419,8 +437,8 @@ cudaError_t launch_linear_fp8(const uint8_t *xq, const float *xscale, const uint
                               cudaStream_t stream) {
     if (lanes <= 0) return cudaSuccess;
     if (k % 128 != 0) return cudaErrorInvalidValue;
-    const Fp8LinearArgs args{xq, xscale, {w, nullptr}, {wscale, nullptr}, y, residual, lanes, n, k, epilogue};
-    const int rows = FP8_WARPS * FP8_ROWS;
+    const int passes = fp8_passes((n + 63) / 64, lanes), rows = 32 * passes;
+    const Fp8LinearArgs args{xq, xscale, {w, nullptr}, {wscale, nullptr}, y, residual, lanes, n, k, epilogue, passes};
     return launch_rows(linear_fp8_kernel, dim3((n + rows - 1) / rows, (lanes + TILE_LANES - 1) / TILE_LANES), lanes, stream, args);
 }
 
@@ -429,8 +447,8 @@ cudaError_t launch_linear_silu_multiply_fp8(const uint8_t *xq, const float *xsca
                                             uint16_t *y, int lanes, int n, int k, cudaStream_t stream) {
     if (lanes <= 0) return cudaSuccess;
     if (k % 128 != 0) return cudaErrorInvalidValue;
-    const Fp8LinearArgs args{xq, xscale, {wg, wu}, {wg_scale, wu_scale}, y, nullptr, lanes, n, k, EPILOGUE_BF16};
-    const int rows = FP8_WARPS * FP8_ROWS / 2;
+    const int passes = fp8_passes((n + 31) / 32, lanes), rows = 16 * passes;
+    const Fp8LinearArgs args{xq, xscale, {wg, wu}, {wg_scale, wu_scale}, y, nullptr, lanes, n, k, EPILOGUE_BF16, passes};
     return launch_rows(linear_silu_multiply_fp8_kernel, dim3((n + rows - 1) / rows, (lanes + TILE_LANES - 1) / TILE_LANES), lanes, stream, args);
 }
 

@@ -24,6 +24,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "launch.cuh"
 
 namespace nerve {
 
@@ -45,6 +46,7 @@ linear_bf16_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ 
 
     const int chunks = k / 8;  // uint4 = 8 bf16
     // weights do not depend on the previous kernel: the first loads may be issued before the dependency wait
+    grid_launch_dependents();
     grid_dependency_wait();
     for (int chunk = lane; chunk < chunks; chunk += 32) {
         uint4 wv[ROWS];
@@ -107,20 +109,14 @@ linear_bf16_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ 
 }
 
 cudaError_t launch_linear_bf16(const uint16_t *x, const uint16_t *w, void *y, const uint16_t *residual, int lanes,
-                               int n, int k, int epilogue, float scale, cudaStream_t stream, int *error_flag) {
+                               int n, int k, int epilogue, float scale, cudaStream_t stream, int *error_flag, int form_lanes) {
     if (lanes <= 0) return cudaSuccess;
     // wide batches: the tensor-core GEMM (weights read once per 64 lanes instead of once per 8)
-    if (linear_bf16_gemm_supported(lanes, n, k)) return launch_linear_bf16_gemm(x, w, y, residual, lanes, n, k, epilogue, scale, error_flag, stream);
+    if (linear_bf16_gemm_supported(form_lanes > 0 ? form_lanes : lanes, n, k)) return launch_linear_bf16_gemm(x, w, y, residual, lanes, n, k, epilogue, scale, error_flag, stream);
     constexpr int ROWS = 4;
     int row_ctas = (n + 8 * ROWS - 1) / (8 * ROWS);
-    if (lanes <= 4) {
-        dim3 grid(row_ctas, 1);
-        linear_bf16_kernel<4, ROWS><<<grid, 256, 0, stream>>>(x, w, y, residual, lanes, n, k, epilogue, scale);
-    } else {
-        dim3 grid(row_ctas, (lanes + 7) / 8);
-        linear_bf16_kernel<8, ROWS><<<grid, 256, 0, stream>>>(x, w, y, residual, lanes, n, k, epilogue, scale);
-    }
-    return cudaGetLastError();
+    if (lanes <= 4) return launch_dependent(linear_bf16_kernel<4, ROWS>, dim3(row_ctas), dim3(256), 0, 1, stream, x, w, y, residual, lanes, n, k, epilogue, scale);
+    return launch_dependent(linear_bf16_kernel<8, ROWS>, dim3(row_ctas, (lanes + 7) / 8), dim3(256), 0, 1, stream, x, w, y, residual, lanes, n, k, epilogue, scale);
 }
 
 // parallel_linear_silu_multiply_bf16.comp.template:58-72
@@ -135,6 +131,7 @@ linear_silu_multiply_bf16_kernel(const uint16_t *__restrict__ x, const uint16_t 
     float gate[MT], up[MT];
 #pragma unroll
     for (int m = 0; m < MT; m++) gate[m] = up[m] = 0.0f;
+    grid_launch_dependents();
     grid_dependency_wait();
     for (int col = lane * 2; col < k; col += 64) {
         uint32_t g = *reinterpret_cast<const uint32_t *>(wg + static_cast<size_t>(row) * k + col);
@@ -167,8 +164,7 @@ cudaError_t launch_linear_silu_multiply_bf16(const uint16_t *x, const uint16_t *
                                              int lanes, int n, int k, cudaStream_t stream) {
     if (lanes <= 0) return cudaSuccess;
     dim3 grid((n + 7) / 8, (lanes + 7) / 8);
-    linear_silu_multiply_bf16_kernel<8><<<grid, 256, 0, stream>>>(x, wg, wu, y, lanes, n, k);
-    return cudaGetLastError();
+    return launch_dependent(linear_silu_multiply_bf16_kernel<8>, grid, dim3(256), 0, 1, stream, x, wg, wu, y, lanes, n, k);
 }
 
 // ----------------------------------------------------------------------------- INT4 g128 (tensor cores)
@@ -365,23 +361,6 @@ linear_int4_mma_kernel(const Int4Launch p) {
     }
 }
 
-// Launch with the programmatic-dependent-launch attribute so the weight prefetch
-// of this kernel overlaps the tail of the previous kernel in the stream.
-template <typename Kernel>
-static cudaError_t launch_pdl(Kernel kernel, dim3 grid, dim3 block, cudaStream_t stream, const Int4Launch &params) {
-    cudaLaunchConfig_t config = {};
-    config.gridDim = grid;
-    config.blockDim = block;
-    config.dynamicSmemBytes = 0;
-    config.stream = stream;
-    cudaLaunchAttribute attribute[1];
-    attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute[0].val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = attribute;
-    config.numAttrs = 1;
-    return cudaLaunchKernelEx(&config, kernel, params);
-}
-
 cudaError_t launch_linear_int4_multi(const uint16_t *x, const void *prepared, int branches, const uint32_t *const *qweights,
                                      const uint16_t *const *scales, uint16_t *const *ys, const int *ns,
                                      const uint16_t *residual, int lanes, int k, int epilogue, cudaStream_t stream, int *error_flag) {
@@ -410,7 +389,7 @@ cudaError_t launch_linear_int4_multi(const uint16_t *x, const void *prepared, in
         tiles += (ns[b] + 16 * rt - 1) / (16 * rt);
     }
     dim3 grid(tiles);
-    return launch_pdl(linear_int4_mma_kernel<1, false, 4>, grid, dim3(INT4_WARPS * 32), stream, params);
+    return launch_dependent(linear_int4_mma_kernel<1, false, 4>, grid, dim3(INT4_WARPS * 32), 0, 1, stream, params);
 }
 
 cudaError_t launch_linear_int4(const uint16_t *x, const void *prepared, const uint32_t *qweight, const uint16_t *scales, uint16_t *y,
@@ -444,7 +423,7 @@ cudaError_t launch_linear_int4_silu_pair(const uint16_t *x, const void *prepared
     params.branch[1] = Int4Branch{up_q, up_s, nullptr, n, 0};
     params.branch[2] = Int4Branch{nullptr, nullptr, y, n, 0};
     dim3 grid((n + 15) / 16);
-    return launch_pdl(linear_int4_mma_kernel<2, true, 2>, grid, dim3(INT4_WARPS * 32), stream, params);
+    return launch_dependent(linear_int4_mma_kernel<2, true, 2>, grid, dim3(INT4_WARPS * 32), 0, 1, stream, params);
 }
 
 }  // namespace nerve
