@@ -70,6 +70,20 @@ __device__ __forceinline__ bool wait_barrier(uint32_t barrier, uint32_t parity, 
 __device__ __forceinline__ void commit_to(uint32_t barrier) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(barrier) : "memory");
 }
+// One lane of a converged warp.  The issuing warps run their loops as a whole, on values the compiler can keep in uniform
+// registers, and only the instructions themselves under this predicate: with the loop inside a one-thread branch every
+// MMA operand was moved to a uniform register first, and a group of eight MMAs took 890 cycles to issue instead of 325.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t elected;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "elect.sync _|p, 0xffffffff;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(elected));
+    return elected != 0;
+}
 __device__ __forceinline__ uint32_t shared_address(const void *pointer) { return static_cast<uint32_t>(__cvta_generic_to_shared(pointer)); }
 
 // Half-precision pair arithmetic on 32-bit words.
@@ -153,7 +167,7 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
     uint16_t *const scales = reinterpret_cast<uint16_t *>(raw + a.raw_stages * SLOT);
     const uint32_t a_full = shared_address(smem) + a.barrier_offset, a_empty = a_full + 8 * GEMM_MAX_A_STAGES, b_full = a_empty + 8 * GEMM_MAX_A_STAGES,
                    b_empty = b_full + 8 * GEMM_MAX_B_STAGES, all_done = b_empty + 8 * GEMM_MAX_B_STAGES, tmem_slot = all_done + 8;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp: uniform
     grid_launch_dependents();
 
     if (threadIdx.x == 0) {
@@ -177,6 +191,7 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     uint32_t tmem;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot) : "memory");
+    tmem = __reduce_or_sync(0xffffffffu, tmem);  // a uniform register
     const uint32_t d_stride = (static_cast<uint32_t>(a.tile_lanes) + 31u) & ~31u, tmem_a = tmem + ROW_TILES * d_stride;
 
     bool alive = true;
@@ -310,25 +325,25 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (warp == WARPS) {
-        if (lane == 0) {
-            // instruction descriptor: f32 accumulator, A and B fp16, both K-major, N / 8 in bits 17-22, M / 16 in bits 24-28
-            const uint32_t instruction = (1u << 4) | (static_cast<uint32_t>(n_lanes / 8) << 17) | (8u << 24);
-            int stage_a = 0, stage_b = 0;
-            uint32_t parity_a = 0, parity_b = 0;
-            for (int group = 0; group < own_groups; group++) {
-                if (!wait_barrier(b_full + stage_b * 8, parity_b, a.error_flag) || !wait_barrier(a_full + stage_a * 8, parity_a, a.error_flag)) {
-                    alive = false;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t b_address = shared_address(smem) + static_cast<uint32_t>(stage_b) * b_stage_bytes;
+        // instruction descriptor: f32 accumulator, A and B fp16, both K-major, N / 8 in bits 17-22, M / 16 in bits 24-28
+        const uint32_t instruction = (1u << 4) | (static_cast<uint32_t>(n_lanes / 8) << 17) | (8u << 24);
+        const uint64_t b_first = swizzled_descriptor(shared_address(smem)), b_half = static_cast<uint64_t>(n_lanes) * 8;  // descriptors count 16 bytes
+        int stage_a = 0, stage_b = 0;
+        uint32_t parity_a = 0, parity_b = 0;
+        for (int group = 0; group < own_groups; group++) {
+            if (!wait_barrier(b_full + stage_b * 8, parity_b, a.error_flag) || !wait_barrier(a_full + stage_a * 8, parity_a, a.error_flag)) {
+                alive = false;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (elect_one()) {
+                const uint64_t b_stage = b_first + static_cast<uint64_t>(stage_b) * (b_stage_bytes >> 4);
 #pragma unroll
                 for (int t = 0; t < ROW_TILES; t++) {
-                    const uint32_t d_address = tmem + t * d_stride;
-                    const uint32_t a_address = tmem_a + static_cast<uint32_t>(stage_a * ROW_TILES + t) * 64;
+                    const uint32_t d_address = tmem + t * d_stride, a_address = tmem_a + static_cast<uint32_t>(stage_a * ROW_TILES + t) * 64;
 #pragma unroll
                     for (int step = 0; step < 8; step++) {  // K = 16 per instruction; four steps to a 128-byte row of the swizzled tile
-                        const uint64_t b_descriptor = swizzled_descriptor(b_address + static_cast<uint32_t>(step >> 2) * static_cast<uint32_t>(n_lanes) * 128 + (step & 3) * 32);
+                        const uint64_t b_descriptor = b_stage + (step >> 2) * b_half + (step & 3) * 2;
                         const uint32_t accumulate = (group > 0 || step > 0) ? 1u : 0u;
                         asm volatile(
                             "{\n"
@@ -342,36 +357,43 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
                 }
                 commit_to(a_empty + stage_a * 8);
                 commit_to(b_empty + stage_b * 8);
-                if (++stage_a == a.a_stages) {
-                    stage_a = 0;
-                    parity_a ^= 1;
-                }
-                if (++stage_b == a.b_stages) {
-                    stage_b = 0;
-                    parity_b ^= 1;
-                }
             }
-            commit_to(all_done);
+            __syncwarp();
+            if (++stage_a == a.a_stages) {
+                stage_a = 0;
+                parity_a ^= 1;
+            }
+            if (++stage_b == a.b_stages) {
+                stage_b = 0;
+                parity_b ^= 1;
+            }
         }
-    } else if (lane == 0) {
+        if (elect_one()) commit_to(all_done);
+        __syncwarp();
+    } else {
         grid_dependency_wait();
-        const uint8_t *source = a.x + static_cast<size_t>(m0 >> 3) * 1024;
+        const uint8_t *source = a.x + static_cast<size_t>(2 * first_group) * a.lane_blocks * 1024 + static_cast<size_t>(m0 >> 3) * 1024;
+        const size_t part_bytes = static_cast<size_t>(a.lane_blocks) * 1024;
         const uint32_t bytes = static_cast<uint32_t>(n_lanes) * 128;
         int stage = 0;
         uint32_t parity = 1;  // the first round waits for no release
         for (int group = 0; group < own_groups; group++) {
             if (!wait_barrier(b_empty + stage * 8, parity, a.error_flag)) {
-                for (int g = group - a.b_stages; g < group; g++)  // the copies in flight land before the CTA gives its memory up
+                for (int g = group > a.b_stages ? group - a.b_stages : 0; g < group; g++)  // the copies in flight land before the CTA gives its memory up
                     wait_barrier(b_full + (g % a.b_stages) * 8, static_cast<uint32_t>((g / a.b_stages) & 1), a.error_flag);
                 break;
             }
-            const uint32_t target = shared_address(smem) + static_cast<uint32_t>(stage) * b_stage_bytes, full = b_full + stage * 8;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"(2 * bytes) : "memory");
+            if (elect_one()) {
+                const uint32_t target = shared_address(smem) + static_cast<uint32_t>(stage) * b_stage_bytes, full = b_full + stage * 8;
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"(2 * bytes) : "memory");
 #pragma unroll
-            for (int part = 0; part < 2; part++)
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(target + part * bytes),
-                             "l"(source + static_cast<size_t>(2 * (first_group + group) + part) * a.lane_blocks * 1024), "r"(bytes), "r"(full)
-                             : "memory");
+                for (int part = 0; part < 2; part++)
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(target + part * bytes),
+                                 "l"(source + static_cast<size_t>(part) * part_bytes), "r"(bytes), "r"(full)
+                                 : "memory");
+            }
+            __syncwarp();
+            source += 2 * part_bytes;
             if (++stage == a.b_stages) {
                 stage = 0;
                 parity ^= 1;
@@ -423,15 +445,22 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
     if (good && threadIdx.x < WARPS * 32 && row < n) {
         auto pair_sum = [&](int m, int at) {
             if (splits == 1) return *reinterpret_cast<const float2 *>(sums + m * ROWS + at);
-            float2 sum = make_float2(0.0f, 0.0f);
+            // every split's share is asked for before the first one is added: one round trip to the peers instead of one each
+            float2 part[8];
             const uint32_t local = shared_address(sums + m * ROWS + at);
-            for (int s = 0; s < splits; s++) {
+#pragma unroll
+            for (int s = 0; s < 8; s++) {
+                if (s >= splits) break;
                 uint32_t remote;
-                float2 part;
                 asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(s));
-                asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(part.x), "=f"(part.y) : "r"(remote));
-                sum.x += part.x;
-                sum.y += part.y;
+                asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(part[s].x), "=f"(part[s].y) : "r"(remote));
+            }
+            float2 sum = part[0];
+#pragma unroll
+            for (int s = 1; s < 8; s++) {
+                if (s >= splits) break;
+                sum.x += part[s].x;
+                sum.y += part[s].y;
             }
             return sum;
         };
@@ -613,16 +642,19 @@ GemmPlan plan_gemm(int matrix_tiles, int lanes, int groups, bool silu) {
                 int per_sm = 0;
                 for (int share = row_tiles == 1 && tile_lanes <= 64 ? 2 : 1; share >= 1 && per_sm == 0; share--) {
                     const size_t limit = share == 2 ? GEMM_SMEM_TWO : GEMM_SMEM_ONE;
-                    for (int raw = row_tiles == 2 ? 4 : 6; raw >= 3 && per_sm == 0; raw--)
-                        for (int b = std::min(GEMM_MAX_B_STAGES, std::max(2, own)); b >= 2; b--) {
-                            if (raw > (row_tiles == 2 ? 3 : 4) && b < 4 && b < own) break;  // rather fewer raw stages than fewer than four of the activations
+                    // stages: the pair that looks furthest ahead, counted in groups, on its shorter side (a raw slot holds
+                    // two groups, and the one being read does not count)
+                    int best_ahead = 0;
+                    for (int raw = 3; raw <= 6; raw++)
+                        for (int b = 2; b <= GEMM_MAX_B_STAGES; b++) {
                             const size_t bytes = std::max(static_cast<size_t>(b) * b_stage + static_cast<size_t>(raw) * 16384 * row_tiles + scales, sums);
-                            if (bytes > limit) continue;
+                            const int ahead = std::min(2 * (raw - 1), b);
+                            if (bytes > limit || ahead <= best_ahead) continue;
+                            best_ahead = ahead;
                             plan.b_stages = b;
                             plan.raw_stages = raw;
                             plan.smem = bytes;
                             per_sm = share;
-                            break;
                         }
                 }
                 if (per_sm == 0) continue;
