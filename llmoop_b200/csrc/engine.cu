@@ -571,10 +571,11 @@ Engine::Engine(std::shared_ptr<MountedModel> model) : model_(std::move(model)) {
     for (const ComponentPlan &layer : plan.layers) scan(layer);
     for (const ComponentPlan &layer : plan.draft_layers) scan(layer);
     // Scratch of the split attention.  The persistent kernel (at most eight lanes) takes 64-token splits over the
-    // whole ring.  On the kernel-per-operator path verify, draft and single-tick batches take splits of a length fixed
-    // per engine - 128 tokens (64 in FP8 packages) where the partials of the largest batch over the whole ring fit 1 GB,
-    // else the next multiple that makes them fit - so that the arithmetic of such a lane does not depend on its batch;
-    // prefill chunks are split only as far as they need to be to fill the chip (plan_splits), except in FP8 packages.
+    // whole ring.  On the kernel-per-operator path verify, draft and single-tick batches take splits of a fixed length,
+    // so that the arithmetic of such a lane does not depend on its batch: 128 tokens where the partials of the batch over
+    // the whole ring fit the scratch (1 GB at most), else the next multiple (plan_splits); prefill chunks are split only
+    // as far as they need to be to fill the chip.  FP8 packages take one length for everything: 64 tokens where the
+    // partials of the largest batch fit, else the next multiple.
     auto has_fp8 = [](const ComponentPlan &component) {
         for (const OpSpec &op : component.ops)
             for (const WeightRef &w : op.weights)
@@ -594,11 +595,12 @@ Engine::Engine(std::shared_ptr<MountedModel> model) : model_(std::move(model)) {
     const size_t partial_bytes = static_cast<size_t>(max_head_width + 2) * sizeof(float);
     const size_t budget = (size_t(1) << 30) / partial_bytes;
     const size_t op_base = scalar_attention_ ? 64 : 128, all = static_cast<size_t>(options.max_lanes) * max_q_heads * ((model_->capacity() + op_base - 1) / op_base);
-    op_split_tokens_ = static_cast<int>(op_base * std::max<size_t>(1, (all + budget - 1) / budget));
+    op_split_tokens_ = static_cast<int>(op_base * (scalar_attention_ ? std::max<size_t>(1, (all + budget - 1) / budget) : 1));
     const size_t op_splits = (model_->capacity() + op_split_tokens_ - 1) / op_split_tokens_;
     // (the persistent kernel merges rows of more than 32 splits in two levels: one more partial per 32 splits)
     const size_t small_batches = static_cast<size_t>(std::min(options.max_lanes, 8)) * max_q_heads * (max_splits_ + (max_splits_ + 31) / 32);
-    attention_partials_ = std::max(small_batches, static_cast<size_t>(options.max_lanes) * max_q_heads * op_splits);
+    const size_t largest_batches = static_cast<size_t>(options.max_lanes) * max_q_heads * op_splits;
+    attention_partials_ = std::max(small_batches, scalar_attention_ ? largest_batches : std::min(largest_batches, std::max(budget, static_cast<size_t>(options.max_lanes) * max_q_heads)));
     attention_scratch_ = device_alloc(attention_partials_ * partial_bytes);
     attention_blocks_ = device_alloc(lanes * sizeof(AttentionBlock));  // (a block covers at least one lane)
 
@@ -1392,7 +1394,7 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
                     } else {
                         check(launch_linear_bf16(u16(op.inputs[0]), static_cast<const uint16_t *>(weight(w.tensor)), ptr(op.outputs[branch]), nullptr,
                                                  lanes, static_cast<int>(w.n), static_cast<int>(w.k), EPILOGUE_BF16, 1.0f, st, static_cast<int *>(kernel_error_.ptr),
-                                                 current_form_lanes_),
+                                                 bf16_form(lanes)),
                               "linear_bf16");
                     }
                 } else if (w.storage == TensorStorage::INT4_CT) {
@@ -1416,7 +1418,7 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
             if (w.storage == TensorStorage::BF16) {
                 check(launch_linear_bf16(u16(op.inputs[0]), static_cast<const uint16_t *>(weight(w.tensor)), ptr(op.outputs[0]),
                                          u16(op.residual_input), lanes, static_cast<int>(w.n), static_cast<int>(w.k),
-                                         EPILOGUE_RESIDUAL_ROUNDED, 1.0f, st, static_cast<int *>(kernel_error_.ptr)),
+                                         EPILOGUE_RESIDUAL_ROUNDED, 1.0f, st, static_cast<int *>(kernel_error_.ptr), bf16_form(lanes)),
                       "linear_residual_bf16");
             } else if (w.storage == TensorStorage::FP8_BLOCK) {
                 check(launch_linear_fp8(static_cast<const uint8_t *>(ptr(op.inputs[0])), static_cast<const float *>(ptr(op.inputs[1])),
@@ -1621,8 +1623,10 @@ int Engine::plan_splits(int lanes, int lanes_per_stream, uint64_t newest_tick) {
         return std::min(count, most);
     };
     current_splits_ = bucket(split_tokens_);
-    current_op_split_tokens_ = op_split_tokens_;
-    current_op_splits_ = bucket(op_split_tokens_);
+    // (a wider batch than the scratch has room for at that length takes the next multiple)
+    const size_t whole_ring = static_cast<size_t>(lanes) * max_q_heads_ * ((model_->capacity() + op_split_tokens_ - 1) / op_split_tokens_);
+    current_op_split_tokens_ = op_split_tokens_ * static_cast<int>(std::max<size_t>(1, (whole_ring + attention_partials_ - 1) / attention_partials_));
+    current_op_splits_ = bucket(current_op_split_tokens_);
     const ModelPlan &plan = model_->plan();
     const auto attention = std::find_if(plan.layers.begin(), plan.layers.end(), [](const ComponentPlan &layer) { return layer.has_kv; });
     if (!scalar_attention_ && attention != plan.layers.end() && attention_is_prefill(lanes_per_stream, attention->q_heads, attention->kv_heads)) {
@@ -2028,7 +2032,7 @@ void Engine::run_speculative_cycles(std::vector<Stream *> &batch, int drafts, co
     }
     sync_block_tables();
     upload(base, staging.data(), upload_words * sizeof(uint32_t), "cycle state upload");
-    const int splits = plan_splits(streams, 1, newest_tick);
+    const int splits = plan_splits(lanes, 1, newest_tick);
 
     backup_pending();
     cuda_check(cudaEventRecord(event_begin_, cuda_stream_), "event record");

@@ -427,7 +427,13 @@ private:
     int current_op_split_tokens_ = 128, current_op_splits_ = 1;  // split length and count of the next launches on that path
     DeviceBuffer attention_blocks_;         // row blocks of a ragged prefill batch
     int current_blocks_ = 0;                // ... of the next launches (0: uniform batch)
-    int current_form_lanes_ = 0;            // lanes by which the next launches choose the form of a bf16 linear (0: the batch's)
+    int current_form_lanes_ = 0;            // lanes of one stream's chunk in the next launches (0: those of the batch)
+    // FP8 packages fix the form of their layers' bf16 linears (routers) by the lanes of one stream's chunk, so that a
+    // token's experts do not depend on the other streams of its batch.
+    LinearForm bf16_form(int lanes) const {
+        if (!scalar_attention_) return LINEAR_AUTO;
+        return (current_form_lanes_ > 0 ? current_form_lanes_ : lanes) >= 16 ? LINEAR_TENSOR : LINEAR_SCALAR;
+    }
     bool ragged_prefill_ = false;           // one table of row blocks serves every layer (equal head shapes)
     bool scalar_attention_ = false;         // FP8 packages: the attention form in scalar f32
     size_t attention_partials_ = 0;         // partials attention_scratch_ holds

@@ -53,10 +53,11 @@ enum LinearEpilogue {
     EPILOGUE_F32_SCALED = 3,      // y_f32 = sum * scale                     (logits; tensor-parallel partial sums)
 };
 
-// y[m][n] = sum_k x[m][k] * W[n][k], bf16 weights.  form_lanes: choose the form (and so the order of additions) of a batch
-// of that many lanes.
+// y[m][n] = sum_k x[m][k] * W[n][k], bf16 weights.  The form fixes the order of additions: by the number of lanes, or the
+// caller's choice (tensor cores where K allows).
+enum LinearForm { LINEAR_AUTO, LINEAR_SCALAR, LINEAR_TENSOR };
 cudaError_t launch_linear_bf16(const uint16_t *x, const uint16_t *w, void *y, const uint16_t *residual, int lanes,
-                               int n, int k, int epilogue, float scale, cudaStream_t stream, int *error_flag = nullptr, int form_lanes = 0);
+                               int n, int k, int epilogue, float scale, cudaStream_t stream, int *error_flag = nullptr, LinearForm form = LINEAR_AUTO);
 // y = bf16( silu_bf16(bf16(x.Wg)) * bf16(x.Wu) )
 cudaError_t launch_linear_silu_multiply_bf16(const uint16_t *x, const uint16_t *wg, const uint16_t *wu, uint16_t *y,
                                              int lanes, int n, int k, cudaStream_t stream);
@@ -165,7 +166,7 @@ cudaError_t launch_rms_norm_prepared(const uint16_t *x, const uint16_t *weight, 
 cudaError_t launch_linear_int4_gemm(const void *prepared, int branches, const uint32_t *const *qweights, const uint16_t *const *scales, void *const *ys,
                                     const int *ns, const uint16_t *residual, int lanes, int k, int epilogue, float scale, bool silu, int *error_flag,
                                     cudaStream_t stream);
-// bf16 weights, batches of 16 lanes and more (tcgen05): called by launch_linear_bf16.
+// bf16 weights, batches of more than 8 lanes (tcgen05): called by launch_linear_bf16.
 bool linear_bf16_gemm_supported(int lanes, int n, int k);
 cudaError_t launch_linear_bf16_gemm(const uint16_t *x, const uint16_t *w, void *y, const uint16_t *residual, int lanes, int n, int k, int epilogue,
                                     float scale, int *error_flag, cudaStream_t stream);

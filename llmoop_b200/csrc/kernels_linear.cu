@@ -109,10 +109,10 @@ linear_bf16_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ 
 }
 
 cudaError_t launch_linear_bf16(const uint16_t *x, const uint16_t *w, void *y, const uint16_t *residual, int lanes,
-                               int n, int k, int epilogue, float scale, cudaStream_t stream, int *error_flag, int form_lanes) {
+                               int n, int k, int epilogue, float scale, cudaStream_t stream, int *error_flag, LinearForm form) {
     if (lanes <= 0) return cudaSuccess;
-    // wide batches: the tensor-core GEMM (weights read once per 64 lanes instead of once per 8)
-    if (linear_bf16_gemm_supported(form_lanes > 0 ? form_lanes : lanes, n, k)) return launch_linear_bf16_gemm(x, w, y, residual, lanes, n, k, epilogue, scale, error_flag, stream);
+    // more than eight lanes: the tensor-core GEMM (weights read once instead of once per eight lanes)
+    if (form != LINEAR_SCALAR && linear_bf16_gemm_supported(form == LINEAR_TENSOR ? 16 : lanes, n, k)) return launch_linear_bf16_gemm(x, w, y, residual, lanes, n, k, epilogue, scale, error_flag, stream);
     constexpr int ROWS = 4;
     int row_ctas = (n + 8 * ROWS - 1) / (8 * ROWS);
     if (lanes <= 4) return launch_dependent(linear_bf16_kernel<4, ROWS>, dim3(row_ctas), dim3(256), 0, 1, stream, x, w, y, residual, lanes, n, k, epilogue, scale);
