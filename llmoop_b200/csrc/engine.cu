@@ -1983,7 +1983,7 @@ void Engine::run_single_ticks(std::vector<Stream *> &batch, const std::function<
 
 // ---------------------------------------------------------------------------- speculative cycles (feedback_generation.rs:66-194)
 
-void Engine::run_speculative_cycles(std::vector<Stream *> &batch, int drafts, const std::function<void(const OutputEvent &)> &on_output,
+void Engine::run_speculative_cycles(std::vector<Stream *> &batch, const std::vector<int> &own, int drafts, const std::function<void(const OutputEvent &)> &on_output,
                                     RunReport &report) {
     const ModelPlan &plan = model_->plan();
     const int streams = static_cast<int>(batch.size());
@@ -1998,16 +1998,17 @@ void Engine::run_speculative_cycles(std::vector<Stream *> &batch, int drafts, co
     uint32_t *stop_tokens = forced + lanes;                      // [streams][MAX_STOP]
     int32_t *stop_counts = reinterpret_cast<int32_t *>(stop_tokens + streams * MAX_STOP_TOKENS);  // [streams]
     int32_t *stream_slots = stop_counts + streams;               // [streams]
-    uint32_t *draft_positions = reinterpret_cast<uint32_t *>(stream_slots + streams);  // [drafts][streams]
+    int32_t *own_drafts = stream_slots + streams;                // [streams]
+    uint32_t *draft_positions = reinterpret_cast<uint32_t *>(own_drafts + streams);  // [drafts][streams]
     uint32_t *verify_positions = draft_positions + drafts * streams;                   // [lanes]
     int32_t *verify_slots = reinterpret_cast<int32_t *>(verify_positions + lanes);     // [lanes]
     uint32_t *draft_tokens = reinterpret_cast<uint32_t *>(verify_slots + lanes);       // [streams]
-    const size_t upload_words = static_cast<size_t>(lanes) * 4 + streams * MAX_STOP_TOKENS + 3 * streams + drafts * streams;
+    const size_t upload_words = static_cast<size_t>(lanes) * 4 + streams * MAX_STOP_TOKENS + 4 * streams + drafts * streams;
     uint32_t *accept_rows = base + upload_words;                 // [streams][4 + 2*width]
 
     std::vector<uint32_t> staging(upload_words, 0);
     uint32_t *s_forced = staging.data() + lanes, *s_stop = s_forced + lanes, *s_counts = s_stop + streams * MAX_STOP_TOKENS;
-    uint32_t *s_slots = s_counts + streams, *s_dpos = s_slots + streams, *s_vpos = s_dpos + drafts * streams;
+    uint32_t *s_slots = s_counts + streams, *s_own = s_slots + streams, *s_dpos = s_own + streams, *s_vpos = s_dpos + drafts * streams;
     uint32_t *s_vslots = s_vpos + lanes, *s_dtokens = s_vslots + lanes;
     uint64_t newest_tick = 0;
     for (int s = 0; s < streams; s++) {
@@ -2025,6 +2026,7 @@ void Engine::run_speculative_cycles(std::vector<Stream *> &batch, int drafts, co
         for (size_t t = 0; t < stops.size(); t++) s_stop[s * MAX_STOP_TOKENS + t] = stops[t];
         s_counts[s] = static_cast<uint32_t>(stops.size());
         s_slots[s] = static_cast<uint32_t>(st.slot);
+        s_own[s] = static_cast<uint32_t>(own[s]);
         for (int i = 0; i < width; i++) {
             s_vpos[s * width + i] = static_cast<uint32_t>(st.next_tick + i);
             s_vslots[s * width + i] = static_cast<uint32_t>(st.slot);
@@ -2077,7 +2079,7 @@ void Engine::run_speculative_cycles(std::vector<Stream *> &batch, int drafts, co
         check(launch_shift_hidden(static_cast<const uint16_t *>(pending_hidden_.ptr), stream_slots, static_cast<const uint16_t *>(normalized_.ptr),
                                   static_cast<uint16_t *>(draft_hidden_in_.ptr), streams, width, static_cast<int>(plan.hidden), cuda_stream_),
               "catch-up hidden");
-        check(launch_accept(verify_tokens, static_cast<const uint32_t *>(records_.ptr), stop_tokens, stop_counts, MAX_STOP_TOKENS, streams, drafts,
+        check(launch_accept(verify_tokens, static_cast<const uint32_t *>(records_.ptr), stop_tokens, stop_counts, own_drafts, MAX_STOP_TOKENS, streams, drafts,
                             accept_rows, static_cast<const uint16_t *>(normalized_.ptr), static_cast<uint16_t *>(pending_hidden_.ptr), stream_slots,
                             static_cast<int>(plan.hidden), cuda_stream_),
               "accept");
@@ -2105,19 +2107,28 @@ void Engine::run_speculative_cycles(std::vector<Stream *> &batch, int drafts, co
         Stream &st = *batch[s];
         const uint32_t *row = host_records_ + s * row_words;
         uint32_t accepted = row[0], committed = row[1], count = row[2];
-        report.speculative.cycle_count++;
-        report.speculative.proposed_draft_token_count += drafts;
-        report.speculative.accepted_draft_token_count += accepted;
-        report.speculative.emitted_token_count += count;
-        if (log_cycles_) {
+        if (own[s] > 0) {  // (a stream with room for one more token takes a plain tick)
+            report.speculative.cycle_count++;
+            report.speculative.proposed_draft_token_count += static_cast<uint64_t>(own[s]);
+            report.speculative.accepted_draft_token_count += accepted;
+            report.speculative.emitted_token_count += count;
+        }
+        if (log_cycles_ && own[s] > 0) {
             CycleRecord record;
             record.stream_id = st.id;
             record.start_tick = st.next_tick;
             record.accepted = accepted;
             record.committed = committed;
             record.emitted_token_ids.assign(row + 4, row + 4 + count);
-            record.target_token_ids.assign(row + 4 + width, row + 4 + 2 * width);
+            record.target_token_ids.assign(row + 4 + width, row + 4 + width + own[s] + 1);
             cycle_log_.push_back(std::move(record));
+        }
+        if (st.active->feedback_closes) {  // the closing tick: the last token is fed back, nothing more is emitted
+            if (prefix_cache_on() && st.history.size() == st.next_tick) st.history.push_back(st.active->feedback_token);
+            st.next_tick += 1;
+            st.active.reset();
+            st.completed_events++;
+            continue;
         }
         st.active->has_feedback = false;
         const uint32_t fed_back = st.active->feedback_token;  // the input of the cycle's first tick; every later tick takes the token before it
@@ -2151,7 +2162,9 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
         uint64_t start_tick;
         size_t emitted_before;
         std::vector<uint32_t> generated;
+        bool closing = false;  // all but its event's closing tick has run
     };
+    std::vector<Work> deferred;  // closing ticks that share the next pass over the weights
     auto note_generated = [](Work &work) {
         if (work.stream->active == nullptr) return;
         const std::vector<uint32_t> &all = work.stream->active->generated;
@@ -2169,9 +2182,13 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
     };
     while (true) {
         if (max_batches && report.batch_count >= max_batches) {
-            report.idle = false;
-            break;
+            if (deferred.empty()) {
+                report.idle = false;
+                break;
+            }
+            // the closing ticks belong to the batches that have run
         }
+        const bool only_closing = max_batches && report.batch_count >= max_batches;
         // 0. control steps: events that were stopped from outside still feed their last token back (the closing
         // tick, placed_prompt_event.rs:320-341); the scheduler no longer tracks them
         {
@@ -2202,20 +2219,23 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
             runtime::SchedulerBudget(std::max<size_t>(1, streams_.size()), chunk_budget, std::numeric_limits<size_t>::max())
                 .with_max_decode_tokens_per_activation(widest_window);
         std::vector<runtime::Activation> scheduled;
-        if (!carried_activations_.empty()) {
+        if (only_closing) {
+        } else if (!carried_activations_.empty()) {
             scheduled.swap(carried_activations_);  // the activations of a batch that failed: the same work again
         } else {
             scheduled = scheduler_.schedule_step(budget).activations;
         }
-        if (scheduled.empty()) break;
+        if (scheduled.empty() && deferred.empty()) break;
         std::vector<Work> works;
-        works.reserve(scheduled.size());
+        works.reserve(scheduled.size() + deferred.size());
         for (runtime::Activation &activation : scheduled) {
             Stream &s = stream(std::stoll(activation.stream_id));
             activate_next_event(s);
             if (!s.active) fail("scheduler activation for stream " + activation.stream_id + " without an input event");
             works.push_back(Work{std::move(activation), &s, s.next_tick, s.active->generated.size(), {}});
         }
+        for (Work &work : deferred) works.push_back(std::move(work));
+        deferred.clear();
         try {
         // 2. prefill chunks, as many streams' in one pass as the lanes allow
         struct Pending {
@@ -2224,7 +2244,7 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
         };
         std::vector<Pending> pending;
         for (Work &work : works) {
-            if (work.activation.kind != runtime::ActivationKind::PrefillChunk) continue;
+            if (work.closing || work.activation.kind != runtime::ActivationKind::PrefillChunk) continue;
             const ActiveEvent &event = *work.stream->active;
             if (event.next_external != work.activation.token_offset || event.input.token_ids.size() < work.activation.token_offset + work.activation.token_ids.size())
                 fail("scheduler and engine disagree about the prompt position of stream " + work.activation.stream_id);
@@ -2281,10 +2301,23 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
             pending.erase(std::remove_if(pending.begin(), pending.end(), [](const Pending &entry) { return entry.left == 0; }), pending.end());
         }
         if (any_prefill) report.prefill_ns += now_ns() - prefill_start;
-        // 3. decode windows: grouped into speculative cycles of equal draft count and single ticks
-        std::map<int, std::vector<Stream *>> speculative;
+        // 3. decode windows.  Streams that speculate share a cycle whatever their draft counts: it runs the largest one,
+        // a stream with a smaller window (its last tokens) ignores the drafts behind it, and one with room for a single
+        // token, or only the closing tick of its event to do, ignores them all - a pass over the weights costs more than
+        // the lanes.  FP8 packages keep cycles of equal
+        // draft count (the form of their routers' sums goes by the lanes of a batch).
+        struct Window {
+            Stream *stream;
+            int drafts;
+        };
+        std::map<int, std::vector<Window>> speculative;
         std::vector<Stream *> single;
         for (Work &work : works) {
+            if (work.closing) {
+                if (work.stream->k > 0 && model_->plan().has_draft) speculative[0].push_back(Window{work.stream, 0});
+                else single.push_back(work.stream);
+                continue;
+            }
             if (work.activation.kind != runtime::ActivationKind::DecodeFeedback) continue;
             Stream &s = *work.stream;
             ActiveEvent &event = *s.active;
@@ -2293,21 +2326,34 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
             // no speculation across or beyond the wrap of the KV ring (see the prefill chunks above): the rejected
             // lanes of a cycle would also overwrite slots that are still inside the window
             const bool ring_wraps = s.next_tick + static_cast<uint64_t>(s.k) + 1 > model_->capacity();
-            if (s.k > 0 && model_->plan().has_draft && !event.feedback_closes && window >= 2 && !ring_wraps) {
-                int drafts = static_cast<int>(std::min<size_t>(s.k, window - 1));
-                speculative[drafts].push_back(&s);
+            if (s.k > 0 && model_->plan().has_draft && !event.feedback_closes && window >= 1 && !ring_wraps) {
+                const int drafts = static_cast<int>(std::min<size_t>(s.k, window - 1));
+                speculative[scalar_attention_ ? drafts : 0].push_back(Window{&s, drafts});
             } else {
                 single.push_back(&s);
             }
         }
         uint64_t start = now_ns();
         for (auto &group : speculative) {
+            int drafts = 0;
+            for (const Window &window : group.second) drafts = std::max(drafts, window.drafts);
+            // (drafts run past a smaller window into slots a later cycle rewrites: the ring must have room for them)
+            auto padded = [&](const Window &window) { return window.stream->next_tick + static_cast<uint64_t>(drafts) + 1 <= model_->capacity(); };
+            std::vector<Window> cycle;
+            for (const Window &window : group.second) {
+                if (drafts > 0 && (window.drafts > 0 || group.second.size() > 1) && padded(window)) cycle.push_back(window);
+                else single.push_back(window.stream);
+            }
             // split groups that would exceed the lane budget
-            size_t per_batch = std::max<size_t>(1, model_->options().max_lanes / (group.first + 1));
-            for (size_t offset = 0; offset < group.second.size(); offset += per_batch) {
-                std::vector<Stream *> batch(group.second.begin() + offset,
-                                            group.second.begin() + std::min(group.second.size(), offset + per_batch));
-                run_speculative_cycles(batch, group.first, on_output, report);
+            size_t per_batch = std::max<size_t>(1, model_->options().max_lanes / (drafts + 1));
+            for (size_t offset = 0; offset < cycle.size(); offset += per_batch) {
+                std::vector<Stream *> batch;
+                std::vector<int> own;
+                for (size_t i = offset; i < std::min(cycle.size(), offset + per_batch); i++) {
+                    batch.push_back(cycle[i].stream);
+                    own.push_back(cycle[i].drafts);
+                }
+                run_speculative_cycles(batch, own, drafts, on_output, report);
                 report.batch_count++;
                 report.activation_count += batch.size();
                 report.max_batch_width = std::max<uint64_t>(report.max_batch_width, batch.size());
@@ -2315,18 +2361,25 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
         }
         if (!single.empty()) run_ticks_in_batches(single);
         // 4. what the activations emitted; then the closing tick of every event that has emitted its last token (the
-        // scheduler reserves one state activation beyond the window for it, stream_runtime.rs:1262-1290)
+        // scheduler reserves one state activation beyond the window for it, stream_runtime.rs:1262-1290): together with
+        // the next step's batch, the activation staying in flight until then - in FP8 packages at once
         std::vector<Stream *> closing;
         for (Work &work : works) {
             note_generated(work);
             Stream &s = *work.stream;
-            if (s.active && s.active->has_feedback && s.active->feedback_closes) closing.push_back(&s);
+            if (!s.active || !s.active->has_feedback || !s.active->feedback_closes) continue;
+            work.closing = true;
+            if (scalar_attention_) closing.push_back(&s);
         }
         if (!closing.empty()) run_ticks_in_batches(closing);
         report.decode_ns += now_ns() - start;
         // 5. outcomes: generated tokens, whether the event goes on, and the ticks the stream advanced by
         for (Work &work : works) {
             Stream &s = *work.stream;
+            if (work.closing && s.active != nullptr) {
+                deferred.push_back(std::move(work));
+                continue;
+            }
             runtime::ActivationOutcome outcome;
             outcome.generated_token_ids = work.generated;
             outcome.continue_generation = s.active != nullptr;

@@ -342,7 +342,7 @@ private:
     void run_prefill_batch(std::vector<PrefillPart> &parts);
     void run_single_ticks(std::vector<Stream *> &batch, const std::function<void(const OutputEvent &)> &on_output,
                           RunReport &report);
-    void run_speculative_cycles(std::vector<Stream *> &batch, int draft_count,
+    void run_speculative_cycles(std::vector<Stream *> &batch, const std::vector<int> &own_drafts, int draft_count,
                                 const std::function<void(const OutputEvent &)> &on_output, RunReport &report);
     void check(cudaError_t status, const char *what);
     void *signal_buffer(const std::string &name);

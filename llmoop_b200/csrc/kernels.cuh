@@ -296,9 +296,9 @@ cudaError_t launch_draft_select(const uint32_t *records, const uint32_t *forced,
                                 uint32_t *next_tokens, uint32_t *verify_tokens, cudaStream_t stream);
 // Longest-matching-prefix acceptance + stop truncation (speculative_decode.rs:54-105) per stream, then
 // pending[slot[s]] = normalized lane (s, committed-1).  out row = {accepted, committed, emitted_count, 0,
-// emitted[drafts+1], targets[drafts+1]}.
+// emitted[drafts+1], targets[drafts+1]}.  own_drafts[s] <= drafts: how many of the drafts count for the stream.
 cudaError_t launch_accept(const uint32_t *verify_tokens, const uint32_t *target_records, const uint32_t *stop_tokens,
-                          const int32_t *stop_counts, int max_stop, int streams, int drafts, uint32_t *out,
+                          const int32_t *stop_counts, const int32_t *own_drafts, int max_stop, int streams, int drafts, uint32_t *out,
                           const uint16_t *normalized, uint16_t *pending, const int32_t *slots, int hidden,
                           cudaStream_t stream);
 

@@ -98,7 +98,7 @@ cudaError_t launch_draft_select(const uint32_t *records, const uint32_t *forced,
 
 __global__ void accept_kernel(const uint32_t *__restrict__ verify_tokens, const uint32_t *__restrict__ target_records,
                               const uint32_t *__restrict__ stop_tokens, const int32_t *__restrict__ stop_counts,
-                              int max_stop, int drafts, uint32_t *__restrict__ out, const uint32_t *__restrict__ normalized,
+                              const int32_t *__restrict__ own_drafts, int max_stop, int drafts, uint32_t *__restrict__ out, const uint32_t *__restrict__ normalized,
                               uint32_t *__restrict__ pending, const int32_t *__restrict__ slots, int words) {
     grid_launch_dependents();
     grid_dependency_wait();
@@ -108,8 +108,9 @@ __global__ void accept_kernel(const uint32_t *__restrict__ verify_tokens, const 
     uint32_t *row = out + static_cast<size_t>(s) * (4 + 2 * width);
     if (threadIdx.x == 0) {
         const uint32_t *inputs = verify_tokens + static_cast<size_t>(s) * width;  // [x, d_1 .. d_k]
+        const int own = own_drafts[s];  // this stream's window; the drafts behind it only keep the batch rectangular
         int accepted = 0;
-        while (accepted < drafts && inputs[accepted + 1] == target_records[(static_cast<size_t>(s) * width + accepted) * 4]) accepted++;
+        while (accepted < own && inputs[accepted + 1] == target_records[(static_cast<size_t>(s) * width + accepted) * 4]) accepted++;
         int committed = accepted + 1;
         int count = 0;
         for (int i = 0; i < accepted; i++) row[4 + count++] = inputs[i + 1];
@@ -139,11 +140,11 @@ __global__ void accept_kernel(const uint32_t *__restrict__ verify_tokens, const 
 }
 
 cudaError_t launch_accept(const uint32_t *verify_tokens, const uint32_t *target_records, const uint32_t *stop_tokens,
-                          const int32_t *stop_counts, int max_stop, int streams, int drafts, uint32_t *out,
+                          const int32_t *stop_counts, const int32_t *own_drafts, int max_stop, int streams, int drafts, uint32_t *out,
                           const uint16_t *normalized, uint16_t *pending, const int32_t *slots, int hidden,
                           cudaStream_t stream) {
     if (streams <= 0) return cudaSuccess;
-    return launch_dependent(accept_kernel, dim3(streams), dim3(256), 0, 1, stream, verify_tokens, target_records, stop_tokens, stop_counts, max_stop, drafts, out, reinterpret_cast<const uint32_t *>(normalized), reinterpret_cast<uint32_t *>(pending), slots, hidden / 2);
+    return launch_dependent(accept_kernel, dim3(streams), dim3(256), 0, 1, stream, verify_tokens, target_records, stop_tokens, stop_counts, own_drafts, max_stop, drafts, out, reinterpret_cast<const uint32_t *>(normalized), reinterpret_cast<uint32_t *>(pending), slots, hidden / 2);
 }
 
 // ---- vocabulary-parallel arg-max ------------------------------------------------------------------------------
