@@ -188,6 +188,12 @@ std::shared_ptr<MountedModel> MountedModel::mount(const std::string &path, const
         if (layer.has_kv) model->kv_bytes_per_token_ += static_cast<uint64_t>(2) * layer.kv_heads * layer.head_width * 2;
     }
     for (const ComponentPlan &layer : plan.draft_layers) add_pool(layer);
+    {
+        std::vector<PagePool> pools;
+        for (size_t i = 0; i < model->kv_pools_.size(); i++) pools.push_back(PagePool{static_cast<uint8_t *>(model->kv_pools_[i].ptr), model->kv_page_bytes_[i]});
+        model->page_pools_ = device_alloc(std::max<size_t>(1, pools.size()) * sizeof(PagePool));
+        cuda_check(cudaMemcpy(model->page_pools_.ptr, pools.data(), pools.size() * sizeof(PagePool), cudaMemcpyHostToDevice), "page pools upload");
+    }
     model->block_table_ = device_alloc(sizeof(int32_t) * options.max_streams * model->pages_per_stream_);
     model->build_rope_tables();
     cuda_check(cudaDeviceGetAttribute(&model->sm_count_, cudaDevAttrMultiProcessorCount, options.device), "cudaDeviceGetAttribute");
@@ -236,6 +242,7 @@ MountedModel::~MountedModel() {
         cudaFree(stack->device_layers.ptr);
     }
     cudaFree(block_table_.ptr);
+    cudaFree(page_pools_.ptr);
 }
 
 const void *MountedModel::tensor(const std::string &name) const {
@@ -632,6 +639,7 @@ Engine::Engine(std::shared_ptr<MountedModel> model) : model_(std::move(model)) {
     for (int slot = options.max_streams - 1; slot >= 0; slot--) free_slots_.push_back(slot);
     for (int page = model_->physical_pages() - 1; page >= 0; page--) free_pages_.push_back(page);
     page_refcount_.assign(model_->physical_pages(), 0);
+    page_copies_device_ = device_alloc(MAX_PAGE_COPIES * sizeof(PageCopy));
     block_table_host_.assign(static_cast<size_t>(options.max_streams) * model_->pages_per_stream(), 0);
 }
 
@@ -642,7 +650,7 @@ Engine::~Engine() {
     for (auto &entry : signals_) cudaFree(entry.second.ptr);
     for (DeviceBuffer *buffer : {&frame_a_, &frame_b_, &embedding_out_, &normalized_, &draft_normalized_, &draft_hidden_in_, &logits_,
                                  &records_, &argmax_scratch_, &sampler_scratch_, &sampler_table_, &lane_tokens_, &lane_positions_, &lane_slots_, &pending_hidden_, &pending_backup_, &attention_scratch_, &attention_blocks_,
-                                 &cycle_state_, &int4_activations_, &moe_quantised_, &moe_quantised_scales_, &moe_groups_, &kernel_error_, &tp_partial_, &tp_exchange_, &tp_description_, &stack_q_, &stack_attention_out_, &stack_activation_, &stack_barrier_, &stack_timing_, &prefix_pending_})
+                                 &cycle_state_, &int4_activations_, &moe_quantised_, &moe_quantised_scales_, &moe_groups_, &kernel_error_, &tp_partial_, &tp_exchange_, &tp_description_, &stack_q_, &stack_attention_out_, &stack_activation_, &stack_barrier_, &stack_timing_, &prefix_pending_, &page_copies_device_})
         cudaFree(buffer->ptr);
     cudaFreeHost(staging_);
     cudaFreeHost(host_records_);
@@ -1151,23 +1159,24 @@ void Engine::ensure_pages(Stream &s, uint64_t last_tick) {
     // a page shared with another stream is replaced by a private copy before it is written (copy-on-write)
     const int page_tokens = model_->options().page_tokens;
     const int pages = static_cast<int>(s.pages.size());
-    if (last_tick >= model_->rope_positions()) fail("stream tick exceeds the mounted position range");
+    if (last_tick >= model_->rope_positions()) {
+        copy_pages();
+        fail("stream tick exceeds the mounted position range");
+    }
     uint64_t first_tick = s.next_tick;
     for (uint64_t page_index = first_tick / page_tokens; page_index <= last_tick / page_tokens; page_index++) {
         int logical = static_cast<int>(page_index % pages);
         int32_t physical = s.pages[logical];
         if (physical >= 0 && page_refcount_[physical] == 1) continue;
-        if (free_pages_.empty()) fail("KV page pool exhausted");
+        if (free_pages_.empty()) {
+            copy_pages();
+            fail("KV page pool exhausted");
+        }
         int32_t fresh = free_pages_.back();
         free_pages_.pop_back();
         page_refcount_[fresh] = 1;
         if (physical >= 0) {  // shared page: copy, then drop the shared reference
-            for (int layer = 0; layer < model_->kv_layer_count(); layer++) {
-                size_t bytes = model_->page_bytes(layer);
-                uint8_t *pool = reinterpret_cast<uint8_t *>(model_->kv_layer(layer).pool);
-                cuda_check(cudaMemcpyAsync(pool + fresh * bytes, pool + physical * bytes, bytes, cudaMemcpyDeviceToDevice, cuda_stream_),
-                           "copy-on-write page copy");
-            }
+            page_copies_.push_back(PageCopy{physical, fresh});
             page_refcount_[physical]--;
         }
         s.pages[logical] = fresh;
@@ -1175,7 +1184,22 @@ void Engine::ensure_pages(Stream &s, uint64_t last_tick) {
     }
 }
 
+// The copies that ensure_pages asked for, all layers of all pages in one launch (a fork of 32 streams writes 32 pages of
+// 33 layers: a thousand copies of 64 KB took 5 ms one by one, on the host and on the stream).  They run before anything
+// that writes a page: every batch comes through sync_block_tables, and a failing ensure_pages through here.
+void Engine::copy_pages() {
+    for (size_t first = 0; first < page_copies_.size(); first += MAX_PAGE_COPIES) {
+        const size_t count = std::min<size_t>(MAX_PAGE_COPIES, page_copies_.size() - first);
+        upload(page_copies_device_.ptr, page_copies_.data() + first, count * sizeof(PageCopy), "page copies upload");
+        check(launch_copy_pages(static_cast<const PagePool *>(model_->page_pools_device()), model_->kv_layer_count(), static_cast<const PageCopy *>(page_copies_device_.ptr),
+                                static_cast<int>(count), cuda_stream_),
+              "copy-on-write page copy");
+    }
+    page_copies_.clear();
+}
+
 void Engine::sync_block_tables() {
+    copy_pages();
     const int pages = model_->pages_per_stream();
     for (auto &entry : streams_) {
         Stream &s = entry.second;

@@ -84,7 +84,7 @@ public:
     uint32_t capacity() const { return static_cast<uint32_t>(pages_per_stream_) * options_.page_tokens; }
     int kv_layer_count() const { return static_cast<int>(kv_pools_.size()); }
     KvLayer kv_layer(int index) const;
-    size_t page_bytes(int index) const { return kv_page_bytes_[index]; }
+    const void *page_pools_device() const { return page_pools_.ptr; }  // PagePool of every KV layer
     int32_t *block_table_device() const { return static_cast<int32_t *>(block_table_.ptr); }
     const uint32_t *rope_table(float theta, int rotary) const;
     uint32_t rope_positions() const { return rope_positions_; }
@@ -117,7 +117,7 @@ private:
     std::vector<DeviceBuffer> kv_pools_;
     std::vector<size_t> kv_page_bytes_;
     std::vector<std::pair<int, int>> kv_shapes_;  // (kv_heads, head_width) per kv layer
-    DeviceBuffer block_table_;
+    DeviceBuffer block_table_, page_pools_;
     int pages_per_stream_ = 0, physical_pages_ = 0;
     std::map<std::pair<uint32_t, int>, DeviceBuffer> rope_tables_;  // (theta bits, rotary) -> table
     uint32_t rope_positions_ = 0;
@@ -345,6 +345,7 @@ private:
     void run_speculative_cycles(std::vector<Stream *> &batch, const std::vector<int> &own_drafts, int draft_count,
                                 const std::function<void(const OutputEvent &)> &on_output, RunReport &report);
     void check(cudaError_t status, const char *what);
+    void copy_pages();
     void *signal_buffer(const std::string &name);
 
     std::shared_ptr<MountedModel> model_;
@@ -353,6 +354,8 @@ private:
     std::vector<int32_t> free_pages_;
     std::vector<int32_t> page_refcount_;
     std::vector<int32_t> block_table_host_;
+    std::vector<PageCopy> page_copies_;  // asked for, not yet enqueued
+    DeviceBuffer page_copies_device_;
     cudaStream_t cuda_stream_ = nullptr;
     cudaEvent_t event_a_ = nullptr, event_b_ = nullptr, event_begin_ = nullptr, event_end_ = nullptr, run_begin_ = nullptr, run_end_ = nullptr;
 

@@ -29,6 +29,17 @@ struct KvLayer {
     uint32_t capacity;  // pages_per_slot * page_tokens (ring length in tokens)
 };
 
+// Copies of KV pages within their pools: pages[i].from -> pages[i].to in every layer's pool.
+struct PagePool {
+    uint8_t *base;
+    size_t page_bytes;  // a multiple of 4
+};
+struct PageCopy {
+    int32_t from, to;
+};
+constexpr int MAX_PAGE_COPIES = 1024;  // of one launch
+cudaError_t launch_copy_pages(const PagePool *pools, int layers, const PageCopy *pages, int count, cudaStream_t stream);
+
 cudaError_t launch_embedding(const uint16_t *table, const uint32_t *tokens, uint16_t *out, int lanes, int width,
                              int vocab, float scale, cudaStream_t stream);
 

@@ -9,6 +9,30 @@
 
 namespace nerve {
 
+// Bound by the pages' bytes (32 pages of 64 KB in 33 layers: 140 MB moved); four CTAs share a page so that a single
+// stream's page still spreads over the chip.
+constexpr int PAGE_COPY_PARTS = 4;
+__global__ void __launch_bounds__(256) copy_pages_kernel(const PagePool *__restrict__ pools, const PageCopy *__restrict__ pages) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const PagePool pool = pools[blockIdx.y];
+    const PageCopy page = pages[blockIdx.x];
+    const uint8_t *from = pool.base + static_cast<size_t>(page.from) * pool.page_bytes;
+    uint8_t *to = pool.base + static_cast<size_t>(page.to) * pool.page_bytes;
+    const size_t first = blockIdx.z * blockDim.x + threadIdx.x, stride = static_cast<size_t>(PAGE_COPY_PARTS) * blockDim.x;
+    if (pool.page_bytes % 16 == 0) {
+#pragma unroll 4
+        for (size_t i = first; i < pool.page_bytes / 16; i += stride) reinterpret_cast<uint4 *>(to)[i] = reinterpret_cast<const uint4 *>(from)[i];
+    } else {
+        for (size_t i = first; i < pool.page_bytes / 4; i += stride) reinterpret_cast<uint32_t *>(to)[i] = reinterpret_cast<const uint32_t *>(from)[i];
+    }
+}
+
+cudaError_t launch_copy_pages(const PagePool *pools, int layers, const PageCopy *pages, int count, cudaStream_t stream) {
+    if (layers <= 0 || count <= 0) return cudaSuccess;
+    return launch_dependent(copy_pages_kernel, dim3(count, layers, PAGE_COPY_PARTS), dim3(256), 0, 1, stream, pools, pages);
+}
+
 // embedding_lookup_bf16.comp.template:31-46: out = bf16(bf16(row) * scale); a
 // token id >= vocab leaves the frame untouched.
 __global__ void embedding_kernel(const uint32_t *__restrict__ table, const uint32_t *__restrict__ tokens,
