@@ -83,8 +83,10 @@ constexpr size_t attention_smem() {
     return tiles > merge ? tiles : merge;
 }
 
+// The verify form of 32 rows takes two CTAs per SM (128 registers, 56 bytes of spills): it waits for its K and V more than
+// it multiplies, and 32 streams x 8 kv heads x splits are several waves of one CTA per SM (44 -> 35 us per launch).
 template <int HD, int ROW_WARPS, int TOKEN_WARPS>
-__global__ void __launch_bounds__(ROW_WARPS *TOKEN_WARPS * 32) attention_tile_kernel(const __grid_constant__ AttentionArgs a) {
+__global__ void __launch_bounds__(ROW_WARPS *TOKEN_WARPS * 32, ROW_WARPS * TOKEN_WARPS == 8 && TOKEN_WARPS > 1 ? 2 : 1) attention_tile_kernel(const __grid_constant__ AttentionArgs a) {
     constexpr int THREADS = ROW_WARPS * TOKEN_WARPS * 32, ROWS = ROW_WARPS * 16;
     constexpr int TOKENS = TILE / TOKEN_WARPS;  // of a tile, per warp
     constexpr int K_STEPS = HD / 16, N_TILES = TOKENS / 8, D_TILES = HD / 8;
