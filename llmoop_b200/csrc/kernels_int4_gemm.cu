@@ -19,7 +19,7 @@
 //   the next warp: one thread issues the MMAs (A from tensor memory, B from shared memory) and commits;
 //   the last warp: one thread copies the activations, which prepare_activations_kernel left in global memory in the
 //              order of the 128-byte-swizzled shared-memory tiles: two bulk copies per group of 128 columns.
-// With ROW_TILES = 2 every activation byte read from L2 feeds two MMAs.  K may be split over a cluster of CTAs whose
+// With ROW_TILES = 2 every activation byte read from L2 feeds two MMAs; stages of half a group make room for 160 lanes there.  K may be split over a cluster of CTAs whose
 // partial sums meet through distributed shared memory (shapes with too few tiles to fill the chip).
 // Waits are bounded; a wait that expires sets the error word, and the CTA still frees its tensor memory.
 #include <cuda_fp16.h>
@@ -37,7 +37,7 @@ namespace {
 template <int ROW_TILES>
 constexpr int gemm_threads() { return ROW_TILES * 256 + 64; }
 constexpr unsigned int GEMM_SPIN_LIMIT = 1u << 17;
-constexpr int GEMM_MAX_B_STAGES = 8, GEMM_MAX_A_STAGES = 4;
+constexpr int GEMM_MAX_B_STAGES = 8, GEMM_MAX_A_STAGES = 4;  // of 64 or 128 columns of K each
 constexpr size_t GEMM_SMEM_ONE = 225 * 1024, GEMM_SMEM_TWO = 111 * 1024;  // one or two CTAs per SM
 constexpr size_t GEMM_BARRIER_BYTES = 256, GEMM_TAIL_BYTES = GEMM_BARRIER_BYTES + 256 * sizeof(float);  // barriers, lane factors
 
@@ -152,7 +152,10 @@ __device__ __forceinline__ void locate_rows(const GemmArgs &a, int block_tile, i
     row = (tile - a.first_tile[matrix]) * 128 + quarter * 32;
 }
 
-template <int ROW_TILES>
+// PARTS: stages of both operands to a group of 128 columns (1 or 2).  Half groups leave tensor memory for two row tiles of
+// 129 to 160 lanes: 28672 x 8192 with 160 lanes is one wave then instead of two (82 -> 72 us), 28672 x 4096 with 2048 lanes
+// seven instead of eleven waves of 256 lanes (490 -> 407 us).
+template <int ROW_TILES, int PARTS>
 __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 : 1) linear_int4_gemm_kernel(const __grid_constant__ GemmArgs a) {
     constexpr int ROWS = 128 * ROW_TILES, WARPS = 8 * ROW_TILES;  // warps that prepare the A operand: two sets, one for every other group
     constexpr uint32_t SLOT = WARPS * 2048;                         // one raw stage: 32 rows x 64 bytes of every such warp
@@ -162,7 +165,8 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
     const int groups = a.k >> 7, first_group = groups * split / splits, own_groups = groups * (split + 1) / splits - first_group;
     const int m0 = blockIdx.x * a.tile_lanes;
     const int n_lanes = min(a.tile_lanes, a.lane_blocks * 8 - m0);  // multiple of 16
-    const uint32_t b_stage_bytes = static_cast<uint32_t>(a.tile_lanes) * 256;
+    constexpr uint32_t A_COLUMNS = 64 / PARTS;  // of tensor memory, per stage and row tile
+    const uint32_t b_stage_bytes = static_cast<uint32_t>(a.tile_lanes) * (256 / PARTS);
     uint8_t *const raw = smem + static_cast<size_t>(a.b_stages) * b_stage_bytes;
     uint16_t *const scales = reinterpret_cast<uint16_t *>(raw + a.raw_stages * SLOT);
     const uint32_t a_full = shared_address(smem) + a.barrier_offset, a_empty = a_full + 8 * GEMM_MAX_A_STAGES, b_full = a_empty + 8 * GEMM_MAX_A_STAGES,
@@ -270,12 +274,19 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
         }
         const uint32_t read_base = warp_raw + static_cast<uint32_t>(lane * 64);
         const uint32_t read_swizzle = static_cast<uint32_t>((lane >> 1) & 3);
-        const uint32_t tmem_rows = tmem_a + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(row_tile) * 64;
+        const uint32_t tmem_rows = tmem_a + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(row_tile) * A_COLUMNS;
         const uint16_t *scale = scales + set * ROWS + row_tile * 128 + quarter * 32 + lane;
         uint32_t read_slot = 0;
         // ring position of the item's group among the A stages, and the parity of its last release (the first round waits for none)
-        int stage = set;
+        int stage = set * PARTS;
         uint32_t parity = 1;
+        auto advance = [&](int by) {
+            stage += by;
+            if (stage >= a.a_stages) {
+                stage -= a.a_stages;
+                parity ^= 1;
+            }
+        };
         for (int item = 0; item < items; item++) {
             request();
             switch (a.raw_stages) {  // the item's own copies have landed
@@ -295,33 +306,32 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
                 asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(words[c].x), "=r"(words[c].y), "=r"(words[c].z), "=r"(words[c].w) : "r"(address));
             }
             read_slot = read_slot + SLOT == slots_end ? 0 : read_slot + SLOT;
-            if (!wait_barrier(a_empty + stage * 8, parity, a.error_flag)) {
-                alive = false;
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t target = tmem_rows + static_cast<uint32_t>(stage) * (64 * ROW_TILES);
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                uint32_t v[4][4];
-                dequantise_word(words[c].x, scale2, v[0]);
-                dequantise_word(words[c].y, scale2, v[1]);
-                dequantise_word(words[c].z, scale2, v[2]);
-                dequantise_word(words[c].w, scale2, v[3]);
-                asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(target + c * 16),
-                             "r"(v[0][0]), "r"(v[0][1]), "r"(v[0][2]), "r"(v[0][3]), "r"(v[1][0]), "r"(v[1][1]), "r"(v[1][2]), "r"(v[1][3]), "r"(v[2][0]),
-                             "r"(v[2][1]), "r"(v[2][2]), "r"(v[2][3]), "r"(v[3][0]), "r"(v[3][1]), "r"(v[3][2]), "r"(v[3][3])
-                             : "memory");
+            for (int part = 0; part < PARTS; part++) {
+                if (alive && !wait_barrier(a_empty + stage * 8, parity, a.error_flag)) alive = false;
+                if (!alive) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t target = tmem_rows + static_cast<uint32_t>(stage) * (A_COLUMNS * ROW_TILES);
+#pragma unroll
+                for (int c = 0; c < 4 / PARTS; c++) {
+                    const uint4 packed = words[part * (4 / PARTS) + c];
+                    uint32_t v[4][4];
+                    dequantise_word(packed.x, scale2, v[0]);
+                    dequantise_word(packed.y, scale2, v[1]);
+                    dequantise_word(packed.z, scale2, v[2]);
+                    dequantise_word(packed.w, scale2, v[3]);
+                    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(target + c * 16),
+                                 "r"(v[0][0]), "r"(v[0][1]), "r"(v[0][2]), "r"(v[0][3]), "r"(v[1][0]), "r"(v[1][1]), "r"(v[1][2]), "r"(v[1][3]), "r"(v[2][0]),
+                                 "r"(v[2][1]), "r"(v[2][2]), "r"(v[2][3]), "r"(v[3][0]), "r"(v[3][1]), "r"(v[3][2]), "r"(v[3][3])
+                                 : "memory");
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a_full + stage * 8) : "memory");
+                advance(part + 1 < PARTS ? 1 : PARTS + 1);  // over the other set's group
             }
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a_full + stage * 8) : "memory");
-            stage += 2;
-            if (stage >= a.a_stages) {
-                stage -= a.a_stages;
-                parity ^= 1;
-            }
+            if (!alive) break;
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (warp == WARPS) {
@@ -330,7 +340,7 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
         const uint64_t b_first = swizzled_descriptor(shared_address(smem)), b_half = static_cast<uint64_t>(n_lanes) * 8;  // descriptors count 16 bytes
         int stage_a = 0, stage_b = 0;
         uint32_t parity_a = 0, parity_b = 0;
-        for (int group = 0; group < own_groups; group++) {
+        for (int part = 0; part < own_groups * PARTS; part++) {
             if (!wait_barrier(b_full + stage_b * 8, parity_b, a.error_flag) || !wait_barrier(a_full + stage_a * 8, parity_a, a.error_flag)) {
                 alive = false;
                 break;
@@ -340,11 +350,11 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
                 const uint64_t b_stage = b_first + static_cast<uint64_t>(stage_b) * (b_stage_bytes >> 4);
 #pragma unroll
                 for (int t = 0; t < ROW_TILES; t++) {
-                    const uint32_t d_address = tmem + t * d_stride, a_address = tmem_a + static_cast<uint32_t>(stage_a * ROW_TILES + t) * 64;
+                    const uint32_t d_address = tmem + t * d_stride, a_address = tmem_a + static_cast<uint32_t>(stage_a * ROW_TILES + t) * A_COLUMNS;
 #pragma unroll
-                    for (int step = 0; step < 8; step++) {  // K = 16 per instruction; four steps to a 128-byte row of the swizzled tile
+                    for (int step = 0; step < 8 / PARTS; step++) {  // K = 16 per instruction; four steps to a 128-byte row of the swizzled tile
                         const uint64_t b_descriptor = b_stage + (step >> 2) * b_half + (step & 3) * 2;
-                        const uint32_t accumulate = (group > 0 || step > 0) ? 1u : 0u;
+                        const uint32_t accumulate = (part > 0 || step > 0) ? 1u : 0u;
                         asm volatile(
                             "{\n"
                             ".reg .pred p;\n"
@@ -377,23 +387,23 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
         const uint32_t bytes = static_cast<uint32_t>(n_lanes) * 128;
         int stage = 0;
         uint32_t parity = 1;  // the first round waits for no release
-        for (int group = 0; group < own_groups; group++) {
+        for (int item = 0; item < own_groups * PARTS; item++) {
             if (!wait_barrier(b_empty + stage * 8, parity, a.error_flag)) {
-                for (int g = group > a.b_stages ? group - a.b_stages : 0; g < group; g++)  // the copies in flight land before the CTA gives its memory up
+                for (int g = item > a.b_stages ? item - a.b_stages : 0; g < item; g++)  // the copies in flight land before the CTA gives its memory up
                     wait_barrier(b_full + (g % a.b_stages) * 8, static_cast<uint32_t>((g / a.b_stages) & 1), a.error_flag);
                 break;
             }
             if (elect_one()) {
                 const uint32_t target = shared_address(smem) + static_cast<uint32_t>(stage) * b_stage_bytes, full = b_full + stage * 8;
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"(2 * bytes) : "memory");
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"(2 / PARTS * bytes) : "memory");
 #pragma unroll
-                for (int part = 0; part < 2; part++)
+                for (int part = 0; part < 2 / PARTS; part++)
                     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(target + part * bytes),
                                  "l"(source + static_cast<size_t>(part) * part_bytes), "r"(bytes), "r"(full)
                                  : "memory");
             }
             __syncwarp();
-            source += 2 * part_bytes;
+            source += 2 / PARTS * part_bytes;
             if (++stage == a.b_stages) {
                 stage = 0;
                 parity ^= 1;
@@ -609,46 +619,50 @@ __global__ void __launch_bounds__(PREPARE_THREADS) prepare_activations_kernel(co
 }
 
 struct GemmPlan {
-    int row_tiles = 1, lane_tiles = 1, tile_lanes = 16, splits = 1, a_stages = 2, b_stages = 2, raw_stages = 3;
+    int row_tiles = 1, parts = 1, lane_tiles = 1, tile_lanes = 16, splits = 1, a_stages = 2, b_stages = 2, raw_stages = 3;
     uint32_t tmem_columns = 512;
     size_t smem = 0;
 };
 
-// Tile shape and K split by an estimate of the launch's time in SM cycles.  Per group of 128 columns a CTA needs 4
-// cycles per lane and row tile on the tensor cores and about 280 per row tile to dequantise; a wave that is not full
-// costs as much as a full one, every CTA pays for filling its pipeline and for its epilogue, and two CTAs share an SM
-// where shared and tensor memory allow.
+// Tile shape and K split by an estimate of the launch's time in SM cycles, fitted to the times of every plan at 84 points
+// (16 .. 2048 lanes of six matrices from 4096 x 4096 to 28672 x 8192; the plan it takes is 2 % slower than the best one on
+// average, an estimate without the dequantisation's latency took 7 %).  Per group of 128 columns a CTA needs 5.6 cycles per
+// lane and row tile on the tensor cores (4 at the pipe's nominal rate) or the time of its operand warps, which wait more
+// than they work: two CTAs of an SM do not slow one another down.  A wave that is not full costs as much as a full one, and
+// every CTA pays for filling its pipeline and for its epilogue, split ones for meeting their peers.
 GemmPlan plan_gemm(int matrix_tiles, int lanes, int groups, bool silu) {
     const int padded = (lanes + 15) / 16 * 16;
     GemmPlan best;
     double best_cycles = 1e30;
-    for (int row_tiles = 1; row_tiles <= 2; row_tiles++) {
-        const int most = 256 / row_tiles;
+    for (int form = 0; form < 3; form++) {
+        const int row_tiles = form == 0 ? 1 : 2, parts = form == 2 ? 2 : 1;
+        const int most = form == 0 ? 256 : form == 1 ? 128 : 160;
         const int fewest_tiles = (padded + most - 1) / most;
         // (a SiLU pair covers 64 rows of both matrices per row tile)
         const int blocks = silu ? (row_tiles == 2 ? matrix_tiles / 2 : matrix_tiles) : (matrix_tiles + row_tiles - 1) / row_tiles;
         for (int lane_tiles = fewest_tiles; lane_tiles <= fewest_tiles + 2; lane_tiles++) {
             const int tile_lanes = ((padded + lane_tiles - 1) / lane_tiles + 15) / 16 * 16;
-            if (tile_lanes > most || (lane_tiles > 1 && tile_lanes * (lane_tiles - 1) >= padded)) continue;
+            if (tile_lanes > most || (form == 2 && tile_lanes <= 128) || (lane_tiles > 1 && tile_lanes * (lane_tiles - 1) >= padded)) continue;
             for (int splits = 1; splits <= 8 && (splits == 1 || splits * 2 <= groups); splits *= 2) {
                 const int own = (groups + splits - 1) / splits;
                 GemmPlan plan;
                 plan.row_tiles = row_tiles;
+                plan.parts = parts;
                 plan.lane_tiles = lane_tiles;
                 plan.tile_lanes = tile_lanes;
                 plan.splits = splits;
-                const size_t scales = static_cast<size_t>(own) * 256 * row_tiles, b_stage = static_cast<size_t>(tile_lanes) * 256;
+                const size_t scales = static_cast<size_t>(own) * 256 * row_tiles, b_stage = static_cast<size_t>(tile_lanes) * (256 / parts);
                 const size_t sums = static_cast<size_t>(tile_lanes) * 512 * row_tiles;
                 int per_sm = 0;
                 for (int share = row_tiles == 1 && tile_lanes <= 64 ? 2 : 1; share >= 1 && per_sm == 0; share--) {
                     const size_t limit = share == 2 ? GEMM_SMEM_TWO : GEMM_SMEM_ONE;
-                    // stages: the pair that looks furthest ahead, counted in groups, on its shorter side (a raw slot holds
+                    // stages: the pair that looks furthest ahead, counted in stages of B, on its shorter side (a raw slot holds
                     // two groups, and the one being read does not count)
                     int best_ahead = 0;
                     for (int raw = 3; raw <= 6; raw++)
                         for (int b = 2; b <= GEMM_MAX_B_STAGES; b++) {
                             const size_t bytes = std::max(static_cast<size_t>(b) * b_stage + static_cast<size_t>(raw) * 16384 * row_tiles + scales, sums);
-                            const int ahead = std::min(2 * (raw - 1), b);
+                            const int ahead = std::min(2 * parts * (raw - 1), b);
                             if (bytes > limit || ahead <= best_ahead) continue;
                             best_ahead = ahead;
                             plan.b_stages = b;
@@ -660,14 +674,14 @@ GemmPlan plan_gemm(int matrix_tiles, int lanes, int groups, bool silu) {
                 if (per_sm == 0) continue;
                 const int d_columns = (tile_lanes + 31) / 32 * 32 * row_tiles;
                 plan.tmem_columns = per_sm == 2 ? 256 : 512;
-                plan.a_stages = std::min(GEMM_MAX_A_STAGES, (static_cast<int>(plan.tmem_columns) - d_columns) / (64 * row_tiles));
-                if (plan.a_stages < 2) continue;
-                const double per_group = std::max(row_tiles * 4.0 * tile_lanes, row_tiles * 280.0);
-                const double ctas = static_cast<double>(blocks) * lane_tiles * splits;
-                const double waves = std::max(1.0, (ctas + 148 * per_sm - 1) / (148 * per_sm));
-                const double whole = static_cast<double>(static_cast<long>(waves));
-                const double shared_sm = ctas > 148 ? per_sm : 1;
-                const double cycles = whole * (own * per_group * shared_sm + 5000.0 + row_tiles * tile_lanes * 12.0) + (splits > 1 ? 1500.0 : 0.0);
+                plan.a_stages = std::min(GEMM_MAX_A_STAGES, (static_cast<int>(plan.tmem_columns) - d_columns) / (64 / parts * row_tiles));
+                if (plan.a_stages < parts + 1) continue;
+                const int ctas = blocks * lane_tiles * splits, together = ctas > 148 ? per_sm : 1;
+                const double dequantise = row_tiles == 2 ? 430.0 : together == 2 ? 350.0 : 680.0;
+                const double per_group = 200.0 + row_tiles * std::max(5.6 * tile_lanes, dequantise);
+                const int waves = (ctas + 148 * per_sm - 1) / (148 * per_sm);
+                const double cycles = waves * (own * per_group * together + 7700.0 + 25.0 * row_tiles * tile_lanes) +
+                                      (splits > 1 ? 650.0 * splits + 25.0 * row_tiles * tile_lanes : 0.0);
                 if (cycles < best_cycles) {
                     best_cycles = cycles;
                     best = plan;
@@ -752,7 +766,7 @@ cudaError_t launch_linear_int4_gemm(const void *prepared, int branches, const ui
     int blocks = (tiles + plan.row_tiles - 1) / plan.row_tiles;
     if (silu) blocks = (ns[0] + 64 * plan.row_tiles - 1) / (64 * plan.row_tiles);
     const dim3 grid(plan.lane_tiles, blocks, plan.splits);
-    auto kernel = plan.row_tiles == 2 ? linear_int4_gemm_kernel<2> : linear_int4_gemm_kernel<1>;
+    auto kernel = plan.row_tiles == 1 ? linear_int4_gemm_kernel<1, 1> : plan.parts == 1 ? linear_int4_gemm_kernel<2, 1> : linear_int4_gemm_kernel<2, 2>;
     cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(GEMM_SMEM_ONE + GEMM_TAIL_BYTES));
     if (status != cudaSuccess) return status;
     return launch_dependent(kernel, grid, dim3(plan.row_tiles == 2 ? gemm_threads<2>() : gemm_threads<1>()), plan.smem + GEMM_TAIL_BYTES, plan.splits, stream, args);

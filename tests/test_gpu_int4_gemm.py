@@ -13,6 +13,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("lanes,n,k", [
     (9, 128, 128), (16, 130, 256), (17, 64, 4096), (64, 1000, 384), (65, 257, 1152), (128, 96, 2048), (129, 384, 640), (256, 128, 128), (257, 300, 256),
+    (150, 19000, 384), (310, 18945, 128),  # two row tiles of 160 lanes: half groups
 ])
 @pytest.mark.parametrize("x_scale,w_scale", [(1.0, 0.02), (2.0 ** 90, 2.0 ** -60), (2.0 ** -100, 2.0 ** 40)])
 def test_int4_gemm_edges_match_oracle(lanes, n, k, x_scale, w_scale):
