@@ -344,40 +344,66 @@ __global__ void __launch_bounds__(ROW_WARPS *TOKEN_WARPS * 32, ROW_WARPS * TOKEN
 // these layers keep the plain f32 order of additions - one product after the other, no split probabilities.
 __device__ __forceinline__ uint4 load16(const void *address) { return *reinterpret_cast<const uint4 *>(address); }
 
-template <int HD, int GROUP, int QL>
-constexpr size_t attention_f32_smem() {
-    constexpr int Q = QL * GROUP;
-    // K tile (padded rows), V tile, Q tile, probabilities, three per-query rows, the lanes' ticks
-    return static_cast<size_t>(TILE) * (HD + 8) * 2 + static_cast<size_t>(TILE) * HD * 2 + static_cast<size_t>(Q) * HD * 2 + static_cast<size_t>(Q) * TILE * 4 +
-           3 * Q * 4 + ((QL * 4 + 15) / 16) * 16;
+// Two f32 sums in one register pair (fma.rn.f32x2 rounds each as fmaf does).
+using float_pair = unsigned long long;
+__device__ __forceinline__ float_pair pair_of(float lo, float hi) {
+    float_pair out;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(out) : "f"(lo), "f"(hi));
+    return out;
+}
+__device__ __forceinline__ float2 halves_of(float_pair v) {
+    float2 out;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(out.x), "=f"(out.y) : "l"(v));
+    return out;
+}
+__device__ __forceinline__ float_pair pair_fma(float_pair a, float_pair b, float_pair c) {
+    float_pair out;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(out) : "l"(a), "l"(b), "l"(c));
+    return out;
 }
 
-// A CTA of 128 threads serves QL consecutive lanes of one stream x the GROUP query heads of one kv head (Q = QL*GROUP query
-// vectors) over one split of the context, tile by tile (TILE tokens):
-//   1. the K and V tiles are staged in shared memory with 16-byte loads issued back to back (one exposed
-//      latency per tile instead of one per token);
-//   2. scores: thread (t = tid % TILE, half = tid / TILE) dots K row t with Q/2 queries (K row stride is padded
-//      to HD+8 elements so the 16-byte shared loads of 8 consecutive rows hit distinct banks);
-//   3. per-query online softmax over the tile (one warp per query slice), probabilities to shared memory;
-//   4. P.V: thread d owns output dims d, d+128, .. for all Q queries, V rows read conflict-free.
-// A batch may mix streams: each stream contributes `lanes_per_stream` consecutive lanes, and a team never spans
-// two streams.  `group_slot` enumerates (stream, lane group) pairs.
 template <int HD, int GROUP, int QL>
-__device__ void attention_f32_body(const uint16_t *__restrict__ q, const KvLayer &kv, const LaneTable &lanes_meta, int lanes,
-                                   int lanes_per_stream, int q_heads, float scale, int split_tokens, int max_splits,
-                                   float *__restrict__ scratch, const AttentionBlock *__restrict__ ragged, int kv_head, int split, int group_slot,
-                                   uint8_t *smem_raw, int tid) {
-    constexpr int Q = QL * GROUP;
-    constexpr int KSTRIDE = HD + 8;
-    constexpr int DPT = HD / 128 > 0 ? HD / 128 : 1;  // output dims per thread (HD = 128 -> 1)
-    uint16_t *k_tile = reinterpret_cast<uint16_t *>(smem_raw);                 // [TILE][KSTRIDE]
-    uint16_t *v_tile = k_tile + TILE * KSTRIDE;                                 // [TILE][HD]
-    uint16_t *q_tile = v_tile + TILE * HD;                                      // [Q][HD]
-    float *p_tile = reinterpret_cast<float *>(q_tile + Q * HD);                 // [Q][TILE]
-    float *row_max = p_tile + Q * TILE;                                         // [Q]
-    float *row_sum = row_max + Q;                                               // [Q]
-    float *row_alpha = row_sum + Q;                                             // [Q]
-    uint32_t *lane_tick = reinterpret_cast<uint32_t *>(row_alpha + Q);          // [QL]
+struct AttentionF32 {
+    static constexpr int Q = QL * GROUP, THREADS = 128;
+    static constexpr int K_STRIDE = HD + 8;   // elements: 16-byte loads of eight consecutive rows hit distinct banks
+    static constexpr int P_STRIDE = Q + 4;    // floats: so do 16-byte stores
+    // scores: four queries x SCORE_TOKENS tokens per thread; a warp's threads share the queries
+    static constexpr int SCORE_SETS = Q / 4, SCORE_THREADS = THREADS / SCORE_SETS < TILE ? THREADS / SCORE_SETS : TILE;  // per set of queries
+    static constexpr int SCORE_TOKENS = TILE / SCORE_THREADS;
+    // P.V: two output dims x VALUE_QUERIES queries per thread
+    static constexpr int VALUE_SETS = THREADS / (HD / 2) < Q / 2 ? THREADS / (HD / 2) : Q / 2, VALUE_QUERIES = Q / VALUE_SETS;
+    static_assert(Q % 4 == 0 && VALUE_QUERIES % 2 == 0, "queries are taken in pairs");
+    struct Shared {
+        uint16_t k[TILE * K_STRIDE];  // K rows
+        uint16_t v[TILE * HD];        // V rows
+        float q[HD * Q];              // [dim][query]
+        float p[TILE * P_STRIDE];     // [token][query]: scores, then probabilities
+        float row_max[Q], row_sum[Q], row_alpha[Q];
+        uint32_t lane_tick[QL];
+        size_t offset[TILE];          // of the tile's K rows in the pool
+    };
+};
+
+// A CTA of 128 threads serves QL consecutive lanes of one stream x the GROUP query heads of one kv head (Q = QL*GROUP query
+// vectors) over one split of the context, tile by tile (TILE tokens): K and V rows through cp.async, scores, online softmax
+// per query, P.V.  Every score and every output dimension is one chain of f32 multiply-adds, over the head's dimensions and
+// over the tokens in order; two queries share a packed instruction.  The FP32 pipe and the shared-memory loads of the
+// operands bound it about equally: the queries are widened once, and a thread takes 4 queries x 2 tokens (scores) or 8
+// queries x 2 dims (P.V), so that a load feeds four packed operations.  (One token, eight queries unpacked per product and
+// one load per product before: 60 us for 24 lanes of 8 streams at a 1024-token context;
+// this 31.)
+// A batch may mix streams: each stream contributes `lanes_per_stream` consecutive lanes, and a CTA never spans two streams.
+template <int HD, int GROUP, int QL>
+__global__ void __launch_bounds__(128)
+attention_f32_kernel(const uint16_t *__restrict__ q, KvLayer kv, LaneTable lanes_meta, int lanes, int lanes_per_stream,
+                     int q_heads, float scale, int split_tokens, int max_splits, float *__restrict__ scratch, const AttentionBlock *__restrict__ ragged) {
+    using Form = AttentionF32<HD, GROUP, QL>;
+    constexpr int Q = Form::Q, THREADS = Form::THREADS;
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    typename Form::Shared &shared = *reinterpret_cast<typename Form::Shared *>(smem_raw);
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int kv_head = blockIdx.x, split = blockIdx.y, group_slot = blockIdx.z, tid = threadIdx.x;
 
     // lanes of one stream are consecutive and every stream of the batch has `lanes_per_stream` of them
     const int groups_per_stream = (lanes_per_stream + QL - 1) / QL;
@@ -393,208 +419,245 @@ __device__ void attention_f32_body(const uint16_t *__restrict__ q, const KvLayer
     const int slot = lanes_meta.slot[lane0];
     if (slot < 0) return;
     const uint32_t capacity = kv.capacity;
-    __syncthreads();  // the previous item of this team no longer reads the shared arrays
-    // the newest tick among this team's lanes bounds the context the CTA has to look at
-    uint32_t newest = 0;
-    if (tid < QL) {
-        int lane = lane0 + tid;
-        bool valid = lane < lanes && group_index * QL + tid < lanes_per_stream;
-        lane_tick[tid] = valid ? lanes_meta.position[lane] : 0xffffffffu;
-    }
-    __syncthreads();
+    // the newest tick among this CTA's lanes bounds the context it has to look at
+    uint32_t tick_of[QL], newest = 0;
 #pragma unroll
-    for (int i = 0; i < QL; i++)
-        if (lane_tick[i] != 0xffffffffu && lane_tick[i] > newest) newest = lane_tick[i];
+    for (int i = 0; i < QL; i++) {
+        const bool valid = lane0 + i < lanes && group_index * QL + i < lanes_per_stream;
+        tick_of[i] = valid ? lanes_meta.position[lane0 + i] : 0xffffffffu;
+        if (valid) newest = max(newest, tick_of[i]);
+    }
     const uint32_t tokens = newest + 1u < capacity ? newest + 1u : capacity;  // attended window of the newest lane
     const uint32_t first_tick = newest + 1u - tokens;
     const uint32_t begin = static_cast<uint32_t>(split) * split_tokens;
     if (begin >= tokens) return;
     const uint32_t end = begin + split_tokens < tokens ? begin + split_tokens : tokens;
+    if (tid < QL) {
+#pragma unroll
+        for (int i = 0; i < QL; i++)
+            if (tid == i) shared.lane_tick[i] = tick_of[i];
+    }
 
-    for (int index = tid; index < Q * HD / 8; index += 128) {
-        int query = index / (HD / 8), piece = index % (HD / 8);
-        int lane = lane0 + query / GROUP;
+    auto offset_of = [&](uint32_t tile_begin) {  // of row tid of a tile (rows beyond the split repeat its last one)
+        uint32_t ring = first_tick + min(tile_begin + static_cast<uint32_t>(tid), end - 1);
+        if (ring >= capacity) ring %= capacity;
+        return kv_token_offset(kv, slot, ring, kv_head, false);
+    };
+    const size_t value_half = static_cast<size_t>(kv.kv_heads) * kv.page_tokens * HD;
+    const uint32_t k_address = static_cast<uint32_t>(__cvta_generic_to_shared(shared.k)), v_address = static_cast<uint32_t>(__cvta_generic_to_shared(shared.v));
+    if (tid < TILE) shared.offset[tid] = offset_of(begin);
+    for (int index = tid; index < Q * HD / 8; index += THREADS) {
+        const int query = index % Q, piece = index / Q, lane = lane0 + query / GROUP;
         uint4 value = make_uint4(0, 0, 0, 0);
-        if (lane_tick[query / GROUP] != 0xffffffffu)
+        if (lane < lanes && group_index * QL + query / GROUP < lanes_per_stream)
             value = load16(q + (static_cast<size_t>(lane) * q_heads + kv_head * GROUP + query % GROUP) * HD + piece * 8);
-        *reinterpret_cast<uint4 *>(q_tile + query * HD + piece * 8) = value;
+        const uint32_t words[4] = {value.x, value.y, value.z, value.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            shared.q[(piece * 8 + 2 * i) * Q + query] = bf16_lo(words[i]);
+            shared.q[(piece * 8 + 2 * i + 1) * Q + query] = bf16_hi(words[i]);
+        }
     }
     if (tid < Q) {
-        row_max[tid] = -3.4028234663852886e38f;
-        row_sum[tid] = 0.0f;
+        shared.row_max[tid] = -3.4028234663852886e38f;
+        shared.row_sum[tid] = 0.0f;
     }
-    float acc[Q][DPT];
+    // P.V: this thread's dims and queries
+    constexpr int VQ = Form::VALUE_QUERIES;
+    const int value_set = tid / (HD / 2), value_dim = (tid % (HD / 2)) * 2;
+    bool value_active = value_set < Form::VALUE_SETS;
+    {
+        bool any = false;
 #pragma unroll
-    for (int query = 0; query < Q; query++)
+        for (int i = 0; i < QL; i++) any |= tick_of[i] != 0xffffffffu && i >= value_set * VQ / GROUP && i <= (value_set * VQ + VQ - 1) / GROUP;
+        value_active &= any;
+    }
+    float_pair acc[2][VQ / 2];
 #pragma unroll
-        for (int d = 0; d < DPT; d++) acc[query][d] = 0.0f;
+    for (int i = 0; i < VQ / 2; i++) acc[0][i] = acc[1][i] = 0ull;
 
     for (uint32_t tile_begin = begin; tile_begin < end; tile_begin += TILE) {
         const int count = static_cast<int>(end - tile_begin < TILE ? end - tile_begin : TILE);
-        __syncthreads();  // previous tile fully consumed (and q_tile / row_* initialised)
-        // ---- stage K and V rows: HD/8 16-byte pieces per row
-        for (int index = tid; index < count * (HD / 8); index += 128) {
-            int t = index / (HD / 8), piece = index % (HD / 8);
-            uint32_t ring = (first_tick + tile_begin + t) % capacity;
-            const uint16_t *krow = kv.pool + kv_token_offset(kv, slot, ring, kv_head, false);
-            const uint16_t *vrow = kv.pool + kv_token_offset(kv, slot, ring, kv_head, true);
-            *reinterpret_cast<uint4 *>(k_tile + t * KSTRIDE + piece * 8) = load16(krow + piece * 8);
-            *reinterpret_cast<uint4 *>(v_tile + t * HD + piece * 8) = load16(vrow + piece * 8);
+        __syncthreads();  // the previous tile is consumed (and the queries, offsets and row states are in place)
+#pragma unroll
+        for (int i = 0; i < TILE * (HD / 8) / THREADS; i++) {
+            const int index = tid + i * THREADS, t = index / (HD / 8), piece = index % (HD / 8);
+            const uint16_t *source = kv.pool + shared.offset[t] + piece * 8;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(k_address + (t * Form::K_STRIDE + piece * 8) * 2), "l"(source) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(v_address + (t * HD + piece * 8) * 2), "l"(source + value_half) : "memory");
         }
+        size_t next_offset = 0;
+        if (tid < TILE && tile_begin + TILE < end) next_offset = offset_of(tile_begin + TILE);
+        asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
+        if (tid < TILE && tile_begin + TILE < end) shared.offset[tid] = next_offset;
         // ---- scores
         {
-            const int t = tid % TILE, half = tid / TILE;
-            constexpr int QH = Q / 2 > 0 ? Q / 2 : 1;
-            float score[QH];
+            constexpr int ST = Form::SCORE_TOKENS;
+            const int set = tid / Form::SCORE_THREADS, t0 = tid % Form::SCORE_THREADS;
+            const bool active = set < Form::SCORE_SETS;
+            float_pair score[ST][2];
 #pragma unroll
-            for (int i = 0; i < QH; i++) score[i] = 0.0f;
-            if (t < count && half * QH < Q) {
+            for (int i = 0; i < ST; i++) score[i][0] = score[i][1] = 0ull;
+            if (active) {
+                const float *queries = shared.q + set * 4;
+#pragma unroll 4
                 for (int piece = 0; piece < HD / 8; piece++) {
-                    uint4 kraw = *reinterpret_cast<const uint4 *>(k_tile + t * KSTRIDE + piece * 8);
-                    const uint32_t kw[4] = {kraw.x, kraw.y, kraw.z, kraw.w};
+                    uint4 k[ST];
 #pragma unroll
-                    for (int i = 0; i < QH; i++) {
-                        uint4 qraw = *reinterpret_cast<const uint4 *>(q_tile + (half * QH + i) * HD + piece * 8);
-                        const uint32_t qw[4] = {qraw.x, qraw.y, qraw.z, qraw.w};
+                    for (int i = 0; i < ST; i++)
+                        k[i] = *reinterpret_cast<const uint4 *>(shared.k + (t0 + i * Form::SCORE_THREADS) * Form::K_STRIDE + piece * 8);
 #pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            score[i] = fmaf(bf16_lo(qw[j]), bf16_lo(kw[j]), score[i]);
-                            score[i] = fmaf(bf16_hi(qw[j]), bf16_hi(kw[j]), score[i]);
+                    for (int d = 0; d < 8; d++) {
+                        const ulonglong2 four = *reinterpret_cast<const ulonglong2 *>(queries + (piece * 8 + d) * Q);
+#pragma unroll
+                        for (int i = 0; i < ST; i++) {
+                            const uint32_t word = d < 2 ? k[i].x : d < 4 ? k[i].y : d < 6 ? k[i].z : k[i].w;
+                            const float value = (d & 1) ? bf16_hi(word) : bf16_lo(word);
+                            const float_pair both = pair_of(value, value);
+                            score[i][0] = pair_fma(four.x, both, score[i][0]);
+                            score[i][1] = pair_fma(four.y, both, score[i][1]);
                         }
                     }
                 }
-            }
-            const uint32_t token_tick = first_tick + tile_begin + t;
 #pragma unroll
-            for (int i = 0; i < QH; i++) {
-                int query = half * QH + i;
-                if (query >= Q) break;
-                uint32_t tick = lane_tick[query / GROUP];
-                // causal + ring window of this lane: ticks in (tick - capacity, tick]
-                bool visible = t < count && tick != 0xffffffffu && token_tick <= tick && token_tick + capacity > tick;
-                p_tile[query * TILE + t] = visible ? score[i] * scale : -INFINITY;
+                for (int i = 0; i < ST; i++) {
+                    const int t = t0 + i * Form::SCORE_THREADS;
+                    const uint32_t token_tick = first_tick + tile_begin + t;
+                    const float2 first = halves_of(score[i][0]), second = halves_of(score[i][1]);
+                    float out[4] = {first.x, first.y, second.x, second.y};
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const uint32_t tick = shared.lane_tick[(set * 4 + j) / GROUP];
+                        // causal + ring window of this lane: ticks in (tick - capacity, tick]
+                        const bool visible = t < count && tick != 0xffffffffu && token_tick <= tick && token_tick + capacity > tick;
+                        out[j] = visible ? out[j] * scale : -INFINITY;
+                    }
+                    *reinterpret_cast<float4 *>(shared.p + t * Form::P_STRIDE + set * 4) = make_float4(out[0], out[1], out[2], out[3]);
+                }
             }
         }
         __syncthreads();
         // ---- online softmax: warp w handles queries w, w+4, ...
         {
             const int warp = tid >> 5, lane_id = tid & 31;
+#pragma unroll
             for (int query = warp; query < Q; query += 4) {
-                float s0 = p_tile[query * TILE + lane_id], s1 = p_tile[query * TILE + 32 + lane_id];
-                float tile_max = warp_max(fmaxf(s0, s1));
-                float old_max = row_max[query];
-                float next_max = fmaxf(old_max, tile_max);
+                float *row = shared.p + query;
+                const float s0 = row[lane_id * Form::P_STRIDE], s1 = row[(32 + lane_id) * Form::P_STRIDE];
+                const float tile_max = warp_max(fmaxf(s0, s1));
+                const float old_max = shared.row_max[query];
+                const float next_max = fmaxf(old_max, tile_max);
                 float p0 = 0.0f, p1 = 0.0f, alpha = 1.0f;
                 if (next_max > -3.0e38f) {
                     alpha = expf(old_max - next_max);
                     p0 = s0 == -INFINITY ? 0.0f : expf(s0 - next_max);
                     p1 = s1 == -INFINITY ? 0.0f : expf(s1 - next_max);
                 }
-                float tile_sum = warp_sum(p0 + p1);
-                p_tile[query * TILE + lane_id] = p0;
-                p_tile[query * TILE + 32 + lane_id] = p1;
+                const float tile_sum = warp_sum(p0 + p1);
+                row[lane_id * Form::P_STRIDE] = p0;
+                row[(32 + lane_id) * Form::P_STRIDE] = p1;
+                __syncwarp();
                 if (lane_id == 0) {
-                    row_alpha[query] = alpha;
-                    row_sum[query] = row_sum[query] * alpha + tile_sum;
-                    row_max[query] = next_max;
+                    shared.row_alpha[query] = alpha;
+                    shared.row_sum[query] = shared.row_sum[query] * alpha + tile_sum;
+                    shared.row_max[query] = next_max;
                 }
             }
         }
         __syncthreads();
         // ---- P.V
+        if (value_active) {
+            const float *row = shared.p + value_set * VQ;
+            const uint16_t *values = shared.v + value_dim;
 #pragma unroll
-        for (int query = 0; query < Q; query++) {
-            float alpha = row_alpha[query];
+            for (int i = 0; i < VQ / 2; i++) {
+                const float a0 = shared.row_alpha[value_set * VQ + 2 * i], a1 = shared.row_alpha[value_set * VQ + 2 * i + 1];
 #pragma unroll
-            for (int d = 0; d < DPT; d++) acc[query][d] *= alpha;
-        }
-        if (tid < HD || DPT > 1) {
+                for (int d = 0; d < 2; d++) {
+                    const float2 sum = halves_of(acc[d][i]);
+                    acc[d][i] = pair_of(sum.x * a0, sum.y * a1);
+                }
+            }
+#pragma unroll 4
             for (int t = 0; t < count; t++) {
-                float vv[DPT];
+                const uint32_t word = *reinterpret_cast<const uint32_t *>(values + t * HD);
+                const float_pair v0 = pair_of(bf16_lo(word), bf16_lo(word)), v1 = pair_of(bf16_hi(word), bf16_hi(word));
 #pragma unroll
-                for (int d = 0; d < DPT; d++) vv[d] = (tid + d * 128 < HD) ? bf16_bits_to_f32(v_tile[t * HD + tid + d * 128]) : 0.0f;
-#pragma unroll
-                for (int query = 0; query < Q; query++) {
-                    float p = p_tile[query * TILE + t];
-#pragma unroll
-                    for (int d = 0; d < DPT; d++) acc[query][d] = fmaf(p, vv[d], acc[query][d]);
+                for (int i = 0; i < VQ / 2; i++) {
+                    const float_pair probabilities = *reinterpret_cast<const float_pair *>(row + t * Form::P_STRIDE + 2 * i);
+                    acc[0][i] = pair_fma(probabilities, v0, acc[0][i]);
+                    acc[1][i] = pair_fma(probabilities, v1, acc[1][i]);
                 }
             }
         }
     }
-    __syncthreads();
+    if (value_active) {
 #pragma unroll
-    for (int query = 0; query < Q; query++) {
-        if (lane_tick[query / GROUP] == 0xffffffffu) continue;
-        int lane = lane0 + query / GROUP;
-        float *out = scratch + ((static_cast<size_t>(lane) * q_heads + kv_head * GROUP + query % GROUP) * max_splits + split) * (HD + 2);
-#pragma unroll
-        for (int d = 0; d < DPT; d++)
-            if (tid + d * 128 < HD) out[tid + d * 128] = acc[query][d];
-        if (tid == 0) {
-            out[HD] = row_max[query];
-            out[HD + 1] = row_sum[query];
+        for (int i = 0; i < VQ; i++) {
+            const int query = value_set * VQ + i;
+            if (shared.lane_tick[query / GROUP] == 0xffffffffu) continue;
+            float *out = scratch + ((static_cast<size_t>(lane0 + query / GROUP) * q_heads + kv_head * GROUP + query % GROUP) * max_splits + split) * (HD + 2);
+            const float2 first = halves_of(acc[0][i / 2]), second = halves_of(acc[1][i / 2]);
+            *reinterpret_cast<float2 *>(out + value_dim) = (i & 1) ? make_float2(first.y, second.y) : make_float2(first.x, second.x);
         }
     }
-}
-
-template <int HD, int GROUP, int QL>
-__global__ void __launch_bounds__(128)
-attention_f32_kernel(const uint16_t *__restrict__ q, KvLayer kv, LaneTable lanes_meta, int lanes, int lanes_per_stream,
-                     int q_heads, float scale, int split_tokens, int max_splits, float *__restrict__ scratch, const AttentionBlock *__restrict__ ragged) {
-    extern __shared__ __align__(16) uint8_t smem_raw[];
-    grid_launch_dependents();
-    grid_dependency_wait();
-    attention_f32_body<HD, GROUP, QL>(q, kv, lanes_meta, lanes, lanes_per_stream, q_heads, scale, split_tokens, max_splits, scratch, ragged, blockIdx.x,
-                                      blockIdx.y, blockIdx.z, smem_raw, threadIdx.x);
-}
-
-// Log-sum-exp merge of the split partials of one (lane, q head) pair by one warp.
-__device__ __forceinline__ void attention_f32_merge_pair(const float *__restrict__ scratch, uint16_t *__restrict__ out, const KvLayer &kv,
-                                                     const LaneTable &lanes_meta, int pair, int lane_id, int q_heads, int head_width,
-                                                     int split_tokens, int max_splits) {
-    int lane = pair / q_heads;
-    int slot = lanes_meta.slot[lane];
-    if (slot < 0) return;
-    uint32_t tick = lanes_meta.position[lane];
-    uint32_t tokens = tick + 1u < kv.capacity ? tick + 1u : kv.capacity;
-    int splits = static_cast<int>((tokens + split_tokens - 1) / split_tokens);
-    if (splits > max_splits) splits = max_splits;
-    const float *base = scratch + static_cast<size_t>(pair) * max_splits * (head_width + 2);
-    auto read = [&](const float *address) { return *address; };
-    float maximum = -3.4028234663852886e38f;
-    for (int s = 0; s < splits; s++) maximum = fmaxf(maximum, read(base + static_cast<size_t>(s) * (head_width + 2) + head_width));
-    float denominator = 0.0f;
-    for (int s = 0; s < splits; s++) {
-        const float *part = base + static_cast<size_t>(s) * (head_width + 2);
-        denominator += read(part + head_width + 1) * expf(read(part + head_width) - maximum);
-    }
-    for (int d = lane_id; d < head_width; d += 32) {
-        float acc = 0.0f;
-        for (int s = 0; s < splits; s++) {
-            const float *part = base + static_cast<size_t>(s) * (head_width + 2);
-            acc += read(part + d) * expf(read(part + head_width) - maximum);
-        }
-        out[static_cast<size_t>(pair) * head_width + d] =
-            static_cast<uint16_t>(f32_to_bf16_bits(denominator == 0.0f ? 0.0f : acc / denominator));
+    if (tid < Q && shared.lane_tick[tid / GROUP] != 0xffffffffu) {
+        float *out = scratch + ((static_cast<size_t>(lane0 + tid / GROUP) * q_heads + kv_head * GROUP + tid % GROUP) * max_splits + split) * (HD + 2);
+        out[HD] = shared.row_max[tid];
+        out[HD + 1] = shared.row_sum[tid];
     }
 }
 
+// Log-sum-exp merge of the split partials of one (lane, q head) pair by one warp: thread s weighs split s, the weighted
+// partials are added split by split in order, as are the sums.  (Every thread weighing every split for each of its dims, one
+// load after the other: 9 us for 17 splits; this 5.)
 __global__ void attention_f32_merge_kernel(const float *__restrict__ scratch, uint16_t *__restrict__ out, KvLayer kv,
                                            LaneTable lanes_meta, int lanes, int q_heads, int head_width, int split_tokens,
                                            int max_splits) {
     grid_launch_dependents();
     grid_dependency_wait();
-    int pair = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int pair = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), thread = threadIdx.x & 31;
     if (pair >= lanes * q_heads) return;
-    attention_f32_merge_pair(scratch, out, kv, lanes_meta, pair, threadIdx.x & 31, q_heads, head_width, split_tokens, max_splits);
+    const int lane = pair / q_heads;
+    if (lanes_meta.slot[lane] < 0) return;
+    const uint32_t tick = lanes_meta.position[lane];
+    const uint32_t tokens = tick + 1u < kv.capacity ? tick + 1u : kv.capacity;
+    const int splits = min(static_cast<int>((tokens + split_tokens - 1) / split_tokens), max_splits), stride = head_width + 2;
+    const float *base = scratch + static_cast<size_t>(pair) * max_splits * stride;
+    float maximum = -3.4028234663852886e38f;
+    for (int s = thread; s < splits; s += 32) maximum = fmaxf(maximum, base[static_cast<size_t>(s) * stride + head_width]);
+    maximum = warp_max(maximum);
+    constexpr int DIMS = 4;  // heads of at most 128
+    float denominator = 0.0f, acc[DIMS] = {};
+    for (int first = 0; first < splits; first += 32) {
+        float weight = 0.0f, sum = 0.0f;
+        if (first + thread < splits) {
+            const float *state = base + static_cast<size_t>(first + thread) * stride + head_width;
+            weight = expf(state[0] - maximum);
+            sum = state[1];
+        }
+        const int count = min(32, splits - first);
+#pragma unroll 4
+        for (int s = 0; s < count; s++) {
+            const float w = __shfl_sync(0xffffffffu, weight, s);
+            const float *part = base + static_cast<size_t>(first + s) * stride;
+            denominator = fmaf(__shfl_sync(0xffffffffu, sum, s), w, denominator);
+#pragma unroll
+            for (int i = 0; i < DIMS; i++)
+                if (thread + 32 * i < head_width) acc[i] = fmaf(part[thread + 32 * i], w, acc[i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < DIMS; i++)
+        if (thread + 32 * i < head_width)
+            out[static_cast<size_t>(pair) * head_width + thread + 32 * i] = static_cast<uint16_t>(f32_to_bf16_bits(denominator == 0.0f ? 0.0f : acc[i] / denominator));
 }
 
 template <int HD, int GROUP, int QL>
 cudaError_t launch_f32(const AttentionArgs &a, cudaStream_t stream) {
     auto kernel = attention_f32_kernel<HD, GROUP, QL>;
-    constexpr size_t smem = attention_f32_smem<HD, GROUP, QL>();
+    constexpr size_t smem = sizeof(typename AttentionF32<HD, GROUP, QL>::Shared);
     cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (status != cudaSuccess) return status;
     const int groups = a.blocks != nullptr ? a.row_blocks : a.lanes / a.lanes_per_stream * ((a.lanes_per_stream + QL - 1) / QL);
