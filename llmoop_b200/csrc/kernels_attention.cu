@@ -680,10 +680,13 @@ cudaError_t launch_f32_of_width(const AttentionArgs &args, cudaStream_t stream) 
 }
 
 // Heads of at most 32 (tiny models, short contexts: latency, not bandwidth): one warp per (lane, q head), scalar f32; its
-// threads take every 32nd token with a softmax of their own and merge in the end.  (One thread per (lane, q head), the
-// form this replaced, took 32 us for a 30-token context; this takes 8.)
+// threads take every 32nd token with a softmax of their own and merge in the end.  HD: the head width where rows are whole
+// 16-byte words, else 0.  The rows of a token are requested together, and the merge halves the dims a thread holds with
+// every exchange.  (Element by element and five exchanges per dim: 7.6 us for a 50-token context; this 2.5.)
+template <int HD>
 __global__ void attention_small_kernel(const uint16_t *__restrict__ q, uint16_t *__restrict__ out, KvLayer kv,
                                        LaneTable lanes_meta, int lanes, int q_heads, float scale) {
+    constexpr int WIDTH = HD > 0 ? HD : 32;
     grid_launch_dependents();
     grid_dependency_wait();
     const int index = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), thread = threadIdx.x & 31;
@@ -691,48 +694,78 @@ __global__ void attention_small_kernel(const uint16_t *__restrict__ q, uint16_t 
     const int lane = index / q_heads, head = index % q_heads;
     const int slot = lanes_meta.slot[lane];
     if (slot < 0) return;
-    const int hd = kv.head_width;
+    const int hd = HD > 0 ? HD : kv.head_width;
     const int kv_head = head / (q_heads / kv.kv_heads);
     const uint32_t tick = lanes_meta.position[lane];
     const uint32_t capacity = kv.capacity;
     const uint32_t tokens = tick + 1u < capacity ? tick + 1u : capacity;
     const uint32_t first_tick = tick + 1u - tokens;
-    const uint16_t *qv = q + (static_cast<size_t>(lane) * q_heads + head) * hd;
-    float query[32], acc[32];
+    auto read_row = [&](const uint16_t *row, float (&values)[WIDTH]) {
+        if (HD > 0) {
+            uint4 words[WIDTH / 8];
 #pragma unroll
-    for (int d = 0; d < 32; d++) {
-        query[d] = d < hd ? bf16_bits_to_f32(qv[d]) : 0.0f;
-        acc[d] = 0.0f;
-    }
+            for (int i = 0; i < WIDTH / 8; i++) words[i] = reinterpret_cast<const uint4 *>(row)[i];
+#pragma unroll
+            for (int i = 0; i < WIDTH / 8; i++) {
+                const uint32_t four[4] = {words[i].x, words[i].y, words[i].z, words[i].w};
+#pragma unroll
+                for (int w = 0; w < 4; w++) {
+                    values[8 * i + 2 * w] = bf16_lo(four[w]);
+                    values[8 * i + 2 * w + 1] = bf16_hi(four[w]);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int d = 0; d < WIDTH; d++) values[d] = d < hd ? bf16_bits_to_f32(row[d]) : 0.0f;
+        }
+    };
+    float query[WIDTH], acc[WIDTH];
+    read_row(q + (static_cast<size_t>(lane) * q_heads + head) * hd, query);
+#pragma unroll
+    for (int d = 0; d < WIDTH; d++) acc[d] = 0.0f;
     float maximum = LOWEST, denominator = 0.0f;
     for (uint32_t i = thread; i < tokens; i += 32) {
-        const uint32_t ring = (first_tick + i) % capacity;
-        const uint16_t *kr = kv.pool + kv_token_offset(kv, slot, ring, kv_head, false);
-        const uint16_t *vr = kv.pool + kv_token_offset(kv, slot, ring, kv_head, true);
+        uint32_t ring = first_tick + i;
+        if (ring >= capacity) ring %= capacity;
+        const uint16_t *row = kv.pool + kv_token_offset(kv, slot, ring, kv_head, false);
+        float key[WIDTH], value[WIDTH];
+        read_row(row, key);
+        read_row(row + static_cast<size_t>(kv.kv_heads) * kv.page_tokens * hd, value);
         float dot = 0.0f;
 #pragma unroll
-        for (int d = 0; d < 32; d++)
-            if (d < hd) dot = fmaf(query[d], bf16_bits_to_f32(kr[d]), dot);
+        for (int d = 0; d < WIDTH; d++) dot = fmaf(query[d], key[d], dot);
         const float score = dot * scale, next_max = fmaxf(maximum, score);
         const float alpha = expf(maximum - next_max), beta = expf(score - next_max);
         denominator = denominator * alpha + beta;
         maximum = next_max;
 #pragma unroll
-        for (int d = 0; d < 32; d++)
-            if (d < hd) acc[d] = acc[d] * alpha + beta * bf16_bits_to_f32(vr[d]);
+        for (int d = 0; d < WIDTH; d++) acc[d] = acc[d] * alpha + beta * value[d];
     }
     const float whole_max = warp_max(maximum), weight = expf(maximum - whole_max);
     denominator = warp_sum(denominator * weight);
-    float own = 0.0f;  // thread d keeps dimension d
 #pragma unroll
-    for (int d = 0; d < 32; d++) {
-        if (d >= hd) break;
-        const float sum = warp_sum(acc[d] * weight);
-        if (thread == d) own = sum;
+    for (int d = 0; d < WIDTH; d++) acc[d] *= weight;
+    // the dims' sums over the warp: every exchange (distance 16, 8, ..) adds the partner's share of half of them
+    int dim = 0;
+#pragma unroll
+    for (int step = 0; step < 5; step++) {
+        const int distance = 16 >> step, live = WIDTH >> step;
+        if (live > 1) {
+            const bool upper = (thread & distance) != 0;
+#pragma unroll
+            for (int i = 0; i < live / 2; i++) {
+                const float keep = upper ? acc[live / 2 + i] : acc[i], send = upper ? acc[i] : acc[live / 2 + i];
+                acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, distance);
+            }
+            if (upper) dim += live / 2;
+        } else {
+            acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], distance);  // fewer dims than threads: several end up with the same one
+        }
     }
-    if (thread < hd)
-        out[(static_cast<size_t>(lane) * q_heads + head) * hd + thread] =
-            static_cast<uint16_t>(f32_to_bf16_bits(denominator == 0.0f ? 0.0f : own / denominator));
+    constexpr int SHARERS = 32 / WIDTH;
+    if (thread % SHARERS == 0 && dim < hd)
+        out[(static_cast<size_t>(lane) * q_heads + head) * hd + dim] =
+            static_cast<uint16_t>(f32_to_bf16_bits(denominator == 0.0f ? 0.0f : acc[0] / denominator));
 }
 
 // Log-sum-exp merge of the split partials; one warp per (lane, q head).
@@ -834,7 +867,9 @@ cudaError_t launch_attention(const uint16_t *q, uint16_t *out, const KvLayer &kv
     const bool wide = kv.head_width == 64 || kv.head_width == 128;
     if (!wide || (group != 1 && group != 2 && group != 4 && group != 8)) {
         if (kv.head_width > 32) return cudaErrorInvalidValue;
-        return launch_dependent(attention_small_kernel, dim3((lanes * q_heads + 3) / 4), dim3(128), 0, 1, stream, q, out, kv, lanes_meta, lanes, q_heads, scale);
+        auto kernel = kv.head_width == 32 ? attention_small_kernel<32> : kv.head_width == 16 ? attention_small_kernel<16>
+                    : kv.head_width == 8 ? attention_small_kernel<8> : attention_small_kernel<0>;
+        return launch_dependent(kernel, dim3((lanes * q_heads + 3) / 4), dim3(128), 0, 1, stream, q, out, kv, lanes_meta, lanes, q_heads, scale);
     }
     AttentionArgs args = {};
     args.q = q;
