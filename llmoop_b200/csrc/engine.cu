@@ -502,12 +502,8 @@ Engine::Engine(std::shared_ptr<MountedModel> model) : model_(std::move(model)) {
     const ModelPlan &plan = model_->plan();
     cuda_check(cudaSetDevice(options.device), "cudaSetDevice");
     cuda_check(cudaStreamCreateWithFlags(&cuda_stream_, cudaStreamNonBlocking), "cudaStreamCreate");
-    cuda_check(cudaEventCreate(&event_a_), "cudaEventCreate");
-    cuda_check(cudaEventCreate(&event_b_), "cudaEventCreate");
-    cuda_check(cudaEventCreate(&event_begin_), "cudaEventCreate");
     cuda_check(cudaEventCreate(&run_begin_), "cudaEventCreate");
     cuda_check(cudaEventCreate(&run_end_), "cudaEventCreate");
-    cuda_check(cudaEventCreate(&event_end_), "cudaEventCreate");
     const size_t lanes = options.max_lanes;
     const size_t frame = static_cast<size_t>(plan.hidden) * 2;
 
@@ -617,6 +613,7 @@ Engine::Engine(std::shared_ptr<MountedModel> model) : model_(std::move(model)) {
     staging_bytes_ = std::max<size_t>(size_t(1) << 20, lanes * 1024 + static_cast<size_t>(options.max_streams) * model_->pages_per_stream() * 8);
     cuda_check(cudaMallocHost(&staging_, staging_bytes_), "cudaMallocHost");
     cuda_check(cudaMallocHost(&host_records_, lanes * 64 * sizeof(uint32_t)), "cudaMallocHost");
+    cuda_check(cudaMallocHost(&host_cycle_, cycle_state_.bytes), "cudaMallocHost");
 
     kernel_error_ = device_alloc(sizeof(int));
     if (options.tp_size > 1) tp_partial_ = device_alloc(lanes * static_cast<size_t>(plan.hidden) * sizeof(float));
@@ -654,15 +651,12 @@ Engine::~Engine() {
         cudaFree(buffer->ptr);
     cudaFreeHost(staging_);
     cudaFreeHost(host_records_);
+    cudaFreeHost(host_cycle_);
     for (cudaEvent_t event : profile_events_) cudaEventDestroy(event);
     for (auto &entry : graphs_)
         if (entry.second.exec) cudaGraphExecDestroy(entry.second.exec);
-    cudaEventDestroy(event_a_);
-    cudaEventDestroy(event_b_);
-    cudaEventDestroy(event_begin_);
     cudaEventDestroy(run_begin_);
     cudaEventDestroy(run_end_);
-    cudaEventDestroy(event_end_);
     cudaStreamDestroy(cuda_stream_);
 }
 
@@ -1672,7 +1666,7 @@ int Engine::plan_splits(int lanes, int lanes_per_stream, uint64_t newest_tick) {
     return current_splits_ | (current_op_splits_ << 16);
 }
 
-// Runs `body` (stream-ordered launches only: no uploads, read-backs or synchronisation) directly the first time a
+// Runs `body` (stream-ordered work only, of the same addresses every time: no uploads, no synchronisation) directly the first time a
 // key is seen, then captures it into a CUDA graph and replays the graph from the third call on.
 void Engine::run_phase(const std::vector<int> &key, const std::function<void()> &body) {
     // Tensor-parallel engines replay graphs only for phases that contain no NCCL call: every forward of the phase
@@ -1931,10 +1925,6 @@ void Engine::emit(Stream &s, uint32_t token, uint64_t tick, const std::function<
 // replayed) - and the call fails, as the reference restores the state of a failed cycle
 // (placed_stream_processor/feedback_generation.rs:188-192).
 
-void Engine::backup_pending() {
-    cuda_check(cudaMemcpyAsync(pending_backup_.ptr, pending_hidden_.ptr, pending_hidden_.bytes, cudaMemcpyDeviceToDevice, cuda_stream_), "pending hidden backup");
-}
-
 void Engine::check_kernel_status(const uint32_t *status_word) {
     if (*status_word == 0) return;
     const int code = static_cast<int>(*status_word);
@@ -1967,25 +1957,28 @@ void Engine::run_single_ticks(std::vector<Stream *> &batch, const std::function<
     sync_block_tables();
     upload_lanes(positions, slots, 1);
     upload_tokens(tokens.data(), lanes);
-    if (plan.has_draft) backup_pending();
-    target_forward(lanes, any_emit);
-    if (plan.has_draft) {
-        check(launch_gather_rows(static_cast<const uint16_t *>(pending_hidden_.ptr), static_cast<const int32_t *>(lane_slots_.ptr),
-                                 static_cast<uint16_t *>(draft_hidden_in_.ptr), lanes, static_cast<int>(plan.hidden), cuda_stream_),
-              "gather pending hidden");
-        draft_forward(lanes, static_cast<const uint16_t *>(draft_hidden_in_.ptr), false);
-        check(launch_commit_hidden(static_cast<const uint16_t *>(normalized_.ptr), static_cast<const int32_t *>(lane_slots_.ptr),
-                                   static_cast<uint16_t *>(pending_hidden_.ptr), lanes, static_cast<int>(plan.hidden), cuda_stream_),
-              "commit target hidden");
-    }
-    if (any_emit) {
-        cuda_check(cudaMemcpyAsync(host_records_, records_.ptr, lanes * 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, cuda_stream_),
-                   "record readback");
-        counters_.d2h_bytes += lanes * 16;
-    }
+    const int splits = current_splits_ | (current_op_splits_ << 16);
     uint32_t *status_word = host_records_ + static_cast<size_t>(lanes) * 4;
-    cuda_check(cudaMemcpyAsync(status_word, kernel_error_.ptr, sizeof(int), cudaMemcpyDeviceToHost, cuda_stream_), "kernel status readback");
-    counters_.d2h_bytes += 4;
+    run_phase({1, lanes, 0, splits, stochastic_streams_ != 0 ? 1 : 0, stack_enabled_ ? 1 : 0, any_emit ? 1 : 0}, [&] {
+        if (plan.has_draft)
+            check(launch_begin_cycle(static_cast<const uint16_t *>(pending_hidden_.ptr), nullptr, nullptr, 0, static_cast<uint16_t *>(pending_backup_.ptr),
+                                     model_->options().max_streams, static_cast<int>(plan.hidden), nullptr, cuda_stream_),
+                  "pending hidden backup");
+        target_forward(lanes, any_emit);
+        if (plan.has_draft) {
+            check(launch_gather_rows(static_cast<const uint16_t *>(pending_hidden_.ptr), static_cast<const int32_t *>(lane_slots_.ptr),
+                                     static_cast<uint16_t *>(draft_hidden_in_.ptr), lanes, static_cast<int>(plan.hidden), cuda_stream_),
+                  "gather pending hidden");
+            draft_forward(lanes, static_cast<const uint16_t *>(draft_hidden_in_.ptr), false);
+            check(launch_commit_hidden(static_cast<const uint16_t *>(normalized_.ptr), static_cast<const int32_t *>(lane_slots_.ptr),
+                                       static_cast<uint16_t *>(pending_hidden_.ptr), lanes, static_cast<int>(plan.hidden), cuda_stream_),
+                  "commit target hidden");
+        }
+        if (any_emit)
+            cuda_check(cudaMemcpyAsync(host_records_, records_.ptr, lanes * 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, cuda_stream_), "record readback");
+        cuda_check(cudaMemcpyAsync(status_word, kernel_error_.ptr, sizeof(int), cudaMemcpyDeviceToHost, cuda_stream_), "kernel status readback");
+    });
+    counters_.d2h_bytes += (any_emit ? lanes * 16 : 0) + 4;
     synchronize("tick synchronize");
     check_kernel_status(status_word);
     for (int i = 0; i < lanes; i++) {
@@ -2057,70 +2050,65 @@ void Engine::run_speculative_cycles(std::vector<Stream *> &batch, const std::vec
         }
     }
     sync_block_tables();
-    upload(base, staging.data(), upload_words * sizeof(uint32_t), "cycle state upload");
+    std::memcpy(host_cycle_, staging.data(), upload_words * sizeof(uint32_t));  // the last cycle's copy is done: every cycle ends with a synchronisation
+    counters_.h2d_bytes += upload_words * sizeof(uint32_t);
     const int splits = plan_splits(lanes, 1, newest_tick);
 
-    backup_pending();
-    cuda_check(cudaEventRecord(event_begin_, cuda_stream_), "event record");
-    // ---- draft loop: `drafts` serial steps over `streams` lanes
+    // The whole cycle is one graph with its two copies; its times are stamped by kernels that run anyway.  A graph launch,
+    // a copy or an event between two graphs left the device idle for 5 to 20 us each.
+    const size_t row_words = 4 + 2 * width, mark_offset = (upload_words + streams * row_words + 1) & ~size_t(1);
+    unsigned long long *marks = reinterpret_cast<unsigned long long *>(base + mark_offset);
+    const size_t result_words = mark_offset - upload_words + CYCLE_MARKS * 2;
     run_phase({0, streams, drafts, splits, stochastic_streams_ != 0 ? 1 : 0, stack_enabled_ ? 1 : 0}, [&] {
+        cuda_check(cudaMemcpyAsync(base, host_cycle_, upload_words * sizeof(uint32_t), cudaMemcpyHostToDevice, cuda_stream_), "cycle state upload");
+        check(launch_begin_cycle(static_cast<const uint16_t *>(pending_hidden_.ptr), stream_slots, static_cast<uint16_t *>(draft_hidden_in_.ptr),
+                                 drafts > 0 ? streams : 0, static_cast<uint16_t *>(pending_backup_.ptr), model_->options().max_streams,
+                                 static_cast<int>(plan.hidden), marks, cuda_stream_),
+              "pending hidden");
+        // ---- draft loop: `drafts` serial steps over `streams` lanes
         for (int j = 0; j < drafts; j++) {
             current_lanes_ = LaneTable{draft_positions + static_cast<size_t>(j) * streams, stream_slots};
             current_tokens_ = draft_tokens;
             current_width_ = 1;
             if (j == 0) {
-                check(launch_gather_rows(static_cast<const uint16_t *>(pending_hidden_.ptr), stream_slots,
-                                         static_cast<uint16_t *>(draft_hidden_in_.ptr), streams, static_cast<int>(plan.hidden), cuda_stream_),
-                      "gather pending hidden");
                 draft_forward(streams, static_cast<const uint16_t *>(draft_hidden_in_.ptr), true);
             } else {
                 draft_forward(streams, static_cast<const uint16_t *>(draft_normalized_.ptr), true);
             }
-            check(launch_draft_select(static_cast<const uint32_t *>(records_.ptr), forced, j, streams, drafts, draft_tokens, verify_tokens,
+            check(launch_draft_select(static_cast<const uint32_t *>(records_.ptr), forced, j, streams, drafts, draft_tokens, verify_tokens, marks,
                                       cuda_stream_),
                   "draft select");
         }
-    });
-    cuda_check(cudaEventRecord(event_a_, cuda_stream_), "event record");
 
-    // ---- verify: all candidates of all streams in one batch of lanes
-    run_phase({1, streams, drafts, splits, stochastic_streams_ != 0 ? 1 : 0, stack_enabled_ ? 1 : 0}, [&] {
+        // ---- verify: all candidates of all streams in one batch of lanes
         current_lanes_ = LaneTable{verify_positions, verify_slots};
         current_tokens_ = verify_tokens;
         current_width_ = width;
         target_forward(lanes, true);
-    });
-    cuda_check(cudaEventRecord(event_b_, cuda_stream_), "event record");
 
-    // ---- accept on the device, then the draft catch-up over the same lanes: state steps for the verify inputs
-    // with the target's hidden states.  Lanes beyond the committed prefix write slots that the next cycle
-    // overwrites before reading (like the draft loop's own tentative writes in the reference).
-    const size_t row_words = 4 + 2 * width;
-    run_phase({2, streams, drafts, splits, stochastic_streams_ != 0 ? 1 : 0, stack_enabled_ ? 1 : 0}, [&] {
-        current_lanes_ = LaneTable{verify_positions, verify_slots};
-        current_tokens_ = verify_tokens;
-        current_width_ = width;
+        // ---- accept on the device, then the draft catch-up over the same lanes: state steps for the verify inputs
+        // with the target's hidden states.  Lanes beyond the committed prefix write slots that the next cycle
+        // overwrites before reading (like the draft loop's own tentative writes in the reference).
         check(launch_shift_hidden(static_cast<const uint16_t *>(pending_hidden_.ptr), stream_slots, static_cast<const uint16_t *>(normalized_.ptr),
-                                  static_cast<uint16_t *>(draft_hidden_in_.ptr), streams, width, static_cast<int>(plan.hidden), cuda_stream_),
+                                  static_cast<uint16_t *>(draft_hidden_in_.ptr), streams, width, static_cast<int>(plan.hidden), marks, cuda_stream_),
               "catch-up hidden");
         check(launch_accept(verify_tokens, static_cast<const uint32_t *>(records_.ptr), stop_tokens, stop_counts, own_drafts, MAX_STOP_TOKENS, streams, drafts,
                             accept_rows, static_cast<const uint16_t *>(normalized_.ptr), static_cast<uint16_t *>(pending_hidden_.ptr), stream_slots,
                             static_cast<int>(plan.hidden), cuda_stream_),
               "accept");
         draft_forward(lanes, static_cast<const uint16_t *>(draft_hidden_in_.ptr), false);
+        check(launch_finish_cycle(marks, static_cast<const int *>(kernel_error_.ptr), cuda_stream_), "cycle status");
+        cuda_check(cudaMemcpyAsync(host_records_, accept_rows, result_words * sizeof(uint32_t), cudaMemcpyDeviceToHost, cuda_stream_), "accept readback");
     });
-    cuda_check(cudaEventRecord(event_end_, cuda_stream_), "event record");
-    cuda_check(cudaMemcpyAsync(host_records_, accept_rows, streams * row_words * sizeof(uint32_t), cudaMemcpyDeviceToHost, cuda_stream_),
-               "accept readback");
-    uint32_t *status_word = host_records_ + static_cast<size_t>(streams) * row_words;
-    cuda_check(cudaMemcpyAsync(status_word, kernel_error_.ptr, sizeof(int), cudaMemcpyDeviceToHost, cuda_stream_), "kernel status readback");
-    counters_.d2h_bytes += streams * row_words * 4 + 4;
+    counters_.d2h_bytes += result_words * sizeof(uint32_t);
     synchronize("cycle synchronize");
-    check_kernel_status(status_word);  // nothing of a failed cycle is emitted
-    float verify_ms = 0.0f, draft_ms = 0.0f, catch_up_ms = 0.0f;
-    cuda_check(cudaEventElapsedTime(&verify_ms, event_a_, event_b_), "event elapsed");
-    cuda_check(cudaEventElapsedTime(&draft_ms, event_begin_, event_a_), "event elapsed");
-    cuda_check(cudaEventElapsedTime(&catch_up_ms, event_b_, event_end_), "event elapsed");
+    unsigned long long times[CYCLE_MARKS];
+    std::memcpy(times, host_records_ + (mark_offset - upload_words), sizeof(times));
+    const uint32_t status_word = static_cast<uint32_t>(times[CYCLE_STATUS]);
+    check_kernel_status(&status_word);  // nothing of a failed cycle is emitted
+    if (drafts == 0) times[CYCLE_DRAFTED] = times[CYCLE_BEGIN];
+    const float verify_ms = static_cast<float>(times[CYCLE_VERIFIED] - times[CYCLE_DRAFTED]) * 1e-6f, draft_ms = static_cast<float>(times[CYCLE_DRAFTED] - times[CYCLE_BEGIN]) * 1e-6f,
+                catch_up_ms = static_cast<float>(times[CYCLE_END] - times[CYCLE_VERIFIED]) * 1e-6f;
     report.verify_ms_sum += verify_ms;
     report.verify_steps++;
     uint64_t kv_bytes = 0;

@@ -357,7 +357,7 @@ private:
     std::vector<PageCopy> page_copies_;  // asked for, not yet enqueued
     DeviceBuffer page_copies_device_;
     cudaStream_t cuda_stream_ = nullptr;
-    cudaEvent_t event_a_ = nullptr, event_b_ = nullptr, event_begin_ = nullptr, event_end_ = nullptr, run_begin_ = nullptr, run_end_ = nullptr;
+    cudaEvent_t run_begin_ = nullptr, run_end_ = nullptr;
 
     // workspaces
     std::map<std::string, DeviceBuffer> signals_;
@@ -393,7 +393,6 @@ private:
     bool run_stack(const StackPlan &stack, int lanes, void *hidden);
     void project_and_sample(const uint16_t *normalized, const std::string &projection_tensor, float scale, int lanes, const int32_t *slots,
                             const uint32_t *ticks, const char *what);
-    void backup_pending();
     void check_kernel_status(const uint32_t *status_word);  // throws (after restoring the pending hidden states) when a kernel reported an error
     DeviceBuffer cycle_state_;              // device-side per-batch cycle arrays (see engine.cu)
     // Pinned staging arena for host->device uploads: every upload between two host synchronisations gets its
@@ -401,6 +400,7 @@ private:
     uint8_t *staging_ = nullptr;
     size_t staging_bytes_ = 0, staging_used_ = 0;
     uint32_t *host_records_ = nullptr;      // pinned readback area
+    uint32_t *host_cycle_ = nullptr;        // pinned: what a speculative cycle starts from, copied by its graph
     int split_tokens_ = 256, max_splits_ = 1;
     int prefill_chunk_ = 64;
     bool use_graphs_ = true, log_cycles_ = false;

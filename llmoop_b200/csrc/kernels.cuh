@@ -291,11 +291,16 @@ cudaError_t launch_round_add(const float *sums, const uint16_t *residual, uint16
 
 // ---- glue of the speculative cycle (all tiny) ----
 // dst[i] = src[index[i]] for rows of `width` bf16.
+// Times (nanoseconds, device clock) and the status of a speculative cycle.
+enum CycleMark { CYCLE_BEGIN, CYCLE_DRAFTED, CYCLE_VERIFIED, CYCLE_END, CYCLE_STATUS, CYCLE_MARKS };
+cudaError_t launch_begin_cycle(const uint16_t *pending, const int32_t *slots, uint16_t *gathered, int rows, uint16_t *backup, int max_streams, int hidden,
+                               unsigned long long *marks, cudaStream_t stream);
+cudaError_t launch_finish_cycle(unsigned long long *marks, const int *error_word, cudaStream_t stream);
 cudaError_t launch_gather_rows(const uint16_t *src, const int32_t *index, uint16_t *dst, int rows, int width,
                                cudaStream_t stream);
 // Hidden inputs of the draft catch-up: lane (s, 0) takes pending[slot[s]], lane (s, i>0) takes normalized (s, i-1).
 cudaError_t launch_shift_hidden(const uint16_t *pending, const int32_t *slots, const uint16_t *normalized,
-                                uint16_t *dst, int streams, int lanes_per_stream, int hidden, cudaStream_t stream);
+                                uint16_t *dst, int streams, int lanes_per_stream, int hidden, unsigned long long *marks, cudaStream_t stream);
 // The same for lanes of any number per stream (neighbouring lanes of one slot are one stream's), and the way back: the
 // normalised frame of every stream's last lane becomes its pending hidden state.
 cudaError_t launch_shift_hidden_lanes(const uint16_t *pending, const int32_t *slots, const uint16_t *normalized, uint16_t *dst, int lanes, int hidden,
@@ -304,7 +309,7 @@ cudaError_t launch_commit_hidden(const uint16_t *normalized, const int32_t *slot
 // After draft step `step`: token = forced[s][step] unless it is 0xffffffff, else the sampled record; written to
 // next_tokens[s] and verify_tokens[s][step + 1].
 cudaError_t launch_draft_select(const uint32_t *records, const uint32_t *forced, int step, int streams, int drafts,
-                                uint32_t *next_tokens, uint32_t *verify_tokens, cudaStream_t stream);
+                                uint32_t *next_tokens, uint32_t *verify_tokens, unsigned long long *marks, cudaStream_t stream);
 // Longest-matching-prefix acceptance + stop truncation (speculative_decode.rs:54-105) per stream, then
 // pending[slot[s]] = normalized lane (s, committed-1).  out row = {accepted, committed, emitted_count, 0,
 // emitted[drafts+1], targets[drafts+1]}.  own_drafts[s] <= drafts: how many of the drafts count for the stream.

@@ -8,6 +8,12 @@
 
 namespace nerve {
 
+__device__ __forceinline__ unsigned long long global_time() {
+    unsigned long long now;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+    return now;
+}
+
 __global__ void gather_rows_kernel(const uint32_t *__restrict__ src, const int32_t *__restrict__ index,
                                    uint32_t *__restrict__ dst, int words) {
     grid_launch_dependents();
@@ -25,12 +31,44 @@ cudaError_t launch_gather_rows(const uint16_t *src, const int32_t *index, uint16
     return launch_dependent(gather_rows_kernel, dim3(rows), dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(src), index, reinterpret_cast<uint32_t *>(dst), width / 2);
 }
 
+// What a cycle starts with, in one launch: the batch's rows of `pending` gathered, all of `pending` saved (blocks behind the
+// gathered rows, one per slot), the time.
+__global__ void begin_cycle_kernel(const uint32_t *__restrict__ pending, const int32_t *__restrict__ slots, uint32_t *__restrict__ gathered, int rows,
+                                   uint32_t *__restrict__ backup, int words, unsigned long long *marks) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int block = blockIdx.x;
+    if (block == 0 && threadIdx.x == 0 && marks != nullptr) marks[CYCLE_BEGIN] = global_time();
+    const int source = block < rows ? slots[block] : block - rows;
+    if (source < 0) return;
+    const uint32_t *from = pending + static_cast<size_t>(source) * words;
+    uint32_t *to = block < rows ? gathered + static_cast<size_t>(block) * words : backup + static_cast<size_t>(source) * words;
+    for (int word = threadIdx.x; word < words; word += blockDim.x) to[word] = from[word];
+}
+cudaError_t launch_begin_cycle(const uint16_t *pending, const int32_t *slots, uint16_t *gathered, int rows, uint16_t *backup, int max_streams, int hidden,
+                               unsigned long long *marks, cudaStream_t stream) {
+    return launch_dependent(begin_cycle_kernel, dim3(rows + max_streams), dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(pending), slots,
+                            reinterpret_cast<uint32_t *>(gathered), rows, reinterpret_cast<uint32_t *>(backup), hidden / 2, marks);
+}
+
+// ... and ends with: the time, and the error word next to the results, so that one copy brings all of it to the host.
+__global__ void finish_cycle_kernel(unsigned long long *marks, const int *error_word) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    marks[CYCLE_END] = global_time();
+    marks[CYCLE_STATUS] = static_cast<unsigned long long>(static_cast<unsigned int>(*error_word));
+}
+cudaError_t launch_finish_cycle(unsigned long long *marks, const int *error_word, cudaStream_t stream) {
+    return launch_dependent(finish_cycle_kernel, dim3(1), dim3(1), 0, 1, stream, marks, error_word);
+}
+
 __global__ void shift_hidden_kernel(const uint32_t *__restrict__ pending, const int32_t *__restrict__ slots,
                                     const uint32_t *__restrict__ normalized, uint32_t *__restrict__ dst,
-                                    int lanes_per_stream, int words) {
+                                    int lanes_per_stream, int words, unsigned long long *marks) {
     grid_launch_dependents();
     grid_dependency_wait();
     int lane = blockIdx.x;
+    if (lane == 0 && threadIdx.x == 0) marks[CYCLE_VERIFIED] = global_time();
     int s = lane / lanes_per_stream, i = lane % lanes_per_stream;
     const uint32_t *source = i == 0 ? pending + static_cast<size_t>(slots[s]) * words
                                     : normalized + static_cast<size_t>(lane - 1) * words;
@@ -38,9 +76,9 @@ __global__ void shift_hidden_kernel(const uint32_t *__restrict__ pending, const 
 }
 
 cudaError_t launch_shift_hidden(const uint16_t *pending, const int32_t *slots, const uint16_t *normalized,
-                                uint16_t *dst, int streams, int lanes_per_stream, int hidden, cudaStream_t stream) {
+                                uint16_t *dst, int streams, int lanes_per_stream, int hidden, unsigned long long *marks, cudaStream_t stream) {
     if (streams <= 0) return cudaSuccess;
-    return launch_dependent(shift_hidden_kernel, dim3(streams * lanes_per_stream), dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(pending), slots, reinterpret_cast<const uint32_t *>(normalized), reinterpret_cast<uint32_t *>(dst), lanes_per_stream, hidden / 2);
+    return launch_dependent(shift_hidden_kernel, dim3(streams * lanes_per_stream), dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(pending), slots, reinterpret_cast<const uint32_t *>(normalized), reinterpret_cast<uint32_t *>(dst), lanes_per_stream, hidden / 2, marks);
 }
 
 // Prefill batches: the lanes of a stream are neighbours, a lane whose neighbour has another slot is its stream's first or last.
@@ -76,10 +114,11 @@ cudaError_t launch_commit_hidden(const uint16_t *normalized, const int32_t *slot
 
 __global__ void draft_select_kernel(const uint32_t *__restrict__ records, const uint32_t *__restrict__ forced, int step,
                                     int streams, int drafts, uint32_t *__restrict__ next_tokens,
-                                    uint32_t *__restrict__ verify_tokens) {
+                                    uint32_t *__restrict__ verify_tokens, unsigned long long *marks) {
     grid_launch_dependents();
     grid_dependency_wait();
     int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s == 0) marks[CYCLE_DRAFTED] = global_time();  // the last step's stays
     if (s >= streams) return;
     uint32_t token = records[static_cast<size_t>(s) * 4];
     if (forced != nullptr) {
@@ -91,9 +130,9 @@ __global__ void draft_select_kernel(const uint32_t *__restrict__ records, const 
 }
 
 cudaError_t launch_draft_select(const uint32_t *records, const uint32_t *forced, int step, int streams, int drafts,
-                                uint32_t *next_tokens, uint32_t *verify_tokens, cudaStream_t stream) {
+                                uint32_t *next_tokens, uint32_t *verify_tokens, unsigned long long *marks, cudaStream_t stream) {
     if (streams <= 0) return cudaSuccess;
-    return launch_dependent(draft_select_kernel, dim3((streams + 63) / 64), dim3(64), 0, 1, stream, records, forced, step, streams, drafts, next_tokens, verify_tokens);
+    return launch_dependent(draft_select_kernel, dim3((streams + 63) / 64), dim3(64), 0, 1, stream, records, forced, step, streams, drafts, next_tokens, verify_tokens, marks);
 }
 
 __global__ void accept_kernel(const uint32_t *__restrict__ verify_tokens, const uint32_t *__restrict__ target_records,
