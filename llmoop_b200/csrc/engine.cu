@@ -1401,6 +1401,45 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
                 index = last;
                 break;
             }
+            {
+                // matrices that share their input (q, k, v: branches of one node, or neighbours) in one launch, where a form
+                // of several matrices exists: FP8, and bf16 in scalar f32
+                auto joins = [&](const OpSpec &other) {
+                    if (other.kind != OpKind::Linear || other.tp_partial || other.inputs != op.inputs || other.prequantized_input != op.prequantized_input) return false;
+                    for (const WeightRef &w : other.weights) {
+                        if (w.storage != op.weights[0].storage || w.k != op.weights[0].k) return false;
+                        if (w.storage == TensorStorage::BF16) {
+                            if (!linear_bf16_is_scalar(lanes, static_cast<int>(w.n), static_cast<int>(w.k), bf16_form(lanes)) ||
+                                (lanes <= 8 && streaming_projection_ && model_->projection_table(w.tensor) != nullptr))
+                                return false;
+                        } else if (w.storage != TensorStorage::FP8_BLOCK || !op.prequantized_input) {
+                            return false;
+                        }
+                    }
+                    return true;
+                };
+                LinearBranches branches;
+                size_t last = index;
+                while (last < plan.ops.size() && branches.count + plan.ops[last].weights.size() <= 3 && joins(plan.ops[last])) {
+                    for (size_t branch = 0; branch < plan.ops[last].weights.size(); branch++) {
+                        const WeightRef &w = plan.ops[last].weights[branch];
+                        branches.add(weight(w.tensor), w.storage == TensorStorage::FP8_BLOCK ? static_cast<const uint16_t *>(weight(w.scale)) : nullptr,
+                                     ptr(plan.ops[last].outputs[branch]), static_cast<int>(w.n));
+                    }
+                    last++;
+                }
+                if (branches.count > 1) {
+                    const int k = static_cast<int>(op.weights[0].k);
+                    if (op.weights[0].storage == TensorStorage::FP8_BLOCK)
+                        check(launch_linear_fp8_multi(static_cast<const uint8_t *>(ptr(op.inputs[0])), static_cast<const float *>(ptr(op.inputs[1])), branches, nullptr,
+                                                      lanes, k, EPILOGUE_BF16, st),
+                              "linear_fp8");
+                    else
+                        check(launch_linear_bf16_scalar(u16(op.inputs[0]), branches, nullptr, lanes, k, EPILOGUE_BF16, 1.0f, st), "linear_bf16");
+                    index = last - 1;
+                    break;
+                }
+            }
             for (size_t branch = 0; branch < op.weights.size(); branch++) {
                 const WeightRef &w = op.weights[branch];
                 if (w.storage == TensorStorage::BF16) {

@@ -67,6 +67,26 @@ enum LinearEpilogue {
 // y[m][n] = sum_k x[m][k] * W[n][k], bf16 weights.  The form fixes the order of additions: by the number of lanes, or the
 // caller's choice (tensor cores where K allows).
 enum LinearForm { LINEAR_AUTO, LINEAR_SCALAR, LINEAR_TENSOR };
+bool linear_bf16_is_scalar(int lanes, int n, int k, LinearForm form);
+// Up to three matrices that share their input (q, k, v) in one launch.
+struct LinearBranches {
+    int count = 0;
+    const void *w[3] = {};
+    const uint16_t *scale[3] = {};  // FP8: block scales
+    void *y[3] = {};
+    int n[3] = {};
+    void add(const void *weights, const uint16_t *scales, void *out, int rows) {
+        w[count] = weights;
+        scale[count] = scales;
+        y[count] = out;
+        n[count++] = rows;
+    }
+};
+// bf16, eight lanes or fewer at a time in scalar f32 (the form launch_linear_bf16 takes for LINEAR_SCALAR or up to eight lanes).
+cudaError_t launch_linear_bf16_scalar(const uint16_t *x, const LinearBranches &branches, const uint16_t *residual, int lanes, int k, int epilogue, float scale,
+                                      cudaStream_t stream);
+cudaError_t launch_linear_fp8_multi(const uint8_t *xq, const float *xscale, const LinearBranches &branches, const uint16_t *residual, int lanes, int k,
+                                    int epilogue, cudaStream_t stream);
 cudaError_t launch_linear_bf16(const uint16_t *x, const uint16_t *w, void *y, const uint16_t *residual, int lanes,
                                int n, int k, int epilogue, float scale, cudaStream_t stream, int *error_flag = nullptr, LinearForm form = LINEAR_AUTO);
 // y = bf16( silu_bf16(bf16(x.Wg)) * bf16(x.Wu) )

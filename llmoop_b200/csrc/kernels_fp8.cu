@@ -202,34 +202,38 @@ __device__ __forceinline__ void by_count(int count, Two two, Four four, Eight ei
 struct Fp8LinearArgs {
     const uint8_t *xq;
     const float *xscale;
-    const uint8_t *w[2];  // a SiLU pair: gate, up
-    const uint16_t *wscale[2];
-    uint16_t *y;
+    const uint8_t *w[3];  // a SiLU pair: gate, up; else matrices that share the input
+    const uint16_t *wscale[3];
+    uint16_t *y[3];
+    int n[3];
+    int first[4];  // matrix b owns the row tiles first[b] .. first[b + 1] - 1
     const uint16_t *residual;
-    int lanes, n, k, epilogue;
+    int lanes, k, epilogue;
     int passes;  // a CTA covers 32 or 64 rows (1 or 2)
 };
 
 template <int M>
 __device__ __forceinline__ void fp8_linear_tile(const Fp8LinearArgs &a, int m0, int count, float *smem) {
     const int warp = threadIdx.x >> 5, thread = threadIdx.x & 31, blocks = a.k >> 7;
+    const int tile = blockIdx.x, matrix = tile < a.first[1] ? 0 : tile < a.first[2] ? 1 : 2, rows = a.n[matrix];
+    const uint8_t *const w = a.w[matrix];
     auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, a.k, first, n, count, smem, [&](int m) { return m0 + m; }); };
     const int warps = 32 * a.passes / RowSums<M>::ROWS;  // with rows to do in a pass
     for (int pass = 0; pass < (warps > FP8_WARPS ? 2 : 1); pass++) {
-        const int row0 = blockIdx.x * 32 * a.passes + (pass * FP8_WARPS + warp) * RowSums<M>::ROWS;
+        const int row0 = (tile - a.first[matrix]) * 32 * a.passes + (pass * FP8_WARPS + warp) * RowSums<M>::ROWS;
         RowSums<M> sums;
-        const uint16_t *scale_row = a.wscale[0] + static_cast<size_t>(min(row0, a.n - 1) >> 7) * blocks;  // eight rows lie in one block of 128
-        sums.run([&](int r) { return a.w[0] + static_cast<size_t>(min(row0 + r, a.n - 1)) * a.k; }, scale_row, scale_row, blocks, smem, pass > 0, stage);
+        const uint16_t *scale_row = a.wscale[matrix] + static_cast<size_t>(min(row0, rows - 1) >> 7) * blocks;  // eight rows lie in one block of 128
+        sums.run([&](int r) { return w + static_cast<size_t>(min(row0 + r, rows - 1)) * a.k; }, scale_row, scale_row, blocks, smem, pass > 0, stage);
         if (RowSums<M>::VALUES < 32 && (thread & 1) != 0) continue;
 #pragma unroll
         for (int i = 0; i < RowSums<M>::PER_THREAD; i++) {
             const int output = RowSums<M>::index(thread, i), row = row0 + output / M, m = output % M;
-            if (row >= a.n || m >= count || warp >= warps) continue;
-            const size_t out = static_cast<size_t>(m0 + m) * a.n + row;
+            if (row >= rows || m >= count || warp >= warps) continue;
+            const size_t out = static_cast<size_t>(m0 + m) * rows + row;
             float sum = sums.sums[i];
             if (a.epilogue == EPILOGUE_RESIDUAL_F32) sum = bf16_bits_to_f32(a.residual[out]) + sum;
             else if (a.epilogue == EPILOGUE_RESIDUAL_ROUNDED) sum = round_bf16(sum) + bf16_bits_to_f32(a.residual[out]);
-            a.y[out] = static_cast<uint16_t>(f32_to_bf16_bits(sum));
+            a.y[matrix][out] = static_cast<uint16_t>(f32_to_bf16_bits(sum));
         }
     }
 }
@@ -268,13 +272,13 @@ __device__ __forceinline__ void fp8_silu_tile(const Fp8LinearArgs &a, int m0, in
     constexpr int HALF = RowSums<M>::ROWS / 2;
     const int warps = 32 * a.passes / RowSums<M>::ROWS;
     for (int pass = 0; pass < (warps > FP8_WARPS ? 2 : 1); pass++) {
-        const int row0 = blockIdx.x * 16 * a.passes + (pass * FP8_WARPS + warp) * HALF, first = min(row0, a.n - 1);
+        const int row0 = blockIdx.x * 16 * a.passes + (pass * FP8_WARPS + warp) * HALF, first = min(row0, a.n[0] - 1);
         RowSums<M> sums;
-        sums.run([&](int r) { return a.w[r / HALF] + static_cast<size_t>(min(row0 + r % HALF, a.n - 1)) * a.k; }, a.wscale[0] + static_cast<size_t>(first >> 7) * blocks,
+        sums.run([&](int r) { return a.w[r / HALF] + static_cast<size_t>(min(row0 + r % HALF, a.n[0] - 1)) * a.k; }, a.wscale[0] + static_cast<size_t>(first >> 7) * blocks,
                  a.wscale[1] + static_cast<size_t>(first >> 7) * blocks, blocks, smem, pass > 0, stage);
         silu_outputs<M>(sums, [&](int r, int m, float gate, float up) {
-            if (row0 + r >= a.n || m >= count || warp >= warps) return;
-            a.y[static_cast<size_t>(m0 + m) * a.n + row0 + r] = static_cast<uint16_t>(f32_to_bf16_bits(rounded_silu(gate) * up));
+            if (row0 + r >= a.n[0] || m >= count || warp >= warps) return;
+            a.y[0][static_cast<size_t>(m0 + m) * a.n[0] + row0 + r] = static_cast<uint16_t>(f32_to_bf16_bits(rounded_silu(gate) * up));
         });
     }
 }
@@ -435,11 +439,38 @@ int fp8_passes(int row_tiles, int lanes) { return row_tiles * ((lanes + TILE_LAN
 cudaError_t launch_linear_fp8(const uint8_t *xq, const float *xscale, const uint8_t *w, const uint16_t *wscale,
                               uint16_t *y, const uint16_t *residual, int lanes, int n, int k, int epilogue,
                               cudaStream_t stream) {
+    LinearBranches branches;
+    branches.add(w, wscale, y, n);
+    return launch_linear_fp8_multi(xq, xscale, branches, residual, lanes, k, epilogue, stream);
+}
+
+cudaError_t launch_linear_fp8_multi(const uint8_t *xq, const float *xscale, const LinearBranches &branches, const uint16_t *residual, int lanes, int k,
+                                    int epilogue, cudaStream_t stream) {
     if (lanes <= 0) return cudaSuccess;
     if (k % 128 != 0) return cudaErrorInvalidValue;
-    const int passes = fp8_passes((n + 63) / 64, lanes), rows = 32 * passes;
-    const Fp8LinearArgs args{xq, xscale, {w, nullptr}, {wscale, nullptr}, y, residual, lanes, n, k, epilogue, passes};
-    return launch_rows(linear_fp8_kernel, dim3((n + rows - 1) / rows, (lanes + TILE_LANES - 1) / TILE_LANES), lanes, stream, args);
+    Fp8LinearArgs args = {};
+    int tiles = 0;
+    for (int b = 0; b < branches.count; b++) tiles += (branches.n[b] + 63) / 64;
+    args.passes = fp8_passes(tiles, lanes);
+    tiles = 0;
+    for (int b = 0; b < 3; b++) {
+        args.first[b] = tiles;
+        if (b >= branches.count) continue;
+        args.w[b] = static_cast<const uint8_t *>(branches.w[b]);
+        args.wscale[b] = branches.scale[b];
+        args.y[b] = static_cast<uint16_t *>(branches.y[b]);
+        args.n[b] = branches.n[b];
+        tiles += (branches.n[b] + 32 * args.passes - 1) / (32 * args.passes);
+    }
+    args.first[3] = tiles;
+    for (int b = branches.count; b < 3; b++) args.first[b] = tiles;
+    args.xq = xq;
+    args.xscale = xscale;
+    args.residual = residual;
+    args.lanes = lanes;
+    args.k = k;
+    args.epilogue = epilogue;
+    return launch_rows(linear_fp8_kernel, dim3(tiles, (lanes + TILE_LANES - 1) / TILE_LANES), lanes, stream, args);
 }
 
 cudaError_t launch_linear_silu_multiply_fp8(const uint8_t *xq, const float *xscale, const uint8_t *wg,
@@ -448,7 +479,19 @@ cudaError_t launch_linear_silu_multiply_fp8(const uint8_t *xq, const float *xsca
     if (lanes <= 0) return cudaSuccess;
     if (k % 128 != 0) return cudaErrorInvalidValue;
     const int passes = fp8_passes((n + 31) / 32, lanes), rows = 16 * passes;
-    const Fp8LinearArgs args{xq, xscale, {wg, wu}, {wg_scale, wu_scale}, y, nullptr, lanes, n, k, EPILOGUE_BF16, passes};
+    Fp8LinearArgs args = {};
+    args.xq = xq;
+    args.xscale = xscale;
+    args.w[0] = wg;
+    args.w[1] = wu;
+    args.wscale[0] = wg_scale;
+    args.wscale[1] = wu_scale;
+    args.y[0] = y;
+    args.n[0] = n;
+    args.lanes = lanes;
+    args.k = k;
+    args.epilogue = EPILOGUE_BF16;
+    args.passes = passes;
     return launch_rows(linear_silu_multiply_fp8_kernel, dim3((n + rows - 1) / rows, (lanes + TILE_LANES - 1) / TILE_LANES), lanes, stream, args);
 }
 

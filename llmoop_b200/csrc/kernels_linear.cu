@@ -30,12 +30,23 @@ namespace nerve {
 
 // ----------------------------------------------------------------------------- bf16 weights
 
+struct Bf16Rows {  // the matrices of a launch: matrix b owns the CTAs first[b] .. first[b + 1] - 1
+    const uint16_t *w[3];
+    void *y[3];
+    int n[3], first[4];
+};
+
+// One launch for all matrices of an input: at the sizes this form is for, a launch of its own costs as much as the work
+// (64 x 64, q, k and v: 1.8 us each).
 template <int MT, int ROWS>
 __global__ void __launch_bounds__(256)
-linear_bf16_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ w, void *__restrict__ y,
-                   const uint16_t *__restrict__ residual, int lanes, int n, int k, int epilogue, float scale) {
+linear_bf16_kernel(const uint16_t *__restrict__ x, const __grid_constant__ Bf16Rows rows,
+                   const uint16_t *__restrict__ residual, int lanes, int k, int epilogue, float scale) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row0 = (blockIdx.x * 8 + warp) * ROWS;
+    const int block = blockIdx.x, branch = block < rows.first[1] ? 0 : block < rows.first[2] ? 1 : 2;
+    const uint16_t *__restrict__ w = rows.w[branch];
+    void *__restrict__ y = rows.y[branch];
+    const int n = rows.n[branch], row0 = ((block - rows.first[branch]) * 8 + warp) * ROWS;
     const int m0 = blockIdx.y * MT;
     if (row0 >= n) return;
     float acc[ROWS][MT];
@@ -108,15 +119,38 @@ linear_bf16_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ 
     }
 }
 
+bool linear_bf16_is_scalar(int lanes, int n, int k, LinearForm form) {
+    return form == LINEAR_SCALAR || !linear_bf16_gemm_supported(form == LINEAR_TENSOR ? 16 : lanes, n, k);
+}
+
 cudaError_t launch_linear_bf16(const uint16_t *x, const uint16_t *w, void *y, const uint16_t *residual, int lanes,
                                int n, int k, int epilogue, float scale, cudaStream_t stream, int *error_flag, LinearForm form) {
     if (lanes <= 0) return cudaSuccess;
     // more than eight lanes: the tensor-core GEMM (weights read once instead of once per eight lanes)
-    if (form != LINEAR_SCALAR && linear_bf16_gemm_supported(form == LINEAR_TENSOR ? 16 : lanes, n, k)) return launch_linear_bf16_gemm(x, w, y, residual, lanes, n, k, epilogue, scale, error_flag, stream);
+    if (!linear_bf16_is_scalar(lanes, n, k, form)) return launch_linear_bf16_gemm(x, w, y, residual, lanes, n, k, epilogue, scale, error_flag, stream);
+    LinearBranches branches;
+    branches.add(w, nullptr, y, n);
+    return launch_linear_bf16_scalar(x, branches, residual, lanes, k, epilogue, scale, stream);
+}
+
+cudaError_t launch_linear_bf16_scalar(const uint16_t *x, const LinearBranches &branches, const uint16_t *residual, int lanes, int k, int epilogue, float scale,
+                                      cudaStream_t stream) {
+    if (lanes <= 0) return cudaSuccess;
     constexpr int ROWS = 4;
-    int row_ctas = (n + 8 * ROWS - 1) / (8 * ROWS);
-    if (lanes <= 4) return launch_dependent(linear_bf16_kernel<4, ROWS>, dim3(row_ctas), dim3(256), 0, 1, stream, x, w, y, residual, lanes, n, k, epilogue, scale);
-    return launch_dependent(linear_bf16_kernel<8, ROWS>, dim3(row_ctas, (lanes + 7) / 8), dim3(256), 0, 1, stream, x, w, y, residual, lanes, n, k, epilogue, scale);
+    Bf16Rows rows = {};
+    int ctas = 0;
+    for (int b = 0; b < 3; b++) {
+        rows.first[b] = ctas;
+        if (b >= branches.count) continue;
+        rows.w[b] = static_cast<const uint16_t *>(branches.w[b]);
+        rows.y[b] = branches.y[b];
+        rows.n[b] = branches.n[b];
+        ctas += (branches.n[b] + 8 * ROWS - 1) / (8 * ROWS);
+    }
+    rows.first[3] = ctas;
+    for (int b = branches.count; b < 3; b++) rows.first[b] = ctas;
+    if (lanes <= 4) return launch_dependent(linear_bf16_kernel<4, ROWS>, dim3(ctas), dim3(256), 0, 1, stream, x, rows, residual, lanes, k, epilogue, scale);
+    return launch_dependent(linear_bf16_kernel<8, ROWS>, dim3(ctas, (lanes + 7) / 8), dim3(256), 0, 1, stream, x, rows, residual, lanes, k, epilogue, scale);
 }
 
 // parallel_linear_silu_multiply_bf16.comp.template:58-72
