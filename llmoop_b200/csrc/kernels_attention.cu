@@ -1016,6 +1016,7 @@ __global__ void argmax_partial_kernel(const float *__restrict__ logits, float *_
     const float *row = logits + static_cast<size_t>(lane) * vocab;
     float best = 0.0f;
     uint32_t token = 0xffffffffu;
+#pragma unroll 4
     for (int index = begin + threadIdx.x; index < end; index += blockDim.x) {
         float candidate = row[index];
         if (token == 0xffffffffu || candidate > best) {  // strictly greater keeps the lowest id within a thread
