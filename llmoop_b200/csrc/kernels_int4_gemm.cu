@@ -8,7 +8,8 @@
 // row's largest scale lies in [2^11, 2^12) - exact for every scale down to 2^-29 of the largest, and below that the
 // loss is 2^-40 of the row's largest weight.  The activations are bf16 times a power of two chosen per lane so that
 // the lane's largest value lies in [2^14, 2^15), as fp16: exact down to 2^-29 of the largest value.  Both powers of
-// two come off again in the epilogue.  No group scale is left to apply to partial sums, so the f32 accumulator stays
+// two come off again in the epilogue.  (Rows whose scales are close together take a cheaper form, dequantise_word_raw, in
+// another range of exponents.)  No group scale is left to apply to partial sums, so the f32 accumulator stays
 // in tensor memory over the whole of K (one that is read back, scaled and added up in registers for every group of
 // 128 columns ran at 140-175 TFLOP/s: the tensor pipe was idle 87 % of the time).
 //
@@ -25,6 +26,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.cuh"
@@ -109,6 +111,23 @@ __device__ __forceinline__ void dequantise_word(uint32_t word, uint32_t scale2, 
     out[1] = mul2(b, scale2);
     out[2] = mul2(c, scale2);
     out[3] = mul2(d, scale2);
+}
+
+// The same values x 2^-24 in four operations less, from the nibbles where they stand: as fp16 bit patterns they are q x 2^-24
+// (x 16 in the next four bits), subnormal and exact, and one fused multiply-add with 2^24 s and -8 s makes (q - 8) s of
+// them - exact as long as s keeps its eight bits above 2^-24, that is for rows whose scales lie within a factor of 64.
+// (16 x 28672 x 8192: 38.2 -> 33.2 us, 32 lanes: 39.4 -> 36.7; from 100 lanes on the tensor pipe is the bound.)
+__device__ __forceinline__ uint32_t fma2(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t out;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(out) : "r"(a), "r"(b), "r"(c));
+    return out;
+}
+__device__ __forceinline__ void dequantise_word_raw(uint32_t word, uint32_t scale2, uint32_t scale2_16th, uint32_t offset2, uint32_t (&out)[4]) {
+    const uint32_t shifted = word >> 8;
+    out[0] = fma2(word & 0x000F000Fu, scale2, offset2);
+    out[1] = fma2(word & 0x00F000F0u, scale2_16th, offset2);
+    out[2] = fma2(shifted & 0x000F000Fu, scale2, offset2);
+    out[3] = fma2(shifted & 0x00F000F0u, scale2_16th, offset2);
 }
 
 // A power of two as f32 from its biased exponent.
@@ -237,10 +256,16 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
         for (int item = 0; item < a.raw_stages - 1; item++) request();
         // the row's scales into shared memory ([group][row], read by this thread alone) and their largest exponent
         float factor;
+        bool raw_operands;  // of all the warp's rows: their largest scale enters as [2^14, 2^15) x 2^-24
         {
             const uint16_t *row_scales = a.scale_rows[matrix] + static_cast<size_t>(min(row0 + lane, n - 1)) * groups + first_group;
             uint16_t *const own = scales + row_tile * 128 + quarter * 32 + lane;
-            uint32_t largest = 16u << 7;
+            uint32_t largest = 16u << 7, smallest = 0x7FFFu;  // of the magnitudes that are not zero
+            auto note = [&](uint32_t bits) {
+                const uint32_t magnitude = bits & 0x7FFFu;
+                largest = max(largest, magnitude);
+                smallest = min(smallest, magnitude == 0 ? 0x7FFFu : magnitude);
+            };
             if (groups % 8 == 0 && own_groups % 8 == 0 && (reinterpret_cast<uintptr_t>(row_scales) & 15) == 0) {
                 constexpr int BATCH = 4;  // 16-byte loads in flight
                 for (int g = 0; g < own_groups; g += 8 * BATCH) {
@@ -255,7 +280,7 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
 #pragma unroll
                         for (int j = 0; j < 8; j++) {
                             const uint32_t bits = (words[j >> 1] >> (16 * (j & 1))) & 0xFFFFu;
-                            largest = max(largest, bits & 0x7FFFu);
+                            note(bits);
                             own[(g + 8 * i + j) * ROWS] = static_cast<uint16_t>(bits);
                         }
                     }
@@ -264,13 +289,14 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
 #pragma unroll 8
                 for (int g = 0; g < own_groups; g++) {
                     const uint16_t bits = __ldg(row_scales + g);
-                    largest = max(largest, static_cast<uint32_t>(bits) & 0x7FFFu);
+                    note(bits);
                     own[g * ROWS] = bits;
                 }
             }
             const int exponent = static_cast<int>(largest >> 7);
-            factor = power_of_two(min(265 - exponent, 254));
-            row_factor = power_of_two(max(exponent - 11, 1));
+            raw_operands = __all_sync(0xffffffffu, static_cast<int>(smallest >> 7) + 6 >= exponent && exponent <= 244);
+            factor = power_of_two(raw_operands ? 268 - exponent : min(265 - exponent, 254));
+            row_factor = power_of_two(raw_operands ? exponent + 10 : max(exponent - 11, 1));
         }
         const uint32_t read_base = warp_raw + static_cast<uint32_t>(lane * 64);
         const uint32_t read_swizzle = static_cast<uint32_t>((lane >> 1) & 3);
@@ -287,52 +313,59 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
                 parity ^= 1;
             }
         };
-        for (int item = 0; item < items; item++) {
-            request();
-            switch (a.raw_stages) {  // the item's own copies have landed
-            case 3: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
-            case 4: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
-            case 5: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
-            default: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
-            }
-            __syncwarp();
-            uint32_t scale2 = __half_as_ushort(__float2half_rn(bf16_bits_to_f32(*scale) * factor));
-            scale2 |= scale2 << 16;
-            scale += 2 * ROWS;
-            uint4 words[4];
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const uint32_t address = read_base + read_slot + ((static_cast<uint32_t>(c) ^ read_swizzle) * 16);
-                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(words[c].x), "=r"(words[c].y), "=r"(words[c].z), "=r"(words[c].w) : "r"(address));
-            }
-            read_slot = read_slot + SLOT == slots_end ? 0 : read_slot + SLOT;
-#pragma unroll
-            for (int part = 0; part < PARTS; part++) {
-                if (alive && !wait_barrier(a_empty + stage * 8, parity, a.error_flag)) alive = false;
-                if (!alive) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t target = tmem_rows + static_cast<uint32_t>(stage) * (A_COLUMNS * ROW_TILES);
-#pragma unroll
-                for (int c = 0; c < 4 / PARTS; c++) {
-                    const uint4 packed = words[part * (4 / PARTS) + c];
-                    uint32_t v[4][4];
-                    dequantise_word(packed.x, scale2, v[0]);
-                    dequantise_word(packed.y, scale2, v[1]);
-                    dequantise_word(packed.z, scale2, v[2]);
-                    dequantise_word(packed.w, scale2, v[3]);
-                    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(target + c * 16),
-                                 "r"(v[0][0]), "r"(v[0][1]), "r"(v[0][2]), "r"(v[0][3]), "r"(v[1][0]), "r"(v[1][1]), "r"(v[1][2]), "r"(v[1][3]), "r"(v[2][0]),
-                                 "r"(v[2][1]), "r"(v[2][2]), "r"(v[2][3]), "r"(v[3][0]), "r"(v[3][1]), "r"(v[3][2]), "r"(v[3][3])
-                                 : "memory");
+        auto prepare = [&](auto raw) {
+            for (int item = 0; item < items; item++) {
+                request();
+                switch (a.raw_stages) {  // the item's own copies have landed
+                case 3: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+                case 4: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+                case 5: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+                default: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
                 }
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a_full + stage * 8) : "memory");
-                advance(part + 1 < PARTS ? 1 : PARTS + 1);  // over the other set's group
+                uint32_t scale2 = __half_as_ushort(__float2half_rn(bf16_bits_to_f32(*scale) * factor));
+                scale2 |= scale2 << 16;
+                scale += 2 * ROWS;
+                uint4 words[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const uint32_t address = read_base + read_slot + ((static_cast<uint32_t>(c) ^ read_swizzle) * 16);
+                    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(words[c].x), "=r"(words[c].y), "=r"(words[c].z), "=r"(words[c].w) : "r"(address));
+                }
+                read_slot = read_slot + SLOT == slots_end ? 0 : read_slot + SLOT;
+                const uint32_t scale2_16th = mul2(scale2, 0x2C002C00u), offset2 = mul2(scale2, 0x80088008u);  // s / 16; -2^-21 s
+#pragma unroll
+                for (int part = 0; part < PARTS; part++) {
+                    if (alive && !wait_barrier(a_empty + stage * 8, parity, a.error_flag)) alive = false;
+                    if (!alive) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t target = tmem_rows + static_cast<uint32_t>(stage) * (A_COLUMNS * ROW_TILES);
+#pragma unroll
+                    for (int c = 0; c < 4 / PARTS; c++) {
+                        const uint4 packed = words[part * (4 / PARTS) + c];
+                        uint32_t v[4][4];
+                        const uint32_t four[4] = {packed.x, packed.y, packed.z, packed.w};
+#pragma unroll
+                        for (int w = 0; w < 4; w++) {
+                            if (raw) dequantise_word_raw(four[w], scale2, scale2_16th, offset2, v[w]);
+                            else dequantise_word(four[w], scale2, v[w]);
+                        }
+                        asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(target + c * 16),
+                                     "r"(v[0][0]), "r"(v[0][1]), "r"(v[0][2]), "r"(v[0][3]), "r"(v[1][0]), "r"(v[1][1]), "r"(v[1][2]), "r"(v[1][3]), "r"(v[2][0]),
+                                     "r"(v[2][1]), "r"(v[2][2]), "r"(v[2][3]), "r"(v[3][0]), "r"(v[3][1]), "r"(v[3][2]), "r"(v[3][3])
+                                     : "memory");
+                    }
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a_full + stage * 8) : "memory");
+                    advance(part + 1 < PARTS ? 1 : PARTS + 1);  // over the other set's group
+                }
+                if (!alive) break;
             }
-            if (!alive) break;
-        }
+        };
+        if (raw_operands) prepare(std::true_type{});
+        else prepare(std::false_type{});
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (warp == WARPS) {
         // instruction descriptor: f32 accumulator, A and B fp16, both K-major, N / 8 in bits 17-22, M / 16 in bits 24-28

@@ -1,7 +1,8 @@
 """The INT4 tensor-core linear of more than eight lanes at the edges of its tiles and ranges, through the operator-level
 entry point against the CPU oracle: lane tiles of 16 with remainders, one and two row tiles per CTA, ragged last row
 tiles, a single group of K, K split over a cluster, more than one lane tile; activations and group scales far from 1
-(both enter the tensor core as fp16 behind a power of two per lane and per row)."""
+(both enter the tensor core as fp16 behind a power of two per lane and per row), and scales of a row far from and close
+to one another (two forms of the operands)."""
 
 import ctypes
 
@@ -15,8 +16,8 @@ pytestmark = pytest.mark.gpu
     (9, 128, 128), (16, 130, 256), (17, 64, 4096), (64, 1000, 384), (65, 257, 1152), (128, 96, 2048), (129, 384, 640), (256, 128, 128), (257, 300, 256),
     (150, 19000, 384), (310, 18945, 128),  # two row tiles of 160 lanes: half groups
 ])
-@pytest.mark.parametrize("x_scale,w_scale", [(1.0, 0.02), (2.0 ** 90, 2.0 ** -60), (2.0 ** -100, 2.0 ** 40)])
-def test_int4_gemm_edges_match_oracle(lanes, n, k, x_scale, w_scale):
+@pytest.mark.parametrize("x_scale,w_scale,spread", [(1.0, 0.02, 8), (2.0 ** 90, 2.0 ** -60, 3), (2.0 ** -100, 2.0 ** 40, 5)])
+def test_int4_gemm_edges_match_oracle(lanes, n, k, x_scale, w_scale, spread):
     import torch
 
     import llmoop_b200 as nb
@@ -26,7 +27,7 @@ def test_int4_gemm_edges_match_oracle(lanes, n, k, x_scale, w_scale):
 
     rng = np.random.default_rng(lanes * 7 + n + k)
     packed, scales = quantize_int4_group(rng.standard_normal((n, k), dtype=np.float32))
-    scales = f32_to_bf16_bits(bf16_bits_to_f32(scales) * np.float32(w_scale) * (2.0 ** rng.integers(-8, 1, size=scales.shape)).astype(np.float32))
+    scales = f32_to_bf16_bits(bf16_bits_to_f32(scales) * np.float32(w_scale) * (2.0 ** rng.integers(-spread, 1, size=scales.shape)).astype(np.float32))
     x = rng.standard_normal((lanes, k), dtype=np.float32) * np.float32(x_scale)
     x[:, ::7] *= np.float32(2.0 ** -12)  # far smaller values beside them
     x = f32_to_bf16_bits(x)
