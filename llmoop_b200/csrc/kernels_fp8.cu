@@ -10,10 +10,12 @@
 //
 // A warp computes ROWS x M outputs: thread l owns column group l, keeps ROWS x M partial sums in registers and walks the
 // blocks; weights come straight from global memory (one coalesced 128-byte row piece per warp and block, requested
-// PIPE blocks ahead), the activations as f32 from shared memory, two lanes to a packed f32x2 operand.  Per block and
-// warp: 5 FP32 operations per weight word and lane against 6 conversions per weight word, so from eight lanes on the
-// FP32 pipe is the bound (1024 lanes x 2048 x 4096: 480 us with one row and eight lanes per warp, the form this
-// replaced), below that the weight bytes.
+// PIPE blocks ahead), the activations as fp16 from shared memory.  The products of a column group are added up with
+// fp16 x fp16 + f32 multiply-adds (exact products, so the same roundings as on widened values), the scaled sums two lanes
+// to a packed f32x2 operand: per weight word and lane four of the former and half of the latter, at an FP32 pipe of 25 and
+// 30 TMAC/s, so about 20 TMAC/s is the bound from eight lanes on, below that the weight bytes.  1024 lanes x 4096 x 2048:
+// 617 us with both operands widened to f32 (14 TMAC/s; the shared-memory loads and the conversions were at the same
+// bound), now 533; x 2048 x 4096: 676 -> 509 us.
 // Sparse experts are grouped: a small kernel sorts the (token, route) pairs by expert into tiles of up to eight, and an
 // expert's rows are read once per tile instead of once per pair.
 #include <cstdlib>
@@ -27,7 +29,7 @@ namespace nerve {
 namespace {
 
 constexpr int FP8_WARPS = 8, FP8_ROWS = 8, TILE_LANES = 8;
-constexpr int CHUNK = 16;  // blocks of 128 columns whose activations are staged at a time: 64 KB for eight lanes, two CTAs per SM
+constexpr int CHUNK = 32;  // blocks of 128 columns whose activations are staged at a time: 66 KB for eight lanes, two CTAs per SM
 
 using pair_t = unsigned long long;  // two f32
 __device__ __forceinline__ pair_t pack(float lo, float hi) {
@@ -45,40 +47,66 @@ __device__ __forceinline__ pair_t mul(pair_t a, pair_t b) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(out) : "l"(a), "l"(b));
     return out;
 }
+// a.lo * b.lo + c and a.hi * b.hi + c of fp16 pairs in f32: the product of two e4m3 values is exact, so these round as the
+// f32 multiply-add of the widened values does - without widening them, and with half the bytes in shared memory
+__device__ __forceinline__ float mixed_fma_lo(uint32_t a, uint32_t b, float c) {
+    asm("{\n.reg .b16 al, ah, bl, bh;\nmov.b32 {al, ah}, %1;\nmov.b32 {bl, bh}, %2;\nfma.rn.f32.f16 %0, al, bl, %0;\n}\n" : "+f"(c) : "r"(a), "r"(b));
+    return c;
+}
+__device__ __forceinline__ float mixed_fma_hi(uint32_t a, uint32_t b, float c) {
+    asm("{\n.reg .b16 al, ah, bl, bh;\nmov.b32 {al, ah}, %1;\nmov.b32 {bl, bh}, %2;\nfma.rn.f32.f16 %0, ah, bh, %0;\n}\n" : "+f"(c) : "r"(a), "r"(b));
+    return c;
+}
 __device__ __forceinline__ pair_t fma2(pair_t a, pair_t b, pair_t c) {
     pair_t out;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(out) : "l"(a), "l"(b), "l"(c));
     return out;
 }
-// four e4m3 values of a word as f32, exact
-__device__ __forceinline__ void widen(uint32_t word, float (&out)[4]) {
-    uint32_t lo, hi;
-    asm("{\n.reg .b16 a, b;\nmov.b32 {a, b}, %2;\ncvt.rn.f16x2.e4m3x2 %0, a;\ncvt.rn.f16x2.e4m3x2 %1, b;\n}\n" : "=r"(lo), "=r"(hi) : "r"(word));
-    const float2 first = __half22float2(*reinterpret_cast<const __half2 *>(&lo)), second = __half22float2(*reinterpret_cast<const __half2 *>(&hi));
-    out[0] = first.x;
-    out[1] = first.y;
-    out[2] = second.x;
-    out[3] = second.y;
+// four e4m3 values of a word as two fp16 pairs, exact
+__device__ __forceinline__ uint2 widen(uint32_t word) {
+    uint2 out;
+    asm("{\n.reg .b16 a, b;\nmov.b32 {a, b}, %2;\ncvt.rn.f16x2.e4m3x2 %0, a;\ncvt.rn.f16x2.e4m3x2 %1, b;\n}\n" : "=r"(out.x), "=r"(out.y) : "r"(word));
+    return out;
 }
 
 // The activations of up to M lanes (rows of xq / xscale picked by `row_of`) in shared memory:
-// x [block][lane pair][column pair][thread][column of the pair][lane of the pair] f32, scales [block][M].
+// x [block][lane pair][thread][lane of the pair][column] fp16, scales [block][M] f32.
 template <int M>
-__device__ __forceinline__ size_t x_index(int block, int pair, int half, int thread) {
-    return ((static_cast<size_t>(block) * (M / 2) + pair) * 2 + half) * 128 + thread * 4;
-}
+constexpr size_t x_bytes() { return static_cast<size_t>(CHUNK) * 128 * M * 2; }
 template <int M, typename RowOf>
-__device__ __forceinline__ void stage_activations(const uint8_t *__restrict__ xq, const float *__restrict__ xscale, int k, int first, int blocks, int count, float *x,
+__device__ __forceinline__ void stage_activations(const uint8_t *__restrict__ xq, const float *__restrict__ xscale, int k, int first, int blocks, int count, uint8_t *smem,
                                                   RowOf row_of) {
     const int words = blocks * 32, all_blocks = k >> 7;
-    float *scales = x + static_cast<size_t>(CHUNK) * 128 * M;
-    for (int index = threadIdx.x; index < words * (M / 2); index += FP8_WARPS * 32) {
-        const int pair = index / words, word = index - pair * words, block = word >> 5, thread = word & 31;
-        float lo[4] = {}, hi[4] = {};
-        if (2 * pair < count) widen(reinterpret_cast<const uint32_t *>(xq + static_cast<size_t>(row_of(2 * pair)) * k)[first * 32 + word], lo);
-        if (2 * pair + 1 < count) widen(reinterpret_cast<const uint32_t *>(xq + static_cast<size_t>(row_of(2 * pair + 1)) * k)[first * 32 + word], hi);
-        *reinterpret_cast<float4 *>(x + x_index<M>(block, pair, 0, thread)) = make_float4(lo[0], hi[0], lo[1], hi[1]);
-        *reinterpret_cast<float4 *>(x + x_index<M>(block, pair, 1, thread)) = make_float4(lo[2], hi[2], lo[3], hi[3]);
+    uint4 *x = reinterpret_cast<uint4 *>(smem);
+    float *scales = reinterpret_cast<float *>(smem + x_bytes<M>());
+    // (pair, word) of this thread's next item; four items' loads in flight (one after the other the staging of eight lanes
+    // of 2048 took 6 of 23 us)
+    int pair = threadIdx.x / words, word = threadIdx.x - pair * words;
+    constexpr int BATCH = 4;
+    while (pair < M / 2) {
+        uint32_t lo[BATCH], hi[BATCH];
+        int target[BATCH];
+#pragma unroll
+        for (int i = 0; i < BATCH; i++) {
+            lo[i] = hi[i] = 0;
+            target[i] = -1;
+            if (pair < M / 2) {
+                if (2 * pair < count) lo[i] = reinterpret_cast<const uint32_t *>(xq + static_cast<size_t>(row_of(2 * pair)) * k)[first * 32 + word];
+                if (2 * pair + 1 < count) hi[i] = reinterpret_cast<const uint32_t *>(xq + static_cast<size_t>(row_of(2 * pair + 1)) * k)[first * 32 + word];
+                target[i] = ((word >> 5) * (M / 2) + pair) * 32 + (word & 31);
+            }
+            word += FP8_WARPS * 32;
+            while (word >= words) {
+                word -= words;
+                pair++;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < BATCH; i++)
+            if (target[i] >= 0) {
+                const uint2 a = widen(lo[i]), b = widen(hi[i]);
+                x[target[i]] = make_uint4(a.x, a.y, b.x, b.y);
+            }
     }
     for (int index = threadIdx.x; index < blocks * M; index += FP8_WARPS * 32) {
         const int m = index % M, block = index / M;
@@ -89,11 +117,11 @@ __device__ __forceinline__ void stage_activations(const uint8_t *__restrict__ xq
 // Sums of ROWS rows x M lanes over all of K; the two halves of the rows may have scale rows of their own (gate and up).
 // Eight lanes take four rows at a time (the partial sums of more do not fit the registers of two CTAs per SM), fewer
 // lanes eight.  On return thread t holds the outputs index(t, i) (or the one of its thread pair for M = 2).
-template <int M>
+template <int M, bool PAIRED>
 struct RowSums {
     static constexpr int ROWS = M == 8 ? 4 : 8;
     static constexpr int VALUES = ROWS * M, PER_THREAD = VALUES >= 32 ? VALUES / 32 : 1;
-    static constexpr int PIPE = M == 2 ? 4 : 2;  // blocks of weights in flight
+    static constexpr int PIPE = M == 8 && PAIRED ? 2 : 4;  // blocks of weights in flight
     float sums[PER_THREAD];
 
     // output index = row * M + lane
@@ -105,8 +133,9 @@ struct RowSums {
 
     // stage(first, n) brings the activations of blocks first .. first + n - 1 into x (which may hold all of them already)
     template <typename RowPointer, typename Stage>
-    __device__ void run(RowPointer row_pointer, const uint16_t *__restrict__ scales_a, const uint16_t *__restrict__ scales_b, int blocks, float *x, bool staged_already, Stage stage_blocks) {
-        const float *x_scales = x + static_cast<size_t>(CHUNK) * 128 * M;
+    __device__ void run(RowPointer row_pointer, const uint16_t *__restrict__ scales_a, const uint16_t *__restrict__ scales_b, int blocks, const uint8_t *smem, bool staged_already, Stage stage_blocks) {
+        const uint4 *x = reinterpret_cast<const uint4 *>(smem);
+        const float *x_scales = reinterpret_cast<const float *>(smem + x_bytes<M>());
         const int thread = threadIdx.x & 31;
         const uint32_t *source[ROWS];
 #pragma unroll
@@ -121,7 +150,12 @@ struct RowSums {
         for (int r = 0; r < ROWS; r++)
 #pragma unroll
             for (int p = 0; p < M / 2; p++) acc[r][p] = 0ull;
+        float scale_a = 0.0f, scale_b = 0.0f;  // of block (32 i + thread)
         for (int base = 0; base < blocks; base += PIPE) {
+            if (base % 32 == 0 && base + thread < blocks) {
+                scale_a = bf16_bits_to_f32(__ldg(scales_a + base + thread));
+                if (PAIRED) scale_b = bf16_bits_to_f32(__ldg(scales_b + base + thread));
+            }
             if (base % CHUNK == 0 && (!staged_already || blocks > CHUNK)) {
                 __syncthreads();
                 stage_blocks(base, min(CHUNK, blocks - base));
@@ -131,32 +165,24 @@ struct RowSums {
             for (int stage = 0; stage < PIPE; stage++) {
                 const int block = base + stage, staged = block % CHUNK;
                 if (block >= blocks) break;
-                const float wa = bf16_bits_to_f32(__ldg(scales_a + block)), wb = bf16_bits_to_f32(__ldg(scales_b + block));
-                pair_t xv[M / 2][4], sa[M / 2], sb[M / 2];
+                const float wa = __shfl_sync(0xffffffffu, scale_a, block & 31), wb = PAIRED ? __shfl_sync(0xffffffffu, scale_b, block & 31) : wa;
+                uint4 xv[M / 2];
+                pair_t sa[M / 2], sb[M / 2];
 #pragma unroll
                 for (int p = 0; p < M / 2; p++) {
-                    const ulonglong2 first = *reinterpret_cast<const ulonglong2 *>(x + x_index<M>(staged, p, 0, thread));
-                    const ulonglong2 second = *reinterpret_cast<const ulonglong2 *>(x + x_index<M>(staged, p, 1, thread));
-                    xv[p][0] = first.x;
-                    xv[p][1] = first.y;
-                    xv[p][2] = second.x;
-                    xv[p][3] = second.y;
+                    xv[p] = x[(staged * (M / 2) + p) * 32 + thread];
                     const pair_t xs = *reinterpret_cast<const pair_t *>(x_scales + staged * M + 2 * p);
                     sa[p] = mul(xs, pack(wa, wa));
-                    sb[p] = mul(xs, pack(wb, wb));
+                    sb[p] = PAIRED ? mul(xs, pack(wb, wb)) : sa[p];
                 }
 #pragma unroll
                 for (int r = 0; r < ROWS; r++) {
-                    float w[4];
-                    widen(words[stage][r], w);
-                    const pair_t w2[4] = {pack(w[0], w[0]), pack(w[1], w[1]), pack(w[2], w[2]), pack(w[3], w[3])};
+                    const uint2 w = widen(words[stage][r]);
 #pragma unroll
                     for (int p = 0; p < M / 2; p++) {
-                        pair_t d = mul(xv[p][0], w2[0]);
-                        d = fma2(xv[p][1], w2[1], d);
-                        d = fma2(xv[p][2], w2[2], d);
-                        d = fma2(xv[p][3], w2[3], d);
-                        acc[r][p] = fma2(d, r < ROWS / 2 ? sa[p] : sb[p], acc[r][p]);
+                        const float d0 = mixed_fma_hi(xv[p].y, w.y, mixed_fma_lo(xv[p].y, w.y, mixed_fma_hi(xv[p].x, w.x, mixed_fma_lo(xv[p].x, w.x, 0.0f))));
+                        const float d1 = mixed_fma_hi(xv[p].w, w.y, mixed_fma_lo(xv[p].w, w.y, mixed_fma_hi(xv[p].z, w.x, mixed_fma_lo(xv[p].z, w.x, 0.0f))));
+                        acc[r][p] = fma2(pack(d0, d1), r < ROWS / 2 ? sa[p] : sb[p], acc[r][p]);
                     }
                     words[stage][r] = block + PIPE < blocks ? __ldg(source[r] + (block + PIPE) * 32) : 0u;
                 }
@@ -213,21 +239,21 @@ struct Fp8LinearArgs {
 };
 
 template <int M>
-__device__ __forceinline__ void fp8_linear_tile(const Fp8LinearArgs &a, int m0, int count, float *smem) {
+__device__ __forceinline__ void fp8_linear_tile(const Fp8LinearArgs &a, int m0, int count, uint8_t *smem) {
     const int warp = threadIdx.x >> 5, thread = threadIdx.x & 31, blocks = a.k >> 7;
     const int tile = blockIdx.x, matrix = tile < a.first[1] ? 0 : tile < a.first[2] ? 1 : 2, rows = a.n[matrix];
     const uint8_t *const w = a.w[matrix];
     auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, a.k, first, n, count, smem, [&](int m) { return m0 + m; }); };
-    const int warps = 32 * a.passes / RowSums<M>::ROWS;  // with rows to do in a pass
+    const int warps = 32 * a.passes / RowSums<M, false>::ROWS;  // with rows to do in a pass
     for (int pass = 0; pass < (warps > FP8_WARPS ? 2 : 1); pass++) {
-        const int row0 = (tile - a.first[matrix]) * 32 * a.passes + (pass * FP8_WARPS + warp) * RowSums<M>::ROWS;
-        RowSums<M> sums;
+        const int row0 = (tile - a.first[matrix]) * 32 * a.passes + (pass * FP8_WARPS + warp) * RowSums<M, false>::ROWS;
+        RowSums<M, false> sums;
         const uint16_t *scale_row = a.wscale[matrix] + static_cast<size_t>(min(row0, rows - 1) >> 7) * blocks;  // eight rows lie in one block of 128
         sums.run([&](int r) { return w + static_cast<size_t>(min(row0 + r, rows - 1)) * a.k; }, scale_row, scale_row, blocks, smem, pass > 0, stage);
-        if (RowSums<M>::VALUES < 32 && (thread & 1) != 0) continue;
+        if (RowSums<M, false>::VALUES < 32 && (thread & 1) != 0) continue;
 #pragma unroll
-        for (int i = 0; i < RowSums<M>::PER_THREAD; i++) {
-            const int output = RowSums<M>::index(thread, i), row = row0 + output / M, m = output % M;
+        for (int i = 0; i < RowSums<M, false>::PER_THREAD; i++) {
+            const int output = RowSums<M, false>::index(thread, i), row = row0 + output / M, m = output % M;
             if (row >= rows || m >= count || warp >= warps) continue;
             const size_t out = static_cast<size_t>(m0 + m) * rows + row;
             float sum = sums.sums[i];
@@ -240,7 +266,7 @@ __device__ __forceinline__ void fp8_linear_tile(const Fp8LinearArgs &a, int m0, 
 
 // grid (row tiles of 64, lane tiles of 8)
 __global__ void __launch_bounds__(FP8_WARPS * 32, 2) linear_fp8_kernel(const __grid_constant__ Fp8LinearArgs a) {
-    extern __shared__ __align__(16) float fp8_smem[];
+    extern __shared__ __align__(16) uint8_t fp8_smem[];
     grid_launch_dependents();
     grid_dependency_wait();
     const int m0 = blockIdx.y * TILE_LANES, count = min(TILE_LANES, a.lanes - m0);
@@ -250,30 +276,30 @@ __global__ void __launch_bounds__(FP8_WARPS * 32, 2) linear_fp8_kernel(const __g
 
 // rounded_silu(round(gate)) * round(up) from a warp's sums: the first half of the rows is gate, the second the same rows of up
 template <int M, typename Store>
-__device__ __forceinline__ void silu_outputs(const RowSums<M> &sums, Store store) {
+__device__ __forceinline__ void silu_outputs(const RowSums<M, true> &sums, Store store) {
     const int thread = threadIdx.x & 31;
-    constexpr int PER = RowSums<M>::PER_THREAD;
+    constexpr int PER = RowSums<M, true>::PER_THREAD;
     float other[PER];
     // the up sums of a thread's gate outputs sit in the thread 16 further (the top bit of the output index)
 #pragma unroll
     for (int i = 0; i < PER; i++) other[i] = __shfl_xor_sync(0xffffffffu, sums.sums[i], 16);
-    if (thread >= 16 || (RowSums<M>::VALUES < 32 && (thread & 1) != 0)) return;
+    if (thread >= 16 || (RowSums<M, true>::VALUES < 32 && (thread & 1) != 0)) return;
 #pragma unroll
     for (int i = 0; i < PER; i++) {
-        const int output = RowSums<M>::index(thread, i);
+        const int output = RowSums<M, true>::index(thread, i);
         store(output / M, output % M, round_bf16(sums.sums[i]), round_bf16(other[i]));
     }
 }
 
 template <int M>
-__device__ __forceinline__ void fp8_silu_tile(const Fp8LinearArgs &a, int m0, int count, float *smem) {
+__device__ __forceinline__ void fp8_silu_tile(const Fp8LinearArgs &a, int m0, int count, uint8_t *smem) {
     const int warp = threadIdx.x >> 5, blocks = a.k >> 7;
     auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, a.k, first, n, count, smem, [&](int m) { return m0 + m; }); };
-    constexpr int HALF = RowSums<M>::ROWS / 2;
-    const int warps = 32 * a.passes / RowSums<M>::ROWS;
+    constexpr int HALF = RowSums<M, true>::ROWS / 2;
+    const int warps = 32 * a.passes / RowSums<M, true>::ROWS;
     for (int pass = 0; pass < (warps > FP8_WARPS ? 2 : 1); pass++) {
         const int row0 = blockIdx.x * 16 * a.passes + (pass * FP8_WARPS + warp) * HALF, first = min(row0, a.n[0] - 1);
-        RowSums<M> sums;
+        RowSums<M, true> sums;
         sums.run([&](int r) { return a.w[r / HALF] + static_cast<size_t>(min(row0 + r % HALF, a.n[0] - 1)) * a.k; }, a.wscale[0] + static_cast<size_t>(first >> 7) * blocks,
                  a.wscale[1] + static_cast<size_t>(first >> 7) * blocks, blocks, smem, pass > 0, stage);
         silu_outputs<M>(sums, [&](int r, int m, float gate, float up) {
@@ -284,7 +310,7 @@ __device__ __forceinline__ void fp8_silu_tile(const Fp8LinearArgs &a, int m0, in
 }
 
 __global__ void __launch_bounds__(FP8_WARPS * 32, 2) linear_silu_multiply_fp8_kernel(const __grid_constant__ Fp8LinearArgs a) {
-    extern __shared__ __align__(16) float fp8_smem[];
+    extern __shared__ __align__(16) uint8_t fp8_smem[];
     grid_launch_dependents();
     grid_dependency_wait();
     const int m0 = blockIdx.y * TILE_LANES, count = min(TILE_LANES, a.lanes - m0);
@@ -359,17 +385,17 @@ struct MoeArgs {
 
 // grid (tiles of 32 intermediate rows, expert tiles); the activations of a pair are its token's row
 template <int M>
-__device__ __forceinline__ void moe_gate_up_tile(const MoeArgs &a, int4 tile, float *smem) {
+__device__ __forceinline__ void moe_gate_up_tile(const MoeArgs &a, int4 tile, uint8_t *smem) {
     const int warp = threadIdx.x >> 5, k = a.hidden, blocks = k >> 7, count = tile.z;
     const int *order = a.groups.order + tile.y;
     auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, k, first, n, count, smem, [&](int m) { return order[m] / a.top_k; }); };
-    constexpr int HALF = RowSums<M>::ROWS / 2;
+    constexpr int HALF = RowSums<M, true>::ROWS / 2;
     const int expert = tile.x - a.expert_start;
     const uint8_t *w = a.w + static_cast<size_t>(expert) * 2 * a.inter * k;
     const uint16_t *ws = a.wscale + static_cast<size_t>(expert) * ((2 * a.inter + 127) >> 7) * blocks;
-    for (int pass = 0; pass < FP8_ROWS / RowSums<M>::ROWS; pass++) {
+    for (int pass = 0; pass < FP8_ROWS / RowSums<M, true>::ROWS; pass++) {
         const int row0 = (blockIdx.x * FP8_WARPS + warp) * (FP8_ROWS / 2) + pass * HALF, first = min(row0, a.inter - 1);
-        RowSums<M> sums;
+        RowSums<M, true> sums;
         sums.run([&](int r) { return w + static_cast<size_t>((r >= HALF ? a.inter : 0) + min(row0 + r % HALF, a.inter - 1)) * k; },
                  ws + static_cast<size_t>(first >> 7) * blocks, ws + static_cast<size_t>((a.inter + first) >> 7) * blocks, blocks, smem, pass > 0, stage);
         silu_outputs<M>(sums, [&](int r, int m, float gate, float up) {
@@ -381,7 +407,7 @@ __device__ __forceinline__ void moe_gate_up_tile(const MoeArgs &a, int4 tile, fl
 }
 
 __global__ void __launch_bounds__(FP8_WARPS * 32, 2) moe_gate_up_fp8_kernel(const __grid_constant__ MoeArgs a) {
-    extern __shared__ __align__(16) float fp8_smem[];
+    extern __shared__ __align__(16) uint8_t fp8_smem[];
     grid_launch_dependents();
     grid_dependency_wait();
     if (static_cast<int>(blockIdx.y) >= *a.groups.tile_count) return;
@@ -391,22 +417,22 @@ __global__ void __launch_bounds__(FP8_WARPS * 32, 2) moe_gate_up_fp8_kernel(cons
 
 // grid (tiles of 64 hidden rows, expert tiles); out = bf16(bf16(sum) * route weight) per pair
 template <int M>
-__device__ __forceinline__ void moe_down_tile(const MoeArgs &a, int4 tile, float *smem) {
+__device__ __forceinline__ void moe_down_tile(const MoeArgs &a, int4 tile, uint8_t *smem) {
     const int warp = threadIdx.x >> 5, thread = threadIdx.x & 31, k = a.inter, blocks = k >> 7, count = tile.z;
     const int *order = a.groups.order + tile.y;
     auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, k, first, n, count, smem, [&](int m) { return order[m]; }); };
     const int expert = tile.x - a.expert_start;
     const uint8_t *w = a.w + static_cast<size_t>(expert) * a.hidden * k;
     const uint16_t *ws = a.wscale + static_cast<size_t>(expert) * ((a.hidden + 127) >> 7) * blocks;
-    for (int pass = 0; pass < FP8_ROWS / RowSums<M>::ROWS; pass++) {
-        const int row0 = (blockIdx.x * FP8_WARPS + warp) * FP8_ROWS + pass * RowSums<M>::ROWS;
+    for (int pass = 0; pass < FP8_ROWS / RowSums<M, false>::ROWS; pass++) {
+        const int row0 = (blockIdx.x * FP8_WARPS + warp) * FP8_ROWS + pass * RowSums<M, false>::ROWS;
         const uint16_t *scale_row = ws + static_cast<size_t>(min(row0, a.hidden - 1) >> 7) * blocks;
-        RowSums<M> sums;
+        RowSums<M, false> sums;
         sums.run([&](int r) { return w + static_cast<size_t>(min(row0 + r, a.hidden - 1)) * k; }, scale_row, scale_row, blocks, smem, pass > 0, stage);
-        if (RowSums<M>::VALUES < 32 && (thread & 1) != 0) continue;
+        if (RowSums<M, false>::VALUES < 32 && (thread & 1) != 0) continue;
 #pragma unroll
-        for (int i = 0; i < RowSums<M>::PER_THREAD; i++) {
-            const int output = RowSums<M>::index(thread, i), row = row0 + output / M, m = output % M;
+        for (int i = 0; i < RowSums<M, false>::PER_THREAD; i++) {
+            const int output = RowSums<M, false>::index(thread, i), row = row0 + output / M, m = output % M;
             if (row >= a.hidden || m >= count) continue;
             const float weight = bf16_bits_to_f32(a.routes[order[m]] >> 16);
             a.out[static_cast<size_t>(order[m]) * a.hidden + row] = static_cast<uint16_t>(f32_to_bf16_bits(round_bf16(sums.sums[i]) * weight));
@@ -415,7 +441,7 @@ __device__ __forceinline__ void moe_down_tile(const MoeArgs &a, int4 tile, float
 }
 
 __global__ void __launch_bounds__(FP8_WARPS * 32, 2) moe_down_fp8_kernel(const __grid_constant__ MoeArgs a) {
-    extern __shared__ __align__(16) float fp8_smem[];
+    extern __shared__ __align__(16) uint8_t fp8_smem[];
     grid_launch_dependents();
     grid_dependency_wait();
     if (static_cast<int>(blockIdx.y) >= *a.groups.tile_count) return;
@@ -425,7 +451,7 @@ __global__ void __launch_bounds__(FP8_WARPS * 32, 2) moe_down_fp8_kernel(const _
 
 template <typename Args>
 cudaError_t launch_rows(void (*kernel)(Args), dim3 grid, int tile_lanes, cudaStream_t stream, const Args &args) {
-    auto bytes = [](int m) { return static_cast<size_t>(CHUNK) * 128 * m * sizeof(float) + static_cast<size_t>(CHUNK) * m * sizeof(float); };
+    auto bytes = [](int m) { return static_cast<size_t>(CHUNK) * 128 * m * 2 + static_cast<size_t>(CHUNK) * m * sizeof(float); };
     cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes(8)));
     if (status != cudaSuccess) return status;
     return launch_dependent(kernel, grid, dim3(FP8_WARPS * 32), bytes(tile_lanes <= 2 ? 2 : tile_lanes <= 4 ? 4 : 8), 1, stream, args);
