@@ -55,7 +55,7 @@ linear_bf16_kernel(const uint16_t *__restrict__ x, const __grid_constant__ Bf16R
 #pragma unroll
         for (int m = 0; m < MT; m++) acc[r][m] = 0.0f;
 
-    const int chunks = k / 8;  // uint4 = 8 bf16
+    const int chunks = k % 8 == 0 ? k / 8 : 0;  // uint4 = 8 bf16; rows of other widths are not aligned to it
     // weights do not depend on the previous kernel: the first loads may be issued before the dependency wait
     grid_launch_dependents();
     grid_dependency_wait();
@@ -82,7 +82,7 @@ linear_bf16_kernel(const uint16_t *__restrict__ x, const __grid_constant__ Bf16R
             }
         }
     }
-    // tail for k not a multiple of 8 (tiny test shapes)
+    // k not a multiple of 8 (tiny test shapes)
     for (int col = chunks * 8 + lane; col < k; col += 32) {
 #pragma unroll
         for (int r = 0; r < ROWS; r++) {
