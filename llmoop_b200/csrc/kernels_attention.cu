@@ -611,7 +611,7 @@ attention_f32_kernel(const uint16_t *__restrict__ q, KvLayer kv, LaneTable lanes
 
 // Log-sum-exp merge of the split partials of one (lane, q head) pair by one warp: thread s weighs split s, the weighted
 // partials are added split by split in order, as are the sums.  (Every thread weighing every split for each of its dims, one
-// load after the other: 9 us for 17 splits; this 5.)
+// load after the other: 9 us for 17 splits; this, the first rows requested along with the states, 3.3.)
 __global__ void attention_f32_merge_kernel(const float *__restrict__ scratch, uint16_t *__restrict__ out, KvLayer kv,
                                            LaneTable lanes_meta, int lanes, int q_heads, int head_width, int split_tokens,
                                            int max_splits) {
@@ -625,27 +625,38 @@ __global__ void attention_f32_merge_kernel(const float *__restrict__ scratch, ui
     const uint32_t tokens = tick + 1u < kv.capacity ? tick + 1u : kv.capacity;
     const int splits = min(static_cast<int>((tokens + split_tokens - 1) / split_tokens), max_splits), stride = head_width + 2;
     const float *base = scratch + static_cast<size_t>(pair) * max_splits * stride;
-    float maximum = -3.4028234663852886e38f;
-    for (int s = thread; s < splits; s += 32) maximum = fmaxf(maximum, base[static_cast<size_t>(s) * stride + head_width]);
+    constexpr int DIMS = 4, BATCH = 8;  // heads of at most 128; splits whose rows are in flight together
+    float part[BATCH][DIMS];
+    auto fetch = [&](int first) {
+#pragma unroll
+        for (int i = 0; i < BATCH; i++)
+#pragma unroll
+            for (int d = 0; d < DIMS; d++)
+                if (first + i < splits && thread + 32 * d < head_width) part[i][d] = base[static_cast<size_t>(first + i) * stride + thread + 32 * d];
+    };
+    float2 state = make_float2(-3.4028234663852886e38f, 0.0f);
+    if (thread < splits) state = *reinterpret_cast<const float2 *>(base + static_cast<size_t>(thread) * stride + head_width);
+    fetch(0);
+    float maximum = state.x;
+    for (int s = thread + 32; s < splits; s += 32) maximum = fmaxf(maximum, base[static_cast<size_t>(s) * stride + head_width]);
     maximum = warp_max(maximum);
-    constexpr int DIMS = 4;  // heads of at most 128
     float denominator = 0.0f, acc[DIMS] = {};
     for (int first = 0; first < splits; first += 32) {
-        float weight = 0.0f, sum = 0.0f;
-        if (first + thread < splits) {
-            const float *state = base + static_cast<size_t>(first + thread) * stride + head_width;
-            weight = expf(state[0] - maximum);
-            sum = state[1];
-        }
+        float weight = 0.0f;
+        if (first > 0 && first + thread < splits) state = *reinterpret_cast<const float2 *>(base + static_cast<size_t>(first + thread) * stride + head_width);
+        if (first + thread < splits) weight = expf(state.x - maximum);
         const int count = min(32, splits - first);
-#pragma unroll 4
-        for (int s = 0; s < count; s++) {
-            const float w = __shfl_sync(0xffffffffu, weight, s);
-            const float *part = base + static_cast<size_t>(first + s) * stride;
-            denominator = fmaf(__shfl_sync(0xffffffffu, sum, s), w, denominator);
+        for (int s = 0; s < count; s += BATCH) {
+            if (first + s > 0) fetch(first + s);
 #pragma unroll
-            for (int i = 0; i < DIMS; i++)
-                if (thread + 32 * i < head_width) acc[i] = fmaf(part[thread + 32 * i], w, acc[i]);
+            for (int i = 0; i < BATCH; i++) {
+                if (s + i >= count) break;
+                const float w = __shfl_sync(0xffffffffu, weight, s + i);
+                denominator = fmaf(__shfl_sync(0xffffffffu, state.y, s + i), w, denominator);
+#pragma unroll
+                for (int d = 0; d < DIMS; d++)
+                    if (thread + 32 * d < head_width) acc[d] = fmaf(part[i][d], w, acc[d]);
+            }
         }
     }
 #pragma unroll
@@ -782,30 +793,46 @@ __global__ void attention_merge_kernel(const float *__restrict__ scratch, uint16
     const uint32_t tokens = tick + 1u < kv.capacity ? tick + 1u : kv.capacity;
     const int splits = min(static_cast<int>((tokens + split_tokens - 1) / split_tokens), max_splits), stride = head_width + 2;
     const float *base = scratch + static_cast<size_t>(pair) * max_splits * stride;
-    float maximum = LOWEST;
-    for (int s = thread; s < splits; s += 32) maximum = fmaxf(maximum, base[static_cast<size_t>(s) * stride + head_width]);
+    // the first splits' states and rows are requested together: one trip to memory for contexts of a few splits
+    constexpr int BATCH = 8;
+    float2 part[BATCH][2];  // two dimensions per thread and 64 of the head
+    auto fetch = [&](int first) {
+#pragma unroll
+        for (int i = 0; i < BATCH; i++)
+#pragma unroll
+            for (int d = 0; d < 2; d++)
+                if (first + i < splits && 2 * thread + 64 * d < head_width)
+                    part[i][d] = reinterpret_cast<const float2 *>(base + static_cast<size_t>(first + i) * stride)[thread + 32 * d];
+    };
+    float2 state = make_float2(LOWEST, 0.0f);
+    if (thread < splits) state = *reinterpret_cast<const float2 *>(base + static_cast<size_t>(thread) * stride + head_width);
+    fetch(0);
+    float maximum = state.x;
+    for (int s = thread + 32; s < splits; s += 32) maximum = fmaxf(maximum, base[static_cast<size_t>(s) * stride + head_width]);
     maximum = warp_max(maximum);
     float denominator = 0.0f;
-    float2 acc[2] = {};  // two dimensions per thread and 64 of the head
+    float2 acc[2] = {};
     for (int first = 0; first < splits; first += 32) {
         float weight = 0.0f;
         if (first + thread < splits) {
-            const float2 state = *reinterpret_cast<const float2 *>(base + static_cast<size_t>(first + thread) * stride + head_width);
+            if (first > 0) state = *reinterpret_cast<const float2 *>(base + static_cast<size_t>(first + thread) * stride + head_width);
             weight = expf(state.x - maximum);
             denominator = fmaf(state.y, weight, denominator);
         }
         const int count = min(32, splits - first);
-#pragma unroll 4
-        for (int s = 0; s < count; s++) {
-            const float w = __shfl_sync(0xffffffffu, weight, s);
-            const float2 *part = reinterpret_cast<const float2 *>(base + static_cast<size_t>(first + s) * stride);
+        for (int s = 0; s < count; s += BATCH) {
+            if (first + s > 0) fetch(first + s);
 #pragma unroll
-            for (int i = 0; i < 2; i++)
-                if (2 * thread + 64 * i < head_width) {
-                    const float2 v = part[thread + 32 * i];
-                    acc[i].x = fmaf(v.x, w, acc[i].x);
-                    acc[i].y = fmaf(v.y, w, acc[i].y);
-                }
+            for (int i = 0; i < BATCH; i++) {
+                if (s + i >= count) break;
+                const float w = __shfl_sync(0xffffffffu, weight, s + i);
+#pragma unroll
+                for (int d = 0; d < 2; d++)
+                    if (2 * thread + 64 * d < head_width) {
+                        acc[d].x = fmaf(part[i][d].x, w, acc[d].x);
+                        acc[d].y = fmaf(part[i][d].y, w, acc[d].y);
+                    }
+            }
         }
     }
     denominator = warp_sum(denominator);
