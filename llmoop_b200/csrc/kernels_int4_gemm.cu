@@ -572,33 +572,52 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
 // magnitude of the row, then the conversion; a 16-byte piece of eight columns holds them in the order (0,4)(1,5)(2,6)
 // (3,7) the nibble pairs come out in, at its swizzled place in the 8-lane x 64-column atom.  With NORM the row is the
 // RMSNorm of x (rms_norm_bf16.comp.template:49-72), kept in shared memory between its two passes.
+// HELD: 16-byte pieces of the row per thread, kept in registers (0: any number, kept in shared memory or read again); the
+// norm's weights are nobody's output and are on their way while the kernel in front still runs (32 x 4096: 4.1 -> 2.7 us).
 constexpr int PREPARE_THREADS = 512;
-template <bool NORM>
+template <bool NORM, int HELD>
 __global__ void __launch_bounds__(PREPARE_THREADS) prepare_activations_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ weight, float eps,
                                                                              float weight_offset, uint8_t *__restrict__ out, float *__restrict__ factors, int lanes,
                                                                              int lane_blocks, int k) {
-    constexpr int WARPS = PREPARE_THREADS / 32;
+    constexpr int WARPS = PREPARE_THREADS / 32, REGISTERS = HELD > 0 ? HELD : 1;
     extern __shared__ __align__(16) uint4 normalised[];
     __shared__ float warp_sums[WARPS];
     __shared__ uint32_t warp_largest[WARPS];
     const int m = blockIdx.x, pieces = k >> 3;
+    uint4 held[REGISTERS], weights[REGISTERS];
+    auto each_piece = [&](auto body) {  // body(register, piece)
+        if (HELD > 0) {
+#pragma unroll
+            for (int i = 0; i < REGISTERS; i++)
+                if (static_cast<int>(threadIdx.x) + i * PREPARE_THREADS < pieces) body(i, static_cast<int>(threadIdx.x) + i * PREPARE_THREADS);
+        } else {
+            for (int p = threadIdx.x; p < pieces; p += PREPARE_THREADS) body(0, p);
+        }
+    };
     grid_launch_dependents();
+    if (NORM && HELD > 0) each_piece([&](int i, int p) { weights[i] = __ldg(reinterpret_cast<const uint4 *>(weight) + p); });
     grid_dependency_wait();
     const uint4 *row = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(m) * k);
     uint32_t largest = 0;
+    auto note = [&](const uint4 &v) {
+        const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) largest = max(largest, max((words[i] & 0x7FFFu), (words[i] >> 16) & 0x7FFFu));
+    };
     if (m < lanes) {
+        if (HELD > 0) each_piece([&](int i, int p) { held[i] = row[p]; });
         if (NORM) {
             float sum = 0.0f;
-            for (int p = threadIdx.x; p < pieces; p += PREPARE_THREADS) {
-                const uint4 v = row[p];
-                normalised[p] = v;
+            each_piece([&](int i, int p) {
+                const uint4 v = HELD > 0 ? held[i] : row[p];
+                if (HELD == 0) normalised[p] = v;
                 const uint32_t words[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    sum = fmaf(bf16_lo(words[i]), bf16_lo(words[i]), sum);
-                    sum = fmaf(bf16_hi(words[i]), bf16_hi(words[i]), sum);
+                for (int w = 0; w < 4; w++) {
+                    sum = fmaf(bf16_lo(words[w]), bf16_lo(words[w]), sum);
+                    sum = fmaf(bf16_hi(words[w]), bf16_hi(words[w]), sum);
                 }
-            }
+            });
             sum = warp_sum(sum);
             if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = sum;
             __syncthreads();
@@ -606,24 +625,18 @@ __global__ void __launch_bounds__(PREPARE_THREADS) prepare_activations_kernel(co
 #pragma unroll
             for (int w = 0; w < WARPS; w++) total += warp_sums[w];
             const float inv_rms = 1.0f / sqrtf(total * (1.0f / static_cast<float>(k)) + eps);
-            for (int p = threadIdx.x; p < pieces; p += PREPARE_THREADS) {
-                const uint4 v = normalised[p], w = reinterpret_cast<const uint4 *>(weight)[p];
+            each_piece([&](int i, int p) {
+                const uint4 v = HELD > 0 ? held[i] : normalised[p], w = HELD > 0 ? weights[i] : reinterpret_cast<const uint4 *>(weight)[p];
                 auto norm = [&](uint32_t value, uint32_t factor) {
                     return pack_bf16(bf16_lo(value) * inv_rms * (bf16_lo(factor) + weight_offset), bf16_hi(value) * inv_rms * (bf16_hi(factor) + weight_offset));
                 };
                 const uint4 y = make_uint4(norm(v.x, w.x), norm(v.y, w.y), norm(v.z, w.z), norm(v.w, w.w));
-                normalised[p] = y;
-                const uint32_t words[4] = {y.x, y.y, y.z, y.w};
-#pragma unroll
-                for (int i = 0; i < 4; i++) largest = max(largest, max((words[i] & 0x7FFFu), (words[i] >> 16) & 0x7FFFu));
-            }
+                if (HELD > 0) held[i] = y;
+                else normalised[p] = y;
+                note(y);
+            });
         } else {
-            for (int p = threadIdx.x; p < pieces; p += PREPARE_THREADS) {
-                const uint4 v = row[p];
-                const uint32_t words[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                for (int i = 0; i < 4; i++) largest = max(largest, max((words[i] & 0x7FFFu), (words[i] >> 16) & 0x7FFFu));
-            }
+            each_piece([&](int i, int p) { note(HELD > 0 ? held[i] : row[p]); });
         }
         largest = __reduce_max_sync(0xffffffffu, largest);
         if ((threadIdx.x & 31) == 0) warp_largest[threadIdx.x >> 5] = largest;
@@ -634,12 +647,12 @@ __global__ void __launch_bounds__(PREPARE_THREADS) prepare_activations_kernel(co
     const int exponent = max(static_cast<int>(largest >> 7), 16);
     const float factor = power_of_two(min(268 - exponent, 254));
     if (m < lanes && threadIdx.x == 0) factors[m] = power_of_two(max(exponent - 14, 1));
-    for (int p = threadIdx.x; p < pieces; p += PREPARE_THREADS) {
+    each_piece([&](int i, int p) {
         uint4 packed = make_uint4(0, 0, 0, 0);
         if (m < lanes) {
-            const uint4 v = NORM ? normalised[p] : row[p];
-            auto both = [&](uint32_t a, uint32_t b) {
-                const __half2 h = __floats2half2_rn(__uint_as_float(a) * factor, __uint_as_float(b) * factor);
+            const uint4 v = HELD > 0 ? held[i] : NORM ? normalised[p] : row[p];
+            auto both = [&](uint32_t lo, uint32_t hi) {
+                const __half2 h = __floats2half2_rn(__uint_as_float(lo) * factor, __uint_as_float(hi) * factor);
                 return *reinterpret_cast<const uint32_t *>(&h);
             };
             packed.x = both(v.x << 16, v.z << 16);
@@ -648,7 +661,13 @@ __global__ void __launch_bounds__(PREPARE_THREADS) prepare_activations_kernel(co
             packed.w = both(v.y & 0xffff0000u, v.w & 0xffff0000u);
         }
         *reinterpret_cast<uint4 *>(out + (static_cast<size_t>(p >> 3) * lane_blocks + (m >> 3)) * 1024 + (m & 7) * 128 + (((p & 7) ^ (m & 7)) * 16)) = packed;
-    }
+    });
+}
+template <bool NORM>
+auto prepare_kernel(int k) {
+    const int pieces = k / 8;
+    return pieces <= PREPARE_THREADS ? prepare_activations_kernel<NORM, 1> : pieces <= 2 * PREPARE_THREADS ? prepare_activations_kernel<NORM, 2>
+           : pieces <= 4 * PREPARE_THREADS ? prepare_activations_kernel<NORM, 4> : prepare_activations_kernel<NORM, 0>;
 }
 
 struct GemmPlan {
@@ -742,7 +761,7 @@ static float *activation_factors(void *prepared, int lanes, int k) {
 cudaError_t launch_prepare_activations(const uint16_t *x, void *prepared, int lanes, int k, cudaStream_t stream) {
     if (lanes <= 0) return cudaSuccess;
     const int padded = (lanes + 15) / 16 * 16;
-    return launch_dependent(prepare_activations_kernel<false>, dim3(padded), dim3(PREPARE_THREADS), 0, 1, stream, x, static_cast<const uint16_t *>(nullptr), 0.0f,
+    return launch_dependent(prepare_kernel<false>(k), dim3(padded), dim3(PREPARE_THREADS), 0, 1, stream, x, static_cast<const uint16_t *>(nullptr), 0.0f,
                             0.0f, static_cast<uint8_t *>(prepared), activation_factors(prepared, lanes, k), lanes, padded / 8, k);
 }
 
@@ -750,12 +769,13 @@ cudaError_t launch_rms_norm_prepared(const uint16_t *x, const uint16_t *weight, 
                                      cudaStream_t stream) {
     if (lanes <= 0) return cudaSuccess;
     const int padded = (lanes + 15) / 16 * 16;
-    const size_t smem = static_cast<size_t>(width) * 2;
+    auto kernel = prepare_kernel<true>(width);
+    const size_t smem = width / 8 <= 4 * PREPARE_THREADS ? 0 : static_cast<size_t>(width) * 2;
     if (smem > 48 * 1024) {
-        cudaError_t status = cudaFuncSetAttribute(prepare_activations_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (status != cudaSuccess) return status;
     }
-    return launch_dependent(prepare_activations_kernel<true>, dim3(padded), dim3(PREPARE_THREADS), smem, 1, stream, x, weight, eps, weight_offset,
+    return launch_dependent(kernel, dim3(padded), dim3(PREPARE_THREADS), smem, 1, stream, x, weight, eps, weight_offset,
                             static_cast<uint8_t *>(prepared), activation_factors(prepared, lanes, width), lanes, padded / 8, width);
 }
 
