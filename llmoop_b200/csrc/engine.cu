@@ -1250,11 +1250,20 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
                op.weights[0].group == 128;
     };
 
-    // Whether every reader of `signal` is an INT4 linear of one branch.
+    // Whether every reader of `signal` is an INT4 linear of one branch that finds it in the operand buffer: nothing that may
+    // prepare another signal there (an INT4 linear, a norm) stands between the operation before `after` and its last reader.
     auto only_int4_reads = [&](const std::string &signal, size_t after) {
         int readers = 0;
-        for (size_t i = after; i < plan.ops.size(); i++)
-            if (is_int4_single(plan.ops[i]) && plan.ops[i].inputs[0] == signal) readers++;
+        bool overwritten = false;
+        for (size_t i = after; i < plan.ops.size(); i++) {
+            const OpSpec &op = plan.ops[i];
+            if (is_int4_single(op) && op.inputs[0] == signal) {
+                if (overwritten) return false;
+                readers++;
+            } else {
+                overwritten |= op.kind == OpKind::RmsNorm || std::any_of(op.weights.begin(), op.weights.end(), [](const WeightRef &w) { return w.storage == TensorStorage::INT4_CT; });
+            }
+        }
         return readers > 0 && readers == consumers(signal, after);
     };
     // Whether `attention` reads exactly these rotated q and k, and nothing else reads that k.
