@@ -9,7 +9,8 @@
 // finished accumulator out while the other one fills.  Up to about 200 lanes the weight bytes are the bound (a 128256 x
 // 4096 table: 1.05 GB), beyond that the tensor pipe.  (The form this replaced - 64 lanes to a tile, operands copied by
 // all threads between two barriers per block - read that table for 32 lanes in 640 us.)
-// Waits are bounded; a wait that expires sets the error word, and the CTA still frees its tensor memory.
+// Waits are bounded; a wait that expires sets the error word, and the CTA still frees its tensor memory.  The unbounded wait
+// for the kernel in front comes before them in every role, so none of them counts that kernel's time.
 #include <cuda.h>
 
 #include <algorithm>
@@ -26,7 +27,7 @@ constexpr int ROWS = 128, BLOCK_K = 128;                 // weight rows per tile
 constexpr int THREADS = 256, MAX_STAGES = 6;
 constexpr uint32_t A_BYTES = ROWS * BLOCK_K * 2;
 constexpr size_t SMEM_LIMIT = 226 * 1024, CONTROL_BYTES = 256;
-constexpr unsigned int SPIN_LIMIT = 1u << 17;
+constexpr unsigned int SPIN_LIMIT = 1u << 22;  // tries of 1.5 us
 
 __device__ __forceinline__ uint64_t swizzled_descriptor(uint32_t shared_address) {  // K-major, 128-byte swizzle, 1024 bytes between 8-row atoms
     return static_cast<uint64_t>((shared_address & 0x3FFFFu) >> 4) | (1ull << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
@@ -164,6 +165,7 @@ __global__ void __launch_bounds__(THREADS, 1) linear_bf16_gemm_kernel(const __gr
         int stage = 0, round = 0;
         uint32_t parity = 0;
         bool alive = true;
+        grid_dependency_wait();
         for (int tile = blockIdx.x; tile < a.tiles && alive; tile += gridDim.x, round++) {
             const uint32_t accumulator = tmem + (round & 1) * acc_columns;
             if (!wait_barrier(acc_empty + (round & 1) * 8, static_cast<uint32_t>((round / 2 + 1) & 1), a.error_flag)) break;

@@ -22,7 +22,9 @@
 //              order of the 128-byte-swizzled shared-memory tiles: two bulk copies per group of 128 columns.
 // With ROW_TILES = 2 every activation byte read from L2 feeds two MMAs; stages of half a group make room for 160 lanes there.  K may be split over a cluster of CTAs whose
 // partial sums meet through distributed shared memory (shapes with too few tiles to fill the chip).
-// Waits are bounded; a wait that expires sets the error word, and the CTA still frees its tensor memory.
+// Waits are bounded; a wait that expires sets the error word, and the CTA still frees its tensor memory.  No bounded wait
+// counts the time of the kernel in front: every role passes the (unbounded) dependency wait before its first wait that
+// hangs on the activations, which only then are copied.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -38,7 +40,7 @@ namespace {
 
 template <int ROW_TILES>
 constexpr int gemm_threads() { return ROW_TILES * 256 + 64; }
-constexpr unsigned int GEMM_SPIN_LIMIT = 1u << 17;
+constexpr unsigned int GEMM_SPIN_LIMIT = 1u << 22;  // tries of 1.5 us
 constexpr int GEMM_MAX_B_STAGES = 8, GEMM_MAX_A_STAGES = 4;  // of 64 or 128 columns of K each
 constexpr size_t GEMM_SMEM_ONE = 225 * 1024, GEMM_SMEM_TWO = 111 * 1024;  // one or two CTAs per SM
 constexpr size_t GEMM_BARRIER_BYTES = 256, GEMM_TAIL_BYTES = GEMM_BARRIER_BYTES + 256 * sizeof(float);  // barriers, lane factors
@@ -306,11 +308,14 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
         // ring position of the item's group among the A stages, and the parity of its last release (the first round waits for none)
         int stage = set * PARTS;
         uint32_t parity = 1;
+        bool first_round = true;
         auto advance = [&](int by) {
             stage += by;
             if (stage >= a.a_stages) {
                 stage -= a.a_stages;
                 parity ^= 1;
+                if (first_round) grid_dependency_wait();  // from here on the MMAs release the stages
+                first_round = false;
             }
         };
         auto prepare = [&](auto raw) {
@@ -373,6 +378,7 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
         const uint64_t b_first = swizzled_descriptor(shared_address(smem)), b_half = static_cast<uint64_t>(n_lanes) * 8;  // descriptors count 16 bytes
         int stage_a = 0, stage_b = 0;
         uint32_t parity_a = 0, parity_b = 0;
+        grid_dependency_wait();
         for (int part = 0; part < own_groups * PARTS; part++) {
             if (!wait_barrier(b_full + stage_b * 8, parity_b, a.error_flag) || !wait_barrier(a_full + stage_a * 8, parity_a, a.error_flag)) {
                 alive = false;
