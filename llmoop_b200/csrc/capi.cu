@@ -1,6 +1,5 @@
 // extern "C" surface declared in include/nerve_b200.h: exception -> status + thread-local message.
 #include <cstring>
-#include <map>
 #include <mutex>
 #include <exception>
 #include <string>
@@ -74,6 +73,108 @@ void fill_snapshot(nerve_b200_stream_snapshot *out, const nerve::runtime::Stream
     copy_text(out->current_input_event_id, snapshot.current_input_event_id.value_or(""));
 }
 
+// The pool that the INT4 linears of more than eight lanes, at operator level, take the memory of their operand form from: their
+// callers lend none.  Set up by the first such call on a device.
+class OperatorDevice {
+public:
+    static cudaError_t current(OperatorDevice **out) {
+        int device = 0;
+        cudaError_t status = cudaGetDevice(&device);
+        if (status != cudaSuccess) return status;
+        if (device < 0 || device >= MAX_DEVICES) return cudaErrorInvalidDevice;
+        OperatorDevice &own = all()[device];
+        std::lock_guard<std::mutex> lock(own.mutex_);
+        status = own.set_up(device);
+        *out = &own;
+        return status;
+    }
+    // What the pools keep without a user goes back to their devices.
+    static void trim() {
+        for (int device = 0; device < MAX_DEVICES; device++) {
+            OperatorDevice &own = all()[device];
+            std::lock_guard<std::mutex> lock(own.mutex_);
+            if (own.pool_ != nullptr) cudaMemPoolTrimTo(own.pool_, 0);
+        }
+    }
+    // stream-ordered, safe with any number of streams and threads; what the pool keeps beyond 64 MB goes back to the device
+    // at the next synchronisation
+    cudaMemPool_t pool() const { return pool_; }
+
+private:
+    static constexpr int MAX_DEVICES = 64;
+    static OperatorDevice *all() {
+        static OperatorDevice devices[MAX_DEVICES];
+        return devices;
+    }
+    cudaError_t set_up(int device) {
+        if (pool_ != nullptr) return cudaSuccess;
+        // (the first call may come while its stream is being captured: none of this touches the stream)
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaError_t status = cudaThreadExchangeStreamCaptureMode(&mode);
+        if (status != cudaSuccess) return status;
+        status = allocate(device);
+        const cudaError_t restored = cudaThreadExchangeStreamCaptureMode(&mode);
+        return status != cudaSuccess ? status : restored;
+    }
+    cudaError_t allocate(int device) {
+        cudaMemPoolProps properties = {};
+        properties.allocType = cudaMemAllocationTypePinned;
+        properties.location.type = cudaMemLocationTypeDevice;
+        properties.location.id = device;
+        cudaMemPool_t pool = nullptr;
+        cudaError_t status = cudaMemPoolCreate(&pool, &properties);
+        if (status != cudaSuccess) return status;
+        uint64_t keep = uint64_t(64) << 20;
+        status = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (status != cudaSuccess) cudaMemPoolDestroy(pool);
+        else pool_ = pool;
+        return status;
+    }
+    std::mutex mutex_;
+    cudaMemPool_t pool_ = nullptr;
+};
+
+// The activations of an INT4 linear in the GEMM's operand form, from the pool and back to it in the stream's order.
+class PreparedActivations {
+public:
+    PreparedActivations(const OperatorDevice *device, const void *x, int32_t lanes, int32_t k, cudaStream_t stream) : stream_(stream) {
+        if (device == nullptr) return;
+        status_ = cudaMallocFromPoolAsync(&buffer_, int4_activation_bytes(lanes, k), device->pool(), stream);
+        if (status_ == cudaSuccess) status_ = launch_prepare_activations(static_cast<const uint16_t *>(x), buffer_, lanes, k, stream);
+    }
+    ~PreparedActivations() {
+        if (buffer_ != nullptr) cudaFreeAsync(buffer_, stream_);
+    }
+    PreparedActivations(const PreparedActivations &) = delete;
+    cudaError_t status() const { return status_; }
+    const void *get() const { return buffer_; }
+
+private:
+    cudaStream_t stream_;
+    void *buffer_ = nullptr;
+    cudaError_t status_ = cudaSuccess;
+};
+
+// body(device): `device` is set where the call takes memory of the pool.
+template <typename Body>
+int32_t linear_call(const char *name, bool takes_memory, Body body) {
+    return guarded([&] {
+        OperatorDevice *device = nullptr;
+        auto verify = [&](cudaError_t status) {
+            if (status != cudaSuccess) throw std::runtime_error(std::string(name) + ": " + cudaGetErrorString(status));
+        };
+        if (takes_memory) verify(OperatorDevice::current(&device));
+        verify(body(device));
+    });
+}
+
+// One reference less; the last one takes the model and the operator-level linears' unused memory with it.
+void release(nerve_b200_package *package) {
+    if (--package->references != 0) return;
+    delete package;
+    OperatorDevice::trim();
+}
+
 }  // namespace
 
 #pragma GCC visibility push(default)
@@ -110,7 +211,7 @@ int32_t nerve_b200_package_mount(const char *path, const nerve_b200_mount_option
 int32_t nerve_b200_package_unmount(nerve_b200_package *package) {
     return guarded([&] {
         require(package != nullptr, "nerve_b200_package_unmount: null package");
-        if (--package->references == 0) delete package;
+        release(package);
     });
 }
 
@@ -180,7 +281,7 @@ int32_t nerve_b200_engine_destroy(nerve_b200_engine *engine) {
         nerve_b200_package *package = engine->package;
         engine->engine.reset();
         delete engine;
-        if (--package->references == 0) delete package;
+        release(package);
     });
 }
 
@@ -469,85 +570,33 @@ int32_t nerve_b200_debug_target_logits(nerve_b200_engine *engine, int64_t stream
 
 // ---- operator-level entry points
 
-namespace {
-
-// The INT4 linears of more than eight lanes read their activations in the GEMM's operand form; the callers of the
-// operator-level entry points lend no scratch for it, so it comes stream-ordered from a pool of this library's own per
-// device: safe with any number of streams and threads, a call costs no device allocation once the pool is warm, and
-// what the pool keeps beyond 64 MB goes back to the device at the next synchronisation.
-class PreparedActivations {
-public:
-    PreparedActivations(const void *x, int32_t lanes, int32_t n, int32_t k, cudaStream_t stream) : stream_(stream) {
-        if (!linear_int4_gemm_supported(lanes, n, k)) return;
-        cudaMemPool_t pool = nullptr;
-        status_ = device_pool(&pool);
-        if (status_ == cudaSuccess) status_ = cudaMallocFromPoolAsync(&buffer_, int4_activation_bytes(lanes, k), pool, stream);
-        if (status_ == cudaSuccess) status_ = launch_prepare_activations(static_cast<const uint16_t *>(x), buffer_, lanes, k, stream);
-    }
-    ~PreparedActivations() {
-        if (buffer_ != nullptr) cudaFreeAsync(buffer_, stream_);
-    }
-    PreparedActivations(const PreparedActivations &) = delete;
-    cudaError_t status() const { return status_; }
-    const void *get() const { return buffer_; }
-
-private:
-    static cudaError_t device_pool(cudaMemPool_t *out) {
-        static std::mutex mutex;
-        static std::map<int, cudaMemPool_t> pools;
-        int device = 0;
-        cudaError_t status = cudaGetDevice(&device);
-        if (status != cudaSuccess) return status;
-        std::lock_guard<std::mutex> lock(mutex);
-        auto found = pools.find(device);
-        if (found == pools.end()) {
-            cudaMemPoolProps properties = {};
-            properties.allocType = cudaMemAllocationTypePinned;
-            properties.location.type = cudaMemLocationTypeDevice;
-            properties.location.id = device;
-            cudaMemPool_t pool = nullptr;
-            status = cudaMemPoolCreate(&pool, &properties);
-            if (status != cudaSuccess) return status;
-            uint64_t keep = uint64_t(64) << 20;
-            status = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-            if (status != cudaSuccess) return status;
-            found = pools.emplace(device, pool).first;
-        }
-        *out = found->second;
-        return cudaSuccess;
-    }
-    cudaStream_t stream_;
-    void *buffer_ = nullptr;
-    cudaError_t status_ = cudaSuccess;
-};
-
-}  // namespace
-
 int32_t nerve_b200_op_linear_int4(const void *x, const void *qweight, const void *scales, void *y, const void *residual, int32_t lanes,
                                   int32_t n, int32_t k, int32_t group, void *stream) {
-    const PreparedActivations prepared(x, group == 128 ? lanes : 0, n, k, static_cast<cudaStream_t>(stream));
-    if (prepared.status() != cudaSuccess) return cuda_status(prepared.status(), "nerve_b200_op_linear_int4 (activations)");
-    return cuda_status(launch_linear_int4(static_cast<const uint16_t *>(x), prepared.get(), static_cast<const uint32_t *>(qweight),
-                                          static_cast<const uint16_t *>(scales), static_cast<uint16_t *>(y),
-                                          static_cast<const uint16_t *>(residual), lanes, n, k, group,
-                                          residual ? EPILOGUE_RESIDUAL_ROUNDED : EPILOGUE_BF16, static_cast<cudaStream_t>(stream)),
-                       "nerve_b200_op_linear_int4");
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    return linear_call("nerve_b200_op_linear_int4", group == 128 && linear_int4_gemm_supported(lanes, n, k), [&](const OperatorDevice *device) {
+        const PreparedActivations prepared(device, x, lanes, k, st);
+        if (prepared.status() != cudaSuccess) return prepared.status();
+        return launch_linear_int4(static_cast<const uint16_t *>(x), prepared.get(), static_cast<const uint32_t *>(qweight),
+                                  static_cast<const uint16_t *>(scales), static_cast<uint16_t *>(y), static_cast<const uint16_t *>(residual), lanes, n, k,
+                                  group, residual ? EPILOGUE_RESIDUAL_ROUNDED : EPILOGUE_BF16, st);
+    });
 }
 
 int32_t nerve_b200_op_linear_int4_silu_pair(const void *x, const void *gate_q, const void *gate_s, const void *up_q, const void *up_s,
                                             void *y, int32_t lanes, int32_t n, int32_t k, void *stream) {
-    const PreparedActivations prepared(x, lanes, n, k, static_cast<cudaStream_t>(stream));
-    if (prepared.status() != cudaSuccess) return cuda_status(prepared.status(), "nerve_b200_op_linear_int4_silu_pair (activations)");
-    return cuda_status(launch_linear_int4_silu_pair(static_cast<const uint16_t *>(x), prepared.get(), static_cast<const uint32_t *>(gate_q),
-                                                    static_cast<const uint16_t *>(gate_s), static_cast<const uint32_t *>(up_q),
-                                                    static_cast<const uint16_t *>(up_s), static_cast<uint16_t *>(y), lanes, n, k,
-                                                    static_cast<cudaStream_t>(stream)),
-                       "nerve_b200_op_linear_int4_silu_pair");
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    return linear_call("nerve_b200_op_linear_int4_silu_pair", linear_int4_gemm_supported(lanes, n, k), [&](const OperatorDevice *device) {
+        const PreparedActivations prepared(device, x, lanes, k, st);
+        if (prepared.status() != cudaSuccess) return prepared.status();
+        return launch_linear_int4_silu_pair(static_cast<const uint16_t *>(x), prepared.get(), static_cast<const uint32_t *>(gate_q),
+                                            static_cast<const uint16_t *>(gate_s), static_cast<const uint32_t *>(up_q),
+                                            static_cast<const uint16_t *>(up_s), static_cast<uint16_t *>(y), lanes, n, k, st);
+    });
 }
 
 int32_t nerve_b200_op_linear_bf16(const void *x, const void *w, void *y, const void *residual, int32_t lanes, int32_t n, int32_t k,
                                   int32_t to_f32, float scale, void *stream) {
-    int epilogue = to_f32 ? EPILOGUE_F32_SCALED : (residual ? EPILOGUE_RESIDUAL_ROUNDED : EPILOGUE_BF16);
+    const int epilogue = to_f32 ? EPILOGUE_F32_SCALED : (residual ? EPILOGUE_RESIDUAL_ROUNDED : EPILOGUE_BF16);
     return cuda_status(launch_linear_bf16(static_cast<const uint16_t *>(x), static_cast<const uint16_t *>(w), y,
                                           static_cast<const uint16_t *>(residual), lanes, n, k, epilogue, scale,
                                           static_cast<cudaStream_t>(stream)),
