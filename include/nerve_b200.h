@@ -243,10 +243,14 @@ int32_t nerve_b200_debug_target_logits(nerve_b200_engine *engine, int64_t stream
 /* ---- operator-level entry points (device pointers; bf16 activations [lanes][width]) -----------
  * One per shader family on the path; `stream` is a cudaStream_t passed as void* (NULL = default stream).
  *
+ * The linears of more than eight lanes (INT4 and, where k is a multiple of 128, bf16) run kernels with bounded waits.
+ * The calls are asynchronous: if such a wait ever expires, that call's outputs are incomplete and the NEXT such call on
+ * the device fails, once, with a message that says so, and does nothing else.
  * The INT4 linears of more than eight lanes take device memory for their activations (2 bytes per lane, rounded up to a
  * multiple of 16, and column) from a pool that the library keeps per device: stream-ordered, safe with any number of
  * threads and streams, capturable (the graph then owns the memory), at most 64 MB of it kept between calls; unmounting a
- * package gives the unused part back.  The first such call on a device creates the pool.  Callers that must not allocate device memory stay at eight lanes, which take nothing.
+ * package gives the unused part back.  The first such call on a device creates the pool and four bytes of pinned host
+ * memory.  Callers that must not allocate device memory stay at eight lanes, which take nothing.
  */
 /* linear_int4_ct.comp.template:80-150 (+ residual add of add_bf16.comp.template when residual != NULL). */
 int32_t nerve_b200_op_linear_int4(const void *x_device, const void *qweight_device, const void *scales_device,

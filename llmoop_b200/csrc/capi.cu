@@ -73,8 +73,8 @@ void fill_snapshot(nerve_b200_stream_snapshot *out, const nerve::runtime::Stream
     copy_text(out->current_input_event_id, snapshot.current_input_event_id.value_or(""));
 }
 
-// The pool that the INT4 linears of more than eight lanes, at operator level, take the memory of their operand form from: their
-// callers lend none.  Set up by the first such call on a device.
+// What the operator-level linears of more than eight lanes need on a device and their callers do not lend, set up by the first
+// such call there: a pool for the INT4 GEMM's operand form, and the word a kernel whose bounded wait expired leaves behind.
 class OperatorDevice {
 public:
     static cudaError_t current(OperatorDevice **out) {
@@ -99,6 +99,10 @@ public:
     // stream-ordered, safe with any number of streams and threads; what the pool keeps beyond 64 MB goes back to the device
     // at the next synchronisation
     cudaMemPool_t pool() const { return pool_; }
+    // The kernels' error word, in mapped host memory: read without a synchronisation.  Whether an earlier call's kernel has set it;
+    // reported once.
+    int *error_word() const { return device_word_; }
+    bool take_error() { return __atomic_exchange_n(host_word_, 0, __ATOMIC_ACQ_REL) != 0; }
 
 private:
     static constexpr int MAX_DEVICES = 64;
@@ -117,12 +121,22 @@ private:
         return status != cudaSuccess ? status : restored;
     }
     cudaError_t allocate(int device) {
+        cudaError_t status = cudaSuccess;
+        if (host_word_ == nullptr) {
+            int *word = nullptr;
+            status = cudaHostAlloc(reinterpret_cast<void **>(&word), sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
+            if (status != cudaSuccess) return status;
+            *word = 0;
+            host_word_ = word;
+        }
+        status = cudaHostGetDevicePointer(reinterpret_cast<void **>(&device_word_), host_word_, 0);
+        if (status != cudaSuccess) return status;
         cudaMemPoolProps properties = {};
         properties.allocType = cudaMemAllocationTypePinned;
         properties.location.type = cudaMemLocationTypeDevice;
         properties.location.id = device;
         cudaMemPool_t pool = nullptr;
-        cudaError_t status = cudaMemPoolCreate(&pool, &properties);
+        status = cudaMemPoolCreate(&pool, &properties);
         if (status != cudaSuccess) return status;
         uint64_t keep = uint64_t(64) << 20;
         status = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
@@ -132,6 +146,7 @@ private:
     }
     std::mutex mutex_;
     cudaMemPool_t pool_ = nullptr;
+    int *host_word_ = nullptr, *device_word_ = nullptr;
 };
 
 // The activations of an INT4 linear in the GEMM's operand form, from the pool and back to it in the stream's order.
@@ -155,15 +170,20 @@ private:
     cudaError_t status_ = cudaSuccess;
 };
 
-// body(device): `device` is set where the call takes memory of the pool.
+// body(device): `device` is set where the call runs a kernel of bounded waits.
 template <typename Body>
-int32_t linear_call(const char *name, bool takes_memory, Body body) {
+int32_t linear_call(const char *name, bool bounded_waits, Body body) {
     return guarded([&] {
         OperatorDevice *device = nullptr;
         auto verify = [&](cudaError_t status) {
             if (status != cudaSuccess) throw std::runtime_error(std::string(name) + ": " + cudaGetErrorString(status));
         };
-        if (takes_memory) verify(OperatorDevice::current(&device));
+        if (bounded_waits) {
+            verify(OperatorDevice::current(&device));
+            if (device->take_error())
+                throw std::runtime_error(std::string(name) + ": an earlier operator-level linear on this device gave up waiting on its copy pipeline and left outputs "
+                                                             "unwritten; this call has done nothing");
+        }
         verify(body(device));
     });
 }
@@ -578,7 +598,7 @@ int32_t nerve_b200_op_linear_int4(const void *x, const void *qweight, const void
         if (prepared.status() != cudaSuccess) return prepared.status();
         return launch_linear_int4(static_cast<const uint16_t *>(x), prepared.get(), static_cast<const uint32_t *>(qweight),
                                   static_cast<const uint16_t *>(scales), static_cast<uint16_t *>(y), static_cast<const uint16_t *>(residual), lanes, n, k,
-                                  group, residual ? EPILOGUE_RESIDUAL_ROUNDED : EPILOGUE_BF16, st);
+                                  group, residual ? EPILOGUE_RESIDUAL_ROUNDED : EPILOGUE_BF16, st, device != nullptr ? device->error_word() : nullptr);
     });
 }
 
@@ -590,17 +610,18 @@ int32_t nerve_b200_op_linear_int4_silu_pair(const void *x, const void *gate_q, c
         if (prepared.status() != cudaSuccess) return prepared.status();
         return launch_linear_int4_silu_pair(static_cast<const uint16_t *>(x), prepared.get(), static_cast<const uint32_t *>(gate_q),
                                             static_cast<const uint16_t *>(gate_s), static_cast<const uint32_t *>(up_q),
-                                            static_cast<const uint16_t *>(up_s), static_cast<uint16_t *>(y), lanes, n, k, st);
+                                            static_cast<const uint16_t *>(up_s), static_cast<uint16_t *>(y), lanes, n, k, st,
+                                            device != nullptr ? device->error_word() : nullptr);
     });
 }
 
 int32_t nerve_b200_op_linear_bf16(const void *x, const void *w, void *y, const void *residual, int32_t lanes, int32_t n, int32_t k,
                                   int32_t to_f32, float scale, void *stream) {
     const int epilogue = to_f32 ? EPILOGUE_F32_SCALED : (residual ? EPILOGUE_RESIDUAL_ROUNDED : EPILOGUE_BF16);
-    return cuda_status(launch_linear_bf16(static_cast<const uint16_t *>(x), static_cast<const uint16_t *>(w), y,
-                                          static_cast<const uint16_t *>(residual), lanes, n, k, epilogue, scale,
-                                          static_cast<cudaStream_t>(stream)),
-                       "nerve_b200_op_linear_bf16");
+    return linear_call("nerve_b200_op_linear_bf16", linear_bf16_gemm_supported(lanes, n, k), [&](const OperatorDevice *device) {
+        return launch_linear_bf16(static_cast<const uint16_t *>(x), static_cast<const uint16_t *>(w), y, static_cast<const uint16_t *>(residual), lanes, n, k,
+                                  epilogue, scale, static_cast<cudaStream_t>(stream), device != nullptr ? device->error_word() : nullptr);
+    });
 }
 
 int32_t nerve_b200_op_rms_norm(const void *x, const void *weight, void *y, int32_t lanes, int32_t width, float eps, float weight_offset,

@@ -47,7 +47,7 @@ __device__ __forceinline__ bool wait_barrier(uint32_t barrier, uint32_t parity, 
             : "memory");
         if (done) return true;
         if (++spins > SPIN_LIMIT) {
-            if (error_flag != nullptr) atomicExch(error_flag, 3);
+            if (error_flag != nullptr) *static_cast<volatile int *>(error_flag) = 3;  // (may be mapped host memory)
             return false;
         }
     }
