@@ -144,7 +144,7 @@ struct GemmArgs {
     int ns[3];
     int first_tile[4];         // ... matrix b owns the 128-row tiles first_tile[b] .. first_tile[b + 1] - 1
     const uint16_t *residual;
-    int lanes, lane_blocks, tile_lanes, k, epilogue, silu;
+    int lanes, lane_blocks, tile_lanes, k, epilogue, silu, paired;
     float scale;
     int *error_flag;
     int a_stages, b_stages, raw_stages;
@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(gemm_threads<ROW_TILES>(), ROW_TILES == 1 ? 2 
             }
             return sum;
         };
-        const bool whole = (n & 1) == 0;  // both rows exist and their outputs share an aligned word
+        const bool whole = a.paired && (n & 1) == 0;  // both rows exist and their outputs share an aligned word
         const bool second_row = row + 1 < n;
         const int step = WARPS * 32 / pairs;
         constexpr int BATCH = 8;
@@ -815,6 +815,9 @@ cudaError_t launch_linear_int4_gemm(const void *prepared, int branches, const ui
     args.k = k;
     args.epilogue = epilogue;
     args.silu = silu ? 1 : 0;
+    uintptr_t addresses = reinterpret_cast<uintptr_t>(residual);
+    for (int b = 0; b < branches; b++) addresses |= reinterpret_cast<uintptr_t>(ys[b]);
+    args.paired = addresses % 4 == 0 ? 1 : 0;
     args.scale = scale;
     args.error_flag = error_flag;
     args.a_stages = plan.a_stages;
