@@ -2224,6 +2224,7 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
         std::vector<uint32_t> generated;
         bool closing = false;  // all but its event's closing tick has run
     };
+    std::vector<Work> works;     // this step's activations
     std::vector<Work> deferred;  // closing ticks that share the next pass over the weights
     auto note_generated = [](Work &work) {
         if (work.stream->active == nullptr) return;
@@ -2240,6 +2241,7 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
             report.max_batch_width = std::max<uint64_t>(report.max_batch_width, batch.size());
         }
     };
+    try {
     while (true) {
         if (max_batches && report.batch_count >= max_batches) {
             if (deferred.empty()) {
@@ -2286,7 +2288,6 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
             scheduled = scheduler_.schedule_step(budget).activations;
         }
         if (scheduled.empty() && deferred.empty()) break;
-        std::vector<Work> works;
         works.reserve(scheduled.size() + deferred.size());
         for (runtime::Activation &activation : scheduled) {
             Stream &s = stream(std::stoll(activation.stream_id));
@@ -2296,7 +2297,6 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
         }
         for (Work &work : deferred) works.push_back(std::move(work));
         deferred.clear();
-        try {
         // 2. prefill chunks, as many streams' in one pass as the lanes allow
         struct Pending {
             Work *work;
@@ -2438,6 +2438,7 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
             Stream &s = *work.stream;
             if (work.closing && s.active != nullptr) {
                 deferred.push_back(std::move(work));
+                work.stream = nullptr;
                 continue;
             }
             runtime::ActivationOutcome outcome;
@@ -2446,31 +2447,34 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
             outcome.processed_state_activation_count = static_cast<size_t>(s.next_tick - work.start_tick);
             scheduler_.complete_activation(work.activation.id, outcome);
         }
-        } catch (...) {
-            // A batch failed and was discarded: its streams stand where they stood.  Activations that did run are
-            // completed (an event that still owes its closing tick gets it as a control step of the next run), the
-            // others are carried into the next run, which repeats them before it asks the scheduler for more.
-            for (Work &work : works) {
-                Stream &s = *work.stream;
-                note_generated(work);
-                const bool ran = s.next_tick != work.start_tick || !work.generated.empty() || s.active == nullptr;
-                if (!ran) {
-                    carried_activations_.push_back(work.activation);
-                    continue;
-                }
-                runtime::ActivationOutcome outcome;
-                outcome.generated_token_ids = work.generated;
-                const bool owes_closing_tick = s.active && s.active->has_feedback && s.active->feedback_closes;
-                outcome.continue_generation = s.active != nullptr && !owes_closing_tick;
-                outcome.processed_state_activation_count = static_cast<size_t>(s.next_tick - work.start_tick);
-                if (owes_closing_tick) s.detached = true;
-                try {
-                    scheduler_.complete_activation(work.activation.id, outcome);
-                } catch (...) {
-                }
+        works.clear();
+    }
+    } catch (...) {
+        // A batch failed and was discarded: its streams stand where they stood.  Activations that did run are
+        // completed (an event that still owes its closing tick gets it as a control step of the next run), the
+        // others are carried into the next run, which repeats them before it asks the scheduler for more.
+        for (Work &work : deferred) works.push_back(std::move(work));
+        for (Work &work : works) {
+            if (work.stream == nullptr) continue;  // moved on to the closing ticks
+            Stream &s = *work.stream;
+            note_generated(work);
+            const bool ran = s.next_tick != work.start_tick || !work.generated.empty() || s.active == nullptr;
+            if (!ran) {
+                carried_activations_.push_back(work.activation);
+                continue;
             }
-            throw;
+            runtime::ActivationOutcome outcome;
+            outcome.generated_token_ids = work.generated;
+            const bool owes_closing_tick = s.active && s.active->has_feedback && s.active->feedback_closes;
+            outcome.continue_generation = s.active != nullptr && !owes_closing_tick;
+            outcome.processed_state_activation_count = static_cast<size_t>(s.next_tick - work.start_tick);
+            if (owes_closing_tick) s.detached = true;
+            try {
+                scheduler_.complete_activation(work.activation.id, outcome);
+            } catch (...) {
+            }
         }
+        throw;
     }
     cuda_check(cudaEventRecord(run_end_, cuda_stream_), "event record");
     cuda_check(cudaMemcpyAsync(host_records_, kernel_error_.ptr, sizeof(int), cudaMemcpyDeviceToHost, cuda_stream_), "kernel status readback");

@@ -1,0 +1,70 @@
+"""Closing ticks that wait for the next step's batch (an event's last token is fed back together with the other streams'
+next windows): with a limit on the batches of a run, with windows of different lengths in one cycle, and when the step that
+should have run them fails."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def package(tmp_path_factory):
+    from llmoop_b200.package_writer import write_package
+    from llmoop_b200.synth import ModelSpec
+
+    spec = ModelSpec(name="closing_ticks", hidden=512, layers=3, q_heads=8, kv_heads=2, head_dim=64, ffn=1408, vocab=1024, max_positions=512,
+                     quant="int4", std=0.01, seed=7)
+    directory = tmp_path_factory.mktemp("packages") / spec.name
+    write_package(spec, directory)
+    return directory, spec
+
+
+def _mount(directory):
+    import llmoop_b200 as nb
+
+    mounted = nb.Package(directory, capacity_tokens=128, page_tokens=16, max_streams=4, max_lanes=64, verify_level=0)
+    return nb.Engine(mounted), mounted
+
+
+def test_failed_step_keeps_the_closing_tick(package):
+    """Two streams finish their events in one step; the callback stops one of them, whose closing tick then is a control step
+    of its own, and arms a barrier timeout for it.  The other stream, whose closing tick waited for the batch behind, must
+    still take its next event."""
+    import llmoop_b200 as nb
+
+    directory, spec = package
+    rng = np.random.default_rng(8)
+    prompts = [[int(t) for t in rng.integers(0, spec.vocab, size=4)] for _ in range(2)]
+    engine, mounted = _mount(directory)
+
+    def generate(stream, with_failure):
+        engine.add_stream(stream)
+        engine.enqueue_input_event(stream, prompts[0], 3)
+        tokens = []
+        if with_failure:
+            engine.add_stream(9)
+            engine.enqueue_input_event(9, prompts[1], 3)
+
+            def on_output(sid, token, tick, index):
+                if sid == stream:
+                    tokens.append(token)
+                elif index == 2:
+                    engine.stop_stream_after_current(9)
+                    engine.inject_barrier_timeouts(1)
+
+            with pytest.raises(nb.NerveError, match="gave up waiting at a grid barrier"):
+                engine.run_until_idle(on_output=on_output)
+        else:
+            tokens += [token for _, token, _, _ in engine.run_until_idle()[0]]
+        engine.enqueue_input_event(stream, prompts[1], 4)
+        outputs, _ = engine.run_until_idle()
+        tokens += [token for sid, token, _, _ in outputs if sid == stream]
+        return tokens, engine.stream_tick(stream)
+
+    want = generate(1, False)
+    assert len(want[0]) == 7 and want[1] == 4 + 3 + 4 + 4
+    assert generate(2, True) == want
+    assert engine.stream_tick(9) == 4 + 3 and engine.snapshot()["idle"]  # its closing tick has run, too
+    engine.close()
+    mounted.unmount()
