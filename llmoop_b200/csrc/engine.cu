@@ -2374,6 +2374,7 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
         std::vector<Stream *> single;
         for (Work &work : works) {
             if (work.closing) {
+                if (work.stream->active == nullptr) continue;  // its closing tick has run as a control step
                 if (work.stream->k > 0 && model_->plan().has_draft) speculative[0].push_back(Window{work.stream, 0});
                 else single.push_back(work.stream);
                 continue;

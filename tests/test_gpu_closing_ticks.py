@@ -68,3 +68,30 @@ def test_failed_step_keeps_the_closing_tick(package):
     assert engine.stream_tick(9) == 4 + 3 and engine.snapshot()["idle"]  # its closing tick has run, too
     engine.close()
     mounted.unmount()
+
+
+@pytest.mark.parametrize("drafts", [0, 2])
+def test_stopping_a_stream_at_its_last_token(package, drafts):
+    """A callback stops a stream whose event it has just seen the last token of: the closing tick runs as a control step, once,
+    the run reports that the scheduler had given the activation up, and both streams take their next events."""
+    import llmoop_b200 as nb
+
+    directory, spec = package
+    rng = np.random.default_rng(9)
+    prompts = [[int(t) for t in rng.integers(0, spec.vocab, size=4)] for _ in range(2)]
+    engine, mounted = _mount(directory)
+    for stream in (1, 2):
+        engine.add_stream(stream, speculative_draft_tokens=drafts)
+        engine.enqueue_input_event(stream, prompts[0], 3)
+    with pytest.raises(nb.NerveError, match="activation"):
+        engine.run_until_idle(on_output=lambda sid, token, tick, index: engine.stop_stream_after_current(2) if sid == 2 and index == 2 else None)
+    engine.run_until_idle()
+    assert [engine.stream_tick(stream) for stream in (1, 2)] == [7, 7]
+    for stream in (1, 2):
+        engine.enqueue_input_event(stream, prompts[1], 3)
+    outputs, _ = engine.run_until_idle()
+    tokens = [[token for sid, token, _, _ in outputs if sid == stream] for stream in (1, 2)]
+    assert tokens[0] == tokens[1] and len(tokens[0]) == 3
+    assert [engine.stream_tick(stream) for stream in (1, 2)] == [14, 14]
+    engine.close()
+    mounted.unmount()
