@@ -2258,18 +2258,19 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
             for (auto &entry : streams_) {
                 Stream &s = entry.second;
                 if (!s.detached) continue;
+                if (s.active && s.active->has_feedback) {
+                    closing.push_back(&s);  // stays detached until the tick has run: a batch that fails is repeated by the next run
+                    continue;
+                }
                 s.detached = false;
                 if (!s.active) continue;
-                if (s.active->has_feedback) {
-                    closing.push_back(&s);
-                } else {
-                    s.active.reset();
-                    s.completed_events++;
-                }
+                s.active.reset();
+                s.completed_events++;
             }
             if (!closing.empty()) {
                 uint64_t start = now_ns();
                 run_ticks_in_batches(closing);
+                for (Stream *s : closing) s->detached = false;
                 report.decode_ns += now_ns() - start;
             }
         }

@@ -95,3 +95,26 @@ def test_stopping_a_stream_at_its_last_token(package, drafts):
     assert [engine.stream_tick(stream) for stream in (1, 2)] == [14, 14]
     engine.close()
     mounted.unmount()
+
+
+def test_failed_control_step_is_repeated(package):
+    """A stream is stopped between two runs and the batch of its closing tick fails: the next run repeats it, and the stream
+    takes its next event."""
+    import llmoop_b200 as nb
+
+    directory, spec = package
+    prompt = [int(t) for t in np.random.default_rng(10).integers(0, spec.vocab, size=4)]
+    engine, mounted = _mount(directory)
+    engine.add_stream(1)
+    engine.enqueue_input_event(1, prompt, 8)
+    first, _ = engine.run(2)
+    emitted = len(first)
+    engine.stop_stream_after_current(1)
+    engine.inject_barrier_timeouts(1)
+    with pytest.raises(nb.NerveError, match="gave up waiting at a grid barrier"):
+        engine.run_until_idle()
+    engine.enqueue_input_event(1, prompt, 3)
+    outputs, _ = engine.run_until_idle()
+    assert len(outputs) == 3 and engine.stream_tick(1) == 4 + emitted + 4 + 3
+    engine.close()
+    mounted.unmount()
