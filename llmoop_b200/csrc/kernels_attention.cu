@@ -32,14 +32,16 @@ constexpr float LOWEST = -3.4028234663852886e38f;
 // A CTA serves ROW_WARPS x 16 query rows of one (stream, kv head) - row r is query head r % group of the stream's lane
 // r / group, so the query heads that share a kv head share its K/V tiles - over one split of the context.  K and V
 // tiles of 64 tokens go through two shared-memory stages (cp.async one tile ahead, the tokens' page offsets two tiles
-// ahead), Q stays in registers; Q.K^T and P.V run on mma.sync bf16 with f32 sums.  The probabilities enter P.V as a
-// bf16 pair hi + lo, so that they are not rounded to eight bits.
+// ahead), Q stays in registers; Q.K^T and P.V run on mma.sync bf16 with f32 sums.  The probabilities enter P.V as three
+// bf16 terms, which hold all 24 bits of their f32 value, and the sums over the tiles are f32 multiply-adds: the error
+// against 64 bits, before the final rounding, is 2.2e-7 to 3.1e-7 of the output (32 lanes at 550 tokens .. 713 at 8713),
+// where scalar f32 products and sums leave 2.7e-7 to 1.2e-6, and two terms with one running sum left 1.6e-6 to 1.0e-5.
 // TOKEN_WARPS warps share a row tile's context: each takes 64 / TOKEN_WARPS tokens of every tile with a softmax of its
 // own, and they merge at the end.  Prefill chunks (many rows per stream) run 8 x 1 warps; verify and draft batches
 // (few rows, many tokens) 1 or 2 x 4, where four warps per row tile hide the tile's latency.
-// What bounds it: prefill the legacy tensor path (three MMAs per 16 x 8 x 16 of K or V), decode the KV bytes.
-// (One scalar f32 product per thread and token, the form this replaced, took 4.5 ms per 8B layer for 713 lanes at an
-// 8700-token context; this takes 0.5 ms.)
+// What bounds it: prefill the legacy tensor path (four MMAs per 16 x 8 x 16 of K and V), decode the KV bytes.
+// (One scalar f32 product per thread and token, the form this replaced, took 4.8 ms per 8B layer for 713 lanes at an
+// 8713-token context; this takes 0.74 ms, with two terms it took 0.55.)
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -83,7 +85,7 @@ constexpr size_t attention_smem() {
     return tiles > merge ? tiles : merge;
 }
 
-// The verify form of 32 rows takes two CTAs per SM (128 registers, 56 bytes of spills): it waits for its K and V more than
+// The verify form of 32 rows takes two CTAs per SM (128 registers, 76 bytes of spills): it waits for its K and V more than
 // it multiplies, and 32 streams x 8 kv heads x splits are several waves of one CTA per SM (44 -> 35 us per launch).
 template <int HD, int ROW_WARPS, int TOKEN_WARPS>
 __global__ void __launch_bounds__(ROW_WARPS *TOKEN_WARPS * 32, ROW_WARPS * TOKEN_WARPS == 8 && TOKEN_WARPS > 1 ? 2 : 1) attention_tile_kernel(const __grid_constant__ AttentionArgs a) {
@@ -242,32 +244,42 @@ __global__ void __launch_bounds__(ROW_WARPS *TOKEN_WARPS * 32, ROW_WARPS * TOKEN
                     }
                 row_sum[h] = row_sum[h] * factor[h] + sum;  // this thread's columns; added up over the four threads in the end
             }
+            // p = hi + mid + lo, the 24 bits of its f32 value; a tile's products add up from zero, the smallest terms first, and
+            // join the row's sum by one multiply-add, which rounds to nearest where the tensor core's running sum truncates
+            uint32_t p[3][TOKENS / 16][4];
 #pragma unroll
-            for (int d = 0; d < D_TILES; d++) {
-                acc[d][0] *= factor[0];
-                acc[d][1] *= factor[0];
-                acc[d][2] *= factor[1];
-                acc[d][3] *= factor[1];
-            }
-#pragma unroll
-            for (int kt = 0; kt < TOKENS / 16; kt++) {
-                uint32_t hi[4], lo[4];
+            for (int kt = 0; kt < TOKENS / 16; kt++)
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    const float p0 = score[2 * kt + (i >> 1)][2 * (i & 1)], p1 = score[2 * kt + (i >> 1)][2 * (i & 1) + 1];
-                    hi[i] = pack_bf16_rn(p0, p1);
-                    lo[i] = pack_bf16_rn(p0 - bf16_lo(hi[i]), p1 - bf16_hi(hi[i]));
+                    float p0 = score[2 * kt + (i >> 1)][2 * (i & 1)], p1 = score[2 * kt + (i >> 1)][2 * (i & 1) + 1];
+#pragma unroll
+                    for (int term = 0; term < 3; term++) {
+                        const uint32_t packed = pack_bf16_rn(p0, p1);
+                        p[term][kt][i] = packed;
+                        p0 -= bf16_lo(packed);
+                        p1 -= bf16_hi(packed);
+                    }
                 }
 #pragma unroll
-                for (int pair = 0; pair < D_TILES / 2; pair++) {
+            for (int pair = 0; pair < D_TILES / 2; pair++) {
+                uint32_t b[TOKENS / 16][4];
+#pragma unroll
+                for (int kt = 0; kt < TOKENS / 16; kt++) {
                     const int matrix = lane >> 3, t = token_warp * TOKENS + kt * 16 + (matrix & 1) * 8 + (lane & 7);
-                    uint32_t b[4];
-                    load_matrices_transposed(b, v_tile + tile_chunk<HD>(t, pair * 2 + (matrix >> 1)));
-                    mma_bf16(acc[2 * pair], hi, b[0], b[1]);
-                    mma_bf16(acc[2 * pair + 1], hi, b[2], b[3]);
-                    mma_bf16(acc[2 * pair], lo, b[0], b[1]);
-                    mma_bf16(acc[2 * pair + 1], lo, b[2], b[3]);
+                    load_matrices_transposed(b[kt], v_tile + tile_chunk<HD>(t, pair * 2 + (matrix >> 1)));
                 }
+                float sums[2][4] = {};
+#pragma unroll
+                for (int term = 2; term >= 0; term--)
+#pragma unroll
+                    for (int kt = 0; kt < TOKENS / 16; kt++) {
+                        mma_bf16(sums[0], p[term][kt], b[kt][0], b[kt][1]);
+                        mma_bf16(sums[1], p[term][kt], b[kt][2], b[kt][3]);
+                    }
+#pragma unroll
+                for (int d = 0; d < 2; d++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) acc[2 * pair + d][i] = fmaf(acc[2 * pair + d][i], factor[i >> 1], sums[d][i]);
             }
         }
         // (this tile's offsets were last read before the barrier above, when it was requested)
