@@ -1587,7 +1587,7 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
             // the experts' tiles (once per routing) and the quantised input: a frame per lane, or one per (lane, route)
             const MoeGroups groups = moe_groups(moe_groups_.ptr, model_->options().max_lanes, op.top_k, op.experts);
             if (grouped_signal != op.inputs[1]) {
-                check(launch_moe_group(static_cast<const uint32_t *>(ptr(op.inputs[1])), groups, lanes, op.top_k, op.experts, 0, op.experts, st), "moe_group");
+                check(launch_moe_group(static_cast<const uint32_t *>(ptr(op.inputs[1])), groups, lanes, op.top_k, op.experts, st), "moe_group");
                 grouped_signal = op.inputs[1];
             }
             const bool gate_up = op.kind == OpKind::MoeGateUp;
@@ -1596,12 +1596,12 @@ void Engine::run_component(const ComponentPlan &plan, int kv_index, int lanes, c
             check(launch_quantize_fp8(u16(op.inputs[0]), xq, xscale, gate_up ? lanes : lanes * op.top_k, gate_up ? op.moe_hidden : op.moe_inter, st), "expert input");
             if (gate_up)
                 check(launch_moe_gate_up_fp8(xq, xscale, groups, static_cast<const uint8_t *>(weight(w.tensor)), static_cast<const uint16_t *>(weight(w.scale)),
-                                             u16(op.outputs[0]), lanes, op.moe_hidden, op.moe_inter, op.experts, op.top_k, 0, st),
+                                             u16(op.outputs[0]), lanes, op.moe_hidden, op.moe_inter, op.experts, op.top_k, st),
                       "sparse_moe_gate_up");
             else
                 check(launch_moe_down_fp8(xq, xscale, groups, static_cast<const uint32_t *>(ptr(op.inputs[1])), static_cast<const uint8_t *>(weight(w.tensor)),
                                           static_cast<const uint16_t *>(weight(w.scale)), u16(op.outputs[0]), lanes, op.moe_hidden, op.moe_inter, op.experts,
-                                          op.top_k, 0, st),
+                                          op.top_k, st),
                       "sparse_moe_down");
             break;
         }

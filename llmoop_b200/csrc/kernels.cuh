@@ -121,15 +121,14 @@ struct MoeGroups {
 };
 size_t moe_group_bytes(int lanes, int top_k, int experts);
 MoeGroups moe_groups(void *scratch, int lanes, int top_k, int experts);  // carves moe_group_bytes bytes
-cudaError_t launch_moe_group(const uint32_t *routes, const MoeGroups &groups, int lanes, int top_k, int experts, int expert_start, int expert_count,
-                             cudaStream_t stream);
+cudaError_t launch_moe_group(const uint32_t *routes, const MoeGroups &groups, int lanes, int top_k, int experts, cudaStream_t stream);
 // xq / xscale: the hidden frames [lanes], or the intermediates [lanes * top_k], as launch_quantize_fp8 writes them.
 cudaError_t launch_moe_gate_up_fp8(const uint8_t *xq, const float *xscale, const MoeGroups &groups, const uint8_t *w,
                                    const uint16_t *wscale, uint16_t *intermediates, int lanes, int hidden_size,
-                                   int inter, int experts, int top_k, int expert_start, cudaStream_t stream);
+                                   int inter, int experts, int top_k, cudaStream_t stream);
 cudaError_t launch_moe_down_fp8(const uint8_t *xq, const float *xscale, const MoeGroups &groups, const uint32_t *routes, const uint8_t *w,
                                 const uint16_t *wscale, uint16_t *outputs, int lanes, int hidden_size, int inter,
-                                int experts, int top_k, int expert_start, cudaStream_t stream);
+                                int experts, int top_k, cudaStream_t stream);
 cudaError_t launch_moe_reduce(const uint16_t *outputs, uint16_t *y, int lanes, int hidden_size, int top_k,
                               float routed_scale, cudaStream_t stream);
 

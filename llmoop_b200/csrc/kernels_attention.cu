@@ -1059,7 +1059,7 @@ cudaError_t launch_rope_append(const RopeAppend &rope, const KvLayer &kv, const 
     if (kv.head_width == 128 && (rope.q_heads == 0 || whole(rope.q_form)) && whole(rope.k_form) && rope.q_norm == nullptr && rope.k_norm == nullptr) {
         // a head per warp while the lanes do not fill the chip
         constexpr int MANY = 6;
-        if (lanes >= 148) return launch_dependent(rope_append_whole_kernel<MANY>, dim3(lanes, (heads + ROPE_WARPS * MANY - 1) / (ROPE_WARPS * MANY)), dim3(ROPE_WARPS * 32), 0, 1, stream, rope, kv, lanes_meta);
+        if (lanes >= multiprocessors()) return launch_dependent(rope_append_whole_kernel<MANY>, dim3(lanes, (heads + ROPE_WARPS * MANY - 1) / (ROPE_WARPS * MANY)), dim3(ROPE_WARPS * 32), 0, 1, stream, rope, kv, lanes_meta);
         return launch_dependent(rope_append_whole_kernel<1>, dim3(lanes, (heads + ROPE_WARPS - 1) / ROPE_WARPS), dim3(ROPE_WARPS * 32), 0, 1, stream, rope, kv, lanes_meta);
     }
     return launch_dependent(rope_append_kernel, dim3(lanes, (heads + ROPE_WARPS - 1) / ROPE_WARPS), dim3(ROPE_WARPS * 32),

@@ -294,11 +294,8 @@ cudaError_t launch_linear_bf16_gemm(const uint16_t *x, const uint16_t *w, void *
     args.error_flag = error_flag;
     cudaError_t status = cudaFuncSetAttribute(linear_bf16_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SMEM_LIMIT + CONTROL_BYTES));
     if (status != cudaSuccess) return status;
-    int device = 0, sms = 0;
-    if ((status = cudaGetDevice(&device)) != cudaSuccess) return status;
-    if ((status = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) return status;
     const size_t smem = static_cast<size_t>(args.stages) * (A_BYTES + static_cast<size_t>(args.tile_lanes) * BLOCK_K * 2) + CONTROL_BYTES;
-    return launch_dependent(linear_bf16_gemm_kernel, dim3(std::min(args.tiles, sms)), dim3(THREADS), smem, 1, stream, args);
+    return launch_dependent(linear_bf16_gemm_kernel, dim3(std::min(args.tiles, multiprocessors())), dim3(THREADS), smem, 1, stream, args);
 }
 
 }  // namespace nerve

@@ -3,6 +3,8 @@
 // quantisation, MoE routing and reduce.  All are HBM/L2-trivial (KBs per lane);
 // they exist to keep the reference's bf16 rounding points, and are sized so a
 // verify batch (<= 160 lanes) fills the SMs with one CTA per lane (x head).
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.cuh"
 #include "launch.cuh"
@@ -131,7 +133,7 @@ __global__ void add_kernel(const uint32_t *__restrict__ a, const uint32_t *__res
 cudaError_t launch_add(const uint16_t *a, const uint16_t *b, uint16_t *y, size_t count, cudaStream_t stream) {
     size_t words = count / 2;
     int blocks = static_cast<int>((words + 255) / 256);
-    if (blocks > 148 * 8) blocks = 148 * 8;
+    blocks = std::min(blocks, multiprocessors() * 8);
     if (blocks < 1) blocks = 1;
     return launch_dependent(add_kernel, dim3(blocks), dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(a), reinterpret_cast<const uint32_t *>(b), reinterpret_cast<uint32_t *>(y), words);
 }
@@ -152,7 +154,7 @@ __global__ void round_add_kernel(const float *__restrict__ sums, const uint16_t 
 
 cudaError_t launch_round_add(const float *sums, const uint16_t *residual, uint16_t *out, size_t count, cudaStream_t stream) {
     int blocks = static_cast<int>((count + 255) / 256);
-    if (blocks > 148 * 8) blocks = 148 * 8;
+    blocks = std::min(blocks, multiprocessors() * 8);
     if (blocks < 1) blocks = 1;
     return launch_dependent(round_add_kernel, dim3(blocks), dim3(256), 0, 1, stream, sums, residual, out, count);
 }
@@ -173,7 +175,7 @@ cudaError_t launch_silu_multiply(const uint16_t *gate, const uint16_t *up, uint1
                                  cudaStream_t stream) {
     size_t words = count / 2;
     int blocks = static_cast<int>((words + 255) / 256);
-    if (blocks > 148 * 8) blocks = 148 * 8;
+    blocks = std::min(blocks, multiprocessors() * 8);
     if (blocks < 1) blocks = 1;
     return launch_dependent(silu_multiply_kernel, dim3(blocks), dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(gate), reinterpret_cast<const uint32_t *>(up), reinterpret_cast<uint32_t *>(y), words);
 }

@@ -18,8 +18,6 @@
 // bound), now 533; x 2048 x 4096: 676 -> 509 us.
 // Sparse experts are grouped: a small kernel sorts the (token, route) pairs by expert into tiles of up to eight, and an
 // expert's rows are read once per tile instead of once per pair.
-#include <cstdlib>
-
 #include "common.cuh"
 #include "kernels.cuh"
 #include "launch.cuh"
@@ -321,10 +319,9 @@ __global__ void __launch_bounds__(FP8_WARPS * 32, 2) linear_silu_multiply_fp8_ke
 // ---- sparse experts
 
 // Groups the (token, route) pairs by expert: order[] = pair indices expert by expert, tiles[t] = {expert, first place in
-// order, count <= 8}, tile_count.  Experts outside [expert_start, expert_start + expert_count) have no tiles.  One CTA.
+// order, count <= 8}, tile_count.  One CTA.
 constexpr int GROUP_THREADS = 1024, GROUP_MAX_EXPERTS = 1024;
-__global__ void __launch_bounds__(GROUP_THREADS) moe_group_kernel(const uint32_t *__restrict__ routes, int pairs, int experts, int expert_start, int expert_count,
-                                                                 MoeGroups groups) {
+__global__ void __launch_bounds__(GROUP_THREADS) moe_group_kernel(const uint32_t *__restrict__ routes, int pairs, int experts, MoeGroups groups) {
     __shared__ int counts[GROUP_MAX_EXPERTS], places[GROUP_MAX_EXPERTS], tile_places[GROUP_MAX_EXPERTS];
     __shared__ int warp_pairs[32], warp_tiles[32];
     grid_launch_dependents();
@@ -334,7 +331,7 @@ __global__ void __launch_bounds__(GROUP_THREADS) moe_group_kernel(const uint32_t
     __syncthreads();
     auto expert_of = [&](int pair) {
         const int expert = static_cast<int>(routes[pair] & 0xffffu);
-        return expert < experts && expert >= expert_start && expert < expert_start + expert_count ? expert : -1;
+        return expert < experts ? expert : -1;
     };
     for (int pair = threadIdx.x; pair < pairs; pair += GROUP_THREADS) {
         const int expert = expert_of(pair);
@@ -380,7 +377,7 @@ struct MoeArgs {
     const uint16_t *wscale;
     uint16_t *out;
     MoeGroups groups;
-    int hidden, inter, top_k, expert_start;
+    int hidden, inter, top_k;
 };
 
 // grid (tiles of 32 intermediate rows, expert tiles); the activations of a pair are its token's row
@@ -390,7 +387,7 @@ __device__ __forceinline__ void moe_gate_up_tile(const MoeArgs &a, int4 tile, ui
     const int *order = a.groups.order + tile.y;
     auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, k, first, n, count, smem, [&](int m) { return order[m] / a.top_k; }); };
     constexpr int HALF = RowSums<M, true>::ROWS / 2;
-    const int expert = tile.x - a.expert_start;
+    const int expert = tile.x;
     const uint8_t *w = a.w + static_cast<size_t>(expert) * 2 * a.inter * k;
     const uint16_t *ws = a.wscale + static_cast<size_t>(expert) * ((2 * a.inter + 127) >> 7) * blocks;
     for (int pass = 0; pass < FP8_ROWS / RowSums<M, true>::ROWS; pass++) {
@@ -421,7 +418,7 @@ __device__ __forceinline__ void moe_down_tile(const MoeArgs &a, int4 tile, uint8
     const int warp = threadIdx.x >> 5, thread = threadIdx.x & 31, k = a.inter, blocks = k >> 7, count = tile.z;
     const int *order = a.groups.order + tile.y;
     auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, k, first, n, count, smem, [&](int m) { return order[m]; }); };
-    const int expert = tile.x - a.expert_start;
+    const int expert = tile.x;
     const uint8_t *w = a.w + static_cast<size_t>(expert) * a.hidden * k;
     const uint16_t *ws = a.wscale + static_cast<size_t>(expert) * ((a.hidden + 127) >> 7) * blocks;
     for (int pass = 0; pass < FP8_ROWS / RowSums<M, false>::ROWS; pass++) {
@@ -458,7 +455,7 @@ cudaError_t launch_rows(void (*kernel)(Args), dim3 grid, int tile_lanes, cudaStr
 }
 
 // Rows of a CTA: 64 save half of the staging, 32 spread a small launch over more SMs.
-int fp8_passes(int row_tiles, int lanes) { return row_tiles * ((lanes + TILE_LANES - 1) / TILE_LANES) < 296 ? 1 : 2; }
+int fp8_passes(int row_tiles, int lanes) { return row_tiles * ((lanes + TILE_LANES - 1) / TILE_LANES) < 2 * multiprocessors() ? 1 : 2; }
 
 }  // namespace
 
@@ -534,11 +531,10 @@ MoeGroups moe_groups(void *scratch, int lanes, int top_k, int experts) {
     return groups;
 }
 
-cudaError_t launch_moe_group(const uint32_t *routes, const MoeGroups &groups, int lanes, int top_k, int experts, int expert_start, int expert_count,
-                             cudaStream_t stream) {
+cudaError_t launch_moe_group(const uint32_t *routes, const MoeGroups &groups, int lanes, int top_k, int experts, cudaStream_t stream) {
     if (lanes <= 0) return cudaSuccess;
     if (experts > GROUP_MAX_EXPERTS) return cudaErrorInvalidValue;
-    return launch_dependent(moe_group_kernel, dim3(1), dim3(GROUP_THREADS), 0, 1, stream, routes, lanes * top_k, experts, expert_start, expert_count, groups);
+    return launch_dependent(moe_group_kernel, dim3(1), dim3(GROUP_THREADS), 0, 1, stream, routes, lanes * top_k, experts, groups);
 }
 
 static int most_tiles(int lanes, int top_k, int experts) {
@@ -548,20 +544,20 @@ static int most_tiles(int lanes, int top_k, int experts) {
 
 cudaError_t launch_moe_gate_up_fp8(const uint8_t *xq, const float *xscale, const MoeGroups &groups, const uint8_t *w,
                                    const uint16_t *wscale, uint16_t *intermediates, int lanes, int hidden_size,
-                                   int inter, int experts, int top_k, int expert_start, cudaStream_t stream) {
+                                   int inter, int experts, int top_k, cudaStream_t stream) {
     if (lanes <= 0) return cudaSuccess;
     if (hidden_size % 128 != 0) return cudaErrorInvalidValue;
-    const MoeArgs args{xq, xscale, nullptr, w, wscale, intermediates, groups, hidden_size, inter, top_k, expert_start};
+    const MoeArgs args{xq, xscale, nullptr, w, wscale, intermediates, groups, hidden_size, inter, top_k};
     const int rows = FP8_WARPS * FP8_ROWS / 2;
     return launch_rows(moe_gate_up_fp8_kernel, dim3((inter + rows - 1) / rows, most_tiles(lanes, top_k, experts)), TILE_LANES, stream, args);
 }
 
 cudaError_t launch_moe_down_fp8(const uint8_t *xq, const float *xscale, const MoeGroups &groups, const uint32_t *routes, const uint8_t *w,
                                 const uint16_t *wscale, uint16_t *outputs, int lanes, int hidden_size, int inter,
-                                int experts, int top_k, int expert_start, cudaStream_t stream) {
+                                int experts, int top_k, cudaStream_t stream) {
     if (lanes <= 0) return cudaSuccess;
     if (inter % 128 != 0) return cudaErrorInvalidValue;
-    const MoeArgs args{xq, xscale, routes, w, wscale, outputs, groups, hidden_size, inter, top_k, expert_start};
+    const MoeArgs args{xq, xscale, routes, w, wscale, outputs, groups, hidden_size, inter, top_k};
     const int rows = FP8_WARPS * FP8_ROWS;
     return launch_rows(moe_down_fp8_kernel, dim3((hidden_size + rows - 1) / rows, most_tiles(lanes, top_k, experts)), TILE_LANES, stream, args);
 }

@@ -689,6 +689,7 @@ struct GemmPlan {
 // than they work: two CTAs of an SM do not slow one another down.  A wave that is not full costs as much as a full one, and
 // every CTA pays for filling its pipeline and for its epilogue, split ones for meeting their peers.
 GemmPlan plan_gemm(int matrix_tiles, int lanes, int groups, bool silu) {
+    const int sms = multiprocessors();
     const int padded = (lanes + 15) / 16 * 16;
     GemmPlan best;
     double best_cycles = 1e30;
@@ -734,10 +735,10 @@ GemmPlan plan_gemm(int matrix_tiles, int lanes, int groups, bool silu) {
                 plan.tmem_columns = per_sm == 2 ? 256 : 512;
                 plan.a_stages = std::min(GEMM_MAX_A_STAGES, (static_cast<int>(plan.tmem_columns) - d_columns) / (64 / parts * row_tiles));
                 if (plan.a_stages < parts + 1) continue;
-                const int ctas = blocks * lane_tiles * splits, together = ctas > 148 ? per_sm : 1;
+                const int ctas = blocks * lane_tiles * splits, together = ctas > sms ? per_sm : 1;
                 const double dequantise = row_tiles == 2 ? 430.0 : together == 2 ? 350.0 : 680.0;
                 const double per_group = 200.0 + row_tiles * std::max(5.6 * tile_lanes, dequantise);
-                const int waves = (ctas + 148 * per_sm - 1) / (148 * per_sm);
+                const int waves = (ctas + sms * per_sm - 1) / (sms * per_sm);
                 const double cycles = waves * (own * per_group * together + 7700.0 + 25.0 * row_tiles * tile_lanes) +
                                       (splits > 1 ? 650.0 * splits + 25.0 * row_tiles * tile_lanes : 0.0);
                 if (cycles < best_cycles) {

@@ -20,8 +20,6 @@
 // at 3 ALU ops per nibble pair.
 #include <mma.h>
 
-#include <cstdlib>
-
 #include "common.cuh"
 #include "kernels.cuh"
 #include "launch.cuh"
@@ -140,7 +138,7 @@ cudaError_t launch_linear_bf16_scalar(const uint16_t *x, const LinearBranches &b
     // shorter chains and sums (128 rows of 2048 with 24 lanes: 24 -> 10 us).
     int ctas = 0;
     for (int b = 0; b < branches.count; b++) ctas += (branches.n[b] + 31) / 32;
-    const int rows_per_warp = ctas * ((lanes + 7) / 8) < 148 ? 1 : 4;
+    const int rows_per_warp = ctas * ((lanes + 7) / 8) < multiprocessors() ? 1 : 4;
     Bf16Rows rows = {};
     ctas = 0;
     for (int b = 0; b < 3; b++) {

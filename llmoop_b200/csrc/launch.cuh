@@ -6,6 +6,13 @@
 
 namespace nerve {
 
+// Multiprocessors of the current device, for grids and plans that go by waves of them.
+inline int multiprocessors() {
+    int device = 0, count = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || count < 1) return 1;
+    return count;
+}
+
 template <typename... Parameters, typename... Arguments>
 cudaError_t launch_dependent(void (*kernel)(Parameters...), dim3 grid, dim3 block, size_t smem, int cluster_z, cudaStream_t stream, Arguments... arguments) {
     cudaLaunchConfig_t config = {};
