@@ -118,3 +118,40 @@ def test_failed_control_step_is_repeated(package):
     assert len(outputs) == 3 and engine.stream_tick(1) == 4 + emitted + 4 + 3
     engine.close()
     mounted.unmount()
+
+
+@pytest.mark.parametrize("drafts", [0, 2])
+def test_bounded_runs_end_with_their_closing_ticks(package, drafts):
+    """Runs of one batch each: a run that has emitted an event's last token has run its closing tick, too; the tokens are those
+    of one unbounded run."""
+    directory, spec = package
+    rng = np.random.default_rng(12)
+    prompts = [[int(t) for t in rng.integers(0, spec.vocab, size=3)] for _ in range(2)]
+    lengths = (3, 8)
+    engine, mounted = _mount(directory)
+
+    def start(first):
+        for i, (prompt, length) in enumerate(zip(prompts, lengths)):
+            engine.add_stream(first + i, speculative_draft_tokens=drafts)
+            engine.enqueue_input_event(first + i, prompt, length)
+
+    start(1)
+    outputs, _ = engine.run_until_idle()
+    want = [[token for sid, token, _, _ in outputs if sid == stream] for stream in (1, 2)]
+    assert [len(tokens) for tokens in want] == list(lengths)
+    start(11)
+    got = [[], []]
+    for _ in range(40):
+        outputs, report = engine.run(1)
+        for sid, token, _, _ in outputs:
+            got[sid - 11].append(token)
+        for i, (tokens, length) in enumerate(zip(got, lengths)):
+            if len(tokens) == length:
+                assert engine.stream_tick(11 + i) == len(prompts[i]) + length
+                counts = engine.scheduler_stream_counts(11 + i)
+                assert counts["in_flight_activation_count"] == 0 and counts["completed_input_event_count"] == 1, counts
+        if report.idle:
+            break
+    assert got == want
+    engine.close()
+    mounted.unmount()
