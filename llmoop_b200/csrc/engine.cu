@@ -1677,7 +1677,8 @@ void Engine::upload_tokens(const uint32_t *tokens, int count) {
 // rounded up to a power of two so that a handful of graph shapes serves a growing context - 64 tokens in the persistent
 // kernel, the engine's fixed length on the kernel-per-operator path.  A prefill chunk (never replayed from a graph)
 // takes the number of splits that brings its last wave of CTAs, one per SM, closest to full: a CTA walks a tile of 64
-// tokens in about 1.7 us, needs three tiles' time to start, and more than one split costs the merge's traffic.
+// tokens in about 3.2 us, needs three tiles' time to start, and more than one split costs the merge's traffic (713 lanes at
+// 8713 tokens: 697 us in two splits of three waves, 614 in four of five).
 // Returns a word for graph keys.
 int Engine::plan_splits(int lanes, int lanes_per_stream, uint64_t newest_tick) {
     const uint64_t tokens = std::min<uint64_t>(newest_tick + 1, model_->capacity());
@@ -1703,7 +1704,7 @@ int Engine::plan_splits(int lanes, int lanes_per_stream, uint64_t newest_tick) {
         for (int splits = 1; splits <= 16; splits++) {
             if (splits > 1 && (tiles < 4.0 * splits || static_cast<size_t>(lanes) * max_q_heads_ * splits > attention_partials_)) break;
             const double waves = std::ceil(ctas * splits / model_->sm_count());
-            const double microseconds = waves * (std::ceil(tiles / splits) + 3.0) * 1.7 + (splits > 1 ? 4.0 + lanes * attention->q_heads * splits * 2.1e-4 : 0.0);
+            const double microseconds = waves * (std::ceil(tiles / splits) + 3.0) * 3.2 + (splits > 1 ? 4.0 + lanes * attention->q_heads * splits * 2.1e-4 : 0.0);
             if (splits == 1 || microseconds < best) {
                 best = microseconds;
                 current_op_splits_ = splits;

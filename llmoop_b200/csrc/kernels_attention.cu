@@ -34,14 +34,14 @@ constexpr float LOWEST = -3.4028234663852886e38f;
 // tiles of 64 tokens go through two shared-memory stages (cp.async one tile ahead, the tokens' page offsets two tiles
 // ahead), Q stays in registers; Q.K^T and P.V run on mma.sync bf16 with f32 sums.  The probabilities enter P.V as three
 // bf16 terms, which hold all 24 bits of their f32 value, and the sums over the tiles are f32 multiply-adds: the error
-// against 64 bits, before the final rounding, is 2.2e-7 to 3.1e-7 of the output (32 lanes at 550 tokens .. 713 at 8713),
+// against 64 bits, before the final rounding, is 2.2e-7 to 3.9e-7 of the output (32 lanes at 550 tokens .. 713 at 8713),
 // where scalar f32 products and sums leave 2.7e-7 to 1.2e-6, and two terms with one running sum left 1.6e-6 to 1.0e-5.
 // TOKEN_WARPS warps share a row tile's context: each takes 64 / TOKEN_WARPS tokens of every tile with a softmax of its
 // own, and they merge at the end.  Prefill chunks (many rows per stream) run 8 x 1 warps; verify and draft batches
 // (few rows, many tokens) 1 or 2 x 4, where four warps per row tile hide the tile's latency.
 // What bounds it: prefill the legacy tensor path (four MMAs per 16 x 8 x 16 of K and V), decode the KV bytes.
 // (One scalar f32 product per thread and token, the form this replaced, took 4.8 ms per 8B layer for 713 lanes at an
-// 8713-token context; this takes 0.74 ms, with two terms it took 0.55.)
+// 8713-token context; this takes 0.70 ms, with two terms it took 0.55.)
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -85,7 +85,7 @@ constexpr size_t attention_smem() {
     return tiles > merge ? tiles : merge;
 }
 
-// The verify form of 32 rows takes two CTAs per SM (128 registers, 76 bytes of spills): it waits for its K and V more than
+// The verify form of 32 rows takes two CTAs per SM (128 registers, 92 bytes of spills): it waits for its K and V more than
 // it multiplies, and 32 streams x 8 kv heads x splits are several waves of one CTA per SM (44 -> 35 us per launch).
 template <int HD, int ROW_WARPS, int TOKEN_WARPS>
 __global__ void __launch_bounds__(ROW_WARPS *TOKEN_WARPS * 32, ROW_WARPS * TOKEN_WARPS == 8 && TOKEN_WARPS > 1 ? 2 : 1) attention_tile_kernel(const __grid_constant__ AttentionArgs a) {
@@ -244,8 +244,10 @@ __global__ void __launch_bounds__(ROW_WARPS *TOKEN_WARPS * 32, ROW_WARPS * TOKEN
                     }
                 row_sum[h] = row_sum[h] * factor[h] + sum;  // this thread's columns; added up over the four threads in the end
             }
-            // p = hi + mid + lo, the 24 bits of its f32 value; a tile's products add up from zero, the smallest terms first, and
-            // join the row's sum by one multiply-add, which rounds to nearest where the tensor core's running sum truncates
+            // p as three bf16 terms, the 24 bits of its f32 value; a tile's products add up from zero, of sixteen tokens the
+            // smallest terms first, and join the row's sum by one multiply-add, which rounds to nearest where the tensor
+            // core's running sum truncates.  Eight sums at a time hide the latency of the chain (713 lanes at 8713 tokens: two
+            // 741 us, four 723, eight 697).
             uint32_t p[3][TOKENS / 16][4];
 #pragma unroll
             for (int kt = 0; kt < TOKENS / 16; kt++)
@@ -260,26 +262,29 @@ __global__ void __launch_bounds__(ROW_WARPS *TOKEN_WARPS * 32, ROW_WARPS * TOKEN
                         p1 -= bf16_hi(packed);
                     }
                 }
+            constexpr int PAIRS = 4;  // of eight output dims in flight
+            static_assert(D_TILES % (2 * PAIRS) == 0, "the output dims are taken PAIRS pairs at a time");
 #pragma unroll
-            for (int pair = 0; pair < D_TILES / 2; pair++) {
-                uint32_t b[TOKENS / 16][4];
+            for (int first = 0; first < D_TILES; first += 2 * PAIRS) {
+                float sums[2 * PAIRS][4] = {};
 #pragma unroll
                 for (int kt = 0; kt < TOKENS / 16; kt++) {
                     const int matrix = lane >> 3, t = token_warp * TOKENS + kt * 16 + (matrix & 1) * 8 + (lane & 7);
-                    load_matrices_transposed(b[kt], v_tile + tile_chunk<HD>(t, pair * 2 + (matrix >> 1)));
+                    uint32_t b[PAIRS][4];
+#pragma unroll
+                    for (int pair = 0; pair < PAIRS; pair++) load_matrices_transposed(b[pair], v_tile + tile_chunk<HD>(t, first + pair * 2 + (matrix >> 1)));
+#pragma unroll
+                    for (int term = 2; term >= 0; term--)
+#pragma unroll
+                        for (int pair = 0; pair < PAIRS; pair++) {
+                            mma_bf16(sums[2 * pair], p[term][kt], b[pair][0], b[pair][1]);
+                            mma_bf16(sums[2 * pair + 1], p[term][kt], b[pair][2], b[pair][3]);
+                        }
                 }
-                float sums[2][4] = {};
 #pragma unroll
-                for (int term = 2; term >= 0; term--)
+                for (int d = 0; d < 2 * PAIRS; d++)
 #pragma unroll
-                    for (int kt = 0; kt < TOKENS / 16; kt++) {
-                        mma_bf16(sums[0], p[term][kt], b[kt][0], b[kt][1]);
-                        mma_bf16(sums[1], p[term][kt], b[kt][2], b[kt][3]);
-                    }
-#pragma unroll
-                for (int d = 0; d < 2; d++)
-#pragma unroll
-                    for (int i = 0; i < 4; i++) acc[2 * pair + d][i] = fmaf(acc[2 * pair + d][i], factor[i >> 1], sums[d][i]);
+                    for (int i = 0; i < 4; i++) acc[first + d][i] = fmaf(acc[first + d][i], factor[i >> 1], sums[d][i]);
             }
         }
         // (this tile's offsets were last read before the barrier above, when it was requested)
