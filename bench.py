@@ -269,8 +269,8 @@ def cpu_cycle_sample(directory, seconds_budget=150.0, max_cycles=None, cuda_run=
                           "oracle, the kernel-per-operator path and the persistent kernel differ mutually by that much "
                           "(tests/test_gpu_config2_parity.py), so near-ties up to that size may fall either way; accepted_equal says the "
                           "per-cycle bookkeeping followed the oracle through every one of them; control_kernel_per_operator_path is the "
-                          "same replay of the path whose operators match the oracle bit for bit one by one - it parts from the oracle "
-                          "just as often")
+                          "same replay of the path whose operators match the oracle to the last bf16 bit in at least 97 % of their "
+                          "outputs one by one; which of the two parts from the oracle, and how often, varies with the build")
     else:
         token, _ = oracle.prefill(stream, prompt, sample_last=True)
         begin = time.perf_counter()
@@ -406,7 +406,7 @@ def main():
     # the short event the CPU oracle replays afterwards (rank 0): tokens and per-cycle acceptance of this very mount
     sample_run = short_event(engine, 0, prompt, 40)
     # the control of that replay (one GPU): the same event on the kernel-per-operator path, whose operators agree with
-    # the oracle bit for bit at operator level - what the model's own chaos does to a token sequence
+    # the oracle to the last bf16 bit in at least 97 % of their outputs - what the model's own chaos does to a token sequence
     control_run = None
     if world == 1 and info["target_decode_stack"] and os.environ.get("NERVE_B200_DECODE_STACK", "1") != "0":
         engine.set_decode_stack(False)

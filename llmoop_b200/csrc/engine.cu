@@ -574,11 +574,11 @@ Engine::Engine(std::shared_ptr<MountedModel> model) : model_(std::move(model)) {
     for (const ComponentPlan &layer : plan.layers) scan(layer);
     for (const ComponentPlan &layer : plan.draft_layers) scan(layer);
     // Scratch of the split attention.  The persistent kernel (at most eight lanes) takes 64-token splits over the
-    // whole ring.  On the kernel-per-operator path verify, draft and single-tick batches take splits of a fixed length,
-    // so that the arithmetic of such a lane does not depend on its batch: 128 tokens where the partials of the batch over
-    // the whole ring fit the scratch (1 GB at most), else the next multiple (plan_splits); prefill chunks are split only
-    // as far as they need to be to fill the chip.  FP8 packages take one length for everything: 64 tokens where the
-    // partials of the largest batch fit, else the next multiple.
+    // whole ring.  On the kernel-per-operator path verify, draft and single-tick batches take splits of 128 tokens, whatever
+    // their contexts, where the partials of the batch over the whole ring fit the scratch (1 GB at most), else of the next
+    // multiple (plan_splits); prefill chunks are split only as far as they need to be to fill the chip.  So a lane's order of
+    // additions depends on its batch there, as it does in the INT4 linears of more than eight lanes.  FP8 packages take one
+    // length for everything, whatever the batch: 64 tokens where the partials of the largest batch fit, else the next multiple.
     auto has_fp8 = [](const ComponentPlan &component) {
         for (const OpSpec &op : component.ops)
             for (const WeightRef &w : op.weights)

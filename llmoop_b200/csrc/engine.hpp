@@ -425,8 +425,8 @@ private:
     const uint32_t *current_tokens_ = nullptr;
     int current_width_ = 1;                 // lanes per stream of the current batch (stream-major lane order)
     int current_splits_ = 1;                // attention split count (stride of the scratch partials) of this launch
-    int op_split_tokens_ = 128;             // tokens per split of decode batches on the kernel-per-operator path: fixed per engine, so
-                                            // that a lane's arithmetic does not depend on the batch it runs in
+    int op_split_tokens_ = 128;             // tokens per split of decode batches on the kernel-per-operator path, or a multiple of it
+                                            // where a wide batch's partials would not fit the scratch (plan_splits)
     int current_op_split_tokens_ = 128, current_op_splits_ = 1;  // split length and count of the next launches on that path
     DeviceBuffer attention_blocks_;         // row blocks of a ragged prefill batch
     int current_blocks_ = 0;                // ... of the next launches (0: uniform batch)

@@ -190,7 +190,8 @@ cudaError_t launch_output_projection(const uint16_t *x, const void *streamed_tab
 bool linear_int4_gemm_supported(int lanes, int n, int k);
 size_t int4_activation_bytes(int lanes, int k);
 cudaError_t launch_prepare_activations(const uint16_t *x, void *prepared, int lanes, int k, cudaStream_t stream);
-// ... of the RMSNorm of x (the values launch_rms_norm writes), without writing them
+// ... of the RMSNorm of x (the values launch_rms_norm writes, up to the order in which the squares are added), without writing
+// them
 cudaError_t launch_rms_norm_prepared(const uint16_t *x, const uint16_t *weight, void *prepared, int lanes, int width, float eps, float weight_offset,
                                      cudaStream_t stream);
 cudaError_t launch_linear_int4_gemm(const void *prepared, int branches, const uint32_t *const *qweights, const uint16_t *const *scales, void *const *ys,

@@ -11,7 +11,10 @@
 // two come off again in the epilogue.  (Rows whose scales are close together take a cheaper form, dequantise_word_raw, in
 // another range of exponents.)  No group scale is left to apply to partial sums, so the f32 accumulator stays
 // in tensor memory over the whole of K (one that is read back, scaled and added up in registers for every group of
-// 128 columns ran at 140-175 TFLOP/s: the tensor pipe was idle 87 % of the time).
+// 128 columns ran at 140-175 TFLOP/s: the tensor pipe was idle 87 % of the time).  The tensor core truncates its running
+// sum, so the longest chain decides the error against 64 bits: before the output's rounding 3e-7 of the output for 16
+// lanes of 4096 x 4096, at most 9e-6 (512 lanes of 4096 x 14336), where per-group sums had 1e-7 to 3e-7; of the bf16
+// outputs, which their rounding puts 1.66e-3 off, it changes the sixth digit.
 //
 // Roles.  A CTA computes ROW_TILES x 128 weight rows (M side) by up to 256 / ROW_TILES lanes (N side):
 //   8 x ROW_TILES warps bring their rows' packed nibbles into shared memory with cp.async several groups ahead (32 rows x 64
@@ -118,7 +121,7 @@ __device__ __forceinline__ void dequantise_word(uint32_t word, uint32_t scale2, 
 // The same values x 2^-24 in four operations less, from the nibbles where they stand: as fp16 bit patterns they are q x 2^-24
 // (x 16 in the next four bits), subnormal and exact, and one fused multiply-add with 2^24 s and -8 s makes (q - 8) s of
 // them - exact as long as s keeps its eight bits above 2^-24, that is for rows whose scales lie within a factor of 64.
-// (16 x 28672 x 8192: 38.2 -> 33.2 us, 32 lanes: 39.4 -> 36.7; from 100 lanes on the tensor pipe is the bound.)
+// (28672 x 8192, rows of either kind: 43.0 and 31.2 us for 16 lanes, 46.5 and 34.5 for 32, 80.5 and 68.0 for 160.)
 __device__ __forceinline__ uint32_t fma2(uint32_t a, uint32_t b, uint32_t c) {
     uint32_t out;
     asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(out) : "r"(a), "r"(b), "r"(c));
@@ -687,7 +690,10 @@ struct GemmPlan {
 // average, an estimate without the dequantisation's latency took 7 %).  Per group of 128 columns a CTA needs 5.6 cycles per
 // lane and row tile on the tensor cores (4 at the pipe's nominal rate) or the time of its operand warps, which wait more
 // than they work: two CTAs of an SM do not slow one another down.  A wave that is not full costs as much as a full one, and
-// every CTA pays for filling its pipeline and for its epilogue, split ones for meeting their peers.
+// every CTA pays for filling its pipeline and for its epilogue, split ones for meeting their peers.  The number of splits goes
+// with the lanes of the launch, and with it the order of a lane's sums: from nine lanes on a lane's last bits depend on what
+// shares its batch.  (Splits by the matrix alone would cost 6 % of an 8B layer's GEMM time at 512 lanes and 14 % at 32, by
+// this estimate.)
 GemmPlan plan_gemm(int matrix_tiles, int lanes, int groups, bool silu) {
     const int sms = multiprocessors();
     const int padded = (lanes + 15) / 16 * 16;

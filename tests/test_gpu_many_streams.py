@@ -12,7 +12,7 @@ No CPU oracle finishes this size; the test checks properties that hold at any si
     accepted and the emitted tokens are the natural ones again - the verify lanes of accepted drafts reproduce what
     one-token-at-a-time decoding computed (acceptance, in-place KV commit and catch-up at M = 160).  The comparison
     stops k + 1 tokens before the events' ends, where the two runs' last windows shrink differently and batches of
-    fewer than 64 lanes take another kernel.
+    other widths add in another order (K splits by the number of lanes, another kernel below nine).
 Synthetic data: seeded N(0, 0.02) weights, prompts uniform over the vocabulary.
 """
 
@@ -71,7 +71,7 @@ def test_thirty_two_streams_verify_160_lanes_per_cycle():
 
     forced, ticks, report, seconds = _run(engine, prompts, teacher=natural)
     # Compared while both runs verify 160 lanes per cycle: with fewer than k + 1 tokens left the windows shrink, the
-    # batches fall below 64 lanes and another kernel (another order of f32 additions) computes the last tokens.
+    # batches get narrower and the last tokens are computed in another order of f32 additions.
     same_regime = TOKENS - 2 * (DRAFTS + 1)
     mismatches = [(i, next(j for j in range(same_regime) if forced[i][j] != natural[i][j]))
                   for i in range(STREAMS) if forced[i][:same_regime] != natural[i][:same_regime]]
