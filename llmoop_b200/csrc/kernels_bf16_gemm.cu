@@ -6,9 +6,10 @@
 // Persistent: one CTA per SM walks output tiles of 128 weight rows (MMA M) x up to 256 lanes (MMA N).  One warp copies
 // both operands with TMA (128-byte-swizzled tiles of 64 columns) into a ring as deep as shared memory allows, straight
 // on into the next tile; one warp issues the MMAs into one of two accumulators in tensor memory; four warps write the
-// finished accumulator out while the other one fills.  Up to about 200 lanes the weight bytes are the bound (a 128256 x
-// 4096 table: 1.05 GB), beyond that the tensor pipe.  (The form this replaced - 64 lanes to a tile, operands copied by
-// all threads between two barriers per block - read that table for 32 lanes in 640 us.)
+// finished accumulator out while the other one fills.  The weight bytes are the bound up to 64 lanes (a 128256 x 4096 table of
+// 1.05 GB: 160-167 us, the copy rate), the stores of the outputs show from there on (160 lanes: 200 us), and from 200 lanes
+// on the tensor pipe is it.  (The form this replaced - 64 lanes to a tile, operands copied by all threads between two
+// barriers per block - read that table for 32 lanes in 640 us.)
 // Waits are bounded; a wait that expires sets the error word, and the CTA still frees its tensor memory.  The unbounded wait
 // for the kernel in front comes before them in every role, so none of them counts that kernel's time.
 #include <cuda.h>
