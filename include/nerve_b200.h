@@ -170,9 +170,9 @@ typedef struct nerve_b200_run_report {
 } nerve_b200_run_report;
 
 /* run_until_idle_bounded_with_output (placed_prompt_engine.rs:420-589).
- * Streams share batches.  Up to eight lanes (streams x (drafts + 1), or prompt tokens) a stream's arithmetic is the same
- * whatever shares its batch; wider batches choose the order of some f32 sums by their width, so the last bits of a
- * stream's logits, and a token that hangs on them, may depend on its company there. */
+ * Streams share batches.  While the streams that run together make up to eight lanes of decoding (streams x (drafts + 1)), a
+ * stream's arithmetic is the same as if it ran alone, its prompts included; wider batches choose the order of some f32
+ * sums by their width, so the last bits of a stream's logits, and a token that hangs on them, may depend on its company. */
 int32_t nerve_b200_engine_run_until_idle(nerve_b200_engine *engine, nerve_b200_output_callback on_output, void *user,
                                          nerve_b200_run_report *out_report);
 

@@ -2299,7 +2299,12 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
         }
         for (Work &work : deferred) works.push_back(std::move(work));
         deferred.clear();
-        // 2. prefill chunks, as many streams' in one pass as the lanes allow
+        // 2. prefill chunks, as many streams' in one pass as the lanes allow.  Where the step's streams decode in eight lanes
+        // together, a stream is computed as if it were alone, and so are its prompts: one stream's chunk per pass, whose
+        // order of additions does not go by its company (FP8 layers have one order at any width).
+        size_t decode_lanes = 0;
+        for (const Work &work : works) decode_lanes += static_cast<size_t>(work.stream->k) + 1;
+        const bool shared_passes = scalar_attention_ || decode_lanes > 8;
         struct Pending {
             Work *work;
             size_t left;
@@ -2332,7 +2337,7 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
                 // with the prefix cache on, a chunk also stops at the prompt's last page boundary: the state there is retained
                 const uint64_t checkpoint_tick = prefix_checkpoint_tick(s);
                 if (checkpoint_tick > s.next_tick && checkpoint_tick < s.next_tick + static_cast<uint64_t>(count)) count = static_cast<int>(checkpoint_tick - s.next_tick);
-                if (!parts.empty() && (lanes + count > model_->options().max_lanes || (!ragged_prefill_ && count != parts[0].count) || (scalar_attention_ && (count >= 16) != (parts[0].count >= 16)))) continue;
+                if (!parts.empty() && (!shared_passes || lanes + count > model_->options().max_lanes || (!ragged_prefill_ && count != parts[0].count) || (scalar_attention_ && (count >= 16) != (parts[0].count >= 16)))) continue;
                 const bool last = pending[p].work->activation.remaining_prompt_token_count == 0 && static_cast<size_t>(count) == pending[p].left;
                 parts.push_back(PrefillPart{&s, event.input.token_ids.data() + event.next_external, count, last && event.remaining > 0, last, 0, checkpoint_tick});
                 members.push_back(p);

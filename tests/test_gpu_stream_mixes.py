@@ -99,6 +99,39 @@ def test_wide_fp8_heads_in_company_and_alone(tmp_path, q_heads, kv_heads, head):
     package.unmount()
 
 
+@pytest.mark.parametrize("quant,std", [("int4", 0.02), ("bf16", 0.05)])
+@pytest.mark.parametrize("lengths", [(5, 6), (30, 45), (7, 60)])
+def test_streams_of_eight_lanes_together_and_alone(tmp_path, quant, std, lengths):
+    """Two streams with three drafts each decode in eight lanes: tokens and logits are those of each stream alone, bit for bit,
+    whatever the prompts."""
+    import llmoop_b200 as nb
+    from llmoop_b200.package_writer import write_package
+    from llmoop_b200.synth import ModelSpec
+
+    spec = ModelSpec(name=f"mix_{quant}", hidden=512, layers=2, q_heads=4, kv_heads=2, head_dim=128, ffn=512, vocab=256, max_positions=256, quant=quant,
+                     std=std, seed=41)
+    directory = write_package(spec, tmp_path / spec.name)
+    package = nb.Package(directory, capacity_tokens=128, page_tokens=16, max_streams=4, max_lanes=128, verify_level=0)
+    engine = nb.Engine(package)
+    engine.set_prefill_chunk(128)
+
+    def run(prompts):
+        for i, prompt in enumerate(prompts):
+            engine.add_stream(i, speculative_draft_tokens=3)
+            engine.enqueue_input_event(i, prompt, 16)
+        outputs, _ = engine.run_until_idle()
+        logits = [engine.debug_target_logits(i, [5])[0] for i in range(len(prompts))]
+        for i in range(len(prompts)):
+            engine.remove_stream(i)
+        return [([t for sid, t, _, _ in outputs if sid == i], row.tobytes()) for i, row in enumerate(logits)]
+
+    prompts = _prompts(spec.vocab, lengths, sum(lengths))
+    together = run(prompts)
+    assert [run([prompt])[0] for prompt in prompts] == together
+    engine.close()
+    package.unmount()
+
+
 def test_fork_of_more_streams_than_one_launch_copies_pages_for():
     import llmoop_b200 as nb
 
