@@ -2371,18 +2371,18 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
         // 3. decode windows.  Streams that speculate share a cycle whatever their draft counts: it runs the largest one,
         // a stream with a smaller window (its last tokens) ignores the drafts behind it, and one with room for a single
         // token, or only the closing tick of its event to do, ignores them all - a pass over the weights costs more than
-        // the lanes.  FP8 packages keep cycles of equal
-        // draft count (the form of their routers' sums goes by the lanes of a batch).
+        // the lanes.  FP8 packages keep cycles of equal draft count (the form of their routers' sums goes by the lanes of a
+        // batch), and so do streams that decode in eight lanes together but would need more in one cycle.
         struct Window {
             Stream *stream;
             int drafts;
         };
-        std::map<int, std::vector<Window>> speculative;
+        std::vector<Window> windows;
         std::vector<Stream *> single;
         for (Work &work : works) {
             if (work.closing) {
                 if (work.stream->active == nullptr) continue;  // its closing tick has run as a control step
-                if (work.stream->k > 0 && model_->plan().has_draft) speculative[0].push_back(Window{work.stream, 0});
+                if (work.stream->k > 0 && model_->plan().has_draft) windows.push_back(Window{work.stream, 0});
                 else single.push_back(work.stream);
                 continue;
             }
@@ -2396,11 +2396,16 @@ RunReport Engine::run(uint64_t max_batches, const std::function<void(const Outpu
             const bool ring_wraps = s.next_tick + static_cast<uint64_t>(s.k) + 1 > model_->capacity();
             if (s.k > 0 && model_->plan().has_draft && !event.feedback_closes && window >= 1 && !ring_wraps) {
                 const int drafts = static_cast<int>(std::min<size_t>(s.k, window - 1));
-                speculative[scalar_attention_ ? drafts : 0].push_back(Window{&s, drafts});
+                windows.push_back(Window{&s, drafts});
             } else {
                 single.push_back(&s);
             }
         }
+        int widest = 0;
+        for (const Window &window : windows) widest = std::max(widest, window.drafts);
+        const bool equal_drafts = scalar_attention_ || (decode_lanes <= 8 && windows.size() * static_cast<size_t>(widest + 1) > 8);
+        std::map<int, std::vector<Window>> speculative;
+        for (const Window &window : windows) speculative[equal_drafts ? window.drafts : 0].push_back(window);
         uint64_t start = now_ns();
         for (auto &group : speculative) {
             int drafts = 0;

@@ -100,10 +100,10 @@ def test_wide_fp8_heads_in_company_and_alone(tmp_path, q_heads, kv_heads, head):
 
 
 @pytest.mark.parametrize("quant,std", [("int4", 0.02), ("bf16", 0.05)])
-@pytest.mark.parametrize("lengths", [(5, 6), (30, 45), (7, 60)])
-def test_streams_of_eight_lanes_together_and_alone(tmp_path, quant, std, lengths):
-    """Two streams with three drafts each decode in eight lanes: tokens and logits are those of each stream alone, bit for bit,
-    whatever the prompts."""
+@pytest.mark.parametrize("lengths,drafts", [((5, 6), (3, 3)), ((30, 45), (3, 3)), ((7, 60), (3, 3)), ((6, 5), (1, 5)), ((20, 4), (4, 2)), ((3, 3, 3), (0, 4, 1))])
+def test_streams_of_eight_lanes_together_and_alone(tmp_path, quant, std, lengths, drafts):
+    """Streams that decode in eight lanes together, in one cycle or in several: tokens and logits are those of each stream
+    alone, bit for bit, whatever the prompts."""
     import llmoop_b200 as nb
     from llmoop_b200.package_writer import write_package
     from llmoop_b200.synth import ModelSpec
@@ -115,9 +115,9 @@ def test_streams_of_eight_lanes_together_and_alone(tmp_path, quant, std, lengths
     engine = nb.Engine(package)
     engine.set_prefill_chunk(128)
 
-    def run(prompts):
+    def run(prompts, drafts):
         for i, prompt in enumerate(prompts):
-            engine.add_stream(i, speculative_draft_tokens=3)
+            engine.add_stream(i, speculative_draft_tokens=drafts[i])
             engine.enqueue_input_event(i, prompt, 16)
         outputs, _ = engine.run_until_idle()
         logits = [engine.debug_target_logits(i, [5])[0] for i in range(len(prompts))]
@@ -126,8 +126,8 @@ def test_streams_of_eight_lanes_together_and_alone(tmp_path, quant, std, lengths
         return [([t for sid, t, _, _ in outputs if sid == i], row.tobytes()) for i, row in enumerate(logits)]
 
     prompts = _prompts(spec.vocab, lengths, sum(lengths))
-    together = run(prompts)
-    assert [run([prompt])[0] for prompt in prompts] == together
+    together = run(prompts, drafts)
+    assert [run([prompt], [count])[0] for prompt, count in zip(prompts, drafts)] == together
     engine.close()
     package.unmount()
 
