@@ -193,6 +193,8 @@ cudaError_t launch_accept(const uint32_t *verify_tokens, const uint32_t *target_
 // peer (it needs the peer's word of vote v before it can finish v), so the slot of vote v + 2 is free by then.
 __global__ void tensor_parallel_argmax_kernel(const uint32_t *__restrict__ records_local, uint32_t first_token, uint32_t *__restrict__ records,
                                               int lanes, const StackTp *__restrict__ tp_pointer, int *error_flag) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const StackTp &tp = *tp_pointer;
     unsigned long long *control = tp.counter[tp.rank];
     const uint32_t vote = static_cast<uint32_t>(control[STACK_TP_WORD_VOTES]) + 1u;  // every thread reads it before thread 0 moves it on (below)
