@@ -529,6 +529,7 @@ Engine::Engine(std::shared_ptr<MountedModel> model) : model_(std::move(model)) {
     };
     for (const ComponentPlan &layer : plan.layers) widest(layer);
     for (const ComponentPlan &layer : plan.draft_layers) widest(layer);
+    if (plan.has_draft) widest(plan.draft_adapter);
     size_t moe_values = 0, moe_bytes = 0;
     auto experts = [&](const ComponentPlan &component) {
         for (const OpSpec &op : component.ops)
