@@ -628,7 +628,7 @@ Engine::Engine(std::shared_ptr<MountedModel> model) : model_(std::move(model)) {
         if (q_width != 0) {
             stack_q_ = device_alloc(8 * q_width * 2);
             stack_attention_out_ = device_alloc(8 * q_width * 2);
-            stack_activation_ = device_alloc(8 * ffn * 2);
+            stack_activation_ = device_alloc(stack_activation_bytes(static_cast<int>(ffn)));
             stack_barrier_ = device_alloc(STACK_BARRIER_WORDS * sizeof(unsigned int));
             stack_timing_ = device_alloc(std::max<size_t>(1, plan.layers.size()) * 32 * sizeof(unsigned long long));
         }
@@ -1772,7 +1772,7 @@ bool Engine::run_stack(const StackPlan &stack, int lanes, void *hidden) {
     buffers.q = static_cast<uint16_t *>(stack_q_.ptr);
     buffers.attention_scratch = static_cast<float *>(attention_scratch_.ptr);
     buffers.attention_out = static_cast<uint16_t *>(stack_attention_out_.ptr);
-    buffers.activation = static_cast<uint16_t *>(stack_activation_.ptr);
+    buffers.activation = static_cast<uint8_t *>(stack_activation_.ptr);
     buffers.barrier = static_cast<unsigned int *>(stack_barrier_.ptr);
     buffers.error_flag = static_cast<int *>(kernel_error_.ptr);
     buffers.timing = (profile_ && &stack == &model_->target_stack()) ? static_cast<unsigned long long *>(stack_timing_.ptr) : nullptr;

@@ -207,36 +207,39 @@ cudaError_t launch_linear_bf16_gemm(const uint16_t *x, const uint16_t *w, void *
 // every CTA (one per SM) streams its share of each weight matrix while grid-wide barriers separate the steps of a
 // layer.  Weights are read from per-CTA byte streams written at mount (launch_int4_cta_streams).
 
-// How the CTAs of a grid share one matrix of `tiles` 16-row tiles (a gate/up pair tile holds 16 gate rows and the
-// same 16 up rows: rt = 2) over K = groups * 128 columns.  CTA c owns tiles c, c + grid, ...; it works on `slots`
-// of them at a time (one pass), `width` warps per tile, warp i of a tile taking units i, i + width, ... of the
-// tile's `units` = groups * rt blocks of 16x128 nibbles (unit u = group u / rt, matrix u % rt).  Step s of a pass
-// is one stage of the CTA's stream: for every present tile slot, units s * width .. s * width + width - 1
-// (1 KB of nibbles each, zero beyond `units`), followed by the same units' 32-byte scale-pair rows.
+// How the CTAs of a grid share one matrix of `tiles` 16-row tiles over K = groups * 128 columns.  CTA c owns tiles c,
+// c + grid, ...  The rows of a gate/up pair alternate tile by tile (gate, up, gate, ..) and go to the CTAs in runs of
+// sixteen, so that the 128 columns of a run, a quantisation group of the down projection, end in one CTA.  A CTA works on
+// `slots` of its tiles at a time (one pass): 16 warps as slots / 2 pairs of tiles times `width` groups of K, the warp at
+// place i of a pair taking groups i, i + width, ...  Step s of a pass is one stage of the CTA's stream: for every present
+// tile the 16x128 blocks of groups s * width .. s * width + width - 1 (1 KB of nibbles each, zero beyond `groups`), followed
+// by the same blocks' 32-byte scale-pair rows.
 struct MatrixSchedule {
-    int tiles, units, rt, slots, width, steps, grid;
+    int tiles, groups, run, slots, width, steps, grid;
 };
-__host__ __device__ inline MatrixSchedule stack_schedule(int tiles, int groups, int rt, int grid) {
+__host__ __device__ inline MatrixSchedule stack_schedule(int tiles, int groups, bool pair, int grid) {
     MatrixSchedule s;
-    s.tiles = tiles;
-    s.rt = rt;
-    s.units = groups * rt;
+    s.run = pair ? 16 : 1;
+    s.tiles = pair ? 2 * tiles : tiles;
+    s.groups = groups;
     s.grid = grid;
-    const int most = (tiles + grid - 1) / grid;
-    int slots = 1;
-    while (slots < most && slots * 2 <= 16 / rt) slots *= 2;
-    int width = 16 / slots;
-    while (width / 2 >= rt && width / 2 >= s.units) width /= 2;
-    s.slots = slots;
-    s.width = width;
-    s.steps = (s.units + width - 1) / width;
+    const int most = (s.tiles / s.run + grid - 1) / grid * s.run;
+    int pairs = 1;
+    while (2 * pairs < most && pairs < 8) pairs *= 2;
+    s.slots = 2 * pairs;
+    s.width = 16 / pairs;
+    s.steps = (groups + s.width - 1) / s.width;
     return s;
 }
-__host__ __device__ inline int stack_cta_tiles(const MatrixSchedule &s, int cta) { return s.tiles / s.grid + (cta < s.tiles % s.grid ? 1 : 0); }
+__host__ __device__ inline int stack_cta_tiles(const MatrixSchedule &s, int cta) {
+    const int runs = s.tiles / s.run;
+    return (runs / s.grid + (cta < runs % s.grid ? 1 : 0)) * s.run;
+}
+__host__ __device__ inline int stack_cta_tile(const MatrixSchedule &s, int cta, int i) { return (cta + i / s.run * s.grid) * s.run + i % s.run; }
 // Bytes of the stream in front of CTA `cta`'s share (every tile costs width * steps units of 1056 bytes).
 __host__ __device__ inline size_t stack_cta_offset(const MatrixSchedule &s, int cta) {
-    const int extra = s.tiles % s.grid;
-    const size_t tiles_before = static_cast<size_t>(cta) * (s.tiles / s.grid) + (cta < extra ? cta : extra);
+    const int runs = s.tiles / s.run, extra = runs % s.grid;
+    const size_t tiles_before = (static_cast<size_t>(cta) * (runs / s.grid) + (cta < extra ? cta : extra)) * s.run;
     return tiles_before * s.width * s.steps * 1056;
 }
 __host__ __device__ inline size_t stack_stream_bytes(const MatrixSchedule &s) { return static_cast<size_t>(s.tiles) * s.width * s.steps * 1056; }
@@ -257,8 +260,8 @@ struct StackBuffers {
     uint16_t *hidden;            // [lanes][hidden] residual stream, updated in place
     uint16_t *q;                 // [lanes][q_heads * head_width]
     float *attention_scratch;    // split partials
-    uint16_t *attention_out;     // [lanes][q_heads * head_width] fp16 in fragment order (see kernels_stack.cu)
-    uint16_t *activation;        // [lanes][ffn] fp16 in fragment order
+    uint16_t *attention_out;     // [lanes][q_heads * head_width]
+    uint8_t *activation;         // [lanes][ffn] in operand form: stack_activation_bytes(ffn) bytes (see kernels_stack.cu)
     unsigned int *barrier;       // STACK_BARRIER_WORDS words, zero before the first launch
     int *error_flag;             // set when a bounded wait expires (2: grid barrier or peer, 3: weight pipeline)
     unsigned long long *timing;  // optional [layers][32] nanosecond stamps of CTA 0 (step boundaries), or nullptr
@@ -293,12 +296,12 @@ struct RelayoutSegment {
     int rows;
     int rope_head_width;
 };
-// Segments share K; their tiles follow one another, or - with `pair` - segment 0 and 1 are interleaved unit by unit
-// (gate, up).  Every segment's row count must be a multiple of 16.  `rows` of int4_cta_stream_bytes is the sum of
+// Segments share K; their tiles follow one another, or - with `pair` - those of segment 0 and 1 alternate (gate, up).  Every segment's row count must be a multiple of 16.  `rows` of int4_cta_stream_bytes is the sum of
 // the segments' rows (one segment's for a pair).
 size_t int4_cta_stream_bytes(int rows, int k, bool pair, int grid);
 cudaError_t launch_int4_cta_streams(const RelayoutSegment *segments, int count, bool pair, int k, int grid, uint8_t *out,
                                     cudaStream_t stream);
+size_t stack_activation_bytes(int ffn);  // of StackBuffers::activation, for any batch
 // Whether the stack kernel is built for this shape and batch; *smem_bytes receives its dynamic shared memory.
 bool decode_stack_supported(const StackShape &shape, int lanes, size_t *smem_bytes);
 cudaError_t launch_decode_stack(const StackLayer *layers_device, int layer_count, const StackShape &shape,

@@ -8,38 +8,36 @@
 // SM stays resident and the weight stream never stops for a step boundary:
 //
 //  * weights: at mount every matrix is rewritten as one contiguous byte stream per CTA, in exactly the order the
-//    CTA consumes it (see stack_schedule in kernels.cuh).  A stream is a sequence of stages; a stage is one
-//    16x128 block of packed nibbles (1 KB) plus its 32 bytes of scales for each of up to 16 warps.
+//    CTA consumes it (see stack_schedule in kernels.cuh).  A stream is a sequence of stages; a stage is up to two
+//    16x128 blocks of packed nibbles (1 KB each) and their 32 bytes of scales for each of 16 warps.
 //  * a producer thread (warp 16) walks the CTA's stages of all matrices of all layers and brings them into a ring
 //    in shared memory with one bulk asynchronous copy per stage (mbarrier transaction counts; no cluster forms),
-//    as far ahead as the ring allows - through the grid barriers, the attention step and the epilogues - and asks
-//    L2 for the stages after those (cp.async.bulk.prefetch.L2) so that HBM keeps streaming while the SMs wait on
-//    one another.
-//  * 16 consumer warps: a CTA works on all its tiles of a matrix at once - warp w owns tile slot w / W and every
-//    W-th block of K - so a matrix costs one cross-warp reduction and one epilogue pass per CTA instead of one per
-//    tile.  Nibbles become exact fp16 (q - 8) operands (lop3 into the mantissa of 1024, one fp16 subtract or fma),
-//    eight mma.sync m16n8k16 per block accumulate in f32, the group scale multiplies the block's f32 product as in
+//    as far ahead as the ring allows - through the grid barriers, the attention step and the epilogues.
+//  * 16 consumer warps: a warp multiplies two tiles of 16 rows with every width-th group (128 columns) of K, so a
+//    matrix costs one cross-warp reduction and one epilogue pass per CTA instead of one per tile.  The products are
+//    integers: weights as signed bytes, activations as three signed bytes each, mma.sync m16n8k32 with exact 32-bit
+//    sums (see "matrix blocks"); the group scale multiplies the group's sum in f32 as in
 //    linear_int4_ct.comp.template:80-150.
-//  * activations: the inputs of q/k/v and gate/up are normalised (rms_norm_bf16.comp.template:49-72) by every CTA
-//    into shared memory in mma B-fragment order; the inputs of o and down are written by their producers
-//    (attention merge, SiLU epilogue) to global memory already in fragment order and ride the ring, one slice per
-//    stage, once the grid barrier in front of the step has opened.
+//  * activations: the inputs of q/k/v and gate/up (rms_norm_bf16.comp.template:49-72) and of o are brought into
+//    operand form in shared memory by every CTA; the inputs of down leave the SiLU epilogue in operand form (the
+//    eight tiles of a gate/up pass are one quantisation group of down's columns) and ride a ring of their own, one
+//    slice per step, once the grid barrier in front of the step has opened.
 //  * attention: a team of four warps per (kv head, 64-token split, lane group) on the tensor cores (query rows in
 //    shared memory, K and V rows in registers, all loads of an item requested before its arithmetic); the team that
 //    completes a kv head's last split queues the merge, and after its items the CTA's sixteen warps merge one
 //    (lane, q head) row each - no grid barrier between the splits and their merge.  Lane groups of more than 32
 //    splits are merged in two levels (ranges of 32 splits spread over every warp of the grid, then the ranges of a
 //    row by one warp), with a grid barrier before each level.
-//  * code that runs once per layer (staging, attention, merge, epilogues) is kept short and free of re-read state:
-//    such straight-line code was measured at about 0.27 us per KB of instructions on this kernel (instruction
-//    fetch, not arithmetic), and a value behind a reference is read again after every ordered load.
+//  * registers: everything that outlives a step is kept in shared memory (StackShared), the steps are inlined into one
+//    loop, and the consumers take the registers that the producers hand back.  Half the time of an earlier form of this
+//    kernel was spills: with 227 KB of an SM's memory given to the ring the first-level cache holds about fifty bytes per
+//    thread, and what a function saved around a call came back from L2.
 //  * tensor parallelism (the EXCHANGE instances): o and down push their f32 partial sums, tagged with the exchange
 //    number in the same 8-byte store, into every peer's inbox over NVLink; the owner of an output element waits
 //    for the peers' words in its own memory and adds them in rank order.  No barrier crosses the link.
 //
 // Every wait is bounded: when a bound expires the kernel sets the error word and leaves.
-#include <cuda_fp16.h>
-
+#include <cstddef>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -52,11 +50,20 @@ namespace {
 constexpr int CONSUMER_WARPS = 16;
 constexpr int CONSUMER_THREADS = CONSUMER_WARPS * 32;
 constexpr int STACK_THREADS = CONSUMER_THREADS + 128;  // + the producer warps (registers are allotted four warps at a time)
+// Registers: a launch gives 96 to each of the 640 threads; the producers hand 64 of theirs back, the consumers take 16 more.
+constexpr int PRODUCER_REGISTERS = 32, CONSUMER_REGISTERS = 112;
+static_assert(CONSUMER_THREADS * CONSUMER_REGISTERS + 128 * PRODUCER_REGISTERS <= STACK_THREADS * 96, "the consumers' registers come out of the producers'");
 constexpr int UNIT_BYTES = 1024;                      // packed nibbles of a 16x128 block
 constexpr int UNIT_SCALE_BYTES = 32;                  // its eight scale pairs
 constexpr int UNIT_TOTAL = UNIT_BYTES + UNIT_SCALE_BYTES;
-constexpr int STAGE_WEIGHT_BYTES = 16 * UNIT_TOTAL;   // weight part of a ring stage (16 896 bytes)
+constexpr int STAGE_BYTES = 2 * CONSUMER_WARPS * UNIT_TOTAL;  // a step of a pass: two blocks per consumer warp (33 792 bytes)
 constexpr int MAX_STAGES = 16;
+constexpr uint32_t EMPTY = 8 * MAX_STAGES, SLICE_FULL = 16 * MAX_STAGES, SLICE_EMPTY = 24 * MAX_STAGES;  // barrier arrays, from a slot's `full`
+// Activations in operand form (see stage_rows): two halves and eight factors per group of 128 columns.
+// (an odd number of 64-byte pieces, so that the two halves of a word column fall into different banks)
+__host__ __device__ constexpr uint32_t operand_half_bytes(int lanes) { return static_cast<uint32_t>(lanes) * 192u + (lanes % 2 == 0 ? 64u : 0u); }
+__host__ __device__ constexpr uint32_t operand_group_bytes(int lanes) { return 2u * operand_half_bytes(lanes) + 32u; }
+constexpr uint32_t PRODUCT_BYTES = 8 * 128 * sizeof(float);  // a group of SiLU products of every lane, before it takes operand form
 constexpr unsigned int BARRIER_SPIN_LIMIT = 1u << 20;
 constexpr unsigned int PIPE_SPIN_LIMIT = 1u << 18;  // attempts of about 20 us each at most
 constexpr unsigned int OPEN_SPIN_LIMIT = 1u << 28;  // polls of the barrier count by the slice producer: it has to outlast the consumers' own waits
@@ -74,12 +81,12 @@ struct RelayoutArgs {
     MatrixSchedule schedule;
 };
 
-// Block (stage, cta) writes one stage of one CTA's stream: the present units' nibbles, then their scale pairs.
+// Block (step, cta) writes one step of one CTA's stream: the present tiles' blocks, then their scale pairs.
 __global__ void int4_cta_stream_kernel(const RelayoutArgs args, uint8_t *__restrict__ out) {
     const MatrixSchedule &s = args.schedule;
-    const int cta = blockIdx.y, stage = blockIdx.x;
+    const int cta = blockIdx.y;
     const int here = stack_cta_tiles(s, cta);
-    const int pass = stage / s.steps, step = stage % s.steps;
+    const int pass = blockIdx.x / s.steps, step = blockIdx.x % s.steps;
     int present = here - pass * s.slots;
     if (present <= 0) return;
     if (present > s.slots) present = s.slots;
@@ -88,16 +95,16 @@ __global__ void int4_cta_stream_kernel(const RelayoutArgs args, uint8_t *__restr
                     static_cast<size_t>(step) * present * s.width * UNIT_TOTAL;
     uint4 *weights_out = reinterpret_cast<uint4 *>(base);
     uint32_t *scales_out = reinterpret_cast<uint32_t *>(base + static_cast<size_t>(present) * s.width * UNIT_BYTES);
-    auto locate = [&](int unit_in_stage, int &group, int &which, int &local_tile) {
-        const int slot = unit_in_stage / s.width, i = unit_in_stage % s.width;
-        const int unit = step * s.width + i;
-        if (unit >= s.units) return false;  // padding of a ragged last step: zero nibbles under zero scales
-        group = unit / s.rt;
-        const int tile = cta + (pass * s.slots + slot) * s.grid;
+    auto locate = [&](int unit_in_step, int &group, int &which, int &local_tile) {
+        const int slot = unit_in_step / s.width;
+        group = step * s.width + unit_in_step % s.width;
+        if (group >= s.groups) return false;  // padding of a ragged last step: zeros under zero scales
+        const int tile = stack_cta_tile(s, cta, pass * s.slots + slot);
         which = 0;
         local_tile = tile;
-        if (args.pair) {
-            which = unit % s.rt;
+        if (args.pair) {  // gate and up rows alternate
+            which = tile & 1;
+            local_tile = tile >> 1;
         } else {
             while (which + 1 < args.count && tile >= args.first_tile[which + 1]) which++;
             local_tile = tile - args.first_tile[which];
@@ -115,22 +122,23 @@ __global__ void int4_cta_stream_kernel(const RelayoutArgs args, uint8_t *__restr
     };
     const int units = present * s.width;
     for (int index = threadIdx.x; index < units * 64; index += blockDim.x) {
-        const int unit_in_stage = index >> 6, half = (index >> 5) & 1, lane = index & 31;
+        const int unit_in_step = index >> 6, half = (index >> 5) & 1, lane = index & 31;
         const int g = lane >> 2, j = lane & 3;
         int group = 0, which = 0, local_tile = 0;
         uint4 value = make_uint4(0, 0, 0, 0);
-        if (locate(unit_in_stage, group, which, local_tile)) {
+        if (locate(unit_in_step, group, which, local_tile)) {
             const RelayoutSegment &segment = args.segment[which];
             const int row = source_row(segment, local_tile, g + 8 * half);
             value = *reinterpret_cast<const uint4 *>(segment.qweight + static_cast<size_t>(row) * (args.k >> 3) + group * 16 + j * 4);
+            value.x ^= 0x88888888u, value.y ^= 0x88888888u, value.z ^= 0x88888888u, value.w ^= 0x88888888u;  // q -> q - 8 in two's complement
         }
         weights_out[index] = value;
     }
     for (int index = threadIdx.x; index < units * 8; index += blockDim.x) {
-        const int unit_in_stage = index >> 3, g = index & 7;
+        const int unit_in_step = index >> 3, g = index & 7;
         int group = 0, which = 0, local_tile = 0;
         uint32_t value = 0;
-        if (locate(unit_in_stage, group, which, local_tile)) {
+        if (locate(unit_in_step, group, which, local_tile)) {
             const RelayoutSegment &segment = args.segment[which];
             const uint32_t low = segment.scales[static_cast<size_t>(source_row(segment, local_tile, g)) * groups + group];
             const uint32_t high = segment.scales[static_cast<size_t>(source_row(segment, local_tile, g + 8)) * groups + group];
@@ -149,35 +157,34 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void mma_f16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                              uint32_t b1) {
-    asm(
-        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+// 16x32 signed bytes times 32x8 signed bytes, exact sums.  D and C are different operands: C starts a chain.
+__device__ __forceinline__ void mma_s8_16832(int32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1, int32_t c0,
+                                             int32_t c1, int32_t c2, int32_t c3) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};\n"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c0), "r"(c1), "r"(c2), "r"(c3));
 }
 
-// Two nibbles of `word` (bits 0..3 and 16..19) -> fp16x2 (q - 8, q' - 8), exactly: the nibble lands in the low
-// mantissa bits of 1024.0 (0x6400), 1032 is subtracted.
-__device__ __forceinline__ uint32_t nibbles_low(uint32_t word) {
-    uint32_t biased, out;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(biased) : "r"(word), "n"(0x000F000F), "n"(0x64006400));
-    asm("sub.f16x2 %0, %1, %2;" : "=r"(out) : "r"(biased), "r"(0x64086408u));
-    return out;
+// Pairs of f32 in one register pair (two IEEE operations per instruction).
+__device__ __forceinline__ unsigned long long pair_of(float lo, float hi) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
 }
-// The nibbles at bits 4..7 and 20..23: 1024 + 16 q, times 1/16, minus 72 (one fused multiply-add, exact).
-__device__ __forceinline__ uint32_t nibbles_high(uint32_t word) {
-    uint32_t biased, out;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(biased) : "r"(word), "n"(0x00F000F0), "n"(0x64006400));
-    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(out) : "r"(biased), "r"(0x2C002C00u), "r"(0xD480D480u));
-    return out;
+__device__ __forceinline__ unsigned long long pair_add(unsigned long long a, unsigned long long b) {
+    unsigned long long v;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
 }
-
-// bf16 values (already rounded) as an fp16 pair: exact for magnitudes in [2^-14, 65504]; the activations of a
-// decoder layer (normalised rows, attention outputs, SiLU products) live there.
-__device__ __forceinline__ uint32_t half_pair(float lo, float hi) {
-    const __half2 h = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t *>(&h);
+__device__ __forceinline__ unsigned long long pair_multiply(unsigned long long a, unsigned long long b) {
+    unsigned long long v;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ unsigned long long pair_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+    return v;
 }
 
 __device__ __forceinline__ uint32_t load_acquire(const unsigned int *address) {
@@ -186,28 +193,8 @@ __device__ __forceinline__ uint32_t load_acquire(const unsigned int *address) {
     return value;
 }
 
-__device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
+__device__ __forceinline__ void cta_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }  // of the consumers
 __device__ __forceinline__ void team_barrier(int barrier_id) { asm volatile("bar.sync %0, 128;" ::"r"(barrier_id) : "memory"); }
-
-// All CTAs of the (cooperative, co-resident) grid meet here; only the consumer warps take part.  `target` counts
-// the arrivals expected so far.  A wait that does not complete within the spin limit sets the error flag and lets
-// the CTA go on (its results are then garbage, the host sees the flag); once the flag is up nobody waits any more.
-__device__ __noinline__ void grid_barrier(unsigned int *counter, unsigned int &target, int *error_flag, unsigned int spin_limit) {
-    consumer_sync();
-    if (threadIdx.x == 0) {
-        target += gridDim.x;
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");  // covers the CTA's writes before the barrier above
-        unsigned int spins = 0;
-        while (load_acquire(counter) < target) {
-            if (++spins > spin_limit) {
-                atomicExch(error_flag, 2);
-                break;
-            }
-            if ((spins & 63u) == 0 && *reinterpret_cast<volatile int *>(error_flag) != 0) break;
-        }
-    }
-    consumer_sync();
-}
 
 // ---- mbarrier / bulk copy (shared-space addresses)
 __device__ __forceinline__ void mbarrier_init(uint32_t address, uint32_t count) {
@@ -241,9 +228,6 @@ __device__ __forceinline__ void bulk_load(uint32_t destination, const void *sour
                  "l"(__cvta_generic_to_global(source)), "r"(bytes), "r"(barrier)
                  : "memory");
 }
-__device__ __forceinline__ void prefetch_l2(const void *address, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(address)), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ uint32_t shared_load_acquire(uint32_t address) {
     uint32_t value;
     asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(value) : "r"(address) : "memory");
@@ -259,21 +243,15 @@ __device__ __forceinline__ uint4 shared_load16(uint32_t address) {
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4+%5];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(address), "n"(OFFSET) : "memory");
     return v;
 }
-__device__ __forceinline__ uint32_t shared_load4(uint32_t address) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(address) : "memory");
-    return v;
-}
-
-
 // ------------------------------------------------------------------------------------------ the CTA's view of a matrix
 
 struct PhaseInfo {
-    int tiles_here;       // 16-row tiles of this CTA (tile = cta + i * grid)
+    int tiles_here;       // 16-row tiles of this CTA, see stack_cta_tile
     int passes;           // rounds of `slots` tiles
-    int slots, width, steps, units, rt, groups;
+    int slots, width, steps, groups;
+    int width_log2;       // width is a power of two
+    int window;           // steps whose activations are staged at a time
     uint32_t cta_offset;  // bytes from the matrix's stream to this CTA's share
-    int streamed;         // the activations ride the ring (o, down)
 };
 
 struct StackArgs {
@@ -283,13 +261,114 @@ struct StackArgs {
     StackBuffers buffers;
     LaneTable lanes_meta;
     int lanes, lanes_per_stream, max_splits;
-    int stages, stage_bytes, prefetch_stages, debug_flags;
-    int steps_per_stage;                 // consecutive steps of a pass that travel as one ring stage (1 or 2)
-    int slice_slots, slice_bytes;        // ring of activation slices (o, down) inside the scratch area
+    int stages;
+    int slice_slots, slice_bytes;        // ring of activation slices (down, one step each) inside the scratch area
     uint32_t scratch_bytes;
     const StackTp *tp;  // device copy of the exchange description, or nullptr (single GPU)
     int tp_size;
 };
+
+// Merges a CTA can be left with in a layer: at most one per work item, of at most (1024 - 16) arrival counters x 32 splits
+// on 148 CTAs.
+constexpr int ATTENTION_MERGE_LIST = 256;
+struct AttentionItem {
+    int16_t kv_head, split;     // the kv head, the context split
+    int16_t lane0, lanes;       // the query lanes
+    int32_t slot, arrival;      // the stream's slot; kv_head * group_slots + lane group, the split counter
+    int32_t count, splits;      // tokens of the split (0: nothing to do); splits of the whole context
+    uint32_t first_tick, ring_base;  // of its first token
+};
+// What a warp does in a pass of a matrix: two tiles of 16 rows, every width-th group of K.
+struct WarpBlocks {
+    uint32_t unit, scales;      // its first block inside a stage, and on to that block's scales
+    uint32_t next_tile;         // on to the second tile's block (its scales are 1 / 32 of that further)
+    uint32_t x;                 // its group of the first step: from the staged rows, inside the slice of a step
+    uint32_t x_step;            // on to the group of the next step; slices: to the next slot
+    int steps;                  // steps that hold a group of the warp (0 if it has no tile)
+    int tiles;                  // 1 or 2
+};
+struct OperandPlace {  // where a thread's B fragments are inside a group
+    uint32_t first, second, half, factor;
+};
+
+// What the CTA's threads share, at the start of its shared memory; the scratch area (staged rows and SiLU products /
+// attention teams / slices of down) and the ring follow.  All state that outlives a step is kept
+// here, not in registers: a value that is live across the steps' functions is spilled, and with 227 KB of the SM's memory
+// given to the ring the spills miss the first-level cache (a version with 0.5 KB of them took twice the time).
+struct StackShared {
+    uint64_t full[MAX_STAGES], empty[MAX_STAGES], slice_full[MAX_STAGES], slice_empty[MAX_STAGES];
+    StackArgs a;
+    PhaseInfo info[4];
+    StackLayer layer[2];        // the current layer's description (layer & 1) and the next one's, copied ahead of their use
+    uint32_t scratch, ring;     // offsets from the start
+    uint32_t products;          // where the SiLU products of a pass of gate/up go, f32 [lane][128]: an offset
+    uint32_t place;             // where the consumers stand in the two rings (pack_place)
+    uint32_t open_word;         // counted grid barriers passed (read by the producer of slices)
+    uint32_t barrier_target;    // arrivals expected at the grid barriers so far
+    uint32_t barrier_limit;     // polls
+    WarpBlocks blocks[4][CONSUMER_WARPS];  // of the first pass of each matrix step
+    OperandPlace operand_place[32];     // by lane of the warp
+    uint32_t output[CONSUMER_THREADS];     // o and down: the thread's first output in the residual stream (see matrix_step)
+    uint32_t exchanges;         // tensor-parallel exchanges of earlier launches
+    // lanes
+    uint32_t tick[8];
+    int32_t slot[8];
+    uint64_t kv_row[8];         // element offset of the lane's K row (kv head 0) in a layer's pool, ~0 if it has none
+    uint32_t rope[8 * 64];      // [lane][HD / 2] rotary factors of the lanes' positions
+    // attention: for each team the KV rows of its first work item (the block table is shared by all layers, so the rows
+    // of a (split, lane group) are the same in every layer's pool)
+    int32_t group_slots;        // lane groups of all streams
+    AttentionItem item[4], later_item[4];
+    int32_t merge_count;        // (kv head, lane group) pairs whose last split this CTA's teams completed in this layer ...
+    uint16_t merge_list[ATTENTION_MERGE_LIST];  // ... and which: kv_head * group_slots + group_slot
+    uint32_t row_base[4][64];   // offset (in rows of HD elements) of token t's K row of kv head 0 in a layer's pool
+    float norm_partial[4 * CONSUMER_WARPS];
+    alignas(16) float reduce[CONSUMER_WARPS][2][128];  // the warps' partial sums: [warp][tile of its pair][row][lane]
+};
+extern __shared__ __align__(128) uint8_t smem_raw[];
+__device__ __forceinline__ StackShared &shared() { return *reinterpret_cast<StackShared *>(smem_raw); }
+__device__ __forceinline__ uint32_t shared_address(const void *object) { return static_cast<uint32_t>(__cvta_generic_to_shared(object)); }
+__device__ __forceinline__ uint4 smem16(uint32_t offset) { return *reinterpret_cast<const uint4 *>(smem_raw + offset); }
+__device__ __forceinline__ uint32_t smem4(uint32_t offset) { return *reinterpret_cast<const uint32_t *>(smem_raw + offset); }
+// The thread's number, read anew: what is derived from it is not kept across the steps of a layer.
+__device__ __forceinline__ int thread_now() {
+    int thread;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(thread));
+    return thread;
+}
+
+// All CTAs of the (cooperative, co-resident) grid meet here; only the consumer warps take part.  A wait that does not
+// complete within the spin limit sets the error flag and lets the CTA go on (its results are then garbage, the host sees
+// the flag); once the flag is up nobody waits any more.  Counted barriers are those the producer of slices waits for.
+__device__ __forceinline__ void grid_meet(bool counted) {
+    cta_sync();
+    if (threadIdx.x == 0) {
+        StackShared &sh = shared();
+        unsigned int *counter = sh.a.buffers.barrier;
+        int *error_flag = sh.a.buffers.error_flag;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");  // covers the CTA's writes before the barrier above
+        const unsigned int target = sh.barrier_target + gridDim.x, limit = sh.barrier_limit;
+        sh.barrier_target = target;
+        unsigned int spins = 0;
+        while (load_acquire(counter) < target) {
+            if (++spins > limit) {
+                atomicExch(error_flag, 2);
+                break;
+            }
+            if ((spins & 63u) == 0 && *reinterpret_cast<volatile int *>(error_flag) != 0) break;
+        }
+        if (counted) shared_store_release(shared_address(&sh.open_word), sh.open_word + 1u);
+    }
+    cta_sync();
+}
+__device__ __forceinline__ void stamp(int layer, int index) {  // step times of CTA 0, for tests and profiles
+    unsigned long long *timing = shared().a.buffers.timing;
+    if (timing != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
+        unsigned long long now;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        timing[layer * 32 + index] = now;
+    }
+}
 
 __device__ __forceinline__ const uint8_t *layer_stream(const StackLayer &layer, int phase) {
     return phase == 0 ? layer.qkv : (phase == 1 ? layer.o : (phase == 2 ? layer.gate_up : layer.down));
@@ -301,17 +380,11 @@ __device__ __forceinline__ int stage_present(const PhaseInfo &pi, int pass) {
 }
 
 // ------------------------------------------------------------------------------------------ producers
-// Three single threads (lane 0 of warps 16, 17, 18) walk the CTA's stage sequence - for every layer the four
-// matrices, for every matrix its passes and steps - each on its own: one requests the weights of a stage, one the
-// activation slice of the stages of o and down (once the grid barrier in front of the step has opened), one asks
-// L2 for stages further ahead.  A stage's slot is free when the consumer warps have released its previous use
-// (the `empty` barrier); its `full` barrier completes with two arrivals plus the bytes of the copies.
-
-struct RingAddresses {
-    uint32_t ring, full, empty;                       // weight stages (shared-space addresses)
-    uint32_t slices, slice_full, slice_empty;         // activation slices of the o and down steps
-    uint32_t open_word, issued_word;
-};
+// Two single threads (lane 0 of warps 16 and 17) walk the CTA's sequence - for every layer the four matrices, for
+// every matrix its passes and steps - each on its own: one requests the weights, a step of a pass as one
+// stage, the other the activation slice of every step of down (once the grid barrier in front of it has
+// opened).  A slot is free when the consumer warps have released its previous use (the `empty` barrier); its
+// `full` barrier completes with the producer's arrival plus the bytes of the copy.
 
 struct RingPosition {
     uint32_t slot, parity;  // parity of the `empty` phase that frees the slot for the next use
@@ -321,11 +394,6 @@ __device__ __forceinline__ void ring_advance(RingPosition &position, uint32_t st
         position.slot = 0;
         position.parity ^= 1u;
     }
-}
-__device__ __forceinline__ void ring_skip(RingPosition &position, uint32_t count, uint32_t stages) {
-    const uint32_t to = position.slot + count;
-    position.parity ^= (to / stages) & 1u;
-    position.slot = to % stages;
 }
 // false: gave up (the error flag is set, or was set by somebody else)
 __device__ __forceinline__ bool wait_slot_free(uint32_t empty_address, const RingPosition &position, int *error_flag) {
@@ -344,118 +412,73 @@ __device__ __forceinline__ void linger() {
     for (int i = 0; i < 64; i++) __nanosleep(1000);
 }
 
-__device__ __noinline__ void produce_weights(const StackArgs &a, const PhaseInfo *info, const RingAddresses &ring) {
-    int *error_flag = a.buffers.error_flag;
+__device__ __forceinline__ void produce_weights() {
+    const StackShared &sh = shared();
+    int *error_flag = sh.a.buffers.error_flag;
+    const uint32_t stages = static_cast<uint32_t>(sh.a.stages), ring = shared_address(smem_raw + sh.ring), empty = shared_address(sh.empty), full = shared_address(sh.full);
     RingPosition position{0u, 1u};
-    uint32_t issued = 0;
-    for (int layer = 0; layer < a.layer_count; layer++) {
-        const StackLayer *spec = a.layers + layer;
+    for (int layer = 0; layer < sh.a.layer_count; layer++) {
+        const StackLayer *spec = sh.a.layers + layer;
         for (int phase = 0; phase < 4; phase++) {
-            const PhaseInfo pi = info[phase];
+            const PhaseInfo pi = sh.info[phase];
             if (pi.passes == 0) continue;
             const uint8_t *source = layer_stream(*spec, phase) + pi.cta_offset;
             for (int pass = 0; pass < pi.passes; pass++) {
-                const uint32_t step_bytes = static_cast<uint32_t>(stage_present(pi, pass) * pi.width * UNIT_TOTAL);
-                for (int step = 0; step < pi.steps; step += a.steps_per_stage) {
-                    const int count = pi.steps - step < a.steps_per_stage ? pi.steps - step : a.steps_per_stage;
-                    const uint32_t bytes = step_bytes * static_cast<uint32_t>(count);
-                    if (!wait_slot_free(ring.empty, position, error_flag)) return linger();
-                    const uint32_t full = ring.full + position.slot * 8;
-                    if ((a.debug_flags & 4) && issued >= static_cast<uint32_t>(a.stages)) {
-                        mbarrier_arrive(full);  // timing probe: the consumers work on what the slot already holds
-                    } else {
-                        mbarrier_arrive_expect(full, bytes);
-                        bulk_load(ring.ring + position.slot * static_cast<uint32_t>(a.stage_bytes), source, bytes, full);
-                    }
+                const uint32_t bytes = static_cast<uint32_t>(stage_present(pi, pass) * pi.width * UNIT_TOTAL);
+                for (int step = 0; step < pi.steps; step++) {
+                    if (!wait_slot_free(empty, position, error_flag)) return linger();
+                    mbarrier_arrive_expect(full + position.slot * 8, bytes);
+                    bulk_load(ring + position.slot * static_cast<uint32_t>(STAGE_BYTES), source, bytes, full + position.slot * 8);
                     source += bytes;
-                    ring_advance(position, static_cast<uint32_t>(a.stages));
-                    if (a.debug_flags & 4) issued++;
-                    if (a.prefetch_stages > 0) asm volatile("st.volatile.shared::cta.u32 [%0], %1;" ::"r"(ring.issued_word), "r"(++issued) : "memory");
+                    ring_advance(position, stages);
                 }
             }
         }
     }
 }
 
-__device__ __noinline__ void produce_activations(const StackArgs &a, const PhaseInfo *info, const RingAddresses &ring, int staged) {
-    int *error_flag = a.buffers.error_flag;
-    RingPosition position{0u, 1u};  // in the ring of slices: only the stages of o and down count
-    const uint32_t slice_group_bytes = static_cast<uint32_t>(staged) * 256u;
-    for (int layer = 0; layer < a.layer_count; layer++) {
-        for (int phase = 1; phase < 4; phase += 2) {
-            const PhaseInfo pi = info[phase];
-            if (pi.passes == 0) continue;
-            // the slices were written by other CTAs with ordinary stores before the grid barrier counted here; the
-            // scratch area they land in is free once this CTA's consumers have passed that barrier, too
-            const uint32_t needed = static_cast<uint32_t>(layer * BARRIERS_PER_LAYER + (phase == 1 ? 2 : 4));
-            unsigned int spins = 0;
-            while (shared_load_acquire(ring.open_word) < needed) {
-                if (++spins > OPEN_SPIN_LIMIT) {
-                    atomicExch(error_flag, 3);
-                    return linger();
-                }
-                if ((spins & 255u) == 0 && *reinterpret_cast<volatile int *>(error_flag) != 0) return linger();
-                __nanosleep(20);
+__device__ __forceinline__ void produce_activations() {
+    const StackShared &sh = shared();
+    int *error_flag = sh.a.buffers.error_flag;
+    const uint32_t slots = static_cast<uint32_t>(sh.a.slice_slots), slices = shared_address(smem_raw + sh.scratch), empty = shared_address(sh.slice_empty),
+                   full = shared_address(sh.slice_full), slice_bytes = static_cast<uint32_t>(sh.a.slice_bytes), group_bytes = operand_group_bytes(sh.a.lanes);
+    RingPosition position{0u, 1u};
+    const PhaseInfo pi = sh.info[3];
+    if (pi.passes == 0) return;
+    for (int layer = 0; layer < sh.a.layer_count; layer++) {
+        // the slices were written by other CTAs with ordinary stores before the grid barrier counted here; the
+        // scratch area they land in is free once this CTA's consumers have passed that barrier, too
+        const uint32_t needed = static_cast<uint32_t>(layer * BARRIERS_PER_LAYER + 4);
+        unsigned int spins = 0;
+        while (shared_load_acquire(shared_address(&sh.open_word)) < needed) {
+            if (++spins > OPEN_SPIN_LIMIT) {
+                atomicExch(error_flag, 3);
+                return linger();
             }
-            asm volatile("fence.proxy.async;" ::: "memory");  // ... and the copy engine reads them
-            const uint8_t *base = reinterpret_cast<const uint8_t *>(phase == 1 ? a.buffers.attention_out : a.buffers.activation);
-            const int groups_per_stage = pi.width * a.steps_per_stage;
-            for (int pass = 0; pass < pi.passes; pass++) {
-                for (int first_group = 0; first_group < pi.steps * pi.width; first_group += groups_per_stage) {
-                    if (!wait_slot_free(ring.slice_empty, position, error_flag)) return linger();
-                    int groups = pi.groups - first_group;
-                    if (groups > groups_per_stage) groups = groups_per_stage;
-                    const uint32_t full = ring.slice_full + position.slot * 8;
-                    if (groups > 0) {
-                        const uint32_t bytes = static_cast<uint32_t>(groups) * slice_group_bytes;
-                        mbarrier_arrive_expect(full, bytes);
-                        bulk_load(ring.slices + position.slot * static_cast<uint32_t>(a.slice_bytes), base + static_cast<size_t>(first_group) * slice_group_bytes,
-                                  bytes, full);
-                    } else {
-                        mbarrier_arrive(full);  // a stage of padding only
-                    }
-                    ring_advance(position, static_cast<uint32_t>(a.slice_slots));
-                }
+            if ((spins & 255u) == 0 && *reinterpret_cast<volatile int *>(error_flag) != 0) return linger();
+            __nanosleep(20);
+        }
+        asm volatile("fence.proxy.async;" ::: "memory");  // ... and the copy engine reads them
+        for (int pass = 0; pass < pi.passes; pass++) {
+            const uint8_t *source = sh.a.buffers.activation;
+            for (int first_group = 0; first_group < pi.groups; first_group += pi.width) {
+                if (!wait_slot_free(empty, position, error_flag)) return linger();
+                const int groups = pi.groups - first_group < pi.width ? pi.groups - first_group : pi.width;
+                const uint32_t bytes = static_cast<uint32_t>(groups) * group_bytes;
+                mbarrier_arrive_expect(full + position.slot * 8, bytes);
+                bulk_load(slices + position.slot * slice_bytes, source, bytes, full + position.slot * 8);
+                source += bytes;
+                ring_advance(position, slots);
             }
         }
     }
 }
 
-// Keeps `prefetch_stages` stages beyond the last requested one on their way into L2.
-__device__ __noinline__ void produce_prefetches(const StackArgs &a, const PhaseInfo *info, const RingAddresses &ring) {
-    int *error_flag = a.buffers.error_flag;
-    uint32_t index = 0;
-    for (int layer = 0; layer < a.layer_count; layer++) {
-        const StackLayer *spec = a.layers + layer;
-        for (int phase = 0; phase < 4; phase++) {
-            const PhaseInfo pi = info[phase];
-            if (pi.passes == 0) continue;
-            const uint8_t *source = layer_stream(*spec, phase) + pi.cta_offset;
-            for (int pass = 0; pass < pi.passes; pass++) {
-                const uint32_t step_bytes = static_cast<uint32_t>(stage_present(pi, pass) * pi.width * UNIT_TOTAL);
-                for (int step = 0; step < pi.steps; step += a.steps_per_stage, index++) {
-                    const int count = pi.steps - step < a.steps_per_stage ? pi.steps - step : a.steps_per_stage;
-                    const uint32_t bytes = step_bytes * static_cast<uint32_t>(count);
-                    unsigned int spins = 0;
-                    uint32_t issued;
-                    while (true) {
-                        asm volatile("ld.volatile.shared::cta.u32 %0, [%1];" : "=r"(issued) : "r"(ring.issued_word) : "memory");
-                        if (index < issued + static_cast<uint32_t>(a.prefetch_stages)) break;
-                        if (++spins > OPEN_SPIN_LIMIT || ((spins & 255u) == 0 && *reinterpret_cast<volatile int *>(error_flag) != 0)) return;
-                        __nanosleep(100);
-                    }
-                    if (index >= issued + static_cast<uint32_t>(a.stages)) prefetch_l2(source, bytes);  // nearer stages are being loaded already
-                    source += bytes;
-                }
-            }
-        }
-    }
-}
-
-// Consumer side of the ring: waits (bounded) until stage `slot` holds its data.
-__device__ __forceinline__ void wait_stage(uint32_t full_address, uint32_t parity, int *error_flag) {
+// Waits (bounded) until a barrier's phase of the given parity is complete.
+__device__ __forceinline__ void wait_barrier(uint32_t barrier, uint32_t parity) {
     unsigned int spins = 0;
-    while (!mbarrier_test(full_address, parity)) {
+    while (!mbarrier_test(barrier, parity)) {
+        int *error_flag = shared().a.buffers.error_flag;
         if (++spins > PIPE_SPIN_LIMIT) {
             atomicExch(error_flag, 3);
             break;
@@ -463,148 +486,245 @@ __device__ __forceinline__ void wait_stage(uint32_t full_address, uint32_t parit
         if ((spins & 255u) == 0 && *reinterpret_cast<volatile int *>(error_flag) != 0) break;
     }
 }
-
 // ------------------------------------------------------------------------------------------ activation staging
 
-// Chunk c (8 consecutive columns) of lane m -> the fragment slot of thread (g = m, j) for word w, with
-// group = c / 16, j = (c / 4) % 4, w = c % 4: uint4 index ((group * 4 + w) * staged + m) * 4 + j, holding the fp16
-// pairs (v0,v4) (v1,v5) (v2,v6) (v3,v7) - the B operands of the MMAs that consume nibble pairs (0,4) (1,5) and
-// (2,6) (3,7) of the matching weight word.
-__device__ __forceinline__ int fragment_index(int chunk, int m, int staged) {
-    const int group = chunk >> 4, j = (chunk >> 2) & 3, word = chunk & 3;
-    return ((group * 4 + word) * staged + m) * 4 + j;
+// The operand form of activations.  A group (128 columns) of a lane is held as whole numbers X of 23 bits over one
+// power of two - x = X 2^(e - 21), e the exponent of the largest magnitude of the group (of the warp's two groups where
+// rows are staged) - and X as three signed bytes,
+// X = t0 2^16 + t1 2^8 + t2: the group's products with the four-bit weights then add up exactly in 32-bit integers,
+// whatever their order, and what f32 rounds is the group's sum, as in linear_int4_ct.comp.template:80-150.  A bf16
+// value down to 2^-14 of that largest is carried exactly, a smaller one to 2^-22 of it.
+//
+// A group takes operand_group_bytes(lanes) bytes: [half h][lane][term t][j] pieces of 16 bytes (the B fragments of
+// MMAs 2h and 2h + 1 for thread column j: the digits of the eight columns of word 4j + 2h, even columns first, then
+// those of word 4j + 2h + 1), then one f32 factor per lane, what a unit of t2 times a weight of one is worth.
+__device__ __forceinline__ uint32_t operand_word_offset(int word, int m, int lanes) {  // of term 0; term t is 64 t further
+    return static_cast<uint32_t>((word >> 1) & 1) * operand_half_bytes(lanes) + static_cast<uint32_t>(m) * 192u + static_cast<uint32_t>(word >> 2) * 16u +
+           static_cast<uint32_t>(word & 1) * 8u;
 }
-// Position (in 16-bit elements) of column `column` of lane m in a fragment-ordered buffer.
-__device__ __forceinline__ size_t fragment_element(int column, int m, int staged) {
-    const int e = column & 7;
-    return static_cast<size_t>(fragment_index(column >> 3, m, staged)) * 8 + (e & 3) * 2 + (e >> 2);
+// From the exponent field of a group's largest magnitude: the factor onto X, and the group's factor (2^-4 of it since
+// the MMA sees sixteen times the weights).  A group that holds an infinity or a NaN makes its sums NaN.
+__device__ __forceinline__ float operand_scale(uint32_t exponent) { return __uint_as_float((275u - (exponent < 32u ? 32u : exponent)) << 23); }
+__device__ __forceinline__ float operand_factor(uint32_t exponent) {
+    return __uint_as_float(exponent == 255u ? 0x7fc00000u : ((exponent < 32u ? 32u : exponent) - 25u) << 23);
+}
+// The digits of four whole numbers as three words (term 0 first).  A number comes as the bits of 1.5 * 2^23 + X, which
+// is how f32 rounds to whole numbers; 2^7 in front of each digit makes its byte unsigned, so that no digit borrows from
+// the next.  (The additions are multiply-adds by an opaque one: they leave the half-rate integer pipe to the permutes.)
+constexpr float WHOLE_BIAS = 12582912.0f;
+struct DigitConstants {  // made where they are used: the compiler would keep them in registers through the whole layer
+    uint32_t one, digits;
+    unsigned long long bias;  // a pair
+};
+__device__ __forceinline__ DigitConstants digit_constants() {
+    DigitConstants c;
+    asm volatile("mov.b32 %0, 1;" : "=r"(c.one));
+    asm volatile("mov.b32 %0, 0x00408080;" : "=r"(c.digits));
+    asm volatile("mov.b64 %0, 0x4B4000004B400000;" : "=l"(c.bias));
+    return c;
+}
+__device__ __forceinline__ void operand_digits(uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3, const DigitConstants &c, uint32_t (&terms)[3]) {
+    const uint32_t y0 = x0 * c.one + c.digits, y1 = x1 * c.one + c.digits, y2 = x2 * c.one + c.digits, y3 = x3 * c.one + c.digits;
+    const uint32_t low01 = __byte_perm(y0, y1, 0x5140), low23 = __byte_perm(y2, y3, 0x5140);
+    terms[0] = __byte_perm(__byte_perm(y0, y1, 0x0062), __byte_perm(y2, y3, 0x0062), 0x5410) ^ 0x80808080u;
+    terms[1] = __byte_perm(low01, low23, 0x7632) ^ 0x80808080u;
+    terms[2] = __byte_perm(low01, low23, 0x5410) ^ 0x80808080u;
+}
+__device__ __forceinline__ uint32_t larger_halves(uint32_t a, uint32_t b) {
+    uint32_t v;
+    asm("max.u16x2 %0, %1, %2;" : "=r"(v) : "r"(a), "r"(b));
+    return v;
 }
 
-// rms_norm_bf16.comp.template:49-72 of every staged lane, straight into fragment order (each CTA repeats it:
-// 8 KB per lane from L2).  A thread owns chunk t (and t + 512 when CHUNKS = 2) of each lane, four lanes at a time:
-// one pass over registers for the sums of squares, one block-wide exchange, then normalise, round and permute.
-// Two f32 values rounded to bf16 (nearest even, as the shaders' f32_to_bf16 for every finite value) and carried on
-// as the fp16 pair the tensor cores read: exact, a bf16 of this range fits fp16.
-__device__ __forceinline__ uint32_t bf16_rounded_half_pair(float lo, float hi) {
-    uint32_t packed, halves;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(packed) : "f"(hi), "f"(lo));
-    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(halves) : "f"(bf16_hi(packed)), "f"(bf16_lo(packed)));
-    return halves;
-}
-
-template <int CHUNKS>  // chunks per thread and lane: width <= CHUNKS * 8 * CONSUMER_THREADS
-__device__ __noinline__ void stage_normalised(uint4 *fragments, float *partial, const uint16_t *x, const uint16_t *weight, int width,
-                                                 int staged, float eps, float offset) {
-    const int per_lane = width >> 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// Rows into operand form, groups [first_group, first_group + groups) of them: with `weight` their rms_norm
+// (rms_norm_bf16.comp.template:49-72), without it the bf16 values as they are.  Each CTA repeats it: 8 KB per lane
+// from L2.  A thread owns chunk t (and t + 512 when CHUNKS = 2) of each lane, four lanes at a time: one pass over
+// registers for the sums of squares, one block-wide exchange, then normalise, round, find the exponent and cut the digits.
+template <int CHUNKS, int LANES>  // chunks per thread and lane: width <= CHUNKS * 8 * CONSUMER_THREADS; lanes at a time (1, 2 or 4)
+__device__ __forceinline__ void stage_rows(const uint16_t *x, const uint16_t *weight, int width, int first_group, int groups) {
+    const StackShared &sh = shared();
+    uint8_t *operands = smem_raw + sh.scratch;
+    float *partial = shared().norm_partial;
+    const int lanes = sh.a.lanes, per_lane = width >> 3, thread = thread_now(), warp = thread >> 5, lane = thread & 31;
+    const float eps = sh.a.shape.eps, offset = sh.a.shape.norm_offset;
+    const DigitConstants constants = digit_constants();
     const uint4 *source = reinterpret_cast<const uint4 *>(x);
     uint4 scale_words[CHUNKS];
 #pragma unroll
     for (int c = 0; c < CHUNKS; c++) {
-        const int chunk = threadIdx.x + c * CONSUMER_THREADS;
-        scale_words[c] = chunk < per_lane ? __ldg(reinterpret_cast<const uint4 *>(weight) + chunk) : make_uint4(0, 0, 0, 0);
+        const int chunk = thread + c * CONSUMER_THREADS;
+        scale_words[c] = weight != nullptr && chunk < per_lane ? __ldg(reinterpret_cast<const uint4 *>(weight) + chunk) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll 1
-    for (int m0 = 0; m0 < staged; m0 += 4) {
-        uint4 raw[4][CHUNKS];
+    for (int m0 = 0; m0 < lanes; m0 += LANES) {
+        uint4 raw[LANES][CHUNKS];
 #pragma unroll
-        for (int mm = 0; mm < 4; mm++)
+        for (int mm = 0; mm < LANES; mm++)
 #pragma unroll
             for (int c = 0; c < CHUNKS; c++) {
-                const int chunk = threadIdx.x + c * CONSUMER_THREADS;
+                const int chunk = thread + c * CONSUMER_THREADS;
                 // lanes beyond the batch read the last lane again (their results are not stored)
-                const int m = m0 + mm < staged ? m0 + mm : staged - 1;
+                const int m = m0 + mm < lanes ? m0 + mm : lanes - 1;
                 raw[mm][c] = __ldcg(source + static_cast<size_t>(m) * per_lane + (chunk < per_lane ? chunk : 0));
             }
-        float sums[4];
+        float my_inverse = 1.0f;
+        if (weight != nullptr) {
+            float sums[LANES];
 #pragma unroll
-        for (int mm = 0; mm < 4; mm++) {
-            float sum = 0.0f;
+            for (int mm = 0; mm < LANES; mm++) {
+                float sum = 0.0f;
 #pragma unroll
-            for (int c = 0; c < CHUNKS; c++) {
-                if (CHUNKS > 1 && threadIdx.x + c * CONSUMER_THREADS >= per_lane) continue;
-                const uint32_t words[4] = {raw[mm][c].x, raw[mm][c].y, raw[mm][c].z, raw[mm][c].w};
-#pragma unroll
-                for (int w = 0; w < 4; w++) {
-                    const float lo = bf16_lo(words[w]), hi = bf16_hi(words[w]);
-                    sum = fmaf(lo, lo, sum);
-                    sum = fmaf(hi, hi, sum);
-                }
-            }
-            sums[mm] = (CHUNKS > 1 || static_cast<int>(threadIdx.x) < per_lane) ? sum : 0.0f;
-        }
-        // the four sums cross the warp together: after two exchanges a thread holds the sum of lane 2 * bit0 + bit1
-        {
-            const bool odd = lane & 1;
-            const float keep0 = odd ? sums[2] : sums[0], keep1 = odd ? sums[3] : sums[1];
-            const float send0 = odd ? sums[0] : sums[2], send1 = odd ? sums[1] : sums[3];
-            const float a0 = keep0 + __shfl_xor_sync(0xffffffffu, send0, 1), a1 = keep1 + __shfl_xor_sync(0xffffffffu, send1, 1);
-            const bool upper = lane & 2;
-            float sum = (upper ? a1 : a0) + __shfl_xor_sync(0xffffffffu, upper ? a0 : a1, 2);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 8);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-            if (lane < 4) partial[(2 * (lane & 1) + (lane >> 1)) * CONSUMER_WARPS + warp] = sum;
-        }
-        consumer_sync();
-        // every warp adds up the 16 partials of the four lanes: lanes 8k .. 8k+7 of the warp take lane m0 + k
-        float total = partial[(lane >> 3) * CONSUMER_WARPS + (lane & 7) * 2] + partial[(lane >> 3) * CONSUMER_WARPS + (lane & 7) * 2 + 1];
-        total += __shfl_xor_sync(0xffffffffu, total, 1);
-        total += __shfl_xor_sync(0xffffffffu, total, 2);
-        total += __shfl_xor_sync(0xffffffffu, total, 4);
-        // IEEE sqrt and divide, as a CPU evaluates 1/sqrt(v)
-        const float my_inverse = 1.0f / sqrtf(total * (1.0f / static_cast<float>(width)) + eps);
-#pragma unroll
-        for (int mm = 0; mm < 4; mm++) {
-            const float inv_rms = __shfl_sync(0xffffffffu, my_inverse, mm * 8);
-#pragma unroll
-            for (int c = 0; c < CHUNKS; c++) {
-                const int chunk = threadIdx.x + c * CONSUMER_THREADS;
-                if (chunk < per_lane && m0 + mm < staged) {
-                    const uint32_t in[4] = {raw[mm][c].x, raw[mm][c].y, raw[mm][c].z, raw[mm][c].w};
-                    const uint32_t sc[4] = {scale_words[c].x, scale_words[c].y, scale_words[c].z, scale_words[c].w};
-                    float v[8];
+                for (int c = 0; c < CHUNKS; c++) {
+                    if (CHUNKS > 1 && thread + c * CONSUMER_THREADS >= per_lane) continue;
+                    const uint32_t words[4] = {raw[mm][c].x, raw[mm][c].y, raw[mm][c].z, raw[mm][c].w};
 #pragma unroll
                     for (int w = 0; w < 4; w++) {
-                        v[2 * w] = bf16_lo(in[w]) * inv_rms * (bf16_lo(sc[w]) + offset);
-                        v[2 * w + 1] = bf16_hi(in[w]) * inv_rms * (bf16_hi(sc[w]) + offset);
+                        const float lo = bf16_lo(words[w]), hi = bf16_hi(words[w]);
+                        sum = fmaf(lo, lo, sum);
+                        sum = fmaf(hi, hi, sum);
                     }
-                    fragments[fragment_index(chunk, m0 + mm, staged)] =
-                        make_uint4(bf16_rounded_half_pair(v[0], v[4]), bf16_rounded_half_pair(v[1], v[5]), bf16_rounded_half_pair(v[2], v[6]),
-                                   bf16_rounded_half_pair(v[3], v[7]));
+                }
+                sums[mm] = (CHUNKS > 1 || thread < per_lane) ? sum : 0.0f;
+            }
+            float total;
+            if (LANES == 4) {
+                // the four sums cross the warp together: after two exchanges a thread holds the sum of lane 2 * bit0 + bit1
+                const bool odd = lane & 1;
+                const float keep0 = odd ? sums[LANES / 2] : sums[0], keep1 = odd ? sums[LANES - 1] : sums[LANES / 4];
+                const float send0 = odd ? sums[0] : sums[LANES / 2], send1 = odd ? sums[LANES / 4] : sums[LANES - 1];
+                const float a0 = keep0 + __shfl_xor_sync(0xffffffffu, send0, 1), a1 = keep1 + __shfl_xor_sync(0xffffffffu, send1, 1);
+                const bool upper = lane & 2;
+                float sum = (upper ? a1 : a0) + __shfl_xor_sync(0xffffffffu, upper ? a0 : a1, 2);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+                if (lane < 4) partial[(2 * (lane & 1) + (lane >> 1)) * CONSUMER_WARPS + warp] = sum;
+            } else {
+#pragma unroll
+                for (int mm = 0; mm < LANES; mm++) {
+#pragma unroll
+                    for (int step = 1; step < 32; step *= 2) sums[mm] += __shfl_xor_sync(0xffffffffu, sums[mm], step);
+                    if (lane == 0) partial[mm * CONSUMER_WARPS + warp] = sums[mm];
+                }
+            }
+            cta_sync();
+            // every warp adds up the 16 partials of the lanes: lanes 8k .. 8k+7 of the warp take lane m0 + k
+            const int k = (lane >> 3) < LANES ? lane >> 3 : 0;
+            total = partial[k * CONSUMER_WARPS + (lane & 7) * 2] + partial[k * CONSUMER_WARPS + (lane & 7) * 2 + 1];
+            total += __shfl_xor_sync(0xffffffffu, total, 1);
+            total += __shfl_xor_sync(0xffffffffu, total, 2);
+            total += __shfl_xor_sync(0xffffffffu, total, 4);
+            // IEEE sqrt and divide, as a CPU evaluates 1/sqrt(v)
+            my_inverse = 1.0f / sqrtf(total * (1.0f / static_cast<float>(width)) + eps);
+        }
+#pragma unroll
+        for (int c = 0; c < CHUNKS; c++) {
+            const int chunk = thread + c * CONSUMER_THREADS, group = (chunk >> 4) - first_group;
+            unsigned long long norm[4];
+            if (weight != nullptr) {
+                const uint32_t sc[4] = {scale_words[c].x, scale_words[c].y, scale_words[c].z, scale_words[c].w};
+#pragma unroll
+                for (int w = 0; w < 4; w++) norm[w] = pair_of(bf16_lo(sc[w]) + offset, bf16_hi(sc[w]) + offset);
+            }
+            uint32_t largest[LANES];
+#pragma unroll
+            for (int mm = 0; mm < LANES; mm++) {
+                uint32_t words[4] = {raw[mm][c].x, raw[mm][c].y, raw[mm][c].z, raw[mm][c].w};
+                if (weight != nullptr) {
+                    const float inv_rms = __shfl_sync(0xffffffffu, my_inverse, mm * 8);
+                    const unsigned long long inverse = pair_of(inv_rms, inv_rms);
+#pragma unroll
+                    for (int w = 0; w < 4; w++) {
+                        // rounded to nearest even, as the shaders' f32_to_bf16 for every finite value
+                        const unsigned long long v = pair_multiply(pair_multiply(pair_of(bf16_lo(words[w]), bf16_hi(words[w])), inverse), norm[w]);
+                        asm("{\n.reg .f32 lo, hi;\nmov.b64 {lo, hi}, %1;\ncvt.rn.bf16x2.f32 %0, hi, lo;\n}" : "=r"(words[w]) : "l"(v));
+                    }
+                    raw[mm][c] = make_uint4(words[0], words[1], words[2], words[3]);
+                }
+                if (CHUNKS > 1 && chunk >= per_lane) words[0] = words[1] = words[2] = words[3] = 0;
+                const uint32_t most =
+                    larger_halves(larger_halves(words[0] & 0x7fff7fffu, words[1] & 0x7fff7fffu), larger_halves(words[2] & 0x7fff7fffu, words[3] & 0x7fff7fffu));
+                largest[mm] = larger_halves(most, most >> 16) & 0x7f80u;
+            }
+#pragma unroll
+            for (int mm = 0; mm < LANES; mm++) largest[mm] = __reduce_max_sync(0xffffffffu, largest[mm]) >> 7;
+            if (chunk < per_lane && group >= 0 && group < groups) {
+                const int word = chunk & 15;
+                uint8_t *block = operands + static_cast<uint32_t>(group) * operand_group_bytes(lanes), *place = block + operand_word_offset(word, m0, lanes);
+#pragma unroll
+                for (int mm = 0; mm < LANES; mm++) {
+                    if (m0 + mm >= lanes) break;
+                    const float scale = operand_scale(largest[mm]);
+                    const unsigned long long scales = pair_of(scale, scale);
+                    const uint32_t words[4] = {raw[mm][c].x, raw[mm][c].y, raw[mm][c].z, raw[mm][c].w};
+                    uint32_t whole[4][2], even[3], odd[3];
+#pragma unroll
+                    for (int w = 0; w < 4; w++) {
+                        const unsigned long long v = pair_fma(pair_of(bf16_lo(words[w]), bf16_hi(words[w])), scales, constants.bias);
+                        whole[w][0] = static_cast<uint32_t>(v);
+                        whole[w][1] = static_cast<uint32_t>(v >> 32);
+                    }
+                    operand_digits(whole[0][0], whole[1][0], whole[2][0], whole[3][0], constants, even);
+                    operand_digits(whole[0][1], whole[1][1], whole[2][1], whole[3][1], constants, odd);
+#pragma unroll
+                    for (int t = 0; t < 3; t++) *reinterpret_cast<uint2 *>(place + 192 * mm + 64 * t) = make_uint2(even[t], odd[t]);
+                    if (word == 0) *reinterpret_cast<float *>(block + 2 * operand_half_bytes(lanes) + 4 * (m0 + mm)) = operand_factor(largest[mm]);
                 }
             }
         }
-        if (m0 + 4 < staged) consumer_sync();  // `partial` is rewritten for the next four lanes
+        if (m0 + LANES < lanes) cta_sync();  // `partial` is rewritten for the next four lanes
     }
-    consumer_sync();
+    cta_sync();
+}
+
+template <int TILES>
+__device__ __forceinline__ void stage_any(const uint16_t *x, const uint16_t *weight, int width, int first_group, int groups) {
+    const bool narrow = width <= 8 * CONSUMER_THREADS;
+    if (TILES == 1 && shared().a.lanes == 1) return narrow ? stage_rows<1, 1>(x, weight, width, first_group, groups) : stage_rows<2, 1>(x, weight, width, first_group, groups);
+    constexpr int LANES = TILES == 1 ? 2 : 4;
+    return narrow ? stage_rows<1, LANES>(x, weight, width, first_group, groups) : stage_rows<2, 2>(x, weight, width, first_group, groups);
+}
+
+// A group's 128 columns of one lane (f32 in shared memory) into operand form in global memory, by one warp.
+__device__ __forceinline__ void store_operand_group(uint8_t *block, const float *columns, int m, int lanes) {
+    const int lane = thread_now() & 31, word = lane >> 1, odd = lane & 1;
+    float v[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] = columns[word * 8 + odd + 2 * i];
+    const uint32_t largest = __reduce_max_sync(0xffffffffu, max(max(__float_as_uint(v[0]) & 0x7fffffffu, __float_as_uint(v[1]) & 0x7fffffffu),
+                                                                max(__float_as_uint(v[2]) & 0x7fffffffu, __float_as_uint(v[3]) & 0x7fffffffu)));
+    const uint32_t exponent = largest >> 23;
+    uint32_t terms[3], whole[4];
+    const float scale = operand_scale(exponent);
+#pragma unroll
+    for (int i = 0; i < 4; i++) whole[i] = __float_as_uint(fmaf(v[i], scale, WHOLE_BIAS));
+    operand_digits(whole[0], whole[1], whole[2], whole[3], digit_constants(), terms);
+    uint8_t *place = block + operand_word_offset(word, m, lanes) + 4 * odd;
+#pragma unroll
+    for (int t = 0; t < 3; t++) *reinterpret_cast<uint32_t *>(place + 64 * t) = terms[t];
+    if (lane == 0) *reinterpret_cast<float *>(block + 2 * operand_half_bytes(lanes) + 4 * m) = operand_factor(exponent);
 }
 
 // ------------------------------------------------------------------------------------------ attention
 // A team of four warps serves one context split (64 tokens) of one kv head for the Q = QL * GROUP <= 16 query
 // vectors of QL consecutive lanes of a stream (append_gqa_attention_bf16.comp.template:217-339: f32 scores of
-// bf16 q.k, f32 softmax, f32 p.v); warp w of the team takes tokens 16w .. 16w + 15 of the split.  Scores and p.v
-// run on the tensor cores: q rows are the A operand of S = Q K^T, K rows the B operand (both read with 16-byte
-// loads; the head dimension is permuted identically on both sides); the probabilities are re-used from the
-// accumulator registers as the A operand of O = P V, split into a bf16 high and low part (p = hi + lo to 2^-17),
-// and V is the B operand, its token pairs assembled with byte permutes.  The warps agree on the split's row
-// maxima through shared memory, add up their partial outputs there (HALF head dims per pass), and the team writes
-// one partial (unnormalised output, maximum, sum) per query to the scratch.  The team that completes a kv head's
-// last split merges all of them (log-sum-exp) and writes the head's outputs, fp16 in fragment order, where the o
-// projection's activation slices are copied from.
+// bf16 q.k, f32 softmax, f32 p.v).  Warp w of the team scores tokens 16w .. 16w + 15: q rows are the A operand of
+// S = Q K^T, K rows the B operand (both read with 16-byte loads; the head dimension is permuted identically on both
+// sides).  The warps agree on the split's row maxima, hand their probabilities on as A fragments - split into a bf16
+// high and low part, p = hi + lo to 2^-17 - and warp w then sums dims [w HD / 4, (w + 1) HD / 4) of O = P V over all 64
+// tokens, V as the B operand, its token pairs assembled with byte permutes; the products of 16 tokens add up in the
+// tensor core, the four parts in f32.  (Each warp summing all dims over its own tokens needed the parts added through
+// 17 KB of shared memory per team, in two rounds.)  The team writes one partial (unnormalised output, maximum, sum) per
+// query to the scratch.  The team that completes a kv head's last split queues the merge of all of them.
 
+constexpr int Q_PITCH_PAD = 64;  // bytes: 16-byte reads of a quarter warp fall into distinct banks
 template <int HD>
 __host__ __device__ constexpr size_t attention_team_bytes() {
-    return (4 * 16 * ((HD < 64 ? HD : 64) + 4) + 2 * 4 * 16 + 4) * sizeof(float);  // partial outputs [warp][row][HALF + 4], maxima and sums [warp][row], one flag
+    // query rows, later the probabilities' fragments (high and low), then maxima and sums [warp][row] and the rows of 64 tokens
+    constexpr size_t rows = 16 * (HD * 2 + Q_PITCH_PAD), fragments = 2 * 4 * 32 * 16;
+    return (rows > fragments ? rows : fragments) + (2 * 4 * 16 + 64) * 4;
 }
 
-struct AttentionJob {  // what every attention item of a launch shares
-    const uint16_t *q;
-    float *scratch;
-    uint16_t *out_fragments;
-    unsigned int *arrivals;
-    int lanes, lanes_per_stream, q_heads, kv_heads, max_splits, group_slots, staged;
-    float scale;
-};
 // The scratch of a layer's attention step: every (lane, q head, split) partial is HD floats of unnormalised output in
 // `values` [lane][q head][split][HD] (16-byte aligned rows) and (maximum, sum) in `stats` [lane][q head][split][2]
 // behind all the values - together the (HD + 2) floats per partial the scratch is sized for.
@@ -624,7 +744,7 @@ __device__ __forceinline__ void attention_merge_block(const float *__restrict__ 
     static_assert(VEC == 1 || VEC == 2 || VEC == 4, "a lane owns one, two or four output dims");
     constexpr int CHUNK = VEC == 4 ? 8 : 16;  // rows in flight at a time; a divisor of the block, whose weights sit in the warp's lanes
     static_assert(MERGE_BLOCK % CHUNK == 0, "rounds of the merge must not straddle a block");
-    const int lane_id = threadIdx.x & 31;
+    const int lane_id = thread_now() & 31;
     const int last = count - 1;
     // Rows beyond the last partial are read as the last one again and weigh nothing, so no load is predicated.
     float part[CHUNK][VEC];
@@ -665,95 +785,114 @@ __device__ __forceinline__ void attention_merge_block(const float *__restrict__ 
 
 // How many 64-token splits the partials of a query lane's rows cover: those of the newest lane of its group of QL
 // lanes (a team writes every row of its group for every split of the group; rows of older lanes are masked there).
-__device__ __forceinline__ int attention_group_splits(const AttentionJob &job, const uint32_t *ticks, uint32_t capacity, int query_lane, int ql) {
-    const int stream = query_lane / job.lanes_per_stream, first = ((query_lane % job.lanes_per_stream) / ql) * ql;
+__device__ __forceinline__ int attention_own_splits(uint32_t capacity, uint32_t tick);
+__device__ __forceinline__ int attention_group_splits(uint32_t capacity, int query_lane, int ql) {
+    const StackShared &sh = shared();
+    const int per_stream = sh.a.lanes_per_stream, stream = query_lane / per_stream, first = ((query_lane % per_stream) / ql) * ql;
     uint32_t tick = 0;
-    for (int i = first; i < first + ql && i < job.lanes_per_stream; i++) {
-        const uint32_t other = ticks[stream * job.lanes_per_stream + i];
+    for (int i = first; i < first + ql && i < per_stream; i++) {
+        const uint32_t other = sh.tick[stream * per_stream + i];
         if (other > tick) tick = other;
     }
-    const uint32_t tokens = tick + 1u < capacity ? tick + 1u : capacity;
-    const int splits = static_cast<int>((tokens + 63u) / 64u);
-    return splits < job.max_splits ? splits : job.max_splits;
+    return attention_own_splits(capacity, tick);
 }
 
 // The splits of one lane's own attended window.
-__device__ __forceinline__ int attention_own_splits(const AttentionJob &job, uint32_t capacity, uint32_t tick) {
+__device__ __forceinline__ int attention_own_splits(uint32_t capacity, uint32_t tick) {
     const uint32_t tokens = tick + 1u < capacity ? tick + 1u : capacity;
-    const int splits = static_cast<int>((tokens + 63u) / 64u);
-    return splits < job.max_splits ? splits : job.max_splits;
+    const int splits = static_cast<int>((tokens + 63u) / 64u), most = shared().a.max_splits;
+    return splits < most ? splits : most;
 }
 
 // The scratch behind the split partials: per row and range of MERGE_BLOCK splits one merged partial, laid out like
 // the split partials (values, then statistics).  Used by rows of more than MERGE_BLOCK splits.
-__device__ __forceinline__ float *attention_range_values(const AttentionJob &job, int head_width) {
-    return job.scratch + static_cast<size_t>(job.lanes) * job.q_heads * job.max_splits * (head_width + 2);
+__device__ __forceinline__ float *attention_range_values(const StackArgs &a, int head_width) {
+    return a.buffers.attention_scratch + static_cast<size_t>(a.lanes) * a.shape.q_heads * a.max_splits * (head_width + 2);
 }
 __device__ __forceinline__ int attention_ranges(int max_splits) { return (max_splits + MERGE_BLOCK - 1) / MERGE_BLOCK; }
 
-// A row of at most MERGE_BLOCK splits: merged and written out as fp16 in fragment order by one warp.
+// The merged output of a row, rounded to bf16 (the warp's lanes own consecutive dims).
 template <int HD>
-__device__ __noinline__ void attention_merge_row(const AttentionJob &job, int splits, int query_lane, int head) {
+__device__ __forceinline__ void attention_write_row(int query_lane, int head, float denominator, const float (&acc)[HD / 32]) {
     constexpr int VEC = HD / 32;
-    const int lane_id = threadIdx.x & 31;
-    const size_t row = (static_cast<size_t>(query_lane) * job.q_heads + head) * job.max_splits;
-    float maximum, denominator, acc[VEC];
-    attention_merge_block<HD>(job.scratch + row * HD + lane_id * VEC,
-                              reinterpret_cast<const float2 *>(attention_stats(job.scratch, job.lanes, job.q_heads, job.max_splits, HD)) + row, splits, maximum,
-                              denominator, acc);
+    const StackArgs &a = shared().a;
+    uint16_t *out = a.buffers.attention_out + (static_cast<size_t>(query_lane) * a.shape.q_heads + head) * HD + (thread_now() & 31) * VEC;
+    uint32_t bits[VEC];
 #pragma unroll
-    for (int v = 0; v < VEC; v++) {
-        const float rounded = round_bf16(denominator == 0.0f ? 0.0f : acc[v] / denominator);
-        job.out_fragments[fragment_element(head * HD + lane_id * VEC + v, query_lane, job.staged)] = __half_as_ushort(__float2half_rn(rounded));
-    }
+    for (int v = 0; v < VEC; v++) bits[v] = f32_to_bf16_bits(denominator == 0.0f ? 0.0f : acc[v] / denominator);
+    if (VEC == 4) *reinterpret_cast<uint2 *>(out) = make_uint2(bits[0] | (bits[VEC > 1 ? 1 : 0] << 16), bits[VEC > 2 ? 2 : 0] | (bits[VEC > 3 ? 3 : 0] << 16));
+    else if (VEC == 2) *reinterpret_cast<uint32_t *>(out) = bits[0] | (bits[VEC > 1 ? 1 : 0] << 16);
+    else *out = static_cast<uint16_t>(bits[0]);
+}
+
+// A row of at most MERGE_BLOCK splits: merged and written out by one warp.
+template <int HD>
+__device__ __forceinline__ void attention_merge_row(int splits, int query_lane, int head) {
+    constexpr int VEC = HD / 32;
+    const StackArgs &a = shared().a;
+    const int lane_id = thread_now() & 31;
+    const size_t row = (static_cast<size_t>(query_lane) * a.shape.q_heads + head) * a.max_splits;
+    float maximum, denominator, acc[VEC];
+    attention_merge_block<HD>(a.buffers.attention_scratch + row * HD + lane_id * VEC,
+                              reinterpret_cast<const float2 *>(attention_stats(a.buffers.attention_scratch, a.lanes, a.shape.q_heads, a.max_splits, HD)) + row, splits, maximum,
+                              denominator, acc);
+    attention_write_row<HD>(query_lane, head, denominator, acc);
 }
 
 // Longer rows, first level: one range of MERGE_BLOCK splits of a row into one partial.
 template <int HD>
-__device__ __noinline__ void attention_merge_range(const AttentionJob &job, int splits, int query_lane, int head, int range) {
+__device__ __forceinline__ void attention_merge_range(int splits, int query_lane, int head, int range) {
     constexpr int VEC = HD / 32;
-    const int lane_id = threadIdx.x & 31;
-    const size_t row = static_cast<size_t>(query_lane) * job.q_heads + head;
-    const size_t first = row * job.max_splits + static_cast<size_t>(range) * MERGE_BLOCK;
+    const StackArgs &a = shared().a;
+    const int lane_id = thread_now() & 31;
+    const size_t row = static_cast<size_t>(query_lane) * a.shape.q_heads + head;
+    const size_t first = row * a.max_splits + static_cast<size_t>(range) * MERGE_BLOCK;
     const int count = splits - range * MERGE_BLOCK < MERGE_BLOCK ? splits - range * MERGE_BLOCK : MERGE_BLOCK;
     float maximum, denominator, acc[VEC];
-    attention_merge_block<HD>(job.scratch + first * HD + lane_id * VEC,
-                              reinterpret_cast<const float2 *>(attention_stats(job.scratch, job.lanes, job.q_heads, job.max_splits, HD)) + first, count, maximum,
+    attention_merge_block<HD>(a.buffers.attention_scratch + first * HD + lane_id * VEC,
+                              reinterpret_cast<const float2 *>(attention_stats(a.buffers.attention_scratch, a.lanes, a.shape.q_heads, a.max_splits, HD)) + first, count, maximum,
                               denominator, acc);
-    const int ranges = attention_ranges(job.max_splits);
-    float *values = attention_range_values(job, HD);
+    const int ranges = attention_ranges(a.max_splits);
+    float *values = attention_range_values(a, HD);
     float *out = values + (row * ranges + range) * HD + lane_id * VEC;
 #pragma unroll
     for (int v = 0; v < VEC; v++) out[v] = acc[v];
     if (lane_id == 0) {
-        float2 *statistics = reinterpret_cast<float2 *>(values + static_cast<size_t>(job.lanes) * job.q_heads * ranges * HD) + row * ranges + range;
+        float2 *statistics = reinterpret_cast<float2 *>(values + static_cast<size_t>(a.lanes) * a.shape.q_heads * ranges * HD) + row * ranges + range;
         *statistics = make_float2(maximum, denominator);
     }
 }
 
 // Second level: the row's range partials merged and written out.
 template <int HD>
-__device__ __noinline__ void attention_merge_ranges(const AttentionJob &job, int splits, int query_lane, int head) {
+__device__ __forceinline__ void attention_merge_ranges(int splits, int query_lane, int head) {
     constexpr int VEC = HD / 32;
-    const int lane_id = threadIdx.x & 31;
-    const size_t row = static_cast<size_t>(query_lane) * job.q_heads + head;
-    const int ranges = attention_ranges(job.max_splits), count = (splits + MERGE_BLOCK - 1) / MERGE_BLOCK;
-    const float *values = attention_range_values(job, HD);
+    const StackArgs &a = shared().a;
+    const int lane_id = thread_now() & 31;
+    const size_t row = static_cast<size_t>(query_lane) * a.shape.q_heads + head;
+    const int ranges = attention_ranges(a.max_splits), count = (splits + MERGE_BLOCK - 1) / MERGE_BLOCK;
+    const float *values = attention_range_values(a, HD);
     float maximum, denominator, acc[VEC];
     attention_merge_block<HD>(values + row * ranges * HD + lane_id * VEC,
-                              reinterpret_cast<const float2 *>(values + static_cast<size_t>(job.lanes) * job.q_heads * ranges * HD) + row * ranges, count, maximum,
+                              reinterpret_cast<const float2 *>(values + static_cast<size_t>(a.lanes) * a.shape.q_heads * ranges * HD) + row * ranges, count, maximum,
                               denominator, acc);
-#pragma unroll
-    for (int v = 0; v < VEC; v++) {
-        const float rounded = round_bf16(denominator == 0.0f ? 0.0f : acc[v] / denominator);
-        job.out_fragments[fragment_element(head * HD + lane_id * VEC + v, query_lane, job.staged)] = __half_as_ushort(__float2half_rn(rounded));
-    }
+    attention_write_row<HD>(query_lane, head, denominator, acc);
 }
 
 // Loads through L2 that stay where they are written (the compiler may not sink them towards their use).
 __device__ __forceinline__ uint4 load16_now(const void *address) {
     uint4 v;
     asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(address) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t load4_now(const void *address) {
+    uint32_t v;
+    asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(address) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t load2_now(const void *address) {
+    uint16_t v;
+    asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(v) : "l"(address) : "memory");
     return v;
 }
 __device__ __forceinline__ uint2 load8_now(const void *address) {
@@ -763,7 +902,7 @@ __device__ __forceinline__ uint2 load8_now(const void *address) {
 }
 
 template <int HD>
-__device__ __noinline__ size_t attention_row_base(const KvLayer &kv, int slot, uint32_t ring_base, int token) {
+__device__ __forceinline__ size_t attention_row_base(const KvLayer &kv, int slot, uint32_t ring_base, int token) {
     uint32_t ring = ring_base + static_cast<uint32_t>(token);
     if (ring >= kv.capacity) ring -= kv.capacity;
     const int page = static_cast<int>(ring / kv.page_tokens), within = static_cast<int>(ring % kv.page_tokens);
@@ -771,189 +910,141 @@ __device__ __noinline__ size_t attention_row_base(const KvLayer &kv, int slot, u
     return static_cast<size_t>(physical) * 2 * kv.kv_heads * kv.page_tokens * HD + static_cast<size_t>(within) * HD;
 }
 
-constexpr int ATTENTION_MERGE_LIST = 63;
-// Per-CTA copies of what every layer needs again: the lanes' ticks and stream slots, and for each team the KV rows
-// of its first work item (the block table is shared by all layers, so the rows of a (split, lane group) are the
-// same in every layer's pool).
-struct AttentionCache {
-    AttentionJob job;
-    uint32_t tick[8];
-    int32_t slot[8];
-    int32_t item[4];          // the work item whose rows `row_base` holds, or -1
-    int32_t rows[4];          // how many tokens that item has
-    int32_t merge_count;      // (kv head, lane group) pairs whose last split this CTA's teams completed in this layer ...
-    int32_t merge_list[ATTENTION_MERGE_LIST];  // ... and which: kv_head * group_slots + group_slot
-    uint32_t row_base[4][64]; // offset (in rows of HD elements) of token t's K row of kv head 0 in a layer's pool
-    StackLayer layer[2];      // the current layer's description (layer & 1) and the next one's, copied ahead of their use
-};
+// What work item `item` of the launch's attention steps is.
+template <int QL>
+__device__ __forceinline__ AttentionItem attention_item(const KvLayer &kv, int item) {
+    const StackShared &sh = shared();
+    const int per_stream = sh.a.lanes_per_stream, groups_per_stream = (per_stream + QL - 1) / QL, max_splits = sh.a.max_splits;
+    AttentionItem it;
+    const int rest = item / kv.kv_heads, group_slot = rest / max_splits, stream = group_slot / groups_per_stream, first = (group_slot - stream * groups_per_stream) * QL;
+    it.kv_head = static_cast<int16_t>(item - rest * kv.kv_heads);
+    it.split = static_cast<int16_t>(rest - group_slot * max_splits);
+    it.lane0 = static_cast<int16_t>(stream * per_stream + first);
+    const int left = per_stream - first;
+    it.lanes = static_cast<int16_t>(left < QL ? left : QL);
+    it.slot = sh.slot[it.lane0];
+    it.arrival = it.kv_head * sh.group_slots + group_slot;
+    it.count = 0;
+    if (it.slot < 0) return it;
+    uint32_t newest = 0;
+    for (int i = 0; i < it.lanes; i++) newest = sh.tick[it.lane0 + i] > newest ? sh.tick[it.lane0 + i] : newest;
+    const uint32_t tokens = newest + 1u < kv.capacity ? newest + 1u : kv.capacity;  // attended window of the newest lane
+    const uint32_t begin = static_cast<uint32_t>(it.split) * 64u;
+    if (begin >= tokens) return it;
+    it.first_tick = newest + 1u - tokens + begin;
+    it.ring_base = it.first_tick % kv.capacity;
+    it.count = static_cast<int32_t>(tokens - begin < 64u ? tokens - begin : 64u);
+    const int splits = static_cast<int>((tokens + 63u) / 64u);
+    it.splits = splits < max_splits ? splits : max_splits;
+    return it;
+}
 
 template <int HD, int GROUP, int QL>
-__device__ __noinline__ void attention_team_item(AttentionCache &cache, const KvLayer &kv_shared, int item, uint8_t *scratch_area,
-                                                    unsigned long long *stamps) {
+__device__ __forceinline__ void attention_team_item(int layer, const AttentionItem &it, bool rows_cached) {
     constexpr int Q = QL * GROUP;
-    // the launch's and the layer's descriptions by value: behind a reference every field would be read again after
-    // each of the ordered loads below
-    const KvLayer kv = kv_shared;
-    const AttentionJob job = cache.job;
-    const uint16_t *__restrict__ q = job.q;
-    float *__restrict__ scratch = job.scratch;
-    const int lanes = job.lanes, lanes_per_stream = job.lanes_per_stream, q_heads = job.q_heads, max_splits = job.max_splits;
-    const int group_slots = job.group_slots;
-    const float scale = job.scale;
-    const int team = static_cast<int>(threadIdx.x >> 7), team_warp = static_cast<int>(threadIdx.x >> 5) & 3, barrier_id = 2 + team;
-    float *team_smem = reinterpret_cast<float *>(scratch_area + static_cast<size_t>(team) * attention_team_bytes<HD>());
-    const int kv_head = item % job.kv_heads, split = (item / job.kv_heads) % max_splits, group_slot = (item / job.kv_heads) / max_splits;
-    unsigned int *__restrict__ arrivals = job.arrivals;
-    auto mark = [&](int index) {
-        if (stamps != nullptr) {
-            unsigned long long now;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-            stamps[index] = now;
+    constexpr int QW = HD / 32;         // 16-byte pieces of a q / k row per thread
+    constexpr int DIMS = HD / 4;        // head dims of the output per warp
+    constexpr int DPT = DIMS / 8;       // of which one thread column owns this many: 4, 2 or 1
+    static_assert(Q <= 16 && HD % 32 == 0 && DPT <= 4, "attention team shape");
+    StackShared &sh = shared();
+    const int thread = thread_now(), team = thread >> 7, team_thread = thread & 127, team_warp = team_thread >> 5, lane = thread & 31, g = lane >> 2, j = lane & 3;
+    const int barrier_id = 2 + team;
+    uint8_t *team_smem = smem_raw + sh.scratch + static_cast<uint32_t>(team) * static_cast<uint32_t>(attention_team_bytes<HD>());
+    float *team_max = reinterpret_cast<float *>(team_smem + attention_team_bytes<HD>() - (2 * 4 * 16 + 64) * 4);  // [4][16]
+    float *team_sum = team_max + 4 * 16;                                                                          // [4][16]
+    uint32_t *team_rows = reinterpret_cast<uint32_t *>(team_sum + 4 * 16);                                        // [64]
+    const KvLayer &kv = sh.layer[layer & 1].kv;
+    const int count = it.count, lane0 = it.lane0, kv_head = it.kv_head, q_heads = sh.a.shape.q_heads;
+    stamp(layer, 20);
+    // row numbers (units of HD elements, kv head 0) of the split's K rows: cached for the team's first item, else looked
+    // up through the block table, a token per thread
+    const uint32_t *rows = sh.row_base[team];
+    if (!rows_cached) {
+        if (team_thread < 64) team_rows[team_thread] = team_thread < count ? static_cast<uint32_t>(attention_row_base<HD>(kv, it.slot, it.ring_base, team_thread) / HD) : 0u;
+        team_barrier(barrier_id);
+        rows = team_rows;
+    }
+    // ---- the query rows, as asynchronous copies (they would hold 32 registers per thread)
+    constexpr uint32_t Q_PITCH = HD * 2 + Q_PITCH_PAD;
+    const uint32_t q_shared = shared_address(team_smem);
+#pragma unroll
+    for (int piece = team_thread; piece < 16 * QW * 4; piece += 128) {
+        const int row = piece / (QW * 4), part = piece % (QW * 4);
+        const uint32_t destination = q_shared + static_cast<uint32_t>(row) * Q_PITCH + static_cast<uint32_t>(part) * 16u;
+        if (row / GROUP < it.lanes && row < Q) {
+            const uint16_t *source = sh.a.buffers.q + (static_cast<size_t>(lane0 + row / GROUP) * q_heads + kv_head * GROUP + row % GROUP) * HD + part * 8;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(destination), "l"(source) : "memory");
+        } else {
+            asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(destination), "r"(0u) : "memory");
         }
-    };
-    constexpr int QW = HD / 32;                    // 16-byte pieces of a q / k row per thread
-    constexpr int HALF = HD < 64 ? HD : 64;        // head dims handled per output pass
-    constexpr int DPT = HALF / 8;                  // of which one thread column owns this many
-    static_assert(Q <= 16 && HD % 32 == 0, "attention team shape");
-    const int lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
-    constexpr int PITCH = HALF + 4;                       // row pitch of the partial outputs (bank spread)
-    float *partial_out = team_smem;                       // [4][16][PITCH]
-    float *team_max = team_smem + 4 * 16 * PITCH;         // [4][16]
-    float *team_sum = team_max + 4 * 16;                  // [4][16]
-    unsigned int *team_flag = reinterpret_cast<unsigned int *>(team_sum + 4 * 16);
-    const int groups_per_stream = (lanes_per_stream + QL - 1) / QL;
-    const int stream_index = group_slot / groups_per_stream, group_index = group_slot % groups_per_stream;
-    const int lane0 = stream_index * lanes_per_stream + group_index * QL;
-    if (lane0 >= lanes) return;
-    const int slot = cache.slot[lane0];
-    if (slot < 0) return;
-    const uint32_t capacity = kv.capacity;
-
-    uint32_t newest = 0, tick_row[2] = {0xffffffffu, 0xffffffffu};
-#pragma unroll
-    for (int i = 0; i < QL; i++) {
-        const bool valid = lane0 + i < lanes && group_index * QL + i < lanes_per_stream;
-        const uint32_t tick = valid ? cache.tick[lane0 + i] : 0xffffffffu;
-        if (valid && tick > newest) newest = tick;
-        if (g < Q && g / GROUP == i) tick_row[0] = tick;
-        if (g + 8 < Q && (g + 8) / GROUP == i) tick_row[1] = tick;
     }
-    const uint32_t tokens = newest + 1u < capacity ? newest + 1u : capacity;  // attended window of the newest lane
-    const uint32_t first_tick = newest + 1u - tokens;
-    const uint32_t begin = static_cast<uint32_t>(split) * 64u;
-    if (begin >= tokens) return;  // the whole team leaves: nobody waits at the team barrier
-    mark(20);
-    int expected_splits = static_cast<int>((tokens + 63u) / 64u);
-    if (expected_splits > max_splits) expected_splits = max_splits;
-    const int count = static_cast<int>(tokens - begin < 64u ? tokens - begin : 64u);
-    const int token0 = 16 * team_warp;  // this warp's tokens of the split
-    // element offset of token t's K (or V) row of this kv head: from the team's cached rows, or through the block table
-    const size_t half_page = static_cast<size_t>(kv.kv_heads) * kv.page_tokens * HD;
-    const bool cached = cache.item[team] == item;
-    const uint32_t ring_base = (first_tick + begin) % capacity;
-    // Row numbers (units of HD elements, kv head 0) of the K rows this thread reads (tokens g and g + 8 of the warp's
-    // sixteen) and of its V rows (tokens 2j, 2j + 1, 2j + 8, 2j + 9).  Without cached rows every thread walks the
-    // block table for one token and the warp passes the rows round: one dependent load instead of six in a row.
-    uint32_t k_row[2], v_row[4];
-    if (cached) {
-#pragma unroll
-        for (int nt = 0; nt < 2; nt++) k_row[nt] = cache.row_base[team][(token0 + nt * 8 + g) & 63];
-#pragma unroll
-        for (int t = 0; t < 4; t++) v_row[t] = cache.row_base[team][(token0 + 2 * j + (t & 1) + 8 * (t >> 1)) & 63];
-    } else {
-        const int token = token0 + (lane & 15);
-        const uint32_t mine = token < count ? static_cast<uint32_t>(attention_row_base<HD>(kv, slot, ring_base, token) / HD) : 0u;
-#pragma unroll
-        for (int nt = 0; nt < 2; nt++) k_row[nt] = __shfl_sync(0xffffffffu, mine, nt * 8 + g);
-#pragma unroll
-        for (int t = 0; t < 4; t++) v_row[t] = __shfl_sync(0xffffffffu, mine, 2 * j + (t & 1) + 8 * (t >> 1));
-    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    // ---- K rows of tokens g and g + 8 of the warp's sixteen, requested before the arithmetic
     const size_t head_offset = static_cast<size_t>(kv_head) * kv.page_tokens * HD;
-
-    // ---- S = Q K^T for 16 tokens.  The team's Q query rows go to shared memory with asynchronous copies (they
-    // would otherwise hold 32 registers per thread while the K and V rows are in flight); a row is kept as HD / 32
-    // pieces of 64 bytes, thread column j reading 16 bytes of each - K rows are read from memory the same way, so
-    // the head dimension is permuted identically on both sides of the product.
-    constexpr uint32_t Q_PITCH = HD * 2 + 64;  // bytes; 16-byte reads of a quarter warp fall into distinct banks
-    const uint32_t q_shared = static_cast<uint32_t>(__cvta_generic_to_shared(partial_out));  // free until the first output pass
-    {
-        const int team_thread = team_warp * 32 + lane;
-        for (int piece = team_thread; piece < 16 * QW * 4; piece += 128) {
-            const int row = piece / (QW * 4), part = piece % (QW * 4);
-            const int query_lane = lane0 + row / GROUP;
-            const bool valid = row < Q && query_lane < lanes && group_index * QL + row / GROUP < lanes_per_stream;
-            const uint32_t destination = q_shared + static_cast<uint32_t>(row) * Q_PITCH + static_cast<uint32_t>(part) * 16u;
-            if (valid) {
-                const uint16_t *source = q + (static_cast<size_t>(query_lane) * q_heads + kv_head * GROUP + row % GROUP) * HD + part * 8;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(destination), "l"(source) : "memory");
-            } else {
-                asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(destination), "r"(0u) : "memory");
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    // K rows of tokens g and g + 8, V rows of tokens 2j, 2j+1, 2j+8, 2j+9 of this warp: all requested before the
-    // arithmetic (the V rows of the first output pass now, those of the second when the q registers are free)
+    const uint16_t *keys = kv.pool + head_offset + j * 8, *values = kv.pool + head_offset + static_cast<size_t>(kv.kv_heads) * kv.page_tokens * HD + team_warp * DIMS + g * DPT;
+    const int token0 = 16 * team_warp;
     uint4 kf[2][QW];
 #pragma unroll
     for (int nt = 0; nt < 2; nt++) {
         const int token = token0 + nt * 8 + g;
-        if (token < count) {
-            const uint16_t *krow = kv.pool + static_cast<size_t>(k_row[nt]) * HD + head_offset + j * 8;
+        const uint16_t *krow = keys + static_cast<size_t>(rows[token]) * HD;
 #pragma unroll
-            for (int w = 0; w < QW; w++) kf[nt][w] = load16_now(krow + w * 32);
-        } else {
-#pragma unroll
-            for (int w = 0; w < QW; w++) kf[nt][w] = make_uint4(0, 0, 0, 0);
-        }
+        for (int w = 0; w < QW; w++) kf[nt][w] = token < count ? load16_now(krow + w * 32) : make_uint4(0, 0, 0, 0);
     }
-    size_t v_offset[4];
+    uint32_t tick_row[2];
 #pragma unroll
-    for (int t = 0; t < 4; t++) {
-        const int token = token0 + 2 * j + (t & 1) + 8 * (t >> 1);
-        v_offset[t] = token < count ? static_cast<size_t>(v_row[t]) * HD + half_page + head_offset : static_cast<size_t>(-1);
+    for (int r = 0; r < 2; r++) {
+        const int query = (g + 8 * r) / GROUP;
+        tick_row[r] = g + 8 * r < Q && query < it.lanes ? sh.tick[lane0 + query] : 0xffffffffu;
     }
-    uint32_t v[HD / HALF][4][DPT / 2];
-    auto load_values = [&](int pass) {
-#pragma unroll
-        for (int t = 0; t < 4; t++) {
-            if (v_offset[t] != static_cast<size_t>(-1)) {
-                const uint16_t *vrow = kv.pool + v_offset[t] + pass * HALF + DPT * g;
-                if (DPT == 8) {
-                    const uint4 raw = load16_now(vrow);
-                    v[pass][t][0] = raw.x;
-                    v[pass][t][1] = raw.y;
-                    v[pass][t][DPT / 2 - 2] = raw.z;
-                    v[pass][t][DPT / 2 - 1] = raw.w;
-                } else {
-                    const uint2 raw = load8_now(vrow);
-                    v[pass][t][0] = raw.x;
-                    v[pass][t][DPT / 2 - 1] = raw.y;
-                }
-            } else {
-#pragma unroll
-                for (int w = 0; w < DPT / 2; w++) v[pass][t][w] = 0u;
-            }
-        }
-    };
-    load_values(0);
+    const uint32_t capacity = kv.capacity, first_tick = it.first_tick;
+    const float scale = sh.a.shape.attention_scale;
     asm volatile("cp.async.wait_all;" ::: "memory");
     team_barrier(barrier_id);  // the query rows are in shared memory
     float s[2][4];
+    {
+        float part[2][2][4];  // two chains per tile of eight tokens
 #pragma unroll
-    for (int nt = 0; nt < 2; nt++) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.0f;
+        for (int nt = 0; nt < 2; nt++)
 #pragma unroll
-    for (int w = 0; w < QW; w++) {
-        const uint32_t at = q_shared + static_cast<uint32_t>(g) * Q_PITCH + static_cast<uint32_t>(w) * 64u + static_cast<uint32_t>(j) * 16u;
-        const uint4 q0 = shared_load16<0>(at), q1 = shared_load16<8 * Q_PITCH>(at);
+            for (int c = 0; c < 4; c++) part[nt][0][c] = part[nt][1][c] = 0.0f;
 #pragma unroll
-        for (int nt = 0; nt < 2; nt++) {
-            mma_bf16_16816(s[nt], q0.x, q1.x, q0.y, q1.y, kf[nt][w].x, kf[nt][w].y);
-            mma_bf16_16816(s[nt], q0.z, q1.z, q0.w, q1.w, kf[nt][w].z, kf[nt][w].w);
+        for (int w = 0; w < QW; w++) {
+            const uint32_t at = q_shared + static_cast<uint32_t>(g) * Q_PITCH + static_cast<uint32_t>(w) * 64u + static_cast<uint32_t>(j) * 16u;
+            const uint4 q0 = shared_load16<0>(at), q1 = shared_load16<8 * Q_PITCH>(at);
+#pragma unroll
+            for (int nt = 0; nt < 2; nt++) {
+                mma_bf16_16816(part[nt][0], q0.x, q1.x, q0.y, q1.y, kf[nt][w].x, kf[nt][w].y);
+                mma_bf16_16816(part[nt][1], q0.z, q1.z, q0.w, q1.w, kf[nt][w].z, kf[nt][w].w);
+            }
         }
+#pragma unroll
+        for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) s[nt][c] = part[nt][0][c] + part[nt][1][c];
     }
-    if (HD / HALF > 1) load_values(HD / HALF - 1);
-    mark(21);
+    // the V rows (the warp's dims) of tokens 2j, 2j + 1, 2j + 8, 2j + 9 of every sixteen, in the K rows' registers: they
+    // arrive during the softmax
+    constexpr int VW = DPT > 2 ? 2 : 1;
+    uint32_t v[4][4][VW];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            const int token = 16 * k + 2 * j + (t & 1) + 8 * (t >> 1);
+            const uint16_t *vrow = values + static_cast<size_t>(rows[token]) * HD;
+            v[k][t][0] = v[k][t][VW - 1] = 0u;
+            if (token < count) {
+                if (DPT == 4) {
+                    const uint2 raw = load8_now(vrow);
+                    v[k][t][0] = raw.x;
+                    v[k][t][VW - 1] = raw.y;
+                } else {
+                    v[k][t][0] = DPT == 2 ? load4_now(vrow) : load2_now(vrow);
+                }
+            }
+        }
+    stamp(layer, 21);
 
     // ---- causal / ring mask, scale; the team's row maxima; probabilities
     float row_max[2] = {-INFINITY, -INFINITY};
@@ -962,7 +1053,7 @@ __device__ __noinline__ void attention_team_item(AttentionCache &cache, const Kv
 #pragma unroll
         for (int c = 0; c < 4; c++) {
             const int token = token0 + nt * 8 + 2 * j + (c & 1);
-            const uint32_t tick = tick_row[c >> 1], token_tick = first_tick + begin + token;
+            const uint32_t tick = tick_row[c >> 1], token_tick = first_tick + token;
             const bool visible = token < count && tick != 0xffffffffu && token_tick <= tick && token_tick + capacity > tick;
             s[nt][c] = visible ? s[nt][c] * scale : -INFINITY;
             row_max[c >> 1] = fmaxf(row_max[c >> 1], s[nt][c]);
@@ -994,105 +1085,79 @@ __device__ __noinline__ void attention_team_item(AttentionCache &cache, const Kv
         row_sum[r] += __shfl_xor_sync(0xffffffffu, row_sum[r], 2);
         if (j == 0) team_sum[team_warp * 16 + g + 8 * r] = row_sum[r];
     }
-    mark(22);
-    // probabilities as the A fragment of this warp's 16 tokens: high and low bf16 parts
-    uint32_t ph[4], pl[4];
+    // the probabilities as the A fragment of the warp's 16 tokens, high and low bf16 parts, for every warp of the team (the
+    // query rows are read: the maxima's barrier lies behind the products)
+    uint4 *fragments = reinterpret_cast<uint4 *>(team_smem);  // [high, low][16 tokens][lane]
+    {
+        uint32_t ph[4], pl[4];
 #pragma unroll
-    for (int f = 0; f < 4; f++) {
-        const float first = s[f >> 1][2 * (f & 1)], second = s[f >> 1][2 * (f & 1) + 1];
-        ph[f] = pack_bf16(first, second);
-        pl[f] = pack_bf16(first - bf16_lo(ph[f]), second - bf16_hi(ph[f]));
+        for (int f = 0; f < 4; f++) {
+            const float first = s[f >> 1][2 * (f & 1)], second = s[f >> 1][2 * (f & 1) + 1];
+            ph[f] = pack_bf16(first, second);
+            pl[f] = pack_bf16(first - bf16_lo(ph[f]), second - bf16_hi(ph[f]));
+        }
+        fragments[team_warp * 32 + lane] = make_uint4(ph[0], ph[1], ph[2], ph[3]);
+        fragments[128 + team_warp * 32 + lane] = make_uint4(pl[0], pl[1], pl[2], pl[3]);
     }
+    stamp(layer, 22);
+    team_barrier(barrier_id);
 
-    // ---- O = P V over the warp's tokens, HALF head dims per pass; thread column g owns dims DPT*g .. DPT*g+DPT-1
-    float *mine = partial_out + static_cast<size_t>(team_warp) * 16 * PITCH;
+    // ---- O = P V: the warp's dims over the split's tokens; thread column g owns dims DPT g .. DPT g + DPT - 1 of them
+    float o[DPT][4];
 #pragma unroll
-    for (int pass = 0; pass < HD / HALF; pass++) {
-        float o[DPT][4];
-#pragma unroll
-        for (int i = 0; i < DPT; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
+    for (int k = 0; k < 4; k++) {
+        const uint4 high = fragments[k * 32 + lane], low = fragments[128 + k * 32 + lane];
 #pragma unroll
         for (int i = 0; i < DPT; i++) {
             const uint32_t selector = (i & 1) ? 0x7632u : 0x5410u;
-            const uint32_t b0 = __byte_perm(v[pass][0][i >> 1], v[pass][1][i >> 1], selector), b1 = __byte_perm(v[pass][2][i >> 1], v[pass][3][i >> 1], selector);
-            mma_bf16_16816(o[i], ph[0], ph[1], ph[2], ph[3], b0, b1);
-            mma_bf16_16816(o[i], pl[0], pl[1], pl[2], pl[3], b0, b1);
+            const uint32_t b0 = __byte_perm(v[k][0][i >> 1], v[k][1][i >> 1], selector), b1 = __byte_perm(v[k][2][i >> 1], v[k][3][i >> 1], selector);
+            float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            mma_bf16_16816(part, high.x, high.y, high.z, high.w, b0, b1);
+            mma_bf16_16816(part, low.x, low.y, low.z, low.w, b0, b1);
+#pragma unroll
+            for (int c = 0; c < 4; c++) o[i][c] = k == 0 ? part[c] : o[i][c] + part[c];
         }
-        // accumulator column 2j (+1) of output tile i is head dim DPT * (2j (+1)) + i of the pass
-#pragma unroll
-        for (int r = 0; r < 2; r++)
-#pragma unroll
-            for (int half = 0; half < 2; half++)
-#pragma unroll
-                for (int i = 0; i < DPT; i += 4)
-                    *reinterpret_cast<float4 *>(mine + (g + 8 * r) * PITCH + DPT * (2 * j + half) + i) =
-                        make_float4(o[i][2 * r + half], o[i + 1][2 * r + half], o[i + 2][2 * r + half], o[i + 3][2 * r + half]);
-        team_barrier(barrier_id);
-        // the four partial outputs add up; warp w writes dims [w * HALF / 4, (w + 1) * HALF / 4) of the pass for every
-        // row, four dims per thread and round
-        constexpr int QUADS = HALF / 16;
-#pragma unroll
-        for (int round = 0; round < (16 * QUADS + 31) / 32; round++) {
-            const int task = round * 32 + lane, row = task / QUADS, d = team_warp * (HALF / 4) + (task % QUADS) * 4;
-            const int query_lane = lane0 + row / GROUP;  // rows beyond Q are padding
-            if (row < Q && query_lane < lanes && group_index * QL + row / GROUP < lanes_per_stream) {
-                const float *in = partial_out + row * PITCH + d;
-                const float4 p0 = *reinterpret_cast<const float4 *>(in), p1 = *reinterpret_cast<const float4 *>(in + 16 * PITCH),
-                             p2 = *reinterpret_cast<const float4 *>(in + 32 * PITCH), p3 = *reinterpret_cast<const float4 *>(in + 48 * PITCH);
-                const size_t partial = (static_cast<size_t>(query_lane) * q_heads + kv_head * GROUP + row % GROUP) * max_splits + split;
-                *reinterpret_cast<float4 *>(scratch + partial * HD + pass * HALF + d) =
-                    make_float4(p0.x + p1.x + p2.x + p3.x, p0.y + p1.y + p2.y + p3.y, p0.z + p1.z + p2.z + p3.z, p0.w + p1.w + p2.w + p3.w);
-            }
-        }
-        if (pass == 0 && team_warp == 0 && lane < Q) {
-            const int row = lane, query_lane = lane0 + row / GROUP;
-            if (query_lane < lanes && group_index * QL + row / GROUP < lanes_per_stream) {
-                const size_t partial = (static_cast<size_t>(query_lane) * q_heads + kv_head * GROUP + row % GROUP) * max_splits + split;
-                *reinterpret_cast<float2 *>(attention_stats(scratch, lanes, q_heads, max_splits, HD) + partial * 2) = make_float2(
-                    fmaxf(fmaxf(fmaxf(team_max[row], team_max[16 + row]), fmaxf(team_max[32 + row], team_max[48 + row])), -3.4028234663852886e38f),
-                    team_sum[row] + team_sum[16 + row] + team_sum[32 + row] + team_sum[48 + row]);
-            }
-        }
-        if (pass + 1 < HD / HALF) team_barrier(barrier_id);  // the partial outputs are rewritten by the next pass
     }
-    // ---- the team that completes the kv head's last split merges the splits of its queries; groups of more than
+    // accumulator column 2j (+1) of tile i is dim DPT * (2j (+1)) + i
+    float *scratch = sh.a.buffers.attention_scratch;
+    const int max_splits = sh.a.max_splits;
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        const int row = g + 8 * r;
+        if (tick_row[r] == 0xffffffffu) continue;  // padding
+        const size_t partial = (static_cast<size_t>(lane0 + row / GROUP) * q_heads + kv_head * GROUP + row % GROUP) * max_splits + it.split;
+        float *out = scratch + partial * HD + team_warp * DIMS + 2 * j * DPT;
+        float sums[2][DPT];
+#pragma unroll
+        for (int half = 0; half < 2; half++)
+#pragma unroll
+            for (int i = 0; i < DPT; i++) sums[half][i] = o[i][2 * r + half];
+        if (DPT == 4) {
+            *reinterpret_cast<float4 *>(out) = make_float4(sums[0][0], sums[0][DPT > 1 ? 1 : 0], sums[0][DPT > 2 ? 2 : 0], sums[0][DPT - 1]);
+            *reinterpret_cast<float4 *>(out + 4) = make_float4(sums[1][0], sums[1][DPT > 1 ? 1 : 0], sums[1][DPT > 2 ? 2 : 0], sums[1][DPT - 1]);
+        } else if (DPT == 2) {
+            *reinterpret_cast<float4 *>(out) = make_float4(sums[0][0], sums[0][DPT - 1], sums[1][0], sums[1][DPT - 1]);
+        } else {
+            *reinterpret_cast<float2 *>(out) = make_float2(sums[0][0], sums[1][0]);
+        }
+        if (team_warp == 0 && j == 0)
+            *reinterpret_cast<float2 *>(attention_stats(scratch, sh.a.lanes, q_heads, max_splits, HD) + partial * 2) =
+                make_float2(row_max[r], team_sum[row] + team_sum[16 + row] + team_sum[32 + row] + team_sum[48 + row]);
+    }
+    // ---- the team that completes the kv head's last split notes the merge of its queries for the CTA; groups of more than
     // MERGE_BLOCK splits are merged in two levels by the whole grid after the items
-    mark(23);
-    if (expected_splits > MERGE_BLOCK) {
-        team_barrier(barrier_id);  // the team's shared arrays are free for its next item
-        return;
-    }
-    __threadfence();
-    team_barrier(barrier_id);
-    unsigned int *arrival = arrivals + kv_head * group_slots + group_slot;
-    if (team_warp == 0 && lane == 0) *team_flag = atomicAdd(arrival, 1u);
-    team_barrier(barrier_id);
-    const bool last = *team_flag == static_cast<unsigned int>(expected_splits - 1);
-    mark(24);
-    if (last) {
-        // all splits of this kv head and lane group are in the scratch: the CTA merges them after its items (one row
-        // per warp); a CTA with more such heads than its list holds merges the rest right here
-        team_barrier(barrier_id);  // everybody has read the flag
-        if (team_warp == 0 && lane == 0) {
-            __threadfence();
+    stamp(layer, 23);
+    team_barrier(barrier_id);  // the team's partials are written, and its shared arrays free for its next item
+    if (it.splits <= MERGE_BLOCK && team_thread == 0) {
+        unsigned int *arrival = sh.a.buffers.barrier + ARRIVAL_WORDS_OFFSET + it.arrival;
+        unsigned int before;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(arrival) : "memory");  // covers the team's writes before the barrier
+        if (before == static_cast<unsigned int>(it.splits - 1)) {
             *arrival = 0u;  // for the next layer (several grid barriers away)
-            const int request = atomicAdd(&cache.merge_count, 1);
-            if (request < ATTENTION_MERGE_LIST) cache.merge_list[request] = kv_head * group_slots + group_slot;
-            *team_flag = static_cast<unsigned int>(request);
-        }
-        team_barrier(barrier_id);
-        if (*team_flag >= static_cast<unsigned int>(ATTENTION_MERGE_LIST)) {
-            __threadfence();
-            for (int row = team_warp; row < Q; row += 4) {
-                const int query_lane = lane0 + row / GROUP;
-                if (query_lane < lanes && group_index * QL + row / GROUP < lanes_per_stream)
-                    attention_merge_row<HD>(cache.job, attention_own_splits(cache.job, capacity, cache.tick[query_lane]), query_lane,
-                                            kv_head * GROUP + row % GROUP);
-            }
+            sh.merge_list[atomicAdd(&sh.merge_count, 1)] = static_cast<uint16_t>(it.arrival);
         }
     }
-    team_barrier(barrier_id);  // the team's shared arrays are free for its next item
-    mark(25);
+    stamp(layer, 24);
 }
 
 template <int GROUP>
@@ -1101,737 +1166,628 @@ struct AttentionTeam {
 };
 
 // ------------------------------------------------------------------------------------------ matrix blocks
+// A 16x128 block times the lanes of a batch, as signed bytes: the packed weights are q - 8 in two's complement, so a
+// nibble in the upper half of its byte is sixteen times the weight (one AND for eight weights, a shift in front for
+// the other eight), and an activation is three bytes (see the operand form).  Up to two lanes have their terms in
+// the eight columns of one MMA, up to four in two, up to eight in three:
+//   TILES 1: column 4 lane + term;  TILES 2: tile 0 column 2 lane + term (0, 1), tile 1 column 2 lane (term 2);
+//   TILES 3: tile `term`, column `lane`.
+// Why integers: with exact fp16 operands (q - 8) and per-group f32 sums a block cost 72 instructions of dequantisation
+// (nine for eight nibbles, most at half rate) and eight MMAs; here 24 and 4 TILES, mma.sync taking 32 bytes of K at the
+// rate of 16 fp16.  The accumulators start at 1.5 * 2^23 as an integer, which is the f32 of 1.5 * 2^23 + the sum.
+constexpr float SUM_BIAS_F32 = 12582912.0f;
 
-// One 16x128 block at `weights` (this thread's 16 bytes of rows g and, 512 bytes on, g + 8) against the staged
-// activations of its group: eight MMAs over exact fp16 (q - 8) operands in two accumulation chains.
-struct UnitOperands {
-    uint4 low, high;  // this thread's 32 nibbles of rows g and g + 8
-    uint4 b[4];       // its B fragments of the block's group
-    uint32_t scales;  // bf16 scale of row g | row g + 8
+// f32 sums of a thread over its groups: rows g and g + 8 of one lane (TILES 1: of lane j / 2 in the even thread columns,
+// TILES 2: of lane j), or of lanes 2j and 2j + 1 as a pair (TILES 3).
+template <int TILES>
+struct Accumulators {
+    float row[2];
 };
-__device__ __forceinline__ void unit_load(UnitOperands &u, uint32_t weights, uint32_t scales, uint32_t x, uint32_t word_stride) {
-    u.b[0] = shared_load16<0>(x);
-    u.b[1] = shared_load16<0>(x + word_stride);
-    u.b[2] = shared_load16<0>(x + 2 * word_stride);
-    u.b[3] = shared_load16<0>(x + 3 * word_stride);
-    u.low = shared_load16<0>(weights);
-    u.high = shared_load16<512>(weights);
-    u.scales = shared_load4(scales);
-}
-// Word `WORD` of the block: two MMAs into two of the block's four accumulation chains.
-template <int WORD>
-__device__ __forceinline__ void unit_word(const UnitOperands &u, float (&chains)[4][4]) {
-    const uint32_t wa = WORD == 0 ? u.low.x : (WORD == 1 ? u.low.y : (WORD == 2 ? u.low.z : u.low.w));
-    const uint32_t wb = WORD == 0 ? u.high.x : (WORD == 1 ? u.high.y : (WORD == 2 ? u.high.z : u.high.w));
-    const uint4 &b = u.b[WORD];
-    mma_f16_16816(chains[2 * (WORD & 1)], nibbles_low(wa), nibbles_low(wb), nibbles_high(wa), nibbles_high(wb), b.x, b.y);
-    const uint32_t upper_a = wa >> 8, upper_b = wb >> 8;
-    mma_f16_16816(chains[2 * (WORD & 1) + 1], nibbles_low(upper_a), nibbles_low(upper_b), nibbles_high(upper_a), nibbles_high(upper_b), b.z, b.w);
-}
-__device__ __forceinline__ void unit_finish(const UnitOperands &u, const float (&chains)[4][4], float (&acc)[4]) {
-    const float sa = __uint_as_float(u.scales << 16), sb = __uint_as_float(u.scales & 0xffff0000u);
-    acc[0] = fmaf(sa, (chains[0][0] + chains[1][0]) + (chains[2][0] + chains[3][0]), acc[0]);
-    acc[1] = fmaf(sa, (chains[0][1] + chains[1][1]) + (chains[2][1] + chains[3][1]), acc[1]);
-    acc[2] = fmaf(sb, (chains[0][2] + chains[1][2]) + (chains[2][2] + chains[3][2]), acc[2]);
-    acc[3] = fmaf(sb, (chains[0][3] + chains[1][3]) + (chains[2][3] + chains[3][3]), acc[3]);
-}
-// One 16x128 block against the staged activations of its group: eight MMAs over exact fp16 (q - 8) operands in
-// four accumulation chains; the group scale multiplies the block's f32 product.
-__device__ __forceinline__ void unit_single(const UnitOperands &u, float (&acc)[4]) {
-    float chains[4][4] = {};
-    unit_word<0>(u, chains);
-    unit_word<1>(u, chains);
-    unit_word<2>(u, chains);
-    unit_word<3>(u, chains);
-    unit_finish(u, chains, acc);
-}
-// Two blocks at once, their MMAs interleaved (eight independent chains).
-__device__ __forceinline__ void unit_pair(const UnitOperands &u, const UnitOperands &v, float (&acc)[4]) {
-    float cu[4][4] = {}, cv[4][4] = {};
-    unit_word<0>(u, cu);
-    unit_word<0>(v, cv);
-    unit_word<1>(u, cu);
-    unit_word<1>(v, cv);
-    unit_word<2>(u, cu);
-    unit_word<2>(v, cv);
-    unit_word<3>(u, cu);
-    unit_word<3>(v, cv);
-    unit_finish(u, cu, acc);
-    unit_finish(v, cv, acc);
-}
-
-// The steps of one pass as a warp sees them, in a function of its own so that the loop's registers are allotted
-// apart from the long-lived state of the kernel body.  For every stage of the pass: wait until it has landed,
-// multiply this warp's block (if it has one in this stage) and release the stage.  `x` is the shared-space address
-// of the thread's B fragments of the first step - relative to the stage for activation slices that ride the ring,
-// absolute (moving on by x_step per step) for the normalised rows.
-struct PassResult {
-    float acc[4];
-    uint32_t slot, parity, slice_slot, slice_parity;
-    uint32_t payload[4];  // what the epilogue needs from global memory (the residual values), requested before the steps
+template <>
+struct Accumulators<3> {
+    unsigned long long row[2];
 };
-struct PassRing {  // where the stages are and where this warp stands in them
-    uint32_t ring, full, empty, stages, stage_bytes;
-    uint32_t slices, slice_full, slice_empty, slice_slots, slice_bytes;
+template <int TILES>
+struct ActivationOperands {
+    uint4 b[TILES][2];
+    float factor[2];
 };
-template <bool X_IN_SLICE, int PER_STAGE>
-__device__ __noinline__ PassResult consume_pass(const PassRing ring, uint32_t slot, uint32_t parity, uint32_t slice_slot, uint32_t slice_parity,
-                                                int steps, int active_steps, uint32_t step_bytes, uint32_t weight_offset,
-                                                uint32_t scale_offset, uint32_t x, uint32_t x_step, uint32_t word_stride,
-                                                int *error_flag, const uint16_t *payload, uint32_t payload_stride, int payload_rounds) {
-    constexpr bool x_in_slice = X_IN_SLICE;
-    constexpr int steps_per_stage = PER_STAGE;
-    constexpr bool handshake = true;
-    uint32_t residual[4];
+template <int TILES>
+__device__ __forceinline__ void load_activations(ActivationOperands<TILES> &x, uint32_t group, const OperandPlace &place) {
 #pragma unroll
-    for (int round = 0; round < 4; round++) residual[round] = round < payload_rounds ? __ldcg(payload + static_cast<size_t>(round) * payload_stride) : 0;
-    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    const int lane = threadIdx.x & 31;
-    for (int step = 0; step < steps; step += steps_per_stage) {
-        const uint32_t stage_address = ring.ring + slot * ring.stage_bytes;
-        const uint32_t slice_address = ring.slices + slice_slot * ring.slice_bytes;
-        if (handshake) {
-            wait_stage(ring.full + slot * 8, parity, error_flag);
-            if (x_in_slice) wait_stage(ring.slice_full + slice_slot * 8, slice_parity, error_flag);
+    for (int h = 0; h < 2; h++) {
+        x.b[0][h] = smem16(group + place.first + h * place.half);
+        if (TILES == 2) x.b[TILES - 1][h] = smem16(group + place.second + h * place.half);
+        if (TILES == 3) x.b[TILES > 1 ? 1 : 0][h] = smem16(group + place.first + h * place.half + 64), x.b[TILES - 1][h] = smem16(group + place.first + h * place.half + 128);
+    }
+    if (TILES == 3) {
+        const float2 both = *reinterpret_cast<const float2 *>(smem_raw + group + place.factor);
+        x.factor[0] = both.x, x.factor[1] = both.y;
+    } else {
+        x.factor[0] = x.factor[1] = *reinterpret_cast<const float *>(smem_raw + group + place.factor);
+    }
+}
+// Constants of the products, made where a pass begins: the compiler would keep them in registers through the whole layer.
+struct ProductConstants {
+    int32_t bias;
+    uint32_t sixteen;  // a multiplication goes to the FMA pipe: AND and shift share a pipe of half the rate
+    unsigned long long unbias, term0, term1;  // pairs
+};
+__device__ __forceinline__ ProductConstants product_constants() {
+    ProductConstants c;
+    asm volatile("mov.b32 %0, 0x4B400000;" : "=r"(c.bias));
+    asm volatile("mov.b32 %0, 16;" : "=r"(c.sixteen));
+    asm volatile("mov.b64 %0, 0xCB400000CB400000;" : "=l"(c.unbias));
+    asm volatile("mov.b64 %0, 0x4780000047800000;" : "=l"(c.term0));
+    asm volatile("mov.b64 %0, 0x4380000043800000;" : "=l"(c.term1));
+    return c;
+}
+template <int TILES>
+__device__ __forceinline__ void block_product(const uint4 (&rows)[2], uint32_t scales, const ActivationOperands<TILES> &x, const ProductConstants &c, Accumulators<TILES> &acc) {
+    const uint32_t wa[4] = {rows[0].x, rows[0].y, rows[0].z, rows[0].w}, wb[4] = {rows[1].x, rows[1].y, rows[1].z, rows[1].w};
+    int32_t sums[TILES][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const uint32_t a0 = (wa[i] * c.sixteen) & 0xf0f0f0f0u, a1 = (wb[i] * c.sixteen) & 0xf0f0f0f0u, a2 = wa[i] & 0xf0f0f0f0u, a3 = wb[i] & 0xf0f0f0f0u;
+#pragma unroll
+        for (int t = 0; t < TILES; t++) {
+            const uint4 &b = x.b[t][i >> 1];
+            const uint32_t b0 = (i & 1) ? b.z : b.x, b1 = (i & 1) ? b.w : b.y;
+            int32_t(&sum)[4] = sums[t];
+            if (i == 0) mma_s8_16832(sum, a0, a1, a2, a3, b0, b1, c.bias, c.bias, c.bias, c.bias);
+            else mma_s8_16832(sum, a0, a1, a2, a3, b0, b1, sum[0], sum[1], sum[2], sum[3]);
         }
-        int here = active_steps - step;  // this warp's blocks in the stage
-        if (here > steps_per_stage) here = steps_per_stage;
-        if (here > 0) {
-            const uint32_t x_first = x_in_slice ? slice_address + x : x;
-            UnitOperands u;
-            unit_load(u, stage_address + weight_offset, stage_address + scale_offset, x_first, word_stride);
-            unit_single(u, acc);
-            if (PER_STAGE == 2 && here == 2) {
-                unit_load(u, stage_address + step_bytes + weight_offset, stage_address + step_bytes + scale_offset, x_first + x_step, word_stride);
-                unit_single(u, acc);
+    }
+    const float scale[2] = {__uint_as_float(scales << 16), __uint_as_float(scales & 0xffff0000u)};
+    // the group's sum t0 2^16 + t1 2^8 + t2, rounded to f32 once (but for the last bits of t1 2^8 + t2), times the scale
+    if constexpr (TILES == 3) {
+        const unsigned long long factors = pair_of(x.factor[0], x.factor[1]);
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            unsigned long long term[3];
+#pragma unroll
+            for (int t = 0; t < 3; t++) term[t] = pair_add(pair_of(__int_as_float(sums[t][2 * r]), __int_as_float(sums[t][2 * r + 1])), c.unbias);
+            const unsigned long long sum = pair_fma(term[0], c.term0, pair_fma(term[1], c.term1, term[2]));
+            acc.row[r] = pair_fma(pair_multiply(factors, pair_of(scale[r], scale[r])), sum, acc.row[r]);
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            float term[3];
+            if constexpr (TILES == 1) {
+                const float own = __int_as_float(sums[0][2 * r]) - SUM_BIAS_F32;
+                term[0] = own;
+                term[1] = __int_as_float(sums[0][2 * r + 1]) - SUM_BIAS_F32;
+                term[2] = __shfl_down_sync(0xffffffffu, own, 1);  // term 2 sits one thread column further
+            } else {
+                term[0] = __int_as_float(sums[0][2 * r]) - SUM_BIAS_F32;
+                term[1] = __int_as_float(sums[0][2 * r + 1]) - SUM_BIAS_F32;
+                term[2] = __int_as_float(sums[TILES - 1][2 * r]) - SUM_BIAS_F32;
             }
-            if (!x_in_slice) x += static_cast<uint32_t>(here) * x_step;
-        }
-        __syncwarp();
-        if (lane == 0 && handshake) {
-            mbarrier_arrive(ring.empty + slot * 8);
-            if (x_in_slice) mbarrier_arrive(ring.slice_empty + slice_slot * 8);
-        }
-        if (++slot == ring.stages) {
-            slot = 0;
-            parity ^= 1u;
-        }
-        if (x_in_slice && ++slice_slot == ring.slice_slots) {
-            slice_slot = 0;
-            slice_parity ^= 1u;
+            acc.row[r] = fmaf(scale[r] * x.factor[0], fmaf(term[0], 65536.0f, fmaf(term[1], 256.0f, term[2])), acc.row[r]);
         }
     }
-    PassResult result;
+}
+// A tile's sums of the warp, to sums[row][lane].
+template <int TILES>
+__device__ __forceinline__ void store_sums(float *sums, const Accumulators<TILES> &acc) {
+    const int lane = thread_now() & 31, g = lane >> 2, j = lane & 3;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        result.acc[i] = acc[i];
-        result.payload[i] = residual[i];
+    for (int r = 0; r < 2; r++) {
+        float *row = sums + (g + 8 * r) * 8;
+        if constexpr (TILES == 3) *reinterpret_cast<unsigned long long *>(row + 2 * j) = acc.row[r];
+        else if (TILES == 2) row[j] = acc.row[r];
+        else if ((j & 1) == 0) row[j >> 1] = acc.row[r];
     }
-    result.slot = slot;
-    result.parity = parity;
-    result.slice_slot = slice_slot;
-    result.slice_parity = slice_parity;
-    return result;
 }
 
-// The gate/up step when a stage holds two steps of two blocks per tile slot (gate and up of one group of K each):
-// the slot's two warps take one step each and multiply BOTH its blocks - gate and up rows against the same
-// activations, read once - with the sixteen MMAs interleaved in eight accumulation chains.  Returns the warp's partial
-// sums of the gate rows (acc) and of the up rows (second).
-struct PairResult {
-    float acc[4], second[4];
-    uint32_t slot, parity;
+// The steps of one pass (or of one window of it) as a warp sees them.  Offsets are from the start of shared memory.
+// Where the warps stand in the two rings, in one word: slot, slice slot, and the parities of both.
+struct RingPlace {
+    uint32_t slot, parity, slice_slot, slice_parity;
 };
-struct PairOperands {
-    uint4 low_a, high_a, low_b, high_b;  // this thread's nibbles of rows g and g + 8: gate block, up block
-    uint4 b[4];                          // its B fragments of the group
-    uint32_t scales_a, scales_b;
-};
-template <int WORD>
-__device__ __forceinline__ void pair_word(const PairOperands &p, float (&ca)[4][4], float (&cb)[4][4]) {
-    const uint4 &b = p.b[WORD];
-    const uint32_t wa = WORD == 0 ? p.low_a.x : (WORD == 1 ? p.low_a.y : (WORD == 2 ? p.low_a.z : p.low_a.w));
-    const uint32_t wb = WORD == 0 ? p.high_a.x : (WORD == 1 ? p.high_a.y : (WORD == 2 ? p.high_a.z : p.high_a.w));
-    const uint32_t va = WORD == 0 ? p.low_b.x : (WORD == 1 ? p.low_b.y : (WORD == 2 ? p.low_b.z : p.low_b.w));
-    const uint32_t vb = WORD == 0 ? p.high_b.x : (WORD == 1 ? p.high_b.y : (WORD == 2 ? p.high_b.z : p.high_b.w));
-    mma_f16_16816(ca[2 * (WORD & 1)], nibbles_low(wa), nibbles_low(wb), nibbles_high(wa), nibbles_high(wb), b.x, b.y);
-    mma_f16_16816(cb[2 * (WORD & 1)], nibbles_low(va), nibbles_low(vb), nibbles_high(va), nibbles_high(vb), b.x, b.y);
-    const uint32_t upper_wa = wa >> 8, upper_wb = wb >> 8, upper_va = va >> 8, upper_vb = vb >> 8;
-    mma_f16_16816(ca[2 * (WORD & 1) + 1], nibbles_low(upper_wa), nibbles_low(upper_wb), nibbles_high(upper_wa), nibbles_high(upper_wb), b.z, b.w);
-    mma_f16_16816(cb[2 * (WORD & 1) + 1], nibbles_low(upper_va), nibbles_low(upper_vb), nibbles_high(upper_va), nibbles_high(upper_vb), b.z, b.w);
+__device__ __forceinline__ RingPlace unpack_place(uint32_t packed) { return {packed & 255u, (packed >> 16) & 1u, (packed >> 8) & 255u, (packed >> 17) & 1u}; }
+__device__ __forceinline__ uint32_t pack_place(const RingPlace &at) { return at.slot | (at.slice_slot << 8) | (at.parity << 16) | (at.slice_parity << 17); }
+
+__device__ __forceinline__ WarpBlocks warp_blocks(int phase, int pass, int warp) {
+    const StackShared &sh = shared();
+    const PhaseInfo &pi = sh.info[phase];
+    const int width = pi.width, pair = warp >> pi.width_log2, group = warp & (width - 1), present = stage_present(pi, pass), tiles = present - 2 * pair;
+    const uint32_t group_bytes = operand_group_bytes(sh.a.lanes), first = static_cast<uint32_t>(2 * pair * width + group);
+    WarpBlocks b;
+    b.unit = sh.ring + first * UNIT_BYTES;
+    b.scales = static_cast<uint32_t>(present * width) * UNIT_BYTES + first * UNIT_SCALE_BYTES - first * UNIT_BYTES;
+    b.next_tile = static_cast<uint32_t>(width) * UNIT_BYTES;
+    b.x = sh.scratch + static_cast<uint32_t>(group) * group_bytes;
+    b.x_step = phase == 3 ? static_cast<uint32_t>(sh.a.slice_bytes) : static_cast<uint32_t>(width) * group_bytes;
+    b.steps = tiles <= 0 || group >= pi.groups ? 0 : (pi.groups - group + width - 1) >> pi.width_log2;
+    b.tiles = tiles > 1 ? 2 : 1;
+    return b;
 }
-__device__ __forceinline__ void pair_finish(uint32_t scales, const float (&chains)[4][4], float (&acc)[4]) {
-    const float sa = __uint_as_float(scales << 16), sb = __uint_as_float(scales & 0xffff0000u);
-    acc[0] = fmaf(sa, (chains[0][0] + chains[1][0]) + (chains[2][0] + chains[3][0]), acc[0]);
-    acc[1] = fmaf(sa, (chains[0][1] + chains[1][1]) + (chains[2][1] + chains[3][1]), acc[1]);
-    acc[2] = fmaf(sb, (chains[0][2] + chains[1][2]) + (chains[2][2] + chains[3][2]), acc[2]);
-    acc[3] = fmaf(sb, (chains[0][3] + chains[1][3]) + (chains[2][3] + chains[3][3]), acc[3]);
-}
-// `first_block`: byte offset of the gate block of the warp's slot inside a step; `first_scales`: of its scale row;
-// `mine`: which of the stage's two steps this warp takes; `x`: its B fragments of that step's group in the first stage.
-__device__ __noinline__ PairResult consume_pass_pairs(const PassRing ring, uint32_t slot, uint32_t parity, int steps, bool active, int mine, uint32_t step_bytes,
-                                                      uint32_t first_block, uint32_t first_scales, uint32_t x, uint32_t x_stage_step, uint32_t word_stride,
-                                                      int *error_flag) {
-    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f}, second[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    const int lane = threadIdx.x & 31;
-    for (int step = 0; step < steps; step += 2) {
-        const uint32_t stage_address = ring.ring + slot * ring.stage_bytes;
-        wait_stage(ring.full + slot * 8, parity, error_flag);
-        if (active && step + mine < steps) {
-            const uint32_t base = stage_address + static_cast<uint32_t>(mine) * step_bytes;
-            PairOperands p;
-            p.b[0] = shared_load16<0>(x);
-            p.b[1] = shared_load16<0>(x + word_stride);
-            p.b[2] = shared_load16<0>(x + 2 * word_stride);
-            p.b[3] = shared_load16<0>(x + 3 * word_stride);
-            p.low_a = shared_load16<0>(base + first_block);
-            p.high_a = shared_load16<512>(base + first_block);
-            p.low_b = shared_load16<UNIT_BYTES>(base + first_block);
-            p.high_b = shared_load16<UNIT_BYTES + 512>(base + first_block);
-            p.scales_a = shared_load4(base + first_scales);
-            p.scales_b = shared_load4(base + first_scales + UNIT_SCALE_BYTES);
-            float ca[4][4] = {}, cb[4][4] = {};
-            pair_word<0>(p, ca, cb);
-            pair_word<1>(p, ca, cb);
-            pair_word<2>(p, ca, cb);
-            pair_word<3>(p, ca, cb);
-            pair_finish(p.scales_a, ca, acc);
-            pair_finish(p.scales_b, cb, second);
-            x += x_stage_step;
+
+// Every stage holds, for this warp, the blocks of two tiles and one group of K, multiplied by the same activations: tiles
+// 2 pair and 2 pair + 1 of the pass, group step * width + place.  Leaves the sums in `reduce` - of a window that is not
+// the pass's last, the thread's own sums, which its next window starts from.
+template <int TILES, bool X_IN_SLICE>
+__device__ __forceinline__ uint32_t consume_pass(int phase, int pass, int first_step) {
+    StackShared &sh = shared();
+    const int thread = thread_now(), warp = thread >> 5, lane = thread & 31;
+    const int left = sh.info[phase].steps - first_step, window = sh.info[phase].window, steps = left < window ? left : window;
+    const WarpBlocks blocks = pass == 0 ? sh.blocks[phase][warp] : warp_blocks(phase, pass, warp);
+    const OperandPlace place = sh.operand_place[lane];
+    const int active = blocks.steps - first_step < steps ? blocks.steps - first_step : steps, tiles = blocks.tiles;
+    const uint32_t scales_from_unit = blocks.scales - static_cast<uint32_t>(lane) * 16u + static_cast<uint32_t>(lane >> 2) * 4u, next_tile = blocks.next_tile,
+                   x_step = blocks.x_step;
+    static_assert(offsetof(StackShared, empty) == offsetof(StackShared, full) + EMPTY && offsetof(StackShared, slice_full) == offsetof(StackShared, full) + SLICE_FULL &&
+                      offsetof(StackShared, slice_empty) == offsetof(StackShared, full) + SLICE_EMPTY,
+                  "a slot's barriers are found from its first one");
+    RingPlace at = unpack_place(sh.place);
+    const uint32_t full = shared_address(sh.full), last_barrier = full + 8u * (static_cast<uint32_t>(sh.a.stages) - 1), ring_bytes = (static_cast<uint32_t>(sh.a.stages) - 1) * STAGE_BYTES;
+    const uint32_t last_slice_barrier = full + 8u * static_cast<uint32_t>(sh.a.slice_slots - 1), slices_bytes = static_cast<uint32_t>(sh.a.slice_slots - 1) * x_step;
+    uint32_t barrier = full + at.slot * 8u, slice_barrier = full + at.slice_slot * 8u;
+    uint32_t unit = blocks.unit + static_cast<uint32_t>(lane) * 16u + at.slot * static_cast<uint32_t>(STAGE_BYTES);
+    uint32_t x = blocks.x + (X_IN_SLICE ? at.slice_slot * x_step : 0u);
+    const ProductConstants constants = product_constants();
+    Accumulators<TILES> acc[2];
+    Accumulators<TILES> *carried = reinterpret_cast<Accumulators<TILES> *>(&sh.reduce[0][0][0]) + 2 * thread;
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+        acc[t].row[0] = acc[t].row[1] = 0;
+        if (first_step > 0) acc[t] = carried[t];
+    }
+#pragma unroll 1
+    for (int step = 0; step < steps; step++) {
+        wait_barrier(barrier, at.parity);
+        if (X_IN_SLICE) wait_barrier(slice_barrier + SLICE_FULL, at.slice_parity);
+        if (step < active) {
+            ActivationOperands<TILES> operands;
+            uint4 rows[2][2];
+            uint32_t row_scales[2];
+            rows[0][0] = smem16(unit);
+            rows[0][1] = smem16(unit + 512);
+            row_scales[0] = smem4(unit + scales_from_unit);
+            load_activations<TILES>(operands, x, place);
+            if (tiles > 1) {
+                rows[1][0] = smem16(unit + next_tile);
+                rows[1][1] = smem16(unit + next_tile + 512);
+                row_scales[1] = smem4(unit + scales_from_unit + next_tile / 32u);
+            }
+            block_product<TILES>(rows[0], row_scales[0], operands, constants, acc[0]);
+            if (tiles > 1) block_product<TILES>(rows[1], row_scales[1], operands, constants, acc[1]);
         }
         __syncwarp();
-        if (lane == 0) mbarrier_arrive(ring.empty + slot * 8);
-        if (++slot == ring.stages) {
-            slot = 0;
-            parity ^= 1u;
+        if (lane == 0) {
+            mbarrier_arrive(barrier + EMPTY);
+            if (X_IN_SLICE) mbarrier_arrive(slice_barrier + SLICE_EMPTY);
+        }
+        if (barrier == last_barrier) {
+            barrier = full;
+            unit -= ring_bytes;
+            at.parity ^= 1u;
+        } else {
+            barrier += 8u;
+            unit += STAGE_BYTES;
+        }
+        if (X_IN_SLICE) {
+            if (slice_barrier == last_slice_barrier) {
+                slice_barrier = full;
+                x -= slices_bytes;
+                at.slice_parity ^= 1u;
+            } else {
+                slice_barrier += 8u;
+                x += x_step;
+            }
+        } else {
+            x += x_step;
         }
     }
-    PairResult result;
+    at.slot = (barrier - full) >> 3;
+    at.slice_slot = (slice_barrier - full) >> 3;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        result.acc[i] = acc[i];
-        result.second[i] = second[i];
+    for (int t = 0; t < 2; t++) {
+        if (steps < left) carried[t] = acc[t];
+        else store_sums<TILES>(sh.reduce[warp][t], acc[t]);
     }
-    result.slot = slot;
-    result.parity = parity;
-    return result;
+    return pack_place(at);
 }
 
 // ------------------------------------------------------------------------------------------ the kernel
 
-// EXCHANGE: the tensor-parallel form (o and down leave partial sums that are exchanged between the ranks).
-template <int HD, int GROUP, bool EXCHANGE>
-__global__ void __launch_bounds__(STACK_THREADS, 1) decode_stack_kernel(const StackArgs a) {
-    extern __shared__ __align__(128) uint8_t smem_raw[];
-    if (a.buffers.timing != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
-        unsigned long long now;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-        a.buffers.timing[16] = now;
+// One matrix step of a layer: stage the activations, stream the CTA's weights, finish the outputs.  Phase 0: q | k | v,
+// 1: o, 2: gate and up, 3: down.  EXCHANGE: the tensor-parallel form (o and down leave partial sums that are exchanged
+// between the ranks).
+template <int HD, bool EXCHANGE, int TILES>
+__device__ __forceinline__ void matrix_step(int phase, int layer) {
+    StackShared &sh = shared();
+    stamp(layer, 4 * phase);
+    int pass = 0, first_step = 0;
+#pragma unroll 1
+    while (pass < sh.info[phase].passes) {
+        // ---- activations of q/k/v and gate/up: normalised rows, of o: the attention outputs, staged by every CTA - in
+        // windows of a pass's steps where whole rows are too large; those of down arrive in slices
+        const int window = sh.info[phase].window;
+        if (phase != 3 && (pass == 0 || first_step > 0 || window < sh.info[phase].steps || (phase == 2 && sh.products == sh.scratch))) {  // (products over the rows)
+            const StackLayer &spec = sh.layer[layer & 1];
+            stage_any<TILES>(phase == 1 ? sh.a.buffers.attention_out : sh.a.buffers.hidden, phase == 0 ? spec.input_norm : (phase == 2 ? spec.post_norm : nullptr),
+                             phase == 1 ? sh.a.shape.q_heads * HD : sh.a.shape.hidden, first_step * sh.info[phase].width, window * sh.info[phase].width);
+        }
+        if (pass == 0 && first_step == 0) stamp(layer, 4 * phase + 1);
+        // Epilogue roles: thread t finishes output (high = t & 1, lane m = (t >> 1) & 7, row = ((t >> 4) & 7) + 8 * high)
+        // of tile (t >> 7) + 4 * round of the pass - of gate/up the pair of tiles -, so the rotary partner rows r and r + 8
+        // of a lane sit in neighbouring threads.  The first round's residual value is requested before the arithmetic.
+        uint32_t residual = 0;
+        if (phase & 1) {
+            const int thread = thread_now();
+            if (((thread >> 1) & 7) < sh.a.lanes && (thread >> 7) < stage_present(sh.info[phase], pass))
+                residual = __ldcg(sh.a.buffers.hidden + sh.output[thread] + pass * sh.info[phase].slots * static_cast<int>(gridDim.x) * 16);
+        }
+        const uint32_t place = phase == 3 ? consume_pass<TILES, true>(phase, pass, first_step) : consume_pass<TILES, false>(phase, pass, first_step);
+        stamp(layer, 26 + phase);
+        cta_sync();
+        if (thread_now() == 0) sh.place = place;  // read again behind the next meeting
+        first_step += window;
+        if (first_step < sh.info[phase].steps) {
+            cta_sync();  // every warp is through with the window, its place noted
+            continue;
+        }
+        first_step = 0;
+        const int thread = thread_now(), m = (thread >> 1) & 7, row = ((thread >> 4) & 7) + 8 * (thread & 1);
+        const bool lane_present = m < sh.a.lanes;
+        const int tiles = phase == 2 ? stage_present(sh.info[phase], pass) >> 1 : stage_present(sh.info[phase], pass), width = sh.info[phase].width;
+#pragma unroll 1
+        for (int slot = thread >> 7; slot < tiles; slot += 4) {  // uniform over the warp
+            float first = 0.0f, second = 0.0f;
+            const float *src = &sh.reduce[(phase == 2 ? slot : slot >> 1) * width][phase == 2 ? 0 : slot & 1][row * 8 + m];
+            for (int w = 0; w < width; w++) {
+                first += src[w * 256];
+                if (phase == 2) second += src[w * 256 + 128];
+            }
+            if (phase == 0) {
+                // q / k: rotary_bf16.comp.template:99-109 (non-interleaved, rotary width = head width, five bf16
+                // roundings); k and v go into the lane's KV page (append_gqa_attention_bf16.comp.template:189-215)
+                const int tile = static_cast<int>(blockIdx.x) + (pass * sh.info[phase].slots + slot) * static_cast<int>(gridDim.x);
+                const int q_tiles = (sh.a.shape.q_heads * HD) >> 4, k_tiles = (sh.a.shape.kv_heads * HD) >> 4;
+                const float mine_value = round_bf16(first);
+                const float partner = __shfl_xor_sync(0xffffffffu, mine_value, 1);  // the row 8 further (or 8 back)
+                if (lane_present) {
+                    const KvLayer &kv = sh.layer[layer & 1].kv;
+                    const size_t kv_token = sh.kv_row[m];
+                    const bool kv_writable = kv_token != ~0ull;
+                    const size_t head_stride = static_cast<size_t>(kv.page_tokens) * HD;
+                    if (tile < q_tiles + k_tiles) {
+                        const bool is_q = tile < q_tiles, high = row >= 8;
+                        const int local = is_q ? tile : tile - q_tiles;
+                        const int head = local / (HD >> 4), d = 8 * (local % (HD >> 4)) + (row & 7) + (high ? HD / 2 : 0);
+                        const uint32_t rotation = sh.rope[m * (HD >> 1) + 8 * (local % (HD >> 4)) + (row & 7)];
+                        const float cosine = bf16_lo(rotation), sine = bf16_hi(rotation);
+                        // d < half: x cos + (-x[d + half]) sin;  d >= half: x cos + x[d - half] sin
+                        const float other = high ? partner : -partner;
+                        const uint16_t value = static_cast<uint16_t>(f32_to_bf16_bits(round_bf16(mine_value * cosine) + round_bf16(other * sine)));
+                        if (is_q) sh.a.buffers.q[(static_cast<size_t>(m) * sh.a.shape.q_heads + head) * HD + d] = value;
+                        else if (kv_writable) kv.pool[kv_token + static_cast<size_t>(head) * head_stride + d] = value;
+                    } else if (kv_writable) {
+                        const int index = (tile - q_tiles - k_tiles) * 16 + row;
+                        kv.pool[kv_token + static_cast<size_t>(kv.kv_heads + index / HD) * head_stride + index % HD] = static_cast<uint16_t>(f32_to_bf16_bits(first));
+                    }
+                }
+            } else if (phase == 2) {
+                // silu_multiply_bf16.comp.template:30-52: bf16(silu_bf16(bf16 gate) * bf16 up)
+                if (lane_present)
+                    *reinterpret_cast<float *>(smem_raw + sh.products + (m * 128 + slot * 16 + row) * 4) = round_bf16(rounded_silu(round_bf16(first)) * round_bf16(second));
+            } else if (lane_present) {
+                float total = first;
+                uint16_t *out = sh.a.buffers.hidden + sh.output[thread] + (pass * sh.info[phase].slots + slot - (thread >> 7)) * static_cast<int>(gridDim.x) * 16;
+                if constexpr (EXCHANGE) {
+                    // this rank's share of the sum over K goes to every peer's inbox, value and exchange number in
+                    // one 8-byte store; the peers' shares arrive in this rank's inbox the same way
+                    const StackTp &tp = *sh.a.tp;
+                    int *error_flag = sh.a.buffers.error_flag;
+                    const uint32_t number = sh.exchanges + static_cast<uint32_t>(2 * layer + (phase == 1 ? 1 : 2));
+                    const size_t element = static_cast<size_t>(number & 1u) * STACK_TP_MAX_RANKS * 8 * sh.a.shape.hidden + (out - sh.a.buffers.hidden);
+                    const unsigned long long word = (static_cast<unsigned long long>(number) << 32) | __float_as_uint(first);
+                    for (int r = 0; r < tp.size; r++)
+                        if (r != tp.rank)
+                            asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(reinterpret_cast<unsigned long long *>(tp.exchange[r]) + element +
+                                                                                  static_cast<size_t>(tp.rank) * 8 * sh.a.shape.hidden),
+                                         "l"(word)
+                                         : "memory");
+                    total = 0.0f;
+                    unsigned int spins = 0;
+                    bool gave_up = false;
+                    for (int r = 0; r < tp.size; r++) {  // rank order on every rank: the replicas stay bit-identical
+                        float part = first;
+                        if (r != tp.rank) {
+                            const unsigned long long *source =
+                                reinterpret_cast<const unsigned long long *>(tp.exchange[tp.rank]) + element + static_cast<size_t>(r) * 8 * sh.a.shape.hidden;
+                            unsigned long long got = 0;
+                            while (!gave_up) {
+                                asm volatile("ld.relaxed.sys.global.u64 %0, [%1];" : "=l"(got) : "l"(source) : "memory");
+                                if (static_cast<uint32_t>(got >> 32) == number) break;
+                                if (++spins > STACK_TP_SPIN_LIMIT) {
+                                    atomicExch(error_flag, 2);
+                                    gave_up = true;
+                                } else if ((spins & 255u) == 0 && *reinterpret_cast<volatile int *>(error_flag) != 0) {
+                                    gave_up = true;
+                                }
+                            }
+                            part = __uint_as_float(static_cast<uint32_t>(got));
+                        }
+                        total += part;
+                    }
+                }
+                // linear + residual_add (add_bf16.comp.template:17-24): bf16(bf16(product) + residual), in place
+                const uint32_t before = slot < 4 ? residual : __ldcg(out);
+                *out = static_cast<uint16_t>(f32_to_bf16_bits(round_bf16(total) + bf16_bits_to_f32(before)));
+            }
+        }
+        if (phase == 2) {
+            // the pass's eight tiles of gate and of up are one group of down's columns: into operand form, one warp per lane
+            cta_sync();
+            const int warp = thread_now() >> 5, lanes = sh.a.lanes;
+            if (warp < lanes)
+                store_operand_group(sh.a.buffers.activation + static_cast<size_t>(blockIdx.x + pass * gridDim.x) * operand_group_bytes(lanes),
+                                    reinterpret_cast<const float *>(smem_raw + sh.products) + warp * 128, warp, lanes);
+        }
+        pass++;
+        if (pass < sh.info[phase].passes) cta_sync();  // the partial sums are rewritten by the next pass
     }
+    stamp(layer, 4 * phase + 2);
+}
+
+// Attention of a layer: (kv head, split, stream x lane group) items, one team of four warps each, spread over the SMs
+// first; the teams' shared arrays reuse the scratch area (nothing is staged right now).
+template <int HD, int GROUP>
+__device__ __forceinline__ void attention_step(int layer) {
     constexpr int QL = AttentionTeam<GROUP>::QL;
-    const StackShape &shape = a.shape;
-    const int lanes = a.lanes, staged = lanes < 8 ? lanes : 8;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
+    StackShared &sh = shared();
+    const int total = sh.a.shape.kv_heads * sh.a.max_splits * sh.group_slots;
+    {
+        const int team = thread_now() >> 7;
+        bool first = true;
+#pragma unroll 1
+        for (int item = blockIdx.x + gridDim.x * team; item < total; item += gridDim.x * 4) {
+            if (!first) {
+                if ((thread_now() & 127) == 0) sh.later_item[team] = attention_item<QL>(sh.layer[layer & 1].kv, item);
+                team_barrier(2 + team);
+            }
+            const AttentionItem &it = first ? sh.item[team] : sh.later_item[team];
+            if (it.count > 0) attention_team_item<HD, GROUP, QL>(layer, it, first);
+            first = false;
+        }
+    }
+    cta_sync();
+    stamp(layer, 17);
+    {
+        // merge the heads whose last split was completed here: one (lane, q head) row per warp and round
+        const int requests = sh.merge_count;
+        if (requests > 0) {
+            __threadfence();
+            const int group_slots = sh.group_slots, per_stream = sh.a.lanes_per_stream, groups_per_stream = (per_stream + QL - 1) / QL;
+            for (int index = thread_now() >> 5; index < requests * QL * GROUP; index += CONSUMER_WARPS) {
+                const int request = sh.merge_list[index / (QL * GROUP)], row = index % (QL * GROUP);
+                const int kv_head = request / group_slots, group_slot = request % group_slots;
+                const int group_index = group_slot % groups_per_stream;
+                const int query_lane = (group_slot / groups_per_stream) * per_stream + group_index * QL + row / GROUP;
+                if (query_lane < sh.a.lanes && group_index * QL + row / GROUP < per_stream && sh.slot[query_lane] >= 0)
+                    attention_merge_row<HD>(attention_own_splits(sh.layer[layer & 1].kv.capacity, sh.tick[query_lane]), query_lane, kv_head * GROUP + row % GROUP);
+            }
+        }
+    }
+    if (sh.a.max_splits > MERGE_BLOCK) {
+        // ---- groups of more than MERGE_BLOCK splits: every warp of the grid merges ranges of MERGE_BLOCK splits into one
+        // partial each, then one warp per row merges the row's range partials
+        const int ranges = attention_ranges(sh.a.max_splits), q_heads = sh.a.shape.q_heads, rows = sh.a.lanes * q_heads;
+        const uint32_t capacity = sh.layer[layer & 1].kv.capacity;
+        grid_meet(false);
+        for (int task = blockIdx.x + gridDim.x * (thread_now() >> 5); task < rows * ranges; task += gridDim.x * CONSUMER_WARPS) {
+            const int row = task / ranges, range = task % ranges, query_lane = row / q_heads;
+            if (sh.slot[query_lane] < 0) continue;
+            const int splits = attention_group_splits(capacity, query_lane, QL);
+            if (splits > MERGE_BLOCK && range * MERGE_BLOCK < splits) attention_merge_range<HD>(splits, query_lane, row % q_heads, range);
+        }
+        grid_meet(false);
+        for (int row = blockIdx.x + gridDim.x * (thread_now() >> 5); row < rows; row += gridDim.x * CONSUMER_WARPS) {
+            const int query_lane = row / q_heads;
+            if (sh.slot[query_lane] < 0) continue;
+            const int splits = attention_group_splits(capacity, query_lane, QL);
+            if (splits > MERGE_BLOCK) attention_merge_ranges<HD>(splits, query_lane, row % q_heads);
+        }
+    }
+}
 
-    // shared memory: scratch (fragments / attention teams) | reduce [2][16][16][8] f32 | norm partials | phase table |
-    // barriers | ring
-    uint4 *fragments = reinterpret_cast<uint4 *>(smem_raw);
-    float *reduce = reinterpret_cast<float *>(smem_raw + a.scratch_bytes);
-    float *norm_partial = reduce + 2 * CONSUMER_WARPS * 128;
-    uint32_t *rope_rows = reinterpret_cast<uint32_t *>(norm_partial + 4 * CONSUMER_WARPS);  // [8 lanes][HD / 2] rotary factors of the lanes' positions
-    AttentionCache *attention_cache = reinterpret_cast<AttentionCache *>(rope_rows + 8 * (HD >> 1));
-    PhaseInfo *info = reinterpret_cast<PhaseInfo *>(attention_cache + 1);
-    uint64_t *barriers = reinterpret_cast<uint64_t *>(info + 4);
-    uint32_t *open_word = reinterpret_cast<uint32_t *>(barriers + 4 * MAX_STAGES);  // [0] grid barriers passed, [1] stages requested
-    uint8_t *ring_base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(open_word + 4) + 127) & ~static_cast<uintptr_t>(127));
-    RingAddresses ring;
-    ring.ring = static_cast<uint32_t>(__cvta_generic_to_shared(ring_base));
-    ring.full = static_cast<uint32_t>(__cvta_generic_to_shared(barriers));
-    ring.empty = ring.full + MAX_STAGES * 8;
-    ring.slices = static_cast<uint32_t>(__cvta_generic_to_shared(smem_raw));  // the slices share the scratch area with the fragments
-    ring.slice_full = ring.empty + MAX_STAGES * 8;
-    ring.slice_empty = ring.slice_full + MAX_STAGES * 8;
-    ring.open_word = static_cast<uint32_t>(__cvta_generic_to_shared(open_word));
-    ring.issued_word = ring.open_word + 4;
+constexpr int LAYER_WORDS = static_cast<int>(sizeof(StackLayer) / sizeof(uint32_t));
+static_assert(sizeof(StackLayer) % sizeof(uint32_t) == 0 && sizeof(StackArgs) % sizeof(uint32_t) == 0, "descriptions are copied word by word");
 
-    const int q_width = shape.q_heads * HD, kv_width = shape.kv_heads * HD;
-    const int q_tiles = q_width >> 4, k_tiles = kv_width >> 4;
-    if (threadIdx.x == 0) {
+// At the top of a layer: the next layer's description into the other copy (last read before the previous layer's final
+// barrier; stages of the next layer are requested behind this layer's first meeting at the earliest), and the K and V rows this CTA's teams will read in this layer's attention step on their way into L2.
+template <int HD>
+__device__ __forceinline__ void begin_layer(int layer) {
+    StackShared &sh = shared();
+    const int thread = thread_now();
+    if (thread >= 32 && thread < 32 + LAYER_WORDS && layer + 1 < sh.a.layer_count)
+        reinterpret_cast<uint32_t *>(&sh.layer[(layer + 1) & 1])[thread - 32] = reinterpret_cast<const uint32_t *>(sh.a.layers + layer + 1)[thread - 32];
+    const KvLayer &kv = sh.layer[layer & 1].kv;
+    const int team = thread >> 7, team_thread = thread & 127;
+    if (team_thread < sh.item[team].count) {
+        const size_t half_page = static_cast<size_t>(kv.kv_heads) * kv.page_tokens * HD;
+        const uint16_t *row = kv.pool + static_cast<size_t>(sh.row_base[team][team_thread]) * HD + static_cast<size_t>(sh.item[team].kv_head) * kv.page_tokens * HD;
+#pragma unroll
+        for (int line = 0; line < (HD * 2 + 127) / 128; line++) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t *>(row) + line * 128));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t *>(row + half_page) + line * 128));
+        }
+    }
+}
+
+// What the consumers look up once per launch: the lanes' positions, pages and rotary factors, the KV rows of each team's
+// first attention item.
+template <int HD, int GROUP>
+__device__ __forceinline__ void prepare_launch() {
+    constexpr int QL = AttentionTeam<GROUP>::QL;
+    StackShared &sh = shared();
+    const int thread = threadIdx.x, lanes = sh.a.lanes;
+    if (thread < 4 * CONSUMER_WARPS) sh.blocks[thread >> 4][thread & 15] = warp_blocks(thread >> 4, 0, thread & 15);
+    if (thread < 8) {
+        const uint32_t tick = thread < lanes ? sh.a.lanes_meta.position[thread] : 0u;
+        const int slot = thread < lanes ? sh.a.lanes_meta.slot[thread] : -1;
+        sh.tick[thread] = tick;
+        sh.slot[thread] = slot;
+        const KvLayer &kv = sh.layer[0].kv;
+        uint64_t row = ~0ull;
+        if (slot >= 0 && kv.capacity != 0) {
+            const uint32_t ring_token = tick % kv.capacity;
+            const int physical = kv.block_table[static_cast<size_t>(slot) * kv.pages_per_slot + ring_token / kv.page_tokens];
+            row = static_cast<uint64_t>(physical) * 2 * kv.kv_heads * kv.page_tokens * HD + static_cast<uint64_t>(ring_token % kv.page_tokens) * HD;
+        }
+        sh.kv_row[thread] = row;
+    }
+    for (int index = thread; index < lanes * (HD >> 1); index += CONSUMER_THREADS) {
+        const int m = index / (HD >> 1);
+        sh.rope[index] = __ldg(sh.a.shape.rope_table + static_cast<size_t>(sh.a.lanes_meta.position[m] % sh.a.shape.rope_positions) * (HD >> 1) + (index - m * (HD >> 1)));
+    }
+    cta_sync();
+    const int per_stream = sh.a.lanes_per_stream, groups_per_stream = (per_stream + QL - 1) / QL, group_slots = lanes / per_stream * groups_per_stream;
+    const int total = sh.a.shape.kv_heads * sh.a.max_splits * group_slots;
+    const int team = thread >> 7, team_thread = thread & 127;
+    const int item = static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) * team;
+    if (thread == 0) {
+        sh.merge_count = 0;
+        sh.group_slots = group_slots;
+    }
+    cta_sync();
+    const KvLayer &kv = sh.layer[0].kv;
+    if (team_thread == 0) {
+        sh.item[team].count = 0;
+        if (item < total && kv.capacity != 0) sh.item[team] = attention_item<QL>(kv, item);
+    }
+    cta_sync();
+    if (team_thread < 64)
+        sh.row_base[team][team_thread] =
+            team_thread < sh.item[team].count ? static_cast<uint32_t>(attention_row_base<HD>(kv, sh.item[team].slot, sh.item[team].ring_base, team_thread) / HD) : 0u;
+    sh.output[thread] = static_cast<uint32_t>(((thread >> 1) & 7) * sh.a.shape.hidden + (static_cast<int>(blockIdx.x) + (thread >> 7) * static_cast<int>(gridDim.x)) * 16 +
+                                              ((thread >> 4) & 7) + 8 * (thread & 1));
+    cta_sync();
+}
+
+// The matrices' schedules and the rings' barriers.
+template <int TILES>
+__device__ __forceinline__ void prepare_rings(int q_width, int kv_width) {
+    StackShared &sh = shared();
+    const int thread = threadIdx.x, lanes = sh.a.lanes;
+    if (thread < 4) {
+        const StackShape &shape = sh.a.shape;
         const int grid = static_cast<int>(gridDim.x), cta = static_cast<int>(blockIdx.x);
-        const MatrixSchedule schedules[4] = {stack_schedule((q_width + 2 * kv_width) >> 4, shape.hidden >> 7, 1, grid),
-                                             stack_schedule(shape.hidden >> 4, q_width >> 7, 1, grid),
-                                             stack_schedule(shape.ffn >> 4, shape.hidden >> 7, 2, grid),
-                                             stack_schedule(shape.hidden >> 4, shape.ffn >> 7, 1, grid)};
-        for (int p = 0; p < 4; p++) {
-            const MatrixSchedule &s = schedules[p];
-            PhaseInfo pi;
-            pi.tiles_here = stack_cta_tiles(s, cta);
-            pi.passes = (pi.tiles_here + s.slots - 1) / s.slots;
-            pi.slots = s.slots;
-            pi.width = s.width;
-            pi.steps = s.steps;
-            pi.units = s.units;
-            pi.rt = s.rt;
-            pi.groups = s.units / s.rt;
-            pi.cta_offset = static_cast<uint32_t>(stack_cta_offset(s, cta));
-            pi.streamed = (p == 1 || p == 3) ? 1 : 0;
-            info[p] = pi;
-        }
-        for (int s = 0; s < a.stages; s++) {
-            mbarrier_init(ring.full + s * 8, 1);                 // the producer's arrival with the byte count
-            mbarrier_init(ring.empty + s * 8, CONSUMER_WARPS);  // one arrival per consumer warp
-        }
-        for (int s = 0; s < a.slice_slots; s++) {
-            mbarrier_init(ring.slice_full + s * 8, 1);
-            mbarrier_init(ring.slice_empty + s * 8, CONSUMER_WARPS);
-        }
-        open_word[0] = 0u;
-        open_word[1] = 0u;
+        const MatrixSchedule s = thread == 0   ? stack_schedule((q_width + 2 * kv_width) >> 4, shape.hidden >> 7, false, grid)
+                                 : thread == 1 ? stack_schedule(shape.hidden >> 4, q_width >> 7, false, grid)
+                                 : thread == 2 ? stack_schedule(shape.ffn >> 4, shape.hidden >> 7, true, grid)
+                                               : stack_schedule(shape.hidden >> 4, shape.ffn >> 7, false, grid);
+        PhaseInfo &pi = sh.info[thread];
+        pi.tiles_here = stack_cta_tiles(s, cta);
+        pi.passes = (pi.tiles_here + s.slots - 1) / s.slots;
+        pi.slots = s.slots;
+        pi.width = s.width;
+        pi.width_log2 = 31 - __clz(s.width);
+        pi.steps = s.steps;
+        pi.groups = s.groups;
+        pi.window = pi.steps;
+        if (thread != 3 && static_cast<uint32_t>(pi.groups) * operand_group_bytes(lanes) > sh.a.scratch_bytes)
+            pi.window = static_cast<int>((sh.a.scratch_bytes) / operand_group_bytes(lanes)) / pi.width;
+        pi.cta_offset = static_cast<uint32_t>(stack_cta_offset(s, cta));
+    }
+    if (thread < MAX_STAGES) {
+        mbarrier_init(shared_address(&sh.full[thread]), 1);               // the producer's arrival with the byte count
+        mbarrier_init(shared_address(&sh.empty[thread]), CONSUMER_WARPS);  // one arrival per consumer warp
+        mbarrier_init(shared_address(&sh.slice_full[thread]), 1);
+        mbarrier_init(shared_address(&sh.slice_empty[thread]), CONSUMER_WARPS);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async;" ::: "memory");
     }
+    if (thread >= 32 && thread < 64) {
+        // columns without a lane repeat lane 0's, their results are dropped
+        const int g = (thread & 31) >> 2, j = thread & 3;
+        const int m = TILES == 1 ? g >> 2 : (TILES == 2 ? g >> 1 : g), term = TILES == 1 ? ((g & 3) < 2 ? g & 3 : 2) : (TILES == 2 ? g & 1 : 0);
+        const uint32_t row = static_cast<uint32_t>(m < lanes ? m : 0) * 192u + static_cast<uint32_t>(j) * 16u;
+        OperandPlace place;
+        place.half = operand_half_bytes(lanes);
+        place.first = row + static_cast<uint32_t>(term) * 64u;
+        place.second = row + 128u;
+        place.factor = 2 * place.half + (TILES == 1 ? static_cast<uint32_t>(j >> 1) * 4u : (TILES == 2 ? static_cast<uint32_t>(j) * 4u : static_cast<uint32_t>(j) * 8u));
+        sh.operand_place[thread & 31] = place;
+    }
+    if (thread == 64) {
+        sh.scratch = (static_cast<uint32_t>(sizeof(StackShared)) + 127u) & ~127u;
+        sh.ring = sh.scratch + sh.a.scratch_bytes;
+        const uint32_t staged = static_cast<uint32_t>(sh.a.shape.hidden >> 7) * operand_group_bytes(lanes);
+        sh.products = staged + PRODUCT_BYTES <= sh.a.scratch_bytes ? sh.scratch + staged : sh.scratch;
+        sh.place = 0u;
+        sh.barrier_target = sh.a.buffers.barrier_handicap;
+        sh.barrier_limit = sh.a.buffers.barrier_handicap != 0 ? (1u << 12) : BARRIER_SPIN_LIMIT;
+        sh.open_word = 0u;
+        sh.exchanges = sh.a.tp != nullptr ? static_cast<uint32_t>(sh.a.tp->counter[sh.a.tp->rank][STACK_TP_WORD_CONSUMED]) : 0u;
+    }
     __syncthreads();
+}
 
-    if (warp >= CONSUMER_WARPS) {
-        if (lane == 0) {
-            if (warp == CONSUMER_WARPS) produce_weights(a, info, ring);
-            else if (warp == CONSUMER_WARPS + 1) produce_activations(a, info, ring, staged);
-            else if (warp == CONSUMER_WARPS + 2 && a.prefetch_stages > 0) produce_prefetches(a, info, ring);
-        }
+// TILES: MMA columns in eights (stack_tiles).
+template <int HD, int GROUP, bool EXCHANGE, int TILES>
+__global__ void __launch_bounds__(STACK_THREADS, 1) decode_stack_kernel(const __grid_constant__ StackArgs args) {
+    StackShared &sh = shared();
+    for (int word = threadIdx.x; word < static_cast<int>(sizeof(StackArgs) / sizeof(uint32_t)); word += STACK_THREADS)
+        reinterpret_cast<uint32_t *>(&sh.a)[word] = reinterpret_cast<const uint32_t *>(&args)[word];
+    if (threadIdx.x >= 256 && threadIdx.x < 256 + LAYER_WORDS)
+        reinterpret_cast<uint32_t *>(&sh.layer[0])[threadIdx.x - 256] = reinterpret_cast<const uint32_t *>(args.layers)[threadIdx.x - 256];
+    if (args.layer_count > 1 && threadIdx.x >= 384 && threadIdx.x < 384 + LAYER_WORDS)
+        reinterpret_cast<uint32_t *>(&sh.layer[1])[threadIdx.x - 384] = reinterpret_cast<const uint32_t *>(args.layers + 1)[threadIdx.x - 384];
+    if (args.buffers.timing != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
+        unsigned long long now;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        args.buffers.timing[16] = now;
+    }
+    __syncthreads();
+    prepare_rings<TILES>(sh.a.shape.q_heads * HD, sh.a.shape.kv_heads * HD);
+    if (threadIdx.x >= CONSUMER_THREADS) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PRODUCER_REGISTERS));
+        if (threadIdx.x == CONSUMER_THREADS) produce_weights();
+        else if (threadIdx.x == CONSUMER_THREADS + 32) produce_activations();
         return;
     }
-
-    // ------------------------------------------------------------------ consumers
-    unsigned int target = a.buffers.barrier_handicap, barriers_passed = 0;
-    const unsigned int barrier_spin_limit = a.buffers.barrier_handicap != 0 ? (1u << 12) : BARRIER_SPIN_LIMIT;
-    unsigned int *counter = a.buffers.barrier;
-    int *error_flag = a.buffers.error_flag;
-    uint32_t tag = 0;  // exchanges done so far, earlier launches included
-    unsigned long long *inbox_mine = nullptr;
-    if constexpr (EXCHANGE) {
-        tag = static_cast<uint32_t>(a.tp->counter[a.tp->rank][STACK_TP_WORD_CONSUMED]);
-        inbox_mine = reinterpret_cast<unsigned long long *>(a.tp->exchange[a.tp->rank]);
-    }
-    uint32_t ring_slot = 0, ring_parity = 0, slice_slot = 0, slice_parity = 0;
-    int reduce_parity = 0;
-    PassRing pass_ring;
-    pass_ring.ring = ring.ring;
-    pass_ring.full = ring.full;
-    pass_ring.empty = ring.empty;
-    pass_ring.stages = static_cast<uint32_t>(a.stages);
-    pass_ring.stage_bytes = static_cast<uint32_t>(a.stage_bytes);
-    pass_ring.slices = ring.slices;
-    pass_ring.slice_full = ring.slice_full;
-    pass_ring.slice_empty = ring.slice_empty;
-    pass_ring.slice_slots = static_cast<uint32_t>(a.slice_slots);
-    pass_ring.slice_bytes = static_cast<uint32_t>(a.slice_bytes);
-
-    auto stamp = [&](int layer, int index) {
-        if (a.buffers.timing != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
-            unsigned long long now;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-            a.buffers.timing[layer * 32 + index] = now;
-        }
-    };
-    auto meet = [&]() {
-        grid_barrier(counter, target, error_flag, barrier_spin_limit);
-        barriers_passed++;
-        if (threadIdx.x == 0) shared_store_release(ring.open_word, barriers_passed);
-    };
-
-    // Epilogue roles: thread t finishes output (high = t & 1, lane m = (t >> 1) & 7, row = ((t >> 4) & 7) + 8 * high)
-    // of tile slot (t >> 7) + 4 * round, so the rotary partner rows r and r + 8 of a lane sit in neighbouring threads.
-    const int epilogue_m = (threadIdx.x >> 1) & 7, epilogue_row = ((threadIdx.x >> 4) & 7) + 8 * (threadIdx.x & 1);
-    const int epilogue_slot = threadIdx.x >> 7;
-    const bool epilogue_lane = epilogue_m < lanes;
-    // per-lane constants of the epilogue: position, rotary table row, and the lane's KV row inside a page (the
-    // block table is shared by all layers)
-    uint32_t lane_position = 0;
-    size_t kv_token_base = 0;
-    bool kv_writable = false;
-    if (epilogue_lane) {
-        lane_position = a.lanes_meta.position[epilogue_m];
-        const KvLayer &kv0 = a.layers[0].kv;
-        const int slot = a.lanes_meta.slot[epilogue_m];
-        if (slot >= 0 && kv0.capacity != 0) {
-            const uint32_t ring_token = lane_position % kv0.capacity;
-            const int physical = kv0.block_table[static_cast<size_t>(slot) * kv0.pages_per_slot + ring_token / kv0.page_tokens];
-            kv_token_base = static_cast<size_t>(physical) * 2 * kv0.kv_heads * kv0.page_tokens * HD + static_cast<size_t>(ring_token % kv0.page_tokens) * HD;
-            kv_writable = true;
-        }
-    }
-    for (int index = threadIdx.x; index < staged * (HD >> 1); index += CONSUMER_THREADS) {
-        const int m = index / (HD >> 1);
-        rope_rows[index] = __ldg(shape.rope_table + static_cast<size_t>(a.lanes_meta.position[m] % shape.rope_positions) * (HD >> 1) + (index - m * (HD >> 1)));
-    }
-    constexpr int LAYER_WORDS = static_cast<int>(sizeof(StackLayer) / sizeof(uint32_t));
-    static_assert(sizeof(StackLayer) % sizeof(uint32_t) == 0, "layer descriptions are copied word by word");
-    if (threadIdx.x >= 32 && threadIdx.x < 32 + LAYER_WORDS)
-        reinterpret_cast<uint32_t *>(&attention_cache->layer[0])[threadIdx.x - 32] = reinterpret_cast<const uint32_t *>(a.layers)[threadIdx.x - 32];
-    if (threadIdx.x < 8) {
-        attention_cache->tick[threadIdx.x] = static_cast<int>(threadIdx.x) < lanes ? a.lanes_meta.position[threadIdx.x] : 0u;
-        attention_cache->slot[threadIdx.x] = static_cast<int>(threadIdx.x) < lanes ? a.lanes_meta.slot[threadIdx.x] : -1;
-    }
-    consumer_sync();
-    {
-        // the KV rows of each team's first attention item, looked up once for all layers
-        const int streams = lanes / a.lanes_per_stream;
-        const int groups_per_stream = (a.lanes_per_stream + QL - 1) / QL;
-        const int group_slots = streams * groups_per_stream;
-        const int total = shape.kv_heads * a.max_splits * group_slots;
-        const int team = warp >> 2, team_thread = threadIdx.x & 127;
-        const int item = static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) * team;
-        int cached_item = -1, cached_rows = 0;
-        if (item < total) {
-            const int rest = item / shape.kv_heads, split = rest % a.max_splits, group_slot = rest / a.max_splits;
-            const int lane0 = (group_slot / groups_per_stream) * a.lanes_per_stream + (group_slot % groups_per_stream) * QL;
-            const KvLayer &kv0 = a.layers[0].kv;
-            const int slot = lane0 < lanes ? attention_cache->slot[lane0] : -1;
-            if (slot >= 0 && kv0.capacity != 0) {
-                uint32_t newest = 0;
-                for (int i = 0; i < QL; i++)
-                    if (lane0 + i < lanes && (group_slot % groups_per_stream) * QL + i < a.lanes_per_stream && attention_cache->tick[lane0 + i] > newest)
-                        newest = attention_cache->tick[lane0 + i];
-                const uint32_t tokens = newest + 1u < kv0.capacity ? newest + 1u : kv0.capacity;
-                const uint32_t begin = static_cast<uint32_t>(split) * 64u;
-                if (begin < tokens) {
-                    const uint32_t ring_base = (newest + 1u - tokens + begin) % kv0.capacity;
-                    if (team_thread < 64 && begin + team_thread < tokens)
-                        attention_cache->row_base[team][team_thread] = static_cast<uint32_t>(attention_row_base<HD>(kv0, slot, ring_base, team_thread) / HD);
-                    cached_item = item;
-                    cached_rows = static_cast<int>(tokens - begin < 64u ? tokens - begin : 64u);
-                }
-            }
-        }
-        if (threadIdx.x == 0) {
-            attention_cache->merge_count = 0;
-            AttentionJob job;
-            job.q = a.buffers.q;
-            job.scratch = a.buffers.attention_scratch;
-            job.out_fragments = a.buffers.attention_out;
-            job.arrivals = a.buffers.barrier + ARRIVAL_WORDS_OFFSET;
-            job.lanes = lanes;
-            job.lanes_per_stream = a.lanes_per_stream;
-            job.q_heads = shape.q_heads;
-            job.kv_heads = shape.kv_heads;
-            job.max_splits = a.max_splits;
-            job.group_slots = group_slots;
-            job.staged = staged;
-            job.scale = shape.attention_scale;
-            attention_cache->job = job;
-        }
-        if (team_thread == 0) {
-            attention_cache->item[team] = cached_item;
-            attention_cache->rows[team] = cached_rows;
-        }
-    }
-    consumer_sync();
-    // gate/up in pairs (consume_pass_pairs): when a stage is two steps of (gate, up) blocks per tile slot and the scratch
-    // has room for the up rows' partial sums behind the normalised rows
-    const size_t pair_reduce_offset = static_cast<size_t>(staged) * shape.hidden * 2;
-    // (two copies, alternating like the main array, when the step takes several passes)
-    const int pair_copies = info[2].passes > 1 ? 2 : 1;
-    const bool pairs_enabled = info[2].rt == 2 && info[2].width == 2 && a.steps_per_stage == 2 && !(a.debug_flags & 1) &&
-                               pair_reduce_offset + pair_copies * CONSUMER_WARPS * 128 * sizeof(float) <= a.scratch_bytes;
-    float *reduce_second = reinterpret_cast<float *>(smem_raw + pair_reduce_offset);
-    const int ge = g < staged ? g : 0;  // lanes beyond the batch recompute lane 0; their results are dropped
-    const uint32_t fragment_lane = static_cast<uint32_t>(__cvta_generic_to_shared(fragments)) + static_cast<uint32_t>(ge * 4 + j) * 16u;
-    const uint32_t word_stride = static_cast<uint32_t>(staged) * 4 * sizeof(uint4);  // between the four words of a group
-    const uint32_t group_stride = 4 * word_stride;
-    const int grid = static_cast<int>(gridDim.x);
-
-    for (int layer = 0; layer < a.layer_count; layer++) {
-        const StackLayer *spec = &attention_cache->layer[layer & 1];
-        const KvLayer kv = spec->kv;
-        // the next layer's description: into the other copy (last read before the previous layer's final barrier)
-        if (threadIdx.x >= 32 && threadIdx.x < 32 + LAYER_WORDS && layer + 1 < a.layer_count)
-            reinterpret_cast<uint32_t *>(&attention_cache->layer[(layer + 1) & 1])[threadIdx.x - 32] =
-                reinterpret_cast<const uint32_t *>(a.layers + layer + 1)[threadIdx.x - 32];
-        {
-            // the K and V rows this CTA's teams will read in this layer's attention step: on their way into L2 now
-            const int team = warp >> 2, team_thread = threadIdx.x & 127;
-            const int item = attention_cache->item[team];
-            if (item >= 0 && team_thread < attention_cache->rows[team] && kv.capacity != 0) {
-                const int kv_head = item % shape.kv_heads;
-                const size_t half_page = static_cast<size_t>(kv.kv_heads) * kv.page_tokens * HD;
-                const uint16_t *row = kv.pool + static_cast<size_t>(attention_cache->row_base[team][team_thread]) * HD + static_cast<size_t>(kv_head) * kv.page_tokens * HD;
-#pragma unroll
-                for (int line = 0; line < (HD * 2 + 127) / 128; line++) {
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t *>(row) + line * 128));
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t *>(row + half_page) + line * 128));
-                }
-            }
-        }
-        for (int phase = 0; phase < 4; phase++) {
-            const PhaseInfo pi = info[phase];
-            stamp(layer, 4 * phase);
-            // ---- activations of q/k/v and gate/up: normalised rows into fragment order
-            if (phase == 0 || phase == 2) {
-                const uint16_t *norm_weight = phase == 0 ? spec->input_norm : spec->post_norm;
-                if (shape.hidden <= 8 * CONSUMER_THREADS)
-                    stage_normalised<1>(fragments, norm_partial, a.buffers.hidden, norm_weight, shape.hidden, staged, shape.eps, shape.norm_offset);
-                else
-                    stage_normalised<2>(fragments, norm_partial, a.buffers.hidden, norm_weight, shape.hidden, staged, shape.eps, shape.norm_offset);
-            }
-            stamp(layer, 4 * phase + 1);
-
-            const int slot_of_warp = warp / pi.width, index_in_slot = warp - slot_of_warp * pi.width;
-            for (int pass = 0; pass < pi.passes; pass++) {
-                const int present = stage_present(pi, pass);
-                const bool active = warp < present * pi.width;
-                // the epilogue's residual values are requested before the arithmetic: rounds of four tile slots
-                const uint16_t *payload_address = a.buffers.hidden;
-                int payload_rounds = 0;
-                if (epilogue_lane && (phase == 1 || phase == 3) && epilogue_slot < present) {
-                    payload_address = a.buffers.hidden + static_cast<size_t>(epilogue_m) * shape.hidden +
-                                      (static_cast<size_t>(blockIdx.x) + static_cast<size_t>(pass * pi.slots + epilogue_slot) * grid) * 16 + epilogue_row;
-                    payload_rounds = (present - epilogue_slot + 3) / 4;
-                }
-                // this warp's units of the pass: index_in_slot, + width, ... while below `units`
-                int active_steps = 0;
-                if (active && index_in_slot < pi.units && !(a.debug_flags & 1)) active_steps = (pi.units - index_in_slot + pi.width - 1) / pi.width;
-                const uint32_t lane_fragment = static_cast<uint32_t>(ge * 4 + j) * 16u;
-                // B fragments: of the group the warp's first unit belongs to - in the slice of the stage (o, down), or in
-                // the normalised rows, moving on by width / rt groups per step
-                const uint32_t x_step = static_cast<uint32_t>(pi.width / pi.rt) * group_stride;
-                const uint32_t x_start = pi.streamed ? static_cast<uint32_t>(index_in_slot) * group_stride + lane_fragment
-                                                     : fragment_lane + static_cast<uint32_t>(index_in_slot / pi.rt) * group_stride;
-                const bool pair_mode = phase == 2 && pairs_enabled;
-                PassResult done;
-                float second_acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                if (pair_mode) {
-                    const PairResult pairs = consume_pass_pairs(pass_ring, ring_slot, ring_parity, pi.steps, active, index_in_slot,
-                                                                static_cast<uint32_t>(present * pi.width * UNIT_TOTAL),
-                                                                static_cast<uint32_t>(slot_of_warp * 2) * UNIT_BYTES + static_cast<uint32_t>(lane) * 16u,
-                                                                static_cast<uint32_t>(present * pi.width) * UNIT_BYTES +
-                                                                    static_cast<uint32_t>(slot_of_warp * 2) * UNIT_SCALE_BYTES + static_cast<uint32_t>(g) * 4u,
-                                                                fragment_lane + static_cast<uint32_t>(index_in_slot) * group_stride, 2 * group_stride, word_stride,
-                                                                error_flag);
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        done.acc[i] = pairs.acc[i];
-                        second_acc[i] = pairs.second[i];
-                        done.payload[i] = 0;
-                    }
-                    done.slot = pairs.slot;
-                    done.parity = pairs.parity;
-                    done.slice_slot = slice_slot;
-                    done.slice_parity = slice_parity;
-                } else {
-                    const uint32_t step_bytes = static_cast<uint32_t>(present * pi.width * UNIT_TOTAL);
-                    const uint32_t weight_offset = static_cast<uint32_t>(warp) * UNIT_BYTES + static_cast<uint32_t>(lane) * 16u;
-                    const uint32_t scale_offset = static_cast<uint32_t>(present * pi.width) * UNIT_BYTES + static_cast<uint32_t>(warp) * UNIT_SCALE_BYTES +
-                                                  static_cast<uint32_t>(g) * 4u;
-                    const uint32_t payload_stride = static_cast<uint32_t>(4 * grid * 16);
-                    if (a.steps_per_stage == 2) {
-                        done = pi.streamed ? consume_pass<true, 2>(pass_ring, ring_slot, ring_parity, slice_slot, slice_parity, pi.steps, active_steps, step_bytes,
-                                                                   weight_offset, scale_offset, x_start, x_step, word_stride, error_flag, payload_address,
-                                                                   payload_stride, payload_rounds)
-                                           : consume_pass<false, 2>(pass_ring, ring_slot, ring_parity, slice_slot, slice_parity, pi.steps, active_steps, step_bytes,
-                                                                    weight_offset, scale_offset, x_start, x_step, word_stride, error_flag, payload_address,
-                                                                    payload_stride, payload_rounds);
-                    } else {
-                        done = pi.streamed ? consume_pass<true, 1>(pass_ring, ring_slot, ring_parity, slice_slot, slice_parity, pi.steps, active_steps, step_bytes,
-                                                                   weight_offset, scale_offset, x_start, x_step, word_stride, error_flag, payload_address,
-                                                                   payload_stride, payload_rounds)
-                                           : consume_pass<false, 1>(pass_ring, ring_slot, ring_parity, slice_slot, slice_parity, pi.steps, active_steps, step_bytes,
-                                                                    weight_offset, scale_offset, x_start, x_step, word_stride, error_flag, payload_address,
-                                                                    payload_stride, payload_rounds);
-                    }
-                }
-                ring_slot = done.slot;
-                ring_parity = done.parity;
-                slice_slot = done.slice_slot;
-                slice_parity = done.slice_parity;
-                stamp(layer, 26 + phase);
-                const float (&acc)[4] = done.acc;
-                // ---- the warps' partial sums meet: reduce[parity][warp][row][lane]
-                float *mine = reduce + static_cast<size_t>((reduce_parity * CONSUMER_WARPS + warp) * 128);
-                *reinterpret_cast<float2 *>(mine + g * 8 + 2 * j) = make_float2(acc[0], acc[1]);
-                *reinterpret_cast<float2 *>(mine + (g + 8) * 8 + 2 * j) = make_float2(acc[2], acc[3]);
-                if (pair_mode) {
-                    float *up = reduce_second + static_cast<size_t>(((pair_copies == 2 ? reduce_parity : 0) * CONSUMER_WARPS + warp) * 128);
-                    *reinterpret_cast<float2 *>(up + g * 8 + 2 * j) = make_float2(second_acc[0], second_acc[1]);
-                    *reinterpret_cast<float2 *>(up + (g + 8) * 8 + 2 * j) = make_float2(second_acc[2], second_acc[3]);
-                }
-                consumer_sync();
-                const float *sums = reduce + static_cast<size_t>(reduce_parity * CONSUMER_WARPS * 128);
-                const float *second_sums = reduce_second + static_cast<size_t>((pair_copies == 2 ? reduce_parity : 0) * CONSUMER_WARPS * 128);
-                reduce_parity ^= 1;
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(CONSUMER_REGISTERS));
+    prepare_launch<HD, GROUP>();
 #pragma unroll 1
-                for (int round = 0; round < 4; round++) {
-                    const int slot = epilogue_slot + 4 * round;
-                    if (slot >= present) break;  // uniform over the warp
-                    const int tile = static_cast<int>(blockIdx.x) + (pass * pi.slots + slot) * grid;
-                    const float *src = sums + static_cast<size_t>(slot * pi.width) * 128 + epilogue_row * 8 + epilogue_m;
-                    float first = 0.0f, second = 0.0f;
-                    if (pair_mode) {
-                        // both warps of the slot hold gate sums (here) and up sums (in the second array), of alternate groups
-                        const float *up = second_sums + static_cast<size_t>(slot * pi.width) * 128 + epilogue_row * 8 + epilogue_m;
-                        first = src[0] + src[128];
-                        second = up[0] + up[128];
-                    } else if (pi.rt == 2) {
-                        for (int w = 0; w < pi.width; w += 2) {
-                            first += src[w * 128];
-                            second += src[(w + 1) * 128];
-                        }
-                    } else {
-                        for (int w = 0; w < pi.width; w++) first += src[w * 128];
-                    }
-                    if (phase == 0) {
-                        // q / k: rotary_bf16.comp.template:99-109 (non-interleaved, rotary width = head width, five bf16
-                        // roundings); k and v go into the lane's KV page (append_gqa_attention_bf16.comp.template:189-215)
-                        const float mine_value = round_bf16(first);
-                        const float partner = __shfl_xor_sync(0xffffffffu, mine_value, 1);  // the row 8 further (or 8 back)
-                        if (epilogue_lane) {
-                            const size_t kv_half = static_cast<size_t>(kv.kv_heads) * kv.page_tokens * HD;
-                            if (tile < q_tiles + k_tiles) {
-                                const bool is_q = tile < q_tiles, high = epilogue_row >= 8;
-                                const int local = is_q ? tile : tile - q_tiles;
-                                const int head = local / (HD >> 4), d = 8 * (local % (HD >> 4)) + (epilogue_row & 7) + (high ? HD / 2 : 0);
-                                const uint32_t rotation = rope_rows[epilogue_m * (HD >> 1) + 8 * (local % (HD >> 4)) + (epilogue_row & 7)];
-                                const float cosine = bf16_lo(rotation), sine = bf16_hi(rotation);
-                                // d < half: x cos + (-x[d + half]) sin;  d >= half: x cos + x[d - half] sin
-                                const float other = high ? partner : -partner;
-                                const uint16_t value = static_cast<uint16_t>(f32_to_bf16_bits(round_bf16(mine_value * cosine) + round_bf16(other * sine)));
-                                if (is_q) a.buffers.q[(static_cast<size_t>(epilogue_m) * shape.q_heads + head) * HD + d] = value;
-                                else if (kv_writable) kv.pool[kv_token_base + static_cast<size_t>(head) * kv.page_tokens * HD + d] = value;
-                            } else if (kv_writable) {
-                                const int index = (tile - q_tiles - k_tiles) * 16 + epilogue_row;
-                                kv.pool[kv_token_base + kv_half + static_cast<size_t>(index / HD) * kv.page_tokens * HD + index % HD] =
-                                    static_cast<uint16_t>(f32_to_bf16_bits(first));
-                            }
-                        }
-                    } else if (epilogue_lane) {
-                        const int column = tile * 16 + epilogue_row;
-                        if (phase == 2) {
-                            // silu_multiply_bf16.comp.template:30-52: bf16(silu_bf16(bf16 gate) * bf16 up), kept as fp16 in
-                            // fragment order for the down projection
-                            const float product = round_bf16(rounded_silu(round_bf16(first)) * round_bf16(second));
-                            a.buffers.activation[fragment_element(column, epilogue_m, staged)] = __half_as_ushort(__float2half_rn(product));
-                        } else {
-                            float total = first;
-                            if constexpr (EXCHANGE) {
-                                // this rank's share of the sum over K goes to every peer's inbox, value and exchange number in
-                                // one 8-byte store; the peers' shares arrive in this rank's inbox the same way
-                                const StackTp &tp = *a.tp;
-                                const uint32_t number = tag + 1u;
-                                const size_t element = (static_cast<size_t>(number & 1u) * STACK_TP_MAX_RANKS * 8 + epilogue_m) * shape.hidden + column;
-                                const unsigned long long word = (static_cast<unsigned long long>(number) << 32) | __float_as_uint(first);
-                                for (int r = 0; r < tp.size; r++)
-                                    if (r != tp.rank)
-                                        asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(reinterpret_cast<unsigned long long *>(tp.exchange[r]) + element +
-                                                                                              static_cast<size_t>(tp.rank) * 8 * shape.hidden),
-                                                     "l"(word)
-                                                     : "memory");
-                                total = 0.0f;
-                                unsigned int spins = 0;
-                                bool gave_up = false;
-                                for (int r = 0; r < tp.size; r++) {  // rank order on every rank: the replicas stay bit-identical
-                                    float part = first;
-                                    if (r != tp.rank) {
-                                        const unsigned long long *source = inbox_mine + element + static_cast<size_t>(r) * 8 * shape.hidden;
-                                        unsigned long long got = 0;
-                                        while (!gave_up) {
-                                            asm volatile("ld.relaxed.sys.global.u64 %0, [%1];" : "=l"(got) : "l"(source) : "memory");
-                                            if (static_cast<uint32_t>(got >> 32) == number) break;
-                                            if (++spins > STACK_TP_SPIN_LIMIT) {
-                                                atomicExch(error_flag, 2);
-                                                gave_up = true;
-                                            } else if ((spins & 255u) == 0 && *reinterpret_cast<volatile int *>(error_flag) != 0) {
-                                                gave_up = true;
-                                            }
-                                        }
-                                        part = __uint_as_float(static_cast<uint32_t>(got));
-                                    }
-                                    total += part;
-                                }
-                            }
-                            // linear + residual_add (add_bf16.comp.template:17-24): bf16(bf16(product) + residual), in place
-                            a.buffers.hidden[static_cast<size_t>(epilogue_m) * shape.hidden + column] =
-                                static_cast<uint16_t>(f32_to_bf16_bits(round_bf16(total) + bf16_bits_to_f32(round == 0 ? done.payload[0] : (round == 1 ? done.payload[1] : (round == 2 ? done.payload[2] : done.payload[3])))));
-                        }
-                    }
-                }
+    for (int layer = 0; layer < sh.a.layer_count; layer++) {
+        begin_layer<HD>(layer);
+#pragma unroll 1
+        for (int phase = 0; phase < 4; phase++) {
+            matrix_step<HD, EXCHANGE, TILES>(phase, layer);
+#pragma unroll 1
+            for (bool attended = phase != 0;; attended = true) {
+                if (phase < 3 || layer + 1 < sh.a.layer_count) grid_meet(true);
+                if (phase != 0 || !attended) stamp(layer, 4 * phase + 3);
+                if (attended) break;
+                attention_step<HD, GROUP>(layer);
             }
-            if constexpr (EXCHANGE) {
-                if (phase == 1 || phase == 3) tag += 1u;
-            }
-            stamp(layer, 4 * phase + 2);
-            if (layer + 1 < a.layer_count || phase < 3) meet();
-            stamp(layer, 4 * phase + 3);
-
             if (phase == 0) {
-                // ---- attention: (kv head, split, stream x lane group) items, one team of four warps each, spread
-                // over the SMs first; the teams' shared arrays reuse the fragment area (nothing is staged right now)
-                const int streams = lanes / a.lanes_per_stream;
-                const int group_slots = streams * ((a.lanes_per_stream + QL - 1) / QL);
-                const int total = shape.kv_heads * a.max_splits * group_slots;
-                const int team = warp >> 2;
-                unsigned long long *item_stamps = (a.buffers.timing != nullptr && blockIdx.x == 0 && threadIdx.x == 0) ? a.buffers.timing + layer * 32 : nullptr;
-                for (int item = blockIdx.x + gridDim.x * team; item < total; item += gridDim.x * 4)
-                    attention_team_item<HD, GROUP, QL>(*attention_cache, spec->kv, item, smem_raw, item_stamps);
-                consumer_sync();
-                stamp(layer, 17);
-                {
-                    // merge the heads whose last split was completed here: one (lane, q head) row per warp and round
-                    int requests = attention_cache->merge_count;
-                    if (requests > ATTENTION_MERGE_LIST) requests = ATTENTION_MERGE_LIST;
-                    if (requests > 0) {
-                        __threadfence();
-                        const int groups_per_stream = (a.lanes_per_stream + QL - 1) / QL;
-                        for (int index = warp; index < requests * QL * GROUP; index += CONSUMER_WARPS) {
-                            const int request = attention_cache->merge_list[index / (QL * GROUP)], row = index % (QL * GROUP);
-                            const int kv_head = request / group_slots, group_slot = request % group_slots;
-                            const int group_index = group_slot % groups_per_stream;
-                            const int query_lane = (group_slot / groups_per_stream) * a.lanes_per_stream + group_index * QL + row / GROUP;
-                            if (query_lane < lanes && group_index * QL + row / GROUP < a.lanes_per_stream && attention_cache->slot[query_lane] >= 0)
-                                attention_merge_row<HD>(attention_cache->job, attention_own_splits(attention_cache->job, kv.capacity, attention_cache->tick[query_lane]),
-                                                        query_lane, kv_head * GROUP + row % GROUP);
-                        }
-                    }
-                }
-                if (a.max_splits > MERGE_BLOCK) {
-                    // ---- groups of more than MERGE_BLOCK splits: every warp of the grid merges ranges of MERGE_BLOCK
-                    // splits into one partial each, then one warp per row merges the row's range partials.  The two
-                    // barriers in between are not counted for the producer of slices (it waits for the one below).
-                    const int ranges = attention_ranges(a.max_splits), rows = lanes * shape.q_heads;
-                    grid_barrier(counter, target, error_flag, barrier_spin_limit);
-                    for (int task = blockIdx.x + gridDim.x * warp; task < rows * ranges; task += gridDim.x * CONSUMER_WARPS) {
-                        const int row = task / ranges, range = task % ranges, query_lane = row / shape.q_heads;
-                        if (attention_cache->slot[query_lane] < 0) continue;
-                        const int splits = attention_group_splits(attention_cache->job, attention_cache->tick, kv.capacity, query_lane, QL);
-                        if (splits > MERGE_BLOCK && range * MERGE_BLOCK < splits)
-                            attention_merge_range<HD>(attention_cache->job, splits, query_lane, row % shape.q_heads, range);
-                    }
-                    grid_barrier(counter, target, error_flag, barrier_spin_limit);
-                    for (int row = blockIdx.x + gridDim.x * warp; row < rows; row += gridDim.x * CONSUMER_WARPS) {
-                        const int query_lane = row / shape.q_heads;
-                        if (attention_cache->slot[query_lane] < 0) continue;
-                        const int splits = attention_group_splits(attention_cache->job, attention_cache->tick, kv.capacity, query_lane, QL);
-                        if (splits > MERGE_BLOCK) attention_merge_ranges<HD>(attention_cache->job, splits, query_lane, row % shape.q_heads);
-                    }
-                }
-                meet();
-                if (threadIdx.x == 0) attention_cache->merge_count = 0;  // read again after the next layer's q/k/v barrier at the earliest
+                if (threadIdx.x == 0) sh.merge_count = 0;  // read again after the next layer's q/k/v barrier at the earliest
                 stamp(layer, 18);
             }
         }
     }
 
-    if (a.buffers.timing != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
+    if (args.buffers.timing != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
         unsigned long long now;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-        a.buffers.timing[30] = now;
+        args.buffers.timing[30] = now;
     }
     // The last CTA to leave rearms the barrier words for the next launch (every CTA has passed its last barrier
     // before it counts itself out).
     if (threadIdx.x == 0) {
+        unsigned int *counter = args.buffers.barrier;
         const unsigned int gone = atomicAdd(counter + 1, 1u);
         if (gone == gridDim.x - 1) {
             counter[0] = 0u;
             counter[1] = 0u;
-            if constexpr (EXCHANGE) a.tp->counter[a.tp->rank][STACK_TP_WORD_CONSUMED] = tag;  // the next launch counts on from here
+            // the next launch counts on from here
+            if constexpr (EXCHANGE) args.tp->counter[args.tp->rank][STACK_TP_WORD_CONSUMED] = sh.exchanges + static_cast<uint32_t>(2 * args.layer_count);
             __threadfence();
         }
     }
@@ -1839,44 +1795,41 @@ __global__ void __launch_bounds__(STACK_THREADS, 1) decode_stack_kernel(const St
 
 struct StackPlanSmem {
     size_t scratch, total;
-    int stages, stage_bytes, steps_per_stage, slice_slots, slice_bytes;
+    int stages, slice_slots, slice_bytes;
 };
 
 template <int HD>
 bool plan_smem_for(const StackShape &shape, int lanes, int grid, StackPlanSmem *plan) {
-    const int staged = lanes < 8 ? lanes : 8;
-    const int q_width = shape.q_heads * shape.head_width;
-    const MatrixSchedule o = stack_schedule(shape.hidden >> 4, q_width >> 7, 1, grid);
-    const MatrixSchedule down = stack_schedule(shape.hidden >> 4, shape.ffn >> 7, 1, grid);
-    const int slice_groups = o.width > down.width ? o.width : down.width;
-    // two steps per stage: fewer hand-overs, two blocks per warp and wait, and the gate/up step in pairs - for every
-    // lane count alike, so that the order of a lane's additions does not depend on how many lanes share its launch
-    const int steps_per_stage = 2;
-    const size_t slice = static_cast<size_t>(steps_per_stage) * slice_groups * staged * 256;
-    size_t scratch = static_cast<size_t>(staged) * shape.hidden * 2;  // fragments of a normalised row set
-    const size_t teams = 4 * attention_team_bytes<HD>();
-    if (teams > scratch) scratch = teams;
-    if (2 * slice > scratch) scratch = 2 * slice;
-    // the up rows' partial sums of the gate/up pairs sit behind the normalised rows (one copy at least)
-    const size_t pairs = static_cast<size_t>(staged) * shape.hidden * 2 + CONSUMER_WARPS * 128 * sizeof(float);
-    if (pairs > scratch) scratch = pairs;
+    const int q_width = shape.q_heads * shape.head_width, widest = q_width > shape.hidden ? q_width : shape.hidden;
+    const MatrixSchedule qkv = stack_schedule((q_width + 2 * shape.kv_heads * shape.head_width) >> 4, shape.hidden >> 7, false, grid);
+    const MatrixSchedule o = stack_schedule(shape.hidden >> 4, q_width >> 7, false, grid);
+    const MatrixSchedule down = stack_schedule(shape.hidden >> 4, shape.ffn >> 7, false, grid);
+    const size_t group = operand_group_bytes(lanes), limit = 227 * 1024;
+    const size_t stage = STAGE_BYTES;
+    const size_t fixed = (sizeof(StackShared) + 127) & ~static_cast<size_t>(127);
+    // what the scratch has to hold: the attention teams, two slices of down, a step's groups of the staged rows
+    const size_t slice = static_cast<size_t>(down.width < down.groups ? down.width : down.groups) * group;
+    size_t least = 4 * attention_team_bytes<HD>();
+    if (2 * slice > least) least = 2 * slice;
+    const size_t window = static_cast<size_t>(qkv.width > o.width ? qkv.width : o.width) * group;
+    if (window > least) least = window;
+    if (PRODUCT_BYTES > least) least = PRODUCT_BYTES;
+    // ... and whole rows, unless the ring would be left with less than two stages
+    size_t scratch = static_cast<size_t>(widest >> 7) * group;
+    if (shape.ffn >> 7 > grid) scratch += PRODUCT_BYTES;  // several passes of gate/up: the products beside the rows
+    if (scratch < least) scratch = least;
+    if (fixed + 128 + scratch + 2 * stage > limit) scratch = fixed + 128 + least + 2 * stage > limit ? least : limit - fixed - 128 - 2 * stage;
     scratch = (scratch + 127) & ~static_cast<size_t>(127);
+    if (fixed + scratch + 2 * stage > limit) return false;
     int slice_slots = static_cast<int>(scratch / slice);
     if (slice_slots > MAX_STAGES) slice_slots = MAX_STAGES;
-    const size_t fixed = scratch + 2 * CONSUMER_WARPS * 128 * sizeof(float) + 4 * CONSUMER_WARPS * sizeof(float) + 8 * (HD / 2) * sizeof(uint32_t) +
-                         sizeof(AttentionCache) + 4 * sizeof(PhaseInfo) + 4 * MAX_STAGES * sizeof(uint64_t) + 4 * sizeof(uint32_t) + 128;
-    const size_t stage = (static_cast<size_t>(steps_per_stage) * STAGE_WEIGHT_BYTES + 127) & ~static_cast<size_t>(127);
-    const size_t limit = 227 * 1024;
-    if (fixed + 2 * stage > limit) return false;
-    int stages = static_cast<int>((limit - fixed) / stage);
+    int stages = static_cast<int>((limit - fixed - scratch) / stage);
     if (stages > MAX_STAGES) stages = MAX_STAGES;
     plan->scratch = scratch;
     plan->stages = stages;
-    plan->stage_bytes = static_cast<int>(stage);
-    plan->steps_per_stage = steps_per_stage;
     plan->slice_slots = slice_slots;
     plan->slice_bytes = static_cast<int>(slice);
-    plan->total = fixed + static_cast<size_t>(stages) * stage;
+    plan->total = fixed + scratch + static_cast<size_t>(stages) * stage;
     return true;
 }
 
@@ -1888,11 +1841,17 @@ bool plan_smem(const StackShape &shape, int lanes, int grid, StackPlanSmem *plan
     return false;
 }
 
-template <int HD, int GROUP, bool EXCHANGE>
+template <int HD, int GROUP, bool EXCHANGE, int TILES>
 cudaError_t launch_instance_of(const StackArgs &args, size_t smem, int grid, cudaStream_t stream) {
     // the attribute is per device and per kernel instance: set it on every launch (a cheap host-side call)
-    cudaError_t status = cudaFuncSetAttribute(decode_stack_kernel<HD, GROUP, EXCHANGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaError_t status = cudaFuncSetAttribute(decode_stack_kernel<HD, GROUP, EXCHANGE, TILES>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (status != cudaSuccess) return status;
+    // the consumers would wait forever for registers that the launch did not bring
+    cudaFuncAttributes attributes;
+    status = cudaFuncGetAttributes(&attributes, decode_stack_kernel<HD, GROUP, EXCHANGE, TILES>);
+    if (status != cudaSuccess) return status;
+    if (attributes.numRegs * STACK_THREADS < CONSUMER_THREADS * CONSUMER_REGISTERS + (STACK_THREADS - CONSUMER_THREADS) * PRODUCER_REGISTERS)
+        return cudaErrorInvalidDeviceFunction;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(grid);
     config.blockDim = dim3(STACK_THREADS);
@@ -1903,9 +1862,20 @@ cudaError_t launch_instance_of(const StackArgs &args, size_t smem, int grid, cud
     attribute[0].val.cooperative = 1;
     config.attrs = attribute;
     config.numAttrs = 1;
-    return cudaLaunchKernelEx(&config, decode_stack_kernel<HD, GROUP, EXCHANGE>, args);
+    return cudaLaunchKernelEx(&config, decode_stack_kernel<HD, GROUP, EXCHANGE, TILES>, args);
 }
 
+// MMA columns of a batch in eights: three terms per lane, none of them split over two threads' columns from three lanes on.
+constexpr int stack_tiles(int lanes) { return lanes <= 2 ? 1 : (lanes <= 4 ? 2 : 3); }
+
+template <int HD, int GROUP, bool EXCHANGE>
+cudaError_t launch_instance_of(const StackArgs &args, size_t smem, int grid, cudaStream_t stream) {
+    switch (stack_tiles(args.lanes)) {
+        case 1: return launch_instance_of<HD, GROUP, EXCHANGE, 1>(args, smem, grid, stream);
+        case 2: return launch_instance_of<HD, GROUP, EXCHANGE, 2>(args, smem, grid, stream);
+        default: return launch_instance_of<HD, GROUP, EXCHANGE, 3>(args, smem, grid, stream);
+    }
+}
 template <int HD, int GROUP>
 cudaError_t launch_instance(const StackArgs &args, size_t smem, int grid, cudaStream_t stream) {
     return args.tp_size > 1 ? launch_instance_of<HD, GROUP, true>(args, smem, grid, stream) : launch_instance_of<HD, GROUP, false>(args, smem, grid, stream);
@@ -1913,8 +1883,10 @@ cudaError_t launch_instance(const StackArgs &args, size_t smem, int grid, cudaSt
 
 }  // namespace
 
+size_t stack_activation_bytes(int ffn) { return static_cast<size_t>(ffn >> 7) * operand_group_bytes(8); }
+
 size_t int4_cta_stream_bytes(int rows, int k, bool pair, int grid) {
-    return stack_stream_bytes(stack_schedule(rows / 16, k / 128, pair ? 2 : 1, grid));
+    return stack_stream_bytes(stack_schedule(rows / 16, k / 128, pair, grid));
 }
 
 cudaError_t launch_int4_cta_streams(const RelayoutSegment *segments, int count, bool pair, int k, int grid, uint8_t *out, cudaStream_t stream) {
@@ -1932,10 +1904,10 @@ cudaError_t launch_int4_cta_streams(const RelayoutSegment *segments, int count, 
         args.first_tile[i] = tiles;
         if (!pair || i == 0) tiles += segments[i].rows / 16;
     }
-    if (pair && segments[0].rows != segments[1].rows) return cudaErrorInvalidValue;
+    if (pair && (segments[0].rows != segments[1].rows || segments[0].rows % 128 != 0)) return cudaErrorInvalidValue;
     args.first_tile[count] = tiles;
-    args.schedule = stack_schedule(tiles, k / 128, pair ? 2 : 1, grid);
-    const int passes = ((tiles + grid - 1) / grid + args.schedule.slots - 1) / args.schedule.slots;
+    args.schedule = stack_schedule(tiles, k / 128, pair, grid);
+    const int passes = (stack_cta_tiles(args.schedule, 0) + args.schedule.slots - 1) / args.schedule.slots;
     if (tiles == 0) return cudaSuccess;
     int4_cta_stream_kernel<<<dim3(passes * args.schedule.steps, grid), 256, 0, stream>>>(args, out);
     return cudaGetLastError();
@@ -1943,8 +1915,8 @@ cudaError_t launch_int4_cta_streams(const RelayoutSegment *segments, int count, 
 
 bool decode_stack_supported(const StackShape &shape, int lanes, size_t *smem_bytes) {
     if (lanes < 1 || lanes > 8 || shape.grid < 1) return false;
-    if (shape.hidden > 2 * 8 * CONSUMER_THREADS || shape.hidden % 128 != 0 || shape.ffn % 128 != 0 || (shape.q_heads * shape.head_width) % 128 != 0) return false;
-    if (((shape.q_heads + 2 * shape.kv_heads) * shape.head_width) % 16 != 0) return false;
+    if (shape.hidden > 2 * 8 * CONSUMER_THREADS || shape.q_heads * shape.head_width > 2 * 8 * CONSUMER_THREADS || shape.hidden % 128 != 0 || shape.ffn % 128 != 0 || (shape.q_heads * shape.head_width) % 128 != 0) return false;
+    if (((shape.q_heads + 2 * shape.kv_heads) * shape.head_width) % 16 != 0 || shape.kv_heads * 8 > STACK_BARRIER_WORDS - ARRIVAL_WORDS_OFFSET) return false;
     StackPlanSmem plan;
     if (!plan_smem(shape, lanes, shape.grid, &plan)) return false;
     if (smem_bytes) *smem_bytes = plan.total;
@@ -1971,13 +1943,9 @@ cudaError_t launch_decode_stack(const StackLayer *layers_device, int layer_count
     args.tp = tp_size > 1 ? tp_device : nullptr;
     args.tp_size = tp_size;
     args.stages = plan.stages;
-    args.stage_bytes = plan.stage_bytes;
-    args.steps_per_stage = plan.steps_per_stage;
     args.slice_slots = plan.slice_slots;
     args.slice_bytes = plan.slice_bytes;
     args.scratch_bytes = static_cast<uint32_t>(plan.scratch);
-    args.prefetch_stages = 0;  // stages beyond the ring the producer would ask L2 for: measured, no gain
-    args.debug_flags = 0;      // probe switches of the kernel (1: no hand-over checks, 4: weight stream off after the ring has filled)
     const int group = shape.q_heads / shape.kv_heads;
     if (shape.head_width == 128 && group == 4) return launch_instance<128, 4>(args, plan.total, shape.grid, stream);
     if (shape.head_width == 128 && group == 8) return launch_instance<128, 8>(args, plan.total, shape.grid, stream);
