@@ -1222,49 +1222,52 @@ __device__ __forceinline__ ProductConstants product_constants() {
     asm volatile("mov.b64 %0, 0x4380000043800000;" : "=l"(c.term1));
     return c;
 }
-template <int TILES>
-__device__ __forceinline__ void block_product(const uint4 (&rows)[2], uint32_t scales, const ActivationOperands<TILES> &x, const ProductConstants &c, Accumulators<TILES> &acc) {
-    const uint32_t wa[4] = {rows[0].x, rows[0].y, rows[0].z, rows[0].w}, wb[4] = {rows[1].x, rows[1].y, rows[1].z, rows[1].w};
-    int32_t sums[TILES][4];
+// BLOCKS blocks (of different tiles) against the same activations, their chains of MMAs side by side.
+template <int TILES, int BLOCKS>
+__device__ __forceinline__ void block_products(const uint4 (&rows)[2][2], const uint32_t (&scales)[2], const ActivationOperands<TILES> &x, const ProductConstants &c,
+                                               Accumulators<TILES> (&acc)[2]) {
+    int32_t sums[BLOCKS][TILES][4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const uint32_t a0 = (wa[i] * c.sixteen) & 0xf0f0f0f0u, a1 = (wb[i] * c.sixteen) & 0xf0f0f0f0u, a2 = wa[i] & 0xf0f0f0f0u, a3 = wb[i] & 0xf0f0f0f0u;
 #pragma unroll
-        for (int t = 0; t < TILES; t++) {
-            const uint4 &b = x.b[t][i >> 1];
-            const uint32_t b0 = (i & 1) ? b.z : b.x, b1 = (i & 1) ? b.w : b.y;
-            int32_t(&sum)[4] = sums[t];
-            if (i == 0) mma_s8_16832(sum, a0, a1, a2, a3, b0, b1, c.bias, c.bias, c.bias, c.bias);
-            else mma_s8_16832(sum, a0, a1, a2, a3, b0, b1, sum[0], sum[1], sum[2], sum[3]);
+        for (int b = 0; b < BLOCKS; b++) {
+            const uint4 &upper = rows[b][0], &lower = rows[b][1];
+            const uint32_t wa = i == 0 ? upper.x : (i == 1 ? upper.y : (i == 2 ? upper.z : upper.w)), wb = i == 0 ? lower.x : (i == 1 ? lower.y : (i == 2 ? lower.z : lower.w));
+            const uint32_t a0 = (wa * c.sixteen) & 0xf0f0f0f0u, a1 = (wb * c.sixteen) & 0xf0f0f0f0u, a2 = wa & 0xf0f0f0f0u, a3 = wb & 0xf0f0f0f0u;
+#pragma unroll
+            for (int t = 0; t < TILES; t++) {
+                const uint4 &columns = x.b[t][i >> 1];
+                const uint32_t b0 = (i & 1) ? columns.z : columns.x, b1 = (i & 1) ? columns.w : columns.y;
+                int32_t(&sum)[4] = sums[b][t];
+                if (i == 0) mma_s8_16832(sum, a0, a1, a2, a3, b0, b1, c.bias, c.bias, c.bias, c.bias);
+                else mma_s8_16832(sum, a0, a1, a2, a3, b0, b1, sum[0], sum[1], sum[2], sum[3]);
+            }
         }
     }
-    const float scale[2] = {__uint_as_float(scales << 16), __uint_as_float(scales & 0xffff0000u)};
     // the group's sum t0 2^16 + t1 2^8 + t2, rounded to f32 once (but for the last bits of t1 2^8 + t2), times the scale
-    if constexpr (TILES == 3) {
-        const unsigned long long factors = pair_of(x.factor[0], x.factor[1]);
 #pragma unroll
-        for (int r = 0; r < 2; r++) {
-            unsigned long long term[3];
+    for (int b = 0; b < BLOCKS; b++) {
+        const float scale[2] = {__uint_as_float(scales[b] << 16), __uint_as_float(scales[b] & 0xffff0000u)};
+        if constexpr (TILES == 3) {
+            const unsigned long long factors = pair_of(x.factor[0], x.factor[1]);
 #pragma unroll
-            for (int t = 0; t < 3; t++) term[t] = pair_add(pair_of(__int_as_float(sums[t][2 * r]), __int_as_float(sums[t][2 * r + 1])), c.unbias);
-            const unsigned long long sum = pair_fma(term[0], c.term0, pair_fma(term[1], c.term1, term[2]));
-            acc.row[r] = pair_fma(pair_multiply(factors, pair_of(scale[r], scale[r])), sum, acc.row[r]);
-        }
-    } else {
+            for (int r = 0; r < 2; r++) {
+                unsigned long long term[3];
 #pragma unroll
-        for (int r = 0; r < 2; r++) {
-            float term[3];
-            if constexpr (TILES == 1) {
-                const float own = __int_as_float(sums[0][2 * r]) - SUM_BIAS_F32;
-                term[0] = own;
-                term[1] = __int_as_float(sums[0][2 * r + 1]) - SUM_BIAS_F32;
-                term[2] = __shfl_down_sync(0xffffffffu, own, 1);  // term 2 sits one thread column further
-            } else {
-                term[0] = __int_as_float(sums[0][2 * r]) - SUM_BIAS_F32;
-                term[1] = __int_as_float(sums[0][2 * r + 1]) - SUM_BIAS_F32;
-                term[2] = __int_as_float(sums[TILES - 1][2 * r]) - SUM_BIAS_F32;
+                for (int t = 0; t < 3; t++) term[t] = pair_add(pair_of(__int_as_float(sums[b][t][2 * r]), __int_as_float(sums[b][t][2 * r + 1])), c.unbias);
+                const unsigned long long sum = pair_fma(term[0], c.term0, pair_fma(term[1], c.term1, term[2]));
+                acc[b].row[r] = pair_fma(pair_multiply(factors, pair_of(scale[r], scale[r])), sum, acc[b].row[r]);
             }
-            acc.row[r] = fmaf(scale[r] * x.factor[0], fmaf(term[0], 65536.0f, fmaf(term[1], 256.0f, term[2])), acc.row[r]);
+        } else {
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                float term[3];
+                term[0] = __int_as_float(sums[b][0][2 * r]) - SUM_BIAS_F32;
+                term[1] = __int_as_float(sums[b][0][2 * r + 1]) - SUM_BIAS_F32;
+                if constexpr (TILES == 1) term[2] = __shfl_down_sync(0xffffffffu, term[0], 1);  // term 2 sits one thread column further
+                else term[2] = __int_as_float(sums[b][TILES - 1][2 * r]) - SUM_BIAS_F32;
+                acc[b].row[r] = fmaf(scale[r] * x.factor[0], fmaf(term[0], 65536.0f, fmaf(term[1], 256.0f, term[2])), acc[b].row[r]);
+            }
         }
     }
 }
@@ -1351,9 +1354,10 @@ __device__ __forceinline__ uint32_t consume_pass(int phase, int pass, int first_
                 rows[1][0] = smem16(unit + next_tile);
                 rows[1][1] = smem16(unit + next_tile + 512);
                 row_scales[1] = smem4(unit + scales_from_unit + next_tile / 32u);
+                block_products<TILES, 2>(rows, row_scales, operands, constants, acc);
+            } else {
+                block_products<TILES, 1>(rows, row_scales, operands, constants, acc);
             }
-            block_product<TILES>(rows[0], row_scales[0], operands, constants, acc[0]);
-            if (tiles > 1) block_product<TILES>(rows[1], row_scales[1], operands, constants, acc[1]);
         }
         __syncwarp();
         if (lane == 0) {
@@ -1560,8 +1564,7 @@ __device__ __forceinline__ void attention_step(int layer) {
     {
         // merge the heads whose last split was completed here: one (lane, q head) row per warp and round
         const int requests = sh.merge_count;
-        if (requests > 0) {
-            __threadfence();
+        if (requests > 0) {  // (the partials are visible: the counting thread acquired them in front of the meeting above)
             const int group_slots = sh.group_slots, per_stream = sh.a.lanes_per_stream, groups_per_stream = (per_stream + QL - 1) / QL;
             for (int index = thread_now() >> 5; index < requests * QL * GROUP; index += CONSUMER_WARPS) {
                 const int request = sh.merge_list[index / (QL * GROUP)], row = index % (QL * GROUP);
