@@ -228,6 +228,8 @@ std::shared_ptr<MountedModel> MountedModel::mount(const std::string &path, const
         for (const ComponentPlan &layer : plan.layers) target_kv_layers += layer.has_kv ? 1 : 0;
         model->build_stack(plan.layers, 0, model->target_stack_);
         if (plan.has_draft) model->build_stack(plan.draft_layers, target_kv_layers, model->draft_stack_);
+        model->build_small_stack(plan.layers, 0, false, model->target_small_stack_);
+        if (plan.has_draft) model->build_small_stack(plan.draft_layers, target_kv_layers, true, model->draft_small_stack_);
     }
     return model;
 }
@@ -241,6 +243,8 @@ MountedModel::~MountedModel() {
         for (DeviceBuffer &buffer : stack->storage) cudaFree(buffer.ptr);
         cudaFree(stack->device_layers.ptr);
     }
+    cudaFree(target_small_stack_.device_layers.ptr);
+    cudaFree(draft_small_stack_.device_layers.ptr);
     cudaFree(block_table_.ptr);
     cudaFree(page_pools_.ptr);
 }
@@ -441,6 +445,106 @@ void MountedModel::build_stack(const std::vector<ComponentPlan> &layers, int fir
     out.weight_bytes = bytes;
     out.device_layers = device_alloc(built.size() * sizeof(StackLayer), false);
     cuda_check(cudaMemcpy(out.device_layers.ptr, built.data(), built.size() * sizeof(StackLayer), cudaMemcpyHostToDevice), "stack layer table upload");
+}
+
+// Recognises the kernel list of a dense bf16 layer (rms_norm, q/k/v, rope q, rope k, append attention, o + residual, rms_norm,
+// gate/up + silu, down + residual) whose weights fit the one-launch kernel for small models; a draft's adapter has to be the
+// linear of the concatenated norms of its two inputs.
+void MountedModel::build_small_stack(const std::vector<ComponentPlan> &layers, int first_kv_index, bool draft, SmallStackPlan &out) {
+    static const OpKind expected[9] = {OpKind::RmsNorm, OpKind::Linear, OpKind::Rope, OpKind::Rope, OpKind::AppendAttention, OpKind::LinearResidual,
+                                       OpKind::RmsNorm, OpKind::LinearSiluMultiply, OpKind::LinearResidual};
+    out = SmallStackPlan{};
+    if (layers.empty() || options_.tp_size > 1) return;
+    SmallStackShape shape{};
+    std::vector<SmallStackLayer> built;
+    int kv_index = first_kv_index;
+    for (const ComponentPlan &layer : layers) {
+        if (layer.ops.size() != 9 || !layer.has_kv || layer.boundary_inputs.size() != 1) return;
+        for (int i = 0; i < 9; i++)
+            if (layer.ops[i].kind != expected[i]) return;
+        const OpSpec &norm1 = layer.ops[0], &qkv = layer.ops[1], &rope_q = layer.ops[2], &rope_k = layer.ops[3], &attention = layer.ops[4], &o = layer.ops[5],
+                     &norm2 = layer.ops[6], &gate_up = layer.ops[7], &down = layer.ops[8];
+        const std::string &input = layer.boundary_inputs[0];
+        if (qkv.weights.size() != 3 || qkv.outputs.size() != 3 || o.weights.size() != 1 || gate_up.weights.size() != 2 || down.weights.size() != 1) return;
+        const WeightRef *weights[7] = {&qkv.weights[0], &qkv.weights[1], &qkv.weights[2], &o.weights[0], &gate_up.weights[0], &gate_up.weights[1], &down.weights[0]};
+        const bool wired = norm1.inputs[0] == input && qkv.inputs[0] == norm1.outputs[0] && rope_q.inputs[0] == qkv.outputs[0] && rope_k.inputs[0] == qkv.outputs[1] &&
+                           attention.inputs.size() >= 3 && attention.inputs[0] == rope_q.outputs[0] && attention.inputs[1] == rope_k.outputs[0] &&
+                           attention.inputs[2] == qkv.outputs[2] && o.inputs[0] == attention.outputs[0] && o.residual_input == input && o.residual_rounds_product &&
+                           norm2.inputs[0] == o.outputs[0] && gate_up.inputs[0] == norm2.outputs[0] && down.inputs[0] == gate_up.outputs[0] &&
+                           down.residual_input == o.outputs[0] && down.residual_rounds_product && down.outputs[0] == layer.boundary_output;
+        if (!wired || rope_q.rope.size() != 1 || rope_k.rope.size() != 1) return;
+        const RopeAttrs &rq = rope_q.rope[0], &rk = rope_k.rope[0];
+        SmallStackShape here{};
+        here.hidden = static_cast<int>(qkv.weights[0].k);
+        here.q_heads = attention.q_heads;
+        here.kv_heads = attention.kv_heads;
+        here.head_width = attention.head_width;
+        here.ffn = static_cast<int>(gate_up.weights[0].n);
+        here.eps = norm1.eps;
+        here.norm_offset = norm1.weight_offset;
+        here.attention_scale = attention.attention_scale;
+        const int64_t q_width = int64_t(here.q_heads) * here.head_width, kv_width = int64_t(here.kv_heads) * here.head_width;
+        const int64_t n[7] = {q_width, kv_width, kv_width, here.hidden, here.ffn, here.ffn, here.hidden},
+                      k[7] = {here.hidden, here.hidden, here.hidden, q_width, here.hidden, here.hidden, here.ffn};
+        SmallStackLayer spec{};
+        for (int i = 0; i < 7; i++) {
+            if (weights[i]->storage != TensorStorage::BF16 || weights[i]->n != n[i] || weights[i]->k != k[i]) return;
+            spec.weights[i] = static_cast<const uint16_t *>(tensor(weights[i]->tensor));
+        }
+        spec.weights[7] = static_cast<const uint16_t *>(tensor(norm1.norm_weights[0]));
+        spec.weights[8] = static_cast<const uint16_t *>(tensor(norm2.norm_weights[0]));
+        for (const uint16_t *pointer : spec.weights)
+            if (reinterpret_cast<uintptr_t>(pointer) % 16 != 0) return;
+        if (rq.head_width != here.head_width || rk.head_width != here.head_width || rq.rotary_width != here.head_width || rk.rotary_width != here.head_width || rq.interleaved ||
+            rk.interleaved || float_bits(rq.theta) != float_bits(rk.theta) || rq.heads != here.q_heads || rk.heads != here.kv_heads ||
+            float_bits(norm2.eps) != float_bits(norm1.eps) || float_bits(norm2.weight_offset) != float_bits(norm1.weight_offset) || layer.kv_heads != here.kv_heads ||
+            layer.head_width != here.head_width || q_width % 8 != 0)
+            return;
+        here.rope_table = rope_table(rq.theta, rq.rotary_width);
+        here.rope_positions = rope_positions_;
+        if (built.empty()) shape = here;
+        else if (std::memcmp(&shape, &here, sizeof(shape)) != 0) return;
+        if (!small_stack_supported(shape, static_cast<int>(plan().vocab), 1)) return;
+        spec.kv = kv_layer(kv_index++);
+        built.push_back(spec);
+    }
+    const ModelPlan &model = plan();
+    auto bf16 = [&](const std::string &name) { return static_cast<const uint16_t *>(tensor(name)); };
+    SmallForward &forward = out.forward;
+    forward.embedding = bf16(model.embedding_tensor);
+    forward.embedding_scale = model.embedding_scale;
+    forward.vocab = static_cast<int>(model.vocab);
+    const TransducerPlan &tail = draft ? model.draft_output : model.output;
+    forward.final_norm = bf16(tail.norm_tensor);
+    forward.final_eps = tail.eps;
+    forward.final_offset = tail.weight_offset;
+    forward.table = bf16(tail.projection_tensor);
+    forward.logits_scale = tail.logits_scale;
+    if (draft) {
+        const std::vector<OpSpec> &ops = model.draft_adapter.ops;
+        if (ops.size() != 4 || ops[0].kind != OpKind::RmsNorm || ops[1].kind != OpKind::RmsNorm || ops[2].kind != OpKind::Concat || ops[3].kind != OpKind::Linear) return;
+        const OpSpec &embedding_norm = ops[0].inputs[0] == model.adapter_token_signal ? ops[0] : ops[1], &hidden_norm = &embedding_norm == &ops[0] ? ops[1] : ops[0],
+                     &concat = ops[2], &linear = ops[3];
+        forward.embedding_first = concat.inputs.size() == 2 && concat.inputs[0] == embedding_norm.outputs[0];
+        const bool wired = embedding_norm.inputs[0] == model.adapter_token_signal && hidden_norm.inputs[0] == model.adapter_hidden_signal && concat.inputs.size() == 2 &&
+                           concat.inputs[forward.embedding_first ? 0 : 1] == embedding_norm.outputs[0] && concat.inputs[forward.embedding_first ? 1 : 0] == hidden_norm.outputs[0] &&
+                           linear.inputs[0] == concat.outputs[0] && linear.weights.size() == 1 && linear.outputs[0] == model.draft_adapter.boundary_output;
+        if (!wired || linear.weights[0].storage != TensorStorage::BF16 || linear.weights[0].n != shape.hidden || linear.weights[0].k != 2 * shape.hidden ||
+            float_bits(embedding_norm.eps) != float_bits(hidden_norm.eps) || float_bits(embedding_norm.weight_offset) != float_bits(hidden_norm.weight_offset))
+            return;
+        forward.adapter = bf16(linear.weights[0].tensor);
+        forward.adapter_norms[0] = bf16(embedding_norm.norm_weights[0]);
+        forward.adapter_norms[1] = bf16(hidden_norm.norm_weights[0]);
+        forward.adapter_eps = embedding_norm.eps;
+        forward.adapter_offset = embedding_norm.weight_offset;
+        if (reinterpret_cast<uintptr_t>(forward.adapter) % 16 != 0) return;
+    }
+    if (reinterpret_cast<uintptr_t>(forward.table) % 16 != 0) return;
+    out.available = true;
+    out.shape = shape;
+    out.layers = static_cast<int>(built.size());
+    out.device_layers = device_alloc(built.size() * sizeof(SmallStackLayer), false);
+    cuda_check(cudaMemcpy(out.device_layers.ptr, built.data(), built.size() * sizeof(SmallStackLayer), cudaMemcpyHostToDevice), "small stack layer table upload");
 }
 
 const uint32_t *MountedModel::rope_table(float theta, int rotary) const {
@@ -1666,6 +1770,13 @@ void Engine::upload_lanes(const std::vector<uint32_t> &positions, const std::vec
     uint32_t newest = 0;
     for (uint32_t position : positions) newest = std::max(newest, position);
     current_width_ = lanes_per_stream;
+    std::set<int32_t> seen;
+    streams_apart_ = true;
+    for (size_t i = 0; i < slots.size(); i++) {
+        const size_t in_group = i % static_cast<size_t>(lanes_per_stream);
+        streams_apart_ &= in_group == 0 ? seen.insert(slots[i]).second
+                                        : slots[i] == slots[i - in_group] && positions[i] == positions[i - in_group] + static_cast<uint32_t>(in_group);
+    }
     plan_splits(static_cast<int>(positions.size()), lanes_per_stream, newest);
 }
 
@@ -1790,6 +1901,25 @@ bool Engine::run_stack(const StackPlan &stack, int lanes, void *hidden) {
     return true;
 }
 
+// The whole forward of a small bf16 model in one launch, a stream per CTA; false = the caller runs it kernel by kernel.
+bool Engine::run_small_stack(const SmallStackPlan &stack, int lanes, const uint16_t *hidden_in, uint16_t *normalized, bool want_logits, const char *what) {
+    if (!stack_enabled_ || !stack.available || !streams_apart_ || current_blocks_ > 0 || current_width_ <= 0 || lanes % current_width_ != 0 ||
+        !small_stack_supported(stack.shape, stack.forward.vocab, current_width_))
+        return false;
+    SmallForward forward = stack.forward;
+    forward.tokens = current_tokens_;
+    forward.hidden_in = hidden_in;
+    forward.normalized = normalized;
+    forward.logits = want_logits ? static_cast<float *>(logits_.ptr) : nullptr;
+    forward.records = stochastic_streams_ == 0 ? static_cast<uint32_t *>(records_.ptr) : nullptr;
+    check(launch_small_stack(static_cast<const SmallStackLayer *>(stack.device_layers.ptr), stack.layers, stack.shape, forward, current_lanes_, lanes / current_width_,
+                             current_width_, static_cast<int *>(kernel_error_.ptr), cuda_stream_),
+          what);
+    if (want_logits && stochastic_streams_ != 0)
+        sample_lanes(static_cast<const float *>(logits_.ptr), static_cast<uint32_t *>(records_.ptr), lanes, current_lanes_.slot, current_lanes_.position, what);
+    return true;
+}
+
 std::vector<unsigned long long> Engine::decode_stack_timing() {
     std::vector<unsigned long long> stamps;
     if (!stack_timing_.ptr || !model_->target_stack().available) return stamps;
@@ -1801,6 +1931,7 @@ std::vector<unsigned long long> Engine::decode_stack_timing() {
 
 void Engine::target_forward(int lanes, bool want_logits) {
     const ModelPlan &plan = model_->plan();
+    if (run_small_stack(model_->target_small_stack(), lanes, nullptr, static_cast<uint16_t *>(normalized_.ptr), want_logits, "small model")) return;
     check(launch_embedding(static_cast<const uint16_t *>(model_->tensor(plan.embedding_tensor)), current_tokens_,
                            static_cast<uint16_t *>(frame_a_.ptr), lanes, static_cast<int>(plan.hidden), static_cast<int>(plan.vocab),
                            plan.embedding_scale, cuda_stream_),
@@ -1827,6 +1958,7 @@ void Engine::target_forward(int lanes, bool want_logits) {
 
 void Engine::draft_forward(int lanes, const uint16_t *hidden_in, bool want_logits) {
     const ModelPlan &plan = model_->plan();
+    if (run_small_stack(model_->draft_small_stack(), lanes, hidden_in, want_logits ? static_cast<uint16_t *>(draft_normalized_.ptr) : nullptr, want_logits, "small draft")) return;
     check(launch_embedding(static_cast<const uint16_t *>(model_->tensor(plan.embedding_tensor)), current_tokens_,
                            static_cast<uint16_t *>(embedding_out_.ptr), lanes, static_cast<int>(plan.hidden), static_cast<int>(plan.vocab),
                            plan.embedding_scale, cuda_stream_),
@@ -2115,6 +2247,7 @@ void Engine::run_speculative_cycles(std::vector<Stream *> &batch, const std::vec
                                  drafts > 0 ? streams : 0, static_cast<uint16_t *>(pending_backup_.ptr), model_->options().max_streams,
                                  static_cast<int>(plan.hidden), marks, cuda_stream_),
               "pending hidden");
+        streams_apart_ = true;
         // ---- draft loop: `drafts` serial steps over `streams` lanes
         for (int j = 0; j < drafts; j++) {
             current_lanes_ = LaneTable{draft_positions + static_cast<size_t>(j) * streams, stream_slots};

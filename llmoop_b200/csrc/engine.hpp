@@ -61,6 +61,14 @@ struct StackPlan {
     uint64_t weight_bytes = 0;          // bytes one pass over the stack streams
 };
 
+struct SmallStackPlan {
+    bool available = false;
+    SmallStackShape shape{};
+    int layers = 0;
+    DeviceBuffer device_layers;
+    SmallForward forward{};  // what a launch does around the layers, without the buffers of an engine
+};
+
 struct ExecCounters {
     uint64_t kernel_launches = 0;
     uint64_t graph_launches = 0;
@@ -96,6 +104,8 @@ public:
     uint64_t kv_bytes_per_token() const { return kv_bytes_per_token_; }
     const StackPlan &target_stack() const { return target_stack_; }
     const StackPlan &draft_stack() const { return draft_stack_; }
+    const SmallStackPlan &target_small_stack() const { return target_small_stack_; }
+    const SmallStackPlan &draft_small_stack() const { return draft_small_stack_; }
     // The output projection tables in the streaming kernel's order (by tensor name), or nullptr.
     const void *projection_table(const std::string &name) const {
         auto found = projection_tables_.find(name);
@@ -108,6 +118,7 @@ private:
     void upload_tensors();
     void build_rope_tables();
     void build_stack(const std::vector<ComponentPlan> &layers, int first_kv_index, StackPlan &out);
+    void build_small_stack(const std::vector<ComponentPlan> &layers, int first_kv_index, bool draft, SmallStackPlan &out);
 
     std::shared_ptr<HostPackage> package_;
     ModelPlan plan_;
@@ -123,6 +134,7 @@ private:
     uint32_t rope_positions_ = 0;
     int sm_count_ = 0;  // CTAs of the persistent kernels (one per SM of the mount device)
     StackPlan target_stack_, draft_stack_;
+    SmallStackPlan target_small_stack_, draft_small_stack_;
     std::map<std::string, DeviceBuffer> projection_tables_;
 };
 
@@ -391,6 +403,8 @@ private:
     DeviceBuffer stack_q_, stack_attention_out_, stack_activation_, stack_barrier_, stack_timing_;
     bool stack_enabled_ = true;
     bool run_stack(const StackPlan &stack, int lanes, void *hidden);
+    bool streams_apart_ = false;  // every current_width_ lanes are one stream's, no stream in two of these groups
+    bool run_small_stack(const SmallStackPlan &stack, int lanes, const uint16_t *hidden_in, uint16_t *normalized, bool want_logits, const char *what);
     void project_and_sample(const uint16_t *normalized, const std::string &projection_tensor, float scale, int lanes, const int32_t *slots,
                             const uint32_t *ticks, const char *what);
     void check_kernel_status(const uint32_t *status_word);  // throws (after restoring the pending hidden states) when a kernel reported an error

@@ -308,6 +308,43 @@ cudaError_t launch_decode_stack(const StackLayer *layers_device, int layer_count
                                 const StackBuffers &buffers, const LaneTable &lanes_meta, int lanes, int lanes_per_stream,
                                 int split_tokens, int max_splits, cudaStream_t stream, const StackTp *tp_device = nullptr, int tp_size = 1);
 
+// ---- small dense bf16 models (kernels_small_stack.cu) ----
+// A whole forward in one launch, a CTA per stream, for layers whose weights fit a CTA's shared memory twice.
+struct SmallStackLayer {
+    const uint16_t *weights[9];  // q, k, v, o, gate, up, down (bf16 row-major), the weights of the two norms: 16-byte aligned
+    KvLayer kv;
+};
+struct SmallStackShape {
+    int hidden, q_heads, kv_heads, head_width, ffn;
+    float eps, norm_offset, attention_scale;
+    const uint32_t *rope_table;  // [position][head_width / 2] packed (sin << 16 | cos) bf16, halves rotated against one another
+    uint32_t rope_positions;
+};
+struct SmallForward {
+    const uint16_t *embedding;  // [vocab][hidden]
+    const uint32_t *tokens;     // [lanes]
+    float embedding_scale;
+    int vocab;
+    // a draft's input adapter (nullptr: none): [hidden][2 hidden], the norms of the embedding and of hidden_in
+    const uint16_t *adapter, *adapter_norms[2], *hidden_in;
+    float adapter_eps, adapter_offset;
+    int embedding_first;  // the embedding's norm takes the first columns
+    // the final norm's rows [lanes][hidden] (nullptr: ends behind the layers), the logits [lanes][vocab] (nullptr: none), the
+    // arg-max records (nullptr: none)
+    const uint16_t *final_norm;
+    float final_eps, final_offset;
+    uint16_t *normalized;
+    const uint16_t *table;
+    float logits_scale;
+    float *logits;
+    uint32_t *records;
+};
+constexpr int SMALL_STACK_MAX_LANES = 32;  // per stream
+constexpr int SMALL_STACK_MAX_VOCAB = 1024;
+bool small_stack_supported(const SmallStackShape &shape, int vocab, int lanes_per_stream);
+cudaError_t launch_small_stack(const SmallStackLayer *layers_device, int layer_count, const SmallStackShape &shape, const SmallForward &forward, const LaneTable &lanes_meta,
+                               int streams, int lanes_per_stream, int *error_flag, cudaStream_t stream);
+
 // Tensor-parallel row-parallel linears: out = bf16(bf16(sum) + residual) (or bf16(sum) without residual) from the
 // all-reduced f32 sums [count].
 cudaError_t launch_round_add(const float *sums, const uint16_t *residual, uint16_t *out, size_t count, cudaStream_t stream);
