@@ -233,7 +233,7 @@ struct Fp8LinearArgs {
     int first[4];  // matrix b owns the row tiles first[b] .. first[b + 1] - 1
     const uint16_t *residual;
     int lanes, k, epilogue;
-    int passes;  // a CTA covers 32 or 64 rows (1 or 2)
+    int passes;  // a CTA covers 32 x passes rows
 };
 
 template <int M>
@@ -243,7 +243,7 @@ __device__ __forceinline__ void fp8_linear_tile(const Fp8LinearArgs &a, int m0, 
     const uint8_t *const w = a.w[matrix];
     auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, a.k, first, n, count, smem, [&](int m) { return m0 + m; }); };
     const int warps = 32 * a.passes / RowSums<M, false>::ROWS;  // with rows to do in a pass
-    for (int pass = 0; pass < (warps > FP8_WARPS ? 2 : 1); pass++) {
+    for (int pass = 0; pass < (warps + FP8_WARPS - 1) / FP8_WARPS; pass++) {
         const int row0 = (tile - a.first[matrix]) * 32 * a.passes + (pass * FP8_WARPS + warp) * RowSums<M, false>::ROWS;
         RowSums<M, false> sums;
         const uint16_t *scale_row = a.wscale[matrix] + static_cast<size_t>(min(row0, rows - 1) >> 7) * blocks;  // eight rows lie in one block of 128
@@ -295,7 +295,7 @@ __device__ __forceinline__ void fp8_silu_tile(const Fp8LinearArgs &a, int m0, in
     auto stage = [&](int first, int n) { stage_activations<M>(a.xq, a.xscale, a.k, first, n, count, smem, [&](int m) { return m0 + m; }); };
     constexpr int HALF = RowSums<M, true>::ROWS / 2;
     const int warps = 32 * a.passes / RowSums<M, true>::ROWS;
-    for (int pass = 0; pass < (warps > FP8_WARPS ? 2 : 1); pass++) {
+    for (int pass = 0; pass < (warps + FP8_WARPS - 1) / FP8_WARPS; pass++) {
         const int row0 = blockIdx.x * 16 * a.passes + (pass * FP8_WARPS + warp) * HALF, first = min(row0, a.n[0] - 1);
         RowSums<M, true> sums;
         sums.run([&](int r) { return a.w[r / HALF] + static_cast<size_t>(min(row0 + r % HALF, a.n[0] - 1)) * a.k; }, a.wscale[0] + static_cast<size_t>(first >> 7) * blocks,
@@ -378,9 +378,10 @@ struct MoeArgs {
     uint16_t *out;
     MoeGroups groups;
     int hidden, inter, top_k;
+    int passes;  // a CTA's rows: so many times those its warps hold at a time
 };
 
-// grid (tiles of 32 intermediate rows, expert tiles); the activations of a pair are its token's row
+// grid (tiles of 32 intermediate rows x passes, expert tiles); the activations of a pair are its token's row
 template <int M>
 __device__ __forceinline__ void moe_gate_up_tile(const MoeArgs &a, int4 tile, uint8_t *smem) {
     const int warp = threadIdx.x >> 5, k = a.hidden, blocks = k >> 7, count = tile.z;
@@ -390,8 +391,8 @@ __device__ __forceinline__ void moe_gate_up_tile(const MoeArgs &a, int4 tile, ui
     const int expert = tile.x;
     const uint8_t *w = a.w + static_cast<size_t>(expert) * 2 * a.inter * k;
     const uint16_t *ws = a.wscale + static_cast<size_t>(expert) * ((2 * a.inter + 127) >> 7) * blocks;
-    for (int pass = 0; pass < FP8_ROWS / RowSums<M, true>::ROWS; pass++) {
-        const int row0 = (blockIdx.x * FP8_WARPS + warp) * (FP8_ROWS / 2) + pass * HALF, first = min(row0, a.inter - 1);
+    for (int pass = 0; pass < a.passes * FP8_ROWS / RowSums<M, true>::ROWS; pass++) {
+        const int row0 = blockIdx.x * FP8_WARPS * a.passes * (FP8_ROWS / 2) + (pass * FP8_WARPS + warp) * HALF, first = min(row0, a.inter - 1);
         RowSums<M, true> sums;
         sums.run([&](int r) { return w + static_cast<size_t>((r >= HALF ? a.inter : 0) + min(row0 + r % HALF, a.inter - 1)) * k; },
                  ws + static_cast<size_t>(first >> 7) * blocks, ws + static_cast<size_t>((a.inter + first) >> 7) * blocks, blocks, smem, pass > 0, stage);
@@ -412,7 +413,7 @@ __global__ void __launch_bounds__(FP8_WARPS * 32, 2) moe_gate_up_fp8_kernel(cons
     by_count(tile.z, [&] { moe_gate_up_tile<2>(a, tile, fp8_smem); }, [&] { moe_gate_up_tile<4>(a, tile, fp8_smem); }, [&] { moe_gate_up_tile<8>(a, tile, fp8_smem); });
 }
 
-// grid (tiles of 64 hidden rows, expert tiles); out = bf16(bf16(sum) * route weight) per pair
+// grid (tiles of 64 hidden rows x passes, expert tiles); out = bf16(bf16(sum) * route weight) per pair
 template <int M>
 __device__ __forceinline__ void moe_down_tile(const MoeArgs &a, int4 tile, uint8_t *smem) {
     const int warp = threadIdx.x >> 5, thread = threadIdx.x & 31, k = a.inter, blocks = k >> 7, count = tile.z;
@@ -421,8 +422,8 @@ __device__ __forceinline__ void moe_down_tile(const MoeArgs &a, int4 tile, uint8
     const int expert = tile.x;
     const uint8_t *w = a.w + static_cast<size_t>(expert) * a.hidden * k;
     const uint16_t *ws = a.wscale + static_cast<size_t>(expert) * ((a.hidden + 127) >> 7) * blocks;
-    for (int pass = 0; pass < FP8_ROWS / RowSums<M, false>::ROWS; pass++) {
-        const int row0 = (blockIdx.x * FP8_WARPS + warp) * FP8_ROWS + pass * RowSums<M, false>::ROWS;
+    for (int pass = 0; pass < a.passes * FP8_ROWS / RowSums<M, false>::ROWS; pass++) {
+        const int row0 = blockIdx.x * FP8_WARPS * a.passes * FP8_ROWS + (pass * FP8_WARPS + warp) * RowSums<M, false>::ROWS;
         const uint16_t *scale_row = ws + static_cast<size_t>(min(row0, a.hidden - 1) >> 7) * blocks;
         RowSums<M, false> sums;
         sums.run([&](int r) { return w + static_cast<size_t>(min(row0 + r, a.hidden - 1)) * k; }, scale_row, scale_row, blocks, smem, pass > 0, stage);
@@ -454,8 +455,14 @@ cudaError_t launch_rows(void (*kernel)(Args), dim3 grid, int tile_lanes, cudaStr
     return launch_dependent(kernel, grid, dim3(FP8_WARPS * 32), bytes(tile_lanes <= 2 ? 2 : tile_lanes <= 4 ? 4 : 8), 1, stream, args);
 }
 
-// Rows of a CTA: 64 save half of the staging, 32 spread a small launch over more SMs.
-int fp8_passes(int row_tiles, int lanes) { return row_tiles * ((lanes + TILE_LANES - 1) / TILE_LANES) < 2 * multiprocessors() ? 1 : 2; }
+// Rows of a CTA in units of 32: 64 save half of the staging, 32 spread a small launch over more SMs; 128 and 256 save more of
+// it where some five waves of CTAs are left (1024 lanes of 2048 x 4096: 509 -> 488 us, of 5120 x 2048: 664 -> 632 us).
+int fp8_passes(int row_tiles, int lanes) {  // (row tiles of 64)
+    const long long ctas = static_cast<long long>(row_tiles) * ((lanes + TILE_LANES - 1) / TILE_LANES);
+    int passes = ctas < 2 * multiprocessors() ? 1 : 2;
+    while (passes > 1 && passes < 8 && ctas / passes >= 10 * multiprocessors()) passes *= 2;
+    return passes;
+}
 
 }  // namespace
 
@@ -542,14 +549,24 @@ static int most_tiles(int lanes, int top_k, int experts) {
     return pairs < pairs / TILE_LANES + experts ? pairs : pairs / TILE_LANES + experts;
 }
 
+// A CTA waits for its tile's entry, its pairs and their rows, one after the other, before it stages the activations: about
+// half of its time when it takes 64 rows of a few pairs.  More rows per CTA pay for that once, as long as some five waves
+// of CTAs are left (128 experts of 2048 x 768, 8 per token, gate and up with down: 24 tokens 186 -> 166 us with two passes,
+// 1024 tokens 3090 -> 2680 us with four).
+static int moe_passes(int row_tiles, int expert_tiles) {
+    int passes = 1;
+    while (passes < 4 && static_cast<long long>(row_tiles) * expert_tiles / (2 * passes) >= 10 * multiprocessors()) passes *= 2;
+    return passes;
+}
+
 cudaError_t launch_moe_gate_up_fp8(const uint8_t *xq, const float *xscale, const MoeGroups &groups, const uint8_t *w,
                                    const uint16_t *wscale, uint16_t *intermediates, int lanes, int hidden_size,
                                    int inter, int experts, int top_k, cudaStream_t stream) {
     if (lanes <= 0) return cudaSuccess;
     if (hidden_size % 128 != 0) return cudaErrorInvalidValue;
-    const MoeArgs args{xq, xscale, nullptr, w, wscale, intermediates, groups, hidden_size, inter, top_k};
-    const int rows = FP8_WARPS * FP8_ROWS / 2;
-    return launch_rows(moe_gate_up_fp8_kernel, dim3((inter + rows - 1) / rows, most_tiles(lanes, top_k, experts)), TILE_LANES, stream, args);
+    const int tiles = most_tiles(lanes, top_k, experts), passes = moe_passes((inter + 31) / 32, tiles), rows = FP8_WARPS * passes * FP8_ROWS / 2;
+    const MoeArgs args{xq, xscale, nullptr, w, wscale, intermediates, groups, hidden_size, inter, top_k, passes};
+    return launch_rows(moe_gate_up_fp8_kernel, dim3((inter + rows - 1) / rows, tiles), TILE_LANES, stream, args);
 }
 
 cudaError_t launch_moe_down_fp8(const uint8_t *xq, const float *xscale, const MoeGroups &groups, const uint32_t *routes, const uint8_t *w,
@@ -557,9 +574,9 @@ cudaError_t launch_moe_down_fp8(const uint8_t *xq, const float *xscale, const Mo
                                 int experts, int top_k, cudaStream_t stream) {
     if (lanes <= 0) return cudaSuccess;
     if (inter % 128 != 0) return cudaErrorInvalidValue;
-    const MoeArgs args{xq, xscale, routes, w, wscale, outputs, groups, hidden_size, inter, top_k};
-    const int rows = FP8_WARPS * FP8_ROWS;
-    return launch_rows(moe_down_fp8_kernel, dim3((hidden_size + rows - 1) / rows, most_tiles(lanes, top_k, experts)), TILE_LANES, stream, args);
+    const int tiles = most_tiles(lanes, top_k, experts), passes = moe_passes((hidden_size + 63) / 64, tiles), rows = FP8_WARPS * passes * FP8_ROWS;
+    const MoeArgs args{xq, xscale, routes, w, wscale, outputs, groups, hidden_size, inter, top_k, passes};
+    return launch_rows(moe_down_fp8_kernel, dim3((hidden_size + rows - 1) / rows, tiles), TILE_LANES, stream, args);
 }
 
 }  // namespace nerve
