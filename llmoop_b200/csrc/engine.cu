@@ -2143,7 +2143,7 @@ void Engine::run_single_ticks(std::vector<Stream *> &batch, const std::function<
     uint32_t *status_word = host_records_ + static_cast<size_t>(lanes) * 4;
     run_phase({1, lanes, 0, splits, stochastic_streams_ != 0 ? 1 : 0, stack_enabled_ ? 1 : 0, any_emit ? 1 : 0}, [&] {
         if (plan.has_draft)
-            check(launch_begin_cycle(static_cast<const uint16_t *>(pending_hidden_.ptr), nullptr, nullptr, 0, static_cast<uint16_t *>(pending_backup_.ptr),
+            check(launch_begin_cycle(nullptr, nullptr, 0, static_cast<const uint16_t *>(pending_hidden_.ptr), nullptr, nullptr, 0, static_cast<uint16_t *>(pending_backup_.ptr),
                                      model_->options().max_streams, static_cast<int>(plan.hidden), nullptr, cuda_stream_),
                   "pending hidden backup");
         target_forward(lanes, any_emit);
@@ -2232,18 +2232,19 @@ void Engine::run_speculative_cycles(std::vector<Stream *> &batch, const std::vec
         }
     }
     sync_block_tables();
-    std::memcpy(host_cycle_, staging.data(), upload_words * sizeof(uint32_t));  // the last cycle's copy is done: every cycle ends with a synchronisation
+    std::memcpy(host_cycle_, staging.data(), upload_words * sizeof(uint32_t));  // the last cycle has read it: every cycle ends with a synchronisation
     counters_.h2d_bytes += upload_words * sizeof(uint32_t);
     const int splits = plan_splits(lanes, 1, newest_tick);
 
-    // The whole cycle is one graph with its two copies; its times are stamped by kernels that run anyway.  A graph launch,
-    // a copy or an event between two graphs left the device idle for 5 to 20 us each.
+    // The whole cycle is one graph of kernels, the first of which reads the host's words and the last writes them; its times are
+    // stamped by kernels that run anyway.  A graph launch, a copy or an event between two graphs left the device idle for 5 to
+    // 20 us each.
     const size_t row_words = 4 + 2 * width, mark_offset = (upload_words + streams * row_words + 1) & ~size_t(1);
     unsigned long long *marks = reinterpret_cast<unsigned long long *>(base + mark_offset);
     const size_t result_words = mark_offset - upload_words + CYCLE_MARKS * 2;
     run_phase({0, streams, drafts, splits, stochastic_streams_ != 0 ? 1 : 0, stack_enabled_ ? 1 : 0}, [&] {
-        cuda_check(cudaMemcpyAsync(base, host_cycle_, upload_words * sizeof(uint32_t), cudaMemcpyHostToDevice, cuda_stream_), "cycle state upload");
-        check(launch_begin_cycle(static_cast<const uint16_t *>(pending_hidden_.ptr), stream_slots, static_cast<uint16_t *>(draft_hidden_in_.ptr),
+        check(launch_begin_cycle(host_cycle_, base, static_cast<int>(upload_words), static_cast<const uint16_t *>(pending_hidden_.ptr),
+                                 reinterpret_cast<const int32_t *>(host_cycle_ + (s_slots - staging.data())), static_cast<uint16_t *>(draft_hidden_in_.ptr),
                                  drafts > 0 ? streams : 0, static_cast<uint16_t *>(pending_backup_.ptr), model_->options().max_streams,
                                  static_cast<int>(plan.hidden), marks, cuda_stream_),
               "pending hidden");
@@ -2280,8 +2281,7 @@ void Engine::run_speculative_cycles(std::vector<Stream *> &batch, const std::vec
                             static_cast<int>(plan.hidden), cuda_stream_),
               "accept");
         draft_forward(lanes, static_cast<const uint16_t *>(draft_hidden_in_.ptr), false);
-        check(launch_finish_cycle(marks, static_cast<const int *>(kernel_error_.ptr), cuda_stream_), "cycle status");
-        cuda_check(cudaMemcpyAsync(host_records_, accept_rows, result_words * sizeof(uint32_t), cudaMemcpyDeviceToHost, cuda_stream_), "accept readback");
+        check(launch_finish_cycle(accept_rows, static_cast<int>(result_words), marks, static_cast<const int *>(kernel_error_.ptr), host_records_, cuda_stream_), "cycle status");
     });
     counters_.d2h_bytes += result_words * sizeof(uint32_t);
     synchronize("cycle synchronize");

@@ -414,7 +414,7 @@ private:
     uint8_t *staging_ = nullptr;
     size_t staging_bytes_ = 0, staging_used_ = 0;
     uint32_t *host_records_ = nullptr;      // pinned readback area
-    uint32_t *host_cycle_ = nullptr;        // pinned: what a speculative cycle starts from, copied by its graph
+    uint32_t *host_cycle_ = nullptr;        // pinned: what a speculative cycle starts from, read by its first kernel
     int split_tokens_ = 256, max_splits_ = 1;
     int prefill_chunk_ = 64;
     bool use_graphs_ = true, log_cycles_ = false;

@@ -353,9 +353,9 @@ cudaError_t launch_round_add(const float *sums, const uint16_t *residual, uint16
 // dst[i] = src[index[i]] for rows of `width` bf16.
 // Times (nanoseconds, device clock) and the status of a speculative cycle.
 enum CycleMark { CYCLE_BEGIN, CYCLE_DRAFTED, CYCLE_VERIFIED, CYCLE_END, CYCLE_STATUS, CYCLE_MARKS };
-cudaError_t launch_begin_cycle(const uint16_t *pending, const int32_t *slots, uint16_t *gathered, int rows, uint16_t *backup, int max_streams, int hidden,
-                               unsigned long long *marks, cudaStream_t stream);
-cudaError_t launch_finish_cycle(unsigned long long *marks, const int *error_word, cudaStream_t stream);
+cudaError_t launch_begin_cycle(const uint32_t *host_state, uint32_t *state, int state_words, const uint16_t *pending, const int32_t *host_slots, uint16_t *gathered, int rows,
+                               uint16_t *backup, int max_streams, int hidden, unsigned long long *marks, cudaStream_t stream);
+cudaError_t launch_finish_cycle(const uint32_t *results, int words, unsigned long long *marks, const int *error_word, uint32_t *host_results, cudaStream_t stream);
 cudaError_t launch_gather_rows(const uint16_t *src, const int32_t *index, uint16_t *dst, int rows, int width,
                                cudaStream_t stream);
 // Hidden inputs of the draft catch-up: lane (s, 0) takes pending[slot[s]], lane (s, i>0) takes normalized (s, i-1).

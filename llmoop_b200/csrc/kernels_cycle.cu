@@ -31,35 +31,43 @@ cudaError_t launch_gather_rows(const uint16_t *src, const int32_t *index, uint16
     return launch_dependent(gather_rows_kernel, dim3(rows), dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(src), index, reinterpret_cast<uint32_t *>(dst), width / 2);
 }
 
-// What a cycle starts with, in one launch: the batch's rows of `pending` gathered, all of `pending` saved (blocks behind the
-// gathered rows, one per slot), the time.
-__global__ void begin_cycle_kernel(const uint32_t *__restrict__ pending, const int32_t *__restrict__ slots, uint32_t *__restrict__ gathered, int rows,
-                                   uint32_t *__restrict__ backup, int words, unsigned long long *marks) {
+// What a cycle starts with, in one launch: the host's words (pinned memory, read over the bus) on the device, the batch's rows
+// of `pending` gathered, all of `pending` saved (blocks behind the gathered rows, one per slot), the time.  `slots` is among
+// the host's words, too: the blocks do not wait for one another.
+// (A copy at either end of the graph took its time and one at its border to the kernels, which no early start of the next
+// kernel hides: a cycle of two layers of hidden 64 with one draft took 76 us with them and takes 70.)
+__global__ void begin_cycle_kernel(const uint32_t *host_state, uint32_t *state, int state_words, const uint32_t *__restrict__ pending, const int32_t *slots,
+                                   uint32_t *__restrict__ gathered, int rows, uint32_t *__restrict__ backup, int words, unsigned long long *marks) {
     grid_launch_dependents();
     grid_dependency_wait();
     const int block = blockIdx.x;
     if (block == 0 && threadIdx.x == 0 && marks != nullptr) marks[CYCLE_BEGIN] = global_time();
+    for (int word = block * blockDim.x + threadIdx.x; word < state_words; word += gridDim.x * blockDim.x) state[word] = host_state[word];
     const int source = block < rows ? slots[block] : block - rows;
     if (source < 0) return;
     const uint32_t *from = pending + static_cast<size_t>(source) * words;
     uint32_t *to = block < rows ? gathered + static_cast<size_t>(block) * words : backup + static_cast<size_t>(source) * words;
     for (int word = threadIdx.x; word < words; word += blockDim.x) to[word] = from[word];
 }
-cudaError_t launch_begin_cycle(const uint16_t *pending, const int32_t *slots, uint16_t *gathered, int rows, uint16_t *backup, int max_streams, int hidden,
-                               unsigned long long *marks, cudaStream_t stream) {
-    return launch_dependent(begin_cycle_kernel, dim3(rows + max_streams), dim3(256), 0, 1, stream, reinterpret_cast<const uint32_t *>(pending), slots,
-                            reinterpret_cast<uint32_t *>(gathered), rows, reinterpret_cast<uint32_t *>(backup), hidden / 2, marks);
+cudaError_t launch_begin_cycle(const uint32_t *host_state, uint32_t *state, int state_words, const uint16_t *pending, const int32_t *host_slots, uint16_t *gathered, int rows,
+                               uint16_t *backup, int max_streams, int hidden, unsigned long long *marks, cudaStream_t stream) {
+    return launch_dependent(begin_cycle_kernel, dim3(rows + max_streams), dim3(256), 0, 1, stream, host_state, state, state_words, reinterpret_cast<const uint32_t *>(pending),
+                            host_slots, reinterpret_cast<uint32_t *>(gathered), rows, reinterpret_cast<uint32_t *>(backup), hidden / 2, marks);
 }
 
-// ... and ends with: the time, and the error word next to the results, so that one copy brings all of it to the host.
-__global__ void finish_cycle_kernel(unsigned long long *marks, const int *error_word) {
+// ... and ends with: the time and the error word next to the results, and all of them in the host's memory.
+__global__ void finish_cycle_kernel(const uint32_t *results, int words, unsigned long long *marks, const int *error_word, uint32_t *host_results) {
     grid_launch_dependents();
     grid_dependency_wait();
-    marks[CYCLE_END] = global_time();
-    marks[CYCLE_STATUS] = static_cast<unsigned long long>(static_cast<unsigned int>(*error_word));
+    if (threadIdx.x == 0) {
+        marks[CYCLE_END] = global_time();
+        marks[CYCLE_STATUS] = static_cast<unsigned long long>(static_cast<unsigned int>(*error_word));
+    }
+    __syncthreads();  // the marks are among the words
+    for (int word = threadIdx.x; word < words; word += blockDim.x) host_results[word] = results[word];
 }
-cudaError_t launch_finish_cycle(unsigned long long *marks, const int *error_word, cudaStream_t stream) {
-    return launch_dependent(finish_cycle_kernel, dim3(1), dim3(1), 0, 1, stream, marks, error_word);
+cudaError_t launch_finish_cycle(const uint32_t *results, int words, unsigned long long *marks, const int *error_word, uint32_t *host_results, cudaStream_t stream) {
+    return launch_dependent(finish_cycle_kernel, dim3(1), dim3(256), 0, 1, stream, results, words, marks, error_word, host_results);
 }
 
 __global__ void shift_hidden_kernel(const uint32_t *__restrict__ pending, const int32_t *__restrict__ slots,
