@@ -511,7 +511,6 @@ __device__ __forceinline__ float operand_factor(uint32_t exponent) {
 // The digits of four whole numbers as three words (term 0 first).  A number comes as the bits of 1.5 * 2^23 + X, which
 // is how f32 rounds to whole numbers; 2^7 in front of each digit makes its byte unsigned, so that no digit borrows from
 // the next.  (The additions are multiply-adds by an opaque one: they leave the half-rate integer pipe to the permutes.)
-constexpr float WHOLE_BIAS = 12582912.0f;
 struct DigitConstants {  // made where they are used: the compiler would keep them in registers through the whole layer
     uint32_t one, digits;
     unsigned long long bias;  // a pair
@@ -685,7 +684,11 @@ __device__ __forceinline__ void stage_any(const uint16_t *x, const uint16_t *wei
     return narrow ? stage_rows<1, LANES>(x, weight, width, first_group, groups) : stage_rows<2, 2>(x, weight, width, first_group, groups);
 }
 
-// A group's 128 columns of one lane (f32 in shared memory) into operand form in global memory, by one warp.
+// A group's 128 columns of one lane (f32 in shared memory) into operand form in global memory, by one warp.  The products of
+// SiLU and up have a heavy tail: X has a bit more here (e - 22), which the three digits hold unless the largest mantissa is
+// about the greatest there is; such a group takes the next exponent.  (Against 64 bits, 14336 columns of rounded SiLU
+// products, gates and ups of 1.28 N(0, 1): RMS 9.1e-8 of the output without that bit, 8.5e-8 with it and with the fp16
+// operands and f32 sums this form replaced; 2176 columns 7.1e-8, 5.7e-8 and 6.0e-8.  Normalised rows: 6.4e-8 each.)
 __device__ __forceinline__ void store_operand_group(uint8_t *block, const float *columns, int m, int lanes) {
     const int lane = thread_now() & 31, word = lane >> 1, odd = lane & 1;
     float v[4];
@@ -693,16 +696,16 @@ __device__ __forceinline__ void store_operand_group(uint8_t *block, const float 
     for (int i = 0; i < 4; i++) v[i] = columns[word * 8 + odd + 2 * i];
     const uint32_t largest = __reduce_max_sync(0xffffffffu, max(max(__float_as_uint(v[0]) & 0x7fffffffu, __float_as_uint(v[1]) & 0x7fffffffu),
                                                                 max(__float_as_uint(v[2]) & 0x7fffffffu, __float_as_uint(v[3]) & 0x7fffffffu)));
-    const uint32_t exponent = largest >> 23;
+    const uint32_t exponent = max((largest + 0x18000u) >> 23, 32u);  // (above 1.988 x 2^e: the next one)
     uint32_t terms[3], whole[4];
-    const float scale = operand_scale(exponent);
+    const float scale = __uint_as_float((276u - min(exponent, 255u)) << 23), factor = __uint_as_float(largest >= 0x7f800000u ? 0x7fc00000u : (exponent - 26u) << 23);
 #pragma unroll
-    for (int i = 0; i < 4; i++) whole[i] = __float_as_uint(fmaf(v[i], scale, WHOLE_BIAS));
+    for (int i = 0; i < 4; i++) whole[i] = 0x4B400000u + static_cast<uint32_t>(__float2int_rn(v[i] * scale));
     operand_digits(whole[0], whole[1], whole[2], whole[3], digit_constants(), terms);
     uint8_t *place = block + operand_word_offset(word, m, lanes) + 4 * odd;
 #pragma unroll
     for (int t = 0; t < 3; t++) *reinterpret_cast<uint32_t *>(place + 64 * t) = terms[t];
-    if (lane == 0) *reinterpret_cast<float *>(block + 2 * operand_half_bytes(lanes) + 4 * m) = operand_factor(exponent);
+    if (lane == 0) *reinterpret_cast<float *>(block + 2 * operand_half_bytes(lanes) + 4 * m) = factor;
 }
 
 // ------------------------------------------------------------------------------------------ attention
