@@ -640,7 +640,7 @@ __device__ __forceinline__ void stage_rows(const uint16_t *x, const uint16_t *we
                     }
                     raw[mm][c] = make_uint4(words[0], words[1], words[2], words[3]);
                 }
-                if (CHUNKS > 1 && chunk >= per_lane) words[0] = words[1] = words[2] = words[3] = 0;
+                if (chunk >= per_lane) words[0] = words[1] = words[2] = words[3] = 0;  // beyond the row: no part of the warp's exponent
                 const uint32_t most =
                     larger_halves(larger_halves(words[0] & 0x7fff7fffu, words[1] & 0x7fff7fffu), larger_halves(words[2] & 0x7fff7fffu, words[3] & 0x7fff7fffu));
                 largest[mm] = larger_halves(most, most >> 16) & 0x7f80u;

@@ -1,0 +1,144 @@
+"""The matrix steps of the persistent decode stack kernel against 64-bit arithmetic, one step at a time.
+
+A layer is made so that one of its steps has inputs that are known exactly and outputs that can be read:
+
+* the residual stream is +-1 in its first half and 0 in the second, and the norm's epsilon makes the mean square 1, so a
+  normalised row is the norm's weight with the lane's sign;
+* every stream has one token, so an attention output is the value projection itself;
+* gates of 32 leave SiLU as they are, so a product is 32 times the up projection;
+* scales of zero take the steps behind the tested one out of the residual stream, whose second half is then the output.
+
+Row r of the tested matrix has weights only on columns below its own bound of magnitude, so that a large value in a group
+does not cover what the small ones of the group add up to.  An output may be off by half a bf16 unit and by 2^-20 of the sum
+of its terms' magnitudes (the f32 sums over the groups and the warps: some fifty roundings of 2^-24, and what a tie makes of
+them)."""
+
+import ctypes
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+HERE = Path(__file__).resolve().parent
+PAGE = 16
+
+
+class _Layers(ctypes.Structure):
+    _fields_ = ([("words", ctypes.c_void_p * 7), ("scales", ctypes.c_void_p * 7)] +
+                [(name, ctypes.c_void_p) for name in ("input_norm", "post_norm", "rope", "hidden", "pool", "attention_out", "table", "positions", "slots")] +
+                [(name, ctypes.c_int) for name in ("lanes", "lanes_per_stream", "hidden_width", "q_heads", "kv_heads", "head_width", "ffn", "page_tokens", "pages_per_slot",
+                                                   "attended", "layers", "launches")] +
+                [(name, ctypes.c_float) for name in ("eps", "norm_offset", "attention_scale", "milliseconds")])
+
+
+@pytest.fixture(scope="module")
+def launch(tmp_path_factory):
+    from llmoop_b200 import build
+
+    library = tmp_path_factory.mktemp("stack") / "stack_layers.so"
+    kernels = build.BUILD / "kernels_stack.cu.o"  # (a minute's compilation: taken from the build where it is there)
+    command = [build._nvcc(), *build.NVCC_FLAGS, "-shared", "-o", str(library), str(HERE / "stack_layers.cu"),
+               str(kernels if kernels.exists() else build.CSRC / "kernels_stack.cu")]
+    result = subprocess.run(command, capture_output=True, text=True)
+    assert result.returncode == 0, result.stderr
+    return ctypes.CDLL(str(library)).stack_layers
+
+
+def _bf16(values):
+    """float64 to the nearest bf16, as float64 (finite values)."""
+    bits = np.asarray(values, dtype=np.float32).view(np.uint32).astype(np.uint64)
+    return (((bits + 0x7FFF + ((bits >> 16) & 1)) >> 16) << 16).astype(np.uint32).view(np.float32).astype(np.float64)
+
+
+class _Layer:
+    """Shape, weights (whole numbers -8 .. 7, bf16 scales per 128 columns) and norms of a layer; zeros to begin with."""
+
+    def __init__(self, hidden, q_heads, kv_heads, head, ffn, offset=0.0):
+        self.hidden, self.q_heads, self.kv_heads, self.head, self.ffn, self.offset = hidden, q_heads, kv_heads, head, ffn, offset
+        rows = {"q": (q_heads * head, hidden), "k": (kv_heads * head, hidden), "v": (kv_heads * head, hidden), "o": (hidden, q_heads * head), "gate": (ffn, hidden),
+                "up": (ffn, hidden), "down": (hidden, ffn)}
+        self.weight = {name: np.zeros(shape, dtype=np.int64) for name, shape in rows.items()}
+        self.scale = {name: np.zeros((n, k // 128)) for name, (n, k) in rows.items()}
+        self.norm = {"input": np.ones(hidden) - offset, "post": np.ones(hidden) - offset}
+        self.weight["gate"][:, 0], self.scale["gate"][:, 0] = 4, 8.0  # a gate of 32: column 0 is 1 in every lane
+
+    def single(self, name, values, column=None):
+        """Row r is values[r] (bf16) times one column: the lane's sign of column r + 1 (or `column`)."""
+        rows = np.arange(len(values))
+        columns = rows % (self.hidden // 2 - 1) + 1 if column is None else np.full(len(values), column)
+        self.weight[name][rows, columns] = 1
+        self.scale[name][rows, columns // 128] = values
+        return columns
+
+    def product(self, name, x):
+        """Sums and sums of magnitudes in 64 bits, for rows x of [lanes, k]."""
+        full = self.weight[name] * np.repeat(self.scale[name], 128, axis=1)
+        return x @ full.T, np.abs(x) @ np.abs(full).T
+
+    def run(self, launch, hidden, normalised_sum=0.5):
+        import torch
+
+        def device(array, dtype):
+            return torch.from_numpy(np.ascontiguousarray(array.astype(dtype))).cuda()
+
+        def bf16(array):
+            return torch.from_numpy(np.ascontiguousarray(array, dtype=np.float64)).to(torch.bfloat16).cuda()
+
+        lanes = hidden.shape[0]
+        t = _Layers()
+        keep = []
+        for i, name in enumerate(("q", "k", "v", "o", "gate", "up", "down")):
+            n, k = self.weight[name].shape
+            nibbles = (self.weight[name] + 8).astype(np.uint32).reshape(n, k // 8, 8)
+            keep += [device((nibbles << (4 * np.arange(8, dtype=np.uint32))).sum(-1), np.uint32).view(torch.int32), bf16(self.scale[name])]
+            t.words[i], t.scales[i] = keep[-2].data_ptr(), keep[-1].data_ptr()
+        named = {"input_norm": bf16(self.norm["input"]), "post_norm": bf16(self.norm["post"]), "rope": torch.full((self.head // 2,), 0x3F80, dtype=torch.int32, device="cuda"),
+                 "hidden": bf16(hidden), "pool": torch.zeros((lanes, 2, self.kv_heads, PAGE, self.head), dtype=torch.bfloat16, device="cuda"),
+                 "attention_out": torch.zeros((8, self.q_heads * self.head), dtype=torch.bfloat16, device="cuda"),
+                 "table": torch.arange(lanes, dtype=torch.int32, device="cuda"), "positions": torch.zeros(lanes, dtype=torch.int32, device="cuda"),
+                 "slots": torch.arange(lanes, dtype=torch.int32, device="cuda")}
+        for name, tensor in named.items():
+            setattr(t, name, tensor.data_ptr())
+        for name, value in (("lanes", lanes), ("lanes_per_stream", 1), ("hidden_width", self.hidden), ("q_heads", self.q_heads), ("kv_heads", self.kv_heads),
+                            ("head_width", self.head), ("ffn", self.ffn), ("page_tokens", PAGE), ("pages_per_slot", 1), ("attended", 1), ("layers", 1), ("launches", 1)):
+            setattr(t, name, value)
+        t.eps, t.norm_offset, t.attention_scale = 1.0 - normalised_sum, self.offset, 1.0
+        torch.cuda.synchronize()
+        assert launch(ctypes.byref(t)) == 0
+        values = named["pool"][:, 1, :, 0].reshape(lanes, -1)
+        return named["hidden"].double().cpu().numpy(), values.double().cpu().numpy()
+
+
+def _hidden(rng, lanes, width):
+    rows = np.zeros((lanes, width))
+    rows[:, : width // 2] = rng.choice([-1.0, 1.0], size=(lanes, width // 2))
+    rows[:, 0] = 1.0
+    return rows
+
+
+def _check(got, sums, magnitudes, where):
+    unit = np.exp2(np.floor(np.log2(np.maximum(np.abs(sums), 2.0**-100))) - 7)
+    excess = np.abs(got - sums) - (0.5 * unit + 2.0**-20 * magnitudes)
+    assert np.isfinite(got).all() and excess.max() <= 0, (where, np.unravel_index(excess.argmax(), excess.shape), got.flat[excess.argmax()], sums.flat[excess.argmax()])
+
+
+def test_a_group_at_the_end_of_a_row_keeps_its_own_scale(launch):
+    """Rows of an odd number of groups (384 columns, heads of 32): a warp has one group and threads beyond the row.  The first
+    chunk of the row is a million times as large as the last group."""
+    rng = np.random.default_rng(1)
+    layer = _Layer(512, 12, 6, 32, 256)
+    values = np.where(np.arange(192) < 4, 2.0**12, _bf16(rng.uniform(2.0**-8, 2.0**-4, size=192)))
+    hidden = _hidden(rng, 4, 512)
+    columns = layer.single("v", values)
+    head = np.arange(384) // 32 // 2 * 32 + np.arange(384) % 32  # of the value row, by column of o's input
+    inputs = (hidden[:, columns] * values)[:, head]
+    layer.weight["o"][:] = rng.integers(-8, 8, size=(512, 384))
+    layer.weight["o"][:, :256] = 0
+    layer.scale["o"][:] = _bf16(rng.uniform(0.5, 1.0, size=(512, 3)))
+    out, got = layer.run(launch, hidden)
+    assert np.array_equal(got, hidden[:, columns] * values)
+    sums, magnitudes = layer.product("o", inputs)
+    _check(out[:, 256:], sums[:, 256:], magnitudes[:, 256:], "o")
