@@ -318,7 +318,8 @@ struct StackShared {
     // attention: for each team the KV rows of its first work item (the block table is shared by all layers, so the rows
     // of a (split, lane group) are the same in every layer's pool)
     int32_t group_slots;        // lane groups of all streams
-    AttentionItem item[4], later_item[4];
+    AttentionItem item[4];
+    AttentionItem later_item[2][4];  // taken in turn: an item without tokens has no barrier behind the reading of its count
     int32_t merge_count;        // (kv head, lane group) pairs whose last split this CTA's teams completed in this layer ...
     uint16_t merge_list[ATTENTION_MERGE_LIST];  // ... and which: kv_head * group_slots + group_slot
     uint32_t row_base[4][64];   // offset (in rows of HD elements) of token t's K row of kv head 0 in a layer's pool
@@ -1550,16 +1551,17 @@ __device__ __forceinline__ void attention_step(int layer) {
     const int total = sh.a.shape.kv_heads * sh.a.max_splits * sh.group_slots;
     {
         const int team = thread_now() >> 7;
-        bool first = true;
+        int round = 0;
 #pragma unroll 1
-        for (int item = blockIdx.x + gridDim.x * team; item < total; item += gridDim.x * 4) {
-            if (!first) {
-                if ((thread_now() & 127) == 0) sh.later_item[team] = attention_item<QL>(sh.layer[layer & 1].kv, item);
+        for (int item = blockIdx.x + gridDim.x * team; item < total; item += gridDim.x * 4, round++) {
+            AttentionItem &later = sh.later_item[round & 1][team];
+            if (round > 0) {
+                // (last read two rounds ago: every warp of the team has arrived at the barrier between since)
+                if ((thread_now() & 127) == 0) later = attention_item<QL>(sh.layer[layer & 1].kv, item);
                 team_barrier(2 + team);
             }
-            const AttentionItem &it = first ? sh.item[team] : sh.later_item[team];
-            if (it.count > 0) attention_team_item<HD, GROUP, QL>(layer, it, first);
-            first = false;
+            const AttentionItem &it = round == 0 ? sh.item[team] : later;
+            if (it.count > 0) attention_team_item<HD, GROUP, QL>(layer, it, round == 0);
         }
     }
     cta_sync();

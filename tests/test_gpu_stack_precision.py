@@ -78,7 +78,9 @@ class _Layer:
         full = self.weight[name] * np.repeat(self.scale[name], 128, axis=1)
         return x @ full.T, np.abs(x) @ np.abs(full).T
 
-    def run(self, launch, hidden, normalised_sum=0.5):
+    def run(self, launch, hidden, normalised_sum=0.5, positions=None, pool=None, pages=1, attended=1):
+        """The residual stream and the value projections; with `pool` (a stream per lane, their pages in turn) the attention
+        outputs instead, the lanes at `positions`."""
         import torch
 
         def device(array, dtype):
@@ -96,18 +98,22 @@ class _Layer:
             keep += [device((nibbles << (4 * np.arange(8, dtype=np.uint32))).sum(-1), np.uint32).view(torch.int32), bf16(self.scale[name])]
             t.words[i], t.scales[i] = keep[-2].data_ptr(), keep[-1].data_ptr()
         named = {"input_norm": bf16(self.norm["input"]), "post_norm": bf16(self.norm["post"]), "rope": torch.full((self.head // 2,), 0x3F80, dtype=torch.int32, device="cuda"),
-                 "hidden": bf16(hidden), "pool": torch.zeros((lanes, 2, self.kv_heads, PAGE, self.head), dtype=torch.bfloat16, device="cuda"),
+                 "hidden": bf16(hidden),
+                 "pool": torch.zeros((lanes, 2, self.kv_heads, PAGE, self.head), dtype=torch.bfloat16, device="cuda") if pool is None else bf16(pool),
                  "attention_out": torch.zeros((8, self.q_heads * self.head), dtype=torch.bfloat16, device="cuda"),
-                 "table": torch.arange(lanes, dtype=torch.int32, device="cuda"), "positions": torch.zeros(lanes, dtype=torch.int32, device="cuda"),
+                 "table": torch.arange(lanes * pages, dtype=torch.int32, device="cuda"),
+                 "positions": device(np.zeros(lanes) if positions is None else np.asarray(positions), np.int32),
                  "slots": torch.arange(lanes, dtype=torch.int32, device="cuda")}
         for name, tensor in named.items():
             setattr(t, name, tensor.data_ptr())
         for name, value in (("lanes", lanes), ("lanes_per_stream", 1), ("hidden_width", self.hidden), ("q_heads", self.q_heads), ("kv_heads", self.kv_heads),
-                            ("head_width", self.head), ("ffn", self.ffn), ("page_tokens", PAGE), ("pages_per_slot", 1), ("attended", 1), ("layers", 1), ("launches", 1)):
+                            ("head_width", self.head), ("ffn", self.ffn), ("page_tokens", PAGE), ("pages_per_slot", pages), ("attended", attended), ("layers", 1), ("launches", 1)):
             setattr(t, name, value)
         t.eps, t.norm_offset, t.attention_scale = 1.0 - normalised_sum, self.offset, 1.0
         torch.cuda.synchronize()
         assert launch(ctypes.byref(t)) == 0
+        if pool is not None:
+            return named["attention_out"][:lanes].double().cpu().numpy()
         values = named["pool"][:, 1, :, 0].reshape(lanes, -1)
         return named["hidden"].double().cpu().numpy(), values.double().cpu().numpy()
 
@@ -142,3 +148,36 @@ def test_a_group_at_the_end_of_a_row_keeps_its_own_scale(launch):
     assert np.array_equal(got, hidden[:, columns] * values)
     sums, magnitudes = layer.product("o", inputs)
     _check(out[:, 256:], sums[:, 256:], magnitudes[:, 256:], "o")
+
+
+def test_work_items_without_tokens_between_others(launch):
+    """Eight streams of uneven contexts: splits are laid out for the longest, so teams meet items without tokens between ones
+    that have some.  Bar: half a bf16 unit and, for probabilities in f32 that are handed on in two bf16 parts (2^-17 each),
+    2^-15 of the magnitudes."""
+    import torch
+
+    rng = np.random.default_rng(2)
+    positions, splits = [1099, 69, 1203, 19, 499, 1150, 129, 1023], 32
+    layer = _Layer(512, 16, 8, 32, 256)
+    counts = [[max(0, min(64, position + 1 - 64 * split)) for split in range(splits)] for position in positions]
+    ctas, reached = torch.cuda.get_device_properties(0).multi_processor_count, 0
+    for team in range(4 * ctas):
+        present = [counts[item // 8 // splits][item // 8 % splits] > 0 for item in range(team, 8 * splits * 8, 4 * ctas)]  # (kv heads innermost)
+        reached += any(present[a] and not present[b] and present[c] for c in range(len(present)) for b in range(c) for a in range(b))
+    assert reached > 20
+    hidden = _hidden(rng, 8, 512)
+    values = _bf16(rng.uniform(0.5, 2.0, size=512))
+    columns = layer.single("q", values)
+    pages = splits * 64 // PAGE
+    pool = _bf16(rng.normal(size=(8 * pages, 2, 8, PAGE, 32)))
+    expected, magnitude = np.zeros((8, 16, 32)), np.zeros((8, 16, 32))
+    for m, position in enumerate(positions):
+        rows = pool[m * pages : (m + 1) * pages].transpose(1, 2, 0, 3, 4).reshape(2, 8, -1, 32)[:, :, : position + 1].copy()
+        rows[:, :, position] = 0.0  # what this layer appends
+        q = (hidden[m, columns] * values).reshape(16, 32)
+        for head in range(16):
+            scores = rows[0, head // 2] @ q[head]
+            p = np.exp(scores - scores.max())
+            expected[m, head], magnitude[m, head] = p / p.sum() @ rows[1, head // 2], p / p.sum() @ np.abs(rows[1, head // 2])
+    got = layer.run(launch, hidden, positions=positions, pool=pool, pages=pages, attended=64 * splits)
+    _check(got, expected.reshape(8, -1), 32.0 * magnitude.reshape(8, -1), "attention")
