@@ -1312,6 +1312,11 @@ __device__ __forceinline__ WarpBlocks warp_blocks(int phase, int pass, int warp)
     return b;
 }
 
+template <int TILES>
+__device__ __forceinline__ Accumulators<TILES> *carried_sums(int warp, int lane) {  // inside the warp's own part of `reduce`
+    static_assert(2 * 32 * sizeof(Accumulators<TILES>) <= sizeof(shared().reduce[0]), "a warp's carried sums fit its part");
+    return reinterpret_cast<Accumulators<TILES> *>(&shared().reduce[warp][0][0]) + 2 * lane;
+}
 // Every stage holds, for this warp, the blocks of two tiles and one group of K, multiplied by the same activations: tiles
 // 2 pair and 2 pair + 1 of the pass, group step * width + place.  Leaves the sums in `reduce` - of a window that is not
 // the pass's last, the thread's own sums, which its next window starts from.
@@ -1336,11 +1341,10 @@ __device__ __forceinline__ uint32_t consume_pass(int phase, int pass, int first_
     uint32_t x = blocks.x + (X_IN_SLICE ? at.slice_slot * x_step : 0u);
     const ProductConstants constants = product_constants();
     Accumulators<TILES> acc[2];
-    Accumulators<TILES> *carried = reinterpret_cast<Accumulators<TILES> *>(&sh.reduce[0][0][0]) + 2 * thread;
 #pragma unroll
     for (int t = 0; t < 2; t++) {
         acc[t].row[0] = acc[t].row[1] = 0;
-        if (first_step > 0) acc[t] = carried[t];
+        if (first_step > 0) acc[t] = carried_sums<TILES>(warp, lane)[t];
     }
 #pragma unroll 1
     for (int step = 0; step < steps; step++) {
@@ -1393,7 +1397,7 @@ __device__ __forceinline__ uint32_t consume_pass(int phase, int pass, int first_
     at.slice_slot = (slice_barrier - full) >> 3;
 #pragma unroll
     for (int t = 0; t < 2; t++) {
-        if (steps < left) carried[t] = acc[t];
+        if (steps < left) carried_sums<TILES>(warp, lane)[t] = acc[t];
         else store_sums<TILES>(sh.reduce[warp][t], acc[t]);
     }
     return pack_place(at);
