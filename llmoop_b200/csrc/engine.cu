@@ -723,16 +723,18 @@ Engine::Engine(std::shared_ptr<MountedModel> model) : model_(std::move(model)) {
     kernel_error_ = device_alloc(sizeof(int));
     if (options.tp_size > 1) tp_partial_ = device_alloc(lanes * static_cast<size_t>(plan.hidden) * sizeof(float));
     {
-        size_t q_width = 0, ffn = 0;
+        size_t q_width = 0, ffn = 0, hidden = 0;
         for (const StackPlan *stack : {&model_->target_stack(), &model_->draft_stack()})
             if (stack->available) {
                 q_width = std::max<size_t>(q_width, static_cast<size_t>(stack->shape.q_heads) * stack->shape.head_width);
                 ffn = std::max<size_t>(ffn, stack->shape.ffn);
+                hidden = std::max<size_t>(hidden, stack->shape.hidden);
             }
         if (q_width != 0) {
             stack_q_ = device_alloc(8 * q_width * 2);
             stack_attention_out_ = device_alloc(8 * q_width * 2);
             stack_activation_ = device_alloc(stack_activation_bytes(static_cast<int>(ffn)));
+            stack_residual_ = device_alloc(stack_residual_bytes(static_cast<int>(ffn), static_cast<int>(std::max(q_width, hidden))));
             stack_barrier_ = device_alloc(STACK_BARRIER_WORDS * sizeof(unsigned int));
             stack_timing_ = device_alloc(std::max<size_t>(1, plan.layers.size()) * 32 * sizeof(unsigned long long));
         }
@@ -752,7 +754,7 @@ Engine::~Engine() {
     for (auto &entry : signals_) cudaFree(entry.second.ptr);
     for (DeviceBuffer *buffer : {&frame_a_, &frame_b_, &embedding_out_, &normalized_, &draft_normalized_, &draft_hidden_in_, &logits_,
                                  &records_, &argmax_scratch_, &sampler_scratch_, &sampler_table_, &lane_tokens_, &lane_positions_, &lane_slots_, &pending_hidden_, &pending_backup_, &attention_scratch_, &attention_blocks_,
-                                 &cycle_state_, &int4_activations_, &moe_quantised_, &moe_quantised_scales_, &moe_groups_, &kernel_error_, &tp_partial_, &tp_exchange_, &tp_description_, &stack_q_, &stack_attention_out_, &stack_activation_, &stack_barrier_, &stack_timing_, &prefix_pending_, &page_copies_device_})
+                                 &cycle_state_, &int4_activations_, &moe_quantised_, &moe_quantised_scales_, &moe_groups_, &kernel_error_, &tp_partial_, &tp_exchange_, &tp_description_, &stack_q_, &stack_attention_out_, &stack_activation_, &stack_residual_, &stack_barrier_, &stack_timing_, &prefix_pending_, &page_copies_device_})
         cudaFree(buffer->ptr);
     cudaFreeHost(staging_);
     cudaFreeHost(host_records_);
@@ -1884,6 +1886,7 @@ bool Engine::run_stack(const StackPlan &stack, int lanes, void *hidden) {
     buffers.attention_scratch = static_cast<float *>(attention_scratch_.ptr);
     buffers.attention_out = static_cast<uint16_t *>(stack_attention_out_.ptr);
     buffers.activation = static_cast<uint8_t *>(stack_activation_.ptr);
+    buffers.residual = static_cast<uint8_t *>(stack_residual_.ptr);
     buffers.barrier = static_cast<unsigned int *>(stack_barrier_.ptr);
     buffers.error_flag = static_cast<int *>(kernel_error_.ptr);
     buffers.timing = (profile_ && &stack == &model_->target_stack()) ? static_cast<unsigned long long *>(stack_timing_.ptr) : nullptr;

@@ -400,7 +400,7 @@ private:
     bool tp_connected_ = false;
     void tp_all_reduce(float *values, size_t count);
     // persistent decode stack workspaces ([8 lanes][width]) and its two barrier words
-    DeviceBuffer stack_q_, stack_attention_out_, stack_activation_, stack_barrier_, stack_timing_;
+    DeviceBuffer stack_q_, stack_attention_out_, stack_activation_, stack_residual_, stack_barrier_, stack_timing_;
     bool stack_enabled_ = true;
     bool run_stack(const StackPlan &stack, int lanes, void *hidden);
     bool streams_apart_ = false;  // every current_width_ lanes are one stream's, no stream in two of these groups

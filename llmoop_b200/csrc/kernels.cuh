@@ -262,6 +262,7 @@ struct StackBuffers {
     float *attention_scratch;    // split partials
     uint16_t *attention_out;     // [lanes][q_heads * head_width]
     uint8_t *activation;         // [lanes][ffn] in operand form: stack_activation_bytes(ffn) bytes (see kernels_stack.cu)
+    uint8_t *residual;           // what the operand form loses where a group's values lie far apart: stack_residual_bytes(..) bytes
     unsigned int *barrier;       // STACK_BARRIER_WORDS words, zero before the first launch
     int *error_flag;             // set when a bounded wait expires (2: grid barrier or peer, 3: weight pipeline)
     unsigned long long *timing;  // optional [layers][32] nanosecond stamps of CTA 0 (step boundaries), or nullptr
@@ -302,6 +303,7 @@ size_t int4_cta_stream_bytes(int rows, int k, bool pair, int grid);
 cudaError_t launch_int4_cta_streams(const RelayoutSegment *segments, int count, bool pair, int k, int grid, uint8_t *out,
                                     cudaStream_t stream);
 size_t stack_activation_bytes(int ffn);  // of StackBuffers::activation, for any batch
+size_t stack_residual_bytes(int ffn, int widest);  // of StackBuffers::residual; `widest`: of the hidden and the query rows
 // Whether the stack kernel is built for this shape and batch; *smem_bytes receives its dynamic shared memory.
 bool decode_stack_supported(const StackShape &shape, int lanes, size_t *smem_bytes);
 cudaError_t launch_decode_stack(const StackLayer *layers_device, int layer_count, const StackShape &shape,

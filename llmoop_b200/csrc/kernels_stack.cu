@@ -15,7 +15,7 @@
 //    as far ahead as the ring allows - through the grid barriers, the attention step and the epilogues.
 //  * 16 consumer warps: a warp multiplies two tiles of 16 rows with every width-th group (128 columns) of K, so a
 //    matrix costs one cross-warp reduction and one epilogue pass per CTA instead of one per tile.  The products are
-//    integers: weights as signed bytes, activations as three signed bytes each, mma.sync m16n8k32 with exact 32-bit
+//    integers: weights as signed bytes, activations as four signed bytes each, mma.sync m16n8k32 with exact 32-bit
 //    sums (see "matrix blocks"); the group scale multiplies the group's sum in f32 as in
 //    linear_int4_ct.comp.template:80-150.
 //  * activations: the inputs of q/k/v and gate/up (rms_norm_bf16.comp.template:49-72) and of o are brought into
@@ -60,8 +60,7 @@ constexpr int STAGE_BYTES = 2 * CONSUMER_WARPS * UNIT_TOTAL;  // a step of a pas
 constexpr int MAX_STAGES = 16;
 constexpr uint32_t EMPTY = 8 * MAX_STAGES, SLICE_FULL = 16 * MAX_STAGES, SLICE_EMPTY = 24 * MAX_STAGES;  // barrier arrays, from a slot's `full`
 // Activations in operand form (see stage_rows): two halves and eight factors per group of 128 columns.
-// (an odd number of 64-byte pieces, so that the two halves of a word column fall into different banks)
-__host__ __device__ constexpr uint32_t operand_half_bytes(int lanes) { return static_cast<uint32_t>(lanes) * 192u + (lanes % 2 == 0 ? 64u : 0u); }
+__host__ __device__ constexpr uint32_t operand_half_bytes(int lanes) { return static_cast<uint32_t>(lanes) * 256u; }
 __host__ __device__ constexpr uint32_t operand_group_bytes(int lanes) { return 2u * operand_half_bytes(lanes) + 32u; }
 constexpr uint32_t PRODUCT_BYTES = 8 * 128 * sizeof(float);  // a group of SiLU products of every lane, before it takes operand form
 constexpr unsigned int BARRIER_SPIN_LIMIT = 1u << 20;
@@ -287,7 +286,7 @@ struct WarpBlocks {
     int steps;                  // steps that hold a group of the warp (0 if it has no tile)
     int tiles;                  // 1 or 2
 };
-struct OperandPlace {  // where a thread's B fragments are inside a group
+struct OperandPlace {  // where a thread's B fragments are inside a group: in the first half, and the same with the neighbour's term
     uint32_t first, second, half, factor;
 };
 
@@ -489,51 +488,102 @@ __device__ __forceinline__ void wait_barrier(uint32_t barrier, uint32_t parity) 
 }
 // ------------------------------------------------------------------------------------------ activation staging
 
-// The operand form of activations.  A group (128 columns) of a lane is held as whole numbers X of 23 bits over one
-// power of two - x = X 2^(e - 21), e the exponent of the largest magnitude of the group (of the warp's two groups where
-// rows are staged) - and X as three signed bytes,
-// X = t0 2^16 + t1 2^8 + t2: the group's products with the four-bit weights then add up exactly in 32-bit integers,
-// whatever their order, and what f32 rounds is the group's sum, as in linear_int4_ct.comp.template:80-150.  A bf16
-// value down to 2^-14 of that largest is carried exactly, a smaller one to 2^-22 of it.
+// The operand form of activations.  A group (128 columns) of a lane is held as whole numbers X of 31 bits over one
+// power of two - x = X 2^(e - 29), e the exponent of the largest magnitude of the group (of the warp's two groups where
+// rows are staged) - and X as four signed bytes, X = t0 2^24 + t1 2^16 + t2 2^8 + t3: the group's products with the four-bit
+// weights then add up exactly in 32-bit integers, whatever their order, and what f32 rounds is the group's sum, as in
+// linear_int4_ct.comp.template:80-150.  A bf16 value down to 2^-22 of that largest is carried exactly, a smaller one to
+// 2^(e - 30), which is no further off than an fp16 number (2^-25) while the largest is below 64.  A group with a larger
+// one that has values it cannot hold keeps what they lost, X' 2^(e - 59), in the same form in global memory
+// (StackBuffers::residual); its factor and its digits are negative, and add_residuals multiplies the rest.  (With three
+// bytes the rows without a weight on a large column were off by 1e-2 of a group's sum where it was 10000 beside N(0, 1)
+// products times 0.05.  The fourth byte is free up to four lanes - the MMA's columns were there - and costs a fourth column
+// tile from five on.)
 //
 // A group takes operand_group_bytes(lanes) bytes: [half h][lane][term t][j] pieces of 16 bytes (the B fragments of
 // MMAs 2h and 2h + 1 for thread column j: the digits of the eight columns of word 4j + 2h, even columns first, then
-// those of word 4j + 2h + 1), then one f32 factor per lane, what a unit of t2 times a weight of one is worth.
-__device__ __forceinline__ uint32_t operand_word_offset(int word, int m, int lanes) {  // of term 0; term t is 64 t further
-    return static_cast<uint32_t>((word >> 1) & 1) * operand_half_bytes(lanes) + static_cast<uint32_t>(m) * 192u + static_cast<uint32_t>(word >> 2) * 16u +
+// those of word 4j + 2h + 1; where lane + h is odd the terms are in the order 1, 0, 3, 2, so that a term of two neighbours falls
+// into different banks), then one f32 factor per lane, what a unit of t3 times a weight of one is worth.
+__device__ __forceinline__ uint32_t operand_word_offset(int word, int m, int lanes) {  // of the lane's terms
+    return static_cast<uint32_t>((word >> 1) & 1) * operand_half_bytes(lanes) + static_cast<uint32_t>(m) * 256u + static_cast<uint32_t>(word >> 2) * 16u +
            static_cast<uint32_t>(word & 1) * 8u;
 }
-// From the exponent field of a group's largest magnitude: the factor onto X, and the group's factor (2^-4 of it since
+__host__ __device__ constexpr uint32_t term_offset(int term, int lane_and_half) { return static_cast<uint32_t>(term ^ (lane_and_half & 1)) * 64u; }
+// From the exponent field of a group's largest magnitude: the factor onto X / 2^8, and the group's factor (2^-4 of a unit since
 // the MMA sees sixteen times the weights).  A group that holds an infinity or a NaN makes its sums NaN.
-__device__ __forceinline__ float operand_scale(uint32_t exponent) { return __uint_as_float((275u - (exponent < 32u ? 32u : exponent)) << 23); }
+__device__ __forceinline__ float operand_scale(uint32_t exponent) { return __uint_as_float((275u - (exponent < 40u ? 40u : exponent)) << 23); }
 __device__ __forceinline__ float operand_factor(uint32_t exponent) {
-    return __uint_as_float(exponent == 255u ? 0x7fc00000u : ((exponent < 32u ? 32u : exponent) - 25u) << 23);
+    return __uint_as_float(exponent == 255u ? 0x7fc00000u : ((exponent < 40u ? 40u : exponent) - 33u) << 23);
 }
-// The digits of four whole numbers as three words (term 0 first).  A number comes as the bits of 1.5 * 2^23 + X, which
-// is how f32 rounds to whole numbers; 2^7 in front of each digit makes its byte unsigned, so that no digit borrows from
-// the next.  (The additions are multiply-adds by an opaque one: they leave the half-rate integer pipe to the permutes.)
+__device__ __forceinline__ bool operand_may_lose(uint32_t exponent) { return exponent >= 133u && exponent != 255u; }  // (133: 64)
+constexpr float RESIDUAL_SCALE = 4194304.0f, RESIDUAL_UNIT = 0x1p-30f;  // what is left in units of t3, onto X' / 2^8; the factors' ratio
+// A pair of values as X + 0x00808080: 2^7 in front of the lower digits makes their bytes unsigned, so that no digit borrows from
+// the next.  f32 rounds to whole numbers where it is 1.5 * 2^23 + X; it does so for X / 2^8, then for the 2^8 of what is left.
+// (Additions of integers are multiply-adds by an opaque one: they leave the half-rate integer pipe to the permutes.)
 struct DigitConstants {  // made where they are used: the compiler would keep them in registers through the whole layer
-    uint32_t one, digits;
-    unsigned long long bias;  // a pair
+    uint32_t one, byte, digits;
+    unsigned long long bias, minus, byte_pair;  // pairs
 };
 __device__ __forceinline__ DigitConstants digit_constants() {
     DigitConstants c;
     asm volatile("mov.b32 %0, 1;" : "=r"(c.one));
-    asm volatile("mov.b32 %0, 0x00408080;" : "=r"(c.digits));
+    asm volatile("mov.b32 %0, 256;" : "=r"(c.byte));
+    asm volatile("mov.b32 %0, 0x75408080;" : "=r"(c.digits));  // 0x00808080 - 2^8 0x4B400000 - 0x4B400000
     asm volatile("mov.b64 %0, 0x4B4000004B400000;" : "=l"(c.bias));
+    asm volatile("mov.b64 %0, 0xBF800000BF800000;" : "=l"(c.minus));
+    asm volatile("mov.b64 %0, 0x4380000043800000;" : "=l"(c.byte_pair));
     return c;
 }
-__device__ __forceinline__ void operand_digits(uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3, const DigitConstants &c, uint32_t (&terms)[3]) {
-    const uint32_t y0 = x0 * c.one + c.digits, y1 = x1 * c.one + c.digits, y2 = x2 * c.one + c.digits, y3 = x3 * c.one + c.digits;
-    const uint32_t low01 = __byte_perm(y0, y1, 0x5140), low23 = __byte_perm(y2, y3, 0x5140);
-    terms[0] = __byte_perm(__byte_perm(y0, y1, 0x0062), __byte_perm(y2, y3, 0x0062), 0x5410) ^ 0x80808080u;
-    terms[1] = __byte_perm(low01, low23, 0x7632) ^ 0x80808080u;
-    terms[2] = __byte_perm(low01, low23, 0x5410) ^ 0x80808080u;
+// `left`: what X leaves of the values, in units of X.
+__device__ __forceinline__ void operand_wholes(unsigned long long x, unsigned long long scales, const DigitConstants &c, uint32_t &first, uint32_t &second, unsigned long long &left) {
+    const unsigned long long high = pair_fma(x, scales, c.bias), rest = pair_fma(x, scales, pair_fma(high, c.minus, c.bias)), low = pair_fma(rest, c.byte_pair, c.bias);
+    left = pair_fma(rest, c.byte_pair, pair_fma(low, c.minus, c.bias));
+    first = static_cast<uint32_t>(high) * c.byte + (static_cast<uint32_t>(low) * c.one + c.digits);
+    second = static_cast<uint32_t>(high >> 32) * c.byte + (static_cast<uint32_t>(low >> 32) * c.one + c.digits);
 }
+// The digits of four whole numbers as four words (term 0 first).
+__device__ __forceinline__ void operand_digits(uint32_t y0, uint32_t y1, uint32_t y2, uint32_t y3, uint32_t (&terms)[4]) {
+    const uint32_t low01 = __byte_perm(y0, y1, 0x5140), low23 = __byte_perm(y2, y3, 0x5140), high01 = __byte_perm(y0, y1, 0x7362), high23 = __byte_perm(y2, y3, 0x7362);
+    terms[0] = __byte_perm(high01, high23, 0x7632);
+    terms[1] = __byte_perm(high01, high23, 0x5410) ^ 0x80808080u;
+    terms[2] = __byte_perm(low01, low23, 0x7632) ^ 0x80808080u;
+    terms[3] = __byte_perm(low01, low23, 0x5410) ^ 0x80808080u;
+}
+__device__ __forceinline__ uint32_t operand_negative(uint32_t y) { return 0x01010100u - y; }
 __device__ __forceinline__ uint32_t larger_halves(uint32_t a, uint32_t b) {
     uint32_t v;
     asm("max.u16x2 %0, %1, %2;" : "=r"(v) : "r"(a), "r"(b));
     return v;
+}
+
+// What the four bytes lose of a thread's eight columns (see the operand form); by the sixteen threads of a group together.
+// `place`: its pieces in shared memory, already written; `residual`: those in the residual's group.
+__device__ __noinline__ void keep_residual(uint4 raw, uint32_t exponent, int lane_and_half, uint8_t *place, uint8_t *residual, float *factor) {
+    const DigitConstants c = digit_constants();
+    const float scale = operand_scale(exponent);
+    const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w}, half_warp = 0xffffu << (thread_now() & 16);
+    uint32_t whole[4][2], terms[2][4];
+    unsigned long long left[4];
+    bool lost = false;
+#pragma unroll
+    for (int w = 0; w < 4; w++) {
+        operand_wholes(pair_of(bf16_lo(words[w]), bf16_hi(words[w])), pair_of(scale, scale), c, whole[w][0], whole[w][1], left[w]);
+        lost |= ((left[w] | (left[w] >> 32)) & 0x7fffffffu) != 0;
+    }
+    if (!__any_sync(half_warp, lost)) return;
+#pragma unroll
+    for (int w = 0; w < 4; w++) whole[w][0] = operand_negative(whole[w][0]), whole[w][1] = operand_negative(whole[w][1]);
+#pragma unroll
+    for (int i = 0; i < 2; i++) operand_digits(whole[0][i], whole[1][i], whole[2][i], whole[3][i], terms[i]);
+#pragma unroll
+    for (int t = 0; t < 4; t++) *reinterpret_cast<uint2 *>(place + term_offset(t, lane_and_half)) = make_uint2(terms[0][t], terms[1][t]);
+    if (factor != nullptr) *factor = -operand_factor(exponent);
+#pragma unroll
+    for (int w = 0; w < 4; w++) operand_wholes(left[w], pair_of(RESIDUAL_SCALE, RESIDUAL_SCALE), c, whole[w][0], whole[w][1], left[w]);
+#pragma unroll
+    for (int i = 0; i < 2; i++) operand_digits(whole[0][i], whole[1][i], whole[2][i], whole[3][i], terms[i]);
+#pragma unroll
+    for (int t = 0; t < 4; t++) *reinterpret_cast<uint2 *>(residual + term_offset(t, lane_and_half)) = make_uint2(terms[0][t], terms[1][t]);  // (every CTA writes the same)
 }
 
 // Rows into operand form, groups [first_group, first_group + groups) of them: with `weight` their rms_norm
@@ -547,7 +597,6 @@ __device__ __forceinline__ void stage_rows(const uint16_t *x, const uint16_t *we
     float *partial = shared().norm_partial;
     const int lanes = sh.a.lanes, per_lane = width >> 3, thread = thread_now(), warp = thread >> 5, lane = thread & 31;
     const float eps = sh.a.shape.eps, offset = sh.a.shape.norm_offset;
-    const DigitConstants constants = digit_constants();
     const uint4 *source = reinterpret_cast<const uint4 *>(x);
     uint4 scale_words[CHUNKS];
 #pragma unroll
@@ -651,24 +700,32 @@ __device__ __forceinline__ void stage_rows(const uint16_t *x, const uint16_t *we
             if (chunk < per_lane && group >= 0 && group < groups) {
                 const int word = chunk & 15;
                 uint8_t *block = operands + static_cast<uint32_t>(group) * operand_group_bytes(lanes), *place = block + operand_word_offset(word, m0, lanes);
+                const uint32_t flip = (word & 2) * 32;
+                uint8_t *const pieces[2] = {place + flip, place - flip};  // even and odd ones
+                const DigitConstants constants = digit_constants();
 #pragma unroll
                 for (int mm = 0; mm < LANES; mm++) {
                     if (m0 + mm >= lanes) break;
                     const float scale = operand_scale(largest[mm]);
                     const unsigned long long scales = pair_of(scale, scale);
                     const uint32_t words[4] = {raw[mm][c].x, raw[mm][c].y, raw[mm][c].z, raw[mm][c].w};
-                    uint32_t whole[4][2], even[3], odd[3];
+                    uint32_t whole[4][2], even[4], odd[4];
 #pragma unroll
                     for (int w = 0; w < 4; w++) {
-                        const unsigned long long v = pair_fma(pair_of(bf16_lo(words[w]), bf16_hi(words[w])), scales, constants.bias);
-                        whole[w][0] = static_cast<uint32_t>(v);
-                        whole[w][1] = static_cast<uint32_t>(v >> 32);
+                        unsigned long long left;
+                        operand_wholes(pair_of(bf16_lo(words[w]), bf16_hi(words[w])), scales, constants, whole[w][0], whole[w][1], left);
                     }
-                    operand_digits(whole[0][0], whole[1][0], whole[2][0], whole[3][0], constants, even);
-                    operand_digits(whole[0][1], whole[1][1], whole[2][1], whole[3][1], constants, odd);
+                    operand_digits(whole[0][0], whole[1][0], whole[2][0], whole[3][0], even);
+                    operand_digits(whole[0][1], whole[1][1], whole[2][1], whole[3][1], odd);
 #pragma unroll
-                    for (int t = 0; t < 3; t++) *reinterpret_cast<uint2 *>(place + 192 * mm + 64 * t) = make_uint2(even[t], odd[t]);
-                    if (word == 0) *reinterpret_cast<float *>(block + 2 * operand_half_bytes(lanes) + 4 * (m0 + mm)) = operand_factor(largest[mm]);
+                    for (int t = 0; t < 4; t++) *reinterpret_cast<uint2 *>(pieces[(t + mm) & 1] + 256 * mm + term_offset(t, mm)) = make_uint2(even[t], odd[t]);  // (m0 is even)
+                    float *factor = word == 0 ? reinterpret_cast<float *>(block + 2 * operand_half_bytes(lanes) + 4 * (m0 + mm)) : nullptr;
+                    if (factor != nullptr) *factor = operand_factor(largest[mm]);
+                    if (operand_may_lose(largest[mm]))
+                        keep_residual(raw[mm][c], largest[mm], mm + (word >> 1), place + 256 * mm,
+                                      sh.a.buffers.residual + static_cast<size_t>((sh.a.shape.ffn >> 7) + (chunk >> 4)) * operand_group_bytes(lanes) +
+                                          operand_word_offset(word, m0 + mm, lanes),
+                                      factor);
                 }
             }
         }
@@ -685,27 +742,37 @@ __device__ __forceinline__ void stage_any(const uint16_t *x, const uint16_t *wei
     return narrow ? stage_rows<1, LANES>(x, weight, width, first_group, groups) : stage_rows<2, 2>(x, weight, width, first_group, groups);
 }
 
-// A group's 128 columns of one lane (f32 in shared memory) into operand form in global memory, by one warp.  The products of
-// SiLU and up have a heavy tail: X has a bit more here (e - 22), which the three digits hold unless the largest mantissa is
-// about the greatest there is; such a group takes the next exponent.  (Against 64 bits, 14336 columns of rounded SiLU
-// products, gates and ups of 1.28 N(0, 1): RMS 9.1e-8 of the output without that bit, 8.5e-8 with it and with the fp16
-// operands and f32 sums this form replaced; 2176 columns 7.1e-8, 5.7e-8 and 6.0e-8.  Normalised rows: 6.4e-8 each.)
-__device__ __forceinline__ void store_operand_group(uint8_t *block, const float *columns, int m, int lanes) {
+// A group's 128 columns of one lane (bf16 values as f32 in shared memory) into operand form in global memory, by one warp.
+__device__ __forceinline__ void store_operand_group(uint8_t *block, uint8_t *residual, const float *columns, int m, int lanes) {
     const int lane = thread_now() & 31, word = lane >> 1, odd = lane & 1;
+    const DigitConstants c = digit_constants();
     float v[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) v[i] = columns[word * 8 + odd + 2 * i];
-    const uint32_t largest = __reduce_max_sync(0xffffffffu, max(max(__float_as_uint(v[0]) & 0x7fffffffu, __float_as_uint(v[1]) & 0x7fffffffu),
-                                                                max(__float_as_uint(v[2]) & 0x7fffffffu, __float_as_uint(v[3]) & 0x7fffffffu)));
-    const uint32_t exponent = max((largest + 0x18000u) >> 23, 32u);  // (above 1.988 x 2^e: the next one)
-    uint32_t terms[3], whole[4];
-    const float scale = __uint_as_float((276u - min(exponent, 255u)) << 23), factor = __uint_as_float(largest >= 0x7f800000u ? 0x7fc00000u : (exponent - 26u) << 23);
+    const uint32_t exponent = __reduce_max_sync(0xffffffffu, max(max(__float_as_uint(v[0]) & 0x7fffffffu, __float_as_uint(v[1]) & 0x7fffffffu),
+                                                                 max(__float_as_uint(v[2]) & 0x7fffffffu, __float_as_uint(v[3]) & 0x7fffffffu))) >> 23;
+    const float scale = operand_scale(exponent);
+    float factor = operand_factor(exponent);
+    uint32_t terms[4], whole[4];
+    unsigned long long left[2];
 #pragma unroll
-    for (int i = 0; i < 4; i++) whole[i] = 0x4B400000u + static_cast<uint32_t>(__float2int_rn(v[i] * scale));
-    operand_digits(whole[0], whole[1], whole[2], whole[3], digit_constants(), terms);
-    uint8_t *place = block + operand_word_offset(word, m, lanes) + 4 * odd;
+    for (int i = 0; i < 2; i++) operand_wholes(pair_of(v[2 * i], v[2 * i + 1]), pair_of(scale, scale), c, whole[2 * i], whole[2 * i + 1], left[i]);
+    const uint32_t at = operand_word_offset(word, m, lanes) + 4 * odd;
+    const unsigned long long any = (left[0] | left[1]) & 0x7fffffff7fffffffull;
+    if (operand_may_lose(exponent) && __any_sync(0xffffffffu, any != 0)) {
+        factor = -factor;
 #pragma unroll
-    for (int t = 0; t < 3; t++) *reinterpret_cast<uint32_t *>(place + 64 * t) = terms[t];
+        for (int i = 0; i < 4; i++) whole[i] = operand_negative(whole[i]);
+        uint32_t rest[4];
+#pragma unroll
+        for (int i = 0; i < 2; i++) operand_wholes(left[i], pair_of(RESIDUAL_SCALE, RESIDUAL_SCALE), c, rest[2 * i], rest[2 * i + 1], left[i]);
+        operand_digits(rest[0], rest[1], rest[2], rest[3], terms);
+#pragma unroll
+        for (int t = 0; t < 4; t++) *reinterpret_cast<uint32_t *>(residual + at + term_offset(t, m + (word >> 1))) = terms[t];
+    }
+    operand_digits(whole[0], whole[1], whole[2], whole[3], terms);
+#pragma unroll
+    for (int t = 0; t < 4; t++) *reinterpret_cast<uint32_t *>(block + at + term_offset(t, m + (word >> 1))) = terms[t];
     if (lane == 0) *reinterpret_cast<float *>(block + 2 * operand_half_bytes(lanes) + 4 * m) = factor;
 }
 
@@ -1172,23 +1239,23 @@ struct AttentionTeam {
 // ------------------------------------------------------------------------------------------ matrix blocks
 // A 16x128 block times the lanes of a batch, as signed bytes: the packed weights are q - 8 in two's complement, so a
 // nibble in the upper half of its byte is sixteen times the weight (one AND for eight weights, a shift in front for
-// the other eight), and an activation is three bytes (see the operand form).  Up to two lanes have their terms in
-// the eight columns of one MMA, up to four in two, up to eight in three:
-//   TILES 1: column 4 lane + term;  TILES 2: tile 0 column 2 lane + term (0, 1), tile 1 column 2 lane (term 2);
-//   TILES 3: tile `term`, column `lane`.
+// the other eight), and an activation is four bytes (see the operand form).  Up to two lanes have their terms in
+// the eight columns of one MMA, up to four in two, up to eight in four:
+//   TILES 1: column 4 lane + term;  TILES 2: tile 0 column 2 lane + term (0, 1), tile 1 column 2 lane + term - 2;
+//   TILES 4: tile `term`, column `lane`.
 // Why integers: with exact fp16 operands (q - 8) and per-group f32 sums a block cost 72 instructions of dequantisation
 // (nine for eight nibbles, most at half rate) and eight MMAs; here 24 and 4 TILES, mma.sync taking 32 bytes of K at the
 // rate of 16 fp16.  The accumulators start at 1.5 * 2^23 as an integer, which is the f32 of 1.5 * 2^23 + the sum.
 constexpr float SUM_BIAS_F32 = 12582912.0f;
 
 // f32 sums of a thread over its groups: rows g and g + 8 of one lane (TILES 1: of lane j / 2 in the even thread columns,
-// TILES 2: of lane j), or of lanes 2j and 2j + 1 as a pair (TILES 3).
+// TILES 2: of lane j), or of lanes 2j and 2j + 1 as a pair (TILES 4).
 template <int TILES>
 struct Accumulators {
     float row[2];
 };
 template <>
-struct Accumulators<3> {
+struct Accumulators<4> {
     unsigned long long row[2];
 };
 template <int TILES>
@@ -1196,15 +1263,21 @@ struct ActivationOperands {
     uint4 b[TILES][2];
     float factor[2];
 };
-template <int TILES>
-__device__ __forceinline__ void load_activations(ActivationOperands<TILES> &x, uint32_t group, const OperandPlace &place) {
+// `load16(offset)`: of the group's pieces.
+template <int TILES, class Load>
+__device__ __forceinline__ void load_pieces(ActivationOperands<TILES> &x, const OperandPlace &place, const Load &load16) {
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-        x.b[0][h] = smem16(group + place.first + h * place.half);
-        if (TILES == 2) x.b[TILES - 1][h] = smem16(group + place.second + h * place.half);
-        if (TILES == 3) x.b[TILES > 1 ? 1 : 0][h] = smem16(group + place.first + h * place.half + 64), x.b[TILES - 1][h] = smem16(group + place.first + h * place.half + 128);
+        const uint32_t first = (h == 0 ? place.first : place.second) + h * place.half, second = (h == 0 ? place.second : place.first) + h * place.half;
+        x.b[0][h] = load16(first);
+        if (TILES == 2) x.b[TILES - 1][h] = load16(first + 128);
+        if (TILES == 4) x.b[TILES > 1 ? 1 : 0][h] = load16(second), x.b[TILES > 2 ? 2 : 0][h] = load16(first + 128), x.b[TILES - 1][h] = load16(second + 128);
     }
-    if (TILES == 3) {
+}
+template <int TILES>
+__device__ __forceinline__ void load_activations(ActivationOperands<TILES> &x, uint32_t group, const OperandPlace &place) {
+    load_pieces<TILES>(x, place, [&](uint32_t offset) { return smem16(group + offset); });
+    if (TILES == 4) {
         const float2 both = *reinterpret_cast<const float2 *>(smem_raw + group + place.factor);
         x.factor[0] = both.x, x.factor[1] = both.y;
     } else {
@@ -1215,21 +1288,22 @@ __device__ __forceinline__ void load_activations(ActivationOperands<TILES> &x, u
 struct ProductConstants {
     int32_t bias;
     uint32_t sixteen;  // a multiplication goes to the FMA pipe: AND and shift share a pipe of half the rate
-    unsigned long long unbias, term0, term1;  // pairs
+    unsigned long long unbias, term0, term1, term2;  // pairs
 };
 __device__ __forceinline__ ProductConstants product_constants() {
     ProductConstants c;
     asm volatile("mov.b32 %0, 0x4B400000;" : "=r"(c.bias));
     asm volatile("mov.b32 %0, 16;" : "=r"(c.sixteen));
     asm volatile("mov.b64 %0, 0xCB400000CB400000;" : "=l"(c.unbias));
-    asm volatile("mov.b64 %0, 0x4780000047800000;" : "=l"(c.term0));
-    asm volatile("mov.b64 %0, 0x4380000043800000;" : "=l"(c.term1));
+    asm volatile("mov.b64 %0, 0x4B8000004B800000;" : "=l"(c.term0));
+    asm volatile("mov.b64 %0, 0x4780000047800000;" : "=l"(c.term1));
+    asm volatile("mov.b64 %0, 0x4380000043800000;" : "=l"(c.term2));
     return c;
 }
 // BLOCKS blocks (of different tiles) against the same activations, their chains of MMAs side by side.
 template <int TILES, int BLOCKS>
-__device__ __forceinline__ void block_products(const uint4 (&rows)[2][2], const uint32_t (&scales)[2], const ActivationOperands<TILES> &x, const ProductConstants &c,
-                                               Accumulators<TILES> (&acc)[2]) {
+__device__ __forceinline__ void block_products(uint4 (*rows)[2], const uint32_t *scales, const ActivationOperands<TILES> &x, const ProductConstants &c,
+                                               Accumulators<TILES> *acc) {
     int32_t sums[BLOCKS][TILES][4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
@@ -1248,29 +1322,29 @@ __device__ __forceinline__ void block_products(const uint4 (&rows)[2][2], const 
             }
         }
     }
-    // the group's sum t0 2^16 + t1 2^8 + t2, rounded to f32 once (but for the last bits of t1 2^8 + t2), times the scale
+    // the group's sum t0 2^24 + t1 2^16 + t2 2^8 + t3, rounded to f32 (the lower terms' roundings are below that of what they
+    // join, unless it is zero), times the scale
 #pragma unroll
     for (int b = 0; b < BLOCKS; b++) {
         const float scale[2] = {__uint_as_float(scales[b] << 16), __uint_as_float(scales[b] & 0xffff0000u)};
-        if constexpr (TILES == 3) {
+        if constexpr (TILES == 4) {
             const unsigned long long factors = pair_of(x.factor[0], x.factor[1]);
 #pragma unroll
             for (int r = 0; r < 2; r++) {
-                unsigned long long term[3];
+                unsigned long long term[4];
 #pragma unroll
-                for (int t = 0; t < 3; t++) term[t] = pair_add(pair_of(__int_as_float(sums[b][t][2 * r]), __int_as_float(sums[b][t][2 * r + 1])), c.unbias);
-                const unsigned long long sum = pair_fma(term[0], c.term0, pair_fma(term[1], c.term1, term[2]));
+                for (int t = 0; t < 4; t++) term[t] = pair_add(pair_of(__int_as_float(sums[b][t][2 * r]), __int_as_float(sums[b][t][2 * r + 1])), c.unbias);
+                const unsigned long long sum = pair_fma(term[0], c.term0, pair_fma(term[1], c.term1, pair_fma(term[2], c.term2, term[3])));
                 acc[b].row[r] = pair_fma(pair_multiply(factors, pair_of(scale[r], scale[r])), sum, acc[b].row[r]);
             }
         } else {
 #pragma unroll
             for (int r = 0; r < 2; r++) {
-                float term[3];
-                term[0] = __int_as_float(sums[b][0][2 * r]) - SUM_BIAS_F32;
-                term[1] = __int_as_float(sums[b][0][2 * r + 1]) - SUM_BIAS_F32;
-                if constexpr (TILES == 1) term[2] = __shfl_down_sync(0xffffffffu, term[0], 1);  // term 2 sits one thread column further
-                else term[2] = __int_as_float(sums[b][TILES - 1][2 * r]) - SUM_BIAS_F32;
-                acc[b].row[r] = fmaf(scale[r] * x.factor[0], fmaf(term[0], 65536.0f, fmaf(term[1], 256.0f, term[2])), acc[b].row[r]);
+                const float first = __int_as_float(sums[b][0][2 * r]) - SUM_BIAS_F32, second = __int_as_float(sums[b][0][2 * r + 1]) - SUM_BIAS_F32;
+                float low;  // of terms 2 and 3, which TILES 1 has one thread column further
+                if constexpr (TILES == 1) low = __shfl_down_sync(0xffffffffu, fmaf(first, 256.0f, second), 1);
+                else low = fmaf(__int_as_float(sums[b][TILES - 1][2 * r]) - SUM_BIAS_F32, 256.0f, __int_as_float(sums[b][TILES - 1][2 * r + 1]) - SUM_BIAS_F32);
+                acc[b].row[r] = fmaf(scale[r] * x.factor[0], fmaf(first, 16777216.0f, fmaf(second, 65536.0f, low)), acc[b].row[r]);
             }
         }
     }
@@ -1282,13 +1356,12 @@ __device__ __forceinline__ void store_sums(float *sums, const Accumulators<TILES
 #pragma unroll
     for (int r = 0; r < 2; r++) {
         float *row = sums + (g + 8 * r) * 8;
-        if constexpr (TILES == 3) *reinterpret_cast<unsigned long long *>(row + 2 * j) = acc.row[r];
+        if constexpr (TILES == 4) *reinterpret_cast<unsigned long long *>(row + 2 * j) = acc.row[r];
         else if (TILES == 2) row[j] = acc.row[r];
         else if ((j & 1) == 0) row[j >> 1] = acc.row[r];
     }
 }
 
-// The steps of one pass (or of one window of it) as a warp sees them.  Offsets are from the start of shared memory.
 // Where the warps stand in the two rings, in one word: slot, slice slot, and the parities of both.
 struct RingPlace {
     uint32_t slot, parity, slice_slot, slice_parity;
@@ -1317,11 +1390,79 @@ __device__ __forceinline__ Accumulators<TILES> *carried_sums(int warp, int lane)
     static_assert(2 * 32 * sizeof(Accumulators<TILES>) <= sizeof(shared().reduce[0]), "a warp's carried sums fit its part");
     return reinterpret_cast<Accumulators<TILES> *>(&shared().reduce[warp][0][0]) + 2 * lane;
 }
+// The sign bit of a thread's factors: a group of its lanes has a residual.  `second`: the mask of the second lane's (TILES 4).
+__device__ __forceinline__ uint32_t second_lane_mask() { return 2 * (thread_now() & 3) + 1 < shared().a.lanes ? 0x80000000u : 0u; }
+template <int TILES>
+__device__ __forceinline__ uint32_t factor_signs(const float (&factor)[2], uint32_t second) {
+    return TILES == 4 ? __float_as_uint(factor[0]) | (__float_as_uint(factor[1]) & second) : __float_as_uint(factor[0]);
+}
+
+// The residuals of the warp's groups (see the operand form) times their weights, read again from the stream in global memory,
+// onto the sums of a pass (or of a window of it).  A lane's value does not depend on which other lanes have one.
+template <int TILES>
+__device__ __noinline__ void add_residuals(int phase, int layer, int pass, int first_step, bool carry) {
+    StackShared &sh = shared();
+    const int thread = thread_now(), warp = thread >> 5, lane = thread & 31;
+    const PhaseInfo &pi = sh.info[phase];
+    const WarpBlocks blocks = warp_blocks(phase, pass, warp);
+    const OperandPlace place = sh.operand_place[lane];
+    const uint32_t group_bytes = operand_group_bytes(sh.a.lanes), stage = static_cast<uint32_t>(stage_present(pi, pass) * pi.width * UNIT_TOTAL);
+    const uint8_t *stream = layer_stream(sh.layer[layer & 1], phase) + pi.cta_offset + static_cast<size_t>(pass) * pi.slots * pi.width * pi.steps * UNIT_TOTAL + (blocks.unit - sh.ring);
+    const uint8_t *residuals = sh.a.buffers.residual + (phase == 3 ? 0 : static_cast<size_t>(sh.a.shape.ffn >> 7) * group_bytes);
+    const int last = first_step + pi.window < blocks.steps ? first_step + pi.window : blocks.steps;
+    const ProductConstants constants = product_constants();
+    const uint32_t second = second_lane_mask();
+    Accumulators<TILES> acc[2];
+    acc[0].row[0] = acc[0].row[1] = acc[1].row[0] = acc[1].row[1] = 0;
+    for (int step = first_step; step < last; step++) {
+        const size_t group = static_cast<size_t>(step * pi.width + (warp & (pi.width - 1))) * group_bytes;
+        ActivationOperands<TILES> x;
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const uint32_t at = place.factor + (TILES == 4 ? 4u * i : 0u);
+            x.factor[i] = phase == 3 ? __ldcg(reinterpret_cast<const float *>(sh.a.buffers.activation + group + at))
+                                     : *reinterpret_cast<const float *>(smem_raw + blocks.x + static_cast<uint32_t>(step - first_step) * blocks.x_step + at);
+        }
+        if (!__any_sync(0xffffffffu, factor_signs<TILES>(x.factor, second) >> 31)) continue;
+#pragma unroll
+        for (int i = 0; i < 2; i++) x.factor[i] = __float_as_uint(x.factor[i]) >> 31 ? -x.factor[i] * RESIDUAL_UNIT : 0.0f;  // (NaN is positive)
+        load_pieces<TILES>(x, place, [&](uint32_t offset) { return __ldcg(reinterpret_cast<const uint4 *>(residuals + group + offset)); });
+        for (int t = 0; t < blocks.tiles; t++) {
+            const uint8_t *unit = stream + static_cast<size_t>(step) * stage + t * blocks.next_tile;
+            uint4 rows[1][2] = {{__ldg(reinterpret_cast<const uint4 *>(unit) + lane), __ldg(reinterpret_cast<const uint4 *>(unit) + 32 + lane)}};
+            const uint32_t scales[1] = {__ldg(reinterpret_cast<const uint32_t *>(stream + static_cast<size_t>(step) * stage + blocks.scales + t * (blocks.next_tile / 32u)) + (lane >> 2))};
+            block_products<TILES, 1>(rows, scales, x, constants, acc + t);
+        }
+    }
+    for (int t = 0; t < 2; t++) {
+        if (carry) {
+            Accumulators<TILES> &sums = carried_sums<TILES>(warp, lane)[t];
+            for (int r = 0; r < 2; r++) {
+                if constexpr (TILES == 4) sums.row[r] = pair_add(sums.row[r], acc[t].row[r]);
+                else sums.row[r] += acc[t].row[r];
+            }
+            continue;
+        }
+        const int g = lane >> 2, j = lane & 3;  // as store_sums
+        for (int r = 0; r < 2; r++) {
+            float *row = sh.reduce[warp][t] + (g + 8 * r) * 8;
+            if constexpr (TILES == 4) {
+                unsigned long long *both = reinterpret_cast<unsigned long long *>(row + 2 * j);
+                *both = pair_add(*both, acc[t].row[r]);
+            } else if (TILES == 2) {
+                row[j] += acc[t].row[r];
+            } else if ((j & 1) == 0) {
+                row[j >> 1] += acc[t].row[r];
+            }
+        }
+    }
+}
+
 // Every stage holds, for this warp, the blocks of two tiles and one group of K, multiplied by the same activations: tiles
 // 2 pair and 2 pair + 1 of the pass, group step * width + place.  Leaves the sums in `reduce` - of a window that is not
 // the pass's last, the thread's own sums, which its next window starts from.
 template <int TILES, bool X_IN_SLICE>
-__device__ __forceinline__ uint32_t consume_pass(int phase, int pass, int first_step) {
+__device__ __forceinline__ uint32_t consume_pass(int phase, int layer, int pass, int first_step) {
     StackShared &sh = shared();
     const int thread = thread_now(), warp = thread >> 5, lane = thread & 31;
     const int left = sh.info[phase].steps - first_step, window = sh.info[phase].window, steps = left < window ? left : window;
@@ -1340,6 +1481,8 @@ __device__ __forceinline__ uint32_t consume_pass(int phase, int pass, int first_
     uint32_t unit = blocks.unit + static_cast<uint32_t>(lane) * 16u + at.slot * static_cast<uint32_t>(STAGE_BYTES);
     uint32_t x = blocks.x + (X_IN_SLICE ? at.slice_slot * x_step : 0u);
     const ProductConstants constants = product_constants();
+    uint32_t signs = 0;
+    const uint32_t second = TILES == 4 ? second_lane_mask() : 0u;
     Accumulators<TILES> acc[2];
 #pragma unroll
     for (int t = 0; t < 2; t++) {
@@ -1358,11 +1501,17 @@ __device__ __forceinline__ uint32_t consume_pass(int phase, int pass, int first_
             rows[0][1] = smem16(unit + 512);
             row_scales[0] = smem4(unit + scales_from_unit);
             load_activations<TILES>(operands, x, place);
+            signs |= factor_signs<TILES>(operands.factor, second);
             if (tiles > 1) {
                 rows[1][0] = smem16(unit + next_tile);
                 rows[1][1] = smem16(unit + next_tile + 512);
                 row_scales[1] = smem4(unit + scales_from_unit + next_tile / 32u);
-                block_products<TILES, 2>(rows, row_scales, operands, constants, acc);
+                if constexpr (TILES == 4) {  // (four chains each; the sums of both would not fit the registers)
+                    block_products<TILES, 1>(rows, row_scales, operands, constants, acc);
+                    block_products<TILES, 1>(rows + 1, row_scales + 1, operands, constants, acc + 1);
+                } else {
+                    block_products<TILES, 2>(rows, row_scales, operands, constants, acc);
+                }
             } else {
                 block_products<TILES, 1>(rows, row_scales, operands, constants, acc);
             }
@@ -1400,6 +1549,7 @@ __device__ __forceinline__ uint32_t consume_pass(int phase, int pass, int first_
         if (steps < left) carried_sums<TILES>(warp, lane)[t] = acc[t];
         else store_sums<TILES>(sh.reduce[warp][t], acc[t]);
     }
+    if (__any_sync(0xffffffffu, signs >> 31)) add_residuals<TILES>(phase, layer, pass, first_step, steps < left);
     return pack_place(at);
 }
 
@@ -1433,7 +1583,7 @@ __device__ __forceinline__ void matrix_step(int phase, int layer) {
             if (((thread >> 1) & 7) < sh.a.lanes && (thread >> 7) < stage_present(sh.info[phase], pass))
                 residual = __ldcg(sh.a.buffers.hidden + sh.output[thread] + pass * sh.info[phase].slots * static_cast<int>(gridDim.x) * 16);
         }
-        const uint32_t place = phase == 3 ? consume_pass<TILES, true>(phase, pass, first_step) : consume_pass<TILES, false>(phase, pass, first_step);
+        const uint32_t place = phase == 3 ? consume_pass<TILES, true>(phase, layer, pass, first_step) : consume_pass<TILES, false>(phase, layer, pass, first_step);
         stamp(layer, 26 + phase);
         cta_sync();
         if (thread_now() == 0) sh.place = place;  // read again behind the next meeting
@@ -1538,6 +1688,7 @@ __device__ __forceinline__ void matrix_step(int phase, int layer) {
             const int warp = thread_now() >> 5, lanes = sh.a.lanes;
             if (warp < lanes)
                 store_operand_group(sh.a.buffers.activation + static_cast<size_t>(blockIdx.x + pass * gridDim.x) * operand_group_bytes(lanes),
+                                    sh.a.buffers.residual + static_cast<size_t>(blockIdx.x + pass * gridDim.x) * operand_group_bytes(lanes),
                                     reinterpret_cast<const float *>(smem_raw + sh.products) + warp * 128, warp, lanes);
         }
         pass++;
@@ -1717,13 +1868,14 @@ __device__ __forceinline__ void prepare_rings(int q_width, int kv_width) {
     if (thread >= 32 && thread < 64) {
         // columns without a lane repeat lane 0's, their results are dropped
         const int g = (thread & 31) >> 2, j = thread & 3;
-        const int m = TILES == 1 ? g >> 2 : (TILES == 2 ? g >> 1 : g), term = TILES == 1 ? ((g & 3) < 2 ? g & 3 : 2) : (TILES == 2 ? g & 1 : 0);
-        const uint32_t row = static_cast<uint32_t>(m < lanes ? m : 0) * 192u + static_cast<uint32_t>(j) * 16u;
+        const int column = TILES == 1 ? g >> 2 : (TILES == 2 ? g >> 1 : g), m = column < lanes ? column : 0, term = TILES == 1 ? g & 3 : (TILES == 2 ? g & 1 : 0);
+        const int summed = TILES == 1 ? j >> 1 : (TILES == 2 ? j : 2 * j);  // the lane (the first of two) of the thread's sums
+        const uint32_t row = static_cast<uint32_t>(m) * 256u + static_cast<uint32_t>(j) * 16u;
         OperandPlace place;
         place.half = operand_half_bytes(lanes);
-        place.first = row + static_cast<uint32_t>(term) * 64u;
-        place.second = row + 128u;
-        place.factor = 2 * place.half + (TILES == 1 ? static_cast<uint32_t>(j >> 1) * 4u : (TILES == 2 ? static_cast<uint32_t>(j) * 4u : static_cast<uint32_t>(j) * 8u));
+        place.first = row + term_offset(term, m);
+        place.second = row + term_offset(term, m + 1);
+        place.factor = 2 * place.half + static_cast<uint32_t>(summed < lanes ? summed : 0) * 4u;
         sh.operand_place[thread & 31] = place;
     }
     if (thread == 64) {
@@ -1877,15 +2029,15 @@ cudaError_t launch_instance_of(const StackArgs &args, size_t smem, int grid, cud
     return cudaLaunchKernelEx(&config, decode_stack_kernel<HD, GROUP, EXCHANGE, TILES>, args);
 }
 
-// MMA columns of a batch in eights: three terms per lane, none of them split over two threads' columns from three lanes on.
-constexpr int stack_tiles(int lanes) { return lanes <= 2 ? 1 : (lanes <= 4 ? 2 : 3); }
+// MMA columns of a batch in eights: four terms per lane.
+constexpr int stack_tiles(int lanes) { return lanes <= 2 ? 1 : (lanes <= 4 ? 2 : 4); }
 
 template <int HD, int GROUP, bool EXCHANGE>
 cudaError_t launch_instance_of(const StackArgs &args, size_t smem, int grid, cudaStream_t stream) {
     switch (stack_tiles(args.lanes)) {
         case 1: return launch_instance_of<HD, GROUP, EXCHANGE, 1>(args, smem, grid, stream);
         case 2: return launch_instance_of<HD, GROUP, EXCHANGE, 2>(args, smem, grid, stream);
-        default: return launch_instance_of<HD, GROUP, EXCHANGE, 3>(args, smem, grid, stream);
+        default: return launch_instance_of<HD, GROUP, EXCHANGE, 4>(args, smem, grid, stream);
     }
 }
 template <int HD, int GROUP>
@@ -1896,6 +2048,8 @@ cudaError_t launch_instance(const StackArgs &args, size_t smem, int grid, cudaSt
 }  // namespace
 
 size_t stack_activation_bytes(int ffn) { return static_cast<size_t>(ffn >> 7) * operand_group_bytes(8); }
+
+size_t stack_residual_bytes(int ffn, int widest) { return static_cast<size_t>((ffn >> 7) + (widest >> 7)) * operand_group_bytes(8); }
 
 size_t int4_cta_stream_bytes(int rows, int k, bool pair, int grid) {
     return stack_stream_bytes(stack_schedule(rows / 16, k / 128, pair, grid));

@@ -72,6 +72,7 @@ extern "C" __attribute__((visibility("default"))) int stack_layers(StackLayers *
     buffers.attention_scratch = static_cast<float *>(allocate(static_cast<size_t>(t->lanes) * t->q_heads * (splits + (splits + 31) / 32) * (t->head_width + 2) * 4));
     buffers.attention_out = static_cast<uint16_t *>(t->attention_out);
     buffers.activation = static_cast<uint8_t *>(allocate(stack_activation_bytes(t->ffn)));
+    buffers.residual = static_cast<uint8_t *>(allocate(stack_residual_bytes(t->ffn, t->hidden_width > q_width ? t->hidden_width : q_width)));
     buffers.barrier = static_cast<unsigned int *>(allocate(STACK_BARRIER_WORDS * 4));
     buffers.error_flag = static_cast<int *>(allocate(4));
     const LaneTable meta{static_cast<const uint32_t *>(t->positions), static_cast<const int32_t *>(t->slots)};

@@ -11,7 +11,7 @@ A layer is made so that one of its steps has inputs that are known exactly and o
 Row r of the tested matrix has weights only on columns below its own bound of magnitude, so that a large value in a group
 does not cover what the small ones of the group add up to.  An output may be off by half a bf16 unit and by 2^-20 of the sum
 of its terms' magnitudes (the f32 sums over the groups and the warps: some fifty roundings of 2^-24, and what a tie makes of
-them)."""
+them).  A column below 2^-17 may be off by 2^-25, as an fp16 number is, where no value of its group reaches 64."""
 
 import ctypes
 import subprocess
@@ -76,7 +76,9 @@ class _Layer:
     def product(self, name, x):
         """Sums and sums of magnitudes in 64 bits, for rows x of [lanes, k]."""
         full = self.weight[name] * np.repeat(self.scale[name], 128, axis=1)
-        return x @ full.T, np.abs(x) @ np.abs(full).T
+        largest = np.repeat(np.abs(x).reshape(len(x), -1, 128).max(-1), 128, axis=1)
+        coarse = (np.abs(x) < 2.0**-17) & (largest < 64)  # where a column may be off by 2^-25, as an fp16 number is
+        return x @ full.T, (np.abs(x) + 2.0**-5 * coarse) @ np.abs(full).T
 
     def run(self, launch, hidden, normalised_sum=0.5, positions=None, pool=None, pages=1, attended=1):
         """The residual stream and the value projections; with `pool` (a stream per lane, their pages in turn) the attention
@@ -129,6 +131,101 @@ def _check(got, sums, magnitudes, where):
     unit = np.exp2(np.floor(np.log2(np.maximum(np.abs(sums), 2.0**-100))) - 7)
     excess = np.abs(got - sums) - (0.5 * unit + 2.0**-20 * magnitudes)
     assert np.isfinite(got).all() and excess.max() <= 0, (where, np.unravel_index(excess.argmax(), excess.shape), got.flat[excess.argmax()], sums.flat[excess.argmax()])
+
+
+def _spread(rng, count, kind):
+    """Inputs of a step, in groups that lie far apart: `outlier` has one value of 10^4 among ones of 0.05 in every group, `range`
+    magnitudes from 2^-36 to 2^15; in both a group of zeros, one of ordinary values, one of large whole numbers."""
+    if kind == "outlier":
+        values = rng.normal(size=count) * rng.normal(size=count) * 0.05
+        values[::128] = 1e4
+    else:
+        values = rng.choice([-1.0, 1.0], size=count) * 2.0 ** rng.uniform(-36, 15, size=count)
+    values = _bf16(values)
+    if count >= 512:
+        values[128:256] = _bf16(rng.normal(size=128))
+        values[256:384] = 0.0
+        values[384:512] = rng.integers(60000, 250000, size=128) // 2048 * 2048
+    return values
+
+
+def _bounded(rng, layer, name, values):
+    """Weights of every row on the columns below a bound of its own only."""
+    n, k = layer.weight[name].shape
+    magnitudes = np.abs(values)
+    bounds = rng.choice(magnitudes[magnitudes > 0], size=n)
+    layer.weight[name][:] = np.where(magnitudes[None, :] <= bounds[:, None], rng.integers(-8, 8, size=(n, k)), 0)
+    layer.scale[name][:] = _bf16(rng.uniform(0.5, 1.0, size=(n, k // 128)))
+
+
+def _step_case(step, kind, hidden_width=512, offset=0.0):
+    """(layer, hidden rows of eight lanes, what reads the step's outputs from run()'s results, sums, magnitudes)"""
+    rng = np.random.default_rng(7)
+    layer = _Layer(hidden_width, 16, 8, 32, 768, offset)
+    hidden, half = _hidden(rng, 8, hidden_width), hidden_width // 2
+    if step in ("v", "up"):
+        values = _spread(rng, hidden_width, kind)
+        if offset:  # what the offset leaves of a bf16 weight
+            values = _bf16(values - offset) + offset
+            values = np.where(_bf16(values) == values, values, 1.0)
+        values[0] = 1.0  # (the gates')
+        layer.norm["input" if step == "v" else "post"] = values - offset
+        _bounded(rng, layer, step, np.where(np.arange(hidden_width) < half, values, 0.0))
+        sums, magnitudes = layer.product(step, hidden * values)
+        if step == "v":
+            return layer, hidden, (lambda out, got: got), sums, magnitudes
+        layer.weight["down"][half + np.arange(256), np.arange(256)] = 1
+        layer.scale["down"][half : half + 256, :2] = 1.0
+        magnitudes += 2.0**-38 * magnitudes.max()  # (down hands them on: 2^-58 of a group's largest is the least its form holds)
+        return layer, hidden, (lambda out, got: out[:, half : half + 256] / 32.0), sums[:, :256], magnitudes[:, :256]
+    if step == "o":
+        values = _spread(rng, 256, kind)
+        columns = layer.single("v", values)
+        head = np.arange(512) // 32 // 2 * 32 + np.arange(512) % 32
+        inputs = (hidden[:, columns] * values)[:, head]
+        _bounded(rng, layer, "o", values[head])
+    else:
+        values = _spread(rng, 768, kind)
+        columns = layer.single("up", values)
+        inputs = hidden[:, columns] * values * 32.0
+        _bounded(rng, layer, "down", values)
+    sums, magnitudes = layer.product(step, inputs)
+    return layer, hidden, (lambda out, got: out[:, half:]), sums[:, half:], magnitudes[:, half:]
+
+
+@pytest.mark.parametrize("kind", ["outlier", "range"])
+@pytest.mark.parametrize("step", ["v", "o", "up", "down"])
+def test_values_far_apart_in_a_group(launch, step, kind):
+    """... at every width, each lane bit for bit as alone."""
+    layer, hidden, read, sums, magnitudes = _step_case(step, kind)
+    alone = [read(*layer.run(launch, hidden[m : m + 1]))[0] for m in range(8)]
+    for lanes in (1, 2, 3, 4, 5, 8):
+        got = read(*layer.run(launch, hidden[:lanes]))
+        _check(got, sums[:lanes], magnitudes[:lanes], (step, lanes))
+        assert np.array_equal(got, np.stack(alone[:lanes])), lanes
+
+
+def test_values_far_apart_with_a_norm_offset_and_in_windows(launch):
+    """A norm that adds one to its weights; rows of 8192 columns, which five lanes and more stage in parts."""
+    for hidden_width, offset, widths in ((512, 1.0, (1, 4, 8)), (8192, 0.0, (1, 4, 5, 8))):
+        layer, hidden, read, sums, magnitudes = _step_case("v", "outlier", hidden_width, offset)
+        for lanes in widths:
+            _check(read(*layer.run(launch, hidden[:lanes])), sums[:lanes], magnitudes[:lanes], (hidden_width, lanes))
+
+
+def test_infinities_and_nans_stay_in_their_lane(launch):
+    """A lane whose row holds one has no finite output in a step that reads it; the others are as without it."""
+    layer, hidden, read, sums, magnitudes = _step_case("v", "outlier")
+    expected = read(*layer.run(launch, hidden[:6]))
+    for value in (np.inf, -np.inf, np.nan):
+        rows = hidden[:6].copy()
+        rows[2, 5] = value
+        got = read(*layer.run(launch, rows))
+        others = [0, 1, 3, 4, 5]
+        assert np.isnan(got[2]).all() and np.array_equal(got[others], expected[others])
+    layer, hidden, read, _, _ = _step_case("down", "outlier")
+    layer.scale["up"][layer.weight["up"].any(axis=1).nonzero()[0][-1]] = 2.0**126  # times 32: an infinity in down's last group
+    assert np.isnan(read(*layer.run(launch, hidden[:3]))).all()
 
 
 def test_a_group_at_the_end_of_a_row_keeps_its_own_scale(launch):
