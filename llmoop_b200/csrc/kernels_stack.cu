@@ -500,6 +500,10 @@ __device__ __forceinline__ void wait_barrier(uint32_t barrier, uint32_t parity) 
 // products times 0.05.  The fourth byte is free up to four lanes - the MMA's columns were there - and costs a fourth column
 // tile from five on.)
 //
+// A group that holds a NaN has a NaN for its factor, so that all its sums are.  One with infinities has zeros, a factor of -0 and
+// +-1 for them in the residual, whose factor is an infinity then: a row whose weight there is not 0 gets an infinity, any
+// other a NaN, as from the products (of several infinities in one group the sum of the weights decides).
+//
 // A group takes operand_group_bytes(lanes) bytes: [half h][lane][term t][j] pieces of 16 bytes (the B fragments of
 // MMAs 2h and 2h + 1 for thread column j: the digits of the eight columns of word 4j + 2h, even columns first, then
 // those of word 4j + 2h + 1; where lane + h is odd the terms are in the order 1, 0, 3, 2, so that a term of two neighbours falls
@@ -510,13 +514,16 @@ __device__ __forceinline__ uint32_t operand_word_offset(int word, int m, int lan
 }
 __host__ __device__ constexpr uint32_t term_offset(int term, int lane_and_half) { return static_cast<uint32_t>(term ^ (lane_and_half & 1)) * 64u; }
 // From the exponent field of a group's largest magnitude: the factor onto X / 2^8, and the group's factor (2^-4 of a unit since
-// the MMA sees sixteen times the weights).  A group that holds an infinity or a NaN makes its sums NaN.
+// the MMA sees sixteen times the weights); of finite groups.
 __device__ __forceinline__ float operand_scale(uint32_t exponent) { return __uint_as_float((275u - (exponent < 40u ? 40u : exponent)) << 23); }
-__device__ __forceinline__ float operand_factor(uint32_t exponent) {
-    return __uint_as_float(exponent == 255u ? 0x7fc00000u : ((exponent < 40u ? 40u : exponent) - 33u) << 23);
-}
-__device__ __forceinline__ bool operand_may_lose(uint32_t exponent) { return exponent >= 133u && exponent != 255u; }  // (133: 64)
+__device__ __forceinline__ float operand_factor(uint32_t exponent) { return __uint_as_float(((exponent < 40u ? 40u : exponent) - 33u) << 23); }
+__device__ __forceinline__ bool operand_may_lose(uint32_t exponent) { return exponent >= 133u; }  // (133: 64; 255: not finite)
 constexpr float RESIDUAL_SCALE = 4194304.0f, RESIDUAL_UNIT = 0x1p-30f;  // what is left in units of t3, onto X' / 2^8; the factors' ratio
+__device__ __forceinline__ float special_factor(bool nan, bool infinite) { return __uint_as_float(nan ? 0x7fc00000u : (infinite ? 0x80000000u : 0u)); }
+__device__ __forceinline__ float residual_factor(float factor) {
+    const uint32_t bits = __float_as_uint(factor);
+    return bits >> 31 == 0 ? 0.0f : (bits == 0x80000000u ? INFINITY : -factor * RESIDUAL_UNIT);  // (NaN is positive)
+}
 // A pair of values as X + 0x00808080: 2^7 in front of the lower digits makes their bytes unsigned, so that no digit borrows from
 // the next.  f32 rounds to whole numbers where it is 1.5 * 2^23 + X; it does so for X / 2^8, then for the 2^8 of what is left.
 // (Additions of integers are multiply-adds by an opaque one: they leave the half-rate integer pipe to the permutes.)
@@ -550,38 +557,61 @@ __device__ __forceinline__ void operand_digits(uint32_t y0, uint32_t y1, uint32_
     terms[3] = __byte_perm(low01, low23, 0x5410) ^ 0x80808080u;
 }
 __device__ __forceinline__ uint32_t operand_negative(uint32_t y) { return 0x01010100u - y; }
+constexpr uint32_t OPERAND_ZERO = 0x00808080u;
+__device__ __forceinline__ uint32_t operand_of_infinity(uint32_t bits) {  // of an f32: +-1 if it is infinite
+    return (bits & 0x7fffffffu) != 0x7f800000u ? OPERAND_ZERO : (bits >> 31 ? OPERAND_ZERO - 1u : OPERAND_ZERO + 1u);
+}
 __device__ __forceinline__ uint32_t larger_halves(uint32_t a, uint32_t b) {
     uint32_t v;
     asm("max.u16x2 %0, %1, %2;" : "=r"(v) : "r"(a), "r"(b));
     return v;
 }
 
-// What the four bytes lose of a thread's eight columns (see the operand form); by the sixteen threads of a group together.
+// What the four bytes cannot hold of a thread's eight columns (see the operand form); by the sixteen threads of a group together.
 // `place`: its pieces in shared memory, already written; `residual`: those in the residual's group.
 __device__ __noinline__ void keep_residual(uint4 raw, uint32_t exponent, int lane_and_half, uint8_t *place, uint8_t *residual, float *factor) {
     const DigitConstants c = digit_constants();
     const float scale = operand_scale(exponent);
     const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w}, half_warp = 0xffffu << (thread_now() & 16);
-    uint32_t whole[4][2], terms[2][4];
-    unsigned long long left[4];
-    bool lost = false;
+    uint32_t whole[4][2], rest[4][2], terms[2][4];
+    float marked = -operand_factor(exponent);
+    if (exponent == 255u) {  // (of the warp's two groups; a finite one beside it counts nothing: no sum of the row is)
+        bool nan = false, infinite = false;
 #pragma unroll
-    for (int w = 0; w < 4; w++) {
-        operand_wholes(pair_of(bf16_lo(words[w]), bf16_hi(words[w])), pair_of(scale, scale), c, whole[w][0], whole[w][1], left[w]);
-        lost |= ((left[w] | (left[w] >> 32)) & 0x7fffffffu) != 0;
+        for (int w = 0; w < 4; w++)
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const uint32_t bits = i == 0 ? words[w] << 16 : words[w] & 0xffff0000u;
+                nan |= (bits & 0x7fffffffu) > 0x7f800000u;
+                infinite |= (bits & 0x7fffffffu) == 0x7f800000u;
+                whole[w][i] = OPERAND_ZERO;
+                rest[w][i] = operand_of_infinity(bits);
+            }
+        nan = __any_sync(half_warp, nan);
+        infinite = __any_sync(half_warp, infinite);
+        marked = special_factor(nan, infinite);
+    } else {
+        unsigned long long left[4];
+        bool lost = false;
+#pragma unroll
+        for (int w = 0; w < 4; w++) {
+            operand_wholes(pair_of(bf16_lo(words[w]), bf16_hi(words[w])), pair_of(scale, scale), c, whole[w][0], whole[w][1], left[w]);
+            lost |= ((left[w] | (left[w] >> 32)) & 0x7fffffffu) != 0;
+        }
+        if (!__any_sync(half_warp, lost)) return;
+#pragma unroll
+        for (int w = 0; w < 4; w++) {
+            whole[w][0] = operand_negative(whole[w][0]), whole[w][1] = operand_negative(whole[w][1]);
+            operand_wholes(left[w], pair_of(RESIDUAL_SCALE, RESIDUAL_SCALE), c, rest[w][0], rest[w][1], left[w]);
+        }
     }
-    if (!__any_sync(half_warp, lost)) return;
-#pragma unroll
-    for (int w = 0; w < 4; w++) whole[w][0] = operand_negative(whole[w][0]), whole[w][1] = operand_negative(whole[w][1]);
 #pragma unroll
     for (int i = 0; i < 2; i++) operand_digits(whole[0][i], whole[1][i], whole[2][i], whole[3][i], terms[i]);
 #pragma unroll
     for (int t = 0; t < 4; t++) *reinterpret_cast<uint2 *>(place + term_offset(t, lane_and_half)) = make_uint2(terms[0][t], terms[1][t]);
-    if (factor != nullptr) *factor = -operand_factor(exponent);
+    if (factor != nullptr) *factor = marked;
 #pragma unroll
-    for (int w = 0; w < 4; w++) operand_wholes(left[w], pair_of(RESIDUAL_SCALE, RESIDUAL_SCALE), c, whole[w][0], whole[w][1], left[w]);
-#pragma unroll
-    for (int i = 0; i < 2; i++) operand_digits(whole[0][i], whole[1][i], whole[2][i], whole[3][i], terms[i]);
+    for (int i = 0; i < 2; i++) operand_digits(rest[0][i], rest[1][i], rest[2][i], rest[3][i], terms[i]);
 #pragma unroll
     for (int t = 0; t < 4; t++) *reinterpret_cast<uint2 *>(residual + term_offset(t, lane_and_half)) = make_uint2(terms[0][t], terms[1][t]);  // (every CTA writes the same)
 }
@@ -759,13 +789,27 @@ __device__ __forceinline__ void store_operand_group(uint8_t *block, uint8_t *res
     for (int i = 0; i < 2; i++) operand_wholes(pair_of(v[2 * i], v[2 * i + 1]), pair_of(scale, scale), c, whole[2 * i], whole[2 * i + 1], left[i]);
     const uint32_t at = operand_word_offset(word, m, lanes) + 4 * odd;
     const unsigned long long any = (left[0] | left[1]) & 0x7fffffff7fffffffull;
-    if (operand_may_lose(exponent) && __any_sync(0xffffffffu, any != 0)) {
-        factor = -factor;
-#pragma unroll
-        for (int i = 0; i < 4; i++) whole[i] = operand_negative(whole[i]);
+    if (operand_may_lose(exponent) && (exponent == 255u || __any_sync(0xffffffffu, any != 0))) {
         uint32_t rest[4];
+        if (exponent == 255u) {
+            bool nan = false, infinite = false;
 #pragma unroll
-        for (int i = 0; i < 2; i++) operand_wholes(left[i], pair_of(RESIDUAL_SCALE, RESIDUAL_SCALE), c, rest[2 * i], rest[2 * i + 1], left[i]);
+            for (int i = 0; i < 4; i++) {
+                nan |= v[i] != v[i];
+                infinite |= fabsf(v[i]) == INFINITY;
+                whole[i] = OPERAND_ZERO;
+                rest[i] = operand_of_infinity(__float_as_uint(v[i]));
+            }
+            nan = __any_sync(0xffffffffu, nan);
+            infinite = __any_sync(0xffffffffu, infinite);
+            factor = special_factor(nan, infinite);
+        } else {
+            factor = -factor;
+#pragma unroll
+            for (int i = 0; i < 4; i++) whole[i] = operand_negative(whole[i]);
+#pragma unroll
+            for (int i = 0; i < 2; i++) operand_wholes(left[i], pair_of(RESIDUAL_SCALE, RESIDUAL_SCALE), c, rest[2 * i], rest[2 * i + 1], left[i]);
+        }
         operand_digits(rest[0], rest[1], rest[2], rest[3], terms);
 #pragma unroll
         for (int t = 0; t < 4; t++) *reinterpret_cast<uint32_t *>(residual + at + term_offset(t, m + (word >> 1))) = terms[t];
@@ -1425,7 +1469,7 @@ __device__ __noinline__ void add_residuals(int phase, int layer, int pass, int f
         }
         if (!__any_sync(0xffffffffu, factor_signs<TILES>(x.factor, second) >> 31)) continue;
 #pragma unroll
-        for (int i = 0; i < 2; i++) x.factor[i] = __float_as_uint(x.factor[i]) >> 31 ? -x.factor[i] * RESIDUAL_UNIT : 0.0f;  // (NaN is positive)
+        for (int i = 0; i < 2; i++) x.factor[i] = residual_factor(x.factor[i]);
         load_pieces<TILES>(x, place, [&](uint32_t offset) { return __ldcg(reinterpret_cast<const uint4 *>(residuals + group + offset)); });
         for (int t = 0; t < blocks.tiles; t++) {
             const uint8_t *unit = stream + static_cast<size_t>(step) * stage + t * blocks.next_tile;
