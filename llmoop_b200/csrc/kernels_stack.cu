@@ -620,18 +620,20 @@ __device__ __noinline__ void keep_residual(uint4 raw, uint32_t exponent, int lan
 // (rms_norm_bf16.comp.template:49-72), without it the bf16 values as they are.  Each CTA repeats it: 8 KB per lane
 // from L2.  A thread owns chunk t (and t + 512 when CHUNKS = 2) of each lane, four lanes at a time: one pass over
 // registers for the sums of squares, one block-wide exchange, then normalise, round, find the exponent and cut the digits.
-template <int CHUNKS, int LANES>  // chunks per thread and lane: width <= CHUNKS * 8 * CONSUMER_THREADS; lanes at a time (1, 2 or 4)
-__device__ __forceinline__ void stage_rows(const uint16_t *x, const uint16_t *weight, int width, int first_group, int groups) {
+// With FROM_GROUP (no weight) the threads own chunks from the first group on, whose operand form goes `destination` bytes into
+// the scratch area.
+template <int CHUNKS, int LANES, bool FROM_GROUP = false>  // chunks per thread and lane: columns <= CHUNKS * 8 * CONSUMER_THREADS; lanes at a time (1, 2 or 4)
+__device__ __forceinline__ void stage_rows(const uint16_t *x, const uint16_t *weight, int width, int first_group, int groups, uint32_t destination = 0) {
     const StackShared &sh = shared();
-    uint8_t *operands = smem_raw + sh.scratch;
+    uint8_t *operands = smem_raw + sh.scratch + destination;
     float *partial = shared().norm_partial;
-    const int lanes = sh.a.lanes, per_lane = width >> 3, thread = thread_now(), warp = thread >> 5, lane = thread & 31;
+    const int lanes = sh.a.lanes, per_lane = width >> 3, thread = thread_now(), warp = thread >> 5, lane = thread & 31, first_chunk = thread + (FROM_GROUP ? first_group * 16 : 0);
     const float eps = sh.a.shape.eps, offset = sh.a.shape.norm_offset;
     const uint4 *source = reinterpret_cast<const uint4 *>(x);
     uint4 scale_words[CHUNKS];
 #pragma unroll
     for (int c = 0; c < CHUNKS; c++) {
-        const int chunk = thread + c * CONSUMER_THREADS;
+        const int chunk = first_chunk + c * CONSUMER_THREADS;
         scale_words[c] = weight != nullptr && chunk < per_lane ? __ldg(reinterpret_cast<const uint4 *>(weight) + chunk) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll 1
@@ -641,7 +643,7 @@ __device__ __forceinline__ void stage_rows(const uint16_t *x, const uint16_t *we
         for (int mm = 0; mm < LANES; mm++)
 #pragma unroll
             for (int c = 0; c < CHUNKS; c++) {
-                const int chunk = thread + c * CONSUMER_THREADS;
+                const int chunk = first_chunk + c * CONSUMER_THREADS;
                 // lanes beyond the batch read the last lane again (their results are not stored)
                 const int m = m0 + mm < lanes ? m0 + mm : lanes - 1;
                 raw[mm][c] = __ldcg(source + static_cast<size_t>(m) * per_lane + (chunk < per_lane ? chunk : 0));
@@ -698,7 +700,7 @@ __device__ __forceinline__ void stage_rows(const uint16_t *x, const uint16_t *we
         }
 #pragma unroll
         for (int c = 0; c < CHUNKS; c++) {
-            const int chunk = thread + c * CONSUMER_THREADS, group = (chunk >> 4) - first_group;
+            const int chunk = first_chunk + c * CONSUMER_THREADS, group = (chunk >> 4) - first_group;
             unsigned long long norm[4];
             if (weight != nullptr) {
                 const uint32_t sc[4] = {scale_words[c].x, scale_words[c].y, scale_words[c].z, scale_words[c].w};
@@ -764,8 +766,15 @@ __device__ __forceinline__ void stage_rows(const uint16_t *x, const uint16_t *we
     cta_sync();
 }
 
+// Rows too wide for a thread's two chunks (o's inputs: no norm looks at whole ones), 8192 columns at a time.
+__device__ __noinline__ void stage_wide_rows(const uint16_t *x, int width, int first_group, int groups) {
+    const int end = first_group + groups < width >> 7 ? first_group + groups : width >> 7, at_a_time = 2 * CONSUMER_THREADS / 16;
+    for (int group = first_group; group < end; group += at_a_time)
+        stage_rows<2, 2, true>(x, nullptr, width, group, end - group < at_a_time ? end - group : at_a_time, static_cast<uint32_t>(group - first_group) * operand_group_bytes(shared().a.lanes));
+}
 template <int TILES>
 __device__ __forceinline__ void stage_any(const uint16_t *x, const uint16_t *weight, int width, int first_group, int groups) {
+    if (width > 2 * 8 * CONSUMER_THREADS) return stage_wide_rows(x, width, first_group, groups);
     const bool narrow = width <= 8 * CONSUMER_THREADS;
     if (TILES == 1 && shared().a.lanes == 1) return narrow ? stage_rows<1, 1>(x, weight, width, first_group, groups) : stage_rows<2, 1>(x, weight, width, first_group, groups);
     constexpr int LANES = TILES == 1 ? 2 : 4;
@@ -2125,7 +2134,7 @@ cudaError_t launch_int4_cta_streams(const RelayoutSegment *segments, int count, 
 
 bool decode_stack_supported(const StackShape &shape, int lanes, size_t *smem_bytes) {
     if (lanes < 1 || lanes > 8 || shape.grid < 1) return false;
-    if (shape.hidden > 2 * 8 * CONSUMER_THREADS || shape.q_heads * shape.head_width > 2 * 8 * CONSUMER_THREADS || shape.hidden % 128 != 0 || shape.ffn % 128 != 0 || (shape.q_heads * shape.head_width) % 128 != 0) return false;
+    if (shape.hidden > 2 * 8 * CONSUMER_THREADS || shape.hidden % 128 != 0 || shape.ffn % 128 != 0 || (shape.q_heads * shape.head_width) % 128 != 0) return false;
     if (((shape.q_heads + 2 * shape.kv_heads) * shape.head_width) % 16 != 0 || shape.kv_heads * 8 > STACK_BARRIER_WORDS - ARRIVAL_WORDS_OFFSET) return false;
     StackPlanSmem plan;
     if (!plan_smem(shape, lanes, shape.grid, &plan)) return false;

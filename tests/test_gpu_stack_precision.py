@@ -158,10 +158,10 @@ def _bounded(rng, layer, name, values):
     layer.scale[name][:] = _bf16(rng.uniform(0.5, 1.0, size=(n, k // 128)))
 
 
-def _step_case(step, kind, hidden_width=512, offset=0.0):
+def _step_case(step, kind, hidden_width=512, offset=0.0, heads=(16, 8, 32)):
     """(layer, hidden rows of eight lanes, what reads the step's outputs from run()'s results, sums, magnitudes)"""
     rng = np.random.default_rng(7)
-    layer = _Layer(hidden_width, 16, 8, 32, 768, offset)
+    layer = _Layer(hidden_width, *heads, 768, offset)
     hidden, half = _hidden(rng, 8, hidden_width), hidden_width // 2
     if step in ("v", "up"):
         values = _spread(rng, hidden_width, kind)
@@ -179,9 +179,10 @@ def _step_case(step, kind, hidden_width=512, offset=0.0):
         magnitudes += 2.0**-38 * magnitudes.max()  # (down hands them on: 2^-58 of a group's largest is the least its form holds)
         return layer, hidden, (lambda out, got: out[:, half : half + 256] / 32.0), sums[:, :256], magnitudes[:, :256]
     if step == "o":
-        values = _spread(rng, 256, kind)
+        q_heads, kv_heads, width = heads
+        values = _spread(rng, kv_heads * width, kind)
         columns = layer.single("v", values)
-        head = np.arange(512) // 32 // 2 * 32 + np.arange(512) % 32
+        head = np.arange(q_heads * width) // width // (q_heads // kv_heads) * width + np.arange(q_heads * width) % width  # of the value row, by column of o's input
         inputs = (hidden[:, columns] * values)[:, head]
         _bounded(rng, layer, "o", values[head])
     else:
@@ -211,6 +212,13 @@ def test_values_far_apart_with_a_norm_offset_and_in_windows(launch):
         layer, hidden, read, sums, magnitudes = _step_case("v", "outlier", hidden_width, offset)
         for lanes in widths:
             _check(read(*layer.run(launch, hidden[:lanes])), sums[:lanes], magnitudes[:lanes], (hidden_width, lanes))
+
+
+def test_query_rows_of_more_than_8192_columns(launch):
+    """... whole for one lane, in windows of steps from three on."""
+    layer, hidden, read, sums, magnitudes = _step_case("o", "range", heads=(72, 9, 128))
+    for lanes in (1, 3, 8):
+        _check(read(*layer.run(launch, hidden[:lanes])), sums[:lanes], magnitudes[:lanes], lanes)
 
 
 def test_infinities_and_nans(launch):
