@@ -423,7 +423,7 @@ void MountedModel::build_stack(const std::vector<ComponentPlan> &layers, int fir
             DeviceBuffer stream = device_alloc(std::max<size_t>(16, int4_cta_stream_bytes(rows, kk, pair, here.grid)), false);
             storage.push_back(stream);
             cuda_check(launch_int4_cta_streams(segments, count, pair, kk, here.grid, static_cast<uint8_t *>(stream.ptr), nullptr), "per-CTA INT4 stream copy");
-            bytes += stream.bytes;
+            bytes += static_cast<uint64_t>(pair ? 2 * rows : rows) * (kk / 2 + kk / 128 * 2);  // (without a stream's padding)
             return static_cast<const uint8_t *>(stream.ptr);
         };
         StackLayer spec{};

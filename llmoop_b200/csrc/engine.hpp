@@ -58,7 +58,7 @@ struct StackPlan {
     std::vector<StackLayer> layers;     // host copy of the device array
     DeviceBuffer device_layers;
     std::vector<DeviceBuffer> storage;  // tile-major weights and scales
-    uint64_t weight_bytes = 0;          // bytes one pass over the stack streams
+    uint64_t weight_bytes = 0;          // bytes of the weights one pass over the stack reads
 };
 
 struct SmallStackPlan {

@@ -211,7 +211,8 @@ cudaError_t launch_linear_bf16_gemm(const uint16_t *x, const uint16_t *w, void *
 // c + grid, ...  The rows of a gate/up pair alternate tile by tile (gate, up, gate, ..) and go to the CTAs in runs of
 // sixteen, so that the 128 columns of a run, a quantisation group of the down projection, end in one CTA.  A CTA works on
 // `slots` of its tiles at a time (one pass): 16 warps as slots / 2 pairs of tiles times `width` groups of K, the warp at
-// place i of a pair taking groups i, i + width, ...  Step s of a pass is one stage of the CTA's stream: for every present
+// place i of a pair taking groups i, i + width, ... (no more of them than there are groups: a short K leaves warps without a
+// tile rather than have its stream padded).  Step s of a pass is one stage of the CTA's stream: for every present
 // tile the 16x128 blocks of groups s * width .. s * width + width - 1 (1 KB of nibbles each, zero beyond `groups`), followed
 // by the same blocks' 32-byte scale-pair rows.
 struct MatrixSchedule {
@@ -228,6 +229,7 @@ __host__ __device__ inline MatrixSchedule stack_schedule(int tiles, int groups, 
     while (2 * pairs < most && pairs < 8) pairs *= 2;
     s.slots = 2 * pairs;
     s.width = 16 / pairs;
+    while (s.width / 2 >= groups) s.width /= 2;
     s.steps = (groups + s.width - 1) / s.width;
     return s;
 }

@@ -94,3 +94,5 @@ extern "C" __attribute__((visibility("default"))) int stack_layers(StackLayers *
     if (status != cudaSuccess) return static_cast<int>(status);
     return error != 0 ? -2 - error : 0;
 }
+
+extern "C" __attribute__((visibility("default"))) size_t stream_bytes(int rows, int k, int pair) { return nerve::int4_cta_stream_bytes(rows, k, pair != 0, 148); }

@@ -44,7 +44,10 @@ def launch(tmp_path_factory):
                str(kernels if kernels.exists() else build.CSRC / "kernels_stack.cu")]
     result = subprocess.run(command, capture_output=True, text=True)
     assert result.returncode == 0, result.stderr
-    return ctypes.CDLL(str(library)).stack_layers
+    functions = ctypes.CDLL(str(library))
+    functions.stack_layers.stream_bytes = functions.stream_bytes
+    functions.stream_bytes.restype = ctypes.c_size_t
+    return functions.stack_layers
 
 
 def _bf16(values):
@@ -293,3 +296,11 @@ def test_work_items_without_tokens_between_others(launch):
             expected[m, head], magnitude[m, head] = p / p.sum() @ rows[1, head // 2], p / p.sum() @ np.abs(rows[1, head // 2])
     got = layer.run(launch, hidden, positions=positions, pool=pool, pages=pages, attended=64 * splits)
     _check(got, expected.reshape(8, -1), 32.0 * magnitude.reshape(8, -1), "attention")
+
+
+def test_streams_of_a_short_k_are_not_padded(launch):
+    """A block of 16 x 128 nibbles and its scales is 1056 bytes; a group count that is a power of two leaves no step ragged."""
+    for k in (128, 256, 512, 1024, 2048, 4096):
+        for rows, pair in ((512, 0), (4096, 0), (1024, 1), (14336, 1)):
+            assert launch.stream_bytes(rows, k, pair) == (1 + pair) * rows // 16 * (k // 128) * 1056, (rows, k, pair)
+    assert launch.stream_bytes(1152, 9 * 128, 0) <= 1152 // 16 * 16 * 1056
