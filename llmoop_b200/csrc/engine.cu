@@ -504,7 +504,7 @@ void MountedModel::build_small_stack(const std::vector<ComponentPlan> &layers, i
         here.rope_positions = rope_positions_;
         if (built.empty()) shape = here;
         else if (std::memcmp(&shape, &here, sizeof(shape)) != 0) return;
-        if (!small_stack_supported(shape, static_cast<int>(plan().vocab), 1)) return;
+        if (!small_stack_supported(shape, static_cast<int>(plan().vocab), static_cast<uint32_t>(capacity()), 1)) return;
         spec.kv = kv_layer(kv_index++);
         built.push_back(spec);
     }
@@ -1907,7 +1907,7 @@ bool Engine::run_stack(const StackPlan &stack, int lanes, void *hidden) {
 // The whole forward of a small bf16 model in one launch, a stream per CTA; false = the caller runs it kernel by kernel.
 bool Engine::run_small_stack(const SmallStackPlan &stack, int lanes, const uint16_t *hidden_in, uint16_t *normalized, bool want_logits, const char *what) {
     if (!stack_enabled_ || !stack.available || !streams_apart_ || current_blocks_ > 0 || current_width_ <= 0 || lanes % current_width_ != 0 ||
-        !small_stack_supported(stack.shape, stack.forward.vocab, current_width_))
+        !small_stack_supported(stack.shape, stack.forward.vocab, static_cast<uint32_t>(model_->capacity()), current_width_))
         return false;
     SmallForward forward = stack.forward;
     forward.tokens = current_tokens_;
@@ -1915,7 +1915,8 @@ bool Engine::run_small_stack(const SmallStackPlan &stack, int lanes, const uint1
     forward.normalized = normalized;
     forward.logits = want_logits ? static_cast<float *>(logits_.ptr) : nullptr;
     forward.records = stochastic_streams_ == 0 ? static_cast<uint32_t *>(records_.ptr) : nullptr;
-    check(launch_small_stack(static_cast<const SmallStackLayer *>(stack.device_layers.ptr), stack.layers, stack.shape, forward, current_lanes_, lanes / current_width_,
+    check(launch_small_stack(static_cast<const SmallStackLayer *>(stack.device_layers.ptr), stack.layers, stack.shape, forward, current_lanes_,
+                             static_cast<uint32_t>(model_->capacity()), lanes / current_width_,
                              current_width_, static_cast<int *>(kernel_error_.ptr), cuda_stream_),
           what);
     if (want_logits && stochastic_streams_ != 0)

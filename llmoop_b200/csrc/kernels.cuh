@@ -345,9 +345,9 @@ struct SmallForward {
 };
 constexpr int SMALL_STACK_MAX_LANES = 32;  // per stream
 constexpr int SMALL_STACK_MAX_VOCAB = 1024;
-bool small_stack_supported(const SmallStackShape &shape, int vocab, int lanes_per_stream);
+bool small_stack_supported(const SmallStackShape &shape, int vocab, uint32_t capacity, int lanes_per_stream);
 cudaError_t launch_small_stack(const SmallStackLayer *layers_device, int layer_count, const SmallStackShape &shape, const SmallForward &forward, const LaneTable &lanes_meta,
-                               int streams, int lanes_per_stream, int *error_flag, cudaStream_t stream);
+                               uint32_t capacity, int streams, int lanes_per_stream, int *error_flag, cudaStream_t stream);
 
 // Tensor-parallel row-parallel linears: out = bf16(bf16(sum) + residual) (or bf16(sum) without residual) from the
 // all-reduced f32 sums [count].

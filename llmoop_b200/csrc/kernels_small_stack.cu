@@ -408,19 +408,30 @@ size_t shared_bytes(const SmallStackShape &shape, int lanes) {
 // launches did.  A verify pass of 2 lanes (kernels of the single operations in brackets): hidden 64, FFN 128, 2 layers,
 // vocabulary 256, 20.6 us (34.5), 8 lanes 26 (50), 16 streams 21 (62), 1900 tokens of context 71 (101); hidden 96 with the
 // largest layers that fit and vocabulary 1024 27.8 us (36.4), 1900 tokens 87 (104), but vocabulary 4096 46.5 (37.2).
-bool small_stack_supported(const SmallStackShape &shape, int vocab, int lanes) {
+//
+// The context counts, too: a warp walks the whole window of a (lane, q head), where the other route spreads it over the chip.
+// A layer takes 10, 15 or 62 ns a token (heads of 8, 16, 32) for every sixteen of them, the other route 13 to 19 however many
+// they are, but some 15 us more to begin with (whole calls with the host, hidden 64, 2 layers, 4 heads of 16: 8 lanes 80 us and
+// 111 at 16 tokens, 199 and 180 at 1900, 2029 and 1239 at 32000; 2 lanes 76 and 133, 127 and 164, 965 and 1247; 32 lanes 133 and
+// 130, 592 and 195 at 1900; 3 layers of 8 heads of 8, 8 lanes: 96 and 134, 159 and 153 at 512; a layer of 2 heads of 32, 8 lanes:
+// 78 and 104, 106 and 100 at 512).  So what a whole window takes on top may not exceed those 15 us.  The window is the
+// mount's capacity, not the context, and up to eight lanes the rule is that of eight: what else is in a batch may not
+// change the route of a stream.
+bool small_stack_supported(const SmallStackShape &shape, int vocab, uint32_t capacity, int lanes) {
     if (shape.head_width != 8 && shape.head_width != 16 && shape.head_width != 32) return false;
     if (shape.kv_heads < 1 || shape.q_heads < 1 || shape.q_heads % shape.kv_heads != 0) return false;
     const Sizes z = sizes_of(shape);
     if (shape.hidden < 64 || shape.ffn < 64 || z.q_width < 64) return false;
     if (shape.hidden % 32 != 0 || shape.ffn % 32 != 0 || z.q_width % 32 != 0 || (z.q_width + 2 * z.kv_width) % 16 != 0 || z.kv_width % 8 != 0) return false;
     if (vocab % 16 != 0 || vocab > SMALL_STACK_MAX_VOCAB || lanes < 1 || lanes > SMALL_STACK_MAX_LANES) return false;
-    return shared_bytes(shape, lanes) <= SHARED_LIMIT;
+    const int decided = lanes < 8 ? 8 : lanes, rounds = (decided * shape.q_heads + WARPS - 1) / WARPS;
+    const long long nanoseconds = rounds * (shape.head_width == 8 ? 10 : shape.head_width == 16 ? 15 : 62) - 16;
+    return shared_bytes(shape, decided) <= SHARED_LIMIT && nanoseconds * capacity <= 15000;
 }
 
 cudaError_t launch_small_stack(const SmallStackLayer *layers_device, int layer_count, const SmallStackShape &shape, const SmallForward &forward, const LaneTable &lanes_meta,
-                               int streams, int lanes_per_stream, int *error_flag, cudaStream_t stream) {
-    if (streams < 1 || layer_count < 1 || !small_stack_supported(shape, forward.vocab, lanes_per_stream)) return cudaErrorInvalidValue;
+                               uint32_t capacity, int streams, int lanes_per_stream, int *error_flag, cudaStream_t stream) {
+    if (streams < 1 || layer_count < 1 || !small_stack_supported(shape, forward.vocab, capacity, lanes_per_stream)) return cudaErrorInvalidValue;
     auto kernel = shape.head_width == 32 ? small_stack_kernel<32> : shape.head_width == 16 ? small_stack_kernel<16> : small_stack_kernel<8>;
     // (never lowered: a captured launch keeps its own size)
     const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SHARED_LIMIT);
