@@ -751,13 +751,19 @@ __device__ __forceinline__ void stage_rows(const uint16_t *x, const uint16_t *we
                     operand_digits(whole[0][1], whole[1][1], whole[2][1], whole[3][1], odd);
 #pragma unroll
                     for (int t = 0; t < 4; t++) *reinterpret_cast<uint2 *>(pieces[(t + mm) & 1] + 256 * mm + term_offset(t, mm)) = make_uint2(even[t], odd[t]);  // (m0 is even)
-                    float *factor = word == 0 ? reinterpret_cast<float *>(block + 2 * operand_half_bytes(lanes) + 4 * (m0 + mm)) : nullptr;
-                    if (factor != nullptr) *factor = operand_factor(largest[mm]);
-                    if (operand_may_lose(largest[mm]))
-                        keep_residual(raw[mm][c], largest[mm], mm + (word >> 1), place + 256 * mm,
-                                      sh.a.buffers.residual + static_cast<size_t>((sh.a.shape.ffn >> 7) + (chunk >> 4)) * operand_group_bytes(lanes) +
-                                          operand_word_offset(word, m0 + mm, lanes),
-                                      factor);
+                    if (word == 0) *reinterpret_cast<float *>(block + 2 * operand_half_bytes(lanes) + 4 * (m0 + mm)) = operand_factor(largest[mm]);
+                }
+                uint32_t most = largest[0];
+#pragma unroll
+                for (int mm = 1; mm < LANES; mm++) most = max(most, largest[mm]);
+                if (operand_may_lose(most)) {  // (rare, and apart from the loop: a call in it would cost it registers)
+#pragma unroll
+                    for (int mm = 0; mm < LANES; mm++)
+                        if (m0 + mm < lanes && operand_may_lose(largest[mm]))
+                            keep_residual(raw[mm][c], largest[mm], mm + (word >> 1), place + 256 * mm,
+                                          sh.a.buffers.residual + static_cast<size_t>((sh.a.shape.ffn >> 7) + (chunk >> 4)) * operand_group_bytes(lanes) +
+                                              operand_word_offset(word, m0 + mm, lanes),
+                                          word == 0 ? reinterpret_cast<float *>(block + 2 * operand_half_bytes(lanes) + 4 * (m0 + mm)) : nullptr);
                 }
             }
         }
