@@ -2194,7 +2194,7 @@ void Engine::run_speculative_cycles(std::vector<Stream *> &batch, const std::vec
     const int lanes = streams * width;
     if (lanes > model_->options().max_lanes) fail("verify batch exceeds max_lanes");
 
-    // device cycle arrays carved out of cycle_state_; everything up to `accept_rows` is uploaded in one copy
+    // device cycle arrays carved out of cycle_state_; everything up to `accept_rows` comes from the host's pinned words (launch_begin_cycle)
     uint32_t *base = static_cast<uint32_t *>(cycle_state_.ptr);
     uint32_t *verify_tokens = base;                              // [streams][width]
     uint32_t *forced = verify_tokens + lanes;                    // [streams][drafts]

@@ -262,7 +262,7 @@ __device__ __forceinline__ void fp8_linear_tile(const Fp8LinearArgs &a, int m0, 
     }
 }
 
-// grid (row tiles of 64, lane tiles of 8)
+// grid (row tiles of 32 x passes, lane tiles of 8)
 __global__ void __launch_bounds__(FP8_WARPS * 32, 2) linear_fp8_kernel(const __grid_constant__ Fp8LinearArgs a) {
     extern __shared__ __align__(16) uint8_t fp8_smem[];
     grid_launch_dependents();
