@@ -1,7 +1,7 @@
 """The persistent decode stack kernel at every batch width.
 
-Its products are exact integers (weights as signed bytes, activations as three signed bytes behind a power of two per
-group), with one to three MMA column tiles by the number of lanes: 1-2, 3-4 and 5-8.  A lane's result must not depend on
+Its products are exact integers (weights as signed bytes, activations as four signed bytes behind a power of two per
+group), with one, two or four MMA column tiles by the number of lanes: 1-2, 3-4 and 5-8.  A lane's result must not depend on
 the width, so lane 0 of a batch of n lanes has the logits of the same lane alone, bit for bit, and all of them lie within
 the bars of the other tests of this kernel against the oracle: 2e-2 and 2e-3 (mean) for logits of the scale that 1024
 columns of N(0, 0.01) give them.  Two faithful orders of summation differ by roundings of the hidden state, which the
